@@ -70,6 +70,33 @@ int flash_attention_backward_impl(hl_ctx* ctx, const void* q, const void* k, con
                                   const float* lse, void* dq, void* dk, void* dv, long long ld_dqkv, int batch, int time,
                                   int n_heads, int head_dim, void* scratch, size_t scratch_bytes);
 
+// One f32 product with f64 sums, out[i,j] = epilogue(sum_k A[i,k] * B[k,j]), element strides throughout (ref_f32.cu).  The
+// product is rounded to f32, then the bias is added and rounded, then the epilogue acts, each step rounded as when it
+// was an op of its own.
+enum { F64_STORE = 0, F64_ACCUMULATE = 1 /* out += */, F64_GELU = 2 /* aux_out = gelu(out) */,
+       F64_RESIDUAL = 3 /* out = aux_in + y */, F64_DGELU = 4 /* out = y * gelu'(aux_in) */ };
+struct F64Gemm {
+  const float *a, *b;
+  float* out;
+  long long a_row, a_col, b_row, b_col, o_row, o_col;
+  int m, n, k;
+  int epilogue;
+  const float* bias;    // [n] or null
+  const float* aux_in;  // laid out as out
+  float* aux_out;
+  float* row_sum;       // [m] or null: sum_k A[i,k]
+};
+// One or two independent products in one launch.
+int f64_gemm_run(hl_ctx* ctx, const F64Gemm* problems, int count);
+
+// Causal attention with f64 sums on f32 or bf16 rows with strides; `probs` [B,H,T,T] f32 is written by the forward.  The
+// backward reads it for f32 operands and forms it again for bf16 ones.
+int attention_f64_forward(hl_ctx* ctx, const void* q, const void* k, const void* v, int dtype, long long ld_qkv, void* out,
+                          long long ld_out, float* probs, int batch, int time, int channels, int n_heads);
+int attention_f64_backward(hl_ctx* ctx, const void* q, const void* k, const void* v, int dtype, long long ld_qkv, float* probs,
+                           const void* dout, long long ld_dout, void* dq, void* dk, void* dv, long long ld_dqkv, int batch,
+                           int time, int channels, int n_heads);
+
 struct AdamPlan;
 int adam_plan_create(hl_ctx* ctx, const hl_adamw_tensor* tensors, int count, AdamPlan** out);
 void adam_plan_destroy(AdamPlan* plan);

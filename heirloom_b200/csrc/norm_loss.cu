@@ -101,7 +101,9 @@ __global__ void layer_norm_fwd_kernel(const XT* __restrict__ x, const float* __r
 constexpr int LNB_WARPS = 8;
 constexpr int LNB_MAXJ = 8;
 
-template <typename XT, typename Acc>
+// J: 128-column groups a lane holds sums for, i.e. ceil(features / 128) rounded up to a power of two, so that narrow rows
+// (a byte-level model has 128 features) do not carry, and spill, the registers of the widest ones.
+template <typename XT, typename Acc, int J>
 __global__ void __launch_bounds__(LNB_WARPS * 32)
 layer_norm_bwd_kernel(const XT* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ dy,
                       const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
@@ -111,9 +113,9 @@ layer_norm_bwd_kernel(const XT* __restrict__ x, const float* __restrict__ gamma,
   extern __shared__ float lnb_smem[];  // [LNB_WARPS][2][features]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r0 = blockIdx.x * rows_per_block, r1 = min(rows, r0 + rows_per_block);
-  Acc dg[LNB_MAXJ][4], db[LNB_MAXJ][4];
+  Acc dg[J][4], db[J][4];
 #pragma unroll
-  for (int j = 0; j < LNB_MAXJ; ++j)
+  for (int j = 0; j < J; ++j)
 #pragma unroll
     for (int e = 0; e < 4; ++e) { dg[j][e] = 0; db[j][e] = 0; }
 
@@ -141,7 +143,7 @@ layer_norm_bwd_kernel(const XT* __restrict__ x, const float* __restrict__ gamma,
     }
     Acc s1 = 0, s2 = 0;
 #pragma unroll
-    for (int j = 0; j < LNB_MAXJ; ++j) {
+    for (int j = 0; j < J; ++j) {
       const int c = (j * 32 + lane) * 4;
       if (c < features) {
         float v[4], g[4], d[4];
@@ -162,7 +164,7 @@ layer_norm_bwd_kernel(const XT* __restrict__ x, const float* __restrict__ gamma,
     s1 = warp_sum(s1);
     s2 = warp_sum(s2);
 #pragma unroll
-    for (int j = 0; j < LNB_MAXJ; ++j) {
+    for (int j = 0; j < J; ++j) {
       const int c = (j * 32 + lane) * 4;
       if (c < features) {
         float v[4], g[4], d[4], o[4];
@@ -186,7 +188,7 @@ layer_norm_bwd_kernel(const XT* __restrict__ x, const float* __restrict__ gamma,
   // fold the warps
   float* mine = lnb_smem + (size_t)warp * 2 * features;
 #pragma unroll
-  for (int j = 0; j < LNB_MAXJ; ++j) {
+  for (int j = 0; j < J; ++j) {
     const int c = (j * 32 + lane) * 4;
     if (c < features) {
 #pragma unroll
@@ -203,16 +205,6 @@ layer_norm_bwd_kernel(const XT* __restrict__ x, const float* __restrict__ gamma,
     for (int w = 0; w < LNB_WARPS; ++w) s += (Acc)lnb_smem[(size_t)w * 2 * features + c];
     partial[(size_t)blockIdx.x * 2 * features + c] = (float)s;
   }
-}
-
-__global__ void layer_norm_bwd_fold_kernel(const float* __restrict__ partial, float* __restrict__ dgamma,
-                                           float* __restrict__ dbeta, int features, int blocks) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= 2 * features) return;
-  double s = 0.0;
-  for (int b = 0; b < blocks; ++b) s += (double)partial[(size_t)b * 2 * features + c];
-  if (c < features) { if (dgamma) dgamma[c] = (float)s; }
-  else if (dbeta) dbeta[c - features] = (float)s;
 }
 
 // ---- embedding ------------------------------------------------------------------------------
@@ -486,31 +478,53 @@ int layer_norm_backward_impl(hl_ctx* ctx, const void* x, int x_dtype, const floa
   int blocks = std::min(ctx->sm_count * 2, ceil_div(rows, LNB_WARPS));
   const int rows_per_block = ceil_div(rows, blocks);
   blocks = ceil_div(rows, rows_per_block);
-  int rc = ensure_workspace(ctx, sizeof(float) * (size_t)blocks * 2 * features);
-  if (rc != HL_OK) return rc;
-  float* partial = reinterpret_cast<float*>(ctx->workspace);
+  // the partial rows of dgamma and dbeta wait in the caller's batch when it gave one, else they are folded right here
+  FoldBatch own{};
+  if (!defer) {
+    int rc = ensure_workspace(ctx, sizeof(float) * ((size_t)blocks * 2 * features + 64));
+    if (rc != HL_OK) return rc;
+    own.scratch = reinterpret_cast<float*>(ctx->workspace);
+    own.capacity = ctx->workspace_bytes / sizeof(float);
+    defer = &own;
+  }
+  float* partial = fold_batch_reserve(defer, (size_t)blocks * 2 * features);
+  if (!partial) {
+    int rc = fold_batch_flush(ctx, defer);
+    if (rc != HL_OK) return rc;
+    partial = fold_batch_reserve(defer, (size_t)blocks * 2 * features);
+    HL_REQUIRE(partial, "hl_layer_norm_backward: fold scratch is too small");
+  }
   const size_t smem = sizeof(float) * LNB_WARPS * 2 * (size_t)features;
-  if (x_dtype == HL_F32) {
-    auto k = layer_norm_bwd_kernel<float, double>;
-    HL_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<blocks, LNB_WARPS * 32, smem, ctx->stream>>>((const float*)x, gamma, dy, mean, rstd, residual_grad, dx_f32,
-                                                      (__nv_bfloat16*)dx_bf16, partial, rows, features,
-                                                      rows_per_block, 1e-5f);
-  } else {
-    auto k = layer_norm_bwd_kernel<__nv_bfloat16, float>;
-    HL_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<blocks, LNB_WARPS * 32, smem, ctx->stream>>>((const __nv_bfloat16*)x, gamma, dy, mean, rstd, residual_grad,
-                                                      dx_f32, (__nv_bfloat16*)dx_bf16, partial, rows, features,
-                                                      rows_per_block, 1e-5f);
-  }
+#define HL_LN_BWD(XT, ACC, J)                                                                                          \
+  do {                                                                                                                 \
+    auto k = layer_norm_bwd_kernel<XT, ACC, J>;                                                                        \
+    static bool configured = false;                                                                                    \
+    if (!configured) {                                                                                                 \
+      HL_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(float) * LNB_WARPS * 2 * LNB_MAXJ * 128))); \
+      configured = true;                                                                                               \
+    }                                                                                                                  \
+    k<<<blocks, LNB_WARPS * 32, smem, ctx->stream>>>((const XT*)x, gamma, dy, mean, rstd, residual_grad, dx_f32,       \
+                                                     (__nv_bfloat16*)dx_bf16, partial, rows, features, rows_per_block, \
+                                                     1e-5f);                                                           \
+  } while (0)
+#define HL_LN_BWD_J(XT, ACC)                       \
+  do {                                             \
+    if (features <= 128) HL_LN_BWD(XT, ACC, 1);    \
+    else if (features <= 256) HL_LN_BWD(XT, ACC, 2); \
+    else if (features <= 512) HL_LN_BWD(XT, ACC, 4); \
+    else HL_LN_BWD(XT, ACC, 8);                    \
+  } while (0)
+  if (x_dtype == HL_F32) HL_LN_BWD_J(float, double);
+  else HL_LN_BWD_J(__nv_bfloat16, float);
+#undef HL_LN_BWD_J
+#undef HL_LN_BWD
   HL_LAUNCH_CHECK("layer_norm_bwd_kernel");
-  if (dgamma || dbeta) {
-    layer_norm_bwd_fold_kernel<<<ceil_div(2 * features, 256), 256, 0, ctx->stream>>>(partial, dgamma, dbeta, features,
-                                                                                      blocks);
-    HL_LAUNCH_CHECK("layer_norm_bwd_fold_kernel");
-    count_launch(ctx);
-  }
   count_launch(ctx);
+  fold_batch_add(defer, partial, blocks, 2 * features, features, dgamma, dbeta, nullptr);
+  if (defer == &own) {
+    int rc = fold_batch_flush(ctx, defer);
+    if (rc != HL_OK) return rc;
+  }
   if (dx_colsum) return bias_grad_impl(ctx, dx_f32, HL_F32, dx_colsum, rows, features);
   return HL_OK;
 }

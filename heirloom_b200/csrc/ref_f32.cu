@@ -2,158 +2,638 @@
 // attention with materialised probabilities.  These follow the reference's f32 CUDA entries
 // (heirloom-kernels/src/ptx/kernels.ptx:1290-1659 matmul, :3760-4609 attention) in what they
 // compute, but accumulate in double so that their f32 results round from the same f64 values
-// the reference's CPU path produces (src/tensor.rs:577-590).  Not a throughput path.
-#include "common.cuh"
+// the reference's CPU path produces (src/tensor.rs:577-590).
+//
+// Every product runs on the f64 tensor instruction (mma.m8n8k4): operands are widened once, on their way into shared
+// memory, and a warp then reads one f64 per lane and operand fragment for 256 multiply-adds, where plain f64 FMAs read
+// two operands per multiply-add out of a 16 x 16 tile.
+#include <cooperative_groups.h>
+
+#include "kernels.h"
 
 namespace hl {
 namespace {
 
-constexpr int MT = 16;
+namespace cg = cooperative_groups;
 
-__global__ void matmul_f32_strided_kernel(const float* __restrict__ a, hl_matrix_layout la, const float* __restrict__ b,
-                                          hl_matrix_layout lb, float* __restrict__ out, hl_matrix_layout lo,
-                                          int accumulate) {
-  __shared__ double sa[MT][MT + 1];
-  __shared__ double sb[MT][MT + 1];
-  const long long row = blockIdx.y * (long long)MT + threadIdx.y;
-  const long long col = blockIdx.x * (long long)MT + threadIdx.x;
-  const long long K = la.cols;
-  double acc = 0.0;
-  for (long long k0 = 0; k0 < K; k0 += MT) {
-    const long long ka = k0 + threadIdx.x, kb = k0 + threadIdx.y;
-    sa[threadIdx.y][threadIdx.x] =
-        (row < la.rows && ka < K) ? (double)a[la.offset + row * la.row_stride + ka * la.col_stride] : 0.0;
-    sb[threadIdx.y][threadIdx.x] =
-        (kb < K && col < lb.cols) ? (double)b[lb.offset + kb * lb.row_stride + col * lb.col_stride] : 0.0;
-    __syncthreads();
+// D (8x8) += A (8x4, row lane/4, k lane%4) * B (4x8, k lane%4, column lane/4); D: row lane/4, columns 2*(lane%4) + {0,1}
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+
+__device__ __forceinline__ double widen(float x) { return (double)x; }
+__device__ __forceinline__ double widen(__nv_bfloat16 x) { return (double)__bfloat162float(x); }
+__device__ __forceinline__ void narrow(float* p, double v) { *p = (float)v; }
+__device__ __forceinline__ void narrow(__nv_bfloat16* p, double v) { *p = __float2bfloat16_rn((float)v); }  // through f32
+
+// ---- strided matmul --------------------------------------------------------------------------------
+// One CTA of four warps per TM x TN output tile (32 x 32, or 64 x 64 when those fill the chip), k in steps of 32 through
+// two shared buffers, the next step's operands in registers while the current one is multiplied.  Shared rows are padded
+// so that a half warp's fragment (4 rows x 4 k) falls into 16 different 8-byte banks whichever index is contiguous.
+// Small outputs with a long contraction (weight gradients) are shared by the CTAs of a cluster: each takes a part of k,
+// and the parts are added in rank order through distributed shared memory, so the result does not depend on timing.
+// Up to F64_JOBS independent products go into one launch (an input gradient beside its weight gradient).
+// Measured at 1024 x 128 x 128 on its own: 28 -> 5 us; the 75 launches of the tiny decoder's step became 31.
+constexpr int F64_THREADS = 128;
+constexpr int F64_BK = 32;
+constexpr int F64_JOBS = 2;
+
+struct F64Job {
+  F64Gemm g;
+  int cta0;              // first CTA of this product
+  int tiles, tiles_n;    // output tiles, tile columns
+  int split;             // CTAs per tile: 1 or the cluster size
+  int k_tiles_per_rank;
+};
+struct F64Jobs {
+  F64Job job[F64_JOBS];
+  int count;
+  int cluster;
+};
+
+template <int TM, int TN>
+__global__ void __launch_bounds__(F64_THREADS)
+f64_gemm_kernel(const F64Jobs jobs) {
+  constexpr int FM = TM / 16, FN = TN / 16;      // 8 x 8 fragments per warp: four warps, two by two
+  constexpr int LDK = F64_BK + 4;                // row stride of a tile stored [row][k]
+  constexpr int LDM = TM + 4, LDN = TN + 4;      // row stride of a tile stored [k][row]
+  constexpr int A_ELEMS = TM * LDK, B_ELEMS = TN * LDK;
+  static_assert(F64_BK * LDM <= A_ELEMS && F64_BK * LDN <= B_ELEMS, "both layouts share the buffers");
+  constexpr int LDC = TN + 2;
+  static_assert(TM * LDC + TM <= 2 * (A_ELEMS + B_ELEMS), "the output tile reuses the operand buffers");
+  extern __shared__ double f64_smem[];
+  const int which = (jobs.count > 1 && (int)blockIdx.x >= jobs.job[1].cta0) ? 1 : 0;
+  const F64Job& jb = jobs.job[which];
+  const F64Gemm& g = jb.g;
+  const int local = (int)blockIdx.x - jb.cta0;
+  const int tile = jb.split > 1 ? local / jb.split : local;
+  const int rank = jb.split > 1 ? local % jb.split : 0;
+  if (tile >= jb.tiles) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int row0 = (tile / jb.tiles_n) * TM, col0 = (tile % jb.tiles_n) * TN;
+  const bool a_km = g.a_col == 1, b_km = g.b_row == 1;  // contraction index contiguous in memory
+  const int kt_all = (g.k + F64_BK - 1) / F64_BK;
+  const int kt0 = rank * jb.k_tiles_per_rank, kt1 = min(kt_all, kt0 + jb.k_tiles_per_rank);
+  const bool sums = g.row_sum != nullptr && col0 == 0;
+
+  float ra[TM / 4], rb[TN / 4];
+  auto fetch = [&](int kt) {
+    const int k0 = kt * F64_BK;
 #pragma unroll
-    for (int k = 0; k < MT; ++k) acc += sa[threadIdx.y][k] * sb[k][threadIdx.x];
+    for (int i = 0; i < TM / 4; ++i) {
+      const int e = tid + i * F64_THREADS;
+      const int kk = k0 + (a_km ? e % F64_BK : e / TM), r = row0 + (a_km ? e / F64_BK : e % TM);
+      ra[i] = (r < g.m && kk < g.k) ? __ldg(g.a + r * g.a_row + kk * g.a_col) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < TN / 4; ++i) {
+      const int e = tid + i * F64_THREADS;
+      const int kk = k0 + (b_km ? e % F64_BK : e / TN), c = col0 + (b_km ? e / F64_BK : e % TN);
+      rb[i] = (c < g.n && kk < g.k) ? __ldg(g.b + kk * g.b_row + c * g.b_col) : 0.f;
+    }
+  };
+  auto stash = [&](int buf) {
+    double* sa = f64_smem + buf * (A_ELEMS + B_ELEMS);
+    double* sb = sa + A_ELEMS;
+#pragma unroll
+    for (int i = 0; i < TM / 4; ++i) {
+      const int e = tid + i * F64_THREADS;
+      sa[a_km ? (e / F64_BK) * LDK + e % F64_BK : (e / TM) * LDM + e % TM] = (double)ra[i];
+    }
+#pragma unroll
+    for (int i = 0; i < TN / 4; ++i) {
+      const int e = tid + i * F64_THREADS;
+      sb[b_km ? (e / F64_BK) * LDK + e % F64_BK : (e / TN) * LDN + e % TN] = (double)rb[i];
+    }
+  };
+  const int wm = (warp >> 1) * (TM / 2), wn = (warp & 1) * (TN / 2);
+  const int fr = lane >> 2, fk = lane & 3;
+  const int a_r = a_km ? LDK : 1, a_k = a_km ? 1 : LDM;
+  const int b_r = b_km ? LDK : 1, b_k = b_km ? 1 : LDN;
+  double acc[FM][FN][2], rs[FM][2];
+#pragma unroll
+  for (int i = 0; i < FM; ++i) {
+    rs[i][0] = rs[i][1] = 0.0;
+#pragma unroll
+    for (int j = 0; j < FN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  }
+  const bool my_sums = sums && wn == 0;
+  if (kt0 < kt1) {
+    fetch(kt0);
+    stash(0);
+  }
+  __syncthreads();
+  for (int kt = kt0; kt < kt1; ++kt) {
+    const int buf = (kt - kt0) & 1;
+    if (kt + 1 < kt1) fetch(kt + 1);
+    const double* sa = f64_smem + buf * (A_ELEMS + B_ELEMS) + (wm + fr) * a_r + fk * a_k;
+    const double* sb = f64_smem + buf * (A_ELEMS + B_ELEMS) + A_ELEMS + (wn + fr) * b_r + fk * b_k;
+#pragma unroll
+    for (int kk = 0; kk < F64_BK; kk += 4) {
+      double fa[FM], fb[FN];
+#pragma unroll
+      for (int i = 0; i < FM; ++i) fa[i] = sa[i * 8 * a_r + kk * a_k];
+#pragma unroll
+      for (int j = 0; j < FN; ++j) fb[j] = sb[j * 8 * b_r + kk * b_k];
+#pragma unroll
+      for (int i = 0; i < FM; ++i) {
+#pragma unroll
+        for (int j = 0; j < FN; ++j) dmma(acc[i][j], fa[i], fb[j]);
+        if (my_sums) dmma(rs[i], fa[i], 1.0);  // row sums of A: a bias gradient rides on its weight gradient
+      }
+    }
+    if (kt + 1 < kt1) stash(buf ^ 1);
     __syncthreads();
   }
-  if (row < lo.rows && col < lo.cols) {
-    float* dst = out + lo.offset + row * lo.row_stride + col * lo.col_stride;
-    *dst = accumulate ? (float)((double)*dst + acc) : (float)acc;
+  double* sc = f64_smem;
+  double* srs = f64_smem + TM * LDC;
+#pragma unroll
+  for (int i = 0; i < FM; ++i) {
+#pragma unroll
+    for (int j = 0; j < FN; ++j) {
+      double* d = sc + (wm + i * 8 + fr) * LDC + wn + j * 8 + 2 * fk;
+      d[0] = acc[i][j][0];
+      d[1] = acc[i][j][1];
+    }
+    if (my_sums && fk == 0) srs[wm + i * 8 + fr] = rs[i][0];
+  }
+  const int parts = jb.split;
+  cg::cluster_group cluster = cg::this_cluster();
+  if (parts > 1) cluster.sync(); else __syncthreads();
+  for (int e = rank * F64_THREADS + tid; e < TM * TN; e += parts * F64_THREADS) {
+    const int r = e / TN, c = e % TN;
+    const int row = row0 + r, col = col0 + c;
+    if (row >= g.m || col >= g.n) continue;
+    double v = 0.0;
+    if (parts > 1) {
+      for (int p = 0; p < parts; ++p) v += *cluster.map_shared_rank(sc + r * LDC + c, p);
+    } else {
+      v = sc[r * LDC + c];
+    }
+    const long long at = row * g.o_row + col * g.o_col;
+    float y = g.epilogue == F64_ACCUMULATE ? (float)((double)g.out[at] + v) : (float)v;
+    if (g.bias) y = y + __ldg(g.bias + col);
+    if (g.epilogue == F64_GELU) g.aux_out[at] = (float)gelu_fwd<double>((double)y);
+    else if (g.epilogue == F64_RESIDUAL) y = g.aux_in[at] + y;
+    else if (g.epilogue == F64_DGELU) y = (float)((double)y * gelu_grad<double>((double)g.aux_in[at]));
+    g.out[at] = y;
+  }
+  if (sums && rank == 0 && tid < TM && row0 + tid < g.m) {
+    double v = 0.0;
+    if (parts > 1) {
+      for (int p = 0; p < parts; ++p) v += *cluster.map_shared_rank(srs + tid, p);
+    } else {
+      v = srs[tid];
+    }
+    g.row_sum[row0 + tid] = (float)v;
+  }
+  if (parts > 1) cluster.sync();  // no CTA leaves while another still reads its part
+}
+
+template <int TM, int TN>
+int launch_f64_gemm(hl_ctx* ctx, const F64Gemm* problems, int count) {
+  constexpr size_t smem = sizeof(double) * 2 * (TM + TN) * (F64_BK + 4);
+  auto kern = f64_gemm_kernel<TM, TN>;
+  static bool configured = false;
+  if (!configured) {
+    HL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    configured = true;
+  }
+  F64Jobs jobs{};
+  jobs.count = count;
+  // A contraction longer than 256 is shared as long as its tiles leave SMs idle; eight CTAs is the largest portable cluster.
+  int want[F64_JOBS];
+  jobs.cluster = 1;
+  for (int i = 0; i < count; ++i) {
+    F64Job& j = jobs.job[i];
+    j.g = problems[i];
+    j.tiles_n = ceil_div(j.g.n, TN);
+    j.tiles = ceil_div(j.g.m, TM) * j.tiles_n;
+    want[i] = 1;
+    while (want[i] < 8 && ceil_div(j.g.k, F64_BK) > 8 * want[i] && (long long)j.tiles * want[i] < 2 * ctx->sm_count) want[i] *= 2;
+    jobs.cluster = std::max(jobs.cluster, want[i]);
+  }
+  long long ctas = 0;
+  for (int i = 0; i < count; ++i) {
+    F64Job& j = jobs.job[i];
+    j.cta0 = (int)ctas;
+    j.split = want[i] > 1 ? jobs.cluster : 1;
+    j.k_tiles_per_rank = ceil_div(ceil_div(j.g.k, F64_BK), j.split);
+    ctas += j.split > 1 ? (long long)j.tiles * j.split : ceil_div_ll(j.tiles, jobs.cluster) * jobs.cluster;
+  }
+  HL_REQUIRE(ctas <= 0x7fffffffLL, "hl_matmul_f32_strided: too many tiles for one launch");
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3(F64_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)jobs.cluster; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  HL_CUDA(cudaLaunchKernelEx(&cfg, kern, jobs));
+  HL_LAUNCH_CHECK("f64_gemm_kernel");
+  count_launch(ctx);
+  return HL_OK;
+}
+
+// ---- causal attention ------------------------------------------------------------------------------
+// q, k, v, out: rows of [B*T, *] with heads interleaved along the channels (column h*hd + j, as
+// src/tensor.rs:5156-5177) and a row stride each, f32 or bf16 (widened exactly).  probs: [B,H,T,T].
+//
+// One CTA of four warps per 16 query rows of one (batch, head); the rows' scores against every visible key stay in shared
+// memory as f64, so each score is formed once (a lane per key walking the channels formed it three times, from
+// uncoalesced rows).  The first bound is latency: two passes over the keys in tiles of 32.
+// Measured at B16 H4 T64 hd32: forward 76 -> 9 us, backward 66 -> 15 us.
+constexpr int AT_THREADS = 128;
+constexpr int AT_Q = 16;   // query rows (or key rows) per CTA
+constexpr int AT_K = 32;   // keys (or queries) per tile
+constexpr int AT_GROUPS = 4;  // 8-channel groups per warp and pass: 128 channels at a time
+
+__host__ __device__ inline int at_ld(int n) { return (n + 15) / 16 * 16 + 4; }  // 4 mod 16 doubles: conflict-free fragments
+
+// rows [r0, r0 + ROWS) of a head's [T, hd] slice, widened, zero past T and past hd
+template <int ROWS, typename T>
+__device__ __forceinline__ void at_load(double* dst, int ld, const T* src, long long ld_src, int r0, int T_, int hd) {
+  const int width = ld - 4;
+  for (int e = threadIdx.x; e < ROWS * width; e += AT_THREADS) {
+    const int r = e / width, c = e % width;
+    dst[r * ld + c] = (r0 + r < T_ && c < hd) ? widen(src[(long long)(r0 + r) * ld_src + c]) : 0.0;
   }
 }
 
-// q,k,v,out: [B,T,C], heads interleaved along C (index b*T*C + t*C + h*hd + j, as
-// src/tensor.rs:5156-5177).  probs: [B,H,T,T] (only s <= t is written; the rest is zeroed).
-__global__ void attention_f32_fwd_kernel(const float* __restrict__ q, const float* __restrict__ k,
-                                         const float* __restrict__ v, float* __restrict__ out, float* __restrict__ probs,
-                                         int B, int T, int C, int H) {
-  const int hd = C / H;
+// S[16][keys] = scale * X · Yᵀ over the key tiles [0, n_keys): X in sx, tiles of Y through sy
+template <typename T>
+__device__ __forceinline__ void at_scores(double* ss, int ld_s, const double* sx, double* sy, int ld, const T* y,
+                                          long long ld_y, int n_keys, int T_, int hd, double scale) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fr = lane >> 2, fk = lane & 3;
+  for (int key0 = 0; key0 < n_keys; key0 += AT_K) {
+    __syncthreads();
+    at_load<AT_K>(sy, ld, y, ld_y, key0, T_, hd);
+    __syncthreads();
+    double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+    const double* pa = sx + fr * ld + fk;
+    const double* pb = sy + (warp * 8 + fr) * ld + fk;
+    for (int c = 0; c < hd; c += 4) {
+      const double b = pb[c];
+      dmma(acc[0], pa[c], b);
+      dmma(acc[1], pa[8 * ld + c], b);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      double* d = ss + (i * 8 + fr) * ld_s + key0 + warp * 8 + 2 * fk;
+      d[0] = acc[i][0] * scale;
+      d[1] = acc[i][1] * scale;
+    }
+  }
+  __syncthreads();
+}
+
+// out rows = W[16][n_keys] · Y: W in sw (f64), tiles of Y through sy
+template <typename T, typename OT>
+__device__ __forceinline__ void at_weighted(const double* sw, int ld_s, double* sy, int ld, const T* y, long long ld_y,
+                                            OT* out, long long ld_out, int t0, int n_keys, int T_, int hd) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fr = lane >> 2, fk = lane & 3;
+  const int groups = (hd + 7) / 8;
+  for (int g0 = 0; g0 < groups; g0 += 4 * AT_GROUPS) {
+    double acc[AT_GROUPS][2][2];
+#pragma unroll
+    for (int i = 0; i < AT_GROUPS; ++i) acc[i][0][0] = acc[i][0][1] = acc[i][1][0] = acc[i][1][1] = 0.0;
+    for (int key0 = 0; key0 < n_keys; key0 += AT_K) {
+      __syncthreads();
+      at_load<AT_K>(sy, ld, y, ld_y, key0, T_, hd);
+      __syncthreads();
+      const double* pa = sw + fr * ld_s + key0 + fk;
+#pragma unroll
+      for (int kk = 0; kk < AT_K; kk += 4) {
+        const double a0 = pa[kk], a1 = pa[8 * ld_s + kk];
+#pragma unroll
+        for (int i = 0; i < AT_GROUPS; ++i) {
+          const int grp = g0 + i * 4 + warp;
+          if (grp < groups) {
+            const double b = sy[(kk + fk) * ld + grp * 8 + fr];
+            dmma(acc[i][0], a0, b);
+            dmma(acc[i][1], a1, b);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < AT_GROUPS; ++i) {
+      const int c = (g0 + i * 4 + warp) * 8 + 2 * fk;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int t = t0 + h * 8 + fr;
+        if (t < T_) {
+          if (c < hd) narrow(out + (long long)t * ld_out + c, acc[i][h][0]);
+          if (c + 1 < hd) narrow(out + (long long)t * ld_out + c + 1, acc[i][h][1]);
+        }
+      }
+    }
+  }
+}
+
+// softmax of the visible part of each row, rounded to f32: into probs (zero past the diagonal) and back into ss
+__device__ __forceinline__ void at_softmax(double* ss, int ld_s, float* probs, int t0, int n_keys, int T_) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int r = warp; r < AT_Q; r += 4) {
+    const int t = t0 + r;
+    if (t >= T_) break;  // its rows of ss are multiplied but never stored
+    double* row = ss + r * ld_s;
+    double mx = -INFINITY;
+    for (int s = lane; s <= t; s += 32) mx = max(mx, row[s]);
+    mx = warp_max(mx);
+    double sum = 0.0;
+    for (int s = lane; s <= t; s += 32) {
+      const double e = exp(row[s] - mx);
+      row[s] = e;
+      sum += e;
+    }
+    sum = warp_sum(sum);
+    float* pr = probs + (size_t)t * T_;
+    for (int s = lane; s < max(n_keys, T_); s += 32) {
+      const float p = s <= t ? (float)(row[s] / sum) : 0.f;
+      if (s < n_keys) row[s] = (double)p;
+      if (s < T_) pr[s] = p;
+    }
+  }
+  __syncthreads();
+}
+
+template <typename T>
+__global__ void __launch_bounds__(AT_THREADS)
+attention_f64_fwd_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, long long ld_qkv,
+                         T* __restrict__ out, long long ld_out, float* __restrict__ probs, int T_, int H, int hd, unsigned heads) {
+  extern __shared__ double at_smem[];
+  const int ld = at_ld(hd), ld_s = at_ld((T_ + AT_K - 1) / AT_K * AT_K);
+  double *sx = at_smem, *sy = sx + AT_Q * ld, *ss = sy + AT_K * ld;
+  const int bh = (int)(blockIdx.x % heads), h = bh % H, b = bh / H;
+  const int t0 = ((T_ - 1) / AT_Q - (int)(blockIdx.x / heads)) * AT_Q;  // the longest rows first
+  const int n_keys = (min(T_, t0 + AT_Q) + AT_K - 1) / AT_K * AT_K;
+  const long long head = (long long)b * T_ * ld_qkv + (long long)h * hd;
+  at_load<AT_Q>(sx, ld, q + head, ld_qkv, t0, T_, hd);
+  at_scores(ss, ld_s, sx, sy, ld, k + head, ld_qkv, n_keys, T_, hd, 1.0 / sqrt((double)hd));
+  at_softmax(ss, ld_s, probs + (size_t)bh * T_ * T_, t0, n_keys, T_);
+  at_weighted(ss, ld_s, sy, ld, v + head, ld_qkv, out + (long long)b * T_ * ld_out + (long long)h * hd, ld_out, t0, n_keys, T_, hd);
+}
+
+// Per 16 query rows: (the probabilities again, when they were not kept,) dP, dS (to the f32 scratch) and dQ.
+template <typename T, bool RECOMPUTE>
+__global__ void __launch_bounds__(AT_THREADS)
+attention_f64_bwd_rows_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, long long ld_qkv,
+                              float* __restrict__ probs, const T* __restrict__ dout, long long ld_dout,
+                              float* __restrict__ ds, T* __restrict__ dq, long long ld_dqkv, int T_, int H, int hd, unsigned heads) {
+  extern __shared__ double at_smem[];
+  const int ld = at_ld(hd), ld_s = at_ld((T_ + AT_K - 1) / AT_K * AT_K);
+  double *sx = at_smem, *sy = sx + AT_Q * ld, *ss = sy + AT_K * ld;
+  const int bh = (int)(blockIdx.x % heads), h = bh % H, b = bh / H;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int t0 = ((T_ - 1) / AT_Q - (int)(blockIdx.x / heads)) * AT_Q;
+  const int n_keys = (min(T_, t0 + AT_Q) + AT_K - 1) / AT_K * AT_K;
+  const long long head = (long long)b * T_ * ld_qkv + (long long)h * hd;
+  const double scale = 1.0 / sqrt((double)hd);
+  float* pb = probs + (size_t)bh * T_ * T_;
+  float* db = ds + (size_t)bh * T_ * T_;
+  if constexpr (RECOMPUTE) {
+    at_load<AT_Q>(sx, ld, q + head, ld_qkv, t0, T_, hd);
+    at_scores(ss, ld_s, sx, sy, ld, k + head, ld_qkv, n_keys, T_, hd, scale);
+    at_softmax(ss, ld_s, pb, t0, n_keys, T_);  // read back below by the same warps' lanes: row r by warp r % 4
+  }
+  at_load<AT_Q>(sx, ld, dout + (long long)b * T_ * ld_dout + (long long)h * hd, ld_dout, t0, T_, hd);
+  at_scores(ss, ld_s, sx, sy, ld, v + head, ld_qkv, n_keys, T_, hd, 1.0);  // dP
+  for (int r = warp; r < AT_Q; r += 4) {
+    const int t = t0 + r;
+    if (t >= T_) break;
+    double* row = ss + r * ld_s;
+    const float* pr = pb + (size_t)t * T_;
+    float* dr = db + (size_t)t * T_;
+    double dot = 0.0;
+    for (int s = lane; s <= t; s += 32) dot += row[s] * (double)pr[s];
+    dot = warp_sum(dot);
+    for (int s = lane; s < n_keys; s += 32) {  // the column pass reads no further than this row's last tile
+      const float d = s <= t ? (float)((double)pr[s] * (row[s] - dot) * scale) : 0.f;
+      row[s] = (double)d;
+      if (s < T_) dr[s] = d;
+    }
+  }
+  at_weighted(ss, ld_s, sy, ld, k + head, ld_qkv, dq + (long long)b * T_ * ld_dqkv + (long long)h * hd, ld_dqkv, t0, n_keys, T_, hd);
+}
+
+// Per 16 key rows: dK[s] = sum_{t>=s} dS[t,s] Q[t], dV[s] = sum_{t>=s} P[t,s] dO[t]; fixed order.
+template <typename T>
+__global__ void __launch_bounds__(AT_THREADS)
+attention_f64_bwd_cols_kernel(const T* __restrict__ q, long long ld_qkv, const float* __restrict__ probs,
+                              const float* __restrict__ ds, const T* __restrict__ dout, long long ld_dout,
+                              T* __restrict__ dk, T* __restrict__ dv, long long ld_dqkv, int T_, int H, int hd, unsigned heads) {
+  extern __shared__ double at_smem[];
+  constexpr int CH = 4 * AT_GROUPS * 8;  // channels of one pass
+  const int ld = at_ld(min(hd, CH));
+  constexpr int LDW = AT_Q + 4;
+  double *sq = at_smem, *sdo = sq + AT_K * ld, *swd = sdo + AT_K * ld, *swp = swd + AT_K * LDW;
+  const int bh = (int)(blockIdx.x % heads), h = bh % H, b = bh / H;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fr = lane >> 2, fk = lane & 3;
+  const int s0 = (int)(blockIdx.x / heads) * AT_Q;
+  const float* pb = probs + (size_t)bh * T_ * T_;
+  const float* db = ds + (size_t)bh * T_ * T_;
+  const T* qh = q + (long long)b * T_ * ld_qkv + (long long)h * hd;
+  const T* gh = dout + (long long)b * T_ * ld_dout + (long long)h * hd;
+  const int groups = (hd + 7) / 8;
+  for (int g0 = 0; g0 < groups; g0 += 4 * AT_GROUPS) {
+    double ak[AT_GROUPS][2][2], av[AT_GROUPS][2][2];
+#pragma unroll
+    for (int i = 0; i < AT_GROUPS; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) ak[i][j][0] = ak[i][j][1] = av[i][j][0] = av[i][j][1] = 0.0;
+    for (int t0 = s0 / AT_K * AT_K; t0 < T_; t0 += AT_K) {
+      __syncthreads();
+      at_load<AT_K>(sq, ld, qh + g0 * 8, ld_qkv, t0, T_, hd - g0 * 8);
+      at_load<AT_K>(sdo, ld, gh + g0 * 8, ld_dout, t0, T_, hd - g0 * 8);
+      for (int e = threadIdx.x; e < AT_K * AT_Q; e += AT_THREADS) {
+        const int r = e / AT_Q, c = e % AT_Q;
+        const bool in = t0 + r < T_ && s0 + c <= t0 + r;
+        const size_t at = (size_t)(t0 + r) * T_ + s0 + c;
+        swd[r * LDW + c] = in ? (double)db[at] : 0.0;
+        swp[r * LDW + c] = in ? (double)pb[at] : 0.0;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int kk = 0; kk < AT_K; kk += 4) {
+        const double* wd = swd + (kk + fk) * LDW + fr;
+        const double* wp = swp + (kk + fk) * LDW + fr;
+        const double d0 = wd[0], d1 = wd[8], p0 = wp[0], p1 = wp[8];
+#pragma unroll
+        for (int i = 0; i < AT_GROUPS; ++i) {
+          const int grp = g0 + i * 4 + warp;
+          if (grp < groups) {
+            const double bq = sq[(kk + fk) * ld + (grp - g0) * 8 + fr], bo = sdo[(kk + fk) * ld + (grp - g0) * 8 + fr];
+            dmma(ak[i][0], d0, bq);
+            dmma(ak[i][1], d1, bq);
+            dmma(av[i][0], p0, bo);
+            dmma(av[i][1], p1, bo);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < AT_GROUPS; ++i) {
+      const int c = (g0 + i * 4 + warp) * 8 + 2 * fk;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int s = s0 + j * 8 + fr;
+        if (s < T_) {
+          const long long at = ((long long)b * T_ + s) * ld_dqkv + (long long)h * hd + c;
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            if (c + e < hd) {
+              narrow(dk + at + e, ak[i][j][e]);
+              narrow(dv + at + e, av[i][j][e]);
+            }
+        }
+      }
+    }
+  }
+}
+
+// ---- the same for rows or heads whose scores do not fit in shared memory (T above about 1500): a warp per row ----------
+template <typename T>
+__global__ void attention_f64_fwd_rows_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
+                                              long long ld_qkv, T* __restrict__ out, long long ld_out,
+                                              float* __restrict__ probs, int B, int T_, int H, int hd) {
   const int lane = threadIdx.x & 31;
   const long long w = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (w >= (long long)B * H * T) return;
-  const int t = (int)(w % T);
-  const int h = (int)((w / T) % H);
-  const int b = (int)(w / ((long long)T * H));
+  if (w >= (long long)B * H * T_) return;
+  const int t = (int)(w % T_), h = (int)((w / T_) % H), b = (int)(w / ((long long)T_ * H));
   const double scale = 1.0 / sqrt((double)hd);
-  const float* qr = q + ((size_t)b * T + t) * C + (size_t)h * hd;
-  float* pr = probs + (((size_t)b * H + h) * T + t) * (size_t)T;
+  const long long head = (long long)b * T_ * ld_qkv + (long long)h * hd;
+  const T* qr = q + head + (long long)t * ld_qkv;
+  float* pr = probs + (((size_t)b * H + h) * T_ + t) * (size_t)T_;
+  auto score = [&](int s) {
+    const T* kr = k + head + (long long)s * ld_qkv;
+    double dot = 0.0;
+    for (int j = 0; j < hd; ++j) dot += widen(qr[j]) * widen(kr[j]);
+    return dot * scale;
+  };
   double mx = -INFINITY;
-  for (int s = lane; s <= t; s += 32) {
-    const float* kr = k + ((size_t)b * T + s) * C + (size_t)h * hd;
-    double dot = 0.0;
-    for (int j = 0; j < hd; ++j) dot += (double)qr[j] * (double)kr[j];
-    dot *= scale;
-    mx = max(mx, dot);
-  }
+  for (int s = lane; s <= t; s += 32) mx = max(mx, score(s));
   mx = warp_max(mx);
-  __syncwarp();
   double denom = 0.0;
-  for (int s = lane; s <= t; s += 32) {
-    const float* kr = k + ((size_t)b * T + s) * C + (size_t)h * hd;
-    double dot = 0.0;
-    for (int j = 0; j < hd; ++j) dot += (double)qr[j] * (double)kr[j];
-    denom += exp(dot * scale - mx);
-  }
+  for (int s = lane; s <= t; s += 32) denom += exp(score(s) - mx);
   denom = warp_sum(denom);
-  for (int s = lane; s < T; s += 32) {
-    if (s <= t) {
-      const float* kr = k + ((size_t)b * T + s) * C + (size_t)h * hd;
-      double dot = 0.0;
-      for (int j = 0; j < hd; ++j) dot += (double)qr[j] * (double)kr[j];
-      pr[s] = (float)(exp(dot * scale - mx) / denom);
-    } else {
-      pr[s] = 0.f;
-    }
-  }
+  for (int s = lane; s < T_; s += 32) pr[s] = s <= t ? (float)(exp(score(s) - mx) / denom) : 0.f;
   __syncwarp();
-  float* orow = out + ((size_t)b * T + t) * C + (size_t)h * hd;
+  T* orow = out + ((long long)b * T_ + t) * ld_out + (long long)h * hd;
   for (int j = lane; j < hd; j += 32) {
     double acc = 0.0;
-    for (int s = 0; s <= t; ++s) acc += (double)pr[s] * (double)v[((size_t)b * T + s) * C + (size_t)h * hd + j];
-    orow[j] = (float)acc;
+    for (int s = 0; s <= t; ++s) acc += (double)pr[s] * widen(v[head + (long long)s * ld_qkv + j]);
+    narrow(orow + j, acc);
   }
 }
 
-// Per query row: dP, dS (written to ds scratch) and dQ.
-__global__ void attention_f32_bwd_rows_kernel(const float* __restrict__ k, const float* __restrict__ v,
-                                              const float* __restrict__ probs, const float* __restrict__ dout,
-                                              float* __restrict__ ds, float* __restrict__ dq, int B, int T, int C, int H) {
-  const int hd = C / H;
+template <typename T>
+__global__ void attention_f64_bwd_long_rows_kernel(const T* __restrict__ k, const T* __restrict__ v, long long ld_qkv,
+                                                   const float* __restrict__ probs, const T* __restrict__ dout,
+                                                   long long ld_dout, float* __restrict__ ds, T* __restrict__ dq,
+                                                   long long ld_dqkv, int B, int T_, int H, int hd) {
   const int lane = threadIdx.x & 31;
   const long long w = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (w >= (long long)B * H * T) return;
-  const int t = (int)(w % T);
-  const int h = (int)((w / T) % H);
-  const int b = (int)(w / ((long long)T * H));
+  if (w >= (long long)B * H * T_) return;
+  const int t = (int)(w % T_), h = (int)((w / T_) % H), b = (int)(w / ((long long)T_ * H));
   const double scale = 1.0 / sqrt((double)hd);
-  const float* pr = probs + (((size_t)b * H + h) * T + t) * (size_t)T;
-  float* dsr = ds + (((size_t)b * H + h) * T + t) * (size_t)T;
-  const float* gor = dout + ((size_t)b * T + t) * C + (size_t)h * hd;
-  double dot_sum = 0.0;
-  for (int s = lane; s <= t; s += 32) {
-    const float* vr = v + ((size_t)b * T + s) * C + (size_t)h * hd;
+  const long long head = (long long)b * T_ * ld_qkv + (long long)h * hd;
+  const float* pr = probs + (((size_t)b * H + h) * T_ + t) * (size_t)T_;
+  float* dsr = ds + (((size_t)b * H + h) * T_ + t) * (size_t)T_;
+  const T* gor = dout + ((long long)b * T_ + t) * ld_dout + (long long)h * hd;
+  auto dp_of = [&](int s) {
+    const T* vr = v + head + (long long)s * ld_qkv;
     double dp = 0.0;
-    for (int j = 0; j < hd; ++j) dp += (double)gor[j] * (double)vr[j];
-    dot_sum += dp * (double)pr[s];
-  }
+    for (int j = 0; j < hd; ++j) dp += widen(gor[j]) * widen(vr[j]);
+    return dp;
+  };
+  double dot_sum = 0.0;
+  for (int s = lane; s <= t; s += 32) dot_sum += dp_of(s) * (double)pr[s];
   dot_sum = warp_sum(dot_sum);
-  for (int s = lane; s < T; s += 32) {
-    if (s <= t) {
-      const float* vr = v + ((size_t)b * T + s) * C + (size_t)h * hd;
-      double dp = 0.0;
-      for (int j = 0; j < hd; ++j) dp += (double)gor[j] * (double)vr[j];
-      dsr[s] = (float)((double)pr[s] * (dp - dot_sum) * scale);
-    } else {
-      dsr[s] = 0.f;
-    }
-  }
+  for (int s = lane; s < T_; s += 32) dsr[s] = s <= t ? (float)((double)pr[s] * (dp_of(s) - dot_sum) * scale) : 0.f;
   __syncwarp();
-  float* dqr = dq + ((size_t)b * T + t) * C + (size_t)h * hd;
+  T* dqr = dq + ((long long)b * T_ + t) * ld_dqkv + (long long)h * hd;
   for (int j = lane; j < hd; j += 32) {
     double acc = 0.0;
-    for (int s = 0; s <= t; ++s) acc += (double)dsr[s] * (double)k[((size_t)b * T + s) * C + (size_t)h * hd + j];
-    dqr[j] = (float)acc;
+    for (int s = 0; s <= t; ++s) acc += (double)dsr[s] * widen(k[head + (long long)s * ld_qkv + j]);
+    narrow(dqr + j, acc);
   }
 }
 
-// Per key row: dK[s] = sum_{t>=s} dS[t,s] Q[t], dV[s] = sum_{t>=s} P[t,s] dO[t]; fixed order.
-__global__ void attention_f32_bwd_cols_kernel(const float* __restrict__ q, const float* __restrict__ probs,
-                                              const float* __restrict__ ds, const float* __restrict__ dout,
-                                              float* __restrict__ dk, float* __restrict__ dv, int B, int T, int C, int H) {
+constexpr size_t kAttentionSmem = 227 * 1024;
+size_t at_rows_smem(int T, int hd) {
+  return sizeof(double) * ((size_t)(AT_Q + AT_K) * at_ld(hd) + (size_t)AT_Q * at_ld(ceil_div(T, AT_K) * AT_K));
+}
+size_t at_cols_smem(int hd) { return sizeof(double) * (2 * (size_t)AT_K * at_ld(std::min(hd, 32 * AT_GROUPS)) + 2 * (size_t)AT_K * (AT_Q + 4)); }
+
+template <typename K>
+int at_configure(K kern) {
+  HL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttentionSmem));
+  return HL_OK;
+}
+
+template <typename T>
+int attention_forward_t(hl_ctx* ctx, const T* q, const T* k, const T* v, long long ld_qkv, T* out, long long ld_out,
+                        float* probs, int B, int Tn, int C, int H) {
   const int hd = C / H;
-  const int lane = threadIdx.x & 31;
-  const long long w = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (w >= (long long)B * H * T) return;
-  const int s = (int)(w % T);
-  const int h = (int)((w / T) % H);
-  const int b = (int)(w / ((long long)T * H));
-  const size_t base = ((size_t)b * H + h) * T;
-  for (int j = lane; j < hd; j += 32) {
-    double ak = 0.0, av = 0.0;
-    for (int t = s; t < T; ++t) {
-      const size_t pi = (base + t) * (size_t)T + s;
-      const size_t xi = ((size_t)b * T + t) * C + (size_t)h * hd + j;
-      ak += (double)ds[pi] * (double)q[xi];
-      av += (double)probs[pi] * (double)dout[xi];
+  const size_t smem = at_rows_smem(Tn, hd);
+  const long long heads = (long long)B * H;
+  if (smem <= kAttentionSmem) {
+    static bool configured = false;
+    if (!configured) {
+      int rc = at_configure(attention_f64_fwd_kernel<T>);
+      if (rc != HL_OK) return rc;
+      configured = true;
     }
-    const size_t oi = ((size_t)b * T + s) * C + (size_t)h * hd + j;
-    dk[oi] = (float)ak;
-    dv[oi] = (float)av;
+    attention_f64_fwd_kernel<T><<<(unsigned)(ceil_div(Tn, AT_Q) * heads), AT_THREADS, smem, ctx->stream>>>(
+        q, k, v, ld_qkv, out, ld_out, probs, Tn, H, hd, (unsigned)heads);
+    HL_LAUNCH_CHECK("attention_f64_fwd_kernel");
+  } else {
+    attention_f64_fwd_rows_kernel<T><<<(unsigned)ceil_div_ll(heads * Tn, 4), 128, 0, ctx->stream>>>(q, k, v, ld_qkv, out, ld_out,
+                                                                                                    probs, B, Tn, H, hd);
+    HL_LAUNCH_CHECK("attention_f64_fwd_rows_kernel");
   }
+  count_launch(ctx);
+  return HL_OK;
+}
+
+template <typename T, bool RECOMPUTE>
+int attention_backward_t(hl_ctx* ctx, const T* q, const T* k, const T* v, long long ld_qkv, float* probs, const T* dout,
+                         long long ld_dout, T* dq, T* dk, T* dv, long long ld_dqkv, int B, int Tn, int C, int H) {
+  const int hd = C / H;
+  const long long heads = (long long)B * H;
+  int rc = ensure_workspace(ctx, sizeof(float) * (size_t)heads * Tn * Tn);
+  if (rc != HL_OK) return rc;
+  float* ds = reinterpret_cast<float*>(ctx->workspace);
+  const size_t rows = at_rows_smem(Tn, hd), cols = at_cols_smem(hd);
+  static bool configured = false;
+  if (!configured) {
+    if ((rc = at_configure(attention_f64_bwd_rows_kernel<T, RECOMPUTE>)) != HL_OK) return rc;
+    if ((rc = at_configure(attention_f64_bwd_cols_kernel<T>)) != HL_OK) return rc;
+    configured = true;
+  }
+  if (rows <= kAttentionSmem) {
+    attention_f64_bwd_rows_kernel<T, RECOMPUTE><<<(unsigned)(ceil_div(Tn, AT_Q) * heads), AT_THREADS, rows, ctx->stream>>>(
+        q, k, v, ld_qkv, probs, dout, ld_dout, ds, dq, ld_dqkv, Tn, H, hd, (unsigned)heads);
+    HL_LAUNCH_CHECK("attention_f64_bwd_rows_kernel");
+  } else {
+    if (RECOMPUTE) {  // the output goes where dQ will be written
+      if ((rc = attention_forward_t<T>(ctx, q, k, v, ld_qkv, dq, ld_dqkv, probs, B, Tn, C, H)) != HL_OK) return rc;
+    }
+    attention_f64_bwd_long_rows_kernel<T><<<(unsigned)ceil_div_ll(heads * Tn, 4), 128, 0, ctx->stream>>>(
+        k, v, ld_qkv, probs, dout, ld_dout, ds, dq, ld_dqkv, B, Tn, H, hd);
+    HL_LAUNCH_CHECK("attention_f64_bwd_long_rows_kernel");
+  }
+  attention_f64_bwd_cols_kernel<T><<<(unsigned)(ceil_div(Tn, AT_Q) * heads), AT_THREADS, cols, ctx->stream>>>(
+      q, ld_qkv, probs, ds, dout, ld_dout, dk, dv, ld_dqkv, Tn, H, hd, (unsigned)heads);
+  HL_LAUNCH_CHECK("attention_f64_bwd_cols_kernel");
+  count_launch(ctx, 2);
+  return HL_OK;
 }
 
 int check_attention_dims(int B, int T, int C, int H, const char* who) {
@@ -165,6 +645,36 @@ int check_attention_dims(int B, int T, int C, int H, const char* who) {
 }
 
 }  // namespace
+
+int f64_gemm_run(hl_ctx* ctx, const F64Gemm* problems, int count) {
+  HL_REQUIRE(count >= 1 && count <= F64_JOBS, "f64_gemm_run: one or two products");
+  long long tiles = 0;
+  for (int i = 0; i < count; ++i) tiles += (long long)ceil_div(problems[i].m, 64) * ceil_div(problems[i].n, 64);
+  // 64 x 64 tiles read half as much per multiply-add; below two per SM the smaller tile's parallelism is worth more
+  return tiles >= 2LL * ctx->sm_count ? launch_f64_gemm<64, 64>(ctx, problems, count) : launch_f64_gemm<32, 32>(ctx, problems, count);
+}
+
+int attention_f64_forward(hl_ctx* ctx, const void* q, const void* k, const void* v, int dtype, long long ld_qkv, void* out,
+                          long long ld_out, float* probs, int batch, int time, int channels, int n_heads) {
+  if (dtype == HL_BF16)
+    return attention_forward_t<__nv_bfloat16>(ctx, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v,
+                                              ld_qkv, (__nv_bfloat16*)out, ld_out, probs, batch, time, channels, n_heads);
+  return attention_forward_t<float>(ctx, (const float*)q, (const float*)k, (const float*)v, ld_qkv, (float*)out, ld_out, probs,
+                                    batch, time, channels, n_heads);
+}
+
+int attention_f64_backward(hl_ctx* ctx, const void* q, const void* k, const void* v, int dtype, long long ld_qkv, float* probs,
+                           const void* dout, long long ld_dout, void* dq, void* dk, void* dv, long long ld_dqkv, int batch,
+                           int time, int channels, int n_heads) {
+  if (dtype == HL_BF16)
+    return attention_backward_t<__nv_bfloat16, true>(
+        ctx, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, ld_qkv, probs, (const __nv_bfloat16*)dout,
+        ld_dout, (__nv_bfloat16*)dq, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, ld_dqkv, batch, time, channels, n_heads);
+  return attention_backward_t<float, false>(ctx, (const float*)q, (const float*)k, (const float*)v, ld_qkv, probs,
+                                            (const float*)dout, ld_dout, (float*)dq, (float*)dk, (float*)dv, ld_dqkv, batch,
+                                            time, channels, n_heads);
+}
+
 }  // namespace hl
 
 using namespace hl;
@@ -178,12 +688,15 @@ int hl_matmul_f32_strided(hl_ctx* ctx, const float* a, const hl_matrix_layout* l
   HL_REQUIRE(la->cols == lb->rows, "hl_matmul_f32_strided: inner dimensions differ (" + std::to_string(la->cols) +
                                        " vs " + std::to_string(lb->rows) + ")");
   HL_REQUIRE(lo->rows == la->rows && lo->cols == lb->cols, "hl_matmul_f32_strided: output shape mismatch");
-  dim3 grid((unsigned)ceil_div_ll(lo->cols, MT), (unsigned)ceil_div_ll(lo->rows, MT)), block(MT, MT);
-  HL_REQUIRE(grid.y <= 65535, "hl_matmul_f32_strided: too many rows for one launch");
-  matmul_f32_strided_kernel<<<grid, block, 0, ctx->stream>>>(a, *la, b, *lb, out, *lo, accumulate);
-  HL_LAUNCH_CHECK("matmul_f32_strided_kernel");
-  count_launch(ctx);
-  return HL_OK;
+  HL_REQUIRE(la->rows <= 0x7fffffc0LL && la->cols <= 0x7fffffc0LL && lb->cols <= 0x7fffffc0LL,
+             "hl_matmul_f32_strided: too many rows for one launch");
+  F64Gemm g{};
+  g.a = a + la->offset; g.a_row = la->row_stride; g.a_col = la->col_stride;
+  g.b = b + lb->offset; g.b_row = lb->row_stride; g.b_col = lb->col_stride;
+  g.out = out + lo->offset; g.o_row = lo->row_stride; g.o_col = lo->col_stride;
+  g.m = (int)la->rows; g.n = (int)lb->cols; g.k = (int)la->cols;
+  g.epilogue = accumulate ? F64_ACCUMULATE : F64_STORE;
+  return f64_gemm_run(ctx, &g, 1);
 }
 
 int hl_causal_attention_f32_forward(hl_ctx* ctx, const float* q, const float* k, const float* v, float* out,
@@ -191,12 +704,7 @@ int hl_causal_attention_f32_forward(hl_ctx* ctx, const float* q, const float* k,
   HL_REQUIRE(ctx && q && k && v && out && probs, "hl_causal_attention_f32_forward: null argument");
   int rc = check_attention_dims(batch, time, channels, n_heads, "hl_causal_attention_f32_forward");
   if (rc != HL_OK) return rc;
-  const long long warps = (long long)batch * n_heads * time;
-  attention_f32_fwd_kernel<<<(unsigned)ceil_div_ll(warps, 4), 128, 0, ctx->stream>>>(q, k, v, out, probs, batch, time,
-                                                                                    channels, n_heads);
-  HL_LAUNCH_CHECK("attention_f32_fwd_kernel");
-  count_launch(ctx);
-  return HL_OK;
+  return attention_f64_forward(ctx, q, k, v, HL_F32, channels, out, channels, probs, batch, time, channels, n_heads);
 }
 
 int hl_causal_attention_f32_backward(hl_ctx* ctx, const float* q, const float* k, const float* v, const float* probs,
@@ -205,19 +713,8 @@ int hl_causal_attention_f32_backward(hl_ctx* ctx, const float* q, const float* k
   HL_REQUIRE(ctx && q && k && v && probs && grad_out && dq && dk && dv, "hl_causal_attention_f32_backward: null argument");
   int rc = check_attention_dims(batch, time, channels, n_heads, "hl_causal_attention_f32_backward");
   if (rc != HL_OK) return rc;
-  const size_t ds_bytes = sizeof(float) * (size_t)batch * n_heads * time * time;
-  rc = ensure_workspace(ctx, ds_bytes);
-  if (rc != HL_OK) return rc;
-  float* ds = reinterpret_cast<float*>(ctx->workspace);
-  const long long warps = (long long)batch * n_heads * time;
-  attention_f32_bwd_rows_kernel<<<(unsigned)ceil_div_ll(warps, 4), 128, 0, ctx->stream>>>(k, v, probs, grad_out, ds, dq,
-                                                                                         batch, time, channels, n_heads);
-  HL_LAUNCH_CHECK("attention_f32_bwd_rows_kernel");
-  attention_f32_bwd_cols_kernel<<<(unsigned)ceil_div_ll(warps, 4), 128, 0, ctx->stream>>>(q, probs, ds, grad_out, dk, dv,
-                                                                                         batch, time, channels, n_heads);
-  HL_LAUNCH_CHECK("attention_f32_bwd_cols_kernel");
-  count_launch(ctx, 2);
-  return HL_OK;
+  return attention_f64_backward(ctx, q, k, v, HL_F32, channels, const_cast<float*>(probs), grad_out, channels, dq, dk, dv,
+                                channels, batch, time, channels, n_heads);
 }
 
 }  // extern "C"

@@ -79,10 +79,10 @@ struct hl_decoder {
   std::vector<__nv_bfloat16*> x;  // x[l] is the input of block l; x[L] the final residual stream
   std::vector<LayerActs> la;
   __nv_bfloat16 *z = nullptr, *dlogits = nullptr, *dxb = nullptr, *dh = nullptr, *dob = nullptr, *dqkv = nullptr;
-  // head sizes other than 64 and 128 on the bf16 route: attention runs through the f32 kernels on these shared buffers
+  // head sizes other than 64 and 128 on the bf16 route: attention runs through the f32 kernels, whose probabilities share
+  // one buffer
   bool flash_ok = true;
-  float *fa_q = nullptr, *fa_k = nullptr, *fa_v = nullptr, *fa_o = nullptr, *fa_probs = nullptr, *fa_dq = nullptr,
-        *fa_dk = nullptr, *fa_dv = nullptr, *fa_do = nullptr;
+  float* fa_probs = nullptr;
   float *logits = nullptr, *meanf = nullptr, *rstdf = nullptr, *dx0 = nullptr, *dx1 = nullptr, *dtmp = nullptr;
   int64_t *tokens = nullptr, *targets = nullptr;
   FoldBatch fold;  // column reductions of one block's backward, folded by one launch before its buckets are flushed
@@ -148,12 +148,11 @@ struct hl_decoder {
   int64_t *m_sel_all = nullptr, *m_sel_left = nullptr, *m_sel_right = nullptr;  // concatenated selections of all memory blocks
   // f32 route (reference f32 semantics: f32 tensors, f64 accumulation inside every op)
   struct F32Layer {
-    float *a, *q, *k, *v, *probs, *o, *pr, *r, *c, *h, *g, *f;
+    float *a, *qkv, *probs, *o, *r, *c, *h, *g;
   };
   std::vector<float*> xf;  // residual stream per block input, f32
   std::vector<F32Layer> lf;
-  float *zf = nullptr, *tmp_f = nullptr, *tmp2_f = nullptr, *dlogits_f = nullptr, *d_a = nullptr, *d_b = nullptr,
-        *d_c = nullptr, *d_q = nullptr, *d_k = nullptr, *d_v = nullptr, *d_wide = nullptr, *d_wide2 = nullptr;
+  float *zf = nullptr, *dlogits_f = nullptr, *d_a = nullptr, *d_b = nullptr, *d_c = nullptr, *d_qkv = nullptr, *d_wide = nullptr;
 };
 
 namespace hl {
@@ -363,9 +362,6 @@ int plan_activations(hl_decoder* m, bool measure_only, size_t* bytes_out) {
   m->dob = carve<__nv_bfloat16>(cur, N * d);
   m->dqkv = carve<__nv_bfloat16>(cur, N * 3 * d);
   if (!m->flash_ok) {
-    m->fa_q = carve<float>(cur, N * d); m->fa_k = carve<float>(cur, N * d); m->fa_v = carve<float>(cur, N * d);
-    m->fa_o = carve<float>(cur, N * d); m->fa_do = carve<float>(cur, N * d);
-    m->fa_dq = carve<float>(cur, N * d); m->fa_dk = carve<float>(cur, N * d); m->fa_dv = carve<float>(cur, N * d);
     m->fa_probs = carve<float>(cur, (size_t)c.batch * c.n_heads * c.context * c.context);
   }
   plan_memory_buffers(m, cur);
@@ -403,33 +399,28 @@ int plan_activations_f32(hl_decoder* m, bool measure_only, size_t* bytes_out) {
   for (size_t l = 0; l < L; ++l) {
     hl_decoder::F32Layer& a = m->lf[l];
     a.a = carve<float>(cur, N * d);
-    a.q = carve<float>(cur, N * d);
-    a.k = carve<float>(cur, N * d);
-    a.v = carve<float>(cur, N * d);
+    a.qkv = carve<float>(cur, N * 3 * d);
     a.probs = carve<float>(cur, BHTT);
     a.o = carve<float>(cur, N * d);
-    a.pr = carve<float>(cur, N * d);
     a.r = carve<float>(cur, N * d);
     a.c = carve<float>(cur, N * d);
     a.h = carve<float>(cur, N * F);
     a.g = carve<float>(cur, N * F);
-    a.f = carve<float>(cur, N * d);
   }
   m->zf = carve<float>(cur, N * d);
   m->logits = carve<float>(cur, N * V);
   m->dlogits_f = carve<float>(cur, N * V);
-  m->tmp_f = carve<float>(cur, N * std::max(std::max(std::max(d, F), V),
-                                            m->has_memory ? (size_t)std::max(m->mem.key_dim, m->mem.value_dim) : (size_t)1));
-  m->tmp2_f = carve<float>(cur, N * d);
   m->d_a = carve<float>(cur, N * d);
   m->d_b = carve<float>(cur, N * d);
   m->d_c = carve<float>(cur, N * d);
-  m->d_q = carve<float>(cur, N * d);
-  m->d_k = carve<float>(cur, N * d);
-  m->d_v = carve<float>(cur, N * d);
+  m->d_qkv = carve<float>(cur, N * 3 * d);
   m->d_wide = carve<float>(cur, N * F);
-  m->d_wide2 = carve<float>(cur, N * F);
   plan_memory_buffers(m, cur);
+  // partial rows of a full batch of layer norms' parameter gradients (at most two CTAs per SM, two sums each)
+  m->fold.capacity = (size_t)FoldBatch::kMaxJobs * (2 * (size_t)m->ctx->sm_count * 2 * d + 64);
+  m->fold.scratch = carve<float>(cur, m->fold.capacity);
+  m->fold.n = 0;
+  m->fold.used = 0;
   m->tokens = carve<int64_t>(cur, N);
   m->targets = carve<int64_t>(cur, N);
   m->loss_dev = carve<float>(cur, 4);
@@ -505,65 +496,9 @@ int zero_memory_table_grads(hl_decoder* m) {
   return HL_OK;
 }
 
-// ---- attention for head sizes the tcgen05 kernels are not built for (they take head_dim 64 and 128) -------------
-// The bf16 q, k, v are widened to f32 (exact), the f32 attention kernels run on them and their results are rounded to
-// bf16 where the flash route stores bf16 (attention output, dQ/dK/dV).  Probabilities are not kept per layer: the
-// backward pass runs the forward kernel again into the shared probability buffer.
-__global__ void rows_bf16_to_f32_kernel(const __nv_bfloat16* __restrict__ src, long long ld_src, float* __restrict__ dst,
-                                        long long rows, int cols) {
-  const long long n = rows * cols;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    dst[i] = __bfloat162float(src[(i / cols) * ld_src + (i % cols)]);
-}
-__global__ void rows_f32_to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long ld_dst,
-                                        long long rows, int cols) {
-  const long long n = rows * cols;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    dst[(i / cols) * ld_dst + (i % cols)] = __float2bfloat16_rn(src[i]);
-}
-
-int widen_rows(hl_ctx* ctx, const __nv_bfloat16* src, long long ld_src, float* dst, long long rows, int cols) {
-  const long long want = ceil_div_ll(rows * cols, 256);
-  rows_bf16_to_f32_kernel<<<(unsigned)std::min<long long>(want, (long long)ctx->sm_count * 16), 256, 0, ctx->stream>>>(
-      src, ld_src, dst, rows, cols);
-  HL_LAUNCH_CHECK("rows_bf16_to_f32_kernel");
-  count_launch(ctx);
-  return HL_OK;
-}
-int narrow_rows(hl_ctx* ctx, const float* src, __nv_bfloat16* dst, long long ld_dst, long long rows, int cols) {
-  const long long want = ceil_div_ll(rows * cols, 256);
-  rows_f32_to_bf16_kernel<<<(unsigned)std::min<long long>(want, (long long)ctx->sm_count * 16), 256, 0, ctx->stream>>>(
-      src, dst, ld_dst, rows, cols);
-  HL_LAUNCH_CHECK("rows_f32_to_bf16_kernel");
-  count_launch(ctx);
-  return HL_OK;
-}
-
-int attention_forward_wide(hl_decoder* m, const __nv_bfloat16* qkv, __nv_bfloat16* out) {
-  hl_ctx* ctx = m->ctx;
-  const hl_decoder_config& c = m->cfg;
-  const int N = m->N, d = c.d_model;
-  HL_TRY(widen_rows(ctx, qkv, 3 * d, m->fa_q, N, d));
-  HL_TRY(widen_rows(ctx, qkv + d, 3 * d, m->fa_k, N, d));
-  HL_TRY(widen_rows(ctx, qkv + 2 * d, 3 * d, m->fa_v, N, d));
-  HL_TRY(hl_causal_attention_f32_forward(ctx, m->fa_q, m->fa_k, m->fa_v, m->fa_o, m->fa_probs, c.batch, c.context, d, c.n_heads));
-  if (out) HL_TRY(narrow_rows(ctx, m->fa_o, out, d, N, d));
-  return HL_OK;
-}
-
-int attention_backward_wide(hl_decoder* m, const __nv_bfloat16* qkv, const __nv_bfloat16* dout, __nv_bfloat16* dqkv) {
-  hl_ctx* ctx = m->ctx;
-  const hl_decoder_config& c = m->cfg;
-  const int N = m->N, d = c.d_model;
-  HL_TRY(attention_forward_wide(m, qkv, nullptr));  // q, k, v and the probabilities again
-  HL_TRY(widen_rows(ctx, dout, d, m->fa_do, N, d));
-  HL_TRY(hl_causal_attention_f32_backward(ctx, m->fa_q, m->fa_k, m->fa_v, m->fa_probs, m->fa_do, m->fa_dq, m->fa_dk, m->fa_dv,
-                                          c.batch, c.context, d, c.n_heads));
-  HL_TRY(narrow_rows(ctx, m->fa_dq, dqkv, 3 * d, N, d));
-  HL_TRY(narrow_rows(ctx, m->fa_dk, dqkv + d, 3 * d, N, d));
-  HL_TRY(narrow_rows(ctx, m->fa_dv, dqkv + 2 * d, 3 * d, N, d));
-  return HL_OK;
-}
+// Attention for head sizes the tcgen05 kernels are not built for (they take head_dim 64 and 128): the f32 kernels read the
+// bf16 q, k, v (widened exactly) and round to bf16 where the flash route stores bf16.  Probabilities are not kept per
+// layer, the backward forms them again.
 
 int forward(hl_decoder* m) {
   hl_ctx* ctx = m->ctx;
@@ -580,7 +515,7 @@ int forward(hl_decoder* m) {
     HL_TRY(layer_norm_forward_impl(ctx, m->x[l], HL_BF16, P + o.ln1g, P + o.ln1b, a.a, HL_BF16, a.mean1, a.rstd1, N, d, 1e-5f));
     HL_TRY(g.run(N, 3 * d, d, a.a, d, HL_K_MAJOR, W + o.wqkv, d, HL_K_MAJOR, a.qkv, 3 * d, HL_BF16, HL_EPI_BIAS, P + o.bqkv));
     if (m->flash_ok) HL_TRY(flash_attention_forward_impl(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, 3 * d, a.o, d, a.lse, B, T, H, d / H));
-    else HL_TRY(attention_forward_wide(m, a.qkv, a.o));
+    else HL_TRY(attention_f64_forward(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, HL_BF16, 3 * d, a.o, d, m->fa_probs, B, T, d, H));
     HL_TRY(g.run(N, d, d, a.o, d, HL_K_MAJOR, W + o.wo, d, HL_K_MAJOR, a.r, d, HL_BF16, HL_EPI_BIAS_RESIDUAL, P + o.bo,
                  m->x[l], d));
     HL_TRY(layer_norm_forward_impl(ctx, a.r, HL_BF16, P + o.ln2g, P + o.ln2b, a.c, HL_BF16, a.mean2, a.rstd2, N, d, 1e-5f));
@@ -879,7 +814,8 @@ int backward(hl_decoder* m) {
                                            m->dqkv + d, m->dqkv + 2 * d, 3 * d, B, T, H, d / H, ctx->workspace,
                                            ctx->workspace_bytes));
     } else {
-      HL_TRY(attention_backward_wide(m, a.qkv, m->dob, m->dqkv));
+      HL_TRY(attention_f64_backward(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, HL_BF16, 3 * d, m->fa_probs, m->dob, d, m->dqkv,
+                                    m->dqkv + d, m->dqkv + 2 * d, 3 * d, B, T, d, H));
     }
     HL_TRY(g.run(3 * d, d, N, m->dqkv, 3 * d, HL_MN_MAJOR, a.a, d, HL_MN_MAJOR, G + o.wqkv, d, HL_F32));
     HL_TRY(bias_grad_impl(ctx, m->dqkv, HL_BF16, G + o.bqkv, N, 3 * d, fb));
@@ -915,24 +851,36 @@ int backward(hl_decoder* m) {
 // Op by op what the reference's f32 path does (MemoryTransformerLm::forward / loss,
 // src/memory_transformer.rs:2069-2081, :1604-1610; Linear = matmul(weight.transpose()) then
 // add(bias), src/nn.rs:454-475), every op rounding its f32 result from an f64 accumulation.
-hl_matrix_layout dense(long long rows, long long cols) { return hl_matrix_layout{rows, cols, cols, 1, 0}; }
-hl_matrix_layout transposed(long long rows, long long cols) { return hl_matrix_layout{cols, rows, 1, cols, 0}; }  // view of [rows, cols] storage
-
-int linear_f32(hl_decoder* m, const float* x, const float* w, const float* b, float* y, int rows, int in, int out) {
-  // y = x · Wᵀ (rounded), then + b (rounded)
-  const hl_matrix_layout lx = dense(rows, in), lw = transposed(out, in), ly = dense(rows, out);
-  HL_TRY(hl_matmul_f32_strided(m->ctx, x, &lx, w, &lw, m->tmp_f, &ly, 0));
-  return hl_bias_add_f32(m->ctx, m->tmp_f, b, y, rows, out);
+// x · Wᵀ + b; the epilogue may add a residual (aux_in) or leave gelu of the result in aux_out
+F64Gemm linear_f32(const float* x, const float* w, const float* b, float* y, int rows, int in, int out, int epilogue = F64_STORE,
+                   const float* aux_in = nullptr, float* aux_out = nullptr) {
+  F64Gemm g{};
+  g.a = x; g.a_row = in; g.a_col = 1;
+  g.b = w; g.b_row = 1; g.b_col = in;
+  g.out = y; g.o_row = out; g.o_col = 1;
+  g.m = rows; g.n = out; g.k = in;
+  g.bias = b; g.epilogue = epilogue; g.aux_in = aux_in; g.aux_out = aux_out;
+  return g;
 }
 
-int linear_backward_f32(hl_decoder* m, const float* x, const float* w, const float* dy, float* dx, int accumulate_dx,
-                        float* dw, float* db, int rows, int in, int out) {
-  const hl_matrix_layout ldy = dense(rows, out), lw = dense(out, in), ldx = dense(rows, in);
-  if (dx) HL_TRY(hl_matmul_f32_strided(m->ctx, dy, &ldy, w, &lw, dx, &ldx, accumulate_dx));
-  const hl_matrix_layout ldyt = transposed(rows, out), lx = dense(rows, in), ldw = dense(out, in);
-  HL_TRY(hl_matmul_f32_strided(m->ctx, dy, &ldyt, x, &lx, dw, &ldw, 0));
-  return bias_grad_impl(m->ctx, dy, HL_F32, db, rows, out);
+// dx = dy · W (times gelu'(aux_in), or added to what is there), dw = dyᵀ · x and db, in one launch
+int linear_backward_f32(hl_decoder* m, const float* x, const float* w, const float* dy, float* dx, float* dw, float* db, int rows,
+                        int in, int out, int epilogue = F64_STORE, const float* aux_in = nullptr) {
+  F64Gemm g[2] = {};
+  g[0].a = dy; g[0].a_row = out; g[0].a_col = 1;
+  g[0].b = w; g[0].b_row = in; g[0].b_col = 1;
+  g[0].out = dx; g[0].o_row = in; g[0].o_col = 1;
+  g[0].m = rows; g[0].n = in; g[0].k = out;
+  g[0].epilogue = epilogue; g[0].aux_in = aux_in;
+  g[1].a = dy; g[1].a_row = 1; g[1].a_col = out;
+  g[1].b = x; g[1].b_row = in; g[1].b_col = 1;
+  g[1].out = dw; g[1].o_row = in; g[1].o_col = 1;
+  g[1].m = out; g[1].n = in; g[1].k = rows;
+  g[1].row_sum = db;
+  return f64_gemm_run(m->ctx, g, 2);
 }
+
+int forward_f32_gemm(hl_decoder* m, const F64Gemm& g) { return f64_gemm_run(m->ctx, &g, 1); }
 
 int forward_f32(hl_decoder* m) {
   hl_ctx* ctx = m->ctx;
@@ -944,32 +892,26 @@ int forward_f32(hl_decoder* m) {
     const LayerOffsets& o = m->lo[l];
     hl_decoder::F32Layer& a = m->lf[l];
     HL_TRY(layer_norm_forward_impl(ctx, m->xf[l], HL_F32, P + o.ln1g, P + o.ln1b, a.a, HL_F32, nullptr, nullptr, N, d, 1e-5f));
-    HL_TRY(linear_f32(m, a.a, P + o.wqkv, P + o.bqkv, a.q, N, d, d));
-    HL_TRY(linear_f32(m, a.a, P + o.wqkv + (size_t)d * d, P + o.bqkv + d, a.k, N, d, d));
-    HL_TRY(linear_f32(m, a.a, P + o.wqkv + 2 * (size_t)d * d, P + o.bqkv + 2 * d, a.v, N, d, d));
-    HL_TRY(hl_causal_attention_f32_forward(ctx, a.q, a.k, a.v, a.o, a.probs, B, T, d, H));
-    HL_TRY(linear_f32(m, a.o, P + o.wo, P + o.bo, a.pr, N, d, d));
-    HL_TRY(hl_binary_f32(ctx, HL_ADD, m->xf[l], a.pr, a.r, (size_t)N * d));
+    HL_TRY(forward_f32_gemm(m, linear_f32(a.a, P + o.wqkv, P + o.bqkv, a.qkv, N, d, 3 * d)));
+    HL_TRY(attention_f64_forward(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, HL_F32, 3 * d, a.o, d, a.probs, B, T, d, H));
+    HL_TRY(forward_f32_gemm(m, linear_f32(a.o, P + o.wo, P + o.bo, a.r, N, d, d, F64_RESIDUAL, m->xf[l])));
     HL_TRY(layer_norm_forward_impl(ctx, a.r, HL_F32, P + o.ln2g, P + o.ln2b, a.c, HL_F32, nullptr, nullptr, N, d, 1e-5f));
     if (o.is_memory) {
       MemoryActs& ma = m->ma[l];
       const int kd = m->mem.key_dim, vd = m->mem.value_dim;
-      HL_TRY(linear_f32(m, a.c, P + o.wq_m, P + o.bq_m, ma.query, N, d, kd));
+      HL_TRY(forward_f32_gemm(m, linear_f32(a.c, P + o.wq_m, P + o.bq_m, ma.query, N, d, kd)));
       HL_TRY(memory_core_forward(m, l));
-      HL_TRY(linear_f32(m, a.c, P + o.wg_m, P + o.bg_m, ma.gpre, N, d, vd));
-      HL_TRY(hl_gelu(ctx, ma.gpre, ma.gate, HL_F32, (size_t)N * vd));
+      HL_TRY(forward_f32_gemm(m, linear_f32(a.c, P + o.wg_m, P + o.bg_m, ma.gpre, N, d, vd, F64_GELU, nullptr, ma.gate)));
       HL_TRY(hl_binary_f32(ctx, HL_MUL, ma.weighted, ma.gate, ma.mv, (size_t)N * vd));
-      HL_TRY(linear_f32(m, ma.mv, P + o.wout_m, P + o.bout_m, a.f, N, vd, d));
+      HL_TRY(forward_f32_gemm(m, linear_f32(ma.mv, P + o.wout_m, P + o.bout_m, m->xf[l + 1], N, vd, d, F64_RESIDUAL, a.r)));
     } else {
-    HL_TRY(linear_f32(m, a.c, P + o.w1, P + o.b1, a.h, N, d, F));
-    HL_TRY(hl_gelu(ctx, a.h, a.g, HL_F32, (size_t)N * F));
-    HL_TRY(linear_f32(m, a.g, P + o.w2, P + o.b2, a.f, N, F, d));
+      HL_TRY(forward_f32_gemm(m, linear_f32(a.c, P + o.w1, P + o.b1, a.h, N, d, F, F64_GELU, nullptr, a.g)));
+      HL_TRY(forward_f32_gemm(m, linear_f32(a.g, P + o.w2, P + o.b2, m->xf[l + 1], N, F, d, F64_RESIDUAL, a.r)));
     }
-    HL_TRY(hl_binary_f32(ctx, HL_ADD, a.r, a.f, m->xf[l + 1], (size_t)N * d));
   }
   HL_TRY(layer_norm_forward_impl(ctx, m->xf[c.n_layers], HL_F32, P + m->off_lnf_g, P + m->off_lnf_b, m->zf, HL_F32, nullptr,
                                  nullptr, N, d, 1e-5f));
-  return linear_f32(m, m->zf, P + m->off_head_w, P + m->off_head_b, m->logits, N, d, V);
+  return forward_f32_gemm(m, linear_f32(m->zf, P + m->off_head_w, P + m->off_head_b, m->logits, N, d, V));
 }
 
 int backward_f32(hl_decoder* m) {
@@ -983,15 +925,23 @@ int backward_f32(hl_decoder* m) {
     HL_CUDA(cudaStreamWaitEvent(m->ctx->stream, m->comm_done, 0));
     m->comm_pending = false;
   }
+  FoldBatch* fb = &m->fold;
+  fb->n = 0;
+  fb->used = 0;
+  // Everything up to arena element `done` has been written, the layer norms' parameter gradients apart, which are folded
+  // by one launch per full batch unless a bucket of the gradient exchange is waiting for them.
+  auto finished = [&](size_t done) -> int {
+    if (nccl_active(ctx) || done == m->arena) HL_TRY(fold_batch_flush(ctx, fb));
+    return flush_buckets(m, done);
+  };
   HL_TRY(cross_entropy_impl(ctx, m->logits, V, m->targets, N, V, 1.0f, m->loss_dev, nullptr, m->dlogits_f, HL_F32, V));
   HL_TRY(zero_memory_table_grads(m));
   float* dx = m->d_a;       // gradient of the residual stream
   float* dx_next = m->d_b;
-  HL_TRY(linear_backward_f32(m, m->zf, P + m->off_head_w, m->dlogits_f, m->d_c, 0, G + m->off_head_w, G + m->off_head_b, N,
-                             d, V));
+  HL_TRY(linear_backward_f32(m, m->zf, P + m->off_head_w, m->dlogits_f, m->d_c, G + m->off_head_w, G + m->off_head_b, N, d, V));
   HL_TRY(layer_norm_backward_impl(ctx, m->xf[c.n_layers], HL_F32, P + m->off_lnf_g, m->d_c, nullptr, nullptr, nullptr, dx,
-                                  nullptr, G + m->off_lnf_g, G + m->off_lnf_b, nullptr, N, d));
-  HL_TRY(flush_buckets(m, m->off_lnf_b + d));
+                                  nullptr, G + m->off_lnf_g, G + m->off_lnf_b, nullptr, N, d, fb));
+  HL_TRY(finished(m->off_lnf_b + d));
   for (int l = c.n_layers - 1; l >= 0; --l) {
     const LayerOffsets& o = m->lo[l];
     hl_decoder::F32Layer& a = m->lf[l];
@@ -999,40 +949,35 @@ int backward_f32(hl_decoder* m) {
       MemoryActs& ma = m->ma[l];
       const int kd = m->mem.key_dim, vd = m->mem.value_dim;
       const size_t nv = (size_t)N * vd;
-      HL_TRY(linear_backward_f32(m, ma.mv, P + o.wout_m, dx, m->m_dmv, 0, G + o.wout_m, G + o.bout_m, N, vd, d));
+      HL_TRY(linear_backward_f32(m, ma.mv, P + o.wout_m, dx, m->m_dmv, G + o.wout_m, G + o.bout_m, N, vd, d));
       HL_TRY(hl_binary_f32(ctx, HL_MUL, m->m_dmv, ma.gate, m->m_dweighted, nv));
       HL_TRY(hl_binary_f32(ctx, HL_MUL, m->m_dmv, ma.weighted, m->m_dgate, nv));
       HL_TRY(hl_gelu_backward(ctx, ma.gpre, m->m_dgate, m->m_dgpre, HL_F32, nv));
-      HL_TRY(linear_backward_f32(m, a.c, P + o.wg_m, m->m_dgpre, m->d_c, 0, G + o.wg_m, G + o.bg_m, N, d, vd));
+      HL_TRY(linear_backward_f32(m, a.c, P + o.wg_m, m->m_dgpre, m->d_c, G + o.wg_m, G + o.bg_m, N, d, vd));
       HL_TRY(memory_core_backward(m, l, m->m_dweighted));
-      // the query path's input gradient is added to the gate path's (rounded sum of two rounded terms)
-      HL_TRY(linear_backward_f32(m, a.c, P + o.wq_m, m->m_dq, m->m_dc2, 0, G + o.wq_m, G + o.bq_m, N, d, kd));
-      HL_TRY(hl_binary_f32(ctx, HL_ADD, m->d_c, m->m_dc2, m->d_c, (size_t)N * d));
+      // the query path's input gradient is added to the gate path's
+      HL_TRY(linear_backward_f32(m, a.c, P + o.wq_m, m->m_dq, m->d_c, G + o.wq_m, G + o.bq_m, N, d, kd, F64_ACCUMULATE));
     } else {
-    // y = r + fc2(gelu(fc1(ln2 r)))
-    HL_TRY(linear_backward_f32(m, a.g, P + o.w2, dx, m->d_wide, 0, G + o.w2, G + o.b2, N, F, d));
-    HL_TRY(hl_gelu_backward(ctx, a.h, m->d_wide, m->d_wide2, HL_F32, (size_t)N * F));
-    HL_TRY(linear_backward_f32(m, a.c, P + o.w1, m->d_wide2, m->d_c, 0, G + o.w1, G + o.b1, N, d, F));
+      // y = r + fc2(gelu(fc1(ln2 r)))
+      HL_TRY(linear_backward_f32(m, a.g, P + o.w2, dx, m->d_wide, G + o.w2, G + o.b2, N, F, d, F64_DGELU, a.h));
+      HL_TRY(linear_backward_f32(m, a.c, P + o.w1, m->d_wide, m->d_c, G + o.w1, G + o.b1, N, d, F));
     }
     HL_TRY(layer_norm_backward_impl(ctx, a.r, HL_F32, P + o.ln2g, m->d_c, nullptr, nullptr, dx, dx_next, nullptr, G + o.ln2g,
-                                    G + o.ln2b, nullptr, N, d));
+                                    G + o.ln2b, nullptr, N, d, fb));
     std::swap(dx, dx_next);  // dL/dr
     // r = x + out_proj(attention(q, k, v))
-    HL_TRY(linear_backward_f32(m, a.o, P + o.wo, dx, m->d_c, 0, G + o.wo, G + o.bo, N, d, d));
-    HL_TRY(hl_causal_attention_f32_backward(ctx, a.q, a.k, a.v, a.probs, m->d_c, m->d_q, m->d_k, m->d_v, B, T, d, H));
-    HL_TRY(linear_backward_f32(m, a.a, P + o.wqkv, m->d_q, m->tmp2_f, 0, G + o.wqkv, G + o.bqkv, N, d, d));
-    HL_TRY(linear_backward_f32(m, a.a, P + o.wqkv + (size_t)d * d, m->d_k, m->tmp2_f, 1, G + o.wqkv + (size_t)d * d,
-                               G + o.bqkv + d, N, d, d));
-    HL_TRY(linear_backward_f32(m, a.a, P + o.wqkv + 2 * (size_t)d * d, m->d_v, m->tmp2_f, 1,
-                               G + o.wqkv + 2 * (size_t)d * d, G + o.bqkv + 2 * d, N, d, d));
-    HL_TRY(layer_norm_backward_impl(ctx, m->xf[l], HL_F32, P + o.ln1g, m->tmp2_f, nullptr, nullptr, dx, dx_next, nullptr,
-                                    G + o.ln1g, G + o.ln1b, nullptr, N, d));
+    HL_TRY(linear_backward_f32(m, a.o, P + o.wo, dx, m->d_c, G + o.wo, G + o.bo, N, d, d));
+    HL_TRY(attention_f64_backward(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, HL_F32, 3 * d, a.probs, m->d_c, d, m->d_qkv,
+                                  m->d_qkv + d, m->d_qkv + 2 * d, 3 * d, B, T, d, H));
+    HL_TRY(linear_backward_f32(m, a.a, P + o.wqkv, m->d_qkv, m->d_c, G + o.wqkv, G + o.bqkv, N, d, 3 * d));
+    HL_TRY(layer_norm_backward_impl(ctx, m->xf[l], HL_F32, P + o.ln1g, m->d_c, nullptr, nullptr, dx, dx_next, nullptr,
+                                    G + o.ln1g, G + o.ln1b, nullptr, N, d, fb));
     std::swap(dx, dx_next);
-    HL_TRY(flush_buckets(m, o.ln1b + d));
+    HL_TRY(finished(o.ln1b + d));
   }
   HL_CUDA(cudaMemsetAsync(G + m->off_pos, 0, sizeof(float) * (m->arena - m->off_pos), ctx->stream));
   HL_TRY(hl_embedding_backward(ctx, dx, m->tokens, G + m->off_tok, V, G + m->off_pos, T, N, d));
-  HL_TRY(flush_buckets(m, m->arena));
+  HL_TRY(finished(m->arena));
   if (nccl_active(ctx)) {
     if (m->has_memory || m->sparse_tok_exchange) {
       // the row exchanges read gradients the compute stream is still producing

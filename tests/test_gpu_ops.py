@@ -281,6 +281,42 @@ def test_matmul_f32_strided_views(golden):
     assert np.array_equal(host(cuda.matmul_f32_strided(c, dev(x).t(), dev(g))), ho.f32_round(gb))
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (33, 31, 257), (64, 64, 32), (100, 24, 1030), (1100, 1090, 40)])
+def test_matmul_f32_strided_tiles_and_shared_contractions(m, n, k):
+    """Tile edges, contractions shared by a cluster (k > 256) and the 64 x 64 tile, with either index contiguous: the f64
+    sum of a product rounds to the same f32 as NumPy's (an order-dependent last bit of the f64 sum moves the f32 rounding
+    with probability 2^-28 an element)."""
+    from heirloom_b200 import cuda
+    c = ctx()
+    rng = np.random.default_rng(m + n + k)
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+    want = ho.matmul(a, b)
+    for av in (dev(a), dev(a.T.copy()).t()):
+        for bv in (dev(b), dev(b.T.copy()).t()):
+            assert np.array_equal(host(cuda.matmul_f32_strided(c, av, bv)), want)
+    base = rng.standard_normal((m, n)).astype(np.float32)
+    out = dev(base)
+    cuda.matmul_f32_strided(c, dev(a), dev(b), out=out, accumulate=True)
+    assert_close("accumulate", host(out), base.astype(np.float64) + a.astype(np.float64) @ b.astype(np.float64), rtol=2 ** -23, atol=1e-30)
+
+
+@pytest.mark.parametrize("B,T,H,hd", [(1, 1, 1, 16), (2, 16, 3, 24), (1, 33, 2, 8), (1, 130, 1, 200), (1, 1700, 1, 16)])
+def test_attention_f32_tiles(B, T, H, hd):
+    """Edges of the 16-row and 32-key tiles, head sizes that are no multiple of a fragment or longer than a pass, and a
+    sequence whose scores do not fit in shared memory."""
+    from heirloom_b200 import cuda
+    c = ctx()
+    rng = np.random.default_rng(T + hd)
+    q, k, v, go = (rng.standard_normal((B, T, H * hd)).astype(np.float32) for _ in range(4))
+    o, p = cuda.causal_attention_f32_forward(c, dev(q), dev(k), dev(v), H)
+    oo, po = ho.causal_attention(q, k, v, H, return_probs=True)
+    assert_close("out", host(o), oo, atol=1e-6, rtol=1e-5)
+    assert_close("probs", host(p), ho.f32_round(po), atol=1e-7, rtol=1e-5)
+    grads = cuda.causal_attention_f32_backward(c, dev(q), dev(k), dev(v), p, dev(go), H)
+    for name, got, want in zip("qkv", grads, ho.causal_attention_backward(q, k, v, H, go, probs=po)):
+        assert_close("d" + name, host(got), want, atol=1e-5, rtol=1e-4)
+
+
 def test_attention_f32_golden_and_random(golden):
     from heirloom_b200 import cuda
     c = ctx()
