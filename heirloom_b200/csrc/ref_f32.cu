@@ -29,14 +29,17 @@ __device__ __forceinline__ void narrow(float* p, double v) { *p = (float)v; }
 __device__ __forceinline__ void narrow(__nv_bfloat16* p, double v) { *p = __float2bfloat16_rn((float)v); }  // through f32
 
 // ---- strided matmul --------------------------------------------------------------------------------
-// One CTA of four warps per TM x TN output tile (32 x 32, or 64 x 64 when those fill the chip), k in steps of 32 through
-// two shared buffers, the next step's operands in registers while the current one is multiplied.  Shared rows are padded
-// so that a half warp's fragment (4 rows x 4 k) falls into 16 different 8-byte banks whichever index is contiguous.
+// One CTA of eight warps per TM x TN output tile (32 x 32, or 64 x 64 when those fill the chip), k in steps of 32.  Steps are
+// copied ahead as f32 by cp.async (four bytes a copy: any stride, zero fill at the edges), each thread widens the elements
+// it copied itself into one of two f64 buffers, and one barrier a step separates widening from multiplying.  Shared rows
+// are padded so that a half warp's fragment (4 rows x 4 k) falls into 16 different 8-byte banks whichever index is
+// contiguous.  At these sizes a step is bound by its instruction count (a generic addressing version issued 976 a warp
+// and step for 32 products), so the four combinations of contiguous indices are compiled apart, with one pointer per
+// operand and immediate offsets, and the small tile's warps come in two groups that take half of every step's k each.
 // Small outputs with a long contraction (weight gradients) are shared by the CTAs of a cluster: each takes a part of k,
 // and the parts are added in rank order through distributed shared memory, so the result does not depend on timing.
-// Up to F64_JOBS independent products go into one launch (an input gradient beside its weight gradient).
-// Measured at 1024 x 128 x 128 on its own: 28 -> 5 us; the 75 launches of the tiny decoder's step became 31.
-constexpr int F64_THREADS = 128;
+// Two independent products may share a launch (an input gradient beside its weight gradient).
+constexpr int F64_THREADS = 256;
 constexpr int F64_BK = 32;
 constexpr int F64_JOBS = 2;
 
@@ -53,16 +56,149 @@ struct F64Jobs {
   int cluster;
 };
 
+__device__ __forceinline__ void copy_async4(float* dst_shared, const float* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_shared)), "l"(src),
+               "r"(in ? 4 : 0)
+               : "memory");
+}
+constexpr int f64_depth(int tm) { return tm == 32 ? 4 : 2; }
+
+// One operand of a tile, ROWS x 32 a step.  KM: the contraction index is contiguous in memory.
+template <int ROWS, bool KM>
+struct F64Operand {
+  static constexpr int PER_THREAD = ROWS * F64_BK / F64_THREADS;
+  static constexpr int LD = KM ? F64_BK + 4 : ROWS + 4;     // [row][k] or [k][row]
+  static constexpr int ROW = KM ? LD : 1, K = KM ? 1 : LD;  // element strides in the f64 buffer
+  static constexpr int I_ROWS = KM ? F64_THREADS / F64_BK : 0, I_K = KM ? 0 : F64_THREADS / ROWS;  // from one copy to the next
+  const float* p;      // this thread's first element of the next step
+  long long i_step, k_step;
+  unsigned rows_in;    // per copy: its row exists
+  int k_left;          // contraction elements from this thread's first one to the end
+  int slot;            // its place in the f64 buffer
+  __device__ __forceinline__ void init(const float* base, long long row_stride, long long k_stride, int row0, int rows, int k0, int k) {
+    const int tid = threadIdx.x;
+    const int r = KM ? tid / F64_BK : tid % ROWS, kk = KM ? tid % F64_BK : tid / ROWS;
+    p = base + (row0 + r) * row_stride + (k0 + kk) * k_stride;
+    i_step = I_ROWS * row_stride + I_K * k_stride;
+    k_step = F64_BK * k_stride;
+    rows_in = 0;
+#pragma unroll
+    for (int i = 0; i < PER_THREAD; ++i) rows_in |= (row0 + r + i * I_ROWS < rows ? 1u : 0u) << i;
+    k_left = k - (k0 + kk);
+    slot = r * ROW + kk * K;
+  }
+  __device__ __forceinline__ void request(float* dst, const float* safe) {
+    const float* q = p;
+#pragma unroll
+    for (int i = 0; i < PER_THREAD; ++i) {
+      const bool in = ((rows_in >> i) & 1u) && i * I_K < k_left;
+      copy_async4(dst + i * F64_THREADS, in ? q : safe, in);
+      q += i_step;
+    }
+    p += k_step;
+    k_left -= F64_BK;
+  }
+  __device__ __forceinline__ void widen_into(double* dst, const float* src) const {
+#pragma unroll
+    for (int i = 0; i < PER_THREAD; ++i) dst[slot + i * (I_ROWS * ROW + I_K * K)] = (double)src[i * F64_THREADS];
+  }
+};
+
 template <int TM, int TN>
-__global__ void __launch_bounds__(F64_THREADS)
+struct F64Tile {
+  static constexpr int WK = TM == 32 ? 2 : 1;              // groups of warps along k
+  static constexpr int WM = TM == 32 ? 2 : 4, WN = 2;      // warps along the tile
+  static_assert(WK * WM * WN * 32 == F64_THREADS, "eight warps");
+  static constexpr int FM = TM / (8 * WM), FN = TN / (8 * WN);  // 8 x 8 fragments per warp
+  static constexpr int A_ELEMS = TM * (F64_BK + 4), B_ELEMS = TN * (F64_BK + 4);  // either layout fits
+  static_assert(F64_BK * (TM + 4) <= A_ELEMS && F64_BK * (TN + 4) <= B_ELEMS, "both layouts share the buffers");
+  static constexpr int LDC = TN + 2;
+  static constexpr int PART = TM * LDC + TM;               // one group's sums: the tile and the row sums
+  static_assert(WK * PART <= 2 * (A_ELEMS + B_ELEMS), "the output tile reuses the operand buffers");
+  static constexpr int RAW = (TM + TN) * F64_BK;           // one copied step, in the order the threads copied it
+  static constexpr int DEPTH = f64_depth(TM);
+  static constexpr size_t SMEM = sizeof(double) * 2 * (A_ELEMS + B_ELEMS) + sizeof(float) * DEPTH * RAW;
+};
+
+template <int TM, int TN, bool A_KM, bool B_KM>
+__device__ __forceinline__ void f64_tile_sums(const F64Gemm& g, double* smem, int row0, int col0, int kt0, int kt1, bool sums) {
+  using Z = F64Tile<TM, TN>;
+  using OA = F64Operand<TM, A_KM>;
+  using OB = F64Operand<TN, B_KM>;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float* raw = reinterpret_cast<float*>(smem + 2 * (Z::A_ELEMS + Z::B_ELEMS)) + tid;
+  OA oa;
+  OB ob;
+  oa.init(g.a, g.a_row, g.a_col, row0, g.m, kt0 * F64_BK, g.k);
+  ob.init(g.b, g.b_col, g.b_row, col0, g.n, kt0 * F64_BK, g.k);
+  const int steps = kt1 - kt0;
+  auto request = [&](int step) {
+    if (step < steps) {
+      float* dst = raw + step % Z::DEPTH * Z::RAW;
+      oa.request(dst, g.a);
+      ob.request(dst + OA::PER_THREAD * F64_THREADS, g.b);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int group = warp / (Z::WM * Z::WN), within = warp % (Z::WM * Z::WN);
+  const int wm = within / Z::WN * (Z::FM * 8), wn = within % Z::WN * (Z::FN * 8);
+  const int fr = lane >> 2, fk = lane & 3;
+  constexpr int KG = F64_BK / Z::WK;  // this group's part of a step
+  double acc[Z::FM][Z::FN][2], rs[Z::FM][2];
+#pragma unroll
+  for (int i = 0; i < Z::FM; ++i) {
+    rs[i][0] = rs[i][1] = 0.0;
+#pragma unroll
+    for (int j = 0; j < Z::FN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  }
+  const bool my_sums = sums && wn == 0;
+#pragma unroll
+  for (int s = 0; s < Z::DEPTH; ++s) request(s);
+  for (int step = 0; step < steps; ++step) {
+    double* buf = smem + (step & 1) * (Z::A_ELEMS + Z::B_ELEMS);
+    asm volatile("cp.async.wait_group %0;" ::"n"(Z::DEPTH - 1) : "memory");  // this thread's copies of the step have landed
+    const float* src = raw + step % Z::DEPTH * Z::RAW;
+    oa.widen_into(buf, src);
+    ob.widen_into(buf + Z::A_ELEMS, src + OA::PER_THREAD * F64_THREADS);
+    request(step + Z::DEPTH);
+    __syncthreads();
+    const double* sa = buf + (wm + fr) * OA::ROW + (group * KG + fk) * OA::K;
+    const double* sb = buf + Z::A_ELEMS + (wn + fr) * OB::ROW + (group * KG + fk) * OB::K;
+#pragma unroll
+    for (int kk = 0; kk < KG; kk += 4) {
+      double fa[Z::FM], fb[Z::FN];
+#pragma unroll
+      for (int i = 0; i < Z::FM; ++i) fa[i] = sa[i * 8 * OA::ROW + kk * OA::K];
+#pragma unroll
+      for (int j = 0; j < Z::FN; ++j) fb[j] = sb[j * 8 * OB::ROW + kk * OB::K];
+#pragma unroll
+      for (int i = 0; i < Z::FM; ++i)
+#pragma unroll
+        for (int j = 0; j < Z::FN; ++j) dmma(acc[i][j], fa[i], fb[j]);
+      if (my_sums) {  // row sums of A: a bias gradient rides on its weight gradient
+#pragma unroll
+        for (int i = 0; i < Z::FM; ++i) dmma(rs[i], fa[i], 1.0);
+      }
+    }
+  }
+  __syncthreads();
+  double* sc = smem + group * Z::PART;
+#pragma unroll
+  for (int i = 0; i < Z::FM; ++i) {
+#pragma unroll
+    for (int j = 0; j < Z::FN; ++j) {
+      double* d = sc + (wm + i * 8 + fr) * Z::LDC + wn + j * 8 + 2 * fk;
+      d[0] = acc[i][j][0];
+      d[1] = acc[i][j][1];
+    }
+    if (my_sums && fk == 0) sc[TM * Z::LDC + wm + i * 8 + fr] = rs[i][0];
+  }
+}
+
+template <int TM, int TN>
+__global__ void __launch_bounds__(F64_THREADS, TM == 32 ? 3 : 2)
 f64_gemm_kernel(const F64Jobs jobs) {
-  constexpr int FM = TM / 16, FN = TN / 16;      // 8 x 8 fragments per warp: four warps, two by two
-  constexpr int LDK = F64_BK + 4;                // row stride of a tile stored [row][k]
-  constexpr int LDM = TM + 4, LDN = TN + 4;      // row stride of a tile stored [k][row]
-  constexpr int A_ELEMS = TM * LDK, B_ELEMS = TN * LDK;
-  static_assert(F64_BK * LDM <= A_ELEMS && F64_BK * LDN <= B_ELEMS, "both layouts share the buffers");
-  constexpr int LDC = TN + 2;
-  static_assert(TM * LDC + TM <= 2 * (A_ELEMS + B_ELEMS), "the output tile reuses the operand buffers");
+  using Z = F64Tile<TM, TN>;
   extern __shared__ double f64_smem[];
   const int which = (jobs.count > 1 && (int)blockIdx.x >= jobs.job[1].cta0) ? 1 : 0;
   const F64Job& jb = jobs.job[which];
@@ -71,107 +207,34 @@ f64_gemm_kernel(const F64Jobs jobs) {
   const int tile = jb.split > 1 ? local / jb.split : local;
   const int rank = jb.split > 1 ? local % jb.split : 0;
   if (tile >= jb.tiles) return;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x;
   const int row0 = (tile / jb.tiles_n) * TM, col0 = (tile % jb.tiles_n) * TN;
-  const bool a_km = g.a_col == 1, b_km = g.b_row == 1;  // contraction index contiguous in memory
-  const int kt_all = (g.k + F64_BK - 1) / F64_BK;
-  const int kt0 = rank * jb.k_tiles_per_rank, kt1 = min(kt_all, kt0 + jb.k_tiles_per_rank);
+  const int kt0 = rank * jb.k_tiles_per_rank, kt1 = max(kt0, min((g.k + F64_BK - 1) / F64_BK, kt0 + jb.k_tiles_per_rank));
   const bool sums = g.row_sum != nullptr && col0 == 0;
-
-  float ra[TM / 4], rb[TN / 4];
-  auto fetch = [&](int kt) {
-    const int k0 = kt * F64_BK;
-#pragma unroll
-    for (int i = 0; i < TM / 4; ++i) {
-      const int e = tid + i * F64_THREADS;
-      const int kk = k0 + (a_km ? e % F64_BK : e / TM), r = row0 + (a_km ? e / F64_BK : e % TM);
-      ra[i] = (r < g.m && kk < g.k) ? __ldg(g.a + r * g.a_row + kk * g.a_col) : 0.f;
-    }
-#pragma unroll
-    for (int i = 0; i < TN / 4; ++i) {
-      const int e = tid + i * F64_THREADS;
-      const int kk = k0 + (b_km ? e % F64_BK : e / TN), c = col0 + (b_km ? e / F64_BK : e % TN);
-      rb[i] = (c < g.n && kk < g.k) ? __ldg(g.b + kk * g.b_row + c * g.b_col) : 0.f;
-    }
-  };
-  auto stash = [&](int buf) {
-    double* sa = f64_smem + buf * (A_ELEMS + B_ELEMS);
-    double* sb = sa + A_ELEMS;
-#pragma unroll
-    for (int i = 0; i < TM / 4; ++i) {
-      const int e = tid + i * F64_THREADS;
-      sa[a_km ? (e / F64_BK) * LDK + e % F64_BK : (e / TM) * LDM + e % TM] = (double)ra[i];
-    }
-#pragma unroll
-    for (int i = 0; i < TN / 4; ++i) {
-      const int e = tid + i * F64_THREADS;
-      sb[b_km ? (e / F64_BK) * LDK + e % F64_BK : (e / TN) * LDN + e % TN] = (double)rb[i];
-    }
-  };
-  const int wm = (warp >> 1) * (TM / 2), wn = (warp & 1) * (TN / 2);
-  const int fr = lane >> 2, fk = lane & 3;
-  const int a_r = a_km ? LDK : 1, a_k = a_km ? 1 : LDM;
-  const int b_r = b_km ? LDK : 1, b_k = b_km ? 1 : LDN;
-  double acc[FM][FN][2], rs[FM][2];
-#pragma unroll
-  for (int i = 0; i < FM; ++i) {
-    rs[i][0] = rs[i][1] = 0.0;
-#pragma unroll
-    for (int j = 0; j < FN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-  }
-  const bool my_sums = sums && wn == 0;
-  if (kt0 < kt1) {
-    fetch(kt0);
-    stash(0);
-  }
-  __syncthreads();
-  for (int kt = kt0; kt < kt1; ++kt) {
-    const int buf = (kt - kt0) & 1;
-    if (kt + 1 < kt1) fetch(kt + 1);
-    const double* sa = f64_smem + buf * (A_ELEMS + B_ELEMS) + (wm + fr) * a_r + fk * a_k;
-    const double* sb = f64_smem + buf * (A_ELEMS + B_ELEMS) + A_ELEMS + (wn + fr) * b_r + fk * b_k;
-#pragma unroll
-    for (int kk = 0; kk < F64_BK; kk += 4) {
-      double fa[FM], fb[FN];
-#pragma unroll
-      for (int i = 0; i < FM; ++i) fa[i] = sa[i * 8 * a_r + kk * a_k];
-#pragma unroll
-      for (int j = 0; j < FN; ++j) fb[j] = sb[j * 8 * b_r + kk * b_k];
-#pragma unroll
-      for (int i = 0; i < FM; ++i) {
-#pragma unroll
-        for (int j = 0; j < FN; ++j) dmma(acc[i][j], fa[i], fb[j]);
-        if (my_sums) dmma(rs[i], fa[i], 1.0);  // row sums of A: a bias gradient rides on its weight gradient
-      }
-    }
-    if (kt + 1 < kt1) stash(buf ^ 1);
-    __syncthreads();
-  }
-  double* sc = f64_smem;
-  double* srs = f64_smem + TM * LDC;
-#pragma unroll
-  for (int i = 0; i < FM; ++i) {
-#pragma unroll
-    for (int j = 0; j < FN; ++j) {
-      double* d = sc + (wm + i * 8 + fr) * LDC + wn + j * 8 + 2 * fk;
-      d[0] = acc[i][j][0];
-      d[1] = acc[i][j][1];
-    }
-    if (my_sums && fk == 0) srs[wm + i * 8 + fr] = rs[i][0];
+  if (g.a_col == 1) {
+    if (g.b_row == 1) f64_tile_sums<TM, TN, true, true>(g, f64_smem, row0, col0, kt0, kt1, sums);
+    else f64_tile_sums<TM, TN, true, false>(g, f64_smem, row0, col0, kt0, kt1, sums);
+  } else {
+    if (g.b_row == 1) f64_tile_sums<TM, TN, false, true>(g, f64_smem, row0, col0, kt0, kt1, sums);
+    else f64_tile_sums<TM, TN, false, false>(g, f64_smem, row0, col0, kt0, kt1, sums);
   }
   const int parts = jb.split;
   cg::cluster_group cluster = cg::this_cluster();
   if (parts > 1) cluster.sync(); else __syncthreads();
+  auto total = [&](int at) {  // over the CTAs of the cluster and the groups of each, in order
+    double v = 0.0;
+    for (int p = 0; p < parts; ++p) {
+      const double* s = parts > 1 ? cluster.map_shared_rank(f64_smem + at, p) : f64_smem + at;
+#pragma unroll
+      for (int w = 0; w < Z::WK; ++w) v += s[w * Z::PART];
+    }
+    return v;
+  };
   for (int e = rank * F64_THREADS + tid; e < TM * TN; e += parts * F64_THREADS) {
     const int r = e / TN, c = e % TN;
     const int row = row0 + r, col = col0 + c;
     if (row >= g.m || col >= g.n) continue;
-    double v = 0.0;
-    if (parts > 1) {
-      for (int p = 0; p < parts; ++p) v += *cluster.map_shared_rank(sc + r * LDC + c, p);
-    } else {
-      v = sc[r * LDC + c];
-    }
+    const double v = total(r * Z::LDC + c);
     const long long at = row * g.o_row + col * g.o_col;
     float y = g.epilogue == F64_ACCUMULATE ? (float)((double)g.out[at] + v) : (float)v;
     if (g.bias) y = y + __ldg(g.bias + col);
@@ -180,21 +243,13 @@ f64_gemm_kernel(const F64Jobs jobs) {
     else if (g.epilogue == F64_DGELU) y = (float)((double)y * gelu_grad<double>((double)g.aux_in[at]));
     g.out[at] = y;
   }
-  if (sums && rank == 0 && tid < TM && row0 + tid < g.m) {
-    double v = 0.0;
-    if (parts > 1) {
-      for (int p = 0; p < parts; ++p) v += *cluster.map_shared_rank(srs + tid, p);
-    } else {
-      v = srs[tid];
-    }
-    g.row_sum[row0 + tid] = (float)v;
-  }
+  if (sums && rank == 0 && tid < TM && row0 + tid < g.m) g.row_sum[row0 + tid] = (float)total(TM * Z::LDC + tid);
   if (parts > 1) cluster.sync();  // no CTA leaves while another still reads its part
 }
 
 template <int TM, int TN>
 int launch_f64_gemm(hl_ctx* ctx, const F64Gemm* problems, int count) {
-  constexpr size_t smem = sizeof(double) * 2 * (TM + TN) * (F64_BK + 4);
+  constexpr size_t smem = F64Tile<TM, TN>::SMEM;
   auto kern = f64_gemm_kernel<TM, TN>;
   static bool configured = false;
   if (!configured) {
