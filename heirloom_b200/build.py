@@ -1,6 +1,6 @@
 """Builds the CUDA library in-tree with nvcc for sm_100a (no GPU needed to compile).
 
-`python -m heirloom_b200.build` compiles every `csrc/*.cu` to an object file in parallel and
+`python -m heirloom_b200.build` compiles every `csrc/*.cu` and `csrc/*.cpp` to an object file in parallel and
 links `heirloom_b200/lib/libheirloom_b200.so`.  Objects are rebuilt only when their source or a
 header is newer.
 """
@@ -46,7 +46,7 @@ def _compile(src: Path, verbose: bool) -> Path:
 
 def build(verbose: bool = False) -> Path:
     OUT.mkdir(exist_ok=True)
-    sources = sorted(CSRC.glob("*.cu"))
+    sources = sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cpp"))
     with ThreadPoolExecutor(max_workers=min(8, len(sources))) as pool:
         objs = list(pool.map(lambda s: _compile(s, verbose), sources))
     if LIB.exists() and all(LIB.stat().st_mtime >= o.stat().st_mtime for o in objs):

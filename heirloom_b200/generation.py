@@ -10,6 +10,7 @@ row of logits, as in the reference.
 """
 from __future__ import annotations
 
+import ctypes
 import math
 from dataclasses import dataclass, field
 from typing import List, Optional, Sequence, Tuple
@@ -17,7 +18,8 @@ from typing import List, Optional, Sequence, Tuple
 import numpy as np
 import torch
 
-from ._lib import HeirloomError
+from ._lib import HeirloomError, check, load
+from .cuda import F32, F64
 
 _MASK = (1 << 64) - 1
 
@@ -156,27 +158,28 @@ def sampling_filter(logits: np.ndarray, o: GenerationOptions) -> np.ndarray:
     return fallback
 
 
+class _SamplingOptions(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_double) for n in ("temperature", "top_p", "repetition_penalty", "frequency_penalty",
+                                               "presence_penalty")] + [("top_k", ctypes.c_longlong)]
+
+
+def _sample(logits: np.ndarray, context: np.ndarray, o: GenerationOptions, rng: HeirloomRng) -> Tuple[int, float, float]:
+    """`hl_sample_token` on a contiguous f32 or f64 row; `context` is an int64 vector."""
+    options = _SamplingOptions(o.temperature, 0.0 if o.top_p is None else o.top_p, o.repetition_penalty, o.frequency_penalty,
+                               o.presence_penalty, 0 if o.top_k is None else o.top_k)
+    draw = rng.uniform_f32() if o.temperature != 0.0 else 0.0
+    token, p, log_p = ctypes.c_int64(), ctypes.c_double(), ctypes.c_double()
+    check(load().hl_sample_token(ctypes.c_void_p(logits.ctypes.data), ctypes.c_int(F32 if logits.dtype == np.float32 else F64),
+                                 ctypes.c_longlong(logits.size), ctypes.c_void_p(context.ctypes.data),
+                                 ctypes.c_longlong(context.size), ctypes.byref(options), ctypes.c_double(draw),
+                                 ctypes.byref(token), ctypes.byref(p), ctypes.byref(log_p)))
+    return token.value, p.value, log_p.value
+
+
 def sample_token(logits: Sequence[float], context: Sequence[int], o: GenerationOptions,
                  rng: HeirloomRng) -> Tuple[int, float, float]:
-    adjusted = np.asarray(logits, np.float64).copy()
-    _apply_repetition_controls(adjusted, context, o)
-    if o.temperature > 0.0:
-        adjusted /= o.temperature
-    keep = sampling_filter(adjusted, o)
-    adjusted[~keep] = -np.inf
-    probs = softmax_logits(adjusted)
-    tiny = np.finfo(np.float64).tiny
-    if o.temperature == 0.0:
-        t = argmax_filtered(adjusted)
-        return t, float(probs[t]), math.log(max(float(probs[t]), tiny))
-    draw = rng.uniform_f32()
-    cumulative = 0.0
-    for t, p in enumerate(probs):
-        cumulative += p
-        if draw <= cumulative:
-            return t, float(p), math.log(max(float(p), tiny))
-    t = argmax_filtered(adjusted)
-    return t, float(probs[t]), math.log(max(float(probs[t]), tiny))
+    """(token, probability, log probability) of one step, sampled natively (`hl_sample_token`)."""
+    return _sample(np.ascontiguousarray(logits, np.float64), np.ascontiguousarray(context, np.int64), o, rng)
 
 
 def next_token_logits(model, tokens: Sequence[int]) -> np.ndarray:
@@ -194,17 +197,24 @@ def generate(model, prefix: Sequence[int], options: GenerationOptions, rng: Heir
     options.validate()
     if len(prefix) == 0:
         raise HeirloomError("generation prefix must contain at least one token")
-    tokens = list(int(t) for t in prefix)
+    length = len(prefix)
+    tokens = np.empty(length + options.max_new_tokens, np.int64)
+    tokens[:length] = prefix
     steps: List[GeneratedTokenStep] = []
     reason = "max_new_tokens"
     for _ in range(options.max_new_tokens):
-        token, p, logp = sample_token(next_token_logits(model, tokens), tokens, options, rng)
-        tokens.append(token)
+        window = tokens[max(0, length - model.cfg.context):length]
+        logits = model.next_token_logits_device(torch.from_numpy(window).cuda())
+        if not np.isfinite(logits).all():
+            raise HeirloomError("non-finite generation logits")
+        token, p, logp = _sample(logits, tokens[:length], options, rng)
+        tokens[length] = token
+        length += 1
         steps.append(GeneratedTokenStep(token, p, logp))
         if token == options.eos_id:
             reason = "eos"
             break
-    return GenerationOutput(tokens, len(steps), reason, rng.state, steps)
+    return GenerationOutput(tokens[:length].tolist(), len(steps), reason, rng.state, steps)
 
 
 def generate_greedy(model, prefix: Sequence[int], max_new_tokens: int, eos_id: int) -> List[int]:

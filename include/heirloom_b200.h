@@ -545,6 +545,20 @@ unsigned long long hl_decoder_launches_last_step(hl_decoder* model);
  * timer (NcclCommunicator::start_event_timer, heirloom-kernels/src/cuda.rs:8049-8233). */
 int hl_decoder_comm_exposed_ms(hl_decoder* model, float* total_ms, int* waits);
 
+/* ---- sampling ---------------------------------------------------------------------------------
+ * One token from a row of logits in host memory (f32 or f64), with the reference's controls (sample_token and its filters,
+ * src/nn.rs:1595-1751): penalties over the token ids of `context`, temperature, top-k, top-p, the last maximum at
+ * temperature 0.  `draw` is the uniform number of this step, in [0, 1); it is not looked at when temperature is 0.  Host
+ * function, no device work. */
+typedef struct {
+  double temperature, top_p; /* top_p outside (0, 1): no such filter */
+  double repetition_penalty, frequency_penalty, presence_penalty;
+  long long top_k; /* 0: no such filter */
+} hl_sampling_options;
+int hl_sample_token(const void* logits, int dtype, long long vocab, const int64_t* context, long long n_context,
+                    const hl_sampling_options* options, double draw, int64_t* token, double* probability,
+                    double* log_probability);
+
 #ifdef __cplusplus
 }
 #endif

@@ -49,6 +49,49 @@ def test_greedy_and_filters_follow_the_reference_rules():
     assert gen.sample_token(np.log(probs), [], gen.GenerationOptions(1, 9, temperature=1.0), rng)[0] == want
 
 
+def stated_sample(logits, context, o, rng):
+    """The sampling rules written out over the module's own filters."""
+    x = np.asarray(logits, np.float64).copy()
+    gen._apply_repetition_controls(x, context, o)
+    if o.temperature > 0.0:
+        x /= o.temperature
+    x[~gen.sampling_filter(x, o)] = -np.inf
+    probs = gen.softmax_logits(x)
+    t = gen.argmax_filtered(x)
+    if o.temperature > 0.0:
+        draw, cumulative = rng.uniform_f32(), 0.0
+        for i, p in enumerate(probs):
+            cumulative += p
+            if draw <= cumulative:
+                t = i
+                break
+    return t, float(probs[t])
+
+
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 1000, 50304])
+def test_native_sampling_follows_the_stated_rules(n):
+    """Vocabularies around the lane width and the largest one, every control, ties and -inf entries.  Probabilities are
+    f64 sums in another order: at most n * 2^-53 relative, 1e-11 here."""
+    r = np.random.default_rng(n)
+    context = r.integers(0, n + 3, 50).tolist()  # ids past the vocabulary are ignored
+    for case in range(12 if n < 5000 else 5):
+        logits = r.standard_normal(n) * r.choice([0.1, 3.0, 30.0])
+        if case % 3 == 1:
+            logits = np.round(logits)  # ties
+        if case % 4 == 2:
+            logits[r.random(n) < 0.3] = -np.inf
+        logits[0] = max(logits[0], -50.0)  # at least one finite entry
+        for kw in (dict(), dict(temperature=0.7), dict(temperature=1.3, top_k=5), dict(top_k=3), dict(temperature=1.0, top_p=0.9),
+                   dict(temperature=0.9, top_k=40, top_p=0.5, repetition_penalty=1.2, frequency_penalty=0.1, presence_penalty=0.2),
+                   dict(temperature=0.5, top_k=10 ** 6, top_p=1.0)):
+            o = gen.GenerationOptions(1, 0, **kw)
+            a, b = gen.HeirloomRng(case), gen.HeirloomRng(case)
+            t, p, logp = gen.sample_token(logits, context, o, a)
+            want_t, want_p = stated_sample(logits, context, o, b)
+            assert t == want_t and p == pytest.approx(want_p, rel=1e-11), (case, kw)
+            assert logp == pytest.approx(math.log(max(p, np.finfo(np.float64).tiny))) and a.state == b.state
+
+
 def test_option_validation_messages():
     for kwargs, text in ((dict(temperature=-1.0), "temperature must be non-negative"), (dict(top_k=0), "top_k must be greater than zero"),
                          (dict(top_p=0.0), "top_p must be in"), (dict(repetition_penalty=0.5), "at least 1.0"),
