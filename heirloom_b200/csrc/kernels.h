@@ -97,6 +97,30 @@ int attention_f64_backward(hl_ctx* ctx, const void* q, const void* k, const void
                            const void* dout, long long ld_dout, void* dq, void* dk, void* dv, long long ld_dqkv, int batch,
                            int time, int channels, int n_heads);
 
+// One-token steps (decode.cu).  out[n] = epilogue(W[n,k] · x + bias), with a layer norm of x first when gamma is given.
+enum { GV_STORE = 0, GV_GELU = 1, GV_RESIDUAL = 2 };
+constexpr int kDecodeMaxRow = 24576;  // longest input row, f32 in shared memory
+struct DecodeGemv {
+  const void* x;
+  int x_dtype;
+  const void* w;
+  int w_dtype;
+  const float* bias;
+  void* out;
+  int out_dtype;
+  int n, k;
+  int epilogue;
+  const float *gamma, *beta;
+  const void* residual;      // of the output's type
+  const long long* out_row;  // device: which row of `out` (row stride ld_out) is written; null: row 0
+  long long ld_out;
+};
+int decode_gemv(hl_ctx* ctx, const DecodeGemv& g);
+size_t decode_attention_smem(int dtype, int head_dim, int context);
+int decode_attention(hl_ctx* ctx, const void* qkv, int dtype, long long ld, const long long* pos, void* out, int channels,
+                     int n_heads, int context);
+int decode_embed(hl_ctx* ctx, const float* table, const float* positions, const long long* state, void* out, int dtype, int dim);
+
 struct AdamPlan;
 int adam_plan_create(hl_ctx* ctx, const hl_adamw_tensor* tensors, int count, AdamPlan** out);
 void adam_plan_destroy(AdamPlan* plan);

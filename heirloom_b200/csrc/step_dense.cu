@@ -150,6 +150,16 @@ struct hl_decoder {
   struct F32Layer {
     float *a, *qkv, *probs, *o, *r, *c, *h, *g;
   };
+  // generation: how many positions of sequence 0 have their keys and values in the activation buffers (0: none), the state
+  // of the next one-token step, and that step as a graph once it has run
+  int cached = 0;
+  long long* decode_state = nullptr;       // device: position, token
+  long long* decode_state_host = nullptr;  // pinned
+  float* logits_host = nullptr;            // pinned, [vocab], allocated on first use
+  cudaGraphExec_t decode_graph = nullptr;
+  void* decode_graph_workspace = nullptr;  // the scratch arena the graph was captured with
+  unsigned long long decode_launches = 0;  // kernels in it
+  bool decode_warm = false;
   std::vector<float*> xf;  // residual stream per block input, f32
   std::vector<F32Layer> lf;
   float *zf = nullptr, *dlogits_f = nullptr, *d_a = nullptr, *d_b = nullptr, *d_c = nullptr, *d_qkv = nullptr, *d_wide = nullptr;
@@ -380,6 +390,7 @@ int plan_activations(hl_decoder* m, bool measure_only, size_t* bytes_out) {
   }
   m->tokens = carve<int64_t>(cur, N);
   m->targets = carve<int64_t>(cur, N);
+  m->decode_state = carve<long long>(cur, 2);
   m->loss_dev = carve<float>(cur, 4);
   m->norm_dev = carve<float>(cur, 4);
   m->norm_dev64 = carve<double>(cur, 2);
@@ -423,6 +434,7 @@ int plan_activations_f32(hl_decoder* m, bool measure_only, size_t* bytes_out) {
   m->fold.used = 0;
   m->tokens = carve<int64_t>(cur, N);
   m->targets = carve<int64_t>(cur, N);
+  m->decode_state = carve<long long>(cur, 2);
   m->loss_dev = carve<float>(cur, 4);
   m->norm_dev = carve<float>(cur, 4);
   m->norm_dev64 = carve<double>(cur, 2);
@@ -500,7 +512,21 @@ int zero_memory_table_grads(hl_decoder* m) {
 // bf16 q, k, v (widened exactly) and round to bf16 where the flash route stores bf16.  Probabilities are not kept per
 // layer, the backward forms them again.
 
-int forward(hl_decoder* m) {
+// Final layer norm and head of one row of the residual stream: the logits in row 0 of m->logits.
+int decode_head(hl_decoder* m, const void* x, int dtype) {
+  DecodeGemv g{};
+  g.x = x; g.x_dtype = dtype;
+  g.gamma = m->params + m->off_lnf_g; g.beta = m->params + m->off_lnf_b;
+  g.w = dtype == HL_BF16 ? (const void*)(m->shadow + m->off_head_w) : (const void*)(m->params + m->off_head_w);
+  g.w_dtype = dtype;
+  g.bias = m->params + m->off_head_b;
+  g.out = m->logits; g.out_dtype = HL_F32;
+  g.n = m->cfg.vocab; g.k = m->cfg.d_model;
+  return decode_gemv(m->ctx, g);
+}
+
+// `last_only`: nothing is read but the logits of the last position, which go to row 0 of m->logits.
+int forward(hl_decoder* m, bool last_only = false) {
   hl_ctx* ctx = m->ctx;
   const hl_decoder_config& c = m->cfg;
   const int N = m->N, d = c.d_model, F = c.d_ff, V = c.vocab, B = c.batch, T = c.context, H = c.n_heads;
@@ -548,6 +574,8 @@ int forward(hl_decoder* m) {
     HL_TRY(g.run(N, d, F, a.g, F, HL_K_MAJOR, W + o.w2, F, HL_K_MAJOR, m->x[l + 1], d, HL_BF16, HL_EPI_BIAS_RESIDUAL,
                  P + o.b2, a.r, d));
   }
+  m->cached = 0;
+  if (last_only) return decode_head(m, m->x[c.n_layers] + (size_t)(N - 1) * d, HL_BF16);
   HL_TRY(layer_norm_forward_impl(ctx, m->x[c.n_layers], HL_BF16, P + m->off_lnf_g, P + m->off_lnf_b, m->z, HL_BF16, m->meanf,
                                  m->rstdf, N, d, 1e-5f));
   HL_TRY(g.run(N, V, d, m->z, d, HL_K_MAJOR, W + m->off_head_w, d, HL_K_MAJOR, m->logits, V, HL_F32, HL_EPI_BIAS,
@@ -882,7 +910,7 @@ int linear_backward_f32(hl_decoder* m, const float* x, const float* w, const flo
 
 int forward_f32_gemm(hl_decoder* m, const F64Gemm& g) { return f64_gemm_run(m->ctx, &g, 1); }
 
-int forward_f32(hl_decoder* m) {
+int forward_f32(hl_decoder* m, bool last_only = false) {
   hl_ctx* ctx = m->ctx;
   const hl_decoder_config& c = m->cfg;
   const int N = m->N, d = c.d_model, F = c.d_ff, V = c.vocab, B = c.batch, T = c.context, H = c.n_heads;
@@ -909,6 +937,8 @@ int forward_f32(hl_decoder* m) {
       HL_TRY(forward_f32_gemm(m, linear_f32(a.g, P + o.w2, P + o.b2, m->xf[l + 1], N, F, d, F64_RESIDUAL, a.r)));
     }
   }
+  m->cached = 0;
+  if (last_only) return decode_head(m, m->xf[c.n_layers] + (size_t)(N - 1) * d, HL_F32);
   HL_TRY(layer_norm_forward_impl(ctx, m->xf[c.n_layers], HL_F32, P + m->off_lnf_g, P + m->off_lnf_b, m->zf, HL_F32, nullptr,
                                  nullptr, N, d, 1e-5f));
   return forward_f32_gemm(m, linear_f32(m->zf, P + m->off_head_w, P + m->off_head_b, m->logits, N, d, V));
@@ -990,6 +1020,80 @@ int backward_f32(hl_decoder* m) {
     // the optimizer takes them bucket group by bucket group, every other reader waits for all of them.
     HL_CUDA(cudaEventRecord(m->comm_done, ctx->comm_stream));
     m->comm_pending = true;
+  }
+  return HL_OK;
+}
+
+// ---- one-token steps of generation -----------------------------------------------------------------
+// The row of m->decode_state through the model: its q/k/v go to the cache (row `position` of the activations that a
+// full-window forward left), every other value of the row to row 0 of its buffer, the logits to row 0 of m->logits.  Row by
+// row this is what forward() and forward_f32() compute (N is 1 meanwhile).
+int decode_step(hl_decoder* m) {
+  hl_ctx* ctx = m->ctx;
+  const hl_decoder_config& c = m->cfg;
+  const int d = c.d_model, F = c.d_ff;
+  const bool amp = c.precision == HL_PRECISION_AMP_BF16;
+  const int dt = amp ? HL_BF16 : HL_F32;
+  const float* P = m->params;
+  auto weight = [&](size_t off) -> const void* { return amp ? (const void*)(m->shadow + off) : (const void*)(P + off); };
+  auto gemv = [&](const void* x, size_t w, size_t b, void* out, int n, int k, int epilogue = GV_STORE, const void* residual = nullptr,
+                  size_t ln_g = 0, size_t ln_b = 0) {
+    DecodeGemv g{};
+    g.x = x; g.x_dtype = dt;
+    g.w = weight(w); g.w_dtype = dt;
+    g.bias = P + b;
+    g.out = out; g.out_dtype = dt;
+    g.n = n; g.k = k; g.epilogue = epilogue; g.residual = residual;
+    if (ln_g) { g.gamma = P + ln_g; g.beta = P + ln_b; }
+    return g;
+  };
+  HL_TRY(decode_embed(ctx, P + m->off_tok, P + m->off_pos, m->decode_state, amp ? (void*)m->x[0] : (void*)m->xf[0], dt, d));
+  for (int l = 0; l < c.n_layers; ++l) {
+    const LayerOffsets& o = m->lo[l];
+    void *x, *next, *qkv, *att, *r, *g;
+    if (amp) { x = m->x[l]; next = m->x[l + 1]; qkv = m->la[l].qkv; att = m->la[l].o; r = m->la[l].r; g = m->la[l].g; }
+    else { x = m->xf[l]; next = m->xf[l + 1]; qkv = m->lf[l].qkv; att = m->lf[l].o; r = m->lf[l].r; g = m->lf[l].g; }
+    // the attention output, r and g rows may lie over cached positions' rows: only the q/k/v rows are kept
+    DecodeGemv q = gemv(x, o.wqkv, o.bqkv, qkv, 3 * d, d, GV_STORE, nullptr, o.ln1g, o.ln1b);
+    q.out_row = m->decode_state;
+    q.ld_out = 3 * d;
+    HL_TRY(decode_gemv(ctx, q));
+    HL_TRY(decode_attention(ctx, qkv, dt, 3 * d, m->decode_state, att, d, c.n_heads, c.context));
+    HL_TRY(decode_gemv(ctx, gemv(att, o.wo, o.bo, r, d, d, GV_RESIDUAL, x)));
+    if (o.is_memory) {
+      MemoryActs& ma = m->ma[l];
+      const int kd = m->mem.key_dim, vd = m->mem.value_dim;
+      // f32 weights against the normalised row: as accurate as the pieces the full-window route multiplies
+      auto project = [&](const void* in, int in_dtype, size_t w, size_t b, void* out, int out_dtype, int n, int k, int epilogue,
+                         const void* residual, bool ln) {
+        DecodeGemv p = gemv(in, w, b, out, n, k, epilogue, residual, ln ? o.ln2g : 0, ln ? o.ln2b : 0);
+        p.x_dtype = in_dtype; p.w = P + w; p.w_dtype = HL_F32; p.out_dtype = out_dtype;
+        return decode_gemv(ctx, p);
+      };
+      HL_TRY(project(r, dt, o.wq_m, o.bq_m, ma.query, HL_F32, kd, d, GV_STORE, nullptr, true));
+      HL_TRY(memory_core_forward(m, l));
+      HL_TRY(project(r, dt, o.wg_m, o.bg_m, ma.gate, HL_F32, vd, d, GV_GELU, nullptr, true));
+      HL_TRY(hl_binary_f32(ctx, HL_MUL, ma.weighted, ma.gate, ma.mv, (size_t)vd));
+      HL_TRY(project(ma.mv, HL_F32, o.wout_m, o.bout_m, next, dt, d, vd, GV_RESIDUAL, r, false));
+    } else {
+      HL_TRY(decode_gemv(ctx, gemv(r, o.w1, o.b1, g, F, d, GV_GELU, nullptr, o.ln2g, o.ln2b)));
+      HL_TRY(decode_gemv(ctx, gemv(g, o.w2, o.b2, next, d, F, GV_RESIDUAL, r)));
+    }
+  }
+  return decode_head(m, amp ? (const void*)m->x[c.n_layers] : (const void*)m->xf[c.n_layers], dt);
+}
+
+bool decode_applicable(const hl_decoder* m) {
+  const hl_decoder_config& c = m->cfg;
+  const int dt = c.precision == HL_PRECISION_AMP_BF16 ? HL_BF16 : HL_F32;
+  return c.d_ff <= kDecodeMaxRow && decode_attention_smem(dt, c.d_model / c.n_heads, c.context) <= 48 * 1024 &&
+         (!m->has_memory || m->mem.value_dim <= kDecodeMaxRow);
+}
+
+int ensure_logits_host(hl_decoder* m) {
+  if (!m->logits_host) {
+    HL_CUDA(cudaMallocHost(reinterpret_cast<void**>(&m->logits_host), sizeof(float) * (size_t)m->cfg.vocab + 32));
+    m->decode_state_host = reinterpret_cast<long long*>(m->logits_host + ((m->cfg.vocab + 3) & ~3));
   }
   return HL_OK;
 }
@@ -1245,6 +1349,8 @@ void hl_decoder_destroy(hl_decoder* m) {
   if (m->tok_packed) cudaFree(m->tok_packed);
   cudaFree(m->params); cudaFree(m->grads); cudaFree(m->m); cudaFree(m->v); cudaFree(m->shadow); cudaFree(m->act_arena);
   if (m->loss_host) cudaFreeHost(m->loss_host);
+  if (m->logits_host) cudaFreeHost(m->logits_host);
+  if (m->decode_graph) cudaGraphExecDestroy(m->decode_graph);
   delete m;
 }
 
@@ -1279,6 +1385,7 @@ int hl_decoder_set_param(hl_decoder* m, int index, const float* host, long long 
   const Slot* s;
   HL_TRY(slot_io(m, index, numel, &s, "hl_decoder_set_param"));
   HL_TRY(hl_memcpy_h2d(m->ctx, m->params + s->offset, host, sizeof(float) * s->numel));
+  m->cached = 0;
   return refresh_shadow(m, s->offset, s->numel);
 }
 
@@ -1358,6 +1465,7 @@ int hl_decoder_forward_backward(hl_decoder* m, const int64_t* tokens_dev, const 
 int hl_decoder_optimizer_step(hl_decoder* m) {
   HL_REQUIRE(m, "hl_decoder_optimizer_step: null model");
   const unsigned long long before = m->ctx->counters.launches;
+  m->cached = 0;
   HL_TRY(optimizer_step(m));
   m->launches_last_step += m->ctx->counters.launches - before;
   return HL_OK;
@@ -1534,6 +1642,7 @@ int hl_decoder_optimizer_step_policy(hl_decoder* m, int policy) {
   if (policy == HL_MEMORY_UPDATE_FULL) return hl_decoder_optimizer_step(m);
   HL_REQUIRE(m->has_memory, "hl_decoder_optimizer_step_policy: the model has no memory layers");
   const unsigned long long before = m->ctx->counters.launches;
+  m->cached = 0;
   int rc;
   switch (policy) {
     case HL_MEMORY_UPDATE_MEMORY_ONLY: rc = hl::step_memory_only(m); break;
@@ -1627,17 +1736,95 @@ int hl_decoder_eval_loss(hl_decoder* m, const int64_t* tokens_dev, const int64_t
   return hl_memcpy_d2h(m->ctx, loss_host, m->loss_dev, sizeof(float));
 }
 
-int hl_decoder_next_token_logits(hl_decoder* m, const int64_t* window_dev, int window_len, float* logits_host) {
-  HL_REQUIRE(m && window_dev && logits_host, "hl_decoder_next_token_logits: null argument");
+static int window_logits(hl_decoder* m, const int64_t* window, cudaMemcpyKind kind, int window_len, float* logits_host) {
   HL_REQUIRE(window_len >= 1, "next_token_logits requires at least one token");
   HL_REQUIRE(window_len <= m->cfg.context, "hl_decoder_next_token_logits: the window is longer than the model's context");
-  HL_CUDA(cudaMemcpyAsync(m->tokens, window_dev, sizeof(int64_t) * window_len, cudaMemcpyDeviceToDevice, m->ctx->stream));
+  hl_ctx* ctx = m->ctx;
+  HL_TRY(ensure_logits_host(m));
+  HL_CUDA(cudaMemcpyAsync(m->tokens, window, sizeof(int64_t) * window_len, kind, ctx->stream));
   {
     ScopedShape shape(m, 1, window_len);
-    if (m->cfg.precision == HL_PRECISION_AMP_BF16) HL_TRY(forward(m));
-    else HL_TRY(forward_f32(m));
+    // a final row too long for the matrix-vector kernel's shared memory cannot happen: d_model is at most 1024
+    if (m->cfg.precision == HL_PRECISION_AMP_BF16) HL_TRY(forward(m, true));
+    else HL_TRY(forward_f32(m, true));
   }
-  return hl_memcpy_d2h(m->ctx, logits_host, m->logits + (size_t)(window_len - 1) * m->cfg.vocab, sizeof(float) * m->cfg.vocab);
+  HL_CUDA(cudaMemcpyAsync(m->logits_host, m->logits, sizeof(float) * (size_t)m->cfg.vocab, cudaMemcpyDeviceToHost, ctx->stream));
+  HL_CUDA(cudaStreamSynchronize(ctx->stream));
+  ctx->counters.d2h_bytes += sizeof(float) * (size_t)m->cfg.vocab;
+  memcpy(logits_host, m->logits_host, sizeof(float) * (size_t)m->cfg.vocab);
+  return HL_OK;
+}
+
+int hl_decoder_next_token_logits(hl_decoder* m, const int64_t* window_dev, int window_len, float* logits_host) {
+  HL_REQUIRE(m && window_dev && logits_host, "hl_decoder_next_token_logits: null argument");
+  return window_logits(m, window_dev, cudaMemcpyDeviceToDevice, window_len, logits_host);
+}
+
+int hl_decoder_prefill(hl_decoder* m, const int64_t* window_host, int window_len, float* logits_host) {
+  HL_REQUIRE(m && window_host && logits_host, "hl_decoder_prefill: null argument");
+  HL_TRY(window_logits(m, window_host, cudaMemcpyHostToDevice, window_len, logits_host));
+  m->cached = decode_applicable(m) ? window_len : 0;
+  return HL_OK;
+}
+
+int hl_decoder_cached_positions(hl_decoder* m) { return m ? m->cached : 0; }
+
+int hl_decoder_decode_next(hl_decoder* m, int64_t token, float* logits_host) {
+  HL_REQUIRE(m && logits_host, "hl_decoder_decode_next: null argument");
+  HL_REQUIRE(m->cached > 0, "hl_decoder_decode_next: no window is cached (call hl_decoder_prefill)");
+  HL_REQUIRE(m->cached < m->cfg.context, "hl_decoder_decode_next: the context is full");
+  HL_REQUIRE(token >= 0 && token < m->cfg.vocab, "hl_decoder_decode_next: token id out of range");
+  hl_ctx* ctx = m->ctx;
+  m->decode_state_host[0] = m->cached;
+  m->decode_state_host[1] = token;
+  const int position = m->cached;
+  m->cached = 0;  // until this step has succeeded
+  auto queue = [&]() -> int {
+    HL_CUDA(cudaMemcpyAsync(m->decode_state, m->decode_state_host, 2 * sizeof(long long), cudaMemcpyHostToDevice, ctx->stream));
+    {
+      const int n = m->N;
+      m->N = 1;
+      const int rc = decode_step(m);
+      m->N = n;
+      HL_TRY(rc);
+    }
+    HL_CUDA(cudaMemcpyAsync(m->logits_host, m->logits, sizeof(float) * (size_t)m->cfg.vocab, cudaMemcpyDeviceToHost, ctx->stream));
+    return HL_OK;
+  };
+  // The step is the same every time (position and token are read from memory), so from the second one on it is replayed as a
+  // graph: sixty launches of a few microseconds each cost the host more than the device.
+  if (m->decode_graph && m->decode_graph_workspace != ctx->workspace) {
+    cudaGraphExecDestroy(m->decode_graph);
+    m->decode_graph = nullptr;
+  }
+  if (!m->decode_warm || ctx->profiler) {
+    HL_TRY(queue());
+    m->decode_warm = true;
+  } else {
+    if (m->decode_graph) {
+      ctx->counters.launches += m->decode_launches;
+    } else {
+      const unsigned long long before = ctx->counters.launches;
+      cudaGraph_t graph = nullptr;
+      HL_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+      const int rc = queue();
+      const cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
+      if (rc != HL_OK) { if (graph) cudaGraphDestroy(graph); return rc; }
+      HL_CUDA(e);
+      const cudaError_t e2 = cudaGraphInstantiate(&m->decode_graph, graph, 0);
+      cudaGraphDestroy(graph);
+      HL_CUDA(e2);
+      m->decode_graph_workspace = ctx->workspace;
+      m->decode_launches = ctx->counters.launches - before;
+    }
+    HL_CUDA(cudaGraphLaunch(m->decode_graph, ctx->stream));
+  }
+  HL_CUDA(cudaStreamSynchronize(ctx->stream));
+  ctx->counters.h2d_bytes += 2 * sizeof(long long);
+  ctx->counters.d2h_bytes += sizeof(float) * (size_t)m->cfg.vocab;
+  memcpy(logits_host, m->logits_host, sizeof(float) * (size_t)m->cfg.vocab);
+  m->cached = position + 1;
+  return HL_OK;
 }
 
 int hl_decoder_loss(hl_decoder* m, float* loss_host) {

@@ -5,8 +5,8 @@ follow src/nn.rs:1595-1751 statement by statement (repetition, frequency and pre
 temperature, top-k, top-p, greedy at temperature 0); `evaluate_token_loss` walks the token stream in
 windows of `context` tokens like src/memory_transformer.rs:1813-1912; `generate` is
 src/memory_transformer.rs:1730-1769.  The model work (full-window forward, loss) runs on the GPU
-through `hl_decoder_eval_loss` / `hl_decoder_next_token_logits`; sampling is host arithmetic over one
-row of logits, as in the reference.
+through `hl_decoder_eval_loss` / `hl_decoder_prefill` / `hl_decoder_decode_next`; sampling is host arithmetic over one
+row of logits, as in the reference, in native code.
 """
 from __future__ import annotations
 
@@ -197,14 +197,19 @@ def generate(model, prefix: Sequence[int], options: GenerationOptions, rng: Heir
     options.validate()
     if len(prefix) == 0:
         raise HeirloomError("generation prefix must contain at least one token")
-    length = len(prefix)
+    length, context, cached = len(prefix), model.cfg.context, False
     tokens = np.empty(length + options.max_new_tokens, np.int64)
     tokens[:length] = prefix
     steps: List[GeneratedTokenStep] = []
     reason = "max_new_tokens"
     for _ in range(options.max_new_tokens):
-        window = tokens[max(0, length - model.cfg.context):length]
-        logits = model.next_token_logits_device(torch.from_numpy(window).cuda())
+        # While everything fits in the context the window only grows at its end: its keys and values stay on the device and
+        # a step computes one position.  Past the context every position shifts, and the whole window is run again.
+        if cached and length <= context:
+            logits = model.decode_next(int(tokens[length - 1]))
+        else:
+            logits = model.prefill(tokens[max(0, length - context):length])
+        cached = length < context and model.cached_positions == length
         if not np.isfinite(logits).all():
             raise HeirloomError("non-finite generation logits")
         token, p, logp = _sample(logits, tokens[:length], options, rng)

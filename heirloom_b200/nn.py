@@ -209,6 +209,22 @@ class DecoderLm:
                                                      c_int(window.numel()), out.ctypes.data_as(c_void_p)))
         return out
 
+    def prefill(self, window: np.ndarray) -> np.ndarray:
+        """Logits after a window of 1..context tokens (int64 host vector), which stays cached for `decode_next`."""
+        out = np.empty(self.cfg.vocab, np.float32)
+        check(self._lib.hl_decoder_prefill(self.handle, c_void_p(window.ctypes.data), c_int(window.size), c_void_p(out.ctypes.data)))
+        return out
+
+    def decode_next(self, token: int) -> np.ndarray:
+        """Logits after one more token behind the cached window."""
+        out = np.empty(self.cfg.vocab, np.float32)
+        check(self._lib.hl_decoder_decode_next(self.handle, c_longlong(token), c_void_p(out.ctypes.data)))
+        return out
+
+    @property
+    def cached_positions(self) -> int:
+        return int(self._lib.hl_decoder_cached_positions(self.handle))
+
     def train_step_device(self, tokens: torch.Tensor, targets: torch.Tensor) -> None:
         check(self._lib.hl_decoder_train_step_device(self.handle, c_void_p(tokens.data_ptr()),
                                                      c_void_p(targets.data_ptr())))

@@ -522,6 +522,14 @@ int hl_decoder_eval_loss(hl_decoder* model, const int64_t* tokens_dev, const int
 /* next_token_logits (src/memory_transformer.rs:1930-1984): one window of 1..context tokens, full-window
  * forward, the `vocab` logits of its last position copied to the host. */
 int hl_decoder_next_token_logits(hl_decoder* model, const int64_t* window_dev, int window_len, float* logits_host);
+/* The same for a generation loop (src/memory_transformer.rs:1730-1769), which appends one token at a time: prefill runs the
+ * window (host memory, 1..context tokens) like hl_decoder_next_token_logits and keeps its keys and values, decode_next
+ * appends one token to it and computes that position alone, each returning the `vocab` logits of the last position.  The
+ * cache ends with any other forward pass, with new parameter values or when the context is full; cached_positions tells
+ * how far it reaches (0: nothing cached, or the model's sizes are not supported: use hl_decoder_next_token_logits). */
+int hl_decoder_prefill(hl_decoder* model, const int64_t* window_host, int window_len, float* logits_host);
+int hl_decoder_decode_next(hl_decoder* model, int64_t token, float* logits_host);
+int hl_decoder_cached_positions(hl_decoder* model);
 /* zero_grad + loss + backward (src/bin/heirloom/commands/training.rs:125-167) on device-resident
  * i64 tokens/targets of shape [batch, context].  With an NCCL communicator on the context,
  * 25 MiB gradient buckets are all-reduced on the collective stream as backward produces them. */

@@ -150,3 +150,34 @@ def test_logits_eval_and_generation_on_the_device_match_the_oracle():
             eos = got_tokens[5]
             assert gen.generate(model, stream[:4], gen.GenerationOptions.greedy(6, eos), gen.HeirloomRng(0)).finish_reason == "eos"
         model.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,memory", [(1, False), (2, False), (4, False), (1, True)])
+def test_one_token_steps_equal_the_full_window(heads, memory):
+    """prefill + decode_next against a full-window pass for every length from 1 to the context, head sizes 128, 64 and 32, with
+    and without a memory block: f32 within the rounding of its sums, bf16 within a few steps of bf16 of the logits' scale
+    (each of the two layers rounds its row to bf16 at about ten points, 2^-9 relative each)."""
+    from heirloom_b200 import nn
+    from tests.gpu_util import ctx
+    c = ctx()
+    kw = dict(vocab=72, d_model=128, n_layers=2, n_heads=heads, d_ff=200, context=19)
+    mem = dict(memory_layers=(1,), slots=64, key_dim=32, value_dim=32, top_k=4)
+    stream = np.random.default_rng(3).integers(0, 72, 19)
+    for precision, tol in ((nn.PRECISION_F32, 2e-6), (nn.PRECISION_AMP_BF16, 3e-2)):
+        batch = 64 if memory else 1
+        model = nn.DecoderLm(c, nn.DecoderConfig(batch=batch, precision=precision, **kw), nn.MemoryConfig(**mem) if memory else None)
+        rng = np.random.default_rng(heads)
+        model.load_state_dict({n: (np.ones(s) if ".ln" in n or n.startswith("ln_f") else rng.standard_normal(s) * 0.1)
+                               for n, s in ((n, s) for n, s in model.parameter_shapes().items())})
+        got = [model.prefill(stream[:1])] + [model.decode_next(int(t)) for t in stream[1:]]
+        assert model.cached_positions == 19
+        with pytest.raises(Exception, match="context is full"):
+            model.decode_next(0)
+        for n in range(1, 20):
+            want = gen.next_token_logits(model, stream[:n])
+            assert np.abs(got[n - 1] - want).max() <= tol * max(1.0, np.abs(want).max()), (precision, n)
+        assert model.cached_positions == 0
+        with pytest.raises(Exception, match="no window is cached"):
+            model.decode_next(0)
+        model.close()
