@@ -7,6 +7,7 @@
 #include <stdint.h>
 #include <stddef.h>
 #include <string>
+#include <utility>
 #include <algorithm>
 #include "../../include/heirloom_b200.h"
 
@@ -74,6 +75,29 @@ struct hl_ctx {
 };
 
 namespace hl {
+// Programmatic dependent launch: the kernel may be resident before its predecessor on the stream has finished, so that its
+// launch and its set-up cost no time of their own.  Such a kernel calls pdl_wait() before it touches anything a predecessor
+// wrote (or still reads), and pdl_trigger() to let its own successor come in early; a wait covers all earlier kernels,
+// because each of them waited too before it finished.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2] = {};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
 int ensure_workspace(hl_ctx* ctx, size_t bytes);
 inline void count_launch(hl_ctx* ctx, unsigned long long n = 1) { ctx->counters.launches += n; }
 // SMs a persistent one-CTA-per-SM kernel should fill: all of them, minus those left to the collective kernels.  A CTA of

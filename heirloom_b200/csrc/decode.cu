@@ -3,8 +3,9 @@
 //
 // What bounds them: a step of the GPT-sized model reads 250 MB of bf16 weights (38 us at the copy rate) through some sixty
 // dependent kernels, so it is bound by the latency of each: launch, input row, weights, reduction.  Hence a warp per output
-// element with all of its weight loads in flight at once, layer norms folded into the product that reads them (every CTA
-// normalises the row again, which is cheaper than a kernel of its own), and a step that can be captured and replayed.
+// element with its weight loads in flight before the kernel waits for its predecessor (programmatic dependent launch), layer
+// norms folded into the product that reads them (every CTA normalises the row again, which is cheaper than a kernel of its
+// own), and a step that can be captured and replayed.
 #include <cooperative_groups.h>
 
 #include "kernels.h"
@@ -47,83 +48,160 @@ struct GemvArgs {
   long long ld_out;
   int n, k;
   int epilogue;
-  bool vec;             // rows of w start on 16 bytes
+  int warps_per_row;    // power of two; 1 with a layer norm
+  bool vec;             // rows of w, and x, start on 16 bytes
 };
 
-// out = epilogue(W · x + bias).  WT/XT/OT: weights, input, output; Acc: float on the bf16 route, double where the f32
-// route's sums are f64.  The values are rounded where the full-window kernels round them.
-template <typename WT, typename XT, typename OT, typename Acc>
-__global__ void __launch_bounds__(GV_THREADS)
-decode_gemv_kernel(const GemvArgs a) {
-  extern __shared__ float gv_x[];  // the input row, normalised and rounded to the type it is stored in
-  __shared__ Acc red[32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const XT* x = static_cast<const XT*>(a.x);
-  const int k = a.k;
-  if (a.gamma) {
-    Acc sum = 0;
-    for (int c = threadIdx.x; c < k; c += GV_THREADS) {
-      const float v = as_f32(x[c]);
-      gv_x[c] = v;
-      sum += (Acc)v;
-    }
-    const Acc mean = block_sum(sum, red) / (Acc)k;
-    Acc sq = 0;
-    for (int c = threadIdx.x; c < k; c += GV_THREADS) { const Acc d = (Acc)gv_x[c] - mean; sq += d * d; }
-    const Acc rstd = (Acc)1 / sqrt(block_sum(sq, red) / (Acc)k + (Acc)1e-5f);
-    for (int c = threadIdx.x; c < k; c += GV_THREADS) {
-      const float y = (float)(((Acc)gv_x[c] - mean) * rstd * (Acc)a.gamma[c] + (Acc)a.beta[c]);
-      gv_x[c] = sizeof(XT) == 2 ? bf16_round(y) : y;
-    }
-  } else {
-    for (int c = threadIdx.x; c < k; c += GV_THREADS) gv_x[c] = as_f32(x[c]);
+constexpr int GV_SPAN = 1024;  // contraction elements a warp holds at a time, 32 a lane
+
+template <int N> __device__ __forceinline__ void load_x(const float* p, float (&v)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; i += 4) {
+    const float4 t = *reinterpret_cast<const float4*>(p + i);
+    v[i] = t.x; v[i + 1] = t.y; v[i + 2] = t.z; v[i + 3] = t.w;
   }
-  __syncthreads();
-  constexpr int PN = Pack<WT>::N, STEP = 32 * PN, U = 4;
-  OT* out = static_cast<OT*>(a.out) + (a.out_row ? *a.out_row * a.ld_out : 0);
-  for (int row = blockIdx.x * GV_WARPS + warp; row < a.n; row += gridDim.x * GV_WARPS) {
-    const WT* w = static_cast<const WT*>(a.w) + (size_t)row * k;
-    Acc acc = 0;
-    if (a.vec) {
-      for (int c0 = lane * PN; c0 < k; c0 += U * STEP) {
-        uint4 raw[U];
+}
+template <int N> __device__ __forceinline__ void load_x(const __nv_bfloat16* p, float (&v)[N]) {
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-          raw[u] = c0 + u * STEP < k ? __ldg(reinterpret_cast<const uint4*>(w + c0 + u * STEP)) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int c = c0 + u * STEP;
-          if (c < k) {
-            float v[PN];
-            Pack<WT>::unpack(raw[u], v);
-#pragma unroll
-            for (int e = 0; e < PN; ++e) acc += (Acc)v[e] * (Acc)gv_x[c + e];
-          }
-        }
-      }
-    } else {
-      for (int c = lane; c < k; c += 32) acc += (Acc)as_f32(w[c]) * (Acc)gv_x[c];
-    }
-    acc = warp_sum(acc);
-    if (lane == 0) {
-      // f32 rows round the product before the bias is added, the tensor-core route adds it to the accumulator
-      float y = (float)acc;
-      if (a.bias) y = y + a.bias[row];
-      if (a.epilogue == GV_GELU) {
-        y = sizeof(OT) == 2 ? gelu_fwd_fast(bf16_round(y)) : (float)gelu_fwd<double>((double)y);
-      } else if (a.epilogue == GV_RESIDUAL) {
-        const float r = as_f32(static_cast<const OT*>(a.residual)[row]);
-        y = sizeof(OT) == 2 ? r + bf16_round(y) : r + y;
-      }
-      if constexpr (sizeof(OT) == 2) out[row] = to_bf16(y); else out[row] = y;
-    }
+  for (int i = 0; i < N; i += 4) {
+    const uint2 t = *reinterpret_cast<const uint2*>(p + i);
+    const float2 a = unpack_bf16x2(t.x), b = unpack_bf16x2(t.y);
+    v[i] = a.x; v[i + 1] = a.y; v[i + 2] = b.x; v[i + 3] = b.y;
   }
 }
 
-// Row *pos of the q/k/v rows against rows 0 .. *pos: a cluster of eight CTAs per head, each over an eighth of the keys; the
-// partial maxima, sums and weighted values meet in CTA 0 through distributed shared memory.
+// out = epilogue(W · x + bias).  WT/XT/OT: weights, input, output; Acc: float on the bf16 route, double where the f32
+// route's sums are f64.  The values are rounded where the full-window kernels round them.  A lane holds the same 32 elements
+// of x and of the weight row, so that a row needs no shared memory and a layer norm two warp sums; rows longer than 1024
+// are shared by several warps.
+template <typename WT, typename XT, typename OT, typename Acc>
+__global__ void __launch_bounds__(GV_THREADS)
+decode_gemv_kernel(const GemvArgs a) {
+  constexpr int PN = Pack<WT>::N, STEP = 32 * PN, U = GV_SPAN / STEP;
+  __shared__ Acc parts[GV_WARPS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int wpr = a.warps_per_row, part = warp % wpr, k = a.k;
+  const int row_step = gridDim.x * (GV_WARPS / wpr);
+  const int spans = (k + GV_SPAN * wpr - 1) / (GV_SPAN * wpr);  // how often the warps of a row move on
+  const XT* x = static_cast<const XT*>(a.x);
+  auto column = [&](int span, int u) { return (span * wpr + part) * GV_SPAN + u * STEP + lane * PN; };
+  uint4 raw[U];
+  auto fetch = [&](int row, int span) {
+    const WT* w = static_cast<const WT*>(a.w) + (size_t)row * k;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int c = column(span, u);
+      raw[u] = c < k ? __ldg(reinterpret_cast<const uint4*>(w + c)) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  int row = blockIdx.x * (GV_WARPS / wpr) + warp / wpr;
+  // weights and bias do not depend on any kernel of the step
+  if (a.vec && row < a.n) fetch(row, 0);
+  float bias = a.bias && row < a.n ? __ldg(a.bias + row) : 0.f;
+  pdl_trigger();
+  pdl_wait();
+  const OT* residual = static_cast<const OT*>(a.residual);
+  float res = a.epilogue == GV_RESIDUAL && row < a.n ? as_f32(residual[row]) : 0.f;
+  const long long out_row = a.out_row ? *a.out_row : 0;
+  OT* out = static_cast<OT*>(a.out) + out_row * a.ld_out;
+  float xv[U][PN];
+  auto load_span = [&](int span) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int c = column(span, u);
+      if (c < k) {
+        load_x(x + c, xv[u]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < PN; ++e) xv[u][e] = 0.f;
+      }
+    }
+  };
+  if (a.vec) load_span(0);
+  if (a.gamma) {  // one span, one warp per row
+    float g[U][PN], b[U][PN];
+    Acc sum = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int c = column(0, u);
+      if (c < k) { load_x(a.gamma + c, g[u]); load_x(a.beta + c, b[u]); }
+#pragma unroll
+      for (int e = 0; e < PN; ++e) sum += (Acc)xv[u][e];
+    }
+    const Acc mean = warp_sum(sum) / (Acc)k;
+    Acc sq = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (column(0, u) < k) {
+#pragma unroll
+        for (int e = 0; e < PN; ++e) { const Acc d = (Acc)xv[u][e] - mean; sq += d * d; }
+      }
+    const Acc rstd = (Acc)1 / sqrt(warp_sum(sq) / (Acc)k + (Acc)1e-5f);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (column(0, u) < k) {
+#pragma unroll
+        for (int e = 0; e < PN; ++e) {
+          const float y = (float)(((Acc)xv[u][e] - mean) * rstd * (Acc)g[u][e] + (Acc)b[u][e]);
+          xv[u][e] = sizeof(XT) == 2 ? bf16_round(y) : y;
+        }
+      }
+  }
+  for (int base = blockIdx.x * (GV_WARPS / wpr); base < a.n; base += row_step, row += row_step) {
+    Acc acc = 0;
+    if (row >= a.n) {
+    } else if (a.vec) {
+      for (int span = 0; span < spans; ++span) {
+        uint4 now[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) now[u] = raw[u];
+        // the next weights, of this row or of the warp's next one, travel while these are multiplied
+        if (span + 1 < spans) fetch(row, span + 1);
+        else if (row + row_step < a.n) fetch(row + row_step, 0);
+        if (spans > 1) load_span(span);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          float v[PN];
+          Pack<WT>::unpack(now[u], v);
+#pragma unroll
+          for (int e = 0; e < PN; ++e) acc += (Acc)v[e] * (Acc)xv[u][e];
+        }
+      }
+    } else {
+      const WT* w = static_cast<const WT*>(a.w) + (size_t)row * k;
+      for (int c = part * 32 + lane; c < k; c += 32 * wpr) acc += (Acc)as_f32(w[c]) * (Acc)as_f32(x[c]);
+    }
+    acc = warp_sum(acc);
+    if (wpr > 1) {
+      if (lane == 0) parts[warp] = acc;
+      __syncthreads();
+      if (part == 0)
+        for (int i = 1; i < wpr; ++i) acc += parts[warp + i];
+    }
+    if (lane == 0 && part == 0 && row < a.n) {
+      // f32 rows round the product before the bias is added, the tensor-core route adds it to the accumulator
+      float y = (float)acc;
+      if (a.bias) y = y + bias;
+      if (a.epilogue == GV_GELU) {
+        y = sizeof(OT) == 2 ? gelu_fwd_fast(bf16_round(y)) : (float)gelu_fwd<double>((double)y);
+      } else if (a.epilogue == GV_RESIDUAL) {
+        y = sizeof(OT) == 2 ? res + bf16_round(y) : res + y;
+      }
+      if constexpr (sizeof(OT) == 2) out[row] = to_bf16(y); else out[row] = y;
+    }
+    if (row + row_step < a.n) {
+      if (a.bias) bias = __ldg(a.bias + row + row_step);
+      if (a.epilogue == GV_RESIDUAL) res = as_f32(residual[row + row_step]);
+    }
+    if (wpr > 1) __syncthreads();
+  }
+}
+
+// Row *pos of the q/k/v rows against rows 0 .. *pos: a cluster of eight CTAs per head, each over an eighth of the keys; their
+// maxima, sums and weighted values are pushed into CTA 0's shared memory.  Eight lanes take a key, sixteen bytes each.
 constexpr int DA_CTAS = 8;
 constexpr int DA_THREADS = 128;
+constexpr int DA_SLOTS = DA_THREADS / 8;  // keys at a time
 template <typename T, typename Acc>
 __global__ void __launch_bounds__(DA_THREADS)
 decode_attention_kernel(const T* __restrict__ qkv, long long ld, int channels, const long long* __restrict__ pos,
@@ -131,27 +209,40 @@ decode_attention_kernel(const T* __restrict__ qkv, long long ld, int channels, c
   extern __shared__ double da_smem[];
   Acc* q = reinterpret_cast<Acc*>(da_smem);  // [hd]
   Acc* s = q + hd;                           // [chunk_cap] scores, then weights
-  Acc* o = s + chunk_cap;                    // [hd] weighted values of this CTA
-  Acc* part = o + hd;                        // [DA_THREADS] sums of the thread groups over their keys
-  __shared__ Acc stat[2];                    // maximum, sum
+  Acc* part = s + chunk_cap;                 // [DA_SLOTS][hd] weighted values per key slot
+  Acc* all = part + DA_SLOTS * hd;           // CTA 0: [DA_CTAS][hd + 2] weighted values, maximum, sum of every CTA
   __shared__ Acc red[32];
   cg::cluster_group cluster = cg::this_cluster();
+  pdl_trigger();
+  cluster.sync();  // CTA 0 has started: its shared memory may be written
   const int rank = (int)(blockIdx.x % DA_CTAS), h = (int)(blockIdx.x / DA_CTAS);
+  const T* base = qkv + (long long)h * hd;
+  const int sub = threadIdx.x & 7, slot = threadIdx.x >> 3;
+  constexpr int PN = Pack<T>::N;
+  const bool vec = hd % PN == 0 && channels % PN == 0 && ld % PN == 0;
+  pdl_wait();
   const long long t = *pos;
   const int keys = (int)t + 1, chunk = (keys + DA_CTAS - 1) / DA_CTAS;
   const int k0 = min(keys, rank * chunk), k1 = min(keys, k0 + chunk);
-  const T* base = qkv + (long long)h * hd;
-  const Acc scale = (Acc)1 / sqrt((Acc)hd);
-  for (int c = threadIdx.x; c < hd; c += DA_THREADS) { q[c] = (Acc)as_f32(base[t * ld + c]); o[c] = 0; }
+  for (int c = threadIdx.x; c < hd; c += DA_THREADS) q[c] = (Acc)as_f32(base[t * ld + c]);
   __syncthreads();
-  // eight lanes per key
-  const int sub = threadIdx.x & 7, who = threadIdx.x >> 3;
+  const Acc scale = (Acc)1 / sqrt((Acc)hd);
   Acc mx = -INFINITY;
-  for (int key = k0 + who; key - who < k1; key += DA_THREADS / 8) {
+#pragma unroll 4
+  for (int key = k0 + slot; key - slot < k1; key += DA_SLOTS) {
     Acc dot = 0;
     if (key < k1) {
       const T* kr = base + channels + (long long)key * ld;
-      for (int c = sub; c < hd; c += 8) dot += q[c] * (Acc)as_f32(kr[c]);
+      if (vec) {
+        for (int c = sub * PN; c < hd; c += 8 * PN) {
+          float kv[PN];
+          Pack<T>::unpack(*reinterpret_cast<const uint4*>(kr + c), kv);
+#pragma unroll
+          for (int e = 0; e < PN; ++e) dot += q[c + e] * (Acc)kv[e];
+        }
+      } else {
+        for (int c = sub; c < hd; c += 8) dot += q[c] * (Acc)as_f32(kr[c]);
+      }
     }
     dot += __shfl_xor_sync(0xffffffffu, dot, 1);
     dot += __shfl_xor_sync(0xffffffffu, dot, 2);
@@ -170,50 +261,64 @@ decode_attention_kernel(const T* __restrict__ qkv, long long ld, int channels, c
     sum += e;
   }
   sum = block_sum(sum, red);
-  __syncthreads();
-  // channels across the threads; heads narrower than the block split the keys over groups of threads
-  const int groups = max(1, DA_THREADS / hd);
-  for (int c0 = 0; c0 < hd; c0 += DA_THREADS) {
-    const int c = c0 + (groups > 1 ? (int)threadIdx.x % hd : (int)threadIdx.x), g = groups > 1 ? (int)threadIdx.x / hd : 0;
-    Acc acc = 0;
-    if (c < hd && g < groups) {
-      const T* vr = base + 2 * channels + c;
+  if (vec) {
+    for (int c = sub * PN; c < hd; c += 8 * PN) {
+      Acc acc[PN];
+#pragma unroll
+      for (int e = 0; e < PN; ++e) acc[e] = 0;
 #pragma unroll 4
-      for (int key = k0 + g; key < k1; key += groups) acc += s[key - k0] * (Acc)as_f32(vr[(long long)key * ld]);
+      for (int key = k0 + slot; key < k1; key += DA_SLOTS) {
+        float vv[PN];
+        Pack<T>::unpack(*reinterpret_cast<const uint4*>(base + 2 * channels + (long long)key * ld + c), vv);
+        const Acc w = s[key - k0];
+#pragma unroll
+        for (int e = 0; e < PN; ++e) acc[e] += w * (Acc)vv[e];
+      }
+#pragma unroll
+      for (int e = 0; e < PN; ++e) part[slot * hd + c + e] = acc[e];
     }
-    part[threadIdx.x] = acc;
-    __syncthreads();
-    if (c < hd && g == 0) {
-      for (int i = 1; i < groups; ++i) acc += part[threadIdx.x + i * hd];
-      o[c] = acc;
+  } else {
+    for (int c = sub; c < hd; c += 8) {
+      Acc acc = 0;
+      for (int key = k0 + slot; key < k1; key += DA_SLOTS) acc += s[key - k0] * (Acc)as_f32(base[2 * channels + (long long)key * ld + c]);
+      part[slot * hd + c] = acc;
     }
-    __syncthreads();
   }
-  if (threadIdx.x == 0) { stat[0] = mx; stat[1] = sum; }
+  __syncthreads();
+  Acc* mine = cluster.map_shared_rank(all, 0) + rank * (hd + 2);
+  for (int c = threadIdx.x; c < hd; c += DA_THREADS) {
+    Acc v = 0;
+#pragma unroll
+    for (int i = 0; i < DA_SLOTS; ++i) v += part[i * hd + c];
+    mine[c] = v;
+  }
+  if (threadIdx.x == 0) { mine[hd] = mx; mine[hd + 1] = sum; }
   cluster.sync();
-  if (rank == 0) {
-    Acc m = -INFINITY, l = 0;
-    for (int r = 0; r < DA_CTAS; ++r) m = max(m, *cluster.map_shared_rank(&stat[0], r));
-    Acc f[DA_CTAS];
-    for (int r = 0; r < DA_CTAS; ++r) {
-      const Acc mr = *cluster.map_shared_rank(&stat[0], r);
-      f[r] = mr == (Acc)-INFINITY ? (Acc)0 : exp(mr - m);
-      l += f[r] * *cluster.map_shared_rank(&stat[1], r);
-    }
-    for (int c = threadIdx.x; c < hd; c += DA_THREADS) {
-      Acc v = 0;
-      for (int r = 0; r < DA_CTAS; ++r) v += f[r] * *cluster.map_shared_rank(o + c, r);
-      const float y = (float)(v / l);
-      if constexpr (sizeof(T) == 2) out[h * hd + c] = to_bf16(y); else out[h * hd + c] = y;
-    }
+  if (rank != 0) return;
+  Acc m = -INFINITY, l = 0, f[DA_CTAS];
+#pragma unroll
+  for (int r = 0; r < DA_CTAS; ++r) m = max(m, all[r * (hd + 2) + hd]);
+#pragma unroll
+  for (int r = 0; r < DA_CTAS; ++r) {
+    const Acc mr = all[r * (hd + 2) + hd];
+    f[r] = mr == (Acc)-INFINITY ? (Acc)0 : exp(mr - m);
+    l += f[r] * all[r * (hd + 2) + hd + 1];
   }
-  cluster.sync();  // no CTA leaves while CTA 0 reads its shared memory
+  for (int c = threadIdx.x; c < hd; c += DA_THREADS) {
+    Acc v = 0;
+#pragma unroll
+    for (int r = 0; r < DA_CTAS; ++r) v += f[r] * all[r * (hd + 2) + c];
+    const float y = (float)(v / l);
+    if constexpr (sizeof(T) == 2) out[h * hd + c] = to_bf16(y); else out[h * hd + c] = y;
+  }
 }
 
 // The embedding row of the state's token at the state's position.
 template <typename T>
 __global__ void decode_embed_kernel(const float* __restrict__ table, const float* __restrict__ positions,
                                     const long long* __restrict__ state /* position, token */, T* __restrict__ out, int dim) {
+  pdl_trigger();
+  pdl_wait();
   const float* a = table + state[1] * dim;
   const float* b = positions + state[0] * dim;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < dim; c += gridDim.x * blockDim.x) {
@@ -224,17 +329,9 @@ __global__ void decode_embed_kernel(const float* __restrict__ table, const float
 
 template <typename WT, typename XT, typename OT, typename Acc>
 int launch_gemv(hl_ctx* ctx, const GemvArgs& a) {
-  const size_t smem = sizeof(float) * (size_t)a.k;
-  auto kern = decode_gemv_kernel<WT, XT, OT, Acc>;
-  static bool configured = false;
-  if (!configured) {
-    HL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecodeMaxRow * (int)sizeof(float)));
-    configured = true;
-  }
-  // every output its own warp up to eight CTAs per SM; the vocabulary's rows are walked by those
-  const int grid = std::min(ceil_div(a.n, GV_WARPS), ctx->sm_count * 8);
-  kern<<<grid, GV_THREADS, smem, ctx->stream>>>(a);
-  HL_LAUNCH_CHECK("decode_gemv_kernel");
+  // every output its own warp (or its share of one) up to eight CTAs per SM; the vocabulary's rows are walked by those
+  const int grid = std::min(ceil_div(a.n, GV_WARPS / a.warps_per_row), ctx->sm_count * 8);
+  HL_CUDA(launch_pdl(decode_gemv_kernel<WT, XT, OT, Acc>, grid, GV_THREADS, 0, ctx->stream, 1, a));
   count_launch(ctx);
   return HL_OK;
 }
@@ -242,10 +339,13 @@ int launch_gemv(hl_ctx* ctx, const GemvArgs& a) {
 }  // namespace
 
 int decode_gemv(hl_ctx* ctx, const DecodeGemv& g) {
-  HL_REQUIRE(g.k <= kDecodeMaxRow, "decode_gemv: input row too long");
-  GemvArgs a{g.x, g.gamma, g.beta, g.w, g.bias, g.residual, g.out, g.out_row, g.ld_out, g.n, g.k, g.epilogue, false};
+  GemvArgs a{g.x, g.gamma, g.beta, g.w, g.bias, g.residual, g.out, g.out_row, g.ld_out, g.n, g.k, g.epilogue, 1, false};
   const int per16 = g.w_dtype == HL_BF16 ? 8 : 4;
-  a.vec = g.k % per16 == 0 && (reinterpret_cast<uintptr_t>(g.w) & 15) == 0;
+  a.vec = g.k % per16 == 0 && ((reinterpret_cast<uintptr_t>(g.w) | reinterpret_cast<uintptr_t>(g.x)) & 15) == 0;
+  HL_REQUIRE(!g.gamma || (a.vec && g.k <= GV_SPAN && (reinterpret_cast<uintptr_t>(g.gamma) & 15) == 0 &&
+                          (reinterpret_cast<uintptr_t>(g.beta) & 15) == 0),
+             "decode_gemv: a layer norm takes rows of up to 1024 elements on 16-byte boundaries");
+  while (a.warps_per_row < GV_WARPS && a.warps_per_row * GV_SPAN < g.k) a.warps_per_row *= 2;
   if (g.w_dtype == HL_BF16)
     return g.out_dtype == HL_BF16 ? launch_gemv<__nv_bfloat16, __nv_bfloat16, __nv_bfloat16, float>(ctx, a)
                                   : launch_gemv<__nv_bfloat16, __nv_bfloat16, float, float>(ctx, a);
@@ -256,39 +356,29 @@ int decode_gemv(hl_ctx* ctx, const DecodeGemv& g) {
 
 size_t decode_attention_smem(int dtype, int hd, int context) {
   const size_t acc = dtype == HL_BF16 ? 4 : 8;
-  return acc * (2 * (size_t)hd + (size_t)ceil_div(context, DA_CTAS) + DA_THREADS);
+  return acc * ((size_t)hd + (size_t)ceil_div(context, DA_CTAS) + (size_t)DA_SLOTS * hd + (size_t)DA_CTAS * (hd + 2));
 }
 
 int decode_attention(hl_ctx* ctx, const void* qkv, int dtype, long long ld, const long long* pos, void* out, int channels,
                      int n_heads, int context) {
   const int hd = channels / n_heads, cap = ceil_div(context, DA_CTAS);
   const size_t smem = decode_attention_smem(dtype, hd, context);
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(n_heads * DA_CTAS));
-  cfg.blockDim = dim3(DA_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = ctx->stream;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = DA_CTAS; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
   if (dtype == HL_BF16)
-    HL_CUDA(cudaLaunchKernelEx(&cfg, decode_attention_kernel<__nv_bfloat16, float>, (const __nv_bfloat16*)qkv, ld, channels, pos,
-                               (__nv_bfloat16*)out, hd, cap));
+    HL_CUDA(launch_pdl(decode_attention_kernel<__nv_bfloat16, float>, n_heads * DA_CTAS, DA_THREADS, smem, ctx->stream, DA_CTAS,
+                       (const __nv_bfloat16*)qkv, ld, channels, pos, (__nv_bfloat16*)out, hd, cap));
   else
-    HL_CUDA(cudaLaunchKernelEx(&cfg, decode_attention_kernel<float, double>, (const float*)qkv, ld, channels, pos, (float*)out, hd,
-                               cap));
-  HL_LAUNCH_CHECK("decode_attention_kernel");
+    HL_CUDA(launch_pdl(decode_attention_kernel<float, double>, n_heads * DA_CTAS, DA_THREADS, smem, ctx->stream, DA_CTAS,
+                       (const float*)qkv, ld, channels, pos, (float*)out, hd, cap));
   count_launch(ctx);
   return HL_OK;
 }
 
 int decode_embed(hl_ctx* ctx, const float* table, const float* positions, const long long* state, void* out, int dtype, int dim) {
   const int grid = ceil_div(dim, 256);
-  if (dtype == HL_BF16) decode_embed_kernel<<<grid, 256, 0, ctx->stream>>>(table, positions, state, (__nv_bfloat16*)out, dim);
-  else decode_embed_kernel<<<grid, 256, 0, ctx->stream>>>(table, positions, state, (float*)out, dim);
-  HL_LAUNCH_CHECK("decode_embed_kernel");
+  if (dtype == HL_BF16)
+    HL_CUDA(launch_pdl(decode_embed_kernel<__nv_bfloat16>, grid, 256, 0, ctx->stream, 1, table, positions, state, (__nv_bfloat16*)out, dim));
+  else
+    HL_CUDA(launch_pdl(decode_embed_kernel<float>, grid, 256, 0, ctx->stream, 1, table, positions, state, (float*)out, dim));
   count_launch(ctx);
   return HL_OK;
 }

@@ -99,7 +99,6 @@ int attention_f64_backward(hl_ctx* ctx, const void* q, const void* k, const void
 
 // One-token steps (decode.cu).  out[n] = epilogue(W[n,k] · x + bias), with a layer norm of x first when gamma is given.
 enum { GV_STORE = 0, GV_GELU = 1, GV_RESIDUAL = 2 };
-constexpr int kDecodeMaxRow = 24576;  // longest input row, f32 in shared memory
 struct DecodeGemv {
   const void* x;
   int x_dtype;

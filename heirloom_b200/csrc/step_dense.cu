@@ -1086,8 +1086,7 @@ int decode_step(hl_decoder* m) {
 bool decode_applicable(const hl_decoder* m) {
   const hl_decoder_config& c = m->cfg;
   const int dt = c.precision == HL_PRECISION_AMP_BF16 ? HL_BF16 : HL_F32;
-  return c.d_ff <= kDecodeMaxRow && decode_attention_smem(dt, c.d_model / c.n_heads, c.context) <= 48 * 1024 &&
-         (!m->has_memory || m->mem.value_dim <= kDecodeMaxRow);
+  return decode_attention_smem(dt, c.d_model / c.n_heads, c.context) <= 48 * 1024;
 }
 
 int ensure_logits_host(hl_decoder* m) {
@@ -1744,7 +1743,6 @@ static int window_logits(hl_decoder* m, const int64_t* window, cudaMemcpyKind ki
   HL_CUDA(cudaMemcpyAsync(m->tokens, window, sizeof(int64_t) * window_len, kind, ctx->stream));
   {
     ScopedShape shape(m, 1, window_len);
-    // a final row too long for the matrix-vector kernel's shared memory cannot happen: d_model is at most 1024
     if (m->cfg.precision == HL_PRECISION_AMP_BF16) HL_TRY(forward(m, true));
     else HL_TRY(forward_f32(m, true));
   }
