@@ -18,8 +18,16 @@ struct AdamChunk {
   unsigned int n;
 };
 
-constexpr unsigned int ADAM_CHUNK = 16384;  // elements per block
 constexpr int ADAM_THREADS = 256;
+// Elements per block.  Large sets take 16384, which reaches the copy rate (760 us for 163 M parameters); a set that would
+// then fill less than four blocks per SM is cut finer, down to one 16-byte access per thread and operand: a small model's
+// 0.4 M parameters in 25 blocks of sixteen dependent rounds took 17 us, in 415 blocks of one round 3.
+constexpr unsigned int ADAM_CHUNK_MAX = 16384, ADAM_CHUNK_MIN = ADAM_THREADS * 4;
+unsigned int adam_chunk_for(unsigned long long elements, int sm_count) {
+  unsigned int chunk = ADAM_CHUNK_MAX;
+  while (chunk > ADAM_CHUNK_MIN && elements / chunk < 4ull * (unsigned)sm_count) chunk /= 2;
+  return chunk;
+}
 
 // Separately rounded multiply/add/divide/sqrt: identical bits to the reference kernel, which
 // has no fused multiply-add.
@@ -85,6 +93,7 @@ int validate(const hl_adamw_params* hp, const char* who) {
 struct AdamPlan {
   AdamChunk* chunks_dev = nullptr;
   int count = 0;
+  unsigned int chunk = ADAM_CHUNK_MAX;
   unsigned long long elements = 0;
 };
 
@@ -92,6 +101,8 @@ int adam_plan_create(hl_ctx* ctx, const hl_adamw_tensor* tensors, int count, Ada
   HL_REQUIRE(ctx && tensors && out && count > 0, "adamw plan: null or empty argument");
   std::vector<AdamChunk> chunks;
   unsigned long long elements_total = 0;
+  for (int t = 0; t < count; ++t) elements_total += tensors[t].n;
+  const unsigned int chunk = adam_chunk_for(elements_total, ctx->sm_count);
   for (int t = 0; t < count; ++t) {
     const hl_adamw_tensor& x = tensors[t];
     HL_REQUIRE(x.param && x.grad && x.m && x.v, "adamw plan: null tensor pointer");
@@ -100,18 +111,18 @@ int adam_plan_create(hl_ctx* ctx, const hl_adamw_tensor* tensors, int count, Ada
                "adamw plan: tensors must be 16-byte aligned");
     HL_REQUIRE(!x.shadow_bf16 || (reinterpret_cast<uintptr_t>(x.shadow_bf16) & 7) == 0,
                "adamw plan: bf16 shadow must be 8-byte aligned");
-    for (uint64_t off = 0; off < x.n; off += ADAM_CHUNK) {
+    for (uint64_t off = 0; off < x.n; off += chunk) {
       AdamChunk c;
       c.param = x.param + off; c.grad = x.grad + off; c.m = x.m + off; c.v = x.v + off;
       c.shadow = x.shadow_bf16 ? reinterpret_cast<__nv_bfloat16*>(x.shadow_bf16) + off : nullptr;
-      c.n = (unsigned int)std::min<uint64_t>(ADAM_CHUNK, x.n - off);
+      c.n = (unsigned int)std::min<uint64_t>(chunk, x.n - off);
       chunks.push_back(c);
     }
-    elements_total += x.n;
   }
   AdamPlan* plan = new AdamPlan();
   plan->count = (int)chunks.size();
   plan->elements = elements_total;
+  plan->chunk = chunk;
   if (plan->count > 0) {
     cudaError_t e = cudaMalloc(&plan->chunks_dev, sizeof(AdamChunk) * chunks.size());
     if (e != cudaSuccess) { delete plan; return fail_cuda(e, "cudaMalloc(adamw chunk table)"); }
@@ -130,7 +141,7 @@ void adam_plan_destroy(AdamPlan* plan) {
   delete plan;
 }
 
-int adam_plan_chunk_elements() { return (int)ADAM_CHUNK; }
+int adam_plan_chunk_elements(const AdamPlan* plan) { return (int)plan->chunk; }
 int adam_plan_chunk_count(const AdamPlan* plan) { return plan->count; }
 
 // Chunks [first, first + count) of the table: lets a caller update the part of a gradient arena whose

@@ -1158,7 +1158,7 @@ int optimizer_step(hl_decoder* m) {
   if (!m->comm_pending) return adam_plan_step(ctx, m->plan, &hp);
   // Collectives still in flight: update the arena in groups of buckets, each group as soon as its last
   // all-reduce has finished, so the update of the early buckets overlaps the reduction of the late ones.
-  const size_t chunk = (size_t)adam_plan_chunk_elements();
+  const size_t chunk = (size_t)adam_plan_chunk_elements(m->plan);
   const int chunks_total = adam_plan_chunk_count(m->plan);
   constexpr size_t kGroup = 5;  // buckets per launch
   int first = 0;
