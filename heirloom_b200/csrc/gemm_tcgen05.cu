@@ -754,6 +754,15 @@ bool pairs_enabled(const hl_gemm_desc* d) {
          (d->epilogue == HL_EPI_BIAS || d->epilogue == HL_EPI_BIAS_GELU);
 }
 
+// The small-product kernel decides for itself which products it takes, unless the caller asks for a work split or one of the
+// persistent kernel's forms is forced.
+GemmSmallPlan small_plan(const hl_ctx* ctx, const hl_gemm_desc* d, const GemmPlan& plan, int sms) {
+  auto forced = [](const char* name) { const char* e = getenv(name); return e && e[0] == '1'; };
+  if (d->split_k > 0 || ctx->gemm_skip_kblock >= 0 || forced("HEIRLOOM_GEMM_PAIRS") || forced("HEIRLOOM_GEMM_DYNAMIC"))
+    return GemmSmallPlan{0, 0, false};
+  return gemm_small_plan(d, plan, sms);
+}
+
 }  // namespace
 
 constexpr int kMinDealtKBlocks = 192;  // contraction of 12288 and up
@@ -850,6 +859,8 @@ int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void*
 
   const int sms = persistent_sms(ctx);
   const GemmPlan plan = gemm_plan(d, sms);
+  const GemmSmallPlan small = small_plan(ctx, d, plan, sms);
+  if (small.splits > 0) return gemm_small_run(ctx, d, small, a, b, c, bias, aux_in, aux_out);
   // Whole tiles (of the whole contraction or of equal splits of it; not the dealt-out k blocks) can run on CTA pairs
   // with 256-row tiles.  Measured on alternating calls: 6-7 % faster where the main loop bounds the tile (contractions
   // of 2304 and up), 6-10 % slower at 768, where the epilogue does and the leader waits for both CTAs' epilogue warps.
@@ -995,7 +1006,9 @@ int gemm_bf16_ctx(hl_ctx* ctx, const hl_gemm_desc* desc, const void* a, const vo
                   const void* aux_in, void* aux_out) {
   if (!ctx || !desc) return fail("hl_gemm_bf16: null argument");
   if (desc->m <= 0 || desc->n <= 0 || desc->k <= 0) return fail("hl_gemm_bf16: m, n, k must be positive");
-  const GemmPlan plan = gemm_plan(desc, persistent_sms(ctx));
+  const int sms = persistent_sms(ctx);
+  GemmPlan plan = gemm_plan(desc, sms);
+  if (small_plan(ctx, desc, plan, sms).splits > 0) plan = GemmPlan{1, 0, 0, 0, 0};  // no scratch
   const size_t need = std::max(plan.splitk_bytes, plan.sk_slot_bytes);
   if (need > ctx->workspace_bytes) {
     int rc = ensure_workspace(ctx, need);

@@ -16,6 +16,15 @@ struct GemmPlan {
 GemmPlan gemm_plan(const hl_gemm_desc* d, int sm_count);
 int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, void* c, const float* bias,
                   const void* aux_in, void* aux_out, float* workspace, size_t workspace_bytes, unsigned* stream_flags);
+// Products that leave most of the chip idle in 128 x 256 tiles (gemm_small.cu): how many CTAs share the contraction of one of
+// its 128 x bn tiles (0: not one of them), and whether a CTA has the SM's shared memory to itself.
+struct GemmSmallPlan {
+  int splits, bn;
+  bool deep;
+};
+GemmSmallPlan gemm_small_plan(const hl_gemm_desc* d, const GemmPlan& big, int sm_count);
+int gemm_small_run(hl_ctx* ctx, const hl_gemm_desc* d, const GemmSmallPlan& plan, const void* a, const void* b, void* c,
+                   const float* bias, const void* aux_in, void* aux_out);
 // The GEMM with its scratch taken from (and grown in) the context.
 int gemm_bf16_ctx(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, void* c, const float* bias,
                   const void* aux_in, void* aux_out);
