@@ -164,6 +164,7 @@ flash_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   const uint32_t tmem_dv = tmem_s + 256;    // 64 columns (one channel block of the head)
   const uint32_t tmem_dk = tmem_s + 320;    // 64 columns
   const uint32_t tmem_dq = tmem_s + 384;    // two buffers of 64 columns, alternating by query tile
+  pdl_begin();  // everything above touches nothing a predecessor wrote
 
   FbCursor first;
   fb_load_item(first, 0, p);
@@ -514,6 +515,7 @@ flash_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
 __global__ void __launch_bounds__(256)
 attention_delta_kernel(const __nv_bfloat16* __restrict__ out, long long ld_out, const __nv_bfloat16* __restrict__ dout,
                        long long ld_dout, float* __restrict__ delta, int B, int T, int H, int hd) {
+  pdl_begin();
   const long long pair = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 3;  // (row, head)
   const int part = threadIdx.x & 7;
   const bool in = pair < (long long)B * T * H;
@@ -538,6 +540,7 @@ attention_delta_kernel(const __nv_bfloat16* __restrict__ out, long long ld_out, 
 
 __global__ void dq_to_bf16_kernel(const float* __restrict__ acc, long long ld_acc, __nv_bfloat16* __restrict__ dq,
                                   long long ld_dq, long long rows, int cols) {
+  pdl_begin();
   const long long quads = rows * (cols / 4);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < quads; i += (long long)gridDim.x * blockDim.x) {
     const long long row = i / (cols / 4);
@@ -579,7 +582,7 @@ int flash_attention_backward_impl(hl_ctx* ctx, const void* q, const void* k, con
   HL_CUDA(cudaMemsetAsync(dq_accum, 0, sizeof(float) * rows * C, ctx->stream));
   {
     const long long pairs = (long long)rows * n_heads;
-    attention_delta_kernel<<<(unsigned)ceil_div_ll(pairs * 8, 256), 256, 0, ctx->stream>>>(
+    pdl(attention_delta_kernel, (unsigned)ceil_div_ll(pairs * 8, 256), 256, 0, ctx->stream)(
         reinterpret_cast<const __nv_bfloat16*>(out), ld_out, reinterpret_cast<const __nv_bfloat16*>(dout), ld_dout,
         delta, batch, time, n_heads, head_dim);
     HL_LAUNCH_CHECK("attention_delta_kernel");
@@ -628,20 +631,20 @@ int flash_attention_backward_impl(hl_ctx* ctx, const void* q, const void* k, con
       HL_CUDA(cudaFuncSetAttribute(flash_attention_bwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, FbSizes<64>::SMEM_BYTES));
       configured = true;
     }
-    flash_attention_bwd_kernel<64><<<grid, FB_THREADS, FbSizes<64>::SMEM_BYTES, ctx->stream>>>(mq, mk, mv, mdo, mdq, mdk, mdv, p);
+    pdl(flash_attention_bwd_kernel<64>, grid, FB_THREADS, FbSizes<64>::SMEM_BYTES, ctx->stream)(mq, mk, mv, mdo, mdq, mdk, mdv, p);
   } else {
     static bool configured = false;
     if (!configured) {
       HL_CUDA(cudaFuncSetAttribute(flash_attention_bwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, FbSizes<128>::SMEM_BYTES));
       configured = true;
     }
-    flash_attention_bwd_kernel<128><<<grid, FB_THREADS, FbSizes<128>::SMEM_BYTES, ctx->stream>>>(mq, mk, mv, mdo, mdq, mdk, mdv, p);
+    pdl(flash_attention_bwd_kernel<128>, grid, FB_THREADS, FbSizes<128>::SMEM_BYTES, ctx->stream)(mq, mk, mv, mdo, mdq, mdk, mdv, p);
   }
   HL_LAUNCH_CHECK("flash_attention_bwd_kernel");
   {
     const long long quads = (long long)rows * (C / 4);
     const long long want = ceil_div_ll(quads, 256), cap = (long long)ctx->sm_count * 8;
-    dq_to_bf16_kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, ctx->stream>>>(
+    pdl(dq_to_bf16_kernel, (unsigned)(want < cap ? want : cap), 256, 0, ctx->stream)(
         dq_accum, C, reinterpret_cast<__nv_bfloat16*>(dq), ld_dqkv, (long long)rows, (int)C);
     HL_LAUNCH_CHECK("dq_to_bf16_kernel");
   }

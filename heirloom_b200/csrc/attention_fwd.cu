@@ -122,6 +122,7 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   tc05::tc_fence_after_sync();
   const uint32_t tmem_s0 = sh->tmem_base;         // S buffers at +0 and +64
   const uint32_t tmem_o0 = tmem_s0 + 2 * FA_BN;   // O at +128
+  pdl_begin();  // everything above touches nothing a predecessor wrote
 
   if (warp == FA_SOFTMAX_WARPS) {
     // -------------------------------------------------------------------------- TMA producer
@@ -380,14 +381,14 @@ int flash_attention_forward_impl(hl_ctx* ctx, const void* q, const void* k, cons
       HL_CUDA(cudaFuncSetAttribute(flash_attention_fwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, FaSizes<64>::SMEM_BYTES));
       configured = true;
     }
-    flash_attention_fwd_kernel<64><<<nq * batch * n_heads, FA_THREADS, FaSizes<64>::SMEM_BYTES, ctx->stream>>>(mq, mk, mv, mo, p);
+    pdl(flash_attention_fwd_kernel<64>, nq * batch * n_heads, FA_THREADS, FaSizes<64>::SMEM_BYTES, ctx->stream)(mq, mk, mv, mo, p);
   } else {
     static bool configured = false;
     if (!configured) {
       HL_CUDA(cudaFuncSetAttribute(flash_attention_fwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, FaSizes<128>::SMEM_BYTES));
       configured = true;
     }
-    flash_attention_fwd_kernel<128><<<nq * batch * n_heads, FA_THREADS, FaSizes<128>::SMEM_BYTES, ctx->stream>>>(mq, mk, mv, mo, p);
+    pdl(flash_attention_fwd_kernel<128>, nq * batch * n_heads, FA_THREADS, FaSizes<128>::SMEM_BYTES, ctx->stream)(mq, mk, mv, mo, p);
   }
   HL_LAUNCH_CHECK("flash_attention_fwd_kernel");
   count_launch(ctx);

@@ -81,6 +81,12 @@ namespace hl {
 // because each of them waited too before it finished.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// For a kernel without set-up worth overlapping.  An early trigger does not take SMs from the kernel itself: its dependents
+// come in only when all of its own blocks have started.
+__device__ __forceinline__ void pdl_begin() {
+  pdl_trigger();
+  pdl_wait();
+}
 template <typename... P, typename... A>
 cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, A&&... args) {
   cudaLaunchConfig_t cfg{};
@@ -96,6 +102,21 @@ cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
   cfg.attrs = attr;
   cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
+// pdl(kernel, grid, block, shared memory, stream)(arguments): the launch above in place of <<< >>>, errors through
+// cudaGetLastError like there.
+template <typename... P>
+struct PdlLauncher {
+  void (*kernel)(P...);
+  dim3 grid, block;
+  size_t smem;
+  cudaStream_t stream;
+  void operator()(P... args) const { launch_pdl(kernel, grid, block, smem, stream, 1, args...); }
+};
+template <typename... P>
+PdlLauncher<P...> pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream) {
+  return PdlLauncher<P...>{kernel, grid, block, smem, stream};
 }
 
 int ensure_workspace(hl_ctx* ctx, size_t bytes);

@@ -26,6 +26,7 @@ struct OpDiv { __device__ float operator()(float a, float b) const { return a / 
 template <typename Op>
 __global__ void binary_f32_kernel(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out,
                                   size_t n, bool vec) {
+  pdl_begin();
   Op op;
   const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
   if (vec) {
@@ -44,6 +45,7 @@ __global__ void binary_f32_kernel(const float* __restrict__ a, const float* __re
 template <typename F>
 __global__ void map_f32_kernel(const float* __restrict__ x, const float* __restrict__ y, float* __restrict__ out,
                                size_t n, bool vec, F f) {
+  pdl_begin();
   const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
   if (vec) {
     const size_t n4 = n / 4;
@@ -62,6 +64,7 @@ __global__ void map_f32_kernel(const float* __restrict__ x, const float* __restr
 template <typename F>
 __global__ void map_bf16_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ y,
                                 __nv_bfloat16* __restrict__ out, size_t n, bool vec, F f) {
+  pdl_begin();
   const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
   if (vec) {
     const size_t n8 = n / 8;
@@ -86,6 +89,7 @@ __global__ void map_bf16_kernel(const __nv_bfloat16* __restrict__ x, const __nv_
 
 __global__ void cast_f32_to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, size_t n,
                                         bool vec) {
+  pdl_begin();
   const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
   if (vec) {
     const size_t n8 = n / 8;
@@ -102,6 +106,7 @@ __global__ void cast_f32_to_bf16_kernel(const float* __restrict__ src, __nv_bflo
 
 __global__ void cast_bf16_to_f32_kernel(const __nv_bfloat16* __restrict__ src, float* __restrict__ dst, size_t n,
                                         bool vec) {
+  pdl_begin();
   const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
   if (vec) {
     const size_t n8 = n / 8;
@@ -119,6 +124,7 @@ __global__ void cast_bf16_to_f32_kernel(const __nv_bfloat16* __restrict__ src, f
 
 __global__ void bias_add_f32_kernel(const float* __restrict__ x, const float* __restrict__ bias, float* __restrict__ out,
                                     size_t total, int cols) {
+  pdl_begin();
   const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = tid; i < total; i += stride) out[i] = x[i] + bias[i % cols];
 }
@@ -128,6 +134,7 @@ __global__ void bias_add_f32_kernel(const float* __restrict__ x, const float* __
 template <typename T>
 __global__ void colsum_partial_kernel(const T* __restrict__ g, double* __restrict__ partial, int rows, int cols,
                                       int rows_per_block) {
+  pdl_begin();
   __shared__ double tile[8][33];
   const int col = blockIdx.x * 32 + threadIdx.x;
   const int r0 = blockIdx.y * rows_per_block;
@@ -152,6 +159,7 @@ __global__ void colsum_partial_kernel(const T* __restrict__ g, double* __restric
 }
 
 __global__ void colsum_final_kernel(const double* __restrict__ partial, float* __restrict__ out, int cols, int slabs) {
+  pdl_begin();
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= cols) return;
   double s = 0.0;
@@ -175,6 +183,7 @@ __device__ __forceinline__ double widen_f32(float x) {
 template <int MODE>  // 0 sum, 1 sum of squares
 __global__ void __launch_bounds__(256)
 reduce_partial_kernel(const float* __restrict__ x, size_t n, bool vec, double* __restrict__ partial) {
+  pdl_begin();
   __shared__ double sm[32];
   double acc = 0.0;
   const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
@@ -198,6 +207,7 @@ reduce_partial_kernel(const float* __restrict__ x, size_t n, bool vec, double* _
 }
 
 __global__ void reduce_final_kernel(const double* __restrict__ partial, int count, double scale, float* __restrict__ out) {
+  pdl_begin();
   __shared__ double sm[32];
   double acc = 0.0;
   for (int i = threadIdx.x; i < count; i += blockDim.x) acc += partial[i];
@@ -212,10 +222,10 @@ int reduce_impl(hl_ctx* ctx, const float* x, size_t n, float* out_dev, int mode,
   int rc = ensure_workspace(ctx, sizeof(double) * blocks);
   if (rc != HL_OK) return rc;
   double* partial = reinterpret_cast<double*>(ctx->workspace);
-  if (mode == 1) reduce_partial_kernel<1><<<blocks, 256, 0, ctx->stream>>>(x, n, vec, partial);
-  else reduce_partial_kernel<0><<<blocks, 256, 0, ctx->stream>>>(x, n, vec, partial);
+  if (mode == 1) pdl(reduce_partial_kernel<1>, blocks, 256, 0, ctx->stream)(x, n, vec, partial);
+  else pdl(reduce_partial_kernel<0>, blocks, 256, 0, ctx->stream)(x, n, vec, partial);
   HL_LAUNCH_CHECK("reduce_partial_kernel");
-  reduce_final_kernel<<<1, 256, 0, ctx->stream>>>(partial, blocks, scale, out_dev);
+  pdl(reduce_final_kernel, 1, 256, 0, ctx->stream)(partial, blocks, scale, out_dev);
   HL_LAUNCH_CHECK("reduce_final_kernel");
   count_launch(ctx, 2);
   return HL_OK;
@@ -237,13 +247,13 @@ int bias_grad_impl(hl_ctx* ctx, const void* grad_out, int dtype, float* grad_bia
   double* partial = reinterpret_cast<double*>(ctx->workspace);
   dim3 grid(ceil_div(cols, 32), slabs), block(32, 8);
   if (dtype == HL_BF16)
-    colsum_partial_kernel<__nv_bfloat16><<<grid, block, 0, ctx->stream>>>(
+    pdl(colsum_partial_kernel<__nv_bfloat16>, grid, block, 0, ctx->stream)(
         reinterpret_cast<const __nv_bfloat16*>(grad_out), partial, rows, cols, rows_per_block);
   else
-    colsum_partial_kernel<float><<<grid, block, 0, ctx->stream>>>(reinterpret_cast<const float*>(grad_out), partial,
+    pdl(colsum_partial_kernel<float>, grid, block, 0, ctx->stream)(reinterpret_cast<const float*>(grad_out), partial,
                                                                     rows, cols, rows_per_block);
   HL_LAUNCH_CHECK("colsum_partial_kernel");
-  colsum_final_kernel<<<ceil_div(cols, 256), 256, 0, ctx->stream>>>(partial, grad_bias, cols, slabs);
+  pdl(colsum_final_kernel, ceil_div(cols, 256), 256, 0, ctx->stream)(partial, grad_bias, cols, slabs);
   HL_LAUNCH_CHECK("colsum_final_kernel");
   count_launch(ctx, 2);
   return HL_OK;
@@ -261,10 +271,10 @@ int hl_binary_f32(hl_ctx* ctx, int op, const float* a, const float* b, float* ou
   const bool vec = aligned16(a) && aligned16(b) && aligned16(out);
   const int grid = ew_grid(ctx, vec ? n / 4 + 1 : n);
   switch (op) {
-    case HL_ADD: binary_f32_kernel<OpAdd><<<grid, EW_THREADS, 0, ctx->stream>>>(a, b, out, n, vec); break;
-    case HL_SUB: binary_f32_kernel<OpSub><<<grid, EW_THREADS, 0, ctx->stream>>>(a, b, out, n, vec); break;
-    case HL_MUL: binary_f32_kernel<OpMul><<<grid, EW_THREADS, 0, ctx->stream>>>(a, b, out, n, vec); break;
-    case HL_DIV: binary_f32_kernel<OpDiv><<<grid, EW_THREADS, 0, ctx->stream>>>(a, b, out, n, vec); break;
+    case HL_ADD: pdl(binary_f32_kernel<OpAdd>, grid, EW_THREADS, 0, ctx->stream)(a, b, out, n, vec); break;
+    case HL_SUB: pdl(binary_f32_kernel<OpSub>, grid, EW_THREADS, 0, ctx->stream)(a, b, out, n, vec); break;
+    case HL_MUL: pdl(binary_f32_kernel<OpMul>, grid, EW_THREADS, 0, ctx->stream)(a, b, out, n, vec); break;
+    case HL_DIV: pdl(binary_f32_kernel<OpDiv>, grid, EW_THREADS, 0, ctx->stream)(a, b, out, n, vec); break;
     default: return fail("hl_binary_f32: unknown op");
   }
   HL_LAUNCH_CHECK("binary_f32_kernel");
@@ -296,14 +306,17 @@ int hl_fill_f32(hl_ctx* ctx, float* out, float value, size_t n) {
 
 // ---- plain SGD, index ranges and index concatenation ---------------------------------------------------------
 static __global__ void sgd_update_kernel(float* __restrict__ param, const float* __restrict__ grad, float lr, size_t n) {
+  pdl_begin();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     param[i] = __fsub_rn(param[i], __fmul_rn(lr, grad[i]));  // two roundings, as the reference's mul then sub
 }
 static __global__ void arange_i64_kernel(int64_t* __restrict__ out, size_t n) {
+  pdl_begin();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     out[i] = (int64_t)i;
 }
 static __global__ void copy_i64_kernel(const int64_t* __restrict__ src, int64_t* __restrict__ dst, size_t n) {
+  pdl_begin();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     dst[i] = src[i];
 }
@@ -312,7 +325,7 @@ int hl_sgd_update_f32(hl_ctx* ctx, float* param, const float* grad, float lr, si
   HL_REQUIRE(ctx && ((param && grad) || n == 0), "hl_sgd_update_f32: null argument");
   HL_REQUIRE(lr > 0.f, "sgd_update_f32_buffer learning rate must be positive, got " + std::to_string(lr));
   if (n == 0) return HL_OK;
-  sgd_update_kernel<<<ew_grid(ctx, n), EW_THREADS, 0, ctx->stream>>>(param, grad, lr, n);
+  pdl(sgd_update_kernel, ew_grid(ctx, n), EW_THREADS, 0, ctx->stream)(param, grad, lr, n);
   HL_LAUNCH_CHECK("sgd_update_kernel");
   count_launch(ctx);
   return HL_OK;
@@ -322,7 +335,7 @@ int hl_arange_i64(hl_ctx* ctx, int64_t* out, size_t n) {
   HL_REQUIRE(ctx && (out || n == 0), "hl_arange_i64: null argument");
   HL_REQUIRE(n <= 0xffffffffull, "i64_arange len exceeds the u32 launch limit");
   if (n == 0) return HL_OK;
-  arange_i64_kernel<<<ew_grid(ctx, n), EW_THREADS, 0, ctx->stream>>>(out, n);
+  pdl(arange_i64_kernel, ew_grid(ctx, n), EW_THREADS, 0, ctx->stream)(out, n);
   HL_LAUNCH_CHECK("arange_i64_kernel");
   count_launch(ctx);
   return HL_OK;
@@ -343,7 +356,7 @@ int hl_concat_i64(hl_ctx* ctx, const int64_t* const* inputs, const size_t* lengt
   size_t offset = 0;
   for (int i = 0; i < count; ++i) {
     if (lengths[i] == 0) continue;
-    copy_i64_kernel<<<ew_grid(ctx, lengths[i]), EW_THREADS, 0, ctx->stream>>>(inputs[i], out + offset, lengths[i]);
+    pdl(copy_i64_kernel, ew_grid(ctx, lengths[i]), EW_THREADS, 0, ctx->stream)(inputs[i], out + offset, lengths[i]);
     HL_LAUNCH_CHECK("copy_i64_kernel");
     count_launch(ctx);
     offset += lengths[i];
@@ -379,9 +392,9 @@ int hl_cast(hl_ctx* ctx, const void* src, int src_dtype, void* dst, int dst_dtyp
   const bool vec = aligned16(src) && aligned16(dst);
   const int grid = ew_grid(ctx, vec ? n / 8 + 1 : n);
   if (src_dtype == HL_F32 && dst_dtype == HL_BF16) {
-    cast_f32_to_bf16_kernel<<<grid, EW_THREADS, 0, ctx->stream>>>((const float*)src, (__nv_bfloat16*)dst, n, vec);
+    pdl(cast_f32_to_bf16_kernel, grid, EW_THREADS, 0, ctx->stream)((const float*)src, (__nv_bfloat16*)dst, n, vec);
   } else if (src_dtype == HL_BF16 && dst_dtype == HL_F32) {
-    cast_bf16_to_f32_kernel<<<grid, EW_THREADS, 0, ctx->stream>>>((const __nv_bfloat16*)src, (float*)dst, n, vec);
+    pdl(cast_bf16_to_f32_kernel, grid, EW_THREADS, 0, ctx->stream)((const __nv_bfloat16*)src, (float*)dst, n, vec);
   } else if (src_dtype == HL_F32 && dst_dtype == HL_F32) {
     map_f32_kernel<<<ew_grid(ctx, vec ? n / 4 + 1 : n), EW_THREADS, 0, ctx->stream>>>(
         (const float*)src, (const float*)nullptr, (float*)dst, n, vec,
@@ -398,6 +411,7 @@ int hl_cast(hl_ctx* ctx, const void* src, int src_dtype, void* dst, int dst_dtyp
 // differences are exact in f32, so hi + mid + lo == x whenever the three 8-bit mantissas reach the last bit of x.
 static __global__ void split_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long rows, int cols,
                                   int mode_bits) {
+  pdl_begin();
   const int mode = mode_bits & 3;
   const bool stacked = (mode_bits & HL_SPLIT_STACK_ROWS) != 0;
   const int pieces = mode == HL_SPLIT_HI_LO ? 2 : 3;
@@ -424,7 +438,7 @@ int hl_split_bf16_f32(hl_ctx* ctx, const float* src, void* dst, long long rows, 
   HL_REQUIRE(ctx && src && dst, "hl_split_bf16_f32: null argument");
   HL_REQUIRE(rows > 0 && cols > 0, "hl_split_bf16_f32: requires non-zero rows/cols");
   HL_REQUIRE((mode & ~(3 | HL_SPLIT_STACK_ROWS)) == 0 && (mode & 3) != 3, "hl_split_bf16_f32: unknown mode");
-  split_bf16_kernel<<<ew_grid(ctx, (size_t)rows * cols), EW_THREADS, 0, ctx->stream>>>(src, (__nv_bfloat16*)dst, rows, cols, mode);
+  pdl(split_bf16_kernel, ew_grid(ctx, (size_t)rows * cols), EW_THREADS, 0, ctx->stream)(src, (__nv_bfloat16*)dst, rows, cols, mode);
   HL_LAUNCH_CHECK("split_bf16_kernel");
   count_launch(ctx);
   return HL_OK;
@@ -476,7 +490,7 @@ int hl_bias_add_f32(hl_ctx* ctx, const float* x, const float* bias, float* out, 
   HL_REQUIRE(ctx && x && bias && out, "hl_bias_add_f32: null argument");
   HL_REQUIRE(rows > 0 && cols > 0, "hl_bias_add_f32: rows and cols must be positive");
   const size_t total = (size_t)rows * cols;
-  bias_add_f32_kernel<<<ew_grid(ctx, total), EW_THREADS, 0, ctx->stream>>>(x, bias, out, total, cols);
+  pdl(bias_add_f32_kernel, ew_grid(ctx, total), EW_THREADS, 0, ctx->stream)(x, bias, out, total, cols);
   HL_LAUNCH_CHECK("bias_add_f32_kernel");
   count_launch(ctx);
   return HL_OK;

@@ -42,6 +42,7 @@ __global__ void __launch_bounds__(ROW_WARPS * 32)
 ln_fwd_bf16_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
                    __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows,
                    int features, float eps) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int stride = gridDim.x * ROW_WARPS;
   int row = blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
@@ -113,6 +114,7 @@ ln_bwd_bf16_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
                    const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
                    const float* __restrict__ residual, float* __restrict__ dx_f32, __nv_bfloat16* __restrict__ dx_bf16,
                    float* __restrict__ partial, int rows, int features, int rows_per_block) {
+  pdl_begin();
   constexpr int GROUPS = LnBwdShape<WPR>::GROUPS;
   extern __shared__ float fold_smem[];  // [GROUPS][3][features]
   __shared__ float2 row_sums[2][GROUPS][WPR];
@@ -204,6 +206,7 @@ constexpr int FOLD_WARPS = 32;
 __global__ void __launch_bounds__(FOLD_WARPS * 32)
 fold_partials_kernel(const float* __restrict__ partial, int blocks, int total, float* __restrict__ o0,
                      float* __restrict__ o1, float* __restrict__ o2, int features) {
+  pdl_begin();
   __shared__ double acc[FOLD_WARPS][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
@@ -236,6 +239,7 @@ struct FoldJobs {
 };
 __global__ void __launch_bounds__(FOLD_WARPS * 32)
 fold_batch_kernel(const FoldJobs jobs) {
+  pdl_begin();
   __shared__ double acc[FOLD_WARPS][33];
   const FoldJob& j = jobs.job[blockIdx.y];
   if ((int)blockIdx.x * 32 >= j.total) return;
@@ -269,6 +273,7 @@ fold_batch_kernel(const FoldJobs jobs) {
 template <typename T, int VEC>
 __global__ void __launch_bounds__(ROW_WARPS * 32)
 colsum_vec_kernel(const T* __restrict__ g, float* __restrict__ partial, int rows, int cols, int rows_per_block) {
+  pdl_begin();
   __shared__ float fold[ROW_WARPS][32 * VEC + 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = (blockIdx.x * 32 + lane) * VEC;
@@ -327,7 +332,7 @@ int fold_batch_flush(hl_ctx* ctx, FoldBatch* batch) {
     jobs.job[i] = batch->jobs[i];
     widest = std::max(widest, batch->jobs[i].total);
   }
-  fold_batch_kernel<<<dim3(ceil_div(widest, 32), batch->n), FOLD_WARPS * 32, 0, ctx->stream>>>(jobs);
+  pdl(fold_batch_kernel, dim3(ceil_div(widest, 32), batch->n), FOLD_WARPS * 32, 0, ctx->stream)(jobs);
   HL_LAUNCH_CHECK("fold_batch_kernel");
   count_launch(ctx);
   batch->n = 0;
@@ -345,7 +350,7 @@ int layer_norm_forward_fast(hl_ctx* ctx, const void* x, const float* gamma, cons
   const int grid = std::min(ceil_div(rows, ROW_WARPS), ctx->sm_count * 8);
   const int J = ceil_div(features, 256);
 #define HL_LAUNCH(JJ)                                                                                          \
-  ln_fwd_bf16_kernel<JJ><<<grid, ROW_WARPS * 32, 0, ctx->stream>>>((const __nv_bfloat16*)x, gamma, beta,       \
+  pdl(ln_fwd_bf16_kernel<JJ>, grid, ROW_WARPS * 32, 0, ctx->stream)((const __nv_bfloat16*)x, gamma, beta,       \
                                                                     (__nv_bfloat16*)y, mean, rstd, rows, features, eps)
   switch (J) {
     case 1: HL_LAUNCH(1); break;
@@ -376,7 +381,7 @@ int layer_norm_backward_fast(hl_ctx* ctx, const void* x, const float* gamma, con
   }
   const size_t smem = sizeof(float) * (size_t)groups * 3 * features;  // at most 36 KB
 #define HL_LAUNCH(W)                                                                                              \
-  ln_bwd_bf16_kernel<W><<<blocks, LnBwdShape<W>::THREADS, smem, ctx->stream>>>(                                   \
+  pdl(ln_bwd_bf16_kernel<W>, blocks, LnBwdShape<W>::THREADS, smem, ctx->stream)(                                   \
       (const __nv_bfloat16*)x, gamma, dy, mean, rstd, residual, dx_f32, (__nv_bfloat16*)dx_bf16, partial, rows,   \
       features, rows_per_block)
   switch (wpr) {
@@ -392,7 +397,7 @@ int layer_norm_backward_fast(hl_ctx* ctx, const void* x, const float* gamma, con
     count_launch(ctx);
     return HL_OK;
   }
-  fold_partials_kernel<<<ceil_div(3 * features, 32), FOLD_WARPS * 32, 0, ctx->stream>>>(partial, blocks, 3 * features, dgamma,
+  pdl(fold_partials_kernel, ceil_div(3 * features, 32), FOLD_WARPS * 32, 0, ctx->stream)(partial, blocks, 3 * features, dgamma,
                                                                                      dbeta, dx_colsum, features);
   HL_LAUNCH_CHECK("fold_partials_kernel");
   count_launch(ctx, 2);
@@ -419,10 +424,10 @@ int colsum_fast(hl_ctx* ctx, const void* g, int dtype, float* out, int rows, int
   }
   dim3 grid(col_blocks, slabs);
   if (dtype == HL_BF16)
-    colsum_vec_kernel<__nv_bfloat16, 8><<<grid, ROW_WARPS * 32, 0, ctx->stream>>>((const __nv_bfloat16*)g, partial, rows,
+    pdl(colsum_vec_kernel<__nv_bfloat16, 8>, grid, ROW_WARPS * 32, 0, ctx->stream)((const __nv_bfloat16*)g, partial, rows,
                                                                                    cols, rows_per_block);
   else
-    colsum_vec_kernel<float, 4><<<grid, ROW_WARPS * 32, 0, ctx->stream>>>((const float*)g, partial, rows, cols,
+    pdl(colsum_vec_kernel<float, 4>, grid, ROW_WARPS * 32, 0, ctx->stream)((const float*)g, partial, rows, cols,
                                                                            rows_per_block);
   HL_LAUNCH_CHECK("colsum_vec_kernel");
   if (deferred) {
@@ -430,7 +435,7 @@ int colsum_fast(hl_ctx* ctx, const void* g, int dtype, float* out, int rows, int
     count_launch(ctx);
     return HL_OK;
   }
-  fold_partials_kernel<<<ceil_div(cols, 32), FOLD_WARPS * 32, 0, ctx->stream>>>(partial, slabs, cols, out, nullptr, nullptr,
+  pdl(fold_partials_kernel, ceil_div(cols, 32), FOLD_WARPS * 32, 0, ctx->stream)(partial, slabs, cols, out, nullptr, nullptr,
                                                                              cols);
   HL_LAUNCH_CHECK("fold_partials_kernel");
   count_launch(ctx, 2);

@@ -238,6 +238,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   if (PAIR) tc05::cluster_sync_all(); else __syncthreads();
   tc05::tc_fence_after_sync();
   const uint32_t tmem_base = tail->tmem_base;
+  pdl_begin();  // everything above touches nothing a predecessor wrote
   // Dynamic tile order: the first item of a CTA is its own index, every further one comes from a counter, so a CTA that
   // starts late (its SM was busy with another stream's kernel) simply takes fewer tiles and nobody waits for it.  The
   // producer warp's thread draws the items and hands them to the other roles through a small ring in shared memory.
@@ -684,6 +685,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
 __global__ void splitk_reduce_kernel(const float* __restrict__ partials, float* __restrict__ out, int m, int n,
                                      long long ldc, int splits) {
+  pdl_begin();
   const long long quads = (long long)m * (n / 4);
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < quads; q += (long long)gridDim.x * blockDim.x) {
     const int row = (int)(q / (n / 4));
@@ -707,29 +709,27 @@ int launch_variant(hl_ctx* ctx, const CUtensorMap& ma, const CUtensorMap& mb, co
     configured = true;
   }
   if (PAIR) {
-    // `grid` CTAs in clusters of two neighbouring SMs
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(GEMM_THREADS);
-    cfg.dynamicSmemBytes = GEMM_SMEM_BYTES;
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    // no more pairs than can be resident at once (a GPC with an odd number of free SMs leaves one out)
+    // `grid` CTAs in clusters of two neighbouring SMs; no more pairs than can be resident at once (a GPC with an odd number of free SMs leaves one out)
     static int resident_pairs = 0;
     if (resident_pairs == 0) {
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3((unsigned)grid);
+      cfg.blockDim = dim3(GEMM_THREADS);
+      cfg.dynamicSmemBytes = GEMM_SMEM_BYTES;
+      cudaLaunchAttribute attr{};
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
       int n = 0;
       HL_CUDA(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
       HL_REQUIRE(n > 0, "hl_gemm_bf16: no CTA pair fits on this device");
       resident_pairs = n;
     }
-    if (grid > 2 * resident_pairs) cfg.gridDim = dim3((unsigned)(2 * resident_pairs));
-    HL_CUDA(cudaLaunchKernelEx(&cfg, kern, ma, mb, mc, maux, p));
+    HL_CUDA(launch_pdl(kern, (unsigned)std::min(grid, 2 * resident_pairs), GEMM_THREADS, GEMM_SMEM_BYTES, ctx->stream, 2, ma, mb, mc,
+                       maux, p));
   } else {
-    kern<<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, ctx->stream>>>(ma, mb, mc, maux, p);
+    pdl(kern, grid, GEMM_THREADS, GEMM_SMEM_BYTES, ctx->stream)(ma, mb, mc, maux, p);
   }
   HL_LAUNCH_CHECK("gemm_bf16_tcgen05_kernel");
   count_launch(ctx);
@@ -992,7 +992,7 @@ int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void*
     const long long quads = (long long)d->m * (d->n / 4);
     const long long want_blocks = ceil_div_ll(quads, 256), cap_blocks = (long long)ctx->sm_count * 8;
     const int blocks = (int)(want_blocks < cap_blocks ? want_blocks : cap_blocks);
-    splitk_reduce_kernel<<<blocks, 256, 0, ctx->stream>>>(workspace, reinterpret_cast<float*>(c), d->m, d->n, d->ldc, splits);
+    pdl(splitk_reduce_kernel, blocks, 256, 0, ctx->stream)(workspace, reinterpret_cast<float*>(c), d->m, d->n, d->ldc, splits);
     HL_LAUNCH_CHECK("splitk_reduce_kernel");
     count_launch(ctx);
   }

@@ -16,6 +16,7 @@ constexpr float kNegInf = -INFINITY;
 // One warp per row; k rounds of warp arg-max over the lane's strided elements, chosen entries are
 // remembered in a per-lane bit set (cols <= 32*64).
 __global__ void topk_rows_kernel(const float* __restrict__ scores, int64_t* __restrict__ out, int rows, int cols, int k) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -51,6 +52,7 @@ constexpr int SS_J = 64;   // contraction slice
 __global__ void __launch_bounds__(256)
 side_scores_kernel(const float* __restrict__ query, long long ld_q, int q_off, const float* __restrict__ keys,
                    float* __restrict__ out, int tokens, int side, int half_dim) {
+  pdl_begin();
   __shared__ __align__(16) float sq[SS_J][SS_T];
   __shared__ __align__(16) float sk[SS_J][SS_K];
   const int t0 = blockIdx.y * SS_T, k0 = blockIdx.x * SS_K;
@@ -144,6 +146,7 @@ template <int PER_LANE>
 __global__ void __launch_bounds__(128)
 product_key_topk_kernel(const float* __restrict__ left, const float* __restrict__ right, int64_t* __restrict__ out,
                         int tokens, int side, int top_k, int beam, int* __restrict__ status) {
+  pdl_begin();
   __shared__ unsigned s_hist[4][256];
   __shared__ unsigned s_key[4][32];
   __shared__ int s_index[4][32];
@@ -288,6 +291,7 @@ product_key_topk_kernel(const float* __restrict__ left, const float* __restrict_
 
 __global__ void split_rows_kernel(const int64_t* __restrict__ rows, int64_t* __restrict__ left, int64_t* __restrict__ right,
                                   long long n, int side) {
+  pdl_begin();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const long long r = rows[i];
@@ -301,6 +305,7 @@ __global__ void selected_scores_fwd_kernel(const int64_t* __restrict__ idx, cons
                                            const float* __restrict__ left, const float* __restrict__ right,
                                            float* __restrict__ scores, int tokens, int top_k, int side, int key_dim,
                                            int slots, int* __restrict__ status) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (token >= tokens) return;
@@ -395,6 +400,7 @@ __global__ void selected_scores_bwd_kernel(const int64_t* __restrict__ idx, cons
                                            const float* __restrict__ grad_scores, float* __restrict__ dq, long long ld_dq,
                                            float* __restrict__ dleft, float* __restrict__ dright, int tokens, int top_k,
                                            int side, int key_dim, int slots) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (token >= tokens) return;
@@ -487,6 +493,7 @@ __global__ void __launch_bounds__(256, 2)
 product_key_dkeys_kernel(const int64_t* __restrict__ idx, const float* __restrict__ query, long long ld_q,
                          const float* __restrict__ grad_scores, float* __restrict__ partial, int tokens, int top_k,
                          int side, int half, int slots, int tokens_per_block, int col_blocks) {
+  pdl_begin();
   extern __shared__ __align__(16) float dk_smem[];
   float* w_tile = dk_smem;                          // [DK_TOKENS][DK_ROWS]
   float* q_tile = dk_smem + DK_TOKENS * DK_ROWS;    // [DK_TOKENS][DK_COLS]
@@ -584,6 +591,7 @@ product_key_dkeys_kernel(const int64_t* __restrict__ idx, const float* __restric
 
 __global__ void fold_key_partials_kernel(const float* __restrict__ partial, float* __restrict__ dleft,
                                          float* __restrict__ dright, int blocks, int side, int half) {
+  pdl_begin();
   const size_t per_table = (size_t)side * half;
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= 2 * per_table) return;
@@ -598,6 +606,7 @@ __global__ void fold_key_partials_kernel(const float* __restrict__ partial, floa
 
 // ---- row softmax over a few columns (top-k weights), src/tensor.rs:4521-4602 / autograd.rs:2512-2543 ----
 __global__ void softmax_rows_kernel(const float* __restrict__ x, float* __restrict__ y, int rows, int cols) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -613,6 +622,7 @@ __global__ void softmax_rows_kernel(const float* __restrict__ x, float* __restri
 
 __global__ void softmax_rows_bwd_kernel(const float* __restrict__ y, const float* __restrict__ gy, float* __restrict__ gx,
                                         int rows, int cols) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -630,6 +640,7 @@ __global__ void softmax_rows_bwd_kernel(const float* __restrict__ y, const float
 __global__ void weighted_value_fwd_kernel(const int64_t* __restrict__ idx, const float* __restrict__ weights,
                                           const float* __restrict__ values, float* __restrict__ out, int tokens, int top_k,
                                           int rows, int dim, int* __restrict__ status) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (token >= tokens) return;
@@ -691,6 +702,7 @@ __global__ void weighted_value_bwd_kernel(const int64_t* __restrict__ idx, const
                                           const float* __restrict__ values, const float* __restrict__ grad_out,
                                           float* __restrict__ dweights, float* __restrict__ dvalues, int tokens, int top_k,
                                           int rows, int dim) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (token >= tokens) return;
@@ -724,6 +736,7 @@ __global__ void weighted_value_bwd_kernel(const int64_t* __restrict__ idx, const
 // the traffic that does not stay in registers.
 __global__ void value_event_keys_kernel(const int64_t* __restrict__ idx, long long n, int rows, int* __restrict__ keys,
                                         int* __restrict__ events, float* __restrict__ dweights, int* __restrict__ status) {
+  pdl_begin();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const long long r = idx[i];
@@ -769,6 +782,7 @@ __device__ __forceinline__ void rs_count_tile(const int* __restrict__ keys, long
 
 __global__ void __launch_bounds__(RS_THREADS)
 radix_hist_kernel(const int* __restrict__ keys, long long n, int shift, int* __restrict__ hist, int n_tiles) {
+  pdl_begin();
   __shared__ int wc[RS_WARPS][RS_DIGITS];
   rs_count_tile(keys, n, shift, wc);
   for (int d = threadIdx.x; d < RS_DIGITS; d += RS_THREADS) {
@@ -782,6 +796,7 @@ radix_hist_kernel(const int* __restrict__ keys, long long n, int shift, int* __r
 // Block d scans row d of the digit-major histogram in place (exclusive) and writes the row's total.
 __global__ void __launch_bounds__(RS_THREADS)
 radix_scan_rows_kernel(int* __restrict__ hist, int n_tiles, int* __restrict__ totals) {
+  pdl_begin();
   __shared__ int warp_sums[RS_WARPS];
   __shared__ int carry;
   int* row = hist + (size_t)blockIdx.x * n_tiles;
@@ -813,6 +828,7 @@ __global__ void __launch_bounds__(RS_THREADS)
 radix_scatter_kernel(const int* __restrict__ keys, const int* __restrict__ vals, int* __restrict__ keys_out,
                      int* __restrict__ vals_out, long long n, int shift, const int* __restrict__ starts,
                      const int* __restrict__ totals, int n_tiles) {
+  pdl_begin();
   __shared__ int wc[RS_WARPS][RS_DIGITS];  // counts, then the running output position of each (warp, digit)
   __shared__ int dbase[RS_DIGITS];         // keys with a smaller digit, over all tiles
   __shared__ int wsum[RS_WARPS];
@@ -873,6 +889,7 @@ weighted_value_bwd_sorted_kernel(const int* __restrict__ keys, const int* __rest
                                  const float* __restrict__ weights, const float* __restrict__ values,
                                  const float* __restrict__ grad_out, float* __restrict__ dweights,
                                  float* __restrict__ dvalues, long long n, int top_k, int rows, int dim) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const long long base = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32;
   if (base >= n) return;
@@ -937,6 +954,7 @@ weighted_value_bwd_sorted_kernel(const int* __restrict__ keys, const int* __rest
 // ---- access counts: counts[r] += occurrences of r among the selected rows (kernels.ptx:813-886) ---------------
 __global__ void access_count_rows_kernel(const int64_t* __restrict__ selected, long long n, int rows,
                                          unsigned long long* __restrict__ counts, int* __restrict__ status) {
+  pdl_begin();
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) {
     const long long r = selected[i];
@@ -948,6 +966,7 @@ __global__ void access_count_rows_kernel(const int64_t* __restrict__ selected, l
 // ---- row-set AdamW (src/nn.rs:2256-2323, :2899-2939; kernels.ptx:537-811) -----------------------------------
 __global__ void mark_rows_kernel(const int64_t* __restrict__ selected, long long n, unsigned char* __restrict__ flags,
                                  const unsigned char* __restrict__ row_mask, int rows, int* __restrict__ status) {
+  pdl_begin();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const long long r = selected[i];
@@ -967,6 +986,7 @@ __device__ __forceinline__ void adamw_one(float& p, float g, float& m, float& v,
 __global__ void sparse_adamw_rows_kernel(float* __restrict__ param, float* __restrict__ grad, float* __restrict__ m,
                                          float* __restrict__ v, unsigned char* __restrict__ flags, int rows, int row_dim,
                                          const hl_adamw_params hp, int zero_grad_rows) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows || !flags[row]) return;
@@ -985,6 +1005,7 @@ __global__ void sparse_adamw_rows_kernel(float* __restrict__ param, float* __res
 // warp per flagged row, f64 partial per warp, flags cleared on the way out.
 __global__ void flagged_rows_sum_squares_kernel(const float* __restrict__ grad, unsigned char* __restrict__ flags, int rows,
                                                 int row_dim, double* __restrict__ out) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows || !flags[row]) return;
@@ -1003,6 +1024,7 @@ __global__ void flagged_rows_sum_squares_kernel(const float* __restrict__ grad, 
 // span, an exclusive scan over the spans gives its write position.
 __global__ void __launch_bounds__(1024)
 mask_to_indices_kernel(const unsigned char* __restrict__ mask, int rows, int64_t* __restrict__ out, int* __restrict__ count) {
+  pdl_begin();
   __shared__ int span_start[1025];
   const int per = (rows + 1023) / 1024;
   const int lo = min(rows, (int)threadIdx.x * per), hi = min(rows, lo + per);
@@ -1023,6 +1045,7 @@ mask_to_indices_kernel(const unsigned char* __restrict__ mask, int rows, int64_t
 // dst[i,:] = src[idx[i],:] (gather) or dst[idx[i],:] = src[i,:] (scatter); one warp per row, 16-byte accesses.
 __global__ void move_rows_kernel(const float* __restrict__ src, const int64_t* __restrict__ idx, const int* __restrict__ count_dev,
                                  int n_max, int dim, float* __restrict__ dst, int scatter) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int n = count_dev ? min(*count_dev, n_max) : n_max;
   for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += gridDim.x * (blockDim.x >> 5)) {
@@ -1050,7 +1073,7 @@ int hl_topk_rows_f32(hl_ctx* ctx, const float* scores, int64_t* out, int rows, i
   HL_REQUIRE(rows > 0 && cols > 0, "hl_topk_rows_f32: requires non-zero rows/cols");
   HL_REQUIRE(k > 0 && k <= cols, "hl_topk_rows_f32: k must be in [1, cols]");
   HL_REQUIRE(cols <= 2048, "hl_topk_rows_f32: at most 2048 columns");
-  topk_rows_kernel<<<ceil_div(rows, 4), 128, 0, ctx->stream>>>(scores, out, rows, cols, k);
+  pdl(topk_rows_kernel, ceil_div(rows, 4), 128, 0, ctx->stream)(scores, out, rows, cols, k);
   HL_LAUNCH_CHECK("topk_rows_kernel");
   count_launch(ctx);
   return HL_OK;
@@ -1065,9 +1088,9 @@ int hl_product_key_side_scores_f32(hl_ctx* ctx, const float* query, long long ld
   HL_REQUIRE(ld_query >= key_dim, "hl_product_key_side_scores_f32: query row stride smaller than key_dim");
   const int half = key_dim / 2;
   dim3 grid(ceil_div(side, SS_K), ceil_div(tokens, SS_T));
-  side_scores_kernel<<<grid, 256, 0, ctx->stream>>>(query, ld_query, 0, left_keys, left_scores, tokens, side, half);
+  pdl(side_scores_kernel, grid, 256, 0, ctx->stream)(query, ld_query, 0, left_keys, left_scores, tokens, side, half);
   HL_LAUNCH_CHECK("side_scores_kernel");
-  side_scores_kernel<<<grid, 256, 0, ctx->stream>>>(query, ld_query, half, right_keys, right_scores, tokens, side, half);
+  pdl(side_scores_kernel, grid, 256, 0, ctx->stream)(query, ld_query, half, right_keys, right_scores, tokens, side, half);
   HL_LAUNCH_CHECK("side_scores_kernel");
   count_launch(ctx, 2);
   return HL_OK;
@@ -1081,10 +1104,10 @@ int hl_product_key_topk_from_side_scores(hl_ctx* ctx, const float* left_scores, 
   HL_REQUIRE(beam > 0 && beam <= 32 && beam <= side, "hl_product_key_topk_from_side_scores: beam must be in [1, min(32, side)]");
   HL_REQUIRE(top_k > 0 && top_k <= beam * beam, "hl_product_key_topk_from_side_scores: top_k must be in [1, beam^2]");
   if (side <= 512)
-    product_key_topk_kernel<16><<<ceil_div(tokens, 4), 128, 0, ctx->stream>>>(left_scores, right_scores, out, tokens, side,
+    pdl(product_key_topk_kernel<16>, ceil_div(tokens, 4), 128, 0, ctx->stream)(left_scores, right_scores, out, tokens, side,
                                                                               top_k, beam, ctx->status_dev);
   else
-    product_key_topk_kernel<PK_MAX_PER_LANE><<<ceil_div(tokens, 4), 128, 0, ctx->stream>>>(
+    pdl(product_key_topk_kernel<PK_MAX_PER_LANE>, ceil_div(tokens, 4), 128, 0, ctx->stream)(
         left_scores, right_scores, out, tokens, side, top_k, beam, ctx->status_dev);
   HL_LAUNCH_CHECK("product_key_topk_kernel");
   count_launch(ctx);
@@ -1094,7 +1117,7 @@ int hl_product_key_topk_from_side_scores(hl_ctx* ctx, const float* left_scores, 
 int hl_product_key_split_rows(hl_ctx* ctx, const int64_t* rows, int64_t* left, int64_t* right, long long n, int side) {
   HL_REQUIRE(ctx && rows && left && right, "hl_product_key_split_rows: null argument");
   HL_REQUIRE(n > 0 && side > 0, "hl_product_key_split_rows: requires non-zero rows/side");
-  split_rows_kernel<<<(unsigned)ceil_div_ll(n, 256), 256, 0, ctx->stream>>>(rows, left, right, n, side);
+  pdl(split_rows_kernel, (unsigned)ceil_div_ll(n, 256), 256, 0, ctx->stream)(rows, left, right, n, side);
   HL_LAUNCH_CHECK("split_rows_kernel");
   count_launch(ctx);
   return HL_OK;
@@ -1108,7 +1131,7 @@ int hl_memory_selected_scores_forward(hl_ctx* ctx, const int64_t* indices, const
   if (rc != HL_OK) return rc;
   HL_REQUIRE(side == 0 || (right_keys && key_dim % 2 == 0 && (long long)side * side == slots),
              "hl_memory_selected_scores_forward: product-key mode needs both half tables, even key_dim and square slots");
-  selected_scores_fwd_kernel<<<ceil_div(tokens, 4), 128, 0, ctx->stream>>>(indices, query, ld_query, left_or_keys, right_keys,
+  pdl(selected_scores_fwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream)(indices, query, ld_query, left_or_keys, right_keys,
                                                                            scores, tokens, top_k, side, key_dim, slots,
                                                                            ctx->status_dev);
   HL_LAUNCH_CHECK("selected_scores_fwd_kernel");
@@ -1124,7 +1147,7 @@ int hl_memory_selected_scores_backward(hl_ctx* ctx, const int64_t* indices, cons
   int rc = check_memory_dims(tokens, top_k, key_dim, "hl_memory_selected_scores_backward");
   if (rc != HL_OK) return rc;
   HL_REQUIRE(side == 0 || (right_keys && key_dim % 2 == 0), "hl_memory_selected_scores_backward: product-key mode needs both half tables");
-  selected_scores_bwd_kernel<<<ceil_div(tokens, 4), 128, 0, ctx->stream>>>(
+  pdl(selected_scores_bwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream)(
       indices, query, ld_query, left_or_keys, right_keys, grad_scores, grad_query, ld_grad_query, grad_left_or_keys,
       grad_right_keys, tokens, top_k, side, key_dim, slots);
   HL_LAUNCH_CHECK("selected_scores_bwd_kernel");
@@ -1140,11 +1163,11 @@ int hl_memory_selected_scores_backward(hl_ctx* ctx, const int64_t* indices, cons
     if (rc != HL_OK) return rc;
     float* partial = reinterpret_cast<float*>(ctx->workspace);
     HL_CUDA(cudaFuncSetAttribute(product_key_dkeys_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    product_key_dkeys_kernel<<<dim3(token_blocks, col_blocks * row_blocks, 2), 256, smem, ctx->stream>>>(
+    pdl(product_key_dkeys_kernel, dim3(token_blocks, col_blocks * row_blocks, 2), 256, smem, ctx->stream)(
         indices, query, ld_query, grad_scores, partial, tokens, top_k, side, half, slots, tokens_per_block, col_blocks);
     HL_LAUNCH_CHECK("product_key_dkeys_kernel");
     const size_t total = 2 * (size_t)side * half;
-    fold_key_partials_kernel<<<(unsigned)((total + 255) / 256), 256, 0, ctx->stream>>>(partial, grad_left_or_keys, grad_right_keys,
+    pdl(fold_key_partials_kernel, (unsigned)((total + 255) / 256), 256, 0, ctx->stream)(partial, grad_left_or_keys, grad_right_keys,
                                                                                        token_blocks, side, half);
     HL_LAUNCH_CHECK("fold_key_partials_kernel");
     count_launch(ctx, 2);
@@ -1155,7 +1178,7 @@ int hl_memory_selected_scores_backward(hl_ctx* ctx, const int64_t* indices, cons
 int hl_softmax_rows_f32(hl_ctx* ctx, const float* x, float* y, int rows, int cols) {
   HL_REQUIRE(ctx && x && y, "hl_softmax_rows_f32: null argument");
   HL_REQUIRE(rows > 0 && cols > 0, "hl_softmax_rows_f32: requires non-zero rows/cols");
-  softmax_rows_kernel<<<ceil_div(rows, 4), 128, 0, ctx->stream>>>(x, y, rows, cols);
+  pdl(softmax_rows_kernel, ceil_div(rows, 4), 128, 0, ctx->stream)(x, y, rows, cols);
   HL_LAUNCH_CHECK("softmax_rows_kernel");
   count_launch(ctx);
   return HL_OK;
@@ -1164,7 +1187,7 @@ int hl_softmax_rows_f32(hl_ctx* ctx, const float* x, float* y, int rows, int col
 int hl_softmax_rows_backward_f32(hl_ctx* ctx, const float* y, const float* grad_y, float* grad_x, int rows, int cols) {
   HL_REQUIRE(ctx && y && grad_y && grad_x, "hl_softmax_rows_backward_f32: null argument");
   HL_REQUIRE(rows > 0 && cols > 0, "hl_softmax_rows_backward_f32: requires non-zero rows/cols");
-  softmax_rows_bwd_kernel<<<ceil_div(rows, 4), 128, 0, ctx->stream>>>(y, grad_y, grad_x, rows, cols);
+  pdl(softmax_rows_bwd_kernel, ceil_div(rows, 4), 128, 0, ctx->stream)(y, grad_y, grad_x, rows, cols);
   HL_LAUNCH_CHECK("softmax_rows_bwd_kernel");
   count_launch(ctx);
   return HL_OK;
@@ -1176,7 +1199,7 @@ int hl_memory_weighted_value_forward(hl_ctx* ctx, const int64_t* indices, const 
   int rc = check_memory_dims(tokens, top_k, dim, "hl_memory_weighted_value_forward");
   if (rc != HL_OK) return rc;
   HL_REQUIRE(rows > 0 && dim % 4 == 0, "hl_memory_weighted_value_forward: non-zero rows/row_dim, row_dim a multiple of 4");
-  weighted_value_fwd_kernel<<<ceil_div(tokens, 4), 128, 0, ctx->stream>>>(indices, weights, values, out, tokens, top_k, rows,
+  pdl(weighted_value_fwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream)(indices, weights, values, out, tokens, top_k, rows,
                                                                           dim, ctx->status_dev);
   HL_LAUNCH_CHECK("weighted_value_fwd_kernel");
   count_launch(ctx);
@@ -1204,17 +1227,17 @@ int hl_memory_weighted_value_backward(hl_ctx* ctx, const int64_t* indices, const
     int *keys_a = reinterpret_cast<int*>(ws), *ev_a = reinterpret_cast<int*>(ws + arr);
     int *keys_b = reinterpret_cast<int*>(ws + 2 * arr), *ev_b = reinterpret_cast<int*>(ws + 3 * arr);
     int* hist = reinterpret_cast<int*>(ws + 4 * arr);
-    value_event_keys_kernel<<<(unsigned)ceil_div_ll(n, 256), 256, 0, ctx->stream>>>(indices, n, rows, keys_a, ev_a, grad_weights,
+    pdl(value_event_keys_kernel, (unsigned)ceil_div_ll(n, 256), 256, 0, ctx->stream)(indices, n, rows, keys_a, ev_a, grad_weights,
                                                                                      ctx->status_dev);
     HL_LAUNCH_CHECK("value_event_keys_kernel");
     int passes = 0;
     for (int shift = 0; shift < end_bit; shift += RS_BITS, ++passes) {
-      radix_hist_kernel<<<n_tiles, RS_THREADS, 0, ctx->stream>>>(keys_a, n, shift, hist, n_tiles);
+      pdl(radix_hist_kernel, n_tiles, RS_THREADS, 0, ctx->stream)(keys_a, n, shift, hist, n_tiles);
       HL_LAUNCH_CHECK("radix_hist_kernel");
       int* totals = hist + (size_t)RS_DIGITS * n_tiles;
-      radix_scan_rows_kernel<<<RS_DIGITS, RS_THREADS, 0, ctx->stream>>>(hist, n_tiles, totals);
+      pdl(radix_scan_rows_kernel, RS_DIGITS, RS_THREADS, 0, ctx->stream)(hist, n_tiles, totals);
       HL_LAUNCH_CHECK("radix_scan_rows_kernel");
-      radix_scatter_kernel<<<n_tiles, RS_THREADS, 0, ctx->stream>>>(keys_a, ev_a, keys_b, ev_b, n, shift, hist, totals, n_tiles);
+      pdl(radix_scatter_kernel, n_tiles, RS_THREADS, 0, ctx->stream)(keys_a, ev_a, keys_b, ev_b, n, shift, hist, totals, n_tiles);
       HL_LAUNCH_CHECK("radix_scatter_kernel");
       std::swap(keys_a, keys_b);
       std::swap(ev_a, ev_b);
@@ -1223,16 +1246,16 @@ int hl_memory_weighted_value_backward(hl_ctx* ctx, const int64_t* indices, const
     count_launch(ctx, 3 * passes);
     const unsigned blocks = (unsigned)ceil_div_ll(ceil_div_ll(n, 32), 4);
     if (dim <= 512)
-      weighted_value_bwd_sorted_kernel<4><<<blocks, 128, 0, ctx->stream>>>(keys, ev, weights, values, grad_out, grad_weights,
+      pdl(weighted_value_bwd_sorted_kernel<4>, blocks, 128, 0, ctx->stream)(keys, ev, weights, values, grad_out, grad_weights,
                                                                            grad_values, n, top_k, rows, dim);
     else
-      weighted_value_bwd_sorted_kernel<8><<<blocks, 128, 0, ctx->stream>>>(keys, ev, weights, values, grad_out, grad_weights,
+      pdl(weighted_value_bwd_sorted_kernel<8>, blocks, 128, 0, ctx->stream)(keys, ev, weights, values, grad_out, grad_weights,
                                                                            grad_values, n, top_k, rows, dim);
     HL_LAUNCH_CHECK("weighted_value_bwd_sorted_kernel");
     count_launch(ctx, 2);
     return HL_OK;
   }
-  weighted_value_bwd_kernel<<<ceil_div(tokens, 4), 128, 0, ctx->stream>>>(indices, weights, values, grad_out, grad_weights,
+  pdl(weighted_value_bwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream)(indices, weights, values, grad_out, grad_weights,
                                                                           grad_values, tokens, top_k, rows, dim);
   HL_LAUNCH_CHECK("weighted_value_bwd_kernel");
   count_launch(ctx);
@@ -1246,14 +1269,14 @@ namespace hl {
 int mark_rows_on(hl_ctx* ctx, cudaStream_t stream, const int64_t* selected_rows, long long n_selected, const unsigned char* row_mask,
                  unsigned char* flags, int rows) {
   if (n_selected <= 0) return HL_OK;
-  mark_rows_kernel<<<(unsigned)ceil_div_ll(n_selected, 256), 256, 0, stream>>>(selected_rows, n_selected, flags, row_mask, rows,
+  pdl(mark_rows_kernel, (unsigned)ceil_div_ll(n_selected, 256), 256, 0, stream)(selected_rows, n_selected, flags, row_mask, rows,
                                                                              ctx->status_dev);
   HL_LAUNCH_CHECK("mark_rows_kernel");
   count_launch(ctx);
   return HL_OK;
 }
 int mask_to_indices_on(hl_ctx* ctx, cudaStream_t stream, const unsigned char* mask, int rows, int64_t* out, int* count_dev) {
-  mask_to_indices_kernel<<<1, 1024, 0, stream>>>(mask, rows, out, count_dev);
+  pdl(mask_to_indices_kernel, 1, 1024, 0, stream)(mask, rows, out, count_dev);
   HL_LAUNCH_CHECK("mask_to_indices_kernel");
   count_launch(ctx);
   return HL_OK;
@@ -1262,7 +1285,7 @@ int move_rows_on(hl_ctx* ctx, cudaStream_t stream, const float* src, const int64
                  float* dst, bool scatter) {
   if (n_max <= 0) return HL_OK;
   const int blocks = std::min(ceil_div(n_max, 8), ctx->sm_count * 8);
-  move_rows_kernel<<<blocks, 256, 0, stream>>>(src, idx, count_dev, n_max, dim, dst, scatter ? 1 : 0);
+  pdl(move_rows_kernel, blocks, 256, 0, stream)(src, idx, count_dev, n_max, dim, dst, scatter ? 1 : 0);
   HL_LAUNCH_CHECK("move_rows_kernel");
   count_launch(ctx);
   return HL_OK;
@@ -1278,7 +1301,7 @@ int hl_memory_access_count_rows_i64_u64(hl_ctx* ctx, const int64_t* selected_row
   HL_REQUIRE(n_selected >= 0 && (n_selected == 0 || selected_rows), "hl_memory_access_count_rows_i64_u64: null selected rows");
   if (n_selected == 0) return HL_OK;
   const unsigned blocks = (unsigned)std::min<long long>(ceil_div_ll(n_selected, 256), (long long)ctx->sm_count * 16);
-  access_count_rows_kernel<<<blocks, 256, 0, ctx->stream>>>(selected_rows, n_selected, slots, counts, ctx->status_dev);
+  pdl(access_count_rows_kernel, blocks, 256, 0, ctx->stream)(selected_rows, n_selected, slots, counts, ctx->status_dev);
   HL_LAUNCH_CHECK("access_count_rows_kernel");
   count_launch(ctx);
   return HL_OK;
@@ -1315,10 +1338,10 @@ int hl_sparse_rows_sum_squares_f32(hl_ctx* ctx, const float* grad, const int64_t
   HL_REQUIRE(ctx && grad && selected_rows && row_flags && sum_dev, "hl_sparse_rows_sum_squares_f32: null argument");
   HL_REQUIRE(rows > 0 && row_dim > 0, "hl_sparse_rows_sum_squares_f32: requires non-zero rows/row_dim");
   if (n_selected <= 0) return HL_OK;
-  mark_rows_kernel<<<(unsigned)ceil_div_ll(n_selected, 256), 256, 0, ctx->stream>>>(selected_rows, n_selected, row_flags,
+  pdl(mark_rows_kernel, (unsigned)ceil_div_ll(n_selected, 256), 256, 0, ctx->stream)(selected_rows, n_selected, row_flags,
                                                                                   row_mask, rows, ctx->status_dev);
   HL_LAUNCH_CHECK("mark_rows_kernel");
-  flagged_rows_sum_squares_kernel<<<ceil_div(rows, 8), 256, 0, ctx->stream>>>(grad, row_flags, rows, row_dim, sum_dev);
+  pdl(flagged_rows_sum_squares_kernel, ceil_div(rows, 8), 256, 0, ctx->stream)(grad, row_flags, rows, row_dim, sum_dev);
   HL_LAUNCH_CHECK("flagged_rows_sum_squares_kernel");
   count_launch(ctx, 2);
   return HL_OK;
@@ -1331,10 +1354,10 @@ int hl_sparse_adamw_rows_f32(hl_ctx* ctx, float* param, float* grad, float* m, f
   HL_REQUIRE(rows > 0 && row_dim > 0, "hl_sparse_adamw_rows_f32: requires non-zero rows/row_dim");
   HL_REQUIRE(hp->bias_correction1 > 0.f && hp->bias_correction2 > 0.f, "hl_sparse_adamw_rows_f32: bias corrections must be positive");
   if (n_selected <= 0) return HL_OK;
-  mark_rows_kernel<<<(unsigned)ceil_div_ll(n_selected, 256), 256, 0, ctx->stream>>>(selected_rows, n_selected, row_flags,
+  pdl(mark_rows_kernel, (unsigned)ceil_div_ll(n_selected, 256), 256, 0, ctx->stream)(selected_rows, n_selected, row_flags,
                                                                                   row_mask, rows, ctx->status_dev);
   HL_LAUNCH_CHECK("mark_rows_kernel");
-  sparse_adamw_rows_kernel<<<ceil_div(rows, 8), 256, 0, ctx->stream>>>(param, grad, m, v, row_flags, rows, row_dim, *hp,
+  pdl(sparse_adamw_rows_kernel, ceil_div(rows, 8), 256, 0, ctx->stream)(param, grad, m, v, row_flags, rows, row_dim, *hp,
                                                                        zero_grad_rows);
   HL_LAUNCH_CHECK("sparse_adamw_rows_kernel");
   count_launch(ctx, 2);

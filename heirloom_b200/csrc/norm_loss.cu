@@ -44,6 +44,7 @@ template <typename XT, typename YT, typename Acc, bool VEC4>
 __global__ void layer_norm_fwd_kernel(const XT* __restrict__ x, const float* __restrict__ gamma,
                                       const float* __restrict__ beta, YT* __restrict__ y, float* __restrict__ mean_out,
                                       float* __restrict__ rstd_out, int rows, int features, float eps) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -110,6 +111,7 @@ layer_norm_bwd_kernel(const XT* __restrict__ x, const float* __restrict__ gamma,
                       const float* __restrict__ residual_grad, float* __restrict__ dx_f32,
                       __nv_bfloat16* __restrict__ dx_bf16, float* __restrict__ partial /*[blocks][2][features]*/,
                       int rows, int features, int rows_per_block, float eps) {
+  pdl_begin();
   extern __shared__ float lnb_smem[];  // [LNB_WARPS][2][features]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int r0 = blockIdx.x * rows_per_block, r1 = min(rows, r0 + rows_per_block);
@@ -212,6 +214,7 @@ template <typename OT>
 __global__ void embedding_fwd_kernel(const float* __restrict__ table, int table_rows, const int64_t* __restrict__ idx,
                                      const float* __restrict__ pos_table, int period, OT* __restrict__ out, int n,
                                      int dim, bool round_terms, int* __restrict__ status) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= n) return;
@@ -247,6 +250,7 @@ __global__ void embedding_fwd_kernel(const float* __restrict__ table, int table_
 __global__ void embedding_bwd_kernel(const float* __restrict__ grad_out, const int64_t* __restrict__ idx,
                                      float* __restrict__ grad_table, int table_rows, int n, int dim,
                                      int* __restrict__ status) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= n) return;
@@ -271,6 +275,7 @@ __global__ void embedding_bwd_kernel(const float* __restrict__ grad_out, const i
 // result does not depend on scheduling.
 __global__ void position_grad_kernel(const float* __restrict__ grad_out, float* __restrict__ pos_grad, int period,
                                      int n, int dim) {
+  pdl_begin();
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= (size_t)period * dim) return;
   const int t = (int)(i / dim), c = (int)(i % dim);
@@ -286,6 +291,7 @@ template <typename Acc, typename DT>
 __global__ void cross_entropy_kernel(const float* __restrict__ logits, long long ld, const int64_t* __restrict__ targets,
                                      int rows, int classes, float scale, float* __restrict__ row_loss,
                                      DT* __restrict__ dlogits, long long ld_d, int* __restrict__ status) {
+  pdl_begin();
   __shared__ Acc sm[32];
   const int row = blockIdx.x;
   const float* z = logits + (size_t)row * ld;
@@ -351,6 +357,7 @@ __global__ void __launch_bounds__(CE_THREADS, 2)
 cross_entropy_online_kernel(const float* __restrict__ logits, long long ld, const int64_t* __restrict__ targets,
                             int rows, int classes, float scale, float* __restrict__ row_loss,
                             __nv_bfloat16* __restrict__ dlogits, long long ld_d, int* __restrict__ status) {
+  pdl_begin();
   __shared__ float sm[32];
   constexpr float kLog2e = 1.4426950408889634f;
   constexpr int STEP = CE_THREADS * 4;  // columns covered by one 16-byte load per thread
@@ -414,6 +421,7 @@ cross_entropy_online_kernel(const float* __restrict__ logits, long long ld, cons
 }
 
 __global__ void mean_rows_kernel(const float* __restrict__ row_loss, int rows, float* __restrict__ out) {
+  pdl_begin();
   __shared__ double sm[32];
   double acc = 0.0;
   for (int i = threadIdx.x; i < rows; i += blockDim.x) acc += (double)row_loss[i];
@@ -440,10 +448,10 @@ int layer_norm_forward_impl(hl_ctx* ctx, const void* x, int x_dtype, const float
 #define HL_LN_FWD(XT, YT, ACC)                                                                              \
   do {                                                                                                      \
     if (vec)                                                                                                \
-      layer_norm_fwd_kernel<XT, YT, ACC, true><<<grid, warps * 32, 0, ctx->stream>>>(                       \
+      pdl(layer_norm_fwd_kernel<XT, YT, ACC, true>, grid, warps * 32, 0, ctx->stream)(                       \
           (const XT*)x, gamma, beta, (YT*)y, mean, rstd, rows, features, eps);                              \
     else                                                                                                    \
-      layer_norm_fwd_kernel<XT, YT, ACC, false><<<grid, warps * 32, 0, ctx->stream>>>(                      \
+      pdl(layer_norm_fwd_kernel<XT, YT, ACC, false>, grid, warps * 32, 0, ctx->stream)(                      \
           (const XT*)x, gamma, beta, (YT*)y, mean, rstd, rows, features, eps);                              \
   } while (0)
   if (x_dtype == HL_F32 && y_dtype == HL_F32) HL_LN_FWD(float, float, double);
@@ -503,7 +511,7 @@ int layer_norm_backward_impl(hl_ctx* ctx, const void* x, int x_dtype, const floa
       HL_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(float) * LNB_WARPS * 2 * LNB_MAXJ * 128))); \
       configured = true;                                                                                               \
     }                                                                                                                  \
-    k<<<blocks, LNB_WARPS * 32, smem, ctx->stream>>>((const XT*)x, gamma, dy, mean, rstd, residual_grad, dx_f32,       \
+    pdl(k, blocks, LNB_WARPS * 32, smem, ctx->stream)((const XT*)x, gamma, dy, mean, rstd, residual_grad, dx_f32,       \
                                                      (__nv_bfloat16*)dx_bf16, partial, rows, features, rows_per_block, \
                                                      1e-5f);                                                           \
   } while (0)
@@ -552,18 +560,18 @@ int cross_entropy_impl(hl_ctx* ctx, const float* logits, long long ld, const int
                          (reinterpret_cast<uintptr_t>(logits) & 15) == 0 && (reinterpret_cast<uintptr_t>(dlogits) & 7) == 0 &&
                          classes >= 1024;
   if (online_ok && (dlogits || dlogits_dtype == HL_BF16))
-    cross_entropy_online_kernel<<<std::min(rows, ctx->sm_count * 2), CE_THREADS, 0, ctx->stream>>>(
+    pdl(cross_entropy_online_kernel, std::min(rows, ctx->sm_count * 2), CE_THREADS, 0, ctx->stream)(
         logits, ld, targets, rows, classes, scale, rl, (__nv_bfloat16*)dlogits, ld_dlogits, ctx->status_dev);
   else if (dlogits && dlogits_dtype == HL_BF16)
-    cross_entropy_kernel<float, __nv_bfloat16><<<rows, threads, 0, ctx->stream>>>(
+    pdl(cross_entropy_kernel<float, __nv_bfloat16>, rows, threads, 0, ctx->stream)(
         logits, ld, targets, rows, classes, scale, rl, (__nv_bfloat16*)dlogits, ld_dlogits, ctx->status_dev);
   else
-    cross_entropy_kernel<double, float><<<rows, threads, 0, ctx->stream>>>(
+    pdl(cross_entropy_kernel<double, float>, rows, threads, 0, ctx->stream)(
         logits, ld, targets, rows, classes, scale, rl, (float*)dlogits, ld_dlogits, ctx->status_dev);
   HL_LAUNCH_CHECK("cross_entropy_kernel");
   count_launch(ctx);
   if (loss_dev) {
-    mean_rows_kernel<<<1, 1024, 0, ctx->stream>>>(rl, rows, loss_dev);
+    pdl(mean_rows_kernel, 1, 1024, 0, ctx->stream)(rl, rows, loss_dev);
     HL_LAUNCH_CHECK("mean_rows_kernel");
     count_launch(ctx);
   }
@@ -596,10 +604,10 @@ int hl_embedding_forward(hl_ctx* ctx, const float* table, int table_rows, const 
   ProfileScope prof(ctx, HL_PROF_EMBEDDING, (double)n * dim * (4.0 + (pos_table ? 4.0 : 0.0) + (double)dtype_size(out_dtype)));
   const int warps = 4;
   if (out_dtype == HL_BF16)
-    embedding_fwd_kernel<__nv_bfloat16><<<ceil_div(n, warps), warps * 32, 0, ctx->stream>>>(
+    pdl(embedding_fwd_kernel<__nv_bfloat16>, ceil_div(n, warps), warps * 32, 0, ctx->stream)(
         table, table_rows, idx, pos_table, period, (__nv_bfloat16*)out, n, dim, true, ctx->status_dev);
   else if (out_dtype == HL_F32)
-    embedding_fwd_kernel<float><<<ceil_div(n, warps), warps * 32, 0, ctx->stream>>>(
+    pdl(embedding_fwd_kernel<float>, ceil_div(n, warps), warps * 32, 0, ctx->stream)(
         table, table_rows, idx, pos_table, period, (float*)out, n, dim, false, ctx->status_dev);
   else
     return fail("hl_embedding_forward: output dtype must be f32 or bf16");
@@ -614,14 +622,14 @@ int hl_embedding_backward(hl_ctx* ctx, const float* grad_out, const int64_t* idx
   HL_REQUIRE(n > 0 && dim > 0 && table_rows > 0, "hl_embedding_backward: sizes must be positive");
   ProfileScope prof(ctx, HL_PROF_EMBEDDING, (double)n * dim * 12.0);
   const int warps = 4;
-  embedding_bwd_kernel<<<ceil_div(n, warps), warps * 32, 0, ctx->stream>>>(grad_out, idx, grad_table, table_rows, n,
+  pdl(embedding_bwd_kernel, ceil_div(n, warps), warps * 32, 0, ctx->stream)(grad_out, idx, grad_table, table_rows, n,
                                                                            dim, ctx->status_dev);
   HL_LAUNCH_CHECK("embedding_bwd_kernel");
   count_launch(ctx);
   if (pos_grad) {
     HL_REQUIRE(period > 0, "hl_embedding_backward: period must be positive with a position gradient");
     const size_t total = (size_t)period * dim;
-    position_grad_kernel<<<(unsigned)((total + 255) / 256), 256, 0, ctx->stream>>>(grad_out, pos_grad, period, n, dim);
+    pdl(position_grad_kernel, (unsigned)((total + 255) / 256), 256, 0, ctx->stream)(grad_out, pos_grad, period, n, dim);
     HL_LAUNCH_CHECK("position_grad_kernel");
     count_launch(ctx);
   }

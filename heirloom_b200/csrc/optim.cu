@@ -45,6 +45,7 @@ __device__ __forceinline__ void adamw_element(float& p, float g, float& m, float
 
 __global__ void __launch_bounds__(ADAM_THREADS)
 adamw_chunks_kernel(const AdamChunk* __restrict__ chunks, const hl_adamw_params hp) {
+  pdl_begin();
   const AdamChunk ch = chunks[blockIdx.x];
   const unsigned int n4 = ch.n / 4;
   for (unsigned int i = threadIdx.x; i < n4; i += blockDim.x) {
@@ -72,6 +73,7 @@ adamw_chunks_kernel(const AdamChunk* __restrict__ chunks, const hl_adamw_params 
 
 __global__ void adamw_scalar_kernel(float* __restrict__ param, const float* __restrict__ grad, float* __restrict__ m,
                                     float* __restrict__ v, size_t n, const hl_adamw_params hp) {
+  pdl_begin();
   const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = tid; i < n; i += stride) {
     float p = param[i], mm = m[i], vv = v[i];
@@ -153,7 +155,7 @@ int adam_plan_step_range(hl_ctx* ctx, AdamPlan* plan, const hl_adamw_params* hp,
   if (count == 0) return HL_OK;
   // 28 bytes per parameter (read p, g, m, v; write p, m, v) plus 2 for the bf16 shadow
   ProfileScope prof(ctx, HL_PROF_OPTIMIZER, 30.0 * (double)plan->elements * ((double)count / (double)plan->count));
-  adamw_chunks_kernel<<<count, ADAM_THREADS, 0, ctx->stream>>>(plan->chunks_dev + first, *hp);
+  pdl(adamw_chunks_kernel, count, ADAM_THREADS, 0, ctx->stream)(plan->chunks_dev + first, *hp);
   HL_LAUNCH_CHECK("adamw_chunks_kernel");
   count_launch(ctx);
   return HL_OK;
@@ -175,7 +177,7 @@ int hl_adamw_f32(hl_ctx* ctx, float* param, const float* grad, float* m, float* 
   if (rc != HL_OK) return rc;
   if (n == 0) return HL_OK;
   const int grid = (int)std::min<size_t>((n + 255) / 256, (size_t)ctx->sm_count * 16);
-  adamw_scalar_kernel<<<grid, 256, 0, ctx->stream>>>(param, grad, m, v, n, *hp);
+  pdl(adamw_scalar_kernel, grid, 256, 0, ctx->stream)(param, grad, m, v, n, *hp);
   HL_LAUNCH_CHECK("adamw_scalar_kernel");
   count_launch(ctx);
   return HL_OK;

@@ -198,6 +198,7 @@ __device__ __forceinline__ void f64_tile_sums(const F64Gemm& g, double* smem, in
 template <int TM, int TN>
 __global__ void __launch_bounds__(F64_THREADS, TM == 32 ? 3 : 2)
 f64_gemm_kernel(const F64Jobs jobs) {
+  pdl_begin();
   using Z = F64Tile<TM, TN>;
   extern __shared__ double f64_smem[];
   const int which = (jobs.count > 1 && (int)blockIdx.x >= jobs.job[1].cta0) ? 1 : 0;
@@ -279,18 +280,7 @@ int launch_f64_gemm(hl_ctx* ctx, const F64Gemm* problems, int count) {
     ctas += j.split > 1 ? (long long)j.tiles * j.split : ceil_div_ll(j.tiles, jobs.cluster) * jobs.cluster;
   }
   HL_REQUIRE(ctas <= 0x7fffffffLL, "hl_matmul_f32_strided: too many tiles for one launch");
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)ctas);
-  cfg.blockDim = dim3(F64_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = ctx->stream;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = (unsigned)jobs.cluster; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  HL_CUDA(cudaLaunchKernelEx(&cfg, kern, jobs));
-  HL_LAUNCH_CHECK("f64_gemm_kernel");
+  HL_CUDA(launch_pdl(kern, (unsigned)ctas, F64_THREADS, smem, ctx->stream, jobs.cluster, jobs));
   count_launch(ctx);
   return HL_OK;
 }
@@ -422,6 +412,7 @@ template <typename T>
 __global__ void __launch_bounds__(AT_THREADS)
 attention_f64_fwd_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, long long ld_qkv,
                          T* __restrict__ out, long long ld_out, float* __restrict__ probs, int T_, int H, int hd, unsigned heads) {
+  pdl_begin();
   extern __shared__ double at_smem[];
   const int ld = at_ld(hd), ld_s = at_ld((T_ + AT_K - 1) / AT_K * AT_K);
   double *sx = at_smem, *sy = sx + AT_Q * ld, *ss = sy + AT_K * ld;
@@ -441,6 +432,7 @@ __global__ void __launch_bounds__(AT_THREADS)
 attention_f64_bwd_rows_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, long long ld_qkv,
                               float* __restrict__ probs, const T* __restrict__ dout, long long ld_dout,
                               float* __restrict__ ds, T* __restrict__ dq, long long ld_dqkv, int T_, int H, int hd, unsigned heads) {
+  pdl_begin();
   extern __shared__ double at_smem[];
   const int ld = at_ld(hd), ld_s = at_ld((T_ + AT_K - 1) / AT_K * AT_K);
   double *sx = at_smem, *sy = sx + AT_Q * ld, *ss = sy + AT_K * ld;
@@ -483,6 +475,7 @@ __global__ void __launch_bounds__(AT_THREADS)
 attention_f64_bwd_cols_kernel(const T* __restrict__ q, long long ld_qkv, const float* __restrict__ probs,
                               const float* __restrict__ ds, const T* __restrict__ dout, long long ld_dout,
                               T* __restrict__ dk, T* __restrict__ dv, long long ld_dqkv, int T_, int H, int hd, unsigned heads) {
+  pdl_begin();
   extern __shared__ double at_smem[];
   constexpr int CH = 4 * AT_GROUPS * 8;  // channels of one pass
   const int ld = at_ld(min(hd, CH));
@@ -557,6 +550,7 @@ template <typename T>
 __global__ void attention_f64_fwd_rows_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                                               long long ld_qkv, T* __restrict__ out, long long ld_out,
                                               float* __restrict__ probs, int B, int T_, int H, int hd) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const long long w = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= (long long)B * H * T_) return;
@@ -592,6 +586,7 @@ __global__ void attention_f64_bwd_long_rows_kernel(const T* __restrict__ k, cons
                                                    const float* __restrict__ probs, const T* __restrict__ dout,
                                                    long long ld_dout, float* __restrict__ ds, T* __restrict__ dq,
                                                    long long ld_dqkv, int B, int T_, int H, int hd) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const long long w = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= (long long)B * H * T_) return;
@@ -645,11 +640,11 @@ int attention_forward_t(hl_ctx* ctx, const T* q, const T* k, const T* v, long lo
       if (rc != HL_OK) return rc;
       configured = true;
     }
-    attention_f64_fwd_kernel<T><<<(unsigned)(ceil_div(Tn, AT_Q) * heads), AT_THREADS, smem, ctx->stream>>>(
+    pdl(attention_f64_fwd_kernel<T>, (unsigned)(ceil_div(Tn, AT_Q) * heads), AT_THREADS, smem, ctx->stream)(
         q, k, v, ld_qkv, out, ld_out, probs, Tn, H, hd, (unsigned)heads);
     HL_LAUNCH_CHECK("attention_f64_fwd_kernel");
   } else {
-    attention_f64_fwd_rows_kernel<T><<<(unsigned)ceil_div_ll(heads * Tn, 4), 128, 0, ctx->stream>>>(q, k, v, ld_qkv, out, ld_out,
+    pdl(attention_f64_fwd_rows_kernel<T>, (unsigned)ceil_div_ll(heads * Tn, 4), 128, 0, ctx->stream)(q, k, v, ld_qkv, out, ld_out,
                                                                                                     probs, B, Tn, H, hd);
     HL_LAUNCH_CHECK("attention_f64_fwd_rows_kernel");
   }
@@ -673,18 +668,18 @@ int attention_backward_t(hl_ctx* ctx, const T* q, const T* k, const T* v, long l
     configured = true;
   }
   if (rows <= kAttentionSmem) {
-    attention_f64_bwd_rows_kernel<T, RECOMPUTE><<<(unsigned)(ceil_div(Tn, AT_Q) * heads), AT_THREADS, rows, ctx->stream>>>(
+    pdl(attention_f64_bwd_rows_kernel<T, RECOMPUTE>, (unsigned)(ceil_div(Tn, AT_Q) * heads), AT_THREADS, rows, ctx->stream)(
         q, k, v, ld_qkv, probs, dout, ld_dout, ds, dq, ld_dqkv, Tn, H, hd, (unsigned)heads);
     HL_LAUNCH_CHECK("attention_f64_bwd_rows_kernel");
   } else {
     if (RECOMPUTE) {  // the output goes where dQ will be written
       if ((rc = attention_forward_t<T>(ctx, q, k, v, ld_qkv, dq, ld_dqkv, probs, B, Tn, C, H)) != HL_OK) return rc;
     }
-    attention_f64_bwd_long_rows_kernel<T><<<(unsigned)ceil_div_ll(heads * Tn, 4), 128, 0, ctx->stream>>>(
+    pdl(attention_f64_bwd_long_rows_kernel<T>, (unsigned)ceil_div_ll(heads * Tn, 4), 128, 0, ctx->stream)(
         k, v, ld_qkv, probs, dout, ld_dout, ds, dq, ld_dqkv, B, Tn, H, hd);
     HL_LAUNCH_CHECK("attention_f64_bwd_long_rows_kernel");
   }
-  attention_f64_bwd_cols_kernel<T><<<(unsigned)(ceil_div(Tn, AT_Q) * heads), AT_THREADS, cols, ctx->stream>>>(
+  pdl(attention_f64_bwd_cols_kernel<T>, (unsigned)(ceil_div(Tn, AT_Q) * heads), AT_THREADS, cols, ctx->stream)(
       q, ld_qkv, probs, ds, dout, ld_dout, dk, dv, ld_dqkv, Tn, H, hd, (unsigned)heads);
   HL_LAUNCH_CHECK("attention_f64_bwd_cols_kernel");
   count_launch(ctx, 2);
