@@ -282,6 +282,38 @@ int launch_majors(hl_ctx* ctx, bool a_mn, bool b_mn, const CUtensorMap& ma, cons
 // Examples, persistent kernel against this one: 256 x 384 x 128 6.4 -> 3.7 us, 128 x 128 x 256 (transposed operands) 8.9 -> 4.0,
 // 500 x 768 x 3072 22.4 -> 9.9, 2048 x 512 x 2048 15.2 -> 8.8, 4096 x 512 x 2048 19.1 -> 11.3, 3072 x 768 x 4099 (transposed)
 // 23.8 -> 17.6.
+namespace {
+// CTAs of one wave of clusters of `splits`: a cluster sits in one GPC, so clusters of four and eight leave SMs over.  Asked of
+// the driver once per form; form 0 deep, 1 narrow, 2 wide.
+int wave_ctas(int form, int splits, int sm_count) {
+  static int clusters[3][4] = {};
+  const int at = splits == 1 ? 0 : splits == 2 ? 1 : splits == 4 ? 2 : 3;
+  if (at == 0) return sm_count * (form == 1 ? 2 : 1);
+  int& c = clusters[form][at];
+  if (c == 0) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(splits * 1024));
+    cfg.blockDim = dim3(GS_THREADS);
+    cfg.dynamicSmemBytes = form == 0 ? GsSizes<64, 8>::SMEM : form == 1 ? GsSizes<64, 4>::SMEM : GsSizes<128, 6>::SMEM;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)splits; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    auto ask = [&](auto kern) {
+      int n = 0;
+      const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) == cudaSuccess &&
+                      cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess;
+      if (!ok) cudaGetLastError();
+      return ok && n > 0 ? n : 1;
+    };
+    c = form == 0 ? ask(gemm_small_kernel<true, true, 64, 8>)
+                  : form == 1 ? ask(gemm_small_kernel<true, true, 64, 4>) : ask(gemm_small_kernel<true, true, 128, 6>);
+  }
+  return std::min(c * splits, sm_count * (form == 1 ? 2 : 1));
+}
+}  // namespace
+
 GemmSmallPlan gemm_small_plan(const hl_gemm_desc* d, const GemmPlan& big, int sm_count) {
   const int kb = ceil_div(d->k, GS_BK), m_tiles = ceil_div(d->m, GS_BM);
   const long long narrow = (long long)m_tiles * ceil_div(d->n, 64), wide = (long long)m_tiles * ceil_div(d->n, 128);
@@ -299,9 +331,9 @@ GemmSmallPlan gemm_small_plan(const hl_gemm_desc* d, const GemmPlan& big, int sm
     auto take = [&](float t, int bn, bool deep) {
       if (t < best) { best = t; plan = GemmSmallPlan{s, bn, deep}; }
     };
-    if (narrow * s <= sm_count) take(3.0f + 0.17f * steps + shared, 64, true);
-    else if (narrow * s <= 2 * sm_count) take(3.0f + 0.34f * steps + shared, 64, false);
-    if (wide * s <= sm_count) take(4.4f + 0.21f * steps + (s > 1 ? 2.5f : 0.f), 128, false);
+    if (narrow * s <= wave_ctas(0, s, sm_count)) take(3.0f + 0.17f * steps + shared, 64, true);
+    else if (narrow * s <= wave_ctas(1, s, sm_count)) take(3.0f + 0.34f * steps + shared, 64, false);
+    if (wide * s <= wave_ctas(2, s, sm_count)) take(4.4f + 0.21f * steps + (s > 1 ? 2.5f : 0.f), 128, false);
   }
   return plan;
 }

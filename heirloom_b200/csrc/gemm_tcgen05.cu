@@ -516,7 +516,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             for (uint32_t spins = 0;; ++spins) {
               unsigned seen;
               asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(flag) : "memory");
-              if (seen == p.sk_seq) break;
+              if (seen == p.sk_seq) {
+                // This warp is the flag's only reader: it goes back to zero, so that a replay of this launch with the same
+                // number waits again.
+                *const_cast<unsigned*>(flag) = 0u;
+                break;
+              }
               if ((spins & 63u) == 63u) {
                 if (*abort_flag || tc05::global_timer_ns() - t0 > p.wait_limit_ns) { *abort_flag = 1; ok = false; break; }
                 __nanosleep(64);
@@ -1057,8 +1062,9 @@ namespace {
 constexpr size_t kStaticScratchBytes = size_t(32) << 20;
 static __device__ __align__(256) unsigned char g_gemm_static_scratch[kStaticScratchBytes];
 // Flags of the automatic work split (one word per CTA and epilogue warp), apart from the array
-// above so that split-K partial sums never land on them.  Static device memory starts at zero and
-// launch numbers do not repeat within a process, so a stale flag is never mistaken for a fresh one.
+// above so that split-K partial sums never land on them.  Static device memory starts at zero, a
+// flag returns to zero when it has been read, and launch numbers do not repeat within a process
+// (a launch that gave up can leave one behind), so a stale flag is never mistaken for a fresh one.
 constexpr int kStaticFlagCtas = 256;
 static __device__ __align__(256) unsigned g_gemm_static_flags[kStaticFlagCtas * EPI_WARPS];
 

@@ -241,6 +241,7 @@ int hl_ctx_sync(hl_ctx* ctx) {
       // a kernel that gave up did not hand out all of its tiles: the tile counter starts over with the host's copy
       HL_CUDA(cudaMemsetAsync(ctx->gemm_sched, 0, 64, ctx->stream));
       ctx->gemm_sched_base = 0;
+      ctx->faults += 1;  // captured launches repeat their numbers: whoever holds some starts over with fresh ones
     }
     HL_CUDA(cudaStreamSynchronize(ctx->stream));
     hl::set_error(msg);

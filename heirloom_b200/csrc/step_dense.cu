@@ -52,6 +52,40 @@ struct MemoryActs {
   __nv_bfloat16 *wq3 = nullptr, *wg3 = nullptr, *wout3 = nullptr;
 };
 
+// A model's launch sequences as graphs.  A sequence that comes up a second time with the same sizes, scratch arena and GEMM
+// settings is captured and from then on replayed: a small model's step is some sixty launches (and as many tensor maps) of
+// 2 to 4 us of host time each for kernels of 2 to 5 us.  Everything a sequence reads and writes has a fixed address.
+struct GraphKey {
+  int kind, batch, context;
+  const void* workspace;
+  size_t workspace_bytes;
+  unsigned long long wait_limit_ns;
+  unsigned faults;
+  char pairs, dynamic;  // first characters of the GEMM's environment settings
+  bool operator==(const GraphKey& o) const {
+    return kind == o.kind && batch == o.batch && context == o.context && workspace == o.workspace &&
+           workspace_bytes == o.workspace_bytes && wait_limit_ns == o.wait_limit_ns && faults == o.faults && pairs == o.pairs &&
+           dynamic == o.dynamic;
+  }
+};
+enum { GRAPH_STEP = 0, GRAPH_LOSS = 1, GRAPH_WINDOW = 2, GRAPH_DECODE = 3 };
+struct GraphEntry {
+  GraphKey key{};
+  cudaGraphExec_t exec = nullptr;  // null until the sequence has run once plainly
+  Counters counts{};               // what a replay adds to the context's counters
+  unsigned long long used = 0;
+};
+struct GraphCache {
+  std::vector<GraphEntry> entries;
+  unsigned long long clock = 0;
+  void clear() {
+    for (GraphEntry& e : entries)
+      if (e.exec) cudaGraphExecDestroy(e.exec);
+    entries.clear();
+  }
+};
+constexpr size_t kMaxGraphs = 6;
+
 struct LayerActs {
   __nv_bfloat16 *a, *qkv, *o, *r, *c, *h, *g;
   float *lse, *mean1, *rstd1, *mean2, *rstd2;
@@ -150,16 +184,13 @@ struct hl_decoder {
   struct F32Layer {
     float *a, *qkv, *probs, *o, *r, *c, *h, *g;
   };
-  // generation: how many positions of sequence 0 have their keys and values in the activation buffers (0: none), the state
-  // of the next one-token step, and that step as a graph once it has run
+  // generation: how many positions of sequence 0 have their keys and values in the activation buffers (0: none) and the
+  // state of the next one-token step
   int cached = 0;
   long long* decode_state = nullptr;       // device: position, token
   long long* decode_state_host = nullptr;  // pinned
   float* logits_host = nullptr;            // pinned, [vocab], allocated on first use
-  cudaGraphExec_t decode_graph = nullptr;
-  void* decode_graph_workspace = nullptr;  // the scratch arena the graph was captured with
-  unsigned long long decode_launches = 0;  // kernels in it
-  bool decode_warm = false;
+  GraphCache graphs;
   std::vector<float*> xf;  // residual stream per block input, f32
   std::vector<F32Layer> lf;
   float *zf = nullptr, *dlogits_f = nullptr, *d_a = nullptr, *d_b = nullptr, *d_c = nullptr, *d_qkv = nullptr, *d_wide = nullptr;
@@ -1024,6 +1055,68 @@ int backward_f32(hl_decoder* m) {
   return HL_OK;
 }
 
+// Queues the launches of `queue` on the compute stream, from the second time on as a graph.
+template <typename F>
+int run_graphed(hl_decoder* m, int kind, F queue) {
+  hl_ctx* ctx = m->ctx;
+  // collectives and per-kernel timing are host work of the step; the test hook changes a launch's arguments
+  if (nccl_active(ctx) || ctx->profiler || ctx->gemm_skip_kblock >= 0 || m->comm_pending) return queue();
+  auto setting = [](const char* name) { const char* e = getenv(name); return e ? e[0] : '\0'; };
+  const GraphKey key{kind, m->cfg.batch, m->cfg.context, ctx->workspace, ctx->workspace_bytes, ctx->wait_limit_ns, ctx->faults,
+                     setting("HEIRLOOM_GEMM_PAIRS"), setting("HEIRLOOM_GEMM_DYNAMIC")};
+  std::vector<GraphEntry>& entries = m->graphs.entries;
+  GraphEntry* entry = nullptr;
+  for (GraphEntry& e : entries)
+    if (e.key == key) entry = &e;
+  if (!entry) {
+    if (entries.size() < kMaxGraphs) entries.emplace_back();
+    entry = &*std::min_element(entries.begin(), entries.end(), [](const GraphEntry& a, const GraphEntry& b) { return a.used < b.used; });
+    if (entry->exec) {
+      HL_CUDA(cudaStreamSynchronize(ctx->stream));
+      cudaGraphExecDestroy(entry->exec);
+    }
+    *entry = GraphEntry{};
+    entry->key = key;
+    entry->used = ++m->graphs.clock;
+    HL_TRY(queue());
+    // the plain run may have grown the scratch arena
+    entry->key.workspace = ctx->workspace;
+    entry->key.workspace_bytes = ctx->workspace_bytes;
+    return HL_OK;
+  }
+  entry->used = ++m->graphs.clock;
+  if (!entry->exec) {
+    const Counters before = ctx->counters;
+    cudaGraph_t graph = nullptr;
+    HL_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+    const int rc = queue();
+    const cudaError_t ended = cudaStreamEndCapture(ctx->stream, &graph);
+    if (rc != HL_OK) {
+      if (graph) cudaGraphDestroy(graph);
+      return rc;
+    }
+    HL_CUDA(ended);
+    const cudaError_t made = cudaGraphInstantiate(&entry->exec, graph, 0);
+    cudaGraphDestroy(graph);
+    if (made != cudaSuccess) {
+      entry->exec = nullptr;
+      return fail_cuda(made, "cudaGraphInstantiate");
+    }
+    Counters& c = entry->counts;
+    c.launches = ctx->counters.launches - before.launches;
+    c.gemm_tcgen05_launches = ctx->counters.gemm_tcgen05_launches - before.gemm_tcgen05_launches;
+    c.gemm_pair_launches = ctx->counters.gemm_pair_launches - before.gemm_pair_launches;
+    c.attention_launches = ctx->counters.attention_launches - before.attention_launches;
+  } else {
+    ctx->counters.launches += entry->counts.launches;
+    ctx->counters.gemm_tcgen05_launches += entry->counts.gemm_tcgen05_launches;
+    ctx->counters.gemm_pair_launches += entry->counts.gemm_pair_launches;
+    ctx->counters.attention_launches += entry->counts.attention_launches;
+  }
+  HL_CUDA(cudaGraphLaunch(entry->exec, ctx->stream));
+  return HL_OK;
+}
+
 // ---- one-token steps of generation -----------------------------------------------------------------
 // The row of m->decode_state through the model: its q/k/v go to the cache (row `position` of the activations that a
 // full-window forward left), every other value of the row to row 0 of its buffer, the logits to row 0 of m->logits.  Row by
@@ -1349,7 +1442,7 @@ void hl_decoder_destroy(hl_decoder* m) {
   cudaFree(m->params); cudaFree(m->grads); cudaFree(m->m); cudaFree(m->v); cudaFree(m->shadow); cudaFree(m->act_arena);
   if (m->loss_host) cudaFreeHost(m->loss_host);
   if (m->logits_host) cudaFreeHost(m->logits_host);
-  if (m->decode_graph) cudaGraphExecDestroy(m->decode_graph);
+  m->graphs.clear();
   delete m;
 }
 
@@ -1447,16 +1540,18 @@ int hl_decoder_forward_backward(hl_decoder* m, const int64_t* tokens_dev, const 
     HL_CUDA(cudaMemcpyAsync(m->tokens, tokens_dev, sizeof(int64_t) * m->N, cudaMemcpyDeviceToDevice, m->ctx->stream));
   if (targets_dev != m->targets)
     HL_CUDA(cudaMemcpyAsync(m->targets, targets_dev, sizeof(int64_t) * m->N, cudaMemcpyDeviceToDevice, m->ctx->stream));
-  HL_TRY(prepare_token_rows(m));  // data parallel: the union of the ranks' token rows forms while forward runs
-  if (m->cfg.precision == HL_PRECISION_AMP_BF16) {
-    HL_TRY(forward(m));
-    HL_TRY(prepare_value_rows(m));
-    HL_TRY(backward(m));
-  } else {
+  HL_TRY(run_graphed(m, GRAPH_STEP, [m]() -> int {
+    HL_TRY(prepare_token_rows(m));  // data parallel: the union of the ranks' token rows forms while forward runs
+    if (m->cfg.precision == HL_PRECISION_AMP_BF16) {
+      HL_TRY(forward(m));
+      HL_TRY(prepare_value_rows(m));
+      return backward(m);
+    }
     HL_TRY(forward_f32(m));
     HL_TRY(prepare_value_rows(m));
-    HL_TRY(backward_f32(m));
-  }
+    return backward_f32(m);
+  }));
+  m->cached = 0;
   m->launches_last_step = m->ctx->counters.launches - before;
   return HL_OK;
 }
@@ -1727,10 +1822,13 @@ int hl_decoder_eval_loss(hl_decoder* m, const int64_t* tokens_dev, const int64_t
   HL_CUDA(cudaMemcpyAsync(m->targets, targets_dev, sizeof(int64_t) * n, cudaMemcpyDeviceToDevice, m->ctx->stream));
   {
     ScopedShape shape(m, sequences, m->cfg.context);
-    if (m->cfg.precision == HL_PRECISION_AMP_BF16) HL_TRY(forward(m));
-    else HL_TRY(forward_f32(m));
-    HL_TRY(cross_entropy_impl(m->ctx, m->logits, m->cfg.vocab, m->targets, m->N, m->cfg.vocab, 1.0f, m->loss_dev, nullptr,
-                              nullptr, HL_BF16, m->cfg.vocab));
+    HL_TRY(run_graphed(m, GRAPH_LOSS, [m]() -> int {
+      if (m->cfg.precision == HL_PRECISION_AMP_BF16) HL_TRY(forward(m));
+      else HL_TRY(forward_f32(m));
+      return cross_entropy_impl(m->ctx, m->logits, m->cfg.vocab, m->targets, m->N, m->cfg.vocab, 1.0f, m->loss_dev, nullptr,
+                                nullptr, HL_BF16, m->cfg.vocab);
+    }));
+    m->cached = 0;
   }
   return hl_memcpy_d2h(m->ctx, loss_host, m->loss_dev, sizeof(float));
 }
@@ -1743,8 +1841,8 @@ static int window_logits(hl_decoder* m, const int64_t* window, cudaMemcpyKind ki
   HL_CUDA(cudaMemcpyAsync(m->tokens, window, sizeof(int64_t) * window_len, kind, ctx->stream));
   {
     ScopedShape shape(m, 1, window_len);
-    if (m->cfg.precision == HL_PRECISION_AMP_BF16) HL_TRY(forward(m, true));
-    else HL_TRY(forward_f32(m, true));
+    HL_TRY(run_graphed(m, GRAPH_WINDOW, [m]() { return m->cfg.precision == HL_PRECISION_AMP_BF16 ? forward(m, true) : forward_f32(m, true); }));
+    m->cached = 0;
   }
   HL_CUDA(cudaMemcpyAsync(m->logits_host, m->logits, sizeof(float) * (size_t)m->cfg.vocab, cudaMemcpyDeviceToHost, ctx->stream));
   HL_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1777,7 +1875,7 @@ int hl_decoder_decode_next(hl_decoder* m, int64_t token, float* logits_host) {
   m->decode_state_host[1] = token;
   const int position = m->cached;
   m->cached = 0;  // until this step has succeeded
-  auto queue = [&]() -> int {
+  auto queue = [m, ctx]() -> int {
     HL_CUDA(cudaMemcpyAsync(m->decode_state, m->decode_state_host, 2 * sizeof(long long), cudaMemcpyHostToDevice, ctx->stream));
     {
       const int n = m->N;
@@ -1789,34 +1887,7 @@ int hl_decoder_decode_next(hl_decoder* m, int64_t token, float* logits_host) {
     HL_CUDA(cudaMemcpyAsync(m->logits_host, m->logits, sizeof(float) * (size_t)m->cfg.vocab, cudaMemcpyDeviceToHost, ctx->stream));
     return HL_OK;
   };
-  // The step is the same every time (position and token are read from memory), so from the second one on it is replayed as a
-  // graph: sixty launches of a few microseconds each cost the host more than the device.
-  if (m->decode_graph && m->decode_graph_workspace != ctx->workspace) {
-    cudaGraphExecDestroy(m->decode_graph);
-    m->decode_graph = nullptr;
-  }
-  if (!m->decode_warm || ctx->profiler) {
-    HL_TRY(queue());
-    m->decode_warm = true;
-  } else {
-    if (m->decode_graph) {
-      ctx->counters.launches += m->decode_launches;
-    } else {
-      const unsigned long long before = ctx->counters.launches;
-      cudaGraph_t graph = nullptr;
-      HL_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-      const int rc = queue();
-      const cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
-      if (rc != HL_OK) { if (graph) cudaGraphDestroy(graph); return rc; }
-      HL_CUDA(e);
-      const cudaError_t e2 = cudaGraphInstantiate(&m->decode_graph, graph, 0);
-      cudaGraphDestroy(graph);
-      HL_CUDA(e2);
-      m->decode_graph_workspace = ctx->workspace;
-      m->decode_launches = ctx->counters.launches - before;
-    }
-    HL_CUDA(cudaGraphLaunch(m->decode_graph, ctx->stream));
-  }
+  HL_TRY(run_graphed(m, GRAPH_DECODE, queue));  // position and token are read from memory: the same sequence every time
   HL_CUDA(cudaStreamSynchronize(ctx->stream));
   ctx->counters.h2d_bytes += 2 * sizeof(long long);
   ctx->counters.d2h_bytes += sizeof(float) * (size_t)m->cfg.vocab;
