@@ -340,6 +340,16 @@ int fold_batch_flush(hl_ctx* ctx, FoldBatch* batch) {
   return HL_OK;
 }
 
+int fold_batch_room(hl_ctx* ctx, FoldBatch* batch, size_t elems, float** out) {
+  *out = fold_batch_reserve(batch, elems);
+  if (!*out && batch && batch->n > 0) {
+    int rc = fold_batch_flush(ctx, batch);
+    if (rc != HL_OK) return rc;
+    *out = fold_batch_reserve(batch, elems);
+  }
+  return HL_OK;
+}
+
 bool layer_norm_fast_applicable(int x_dtype, int y_dtype, int features, const void* x, const void* y) {
   return x_dtype == HL_BF16 && y_dtype == HL_BF16 && features % 8 == 0 && features <= 1024 &&
          ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
@@ -372,10 +382,12 @@ int layer_norm_backward_fast(hl_ctx* ctx, const void* x, const float* gamma, con
   int blocks = std::min(2 * ctx->sm_count, ceil_div(rows, groups));
   const int rows_per_block = ceil_div(rows, blocks);
   blocks = ceil_div(rows, rows_per_block);
-  float* partial = fold_batch_reserve(defer, (size_t)blocks * 3 * features);
+  float* partial = nullptr;
+  int rc = fold_batch_room(ctx, defer, (size_t)blocks * 3 * features, &partial);
+  if (rc != HL_OK) return rc;
   const bool deferred = partial != nullptr;
   if (!deferred) {
-    int rc = ensure_workspace(ctx, sizeof(float) * (size_t)blocks * 3 * features);
+    rc = ensure_workspace(ctx, sizeof(float) * (size_t)blocks * 3 * features);
     if (rc != HL_OK) return rc;
     partial = reinterpret_cast<float*>(ctx->workspace);
   }
@@ -415,10 +427,12 @@ int colsum_fast(hl_ctx* ctx, const void* g, int dtype, float* out, int rows, int
   int slabs = std::max(1, std::min(std::min(64, ceil_div(rows, ROW_WARPS * 4)), (ctx->sm_count * 4) / col_blocks));
   const int rows_per_block = ceil_div(rows, slabs);
   slabs = ceil_div(rows, rows_per_block);
-  float* partial = fold_batch_reserve(defer, (size_t)slabs * cols);
+  float* partial = nullptr;
+  int rc = fold_batch_room(ctx, defer, (size_t)slabs * cols, &partial);
+  if (rc != HL_OK) return rc;
   const bool deferred = partial != nullptr;
   if (!deferred) {
-    int rc = ensure_workspace(ctx, sizeof(float) * (size_t)slabs * cols);
+    rc = ensure_workspace(ctx, sizeof(float) * (size_t)slabs * cols);
     if (rc != HL_OK) return rc;
     partial = reinterpret_cast<float*>(ctx->workspace);
   }

@@ -23,15 +23,15 @@ constexpr int GS_BM = 128, GS_BK = 64;
 constexpr int GS_THREADS = 256;
 constexpr int GS_A_BYTES = GS_BM * GS_BK * 2;
 constexpr int GS_MAX_STAGES = 8;
-constexpr int GS_BATCH = 8;  // epilogue passes whose residual rows are requested together
 
 template <int BN, int STAGES>
 struct GsSizes {
   static constexpr int STAGE_BYTES = GS_A_BYTES + BN * GS_BK * 2;   // 24 / 32 KB
   static constexpr int DATA = STAGES * STAGE_BYTES;
   static constexpr int LD = BN + 4;                                 // accumulator rows in shared memory: conflict-free writes
-  static_assert(GS_BM * LD * 4 <= DATA, "the accumulator reuses the stages");
-  static constexpr int SMEM = DATA + 1024 + 256;
+  static_assert((GS_BM * LD + GS_BM) * 4 <= DATA, "the accumulator reuses the stages");
+  static constexpr int ONES = 2048;                                 // 16 x 64 bf16 of 1.0: the right operand of the row sums
+  static constexpr int SMEM = DATA + 1024 + ONES + 256;
   static constexpr int CTAS_PER_SM = SMEM <= 113 * 1024 ? 2 : 1;
 };
 
@@ -49,6 +49,7 @@ struct GsParams {
   long long ldc;
   __nv_bfloat16* aux_out;
   long long ld_aux_out;
+  float* row_sum;  // [m] or null: sum over the contraction of A's rows
   int* status;
 };
 
@@ -64,7 +65,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   using Z = GsSizes<BN, STAGES>;
   extern __shared__ uint8_t gs_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gs_raw) + 1023) & ~uintptr_t(1023));
-  GsTail* tail = reinterpret_cast<GsTail*>(smem + Z::DATA);
+  GsTail* tail = reinterpret_cast<GsTail*>(smem + Z::DATA + Z::ONES);
   volatile int* abort_flag = &tail->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)blockIdx.x % p.splits, tile = (int)blockIdx.x / p.splits;
@@ -82,10 +83,16 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     tc05::tma_prefetch_desc(&map_a);
     tc05::tma_prefetch_desc(&map_b);
   }
+  // Row sums (a bias gradient beside its weight gradient): the tiles of the first column multiply A by a block of ones as
+  // well, sixteen more columns of tensor memory.
+  const bool sums = p.row_sum != nullptr && n0 == 0;
   if (warp == 1) {
-    tc05::tmem_alloc(&tail->tmem_base, BN);
+    tc05::tmem_alloc(&tail->tmem_base, 2 * BN);
     tc05::tmem_relinquish();
   }
+  if (sums && threadIdx.x >= 128)
+    reinterpret_cast<uint4*>(smem + Z::DATA)[threadIdx.x - 128] = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+  tc05::fence_proxy_async_smem();
   tc05::tc_fence_before_sync();
   __syncthreads();
   tc05::tc_fence_after_sync();
@@ -95,8 +102,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
   // This thread's four columns, and the rows it finishes of this CTA's share of the tile; the first residual or
   // pre-activation rows are requested here, before the roles' loops.
-  constexpr int QUADS = BN / 4, ROWS_PER_PASS = GS_THREADS / QUADS, MAX_PASSES = GS_BM / ROWS_PER_PASS;
-  static_assert(MAX_PASSES % GS_BATCH == 0, "whole batches of passes");
+  constexpr int QUADS = BN / 4, ROWS_PER_PASS = GS_THREADS / QUADS;
   const int rows_mine = GS_BM / p.splits, row_first = rank * rows_mine;
   const int quad = threadIdx.x % QUADS, sub = threadIdx.x / QUADS;
   const int col = n0 + quad * 4;
@@ -104,17 +110,15 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const bool need_aux = p.epilogue == HL_EPI_BIAS_RESIDUAL || p.epilogue == HL_EPI_DGELU;
   float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
   if (p.bias && col_ok) bias = __ldg(reinterpret_cast<const float4*>(p.bias + col));
-  uint2 aux[GS_BATCH];
-  auto request_aux = [&](int first) {
-#pragma unroll
-    for (int i = 0; i < GS_BATCH; ++i) {
-      const int r = sub + (first + i) * ROWS_PER_PASS, row = m0 + row_first + r;
-      aux[i] = r < rows_mine && row < p.m && col_ok
-                   ? *reinterpret_cast<const uint2*>(p.aux_in + (size_t)row * p.ld_aux_in + col)
-                   : make_uint2(0u, 0u);
-    }
+  // one pass ahead; a rolled loop, because a CTA that lands on an SM which has not run this kernel yet pays for every cache
+  // line of its code
+  auto fetch_aux = [&](int i) {
+    const int r = sub + i * ROWS_PER_PASS, row = m0 + row_first + r;
+    return need_aux && r < rows_mine && row < p.m && col_ok
+               ? *reinterpret_cast<const uint2*>(p.aux_in + (size_t)row * p.ld_aux_in + col)
+               : make_uint2(0u, 0u);
   };
-  if (need_aux) request_aux(0);
+  uint2 aux = fetch_aux(0);
 
   if (warp == 0) {
     if (tc05::elect_one()) {
@@ -144,6 +148,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   } else if (warp == 1) {
     if (tc05::elect_one()) {
       constexpr uint32_t idesc = tc05::instr_desc_bf16_f32(GS_BM, BN, A_MN, B_MN);
+      constexpr uint32_t idesc_sums = tc05::instr_desc_bf16_f32(GS_BM, 16, A_MN, false);
+      const uint64_t ones = tc05::smem_desc_sw128(tc05::smem_u32(smem + Z::DATA), 16, 1024);
       bool ok = true;
       for (int kb = kb0; kb < kb1; ++kb) {
         const int i = kb - kb0, stage = i % STAGES;
@@ -157,6 +163,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           const uint64_t db = B_MN ? tc05::smem_desc_sw128(sb + ks * (16 * 128), GS_BK * 128, 1024)
                                    : tc05::smem_desc_sw128(sb + ks * 32, 16, 1024);
           tc05::umma_ss(tmem, da, db, idesc, (i > 0 || ks > 0) ? 1u : 0u);
+          if (sums) tc05::umma_ss(tmem + BN, da, ones, idesc_sums, (i > 0 || ks > 0) ? 1u : 0u);
         }
         tc05::umma_commit(&tail->empty[stage]);
       }
@@ -189,21 +196,28 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         *reinterpret_cast<uint4*>(acc + r * Z::LD + c0 + i) = make_uint4(bits[i], bits[i + 1], bits[i + 2], bits[i + 3]);
     }
   }
+  float* acc_sums = acc + GS_BM * Z::LD;
+  if (sums && warp < 4) {
+    uint32_t bits[8];
+    if (have) {
+      tc05::tmem_ld_32x32b_x8(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)BN, bits);
+      tc05::tmem_ld_wait();
+    }
+    acc_sums[warp * 32 + lane] = have ? __uint_as_float(bits[0]) : 0.f;
+  }
   tc05::tc_fence_before_sync();
   cg::cluster_group cluster = cg::this_cluster();
   if (p.splits > 1) cluster.sync(); else __syncthreads();
   if (warp == 1) {
     tc05::tc_fence_after_sync();
-    tc05::tmem_dealloc(tmem, BN);
+    tc05::tmem_dealloc(tmem, 2 * BN);
   }
 #pragma unroll 1
-  for (int first = 0; first * ROWS_PER_PASS < rows_mine; first += GS_BATCH) {
-  if (need_aux && first > 0) request_aux(first);
-#pragma unroll
-  for (int i = 0; i < GS_BATCH; ++i) {
-    const int r = sub + (first + i) * ROWS_PER_PASS;
-    if ((first + i) * ROWS_PER_PASS >= rows_mine) break;
+  for (int i = 0; i * ROWS_PER_PASS < rows_mine; ++i) {
+    const int r = sub + i * ROWS_PER_PASS;
     const int row = m0 + row_first + r;
+    const uint2 aux_now = aux;
+    aux = fetch_aux(i + 1);
     if (r >= rows_mine || row >= p.m || !col_ok) continue;
     float* at = acc + (row_first + r) * Z::LD + quad * 4;
     float v[4];
@@ -227,7 +241,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       g.y = pack_bf16x2(gelu_fwd_fast(v[2]), gelu_fwd_fast(v[3]));
       *reinterpret_cast<uint2*>(p.aux_out + (size_t)row * p.ld_aux_out + col) = g;
     } else if (need_aux) {
-      const float2 a0 = unpack_bf16x2(aux[i].x), a1 = unpack_bf16x2(aux[i].y);
+      const float2 a0 = unpack_bf16x2(aux_now.x), a1 = unpack_bf16x2(aux_now.y);
       const float a[4] = {a0.x, a0.y, a1.x, a1.y};
 #pragma unroll
       for (int e = 0; e < 4; ++e)
@@ -239,6 +253,11 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     else
       *reinterpret_cast<float4*>(static_cast<float*>(p.c) + (size_t)row * p.ldc + col) = make_float4(v[0], v[1], v[2], v[3]);
   }
+  if (sums && threadIdx.x < rows_mine && m0 + row_first + (int)threadIdx.x < p.m) {
+    float v = 0.f;
+    float* at = acc_sums + row_first + threadIdx.x;
+    for (int s = 0; s < p.splits; ++s) v += p.splits > 1 ? *cluster.map_shared_rank(at, s) : *at;
+    p.row_sum[m0 + row_first + threadIdx.x] = v;
   }
   if (p.splits > 1) cluster.sync();  // no CTA leaves while another still reads its sums
   if (!ok || *abort_flag) {
@@ -340,7 +359,7 @@ GemmSmallPlan gemm_small_plan(const hl_gemm_desc* d, const GemmPlan& big, int sm
 
 // Arguments have been checked by the caller (gemm_bf16_run).
 int gemm_small_run(hl_ctx* ctx, const hl_gemm_desc* d, const GemmSmallPlan& plan, const void* a, const void* b, void* c,
-                   const float* bias, const void* aux_in, void* aux_out) {
+                   const float* bias, const void* aux_in, void* aux_out, float* row_sum) {
   const bool a_mn = d->a_layout == HL_MN_MAJOR, b_mn = d->b_layout == HL_MN_MAJOR;
   const int a_k = d->a_k_period > 0 ? d->a_k_period : d->k, b_k = d->b_k_period > 0 ? d->b_k_period : d->k;
   GsParams p{};
@@ -360,6 +379,7 @@ int gemm_small_run(hl_ctx* ctx, const hl_gemm_desc* d, const GemmSmallPlan& plan
   p.c = c; p.ldc = d->ldc;
   p.aux_out = static_cast<__nv_bfloat16*>(aux_out);
   p.ld_aux_out = d->ld_aux_out > 0 ? d->ld_aux_out : d->ldc;
+  p.row_sum = row_sum;
   p.status = ctx->status_dev;
   CUtensorMap ma, mb;
   int rc = a_mn ? make_tensor_map_bf16_2d(&ma, a, (uint64_t)d->m, (uint64_t)a_k, (uint64_t)d->lda, 64, GS_BK)

@@ -821,8 +821,8 @@ size_t gemm_stream_flag_bytes(int sm_count) { return (size_t)sm_count * EPI_WARP
 
 static std::atomic<unsigned> g_stream_launch_number{0};
 
-int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, void* c, const float* bias,
-                  const void* aux_in, void* aux_out, float* workspace, size_t workspace_bytes, unsigned* stream_flags) {
+static int check_gemm(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, void* c, const float* bias,
+                      const void* aux_in, void* aux_out) {
   HL_REQUIRE(ctx && d, "hl_gemm_bf16: null argument");
   HL_REQUIRE(d->m > 0 && d->n > 0 && d->k > 0, "hl_gemm_bf16: m, n, k must be positive");
   HL_REQUIRE(a && b && c, "hl_gemm_bf16: null operand pointer");
@@ -861,7 +861,18 @@ int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void*
     HL_REQUIRE(ld_aux_in % 8 == 0 && ld_aux_in >= d->n && (reinterpret_cast<uintptr_t>(aux_in) & 15) == 0,
                "hl_gemm_bf16: aux_in must be 16-byte aligned with a row stride that is a multiple of 8");
   if (bias) HL_REQUIRE((reinterpret_cast<uintptr_t>(bias) & 15) == 0, "hl_gemm_bf16: bias must be 16-byte aligned");
+  return HL_OK;
+}
 
+int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, void* c, const float* bias,
+                  const void* aux_in, void* aux_out, float* workspace, size_t workspace_bytes, unsigned* stream_flags) {
+  int rc = check_gemm(ctx, d, a, b, c, bias, aux_in, aux_out);
+  if (rc != HL_OK) return rc;
+  const bool a_mn = d->a_layout == HL_MN_MAJOR, b_mn = d->b_layout == HL_MN_MAJOR;
+  const int a_k = d->a_k_period > 0 ? d->a_k_period : d->k;  // contraction extent that A really holds
+  const int b_k = d->b_k_period > 0 ? d->b_k_period : d->k;
+  const long long ld_aux_in = d->ld_aux_in > 0 ? d->ld_aux_in : d->ldc;
+  const long long ld_aux_out = d->ld_aux_out > 0 ? d->ld_aux_out : d->ldc;
   const int sms = persistent_sms(ctx);
   const GemmPlan plan = gemm_plan(d, sms);
   const GemmSmallPlan small = small_plan(ctx, d, plan, sms);
@@ -924,7 +935,6 @@ int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void*
   }
 
   CUtensorMap ma, mb, mc, maux;
-  int rc;
   if (a_mn) rc = make_tensor_map_bf16_2d(&ma, a, (uint64_t)d->m, (uint64_t)a_k, (uint64_t)d->lda, 64, BK);
   else      rc = make_tensor_map_bf16_2d(&ma, a, (uint64_t)a_k, (uint64_t)d->m, (uint64_t)d->lda, BK, BM);
   if (rc != HL_OK) return rc;
@@ -1029,6 +1039,23 @@ int gemm_bf16_ctx(hl_ctx* ctx, const hl_gemm_desc* desc, const void* a, const vo
   }
   return gemm_bf16_run(ctx, desc, a, b, c, bias, aux_in, aux_out, reinterpret_cast<float*>(ctx->workspace),
                        ctx->workspace_bytes, reinterpret_cast<unsigned*>(ctx->gemm_flags));
+}
+}  // namespace hl
+
+namespace hl {
+bool gemm_bf16_small_applies(hl_ctx* ctx, const hl_gemm_desc* d) {
+  const int sms = persistent_sms(ctx);
+  return small_plan(ctx, d, gemm_plan(d, sms), sms).splits > 0;
+}
+int gemm_bf16_row_sums(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, void* c, float* row_sum, bool* done) {
+  *done = false;
+  int rc = check_gemm(ctx, d, a, b, c, nullptr, nullptr, nullptr);
+  if (rc != HL_OK) return rc;
+  const int sms = persistent_sms(ctx);
+  const GemmSmallPlan small = small_plan(ctx, d, gemm_plan(d, sms), sms);
+  if (small.splits == 0) return HL_OK;
+  *done = true;
+  return gemm_small_run(ctx, d, small, a, b, c, nullptr, nullptr, nullptr, row_sum);
 }
 }  // namespace hl
 

@@ -24,10 +24,14 @@ struct GemmSmallPlan {
 };
 GemmSmallPlan gemm_small_plan(const hl_gemm_desc* d, const GemmPlan& big, int sm_count);
 int gemm_small_run(hl_ctx* ctx, const hl_gemm_desc* d, const GemmSmallPlan& plan, const void* a, const void* b, void* c,
-                   const float* bias, const void* aux_in, void* aux_out);
+                   const float* bias, const void* aux_in, void* aux_out, float* row_sum = nullptr);
 // The GEMM with its scratch taken from (and grown in) the context.
 int gemm_bf16_ctx(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, void* c, const float* bias,
                   const void* aux_in, void* aux_out);
+// A plain product with the sums of A's rows over the contraction beside it (a weight gradient and its bias gradient), where
+// that costs no launch of its own; *done tells whether it was one of those, otherwise nothing has been launched.
+bool gemm_bf16_small_applies(hl_ctx* ctx, const hl_gemm_desc* d);
+int gemm_bf16_row_sums(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, void* c, float* row_sum, bool* done);
 
 // Column reductions (layer-norm parameter gradients, bias gradients) end in a fold of per-block partial rows.  A
 // caller that runs several of them before anyone reads the results hands in a FoldBatch: the kernels then leave their
@@ -38,14 +42,17 @@ struct FoldJob {
   float *o0, *o1, *o2;   // column c goes to o(c / features)[c % features]; null outputs are skipped
 };
 struct FoldBatch {
-  static constexpr int kMaxJobs = 8;
+  static constexpr int kMaxJobs = 16;
   FoldJob jobs[kMaxJobs];
   int n = 0;
   float* scratch = nullptr;  // device memory, `capacity` floats
   size_t capacity = 0, used = 0;
 };
-// Room for `elems` partial sums in the batch, or null when the batch is absent or full (the caller then folds at once).
+// Room for `elems` partial sums in the batch, or null when the batch is absent or full.
 float* fold_batch_reserve(FoldBatch* batch, size_t elems);
+// The same, folding what the batch holds when it is full; null (the caller folds at once) when there is no batch or it is too
+// small for this reduction.
+int fold_batch_room(hl_ctx* ctx, FoldBatch* batch, size_t elems, float** out);
 void fold_batch_add(FoldBatch* batch, const float* partial, int blocks, int total, int features, float* o0, float* o1,
                     float* o2);
 int fold_batch_flush(hl_ctx* ctx, FoldBatch* batch);
@@ -69,7 +76,7 @@ bool colsum_fast_applicable(int dtype, int cols, const void* g);
 int colsum_fast(hl_ctx* ctx, const void* g, int dtype, float* out, int rows, int cols, FoldBatch* defer = nullptr);
 int cross_entropy_impl(hl_ctx* ctx, const float* logits, long long ld, const int64_t* targets, int rows, int classes,
                        float grad_scale, float* loss_dev, float* row_loss, void* dlogits, int dlogits_dtype,
-                       long long ld_dlogits);
+                       long long ld_dlogits, float* loss_host = nullptr);
 
 int flash_attention_forward_impl(hl_ctx* ctx, const void* q, const void* k, const void* v, long long ld_qkv, void* out,
                                  long long ld_out, float* lse, int batch, int time, int n_heads, int head_dim);

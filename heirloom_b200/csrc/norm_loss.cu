@@ -284,14 +284,41 @@ __global__ void position_grad_kernel(const float* __restrict__ grad_out, float* 
   pos_grad[i] += (float)s;
 }
 
+// The mean of the row losses, taken by the block that finishes last (a ticket counter, back at zero afterwards) in a fixed
+// order; a kernel of its own for it cost 2 to 10 us a step.  `out_host` may be mapped host memory.
+struct MeanLoss {
+  float* out;
+  float* out_host;
+  unsigned* ticket;
+};
+__device__ __forceinline__ void mean_when_last(const float* row_loss, int rows, const MeanLoss& mean) {
+  if (!mean.out) return;
+  __shared__ double sums[32];
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(mean.ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double acc = 0.0;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < rows; i += blockDim.x) acc += (double)__ldcg(row_loss + i);
+  acc = block_sum(acc, sums);
+  if (threadIdx.x == 0) {
+    const float value = (float)(acc / (double)rows);
+    *mean.out = value;
+    if (mean.out_host) *mean.out_host = value;
+    *mean.ticket = 0u;
+  }
+}
+
 // ---- cross-entropy --------------------------------------------------------------------------
 // One block per row.  Pass 1: online max / sum of exponentials; pass 2 (row still in L2):
 // dlogits = (softmax - onehot) * scale.  Acc = double for the f32 parity route.
 template <typename Acc, typename DT>
-__global__ void cross_entropy_kernel(const float* __restrict__ logits, long long ld, const int64_t* __restrict__ targets,
-                                     int rows, int classes, float scale, float* __restrict__ row_loss,
-                                     DT* __restrict__ dlogits, long long ld_d, int* __restrict__ status) {
-  pdl_begin();
+__device__ __forceinline__ void cross_entropy_row(const float* logits, long long ld, const int64_t* targets, int classes, float scale,
+                                                  float* row_loss, DT* dlogits, long long ld_d, int* status) {
   __shared__ Acc sm[32];
   const int row = blockIdx.x;
   const float* z = logits + (size_t)row * ld;
@@ -345,6 +372,15 @@ __global__ void cross_entropy_kernel(const float* __restrict__ logits, long long
   }
 }
 
+template <typename Acc, typename DT>
+__global__ void cross_entropy_kernel(const float* __restrict__ logits, long long ld, const int64_t* __restrict__ targets,
+                                     int rows, int classes, float scale, float* row_loss,
+                                     DT* __restrict__ dlogits, long long ld_d, int* __restrict__ status, const MeanLoss mean) {
+  pdl_begin();
+  cross_entropy_row<Acc>(logits, ld, targets, classes, scale, row_loss, dlogits, ld_d, status);
+  mean_when_last(row_loss, rows, mean);
+}
+
 // bf16-gradient route: persistent blocks walk rows, so only a few hundred rows (tens of MB)
 // are in flight and the second read of a row is served by L2.  Pass 1 is an online
 // max / sum-of-exponentials (one read), pass 2 writes dlogits = (softmax - onehot) * scale.
@@ -355,8 +391,8 @@ constexpr int CE_THREADS = 512;
 constexpr int CE_UNROLL = 7;
 __global__ void __launch_bounds__(CE_THREADS, 2)
 cross_entropy_online_kernel(const float* __restrict__ logits, long long ld, const int64_t* __restrict__ targets,
-                            int rows, int classes, float scale, float* __restrict__ row_loss,
-                            __nv_bfloat16* __restrict__ dlogits, long long ld_d, int* __restrict__ status) {
+                            int rows, int classes, float scale, float* row_loss,
+                            __nv_bfloat16* __restrict__ dlogits, long long ld_d, int* __restrict__ status, const MeanLoss mean) {
   pdl_begin();
   __shared__ float sm[32];
   constexpr float kLog2e = 1.4426950408889634f;
@@ -418,15 +454,7 @@ cross_entropy_online_kernel(const float* __restrict__ logits, long long ld, cons
     }
     __syncthreads();  // sm is reused by the next row
   }
-}
-
-__global__ void mean_rows_kernel(const float* __restrict__ row_loss, int rows, float* __restrict__ out) {
-  pdl_begin();
-  __shared__ double sm[32];
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < rows; i += blockDim.x) acc += (double)row_loss[i];
-  acc = block_sum(acc, sm);
-  if (threadIdx.x == 0) out[0] = (float)(acc / (double)rows);
+  mean_when_last(row_loss, rows, mean);
 }
 
 }  // namespace
@@ -495,11 +523,10 @@ int layer_norm_backward_impl(hl_ctx* ctx, const void* x, int x_dtype, const floa
     own.capacity = ctx->workspace_bytes / sizeof(float);
     defer = &own;
   }
-  float* partial = fold_batch_reserve(defer, (size_t)blocks * 2 * features);
-  if (!partial) {
-    int rc = fold_batch_flush(ctx, defer);
+  float* partial = nullptr;
+  {
+    int rc = fold_batch_room(ctx, defer, (size_t)blocks * 2 * features, &partial);
     if (rc != HL_OK) return rc;
-    partial = fold_batch_reserve(defer, (size_t)blocks * 2 * features);
     HL_REQUIRE(partial, "hl_layer_norm_backward: fold scratch is too small");
   }
   const size_t smem = sizeof(float) * LNB_WARPS * 2 * (size_t)features;
@@ -539,7 +566,7 @@ int layer_norm_backward_impl(hl_ctx* ctx, const void* x, int x_dtype, const floa
 
 int cross_entropy_impl(hl_ctx* ctx, const float* logits, long long ld, const int64_t* targets, int rows, int classes,
                        float grad_scale, float* loss_dev, float* row_loss, void* dlogits, int dlogits_dtype,
-                       long long ld_dlogits) {
+                       long long ld_dlogits, float* loss_host) {
   HL_REQUIRE(ctx && logits && targets, "hl_cross_entropy: null argument");
   HL_REQUIRE(rows > 0 && classes > 0, "hl_cross_entropy: requires non-empty batch/classes");
   HL_REQUIRE(ld >= classes, "hl_cross_entropy: row stride smaller than the class count");
@@ -556,25 +583,21 @@ int cross_entropy_impl(hl_ctx* ctx, const float* logits, long long ld, const int
   const float scale = grad_scale / (float)rows;
   ProfileScope prof(ctx, HL_PROF_LOSS, (double)rows * classes * (4.0 + (dlogits ? (double)dtype_size(dlogits_dtype) : 0.0)));
   const int threads = classes >= 4096 ? 512 : 256;
+  const MeanLoss mean{loss_dev, loss_host, ctx->gemm_sched + 8};  // a word of the context's zeroed counters
   const bool online_ok = (!dlogits || dlogits_dtype == HL_BF16) && classes % 4 == 0 && ld % 4 == 0 && ld_dlogits % 4 == 0 &&
                          (reinterpret_cast<uintptr_t>(logits) & 15) == 0 && (reinterpret_cast<uintptr_t>(dlogits) & 7) == 0 &&
                          classes >= 1024;
   if (online_ok && (dlogits || dlogits_dtype == HL_BF16))
     pdl(cross_entropy_online_kernel, std::min(rows, ctx->sm_count * 2), CE_THREADS, 0, ctx->stream)(
-        logits, ld, targets, rows, classes, scale, rl, (__nv_bfloat16*)dlogits, ld_dlogits, ctx->status_dev);
+        logits, ld, targets, rows, classes, scale, rl, (__nv_bfloat16*)dlogits, ld_dlogits, ctx->status_dev, mean);
   else if (dlogits && dlogits_dtype == HL_BF16)
     pdl(cross_entropy_kernel<float, __nv_bfloat16>, rows, threads, 0, ctx->stream)(
-        logits, ld, targets, rows, classes, scale, rl, (__nv_bfloat16*)dlogits, ld_dlogits, ctx->status_dev);
+        logits, ld, targets, rows, classes, scale, rl, (__nv_bfloat16*)dlogits, ld_dlogits, ctx->status_dev, mean);
   else
     pdl(cross_entropy_kernel<double, float>, rows, threads, 0, ctx->stream)(
-        logits, ld, targets, rows, classes, scale, rl, (float*)dlogits, ld_dlogits, ctx->status_dev);
+        logits, ld, targets, rows, classes, scale, rl, (float*)dlogits, ld_dlogits, ctx->status_dev, mean);
   HL_LAUNCH_CHECK("cross_entropy_kernel");
   count_launch(ctx);
-  if (loss_dev) {
-    pdl(mean_rows_kernel, 1, 1024, 0, ctx->stream)(rl, rows, loss_dev);
-    HL_LAUNCH_CHECK("mean_rows_kernel");
-    count_launch(ctx);
-  }
   return HL_OK;
 }
 

@@ -88,6 +88,7 @@ constexpr size_t kMaxGraphs = 6;
 
 struct LayerActs {
   __nv_bfloat16 *a, *qkv, *o, *r, *c, *h, *g;
+  __nv_bfloat16 *dy, *dh, *dr, *dqkv;  // bf16 gradients of the block output, h, r and qkv; shared by the layers unless forked
   float *lse, *mean1, *rstd1, *mean2, *rstd2;
 };
 
@@ -112,13 +113,19 @@ struct hl_decoder {
   size_t act_bytes = 0;
   std::vector<__nv_bfloat16*> x;  // x[l] is the input of block l; x[L] the final residual stream
   std::vector<LayerActs> la;
-  __nv_bfloat16 *z = nullptr, *dlogits = nullptr, *dxb = nullptr, *dh = nullptr, *dob = nullptr, *dqkv = nullptr;
+  __nv_bfloat16 *z = nullptr, *dlogits = nullptr, *dob = nullptr, *dxb0 = nullptr;
   // head sizes other than 64 and 128 on the bf16 route: attention runs through the f32 kernels, whose probabilities share
   // one buffer
   bool flash_ok = true;
   float* fa_probs = nullptr;
   float *logits = nullptr, *meanf = nullptr, *rstdf = nullptr, *dx0 = nullptr, *dx1 = nullptr, *dtmp = nullptr;
   int64_t *tokens = nullptr, *targets = nullptr;
+  // Weight gradients beside the backward's chain of input gradients (they depend on it, nothing depends on them): on a second
+  // stream, reading operands that every layer has its own copy of.
+  bool fork_ok = false;
+  cudaStream_t side_stream = nullptr;
+  cudaEvent_t fork_event = nullptr, join_event = nullptr;
+  bool forked = false;  // work has been queued on the side stream since the last join
   FoldBatch fold;  // column reductions of one block's backward, folded by one launch before its buckets are flushed
   float* loss_dev = nullptr;
   float* loss_host = nullptr;  // pinned
@@ -367,6 +374,10 @@ void plan_memory_buffers(hl_decoder* m, uint8_t*& cur) {
   m->m_sel_right = carve<int64_t>(cur, all);
 }
 
+// Operand copies of a step whose weight gradients may run beside the chain of input gradients: what a model of a few
+// thousand tokens needs.  Above it the products fill the chip and the copies would be gigabytes.
+constexpr size_t kForkBytes = size_t(256) << 20;
+
 int plan_activations(hl_decoder* m, bool measure_only, size_t* bytes_out) {
   const hl_decoder_config& c = m->cfg;
   const size_t N = (size_t)m->N, d = c.d_model, F = c.d_ff, V = c.vocab, L = c.n_layers;
@@ -398,10 +409,20 @@ int plan_activations(hl_decoder* m, bool measure_only, size_t* bytes_out) {
   m->dx0 = carve<float>(cur, N * d);
   m->dx1 = carve<float>(cur, N * d);
   m->dtmp = carve<float>(cur, N * d);
-  m->dxb = carve<__nv_bfloat16>(cur, N * d);
-  m->dh = carve<__nv_bfloat16>(cur, N * F);
   m->dob = carve<__nv_bfloat16>(cur, N * d);
-  m->dqkv = carve<__nv_bfloat16>(cur, N * 3 * d);
+  m->dxb0 = carve<__nv_bfloat16>(cur, N * d);  // gradient of the embeddings' sum: written like a block output's, read by nobody
+  m->fork_ok = N * (F + 5 * d) * 2 * L <= kForkBytes;
+  for (size_t l = 0; l < L; ++l) {
+    LayerActs& a = m->la[l];
+    if (l > 0 && !m->fork_ok) {
+      a.dy = m->la[0].dy; a.dh = m->la[0].dh; a.dr = m->la[0].dr; a.dqkv = m->la[0].dqkv;
+      continue;
+    }
+    a.dy = carve<__nv_bfloat16>(cur, N * d);
+    a.dh = carve<__nv_bfloat16>(cur, N * F);
+    a.dr = carve<__nv_bfloat16>(cur, N * d);
+    a.dqkv = carve<__nv_bfloat16>(cur, N * 3 * d);
+  }
   if (!m->flash_ok) {
     m->fa_probs = carve<float>(cur, (size_t)c.batch * c.n_heads * c.context * c.context);
   }
@@ -414,7 +435,7 @@ int plan_activations(hl_decoder* m, bool measure_only, size_t* bytes_out) {
     const size_t wide = m->has_memory ? std::max(F, (size_t)(m->mem.key_dim + m->mem.value_dim)) : F;
     const size_t layer = 2 * ln + 64 * (wide + 3 * d) + 4 * 64;
     const size_t head = ln + 64 * V + 2 * 64;
-    m->fold.capacity = std::max(layer, head);
+    m->fold.capacity = std::max(4 * layer, head);  // several layers' reductions wait for one fold
     m->fold.scratch = carve<float>(cur, m->fold.capacity);
     m->fold.n = 0;
     m->fold.used = 0;
@@ -496,6 +517,51 @@ struct Gemm {
     int _rc = (expr);           \
     if (_rc != HL_OK) return _rc; \
   } while (0)
+
+// While one of these lives, launches of the context go to the side stream, which first waits for everything queued on the
+// compute stream so far.
+struct SideStream {
+  hl_decoder* m;
+  cudaStream_t main;
+  int rc = HL_OK;
+  explicit SideStream(hl_decoder* model) : m(model), main(model->ctx->stream) {
+    cudaError_t e = cudaEventRecord(m->fork_event, main);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(m->side_stream, m->fork_event, 0);
+    if (e != cudaSuccess) rc = fail_cuda(e, "fork to the side stream");
+    m->ctx->stream = m->side_stream;
+    m->forked = true;
+  }
+  ~SideStream() { m->ctx->stream = main; }
+};
+
+int join_side(hl_decoder* m) {
+  if (!m->forked) return HL_OK;
+  m->forked = false;
+  HL_CUDA(cudaEventRecord(m->join_event, m->side_stream));
+  HL_CUDA(cudaStreamWaitEvent(m->ctx->stream, m->join_event, 0));
+  return HL_OK;
+}
+
+// dw[n_out, n_in] = dyᵀ · x and, when asked for, db = column sums of dy (both bf16, one row per token)
+int weight_gradient(hl_decoder* m, const __nv_bfloat16* dy, int n_out, const __nv_bfloat16* x, int n_in, float* dw, float* db) {
+  hl_gemm_desc d{};
+  d.m = n_out; d.n = n_in; d.k = m->N;
+  d.a_layout = HL_MN_MAJOR; d.b_layout = HL_MN_MAJOR;
+  d.lda = n_out; d.ldb = n_in; d.ldc = n_in;
+  d.epilogue = HL_EPI_NONE; d.out_dtype = HL_F32;
+  bool done = false;
+  if (gemm_bf16_small_applies(m->ctx, &d)) {
+    // no scratch arena on this path, so it may run on either stream
+    if (m->fork_ok && !nccl_active(m->ctx) && !m->ctx->profiler) {
+      SideStream side(m);
+      HL_TRY(side.rc);
+      return gemm_bf16_row_sums(m->ctx, &d, dy, x, dw, db, &done);
+    }
+    return gemm_bf16_row_sums(m->ctx, &d, dy, x, dw, db, &done);
+  }
+  HL_TRY(gemm_bf16_ctx(m->ctx, &d, dy, x, dw, nullptr, nullptr, nullptr));
+  return db ? bias_grad_impl(m->ctx, dy, HL_BF16, db, m->N, n_out, &m->fold) : HL_OK;
+}
 
 // ---- memory feed-forward core (both routes): lookup, re-scoring, softmax, weighted value -----------
 // query [N, key_dim] f32 is already in ma[l].query (MemoryFeedForward::forward_named,
@@ -789,22 +855,27 @@ int backward(hl_decoder* m) {
   }
   HL_TRY(zero_memory_table_grads(m));
   // loss and dlogits = (softmax - onehot)/N in bf16, the operand precision of the next GEMMs
-  HL_TRY(cross_entropy_impl(ctx, m->logits, V, m->targets, N, V, 1.0f, m->loss_dev, nullptr, m->dlogits, HL_BF16, V));
-  // lm_head
-  HL_TRY(g.run(V, d, N, m->dlogits, V, HL_MN_MAJOR, m->z, d, HL_MN_MAJOR, G + m->off_head_w, d, HL_F32));
+  HL_TRY(cross_entropy_impl(ctx, m->logits, V, m->targets, N, V, 1.0f, m->loss_dev, nullptr, m->dlogits, HL_BF16, V, m->loss_host));
   FoldBatch* fb = &m->fold;
   fb->n = 0;
   fb->used = 0;
-  HL_TRY(bias_grad_impl(ctx, m->dlogits, HL_BF16, G + m->off_head_b, N, V, fb));
+  // Everything up to arena element `done` has been written, the column reductions in the batch apart: they are folded one
+  // launch per full batch, unless a bucket of the gradient exchange is waiting for them.
+  auto finished = [&](size_t done) -> int {
+    if (nccl_active(ctx) || done == m->arena) HL_TRY(fold_batch_flush(ctx, fb));
+    return flush_buckets(m, done);
+  };
+  // lm_head
+  HL_TRY(weight_gradient(m, m->dlogits, V, m->z, d, G + m->off_head_w, G + m->off_head_b));
   HL_TRY(g.run(N, d, V, m->dlogits, V, HL_K_MAJOR, W + m->off_head_w, d, HL_MN_MAJOR, m->dtmp, d, HL_F32));
   float* dx = m->dx0;
   float* dx_next = m->dx1;
   // every layer-norm backward also returns the column sums of the gradient it writes: the bias
   // gradient of the projection that produced that residual-stream value (fc2 or out_proj)
   HL_TRY(layer_norm_backward_impl(ctx, m->x[c.n_layers], HL_BF16, P + m->off_lnf_g, m->dtmp, m->meanf, m->rstdf, nullptr, dx,
-                                  m->dxb, G + m->off_lnf_g, G + m->off_lnf_b, G + m->lo[c.n_layers - 1].out_bias(), N, d, fb));
-  HL_TRY(fold_batch_flush(ctx, fb));
-  HL_TRY(flush_buckets(m, m->off_lnf_b + d));
+                                  m->la[c.n_layers - 1].dy, G + m->off_lnf_g, G + m->off_lnf_b, G + m->lo[c.n_layers - 1].out_bias(),
+                                  N, d, fb));
+  HL_TRY(finished(m->off_lnf_b + d));
   for (int l = c.n_layers - 1; l >= 0; --l) {
     const LayerOffsets& o = m->lo[l];
     LayerActs& a = m->la[l];
@@ -853,43 +924,41 @@ int backward(hl_decoder* m) {
                    HL_EPI_NONE, nullptr, nullptr, 0, nullptr, 0, 2 * kd));
       HL_TRY(hl_binary_f32(ctx, HL_ADD, m->dtmp, m->m_dc2, m->dtmp, (size_t)N * d));
     } else {
-    // y = r + fc2(gelu(fc1(c)));   dx is dL/dy (f32), dxb its bf16 operand copy
-    HL_TRY(g.run(d, F, N, m->dxb, d, HL_MN_MAJOR, a.g, F, HL_MN_MAJOR, G + o.w2, F, HL_F32));
-    HL_TRY(g.run(N, F, d, m->dxb, d, HL_K_MAJOR, W + o.w2, F, HL_MN_MAJOR, m->dh, F, HL_BF16, HL_EPI_DGELU, nullptr, a.h, F));
-    HL_TRY(g.run(F, d, N, m->dh, F, HL_MN_MAJOR, a.c, d, HL_MN_MAJOR, G + o.w1, d, HL_F32));
-    HL_TRY(bias_grad_impl(ctx, m->dh, HL_BF16, G + o.b1, N, F, fb));
-    HL_TRY(g.run(N, d, F, m->dh, F, HL_K_MAJOR, W + o.w1, d, HL_MN_MAJOR, m->dtmp, d, HL_F32));
+    // y = r + fc2(gelu(fc1(c)));   dx is dL/dy (f32), a.dy its bf16 operand copy
+    HL_TRY(weight_gradient(m, a.dy, d, a.g, F, G + o.w2, nullptr));
+    HL_TRY(g.run(N, F, d, a.dy, d, HL_K_MAJOR, W + o.w2, F, HL_MN_MAJOR, a.dh, F, HL_BF16, HL_EPI_DGELU, nullptr, a.h, F));
+    HL_TRY(weight_gradient(m, a.dh, F, a.c, d, G + o.w1, G + o.b1));
+    HL_TRY(g.run(N, d, F, a.dh, F, HL_K_MAJOR, W + o.w1, d, HL_MN_MAJOR, m->dtmp, d, HL_F32));
     }
     // dr = dx + LN2'(dc)
-    HL_TRY(layer_norm_backward_impl(ctx, a.r, HL_BF16, P + o.ln2g, m->dtmp, a.mean2, a.rstd2, dx, dx_next, m->dxb,
+    HL_TRY(layer_norm_backward_impl(ctx, a.r, HL_BF16, P + o.ln2g, m->dtmp, a.mean2, a.rstd2, dx, dx_next, a.dr,
                                     G + o.ln2g, G + o.ln2b, G + o.bo, N, d, fb));
     std::swap(dx, dx_next);  // dx is now dL/dr
-    HL_TRY(g.run(d, d, N, m->dxb, d, HL_MN_MAJOR, a.o, d, HL_MN_MAJOR, G + o.wo, d, HL_F32));
-    HL_TRY(g.run(N, d, d, m->dxb, d, HL_K_MAJOR, W + o.wo, d, HL_MN_MAJOR, m->dob, d, HL_BF16));
+    HL_TRY(weight_gradient(m, a.dr, d, a.o, d, G + o.wo, nullptr));
+    HL_TRY(g.run(N, d, d, a.dr, d, HL_K_MAJOR, W + o.wo, d, HL_MN_MAJOR, m->dob, d, HL_BF16));
     if (m->flash_ok) {
       const size_t need = flash_attention_backward_scratch_bytes(B, T, H, d / H);
       if (need > ctx->workspace_bytes) HL_TRY(ensure_workspace(ctx, need));
-      HL_TRY(flash_attention_backward_impl(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, 3 * d, a.o, d, m->dob, d, a.lse, m->dqkv,
-                                           m->dqkv + d, m->dqkv + 2 * d, 3 * d, B, T, H, d / H, ctx->workspace,
+      HL_TRY(flash_attention_backward_impl(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, 3 * d, a.o, d, m->dob, d, a.lse, a.dqkv,
+                                           a.dqkv + d, a.dqkv + 2 * d, 3 * d, B, T, H, d / H, ctx->workspace,
                                            ctx->workspace_bytes));
     } else {
-      HL_TRY(attention_f64_backward(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, HL_BF16, 3 * d, m->fa_probs, m->dob, d, m->dqkv,
-                                    m->dqkv + d, m->dqkv + 2 * d, 3 * d, B, T, d, H));
+      HL_TRY(attention_f64_backward(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, HL_BF16, 3 * d, m->fa_probs, m->dob, d, a.dqkv,
+                                    a.dqkv + d, a.dqkv + 2 * d, 3 * d, B, T, d, H));
     }
-    HL_TRY(g.run(3 * d, d, N, m->dqkv, 3 * d, HL_MN_MAJOR, a.a, d, HL_MN_MAJOR, G + o.wqkv, d, HL_F32));
-    HL_TRY(bias_grad_impl(ctx, m->dqkv, HL_BF16, G + o.bqkv, N, 3 * d, fb));
-    HL_TRY(g.run(N, d, 3 * d, m->dqkv, 3 * d, HL_K_MAJOR, W + o.wqkv, d, HL_MN_MAJOR, m->dtmp, d, HL_F32));
+    HL_TRY(weight_gradient(m, a.dqkv, 3 * d, a.a, d, G + o.wqkv, G + o.bqkv));
+    HL_TRY(g.run(N, d, 3 * d, a.dqkv, 3 * d, HL_K_MAJOR, W + o.wqkv, d, HL_MN_MAJOR, m->dtmp, d, HL_F32));
     // dx_in = dr + LN1'(da)
-    HL_TRY(layer_norm_backward_impl(ctx, m->x[l], HL_BF16, P + o.ln1g, m->dtmp, a.mean1, a.rstd1, dx, dx_next, m->dxb,
+    HL_TRY(layer_norm_backward_impl(ctx, m->x[l], HL_BF16, P + o.ln1g, m->dtmp, a.mean1, a.rstd1, dx, dx_next, l > 0 ? m->la[l - 1].dy : m->dxb0,
                                     G + o.ln1g, G + o.ln1b, l > 0 ? G + m->lo[l - 1].out_bias() : nullptr, N, d, fb));
     std::swap(dx, dx_next);
-    HL_TRY(fold_batch_flush(ctx, fb));
-    HL_TRY(flush_buckets(m, o.ln1b + d));
+    HL_TRY(finished(o.ln1b + d));
   }
   // embeddings: scatter-add into zeroed tables
   HL_CUDA(cudaMemsetAsync(G + m->off_pos, 0, sizeof(float) * (m->arena - m->off_pos), ctx->stream));
   HL_TRY(hl_embedding_backward(ctx, dx, m->tokens, G + m->off_tok, V, G + m->off_pos, T, N, d));
-  HL_TRY(flush_buckets(m, m->arena));
+  HL_TRY(join_side(m));
+  HL_TRY(finished(m->arena));
   if (nccl_active(ctx)) {
     if (m->has_memory || m->sparse_tok_exchange) {
       // the row exchanges read gradients the compute stream is still producing
@@ -995,7 +1064,7 @@ int backward_f32(hl_decoder* m) {
     if (nccl_active(ctx) || done == m->arena) HL_TRY(fold_batch_flush(ctx, fb));
     return flush_buckets(m, done);
   };
-  HL_TRY(cross_entropy_impl(ctx, m->logits, V, m->targets, N, V, 1.0f, m->loss_dev, nullptr, m->dlogits_f, HL_F32, V));
+  HL_TRY(cross_entropy_impl(ctx, m->logits, V, m->targets, N, V, 1.0f, m->loss_dev, nullptr, m->dlogits_f, HL_F32, V, m->loss_host));
   HL_TRY(zero_memory_table_grads(m));
   float* dx = m->d_a;       // gradient of the residual stream
   float* dx_next = m->d_b;
@@ -1412,6 +1481,12 @@ static int decoder_create_impl(hl_ctx* ctx, const hl_decoder_config* cfg, const 
     e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
     if (e != cudaSuccess) { *ev = nullptr; return fail_cuda(e, "cudaEventCreate(row exchange)"); }
   }
+  if (m->fork_ok) {
+    e = cudaStreamCreateWithFlags(&m->side_stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&m->fork_event, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&m->join_event, cudaEventDisableTiming);
+    if (e != cudaSuccess) return cleanup(fail_cuda(e, "cudaStreamCreate(side)"));
+  }
   e = cudaEventCreateWithFlags(&m->comm_done, cudaEventDisableTiming);
   if (e != cudaSuccess) return cleanup(fail_cuda(e, "cudaEventCreate"));
   e = cudaStreamSynchronize(ctx->stream);
@@ -1431,6 +1506,9 @@ void hl_decoder_destroy(hl_decoder* m) {
   for (auto ev : m->bucket_ready) if (ev) cudaEventDestroy(ev);
   for (auto ev : m->bucket_done) if (ev) cudaEventDestroy(ev);
   if (m->comm_done) cudaEventDestroy(m->comm_done);
+  if (m->side_stream) cudaStreamDestroy(m->side_stream);
+  if (m->fork_event) cudaEventDestroy(m->fork_event);
+  if (m->join_event) cudaEventDestroy(m->join_event);
   for (cudaEvent_t ev : {m->rows_known, m->tok_count_ready, m->val_count_ready}) if (ev) cudaEventDestroy(ev);
   for (auto ev : m->wait_begin) cudaEventDestroy(ev);
   for (auto ev : m->wait_end) cudaEventDestroy(ev);
@@ -1786,8 +1864,7 @@ int hl_decoder_train_step(hl_decoder* m, const int64_t* tokens_host, const int64
   ctx->counters.h2d_bytes += 2 * sizeof(int64_t) * (size_t)m->N;
   HL_TRY(hl_decoder_forward_backward(m, m->tokens, m->targets));
   HL_TRY(hl_decoder_optimizer_step(m));
-  HL_CUDA(cudaMemcpyAsync(m->loss_host, m->loss_dev, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-  ctx->counters.d2h_bytes += sizeof(float);
+  ctx->counters.d2h_bytes += sizeof(float);  // the loss kernel wrote it to pinned host memory as well
   HL_TRY(hl_ctx_sync(ctx));
   if (loss_host) *loss_host = m->loss_host[0];
   return HL_OK;
