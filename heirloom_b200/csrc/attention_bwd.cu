@@ -13,9 +13,7 @@
 // Replaces the reference's recompute-based backward with scalar f32 atomics
 // (tensor_core.ptx:3111-4407, heirloom-kernels/src/cuda.rs:9256-9294) and, for the values it
 // computes, follows src/tensor/autograd.rs:1626-1914 (bf16 operands, f32 accumulation).
-#include <type_traits>
-
-#include "common.cuh"
+#include "attention_bwd.cuh"
 #include "tc05.cuh"
 
 namespace hl {
@@ -31,22 +29,13 @@ constexpr int FB_TMEM_COLS = 512;
 constexpr int FB_DQ_BYTES = FB_BM * 64 * 4;     // 32 KB: 64 columns of a dQ tile in f32, staged for the TMA reduction
 constexpr int FB_MAX_STAGES = 2;
 
-// Sizes that depend on the head dimension.  A head of 128 channels is worked on as two halves of 64: S and dP use the
-// whole head (their operand tiles are two 64-channel blocks side by side), while dV, dK and dQ of a work item cover
-// one 64-channel block, so that the tensor-memory budget (S 128 + dP 128 + dV 64 + dK 64 + dQ 2 x 64 columns) is the
-// same for both sizes; the two halves are separate work items.  The wider tiles leave room for one K/V buffer and
-// one Q/dO stage only.
-template <int HD>
-struct FbSizes {
-  static_assert(HD == 64 || HD == 128, "head_dim 64 or 128");
-  static constexpr int BLOCKS = HD / 64;
-  static constexpr int TILE_BYTES = BLOCKS * FB_BLOCK;  // 16 KB / 32 KB
-  static constexpr int KV_BUFFERS = HD == 64 ? 2 : 1;
-  static constexpr int Q_STAGES = HD == 64 ? 2 : 1;
-  static constexpr int SMEM_DATA = TILE_BYTES * (2 * KV_BUFFERS + 2 * Q_STAGES) + 2 * FB_PS_BYTES + FB_DQ_BYTES;  // 224 KB
-  static constexpr int SMEM_BYTES = SMEM_DATA + 1024;
-  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
-};
+// Heads of 64 channels (attention_bwd128.cu has those of 128).
+constexpr int FB_HD = 64;
+constexpr int FB_TILE_BYTES = FB_BLOCK;
+constexpr int FB_KV_BUFFERS = 2, FB_Q_STAGES = 2;
+constexpr int FB_SMEM_DATA = FB_TILE_BYTES * (2 * FB_KV_BUFFERS + 2 * FB_Q_STAGES) + 2 * FB_PS_BYTES + FB_DQ_BYTES;  // 224 KB
+constexpr int FB_SMEM_BYTES = FB_SMEM_DATA + 1024;
+static_assert(FB_SMEM_BYTES <= 227 * 1024, "shared memory budget");
 
 struct FbBarriers {
   uint64_t kv_full[FB_MAX_STAGES], kv_empty[FB_MAX_STAGES];
@@ -54,20 +43,6 @@ struct FbBarriers {
   uint64_t sdp_full, sdp_free, p_full, dq_full;
   uint32_t tmem_base;
   int abort_flag;
-};
-
-struct FbParams {
-  int B, T, H;
-  int blocks;          // 64-channel blocks per head: 1 or 2
-  const float* lse;    // [B,H,T]
-  const float* delta;  // [B,H,T] rowsum(dO * O)
-  float* dq_accum;     // f32 [B*T, H*hd], zeroed before the kernel
-  long long ld_dq;
-  __nv_bfloat16* dk;
-  __nv_bfloat16* dv;
-  long long ld_dkv;
-  float scale, scale_log2;
-  int* status;
 };
 
 // A CTA's place in its sequence of query tiles: work item `item` (one key tile of one batch and
@@ -79,7 +54,6 @@ struct FbCursor {
   int it;        // query tile within the item's walk
   int n_tiles;   // length of the walk
   int kj, b, h;  // key tile, batch, head
-  int cb;        // which 64-channel block of the head this item's dV, dK and dQ cover
   __device__ __forceinline__ bool valid() const { return item >= 0; }
 };
 // The CTA's `local`-th item.  Items are sorted by decreasing walk length; rounds alternate direction
@@ -87,18 +61,16 @@ struct FbCursor {
 // per-CTA totals of a static assignment.
 __device__ __forceinline__ void fb_load_item(FbCursor& c, int local, const FbParams& p) {
   const int nq = (p.T + FB_BM - 1) / FB_BM;
-  const int per_kj = p.B * p.H * p.blocks;
+  const int per_kj = p.B * p.H;
   const int total = nq * per_kj;
   const int grid = (int)gridDim.x, cta = (int)blockIdx.x;
   const int item = local * grid + ((local & 1) ? grid - 1 - cta : cta);
   if (item >= total) { c.item = -1; return; }
-  const int rest = item % per_kj;
-  const int bh = rest / p.blocks;
+  const int bh = item % per_kj;
   c.item = item;
   c.local = local;
   c.it = 0;
   c.kj = item / per_kj;
-  c.cb = rest % p.blocks;
   c.b = bh / p.H;
   c.h = bh % p.H;
   c.n_tiles = nq - c.kj;  // query tiles kj .. nq-1
@@ -110,16 +82,11 @@ __device__ __forceinline__ FbCursor fb_next(const FbCursor& c, const FbParams& p
   return n;
 }
 
-template <int HD>
 __global__ void __launch_bounds__(FB_THREADS, 1)
 flash_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                            const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
                            const __grid_constant__ CUtensorMap map_dq, const __grid_constant__ CUtensorMap map_dk,
                            const __grid_constant__ CUtensorMap map_dv, const FbParams p) {
-  using Z = FbSizes<HD>;
-  constexpr int FB_HD = HD;
-  constexpr int FB_TILE_BYTES = Z::TILE_BYTES, FB_KV_BUFFERS = Z::KV_BUFFERS, FB_Q_STAGES = Z::Q_STAGES;
-  constexpr int FB_SMEM_DATA = Z::SMEM_DATA, FB_SMEM_BYTES = Z::SMEM_BYTES;
   extern __shared__ uint8_t fb_smem_raw[];
   const uintptr_t raw = reinterpret_cast<uintptr_t>(fb_smem_raw);
   uint8_t* tiles = reinterpret_cast<uint8_t*>((raw + sizeof(FbBarriers) + 1023) & ~uintptr_t(1023));
@@ -161,7 +128,7 @@ flash_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   tc05::tc_fence_after_sync();
   const uint32_t tmem_s = bars->tmem_base;  // 128 columns
   const uint32_t tmem_dp = tmem_s + 128;    // 128 columns
-  const uint32_t tmem_dv = tmem_s + 256;    // 64 columns (one channel block of the head)
+  const uint32_t tmem_dv = tmem_s + 256;    // 64 columns
   const uint32_t tmem_dk = tmem_s + 320;    // 64 columns
   const uint32_t tmem_dq = tmem_s + 384;    // two buffers of 64 columns, alternating by query tile
   pdl_begin();  // everything above touches nothing a predecessor wrote
@@ -185,36 +152,25 @@ flash_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
           const int kb = c.local % FB_KV_BUFFERS;
           if (!tc05::mbar_wait(&bars->kv_empty[kb], ((uint32_t)(c.local / FB_KV_BUFFERS) & 1u) ^ 1u, abort_flag)) break;
           tc05::mbar_arrive_expect_tx(&bars->kv_full[kb], 2 * FB_TILE_BYTES);
-#pragma unroll
-          for (int blk = 0; blk < Z::BLOCKS; ++blk) {
-            tc05::tma_load_2d(sk + kb * FB_TILE_BYTES + blk * FB_BLOCK, &map_k, &bars->kv_full[kb], c.h * FB_HD + blk * 64,
-                              row_base + c.kj * FB_BN);
-            tc05::tma_load_2d(sv + kb * FB_TILE_BYTES + blk * FB_BLOCK, &map_v, &bars->kv_full[kb], c.h * FB_HD + blk * 64,
-                              row_base + c.kj * FB_BN);
-          }
+          tc05::tma_load_2d(sk + kb * FB_TILE_BYTES, &map_k, &bars->kv_full[kb], c.h * FB_HD, row_base + c.kj * FB_BN);
+          tc05::tma_load_2d(sv + kb * FB_TILE_BYTES, &map_v, &bars->kv_full[kb], c.h * FB_HD, row_base + c.kj * FB_BN);
         }
         const int s = g % FB_Q_STAGES;
         const int qrow = row_base + (c.kj + c.it) * FB_BM;
         // the stage frees only when the tile two back has been consumed: have L2 fetch the tile in the meantime
-#pragma unroll
-        for (int blk = 0; blk < Z::BLOCKS; ++blk) {
-          tc05::tma_prefetch_l2_2d(&map_q, c.h * FB_HD + blk * 64, qrow);
-          tc05::tma_prefetch_l2_2d(&map_do, c.h * FB_HD + blk * 64, qrow);
-        }
+        tc05::tma_prefetch_l2_2d(&map_q, c.h * FB_HD, qrow);
+        tc05::tma_prefetch_l2_2d(&map_do, c.h * FB_HD, qrow);
         if (!tc05::mbar_wait(&bars->q_empty[s], ((uint32_t)(g / FB_Q_STAGES) & 1u) ^ 1u, abort_flag)) break;
         tc05::mbar_arrive_expect_tx(&bars->q_full[s], 2 * FB_TILE_BYTES);
-#pragma unroll
-        for (int blk = 0; blk < Z::BLOCKS; ++blk) {
-          tc05::tma_load_2d(sq + s * FB_TILE_BYTES + blk * FB_BLOCK, &map_q, &bars->q_full[s], c.h * FB_HD + blk * 64, qrow);
-          tc05::tma_load_2d(sdo + s * FB_TILE_BYTES + blk * FB_BLOCK, &map_do, &bars->q_full[s], c.h * FB_HD + blk * 64, qrow);
-        }
+        tc05::tma_load_2d(sq + s * FB_TILE_BYTES, &map_q, &bars->q_full[s], c.h * FB_HD, qrow);
+        tc05::tma_load_2d(sdo + s * FB_TILE_BYTES, &map_do, &bars->q_full[s], c.h * FB_HD, qrow);
       }
     }
   } else if (warp == FB_SOFTMAX_WARPS + 1) {
     // -------------------------------------------------------------------------- MMA issuer
     if (tc05::elect_one() && !*abort_flag) {
       constexpr uint32_t idesc_sdp = tc05::instr_desc_bf16_f32(128, 128, false, false);
-      constexpr uint32_t idesc_dkv = tc05::instr_desc_bf16_f32(128, 64, true, true);   // one channel block of dV / dK
+      constexpr uint32_t idesc_dkv = tc05::instr_desc_bf16_f32(128, 64, true, true);   
       constexpr uint32_t idesc_dq = tc05::instr_desc_bf16_f32(128, 64, false, true);
       const uint32_t ap = tc05::smem_u32(sp), ads = tc05::smem_u32(sds);
       // S = Q·Kᵀ and dP = dO·Vᵀ of query tile number `g` (counted over the whole sequence)
@@ -233,13 +189,13 @@ flash_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         const uint64_t dq0 = tc05::smem_desc_sw128(aq, 16, 1024), dk0 = tc05::smem_desc_sw128(ak, 16, 1024);
         const uint64_t ddo0 = tc05::smem_desc_sw128(ado, 16, 1024), dv0 = tc05::smem_desc_sw128(av, 16, 1024);
 #pragma unroll
-        for (int ks = 0; ks < FB_HD / 16; ++ks) {  // the whole head: four 16-channel steps per 64-channel block
-          const uint64_t step = (uint64_t)((ks / 4) * (FB_BLOCK >> 4) + (ks % 4) * 2);
+        for (int ks = 0; ks < FB_HD / 16; ++ks) {  // 16 channels a step
+          const uint64_t step = (uint64_t)(ks * 2);
           tc05::umma_ss(tmem_s, dq0 + step, dk0 + step, idesc_sdp, ks > 0 ? 1u : 0u);
         }
 #pragma unroll
         for (int ks = 0; ks < FB_HD / 16; ++ks) {
-          const uint64_t step = (uint64_t)((ks / 4) * (FB_BLOCK >> 4) + (ks % 4) * 2);
+          const uint64_t step = (uint64_t)(ks * 2);
           tc05::umma_ss(tmem_dp, ddo0 + step, dv0 + step, idesc_sdp, ks > 0 ? 1u : 0u);
         }
         tc05::umma_commit(&bars->sdp_full);
@@ -251,7 +207,7 @@ flash_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         // S/dP of the next query tile (of this item or of the next one) are issued as soon as this
         // tile's have been read out, so the softmax warps find them ready when they come back
         const FbCursor n = fb_next(c, p);
-        if (FB_Q_STAGES > 1 && n.valid()) {
+        if (n.valid()) {
           if (!tc05::mbar_wait(&bars->sdp_free, (uint32_t)g & 1u, abort_flag)) break;
           tc05::tc_fence_after_sync();
           if (!issue_scores(n, g + 1)) break;
@@ -260,10 +216,9 @@ flash_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         tc05::tc_fence_after_sync();
         const int s = g % FB_Q_STAGES;
         const int kb = c.local % FB_KV_BUFFERS;
-        // dV, dK and dQ of this item cover channel block c.cb of the head
-        const uint32_t ak = tc05::smem_u32(sk + kb * FB_TILE_BYTES) + (uint32_t)(c.cb * FB_BLOCK);
-        const uint32_t aq = tc05::smem_u32(sq + s * FB_TILE_BYTES) + (uint32_t)(c.cb * FB_BLOCK);
-        const uint32_t ado = tc05::smem_u32(sdo + s * FB_TILE_BYTES) + (uint32_t)(c.cb * FB_BLOCK);
+        const uint32_t ak = tc05::smem_u32(sk + kb * FB_TILE_BYTES);
+        const uint32_t aq = tc05::smem_u32(sq + s * FB_TILE_BYTES);
+        const uint32_t ado = tc05::smem_u32(sdo + s * FB_TILE_BYTES);
         const uint64_t a_pt0 = tc05::smem_desc_sw128(ap, FB_BM * 128, 1024);    // P^T  (keys x queries)
         const uint64_t a_dst0 = tc05::smem_desc_sw128(ads, FB_BM * 128, 1024);  // dS^T
         const uint64_t b_do0 = tc05::smem_desc_sw128(ado, FB_BM * 128, 1024);
@@ -287,13 +242,6 @@ flash_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         tc05::umma_commit(&bars->q_empty[s]);
         if (c.it == c.n_tiles - 1) tc05::umma_commit(&bars->kv_empty[kb]);  // the item's K and V are no longer read
         tc05::umma_commit(&bars->dq_full);
-        if (FB_Q_STAGES == 1 && n.valid()) {
-          // one Q/dO stage: the next tile's loads could only start once this tile's products were committed, so its
-          // scores are issued after them (S and dP were read out before P and dS were handed over)
-          if (!tc05::mbar_wait(&bars->sdp_free, (uint32_t)g & 1u, abort_flag)) break;
-          tc05::tc_fence_after_sync();
-          if (!issue_scores(n, g + 1)) break;
-        }
         c = n;
       }
     }
@@ -333,7 +281,7 @@ flash_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       __syncwarp();
       if (lane == 0) {
         const int t0 = (c.kj + c.it) * FB_BM + lg * 32;
-        tc05::tma_reduce_add_3d(&map_dq, my_stage, c.h * FB_HD + c.cb * 64 + half * 32, t0, c.b);
+        tc05::tma_reduce_add_3d(&map_dq, my_stage, c.h * FB_HD + half * 32, t0, c.b);
         tc05::tma_store_commit();
       }
       return true;
@@ -367,7 +315,7 @@ flash_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       tc05::fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) {
-        const int col = c.h * FB_HD + c.cb * 64 + half * 32, key0 = c.kj * FB_BN + lg * 32;
+        const int col = c.h * FB_HD + half * 32, key0 = c.kj * FB_BN + lg * 32;
         tc05::tma_store_3d(&map_dv, my_stage, col, key0, c.b);
         tc05::tma_store_3d(&map_dk, my_stage + 2048, col, key0, c.b);
         tc05::tma_store_commit();
@@ -593,19 +541,15 @@ int flash_attention_backward_impl(hl_ctx* ctx, const void* q, const void* k, con
   }
   CUtensorMap mq, mk, mv, mdo;
   int rc;
-  // boxes of 64 channels (one 128-byte swizzle row); a head of 128 channels takes two boxes per tile
+  // boxes of 64 channels (one 128-byte swizzle row); a head of 128 channels takes two boxes per tile and tiles of 64 keys
+  const uint32_t key_rows = head_dim == 64 ? FB_BN : 64;
   if ((rc = make_tensor_map_bf16_2d(&mq, q, (uint64_t)C, rows, (uint64_t)ld_qkv, 64, FB_BM)) != HL_OK) return rc;
-  if ((rc = make_tensor_map_bf16_2d(&mk, k, (uint64_t)C, rows, (uint64_t)ld_qkv, 64, FB_BN)) != HL_OK) return rc;
-  if ((rc = make_tensor_map_bf16_2d(&mv, v, (uint64_t)C, rows, (uint64_t)ld_qkv, 64, FB_BN)) != HL_OK) return rc;
+  if ((rc = make_tensor_map_bf16_2d(&mk, k, (uint64_t)C, rows, (uint64_t)ld_qkv, 64, key_rows)) != HL_OK) return rc;
+  if ((rc = make_tensor_map_bf16_2d(&mv, v, (uint64_t)C, rows, (uint64_t)ld_qkv, 64, key_rows)) != HL_OK) return rc;
   if ((rc = make_tensor_map_bf16_2d(&mdo, dout, (uint64_t)C, rows, (uint64_t)ld_dout, 64, FB_BM)) != HL_OK) return rc;
   FbParams p{};
   p.B = batch; p.T = time; p.H = n_heads;
-  p.blocks = head_dim / 64;
   p.lse = lse; p.delta = delta;
-  p.dq_accum = dq_accum; p.ld_dq = C;
-  p.dk = reinterpret_cast<__nv_bfloat16*>(dk);
-  p.dv = reinterpret_cast<__nv_bfloat16*>(dv);
-  p.ld_dkv = ld_dqkv;
   p.scale = 1.0f / sqrtf((float)head_dim);
   p.scale_log2 = p.scale * 1.4426950408889634f;
   p.status = ctx->status_dev;
@@ -628,21 +572,16 @@ int flash_attention_backward_impl(hl_ctx* ctx, const void* q, const void* k, con
     if ((rc = make_tensor_map(&mdk, HL_BF16, 3, dk, dims, strides, box, 64)) != HL_OK) return rc;
     if ((rc = make_tensor_map(&mdv, HL_BF16, 3, dv, dims, strides, box, 64)) != HL_OK) return rc;
   }
-  const int grid = std::min(nq * batch * n_heads * p.blocks, persistent_sms(ctx));
   if (head_dim == 64) {
     static bool configured = false;
     if (!configured) {
-      HL_CUDA(cudaFuncSetAttribute(flash_attention_bwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, FbSizes<64>::SMEM_BYTES));
+      HL_CUDA(cudaFuncSetAttribute(flash_attention_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM_BYTES));
       configured = true;
     }
-    pdl(flash_attention_bwd_kernel<64>, grid, FB_THREADS, FbSizes<64>::SMEM_BYTES, ctx->stream)(mq, mk, mv, mdo, mdq, mdk, mdv, p);
+    const int grid = std::min(nq * batch * n_heads, persistent_sms(ctx));
+    pdl(flash_attention_bwd_kernel, grid, FB_THREADS, FB_SMEM_BYTES, ctx->stream)(mq, mk, mv, mdo, mdq, mdk, mdv, p);
   } else {
-    static bool configured = false;
-    if (!configured) {
-      HL_CUDA(cudaFuncSetAttribute(flash_attention_bwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, FbSizes<128>::SMEM_BYTES));
-      configured = true;
-    }
-    pdl(flash_attention_bwd_kernel<128>, grid, FB_THREADS, FbSizes<128>::SMEM_BYTES, ctx->stream)(mq, mk, mv, mdo, mdq, mdk, mdv, p);
+    if ((rc = launch_attention_bwd128(ctx, mq, mk, mv, mdo, mdq, mdk, mdv, p)) != HL_OK) return rc;
   }
   HL_LAUNCH_CHECK("flash_attention_bwd_kernel");
   {
