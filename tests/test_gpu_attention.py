@@ -73,3 +73,10 @@ def test_flash_backward_matches_oracle(B, T, H, hd):
         # values, so compare at a few bf16 ulps of the tensor's scale
         assert_close("flash " + name, g, w, atol=scale * 2 ** -6, rtol=2 ** -5)
         assert np.abs(g - w).mean() <= scale * 2 ** -9
+
+
+@pytest.mark.parametrize("B,T,H", [(1, 2, 1), (2, 63, 1), (1, 64, 2), (3, 65, 1), (1, 129, 3), (40, 192, 5)])
+def test_flash_backward_at_the_edges_of_its_key_tiles(B, T, H):
+    """Heads of 128 channels walk tiles of 64 keys against query tiles of 128: the last key tile absent, full or one row deep,
+    and enough items that a CTA takes several.  (A single position's dQ and dK are exactly zero: nothing to scale a bound by.)"""
+    test_flash_backward_matches_oracle(B, T, H, 128)

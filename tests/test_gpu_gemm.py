@@ -69,6 +69,30 @@ def test_gemm_epilogues_match_the_amp_rounding_points():
     assert_close("dgelu", host(out), acc * ho.gelu_backward(hin, np.ones_like(hin)), atol=2e-2, rtol=2e-3)
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 8, 8), (129, 72, 64), (127, 136, 1096), (256, 64, 4096), (513, 200, 520), (1024, 1160, 264)])
+def test_gemm_of_few_tiles(m, n, k):
+    """One-CTA tiles of 64 and 128 columns, contractions whole and shared by 2 to 8 CTAs, ragged last tiles and last k blocks,
+    every epilogue.  f32 accumulation of k products of unit variance: a few ulps of sqrt(k); bf16 results: one rounding."""
+    from heirloom_b200 import cuda
+    c = ctx()
+    rng = np.random.default_rng(m + 3 * n + 5 * k)
+    a, b, da, db = operands(rng, m, n, k, False, False)
+    bias = rng.standard_normal(n).astype(np.float32)
+    res = ho.bf16_round(rng.standard_normal((m, n)))
+    acc = a @ b
+    atol = 1e-3 * np.sqrt(max(k, 64) / 64)
+    run = lambda **kw: cuda.gemm_bf16(c, da, db, m, n, k, **kw)
+    assert_close("f32", host(run(out_dtype=torch.float32)), acc, atol=atol, rtol=1e-5)
+    assert_close("bias", host(run(epilogue=cuda.EPI_BIAS, bias=dev(bias), out_dtype=torch.float32)), acc + bias, atol=atol, rtol=1e-5)
+    h, g = run(epilogue=cuda.EPI_BIAS_GELU, bias=dev(bias), want_aux_out=True)
+    assert_close("h", host(h), acc + bias, atol=1e-2, rtol=2 ** -7)
+    assert_close("gelu(h)", host(g), ho.bf16_round(ho.gelu_value(host(h))), atol=2e-3, rtol=2 ** -7)
+    out = run(epilogue=cuda.EPI_BIAS_RESIDUAL, bias=dev(bias), aux_in=dev(res, torch.bfloat16))
+    assert_close("residual", host(out), ho.bf16_round(res + ho.bf16_round(acc + bias)), atol=2e-2, rtol=2 ** -6)
+    first, second = host(run(out_dtype=torch.float32)), host(run(out_dtype=torch.float32))
+    assert np.array_equal(first, second)
+
+
 def test_gemm_split_k_is_deterministic_and_matches():
     from heirloom_b200 import cuda
     c = ctx()
