@@ -493,14 +493,15 @@ attention_delta_kernel(const __nv_bfloat16* __restrict__ out, long long ld_out, 
 
 __global__ void dq_to_bf16_kernel(const float* __restrict__ acc, long long ld_acc, __nv_bfloat16* __restrict__ dq,
                                   long long ld_dq, long long rows, int cols) {
-  pdl_begin();
   const long long quads = rows * (cols / 4);
+  pdl_begin(quads > 4ll * gridDim.x * blockDim.x);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < quads; i += (long long)gridDim.x * blockDim.x) {
     const long long row = i / (cols / 4);
     const int c = (int)(i % (cols / 4)) * 4;
     const float4 v = *reinterpret_cast<const float4*>(acc + row * ld_acc + c);
     *reinterpret_cast<uint2*>(dq + row * ld_dq + c) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
   }
+  pdl_trigger();
 }
 
 }  // namespace
@@ -534,7 +535,7 @@ int flash_attention_backward_impl(hl_ctx* ctx, const void* q, const void* k, con
   ProfileScope prof(ctx, HL_PROF_ATTENTION_BWD, 5.0 * batch * n_heads * (double)time * time * head_dim);
   {
     const long long pairs = (long long)rows * n_heads;
-    pdl(attention_delta_kernel, (unsigned)ceil_div_ll(pairs * 8, 256), 256, 0, ctx->stream)(
+    pdl(attention_delta_kernel, (unsigned)ceil_div_ll(pairs * 8, 256), 256, 0, ctx->stream).streaming(8.0 * rows * C)(
         reinterpret_cast<const __nv_bfloat16*>(out), ld_out, reinterpret_cast<const __nv_bfloat16*>(dout), ld_dout,
         delta, dq_accum, batch, time, n_heads, head_dim);
     HL_LAUNCH_CHECK("attention_delta_kernel");
@@ -587,7 +588,7 @@ int flash_attention_backward_impl(hl_ctx* ctx, const void* q, const void* k, con
   {
     const long long quads = (long long)rows * (C / 4);
     const long long want = ceil_div_ll(quads, 256), cap = (long long)ctx->sm_count * 8;
-    pdl(dq_to_bf16_kernel, (unsigned)(want < cap ? want : cap), 256, 0, ctx->stream)(
+    pdl(dq_to_bf16_kernel, (unsigned)(want < cap ? want : cap), 256, 0, ctx->stream).streaming(6.0 * rows * C)(
         dq_accum, C, reinterpret_cast<__nv_bfloat16*>(dq), ld_dqkv, (long long)rows, (int)C);
     HL_LAUNCH_CHECK("dq_to_bf16_kernel");
   }

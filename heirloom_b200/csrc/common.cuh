@@ -88,22 +88,46 @@ __device__ __forceinline__ void pdl_begin() {
   pdl_trigger();
   pdl_wait();
 }
+// The same for a kernel whose blocks stream through memory for a while (`streams`): it calls pdl_trigger() itself when its
+// loop is over, so that no dependent sits on its SMs all that time.
+__device__ __forceinline__ void pdl_begin(bool streams) {
+  if (!streams) pdl_trigger();
+  pdl_wait();
+}
+// `shared_percent` >= 0: the split of the SM's memory into shared memory and L1 that the kernel asks for (see `streaming`).
 template <typename... P, typename... A>
-cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, A&&... args) {
+cudaError_t launch_pdl_split(int shared_percent, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                             int cluster, A&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[2] = {};
+  cudaLaunchAttribute attr[3] = {};
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = (unsigned)cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  int n = 1;
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = (unsigned)cluster; attr[n].val.clusterDim.y = 1; attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (shared_percent >= 0) {
+    attr[n].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[n].val.sharedMemCarveout = (unsigned)shared_percent;
+    ++n;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
+
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, A&&... args) {
+  return launch_pdl_split(-1, kernel, grid, block, smem, stream, cluster, std::forward<A>(args)...);
+}
+
+constexpr double kStreamingBytes = 16e6;
 
 // pdl(kernel, grid, block, shared memory, stream)(arguments): the launch above in place of <<< >>>, errors through
 // cudaGetLastError like there.
@@ -113,7 +137,18 @@ struct PdlLauncher {
   dim3 grid, block;
   size_t smem;
   cudaStream_t stream;
-  void operator()(P... args) const { launch_pdl(kernel, grid, block, smem, stream, 1, args...); }
+  int shared_percent = -1;
+  // A kernel that waits for memory keeps its loads in flight in L1.  Launched as a dependent it starts on SMs that never run
+  // empty, and without a wish of its own it keeps the split that a GEMM left behind: 227 KB of shared memory, hardly any L1
+  // (loss kernel, 16384 x 50304: 1216 us instead of 927; column sums of 16384 x 3072: 49 instead of 30).  Asking for L1 lets
+  // the SM drain first, which a kernel of a few microseconds would feel, so only launches of 16 MB and up (3 us at full rate) ask.
+  // `bytes`: what the launch reads and writes; `percent`: the shared memory of its resident blocks.
+  PdlLauncher streaming(double bytes, int percent = 8) const {
+    PdlLauncher l = *this;
+    l.shared_percent = bytes >= kStreamingBytes ? percent : -1;
+    return l;
+  }
+  void operator()(P... args) const { launch_pdl_split(shared_percent, kernel, grid, block, smem, stream, 1, args...); }
 };
 template <typename... P>
 PdlLauncher<P...> pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream) {
@@ -233,6 +268,32 @@ __device__ __forceinline__ float gelu_fwd_fast(float x) {
   const float hx = 0.5f * x;
   return fmaf(hx, t, hx);
 }
+// Two f32 operations an instruction (the same roundings as two single ones).
+__device__ __forceinline__ unsigned long long as_u64(float2 v) { return (unsigned long long)__float_as_uint(v.y) << 32 | __float_as_uint(v.x); }
+__device__ __forceinline__ float2 as_float2(unsigned long long u) { return make_float2(__uint_as_float((unsigned)u), __uint_as_float((unsigned)(u >> 32))); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(as_u64(a)), "l"(as_u64(b)), "l"(as_u64(c)));
+  return as_float2(r);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(as_u64(a)), "l"(as_u64(b)));
+  return as_float2(r);
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(as_u64(a)), "l"(as_u64(b)));
+  return as_float2(r);
+}
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 gelu_fwd_fast2(float2 x) {
+  constexpr float k0 = 0.7978845608028654f, k1 = 0.7978845608028654f * 0.044715f;
+  const float2 a = mul2(x, fma2(mul2(x, x), both(k1), both(k0)));
+  const float2 t = make_float2(tanh_fast(a.x), tanh_fast(a.y));
+  const float2 hx = mul2(x, both(0.5f));
+  return fma2(hx, t, hx);
+}
 // gelu'(x) = (1 + t)/2 + hx*(1 - t^2)*(k0 + 3*k1*x^2)
 __device__ __forceinline__ float gelu_grad_fast(float x) {
   constexpr float k0 = 0.7978845608028654f, k1 = 0.7978845608028654f * 0.044715f;
@@ -241,6 +302,15 @@ __device__ __forceinline__ float gelu_grad_fast(float x) {
   const float dinner = fmaf(x2, 3.0f * k1, k0);
   const float sech2 = fmaf(-t, t, 1.0f);
   return fmaf(0.5f * x * sech2, dinner, fmaf(0.5f, t, 0.5f));
+}
+__device__ __forceinline__ float2 gelu_grad_fast2(float2 x) {
+  constexpr float k0 = 0.7978845608028654f, k1 = 0.7978845608028654f * 0.044715f;
+  const float2 x2 = mul2(x, x);
+  const float2 a = mul2(x, fma2(x2, both(k1), both(k0)));
+  const float2 t = make_float2(tanh_fast(a.x), tanh_fast(a.y));
+  const float2 dinner = fma2(x2, both(3.0f * k1), both(k0));
+  const float2 sech2 = fma2(make_float2(-t.x, -t.y), t, both(1.0f));
+  return fma2(mul2(mul2(x, both(0.5f)), sech2), dinner, fma2(t, both(0.5f), both(0.5f)));
 }
 
 template <typename T>

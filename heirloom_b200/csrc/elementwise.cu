@@ -222,8 +222,8 @@ int reduce_impl(hl_ctx* ctx, const float* x, size_t n, float* out_dev, int mode,
   int rc = ensure_workspace(ctx, sizeof(double) * blocks);
   if (rc != HL_OK) return rc;
   double* partial = reinterpret_cast<double*>(ctx->workspace);
-  if (mode == 1) pdl(reduce_partial_kernel<1>, blocks, 256, 0, ctx->stream)(x, n, vec, partial);
-  else pdl(reduce_partial_kernel<0>, blocks, 256, 0, ctx->stream)(x, n, vec, partial);
+  if (mode == 1) pdl(reduce_partial_kernel<1>, blocks, 256, 0, ctx->stream).streaming(4.0 * n)(x, n, vec, partial);
+  else pdl(reduce_partial_kernel<0>, blocks, 256, 0, ctx->stream).streaming(4.0 * n)(x, n, vec, partial);
   HL_LAUNCH_CHECK("reduce_partial_kernel");
   pdl(reduce_final_kernel, 1, 256, 0, ctx->stream)(partial, blocks, scale, out_dev);
   HL_LAUNCH_CHECK("reduce_final_kernel");

@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(ROW_WARPS * 32)
 ln_fwd_bf16_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
                    __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows,
                    int features, float eps) {
-  pdl_begin();
+  pdl_begin(rows > (int)gridDim.x * ROW_WARPS);
   const int lane = threadIdx.x & 31;
   const int stride = gridDim.x * ROW_WARPS;
   int row = blockIdx.x * ROW_WARPS + (threadIdx.x >> 5);
@@ -95,6 +95,7 @@ ln_fwd_bf16_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
       }
     }
   }
+  pdl_trigger();
 }
 
 // Layer-norm backward.  A row is shared by WPR warps (a thread owns 8 consecutive columns, so its
@@ -114,8 +115,8 @@ ln_bwd_bf16_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
                    const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
                    const float* __restrict__ residual, float* __restrict__ dx_f32, __nv_bfloat16* __restrict__ dx_bf16,
                    float* __restrict__ partial, int rows, int features, int rows_per_block) {
-  pdl_begin();
   constexpr int GROUPS = LnBwdShape<WPR>::GROUPS;
+  pdl_begin(rows_per_block > 4 * GROUPS);
   extern __shared__ float fold_smem[];  // [GROUPS][3][features]
   __shared__ float2 row_sums[2][GROUPS][WPR];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -183,6 +184,7 @@ ln_bwd_bf16_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
       if (dx_bf16) store8_bf16(dx_bf16 + base, o);
     }
   }
+  pdl_trigger();
   if (active) {
     float* mine = fold_smem + (size_t)group * 3 * features + c;
     store8_f32(mine, dg);
@@ -273,7 +275,7 @@ fold_batch_kernel(const FoldJobs jobs) {
 template <typename T, int VEC>
 __global__ void __launch_bounds__(ROW_WARPS * 32)
 colsum_vec_kernel(const T* __restrict__ g, float* __restrict__ partial, int rows, int cols, int rows_per_block) {
-  pdl_begin();
+  pdl_begin(rows_per_block > 8 * ROW_WARPS);
   __shared__ float fold[ROW_WARPS][32 * VEC + 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = (blockIdx.x * 32 + lane) * VEC;
@@ -294,6 +296,7 @@ colsum_vec_kernel(const T* __restrict__ g, float* __restrict__ partial, int rows
       for (int e = 0; e < VEC; ++e) acc[e] += v[e];
     }
   }
+  pdl_trigger();
 #pragma unroll
   for (int e = 0; e < VEC; ++e) fold[warp][lane * VEC + e] = acc[e];
   __syncthreads();
@@ -360,7 +363,7 @@ int layer_norm_forward_fast(hl_ctx* ctx, const void* x, const float* gamma, cons
   const int grid = std::min(ceil_div(rows, ROW_WARPS), ctx->sm_count * 8);
   const int J = ceil_div(features, 256);
 #define HL_LAUNCH(JJ)                                                                                          \
-  pdl(ln_fwd_bf16_kernel<JJ>, grid, ROW_WARPS * 32, 0, ctx->stream)((const __nv_bfloat16*)x, gamma, beta,       \
+  pdl(ln_fwd_bf16_kernel<JJ>, grid, ROW_WARPS * 32, 0, ctx->stream).streaming(4.0 * rows * features)((const __nv_bfloat16*)x, gamma, beta,       \
                                                                     (__nv_bfloat16*)y, mean, rstd, rows, features, eps)
   switch (J) {
     case 1: HL_LAUNCH(1); break;
@@ -393,7 +396,7 @@ int layer_norm_backward_fast(hl_ctx* ctx, const void* x, const float* gamma, con
   }
   const size_t smem = sizeof(float) * (size_t)groups * 3 * features;  // at most 36 KB
 #define HL_LAUNCH(W)                                                                                              \
-  pdl(ln_bwd_bf16_kernel<W>, blocks, LnBwdShape<W>::THREADS, smem, ctx->stream)(                                   \
+  pdl(ln_bwd_bf16_kernel<W>, blocks, LnBwdShape<W>::THREADS, smem, ctx->stream).streaming(8.0 * rows * features, 44)(                                   \
       (const __nv_bfloat16*)x, gamma, dy, mean, rstd, residual, dx_f32, (__nv_bfloat16*)dx_bf16, partial, rows,   \
       features, rows_per_block)
   switch (wpr) {
@@ -438,10 +441,10 @@ int colsum_fast(hl_ctx* ctx, const void* g, int dtype, float* out, int rows, int
   }
   dim3 grid(col_blocks, slabs);
   if (dtype == HL_BF16)
-    pdl(colsum_vec_kernel<__nv_bfloat16, 8>, grid, ROW_WARPS * 32, 0, ctx->stream)((const __nv_bfloat16*)g, partial, rows,
+    pdl(colsum_vec_kernel<__nv_bfloat16, 8>, grid, ROW_WARPS * 32, 0, ctx->stream).streaming(2.0 * rows * cols, 28)((const __nv_bfloat16*)g, partial, rows,
                                                                                    cols, rows_per_block);
   else
-    pdl(colsum_vec_kernel<float, 4>, grid, ROW_WARPS * 32, 0, ctx->stream)((const float*)g, partial, rows, cols,
+    pdl(colsum_vec_kernel<float, 4>, grid, ROW_WARPS * 32, 0, ctx->stream).streaming(4.0 * rows * cols, 16)((const float*)g, partial, rows, cols,
                                                                            rows_per_block);
   HL_LAUNCH_CHECK("colsum_vec_kernel");
   if (deferred) {

@@ -12,17 +12,16 @@
 // accumulator buffers of 256 tensor-memory columns so the epilogue of tile i overlaps the
 // main loop of tile i+1.  Warp roles: warp 0 TMA producer, warp 1 MMA issuer (one elected
 // thread), warps 2-9 epilogue: two warps per tensor-memory lane group, each taking 128 of the
-// 256 columns.  An epilogue warp moves its 32 rows through two alternating 2 KB swizzled staging
-// tiles and writes them with TMA stores (64-byte row segments, clipped at the tensor edge).
+// 256 columns.  An epilogue warp moves its 32 rows through swizzled 4 KB staging tiles and writes them with TMA stores
+// (128-byte row segments, clipped at the tensor edge).
 //
 // Kernels: the generic one reads epilogue, output type and work split from its parameters; the training step's
 // whole-tile products also have kernels compiled for their one epilogue and output type (template parameter SPEC), whose
 // epilogue warps run straight-line code.
 //
-// Contractions of 2048 and up and the wide forward products, with whole tiles (or equal splits), run on pairs of CTAs: a
-// cluster of two
+// Products with whole tiles (or equal splits) run on pairs of CTAs unless that costs a wave: a cluster of two
 // neighbouring SMs works on a 256 x 256 tile, the even CTA's MMA warp issues tcgen05.mma.cta_group::2 for both, each CTA
-// stages its own 128 rows of A and 128 of B's 256 columns (six 32 KB stages in the same shared memory) and keeps its 128
+// stages its own 128 rows of A and 128 of B's 256 columns (five 32 KB stages in the same shared memory) and keeps its 128
 // accumulator rows in its own tensor memory, so each SM reads half as much of B per MMA.  The even CTA's `full` barriers
 // count both CTAs' TMA bytes, its `tmem_empty` barriers both CTAs' epilogue warps; MMA commits arrive in both CTAs.
 //
@@ -37,6 +36,7 @@
 // normal epilogue, so the result does not depend on timing.  Slots are written before a CTA
 // starts the range it finishes, so no CTA ever waits for one that is itself waiting.
 #include <atomic>
+#include <type_traits>
 
 #include "kernels.h"
 #include "tc05.cuh"
@@ -55,18 +55,24 @@ constexpr int B_STAGE_BYTES = BN * BK * 2;  // 32 KB
 constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
 constexpr int MAX_STAGES = 6;
 // CTA pairs: two CTAs of a cluster on one 256 x 256 tile, each staging its 128 rows of A and 128 of B's 256 columns, so
-// a stage is 32 KB, six of them fit, and every SM reads half as much of B out of shared memory per MMA.
-constexpr int PAIR_STAGES = 6;
+// a stage is 32 KB, and every SM reads half as much of B out of shared memory per MMA.  Five stages leave each epilogue warp two
+// staging tiles.
+constexpr int PAIR_STAGES = 5;
 constexpr int PAIR_B_STAGE_BYTES = B_STAGE_BYTES / 2;
 constexpr int PAIR_STAGE_BYTES = A_STAGE_BYTES + PAIR_B_STAGE_BYTES;
-static_assert(PAIR_STAGES * PAIR_STAGE_BYTES <= STAGES * (A_STAGE_BYTES + B_STAGE_BYTES), "pair stages must fit the same shared memory");
 constexpr int EPI_WARPS = 8;
 constexpr int SCHED_SLOTS = 4;
 constexpr int GEMM_THREADS = (2 + EPI_WARPS) * 32;
 constexpr int TMEM_COLS = 512;
-constexpr int STAGING_BYTES = 4096;  // per epilogue warp: two tiles of 32 rows x 64 bytes
-constexpr size_t GEMM_SMEM_BYTES =
-    size_t(STAGES) * STAGE_BYTES + size_t(EPI_WARPS) * STAGING_BYTES + 1024 /*align slack*/ + 256 /*barriers*/;
+constexpr int EPI_TILE_BYTES = 4096;  // an epilogue warp's staging tile: 32 rows x 128 bytes
+constexpr size_t GEMM_DATA_BYTES = size_t(STAGES) * STAGE_BYTES + size_t(EPI_WARPS) * EPI_TILE_BYTES;
+static_assert(PAIR_STAGES * PAIR_STAGE_BYTES + EPI_WARPS * 2 * EPI_TILE_BYTES <= (int)GEMM_DATA_BYTES, "pair stages must fit the same shared memory");
+constexpr int EPI_BIAS_BYTES = 256;  // per epilogue warp: the bias of 64 columns
+constexpr int TAIL_BYTES = 320;
+// Swizzled tiles want 1024-byte alignment, which dynamic shared memory has (the kernel checks); what is left of 227 KB would not
+// cover an unaligned start.
+constexpr size_t GEMM_SMEM_BYTES = GEMM_DATA_BYTES + TAIL_BYTES + size_t(EPI_WARPS) * EPI_BIAS_BYTES;
+static_assert(GEMM_SMEM_BYTES <= 227 * 1024, "shared memory budget");
 
 struct GemmParams {
   int m, n, k;
@@ -96,12 +102,14 @@ struct SharedTail {
   uint64_t empty[MAX_STAGES];
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
+  uint64_t aux_full[EPI_WARPS];       // pairs: an epilogue warp's residual or pre-activation tile has arrived
   uint64_t sched_full[SCHED_SLOTS];   // dynamic tile order: the producer warp's thread hands the items to the other roles
   uint64_t sched_empty[SCHED_SLOTS];
   int sched_item[SCHED_SLOTS];
   uint32_t tmem_base;
   int abort_flag;
 };
+static_assert(sizeof(SharedTail) <= TAIL_BYTES, "barriers outgrow their place");
 
 enum { ITEM_FULL = 0, ITEM_PART = 1, ITEM_FINISH = 2 };
 struct WorkItem {
@@ -199,14 +207,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_aux,
                          const GemmParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];
   constexpr int NSTAGES = PAIR ? PAIR_STAGES : STAGES;
   constexpr int ST_BYTES = PAIR ? PAIR_STAGE_BYTES : STAGE_BYTES;  // one stage of this CTA
   constexpr int TILE_M = PAIR ? 2 * BM : BM;                       // rows of a work item
   constexpr int B_ROWS = PAIR ? BN / 2 : BN;                       // columns of B this CTA stages
-  uint8_t* staging_base = smem + size_t(STAGES) * STAGE_BYTES;     // same place whatever the stage count
-  SharedTail* tail = reinterpret_cast<SharedTail*>(staging_base + size_t(EPI_WARPS) * STAGING_BYTES);
+  constexpr int EPI_TILES = PAIR ? 2 : 1;                          // staging tiles of an epilogue warp
+  uint8_t* staging_base = smem + size_t(NSTAGES) * ST_BYTES;
+  SharedTail* tail = reinterpret_cast<SharedTail*>(smem + GEMM_DATA_BYTES);
   volatile int* abort_flag = &tail->abort_flag;
 
   const int warp = threadIdx.x >> 5;
@@ -223,11 +231,13 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       tc05::mbar_init(&tail->tmem_full[b], 1);
       tc05::mbar_init(&tail->tmem_empty[b], PAIR ? 2 * EPI_WARPS : EPI_WARPS);
     }
+    if (PAIR)
+      for (int q = 0; q < EPI_WARPS; ++q) tc05::mbar_init(&tail->aux_full[q], 1);
     for (int q = 0; q < SCHED_SLOTS; ++q) {
       tc05::mbar_init(&tail->sched_full[q], 1);
       tc05::mbar_init(&tail->sched_empty[q], 1 + EPI_WARPS);  // the MMA issuer and every epilogue warp read an item
     }
-    tail->abort_flag = 0;
+    tail->abort_flag = (tc05::smem_u32(smem) & 1023u) == 0 ? 0 : 1;
     tc05::fence_barrier_init();
   }
   if (warp == 1) {
@@ -393,9 +403,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     const int ew = warp - 2;
     const int lane_group = warp & 3;  // tensor-memory lanes this warp may read
     const int half = ew >> 2;         // which 128 of the tile's 256 columns
-    // Two 2 KB staging tiles per warp ([32 rows x 64 bytes], 64-byte swizzle), used in turn, so
-    // a TMA store is still reading one tile while the next columns are written into the other.
-    uint8_t* staging = staging_base + size_t(ew) * STAGING_BYTES;
+    // Staging tiles of 32 rows x 128 bytes (128-byte swizzle; 64 bf16 or 32 f32 columns), one per warp or, in a pair, two used
+    // in turn, so that a TMA store is still reading one while the next columns are written into the other.  Rows of 128
+    // bytes halve the requests of 64-byte rows: 16384 x 3072 x 768 with bias and GELU spent 16 of its 81 us on its stores.
+    uint8_t* staging = staging_base + size_t(ew) * (EPI_TILES * EPI_TILE_BYTES);
     int stage_sel = 0;
     const int epi = SPEC == SPEC_PARTIAL ? HL_EPI_NONE : SPEC >= 0 ? SPEC / 2 : p.epilogue;
     const bool partial = SPEC == SPEC_PARTIAL ? true : SPEC >= 0 ? false : p.partial_out != 0;
@@ -419,13 +430,36 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       }
       return get_item<PAIR>(p, local, dst) ? 1 : 0;
     };
-    // Global reads of the epilogue are issued ahead of their use so that their latency hides behind the previous
-    // tile's last chunk, the wait for the accumulator and the previous chunk's arithmetic: the warp's 128 bias values
-    // sit four per lane and are handed around by shuffles, and the residual / pre-activation rows are fetched one
-    // 32-column chunk ahead.  The next tile's item, bias and first rows are asked for before the current tile's last
-    // chunk is worked on.
+    // What the epilogue reads besides the accumulator is asked for ahead of its use.  In a pair the residual or
+    // pre-activation columns come by TMA into the staging tile that the result will leave from, 64 columns ahead; a single
+    // CTA has one tile, and its rows are fetched into registers one 32-column step ahead.  The next tile's item and first
+    // rows are asked for before the current tile's last columns are worked on.
+    const bool aux_tma = PAIR && need_aux;
+    uint32_t aux_loads = 0, aux_waits = 0;  // this warp's tiles asked for and taken
+    auto load_aux_tile = [&](const WorkItem& x, int half_chunk) {  // 64 columns, if they lie inside the matrix
+      const int xcol = x.n_tile * BN + half * 128 + half_chunk * 64;
+      if (xcol >= p.n) return;
+      if (lane == 0) {
+        tc05::tma_store_wait_read();  // the store that last used this tile
+        tc05::mbar_arrive_expect_tx(&tail->aux_full[ew], EPI_TILE_BYTES);
+        tc05::tma_load_2d(staging + (aux_loads & 1u) * EPI_TILE_BYTES, &map_aux, &tail->aux_full[ew], xcol,
+                          x.m_tile * TILE_M + (int)rank * BM + lane_group * 32);
+      }
+      ++aux_loads;
+    };
+    // The warp's 128 bias values sit four per lane; those of the 64 columns being worked on are read back from shared memory
+    // as broadcasts (a shuffle per value was the epilogue's busiest instruction).
+    float* bias_tile = reinterpret_cast<float*>(smem + GEMM_DATA_BYTES + TAIL_BYTES + ew * EPI_BIAS_BYTES);
+    auto fetch_bias_of = [&](const WorkItem& x) -> float4 {
+      const int xcol0 = x.n_tile * BN + half * 128;
+      float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (need_bias && xcol0 + lane * 4 < p.n) b = __ldg(reinterpret_cast<const float4*>(p.bias + xcol0 + lane * 4));
+      return b;
+    };
+    float4 bias_reg = make_float4(0.f, 0.f, 0.f, 0.f), bias_next = bias_reg;
     auto fetch_aux_of = [&](const WorkItem& x, int chunk, uint4 (&dst)[4]) {
-      const int xrow = x.m_tile * TILE_M + (int)rank * BM + lane_group * 32 + lane;
+      if (PAIR) return;
+      const int xrow = x.m_tile * TILE_M + lane_group * 32 + lane;
       const int xcol0 = x.n_tile * BN + half * 128;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
@@ -436,27 +470,22 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                                                         (size_t)xrow * p.ld_aux_in + col));
       }
     };
-    auto fetch_bias_of = [&](const WorkItem& x) -> float4 {
-      const int xcol0 = x.n_tile * BN + half * 128;
-      float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (need_bias && xcol0 + lane * 4 < p.n) b = __ldg(reinterpret_cast<const float4*>(p.bias + xcol0 + lane * 4));
-      return b;
-    };
     WorkItem wn;
     uint4 aux_a[4], aux_b[4];
-    float4 bias_reg = make_float4(0.f, 0.f, 0.f, 0.f), bias_next = bias_reg;
     int have = take_item(0, w);
     if (have == 1) {
       bias_reg = fetch_bias_of(w);
-      fetch_aux_of(w, 0, aux_a);
+      if (aux_tma) load_aux_tile(w, 0);
+      else fetch_aux_of(w, 0, aux_a);
     }
     for (int local = 0; ok && have == 1; ++local) {
       int have_next = -2;  // not asked for yet
-      auto ask_next = [&]() {  // the next item, its bias and its first rows (into the buffer the chunk loop is done with)
+      auto ask_next = [&]() {  // the next item and its first rows (into the buffer the chunk loop is done with)
         have_next = take_item(local + 1, wn);
         if (have_next == 1) {
           bias_next = fetch_bias_of(wn);
-          fetch_aux_of(wn, 0, aux_b);
+          if (aux_tma) load_aux_tile(wn, 0);
+          else fetch_aux_of(wn, 0, aux_b);
         }
       };
       const int split = w.split, n_tile = w.n_tile, m_tile = w.m_tile;
@@ -532,16 +561,19 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
         if (!ok) break;
       }
-      // Sixteen 32-bit words of this lane's row (32 bf16 or 16 f32) go to the free staging tile
-      // and out through one TMA store; at most one earlier store may still be reading.
-      auto emit = [&](const CUtensorMap* map, const uint32_t* w, int col) {
-        if (lane == 0) tc05::tma_store_wait_read1();
+      // A free staging tile, its writes handed to the TMA unit, and the store itself.
+      auto free_tile = [&]() -> uint8_t* {
+        if (lane == 0) {
+          if (EPI_TILES == 2) tc05::tma_store_wait_read1();
+          else tc05::tma_store_wait_read();
+        }
         __syncwarp();
-        uint8_t* tile = staging + stage_sel * (STAGING_BYTES / 2);
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          *reinterpret_cast<uint4*>(tile + lane * 64 + ((q ^ ((lane >> 1) & 3)) << 4)) =
-              make_uint4(w[q * 4], w[q * 4 + 1], w[q * 4 + 2], w[q * 4 + 3]);
+        return staging + stage_sel * EPI_TILE_BYTES;
+      };
+      auto put4 = [&](uint8_t* tile, int unit, const uint32_t* words) {  // 16-byte unit `unit` of this lane's row
+        *reinterpret_cast<uint4*>(tile + lane * 128 + ((unit ^ (lane & 7)) << 4)) = make_uint4(words[0], words[1], words[2], words[3]);
+      };
+      auto store_tile = [&](const CUtensorMap* map, uint8_t* tile, int col) {
         tc05::fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
@@ -549,19 +581,19 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           else tc05::tma_store_2d(map, tile, col, row0);
           tc05::tma_store_commit();
         }
-        stage_sel ^= 1;
+        if (EPI_TILES == 2) stage_sel ^= 1;
       };
-      auto process = [&](int chunk, const uint4 (&aux)[4]) {
-        const int col0 = half_col0 + chunk * 32;
-        uint32_t acc_bits[32];
-        tc05::tmem_ld_32x32b_x32(taddr_row + (uint32_t)(half * 128 + chunk * 32), acc_bits);
-        tc05::tmem_ld_wait();
+      uint8_t* tile = staging;
+      uint32_t gelu_words[32];  // gelu(h) of 64 columns, stored behind h
+      // 32 columns, `sub` of the warp's four: bf16 results fill one half of the tile, f32 results all of it.
+      auto process = [&](auto sub_odd, int sub, uint32_t (&acc_bits)[32], const uint4 (&aux)[4]) {
+        constexpr int ODD = decltype(sub_odd)::value;
         if (SPEC < 0 && w.kind == ITEM_FINISH) {
 #pragma unroll 1
           for (int c = w.first_part; c < (int)blockIdx.x; ++c) {
             if (!cta_has_units(p, c)) continue;
             const float4* part = reinterpret_cast<const float4*>(p.sk_slots + (size_t)c * (BM * BN)) +
-                                 (size_t)(ew * 4 + chunk) * (8 * 32) + lane;
+                                 (size_t)(ew * 4 + sub) * (8 * 32) + lane;
             float4 t[8];  // all eight requests leave before the first sum needs its data
 #pragma unroll
             for (int q = 0; q < 8; ++q) t[q] = __ldcg(part + q * 32);
@@ -574,90 +606,149 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             }
           }
         }
-        uint32_t packed[16], gelu_packed[16], hi_words[16];  // f32 output: packed = columns 0-15, hi_words = 16-31
+        if (aux_tma) {
+          tile = staging + ((aux_waits - 1u) & 1u) * EPI_TILE_BYTES;  // the tile the rows came into
+        } else if (!out_bf16 || !ODD) {
+          tile = free_tile();
+        }
 #pragma unroll
         for (int g = 0; g < 4; ++g) {  // groups of 8 columns
-          float v[8];
+          float2 v[4];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(acc_bits[g * 8 + i]);
-          if (!partial) {
-            if (need_bias) {
-              // columns chunk*32 + g*8 + i of this half live in lane chunk*8 + g*2 + i/4
-              const int src = chunk * 8 + g * 2;
-              v[0] += __shfl_sync(0xffffffffu, bias_reg.x, src); v[1] += __shfl_sync(0xffffffffu, bias_reg.y, src);
-              v[2] += __shfl_sync(0xffffffffu, bias_reg.z, src); v[3] += __shfl_sync(0xffffffffu, bias_reg.w, src);
-              v[4] += __shfl_sync(0xffffffffu, bias_reg.x, src + 1); v[5] += __shfl_sync(0xffffffffu, bias_reg.y, src + 1);
-              v[6] += __shfl_sync(0xffffffffu, bias_reg.z, src + 1); v[7] += __shfl_sync(0xffffffffu, bias_reg.w, src + 1);
+          for (int i = 0; i < 4; ++i) v[i] = make_float2(__uint_as_float(acc_bits[g * 8 + i * 2]), __uint_as_float(acc_bits[g * 8 + i * 2 + 1]));
+          uint32_t words[4];
+          if (need_bias) {
+            const float4 b0 = *reinterpret_cast<const float4*>(bias_tile + ODD * 32 + g * 8);
+            const float4 b1 = *reinterpret_cast<const float4*>(bias_tile + ODD * 32 + g * 8 + 4);
+            v[0] = add2(v[0], make_float2(b0.x, b0.y)); v[1] = add2(v[1], make_float2(b0.z, b0.w));
+            v[2] = add2(v[2], make_float2(b1.x, b1.y)); v[3] = add2(v[3], make_float2(b1.z, b1.w));
+          }
+          if (epi == HL_EPI_BIAS_GELU && !partial) {
+            // h = bf16(acc + bias) is the main output; g = bf16(gelu(h)) the second one
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              words[i] = pack_bf16x2(v[i].x, v[i].y);
+              const float2 gl = gelu_fwd_fast2(make_float2(__uint_as_float(words[i] << 16), __uint_as_float(words[i] & 0xFFFF0000u)));
+              gelu_words[ODD * 16 + g * 4 + i] = pack_bf16x2(gl.x, gl.y);
             }
-            if (epi == HL_EPI_BIAS_GELU) {
-              // h = bf16(acc + bias) is the main output; g = bf16(gelu(h)) the second one
-              // rounded two at a time by the packing conversion (the packed word is the output word as well) and widened
-              // again with one integer op each: a quarter of the instructions of rounding on integer ops
-              float gl[8];
+          } else if ((epi == HL_EPI_BIAS_RESIDUAL || epi == HL_EPI_DGELU) && !partial) {
+            uint32_t rw[4];
+            if (aux_tma) {
+              const uint4 r = *reinterpret_cast<const uint4*>(tile + lane * 128 + (((ODD * 4 + g) ^ (lane & 7)) << 4));
+              rw[0] = r.x; rw[1] = r.y; rw[2] = r.z; rw[3] = r.w;
+            } else {
+              rw[0] = aux[g].x; rw[1] = aux[g].y; rw[2] = aux[g].z; rw[3] = aux[g].w;
+            }
 #pragma unroll
-              for (int i = 0; i < 8; i += 2) {
-                const uint32_t hw = pack_bf16x2(v[i], v[i + 1]);
-                packed[g * 4 + i / 2] = hw;
-                v[i] = __uint_as_float(hw << 16);
-                v[i + 1] = __uint_as_float(hw & 0xFFFF0000u);
-              }
-#pragma unroll
-              for (int i = 0; i < 8; ++i) gl[i] = gelu_fwd_fast(v[i]);
-              gelu_packed[g * 4] = pack_bf16x2(gl[0], gl[1]); gelu_packed[g * 4 + 1] = pack_bf16x2(gl[2], gl[3]);
-              gelu_packed[g * 4 + 2] = pack_bf16x2(gl[4], gl[5]); gelu_packed[g * 4 + 3] = pack_bf16x2(gl[6], gl[7]);
-            } else if (epi == HL_EPI_BIAS_RESIDUAL || epi == HL_EPI_DGELU) {
-              const uint4 r = aux[g];
-              const float2 r0 = unpack_bf16x2(r.x), r1 = unpack_bf16x2(r.y), r2 = unpack_bf16x2(r.z), r3 = unpack_bf16x2(r.w);
-              const float rr[8] = {r0.x, r0.y, r1.x, r1.y, r2.x, r2.y, r3.x, r3.y};
+            for (int i = 0; i < 4; ++i) {
+              const float2 r = make_float2(__uint_as_float(rw[i] << 16), __uint_as_float(rw[i] & 0xFFFF0000u));
               if (epi == HL_EPI_BIAS_RESIDUAL) {
                 // out = bf16(residual + bf16(acc + bias)): the two round trips of the block
-#pragma unroll
-                for (int i = 0; i < 8; i += 2) {
-                  const uint32_t hw = pack_bf16x2(v[i], v[i + 1]);
-                  v[i] = rr[i] + __uint_as_float(hw << 16);
-                  v[i + 1] = rr[i + 1] + __uint_as_float(hw & 0xFFFF0000u);
-                }
+                const uint32_t hw = pack_bf16x2(v[i].x, v[i].y);
+                v[i] = add2(r, make_float2(__uint_as_float(hw << 16), __uint_as_float(hw & 0xFFFF0000u)));
               } else {
-                // out = acc * gelu'(h), h read from aux_in
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = v[i] * gelu_grad_fast(rr[i]);
+                v[i] = mul2(v[i], gelu_grad_fast2(r));  // out = acc * gelu'(h), h read from aux_in
               }
+              words[i] = pack_bf16x2(v[i].x, v[i].y);
             }
-          }
-          if (out_bf16 && epi == HL_EPI_BIAS_GELU) {  // h was packed when it was rounded
           } else if (out_bf16) {
-            packed[g * 4] = pack_bf16x2(v[0], v[1]); packed[g * 4 + 1] = pack_bf16x2(v[2], v[3]);
-            packed[g * 4 + 2] = pack_bf16x2(v[4], v[5]); packed[g * 4 + 3] = pack_bf16x2(v[6], v[7]);
-          } else {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              if (g < 2) packed[g * 8 + i] = __float_as_uint(v[i]);
-              else hi_words[(g - 2) * 8 + i] = __float_as_uint(v[i]);
-            }
+            for (int i = 0; i < 4; ++i) words[i] = pack_bf16x2(v[i].x, v[i].y);
           }
-        }
-        if (out_bf16) {
-          emit(&map_c, packed, col0);
-          if (epi == HL_EPI_BIAS_GELU) emit(&map_aux, gelu_packed, col0);
-        } else {
-          emit(&map_c, packed, col0);
-          if (col0 + 16 < p.n) emit(&map_c, hi_words, col0 + 16);
+          if (out_bf16) {
+            put4(tile, ODD * 4 + g, words);
+          } else {
+            const uint32_t f[8] = {__float_as_uint(v[0].x), __float_as_uint(v[0].y), __float_as_uint(v[1].x), __float_as_uint(v[1].y),
+                                   __float_as_uint(v[2].x), __float_as_uint(v[2].y), __float_as_uint(v[3].x), __float_as_uint(v[3].y)};
+            put4(tile, g * 2, f);
+            put4(tile, g * 2 + 1, f + 4);
+          }
         }
       };
-      // chunks beyond the matrix edge are skipped (the test is uniform across the warp)
+      // 64 columns at a time, the accumulator's next 32 on their way while the current ones are worked on.  Columns beyond
+      // the matrix edge are skipped (the test is uniform across the warp).
+      auto load_acc = [&](int sub, uint32_t (&r)[32]) { tc05::tmem_ld_32x32b_x32(taddr_row + (uint32_t)(half * 128 + sub * 32), r); };
+      auto acc_read = [&]() {  // every accumulator column this warp wants is in registers
+        tc05::tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) release_buffer(buf);
+      };
+      bool released = false;
+      constexpr bool kAhead = SPEC >= 0 || PAIR;  // (the kernel that also adds other CTAs' parts has no registers left for it)
+      uint32_t acc0[32], acc1[32];
+      if (half_col0 < p.n) load_acc(0, acc0);
 #pragma unroll 1
-      for (int chunk = 0; chunk < 4; ++chunk) {
-        if (half_col0 + chunk * 32 >= p.n) break;
-        const bool last = chunk == 3 || half_col0 + (chunk + 1) * 32 >= p.n;
-        if (!last) fetch_aux(chunk + 1, aux_b);
-        else ask_next();
-        process(chunk, aux_a);
+      for (int hc = 0; hc < 2; ++hc) {
+        const int sub = hc * 2, col0 = half_col0 + hc * 64;
+        if (col0 >= p.n) break;
+        const bool second = col0 + 32 < p.n;                 // the chunk's other 32 columns
+        const bool more = hc == 0 && half_col0 + 64 < p.n;   // another chunk
+        if (aux_tma) {
+          if (!tc05::mbar_wait(&tail->aux_full[ew], aux_waits & 1u, abort_flag, p.wait_limit_ns)) { ok = false; break; }
+          ++aux_waits;
+          __syncwarp();
+          if (more) load_aux_tile(w, hc + 1);
+          else ask_next();
+        }
+        if (!kAhead && hc > 0) load_acc(sub, acc0);
+        if (need_bias) {
+          __syncwarp();
+          if ((lane >> 4) == hc) *reinterpret_cast<float4*>(bias_tile + (lane & 15) * 4) = bias_reg;
+          __syncwarp();
+        }
+        tc05::tmem_ld_wait();
+        tc05::tmem_ld_fence(acc0);
+        if (second) {
+          if (kAhead) load_acc(sub + 1, acc1);
+          if (!aux_tma) fetch_aux(sub + 1, aux_b);
+        } else {
+          acc_read();
+          released = true;
+          if (!aux_tma) ask_next();
+        }
+        process(std::integral_constant<int, 0>{}, sub, acc0, aux_a);
+        if (!out_bf16) store_tile(&map_c, tile, col0);
+        if (second) {
+          if (!kAhead) load_acc(sub + 1, acc1);
+          tc05::tmem_ld_wait();
+          tc05::tmem_ld_fence(acc1);
+          if (more) {
+            if (kAhead) load_acc(sub + 2, acc0);
+            if (!aux_tma) fetch_aux(sub + 2, aux_a);
+          } else {
+            acc_read();
+            released = true;
+            if (!aux_tma) {
+              uint4 keep[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) aux_a[q] = aux_b[q];
+              for (int q = 0; q < 4; ++q) keep[q] = aux_b[q];
+              ask_next();  // fetches into aux_b
+#pragma unroll
+              for (int q = 0; q < 4; ++q) { aux_a[q] = aux_b[q]; aux_b[q] = keep[q]; }
+            }
+          }
+          process(std::integral_constant<int, 1>{}, sub + 1, acc1, aux_b);
+          if (!out_bf16) store_tile(&map_c, tile, col0 + 32);
+        } else if (!aux_tma) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) aux_a[q] = aux_b[q];
+        }
+        if (out_bf16) {
+          store_tile(&map_c, tile, col0);  // columns past the edge are clipped
+          if (epi == HL_EPI_BIAS_GELU && !partial) {
+            tile = free_tile();
+#pragma unroll
+            for (int q = 0; q < 4; ++q) put4(tile, q, gelu_words + q * 4);
+            if (second) {
+#pragma unroll
+              for (int q = 4; q < 8; ++q) put4(tile, q, gelu_words + q * 4);
+            }
+            store_tile(&map_aux, tile, col0);
+          }
+        }
       }
-      tc05::tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) release_buffer(buf);
+      if (!released) acc_read();
+      if (!ok) break;
       if (have_next == -2) {  // no chunk of this half lies inside the matrix
         ask_next();
 #pragma unroll
@@ -690,8 +781,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
 __global__ void splitk_reduce_kernel(const float* __restrict__ partials, float* __restrict__ out, int m, int n,
                                      long long ldc, int splits) {
-  pdl_begin();
   const long long quads = (long long)m * (n / 4);
+  pdl_begin(quads > 2ll * gridDim.x * blockDim.x);
   for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < quads; q += (long long)gridDim.x * blockDim.x) {
     const int row = (int)(q / (n / 4));
     const int c4 = (int)(q - (long long)row * (n / 4));
@@ -702,6 +793,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partials, float* 
     }
     *reinterpret_cast<float4*>(out + (size_t)row * ldc + c4 * 4) = acc;
   }
+  pdl_trigger();
 }
 
 template <bool A_MN, bool B_MN, bool PAIR, int SPEC = -1>
@@ -743,20 +835,18 @@ int launch_variant(hl_ctx* ctx, const CUtensorMap& ma, const CUtensorMap& mb, co
   return HL_OK;
 }
 
-// Which products run on CTA pairs: HEIRLOOM_GEMM_PAIRS=1 every whole-tile product, 0 none; unset, those with a contraction
-// of kPairMinK and up and the wide forward products.  Read at every call.
+// Which products run on CTA pairs: HEIRLOOM_GEMM_PAIRS=1 every whole-tile product, 0 none; unset, contractions of kPairMinK and up
+// and whatever does not take more waves of 256-row tiles than of 128-row tiles.  A pair reads a third less per output out of L2,
+// and its epilogue has two staging tiles a warp (16384 rows, contraction 768: 3072 columns with dGELU 89 -> 80 us, 768 columns
+// with residual 26.4 -> 24.8 us).  Read at every call.
 constexpr int kPairMinK = 2048;
-bool pairs_enabled(const hl_gemm_desc* d) {
+bool pairs_enabled(const hl_gemm_desc* d, int splits, int sms) {
   const char* e = getenv("HEIRLOOM_GEMM_PAIRS");
   if (e && e[0] == '1') return true;
   if (e && e[0] == '0') return false;
   if (d->k >= kPairMinK) return true;
-  // Short contractions are bound by what the SMs can pull out of L2 (every tile reads its operands again: the MMA issuer
-  // of the qkv forward product spends three quarters of a tile waiting for operand stages, not for the epilogue), and a
-  // pair reads a third less per output.  It pays where the output is wide: qkv forward 51.3 -> 47.8 us, fc1 forward
-  // 84.5 -> 81.5, lm_head forward 1290 -> 1230; the 768-wide outputs and the input gradients lose a few per cent.
-  return d->a_layout == HL_K_MAJOR && d->b_layout == HL_K_MAJOR && d->n >= 2048 &&
-         (d->epilogue == HL_EPI_BIAS || d->epilogue == HL_EPI_BIAS_GELU);
+  const int columns = ceil_div(d->n, BN) * splits;
+  return ceil_div(ceil_div(d->m, 2 * BM) * columns, sms / 2) <= ceil_div(ceil_div(d->m, BM) * columns, sms);
 }
 
 // The small-product kernel decides for itself which products it takes, unless the caller asks for a work split or one of the
@@ -878,21 +968,20 @@ int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void*
   const GemmSmallPlan small = small_plan(ctx, d, plan, sms);
   if (small.splits > 0) return gemm_small_run(ctx, d, small, a, b, c, bias, aux_in, aux_out);
   // Whole tiles (of the whole contraction or of equal splits of it; not the dealt-out k blocks) can run on CTA pairs
-  // with 256-row tiles.  Measured on alternating calls: 6-7 % faster where the main loop bounds the tile (contractions
-  // of 2304 and up), 6-10 % slower at 768, where the epilogue does and the leader waits for both CTAs' epilogue warps.
-  const bool pair = pairs_enabled(d) && plan.sk_tiles == 0 && d->m > BM && sms >= 2 && ctx->gemm_skip_kblock < 0;
+  // with 256-row tiles.
+  const bool pair = plan.sk_tiles == 0 && d->m > BM && sms >= 2 && ctx->gemm_skip_kblock < 0 && pairs_enabled(d, plan.splits, sms);
   GemmParams p{};
   p.m = d->m; p.n = d->n; p.k = d->k;
   p.m_tiles = ceil_div(d->m, pair ? 2 * BM : BM);
   p.n_tiles = ceil_div(d->n, BN);
   p.k_blocks = ceil_div(d->k, BK);
-  // An A operand that stays in L2 anyway keeps the plain order (one tile column after the other);
-  // a larger one is walked in panels of up to eight tile columns so that it streams from DRAM once.
   p.a_kb_wrap = d->a_k_period > 0 ? d->a_k_period / BK : 0;
   p.b_kb_wrap = d->b_k_period > 0 ? d->b_k_period / BK : 0;
   p.wait_limit_ns = ctx->wait_limit_ns ? ctx->wait_limit_ns : tc05::kWaitLimitNs;
   p.skip_kblock = ctx->gemm_skip_kblock;
-  p.panel_w = (size_t)d->m * (size_t)d->k * 2 <= (size_t(32) << 20) ? 1 : std::min(p.n_tiles, 8);
+// Panels of up to sixteen tile columns: A streams past B's columns, which stay in L2.  One column after the other would read
+  // an A of 25 MB again for each of them while the results push it out of L2 (16384 x 3072 x 768: 81 us, now 77).
+  p.panel_w = std::min(p.n_tiles, 16);
   const int splits = plan.splits;
   const size_t need = plan.splitk_bytes;
   p.splits = splits;
@@ -944,20 +1033,26 @@ int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void*
   if (p.partial_out) {
     const uint64_t dims[3] = {(uint64_t)d->n, (uint64_t)d->m, (uint64_t)splits};
     const uint64_t strides[2] = {(uint64_t)d->n * 4, (uint64_t)d->n * (uint64_t)d->m * 4};
-    const uint32_t box[3] = {16, 32, 1};
-    rc = make_tensor_map(&mc, HL_F32, 3, workspace, dims, strides, box, 64);
+    const uint32_t box[3] = {32, 32, 1};
+    rc = make_tensor_map(&mc, HL_F32, 3, workspace, dims, strides, box, 128);
   } else {
     const uint64_t dims[2] = {(uint64_t)d->n, (uint64_t)d->m};
     const uint64_t strides[1] = {(uint64_t)d->ldc * (d->out_dtype == HL_BF16 ? 2u : 4u)};
-    const uint32_t box[2] = {d->out_dtype == HL_BF16 ? 32u : 16u, 32u};  // 64-byte rows
-    rc = make_tensor_map(&mc, d->out_dtype, 2, c, dims, strides, box, 64);
+    const uint32_t box[2] = {d->out_dtype == HL_BF16 ? 64u : 32u, 32u};  // 128-byte rows
+    rc = make_tensor_map(&mc, d->out_dtype, 2, c, dims, strides, box, 128);
   }
   if (rc != HL_OK) return rc;
   if (d->epilogue == HL_EPI_BIAS_GELU) {
     const uint64_t dims[2] = {(uint64_t)d->n, (uint64_t)d->m};
     const uint64_t strides[1] = {(uint64_t)ld_aux_out * 2};
-    const uint32_t box[2] = {32, 32};
-    rc = make_tensor_map(&maux, HL_BF16, 2, aux_out, dims, strides, box, 64);
+    const uint32_t box[2] = {64, 32};
+    rc = make_tensor_map(&maux, HL_BF16, 2, aux_out, dims, strides, box, 128);
+    if (rc != HL_OK) return rc;
+  } else if (pair && (d->epilogue == HL_EPI_BIAS_RESIDUAL || d->epilogue == HL_EPI_DGELU)) {
+    const uint64_t dims[2] = {(uint64_t)d->n, (uint64_t)d->m};
+    const uint64_t strides[1] = {(uint64_t)ld_aux_in * 2};
+    const uint32_t box[2] = {64, 32};
+    rc = make_tensor_map(&maux, HL_BF16, 2, aux_in, dims, strides, box, 128);
     if (rc != HL_OK) return rc;
   } else {
     maux = mc;
@@ -1007,7 +1102,7 @@ int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void*
     const long long quads = (long long)d->m * (d->n / 4);
     const long long want_blocks = ceil_div_ll(quads, 256), cap_blocks = (long long)ctx->sm_count * 8;
     const int blocks = (int)(want_blocks < cap_blocks ? want_blocks : cap_blocks);
-    pdl(splitk_reduce_kernel, blocks, 256, 0, ctx->stream)(workspace, reinterpret_cast<float*>(c), d->m, d->n, d->ldc, splits);
+    pdl(splitk_reduce_kernel, blocks, 256, 0, ctx->stream).streaming(4.0 * (splits + 1) * d->m * d->n)(workspace, reinterpret_cast<float*>(c), d->m, d->n, d->ldc, splits);
     HL_LAUNCH_CHECK("splitk_reduce_kernel");
     count_launch(ctx);
   }

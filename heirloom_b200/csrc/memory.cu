@@ -1131,7 +1131,7 @@ int hl_memory_selected_scores_forward(hl_ctx* ctx, const int64_t* indices, const
   if (rc != HL_OK) return rc;
   HL_REQUIRE(side == 0 || (right_keys && key_dim % 2 == 0 && (long long)side * side == slots),
              "hl_memory_selected_scores_forward: product-key mode needs both half tables, even key_dim and square slots");
-  pdl(selected_scores_fwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream)(indices, query, ld_query, left_or_keys, right_keys,
+  pdl(selected_scores_fwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream).streaming(4.0 * tokens * top_k * key_dim)(indices, query, ld_query, left_or_keys, right_keys,
                                                                            scores, tokens, top_k, side, key_dim, slots,
                                                                            ctx->status_dev);
   HL_LAUNCH_CHECK("selected_scores_fwd_kernel");

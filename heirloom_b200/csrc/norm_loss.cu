@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(CE_THREADS, 2)
 cross_entropy_online_kernel(const float* __restrict__ logits, long long ld, const int64_t* __restrict__ targets,
                             int rows, int classes, float scale, float* row_loss,
                             __nv_bfloat16* __restrict__ dlogits, long long ld_d, int* __restrict__ status, const MeanLoss mean) {
-  pdl_begin();
+  pdl_begin(true);
   __shared__ float sm[32];
   constexpr float kLog2e = 1.4426950408889634f;
   constexpr int STEP = CE_THREADS * 4;  // columns covered by one 16-byte load per thread
@@ -454,6 +454,7 @@ cross_entropy_online_kernel(const float* __restrict__ logits, long long ld, cons
     }
     __syncthreads();  // sm is reused by the next row
   }
+  pdl_trigger();
   mean_when_last(row_loss, rows, mean);
 }
 
@@ -588,7 +589,7 @@ int cross_entropy_impl(hl_ctx* ctx, const float* logits, long long ld, const int
                          (reinterpret_cast<uintptr_t>(logits) & 15) == 0 && (reinterpret_cast<uintptr_t>(dlogits) & 7) == 0 &&
                          classes >= 1024;
   if (online_ok && (dlogits || dlogits_dtype == HL_BF16))
-    pdl(cross_entropy_online_kernel, std::min(rows, ctx->sm_count * 2), CE_THREADS, 0, ctx->stream)(
+    pdl(cross_entropy_online_kernel, std::min(rows, ctx->sm_count * 2), CE_THREADS, 0, ctx->stream).streaming(4.0 * rows * classes)(
         logits, ld, targets, rows, classes, scale, rl, (__nv_bfloat16*)dlogits, ld_dlogits, ctx->status_dev, mean);
   else if (dlogits && dlogits_dtype == HL_BF16)
     pdl(cross_entropy_kernel<float, __nv_bfloat16>, rows, threads, 0, ctx->stream)(
