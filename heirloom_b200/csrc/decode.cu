@@ -327,6 +327,82 @@ __global__ void decode_embed_kernel(const float* __restrict__ table, const float
   }
 }
 
+// Greedy choice.  A block takes 2048 logits, eight a thread; the block that finishes last adds the blocks' sums in their order.
+// Replaces 200 KB to the host and 145 us of sampling there (50304 logits) by 16 bytes and 6 us.
+__device__ __forceinline__ void greedy_better(float& m, int& i, float m2, int i2) {
+  if (m2 > m || (m2 == m && i2 > i)) { m = m2; i = i2; }
+}
+__global__ void __launch_bounds__(256)
+decode_greedy_kernel(const float* __restrict__ logits, int vocab, GreedyPart* __restrict__ parts, GreedyPart* __restrict__ out,
+                     unsigned* __restrict__ ticket) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ float sm_max[8];
+  __shared__ int sm_index[8], sm_bad;
+  __shared__ double sm_sum[8];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) sm_bad = 0;
+  __syncthreads();
+  float v[8], m = -INFINITY;
+  int index = -1;
+  bool bad = false;
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    const int i = blockIdx.x * 2048 + u * 256 + threadIdx.x;
+    v[u] = i < vocab ? logits[i] : -INFINITY;
+    if (i < vocab) {
+      bad |= !isfinite(v[u]);
+      greedy_better(m, index, v[u], i);
+    }
+  }
+  if (bad) sm_bad = 1;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) greedy_better(m, index, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, index, o));
+  if (lane == 0) { sm_max[warp] = m; sm_index[warp] = index; }
+  __syncthreads();
+  m = sm_max[0];
+  index = sm_index[0];
+#pragma unroll
+  for (int w = 1; w < 8; ++w) greedy_better(m, index, sm_max[w], sm_index[w]);
+  double s = 0.0;
+#pragma unroll
+  for (int u = 0; u < 8; ++u)
+    if (v[u] > -INFINITY) s += exp((double)v[u] - (double)m);
+  s = warp_sum(s);
+  if (lane == 0) sm_sum[warp] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s = 0.0;
+    for (int w = 0; w < 8; ++w) s += sm_sum[w];
+    parts[blockIdx.x] = GreedyPart{s, m, sm_bad ? -1 : index};
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last || warp != 0) return;
+  __threadfence();
+  m = -INFINITY;
+  index = -1;
+  bad = false;
+  for (int b = lane; b < (int)gridDim.x; b += 32) {
+    const float pm = __ldcg(&parts[b].max);
+    const int pi = __ldcg(&parts[b].index);
+    bad |= pi < 0;
+    greedy_better(m, index, pm, pi);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) greedy_better(m, index, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, index, o));
+  bad = __any_sync(0xffffffffu, bad);
+  s = 0.0;
+  for (int b = lane; b < (int)gridDim.x; b += 32) s += __ldcg(&parts[b].sum) * exp((double)__ldcg(&parts[b].max) - (double)m);
+  s = warp_sum(s);
+  if (lane == 0) {
+    *out = GreedyPart{s, m, bad ? -1 : index};
+    *ticket = 0u;
+  }
+}
+
 template <typename WT, typename XT, typename OT, typename Acc>
 int launch_gemv(hl_ctx* ctx, const GemvArgs& a) {
   // every output its own warp (or its share of one) up to eight CTAs per SM; the vocabulary's rows are walked by those
@@ -369,6 +445,13 @@ int decode_attention(hl_ctx* ctx, const void* qkv, int dtype, long long ld, cons
   else
     HL_CUDA(launch_pdl(decode_attention_kernel<float, double>, n_heads * DA_CTAS, DA_THREADS, smem, ctx->stream, DA_CTAS,
                        (const float*)qkv, ld, channels, pos, (float*)out, hd, cap));
+  count_launch(ctx);
+  return HL_OK;
+}
+
+int decode_greedy(hl_ctx* ctx, const float* logits, int vocab, GreedyPart* parts, GreedyPart* out) {
+  HL_CUDA(launch_pdl(decode_greedy_kernel, greedy_parts(vocab), 256, 0, ctx->stream, 1, logits, vocab, parts, out,
+                     ctx->gemm_sched + 9));  // a word of the context's zeroed counters
   count_launch(ctx);
   return HL_OK;
 }

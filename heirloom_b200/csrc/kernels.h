@@ -134,6 +134,17 @@ int decode_gemv(hl_ctx* ctx, const DecodeGemv& g);
 size_t decode_attention_smem(int dtype, int head_dim, int context);
 int decode_attention(hl_ctx* ctx, const void* qkv, int dtype, long long ld, const long long* pos, void* out, int channels,
                      int n_heads, int context);
+// The last maximum of a row of logits and the sum of exponentials below it, without taking the row to the host.  `parts` has
+// room for greedy_parts(vocab) entries.
+struct GreedyPart {
+  double sum;  // of e^(x - max)
+  float max;
+  int index;   // of the last maximum, -1 when a value is not finite
+};
+inline int greedy_parts(int vocab) { return (vocab + 2047) / 2048; }
+int decode_greedy(hl_ctx* ctx, const float* logits, int vocab, GreedyPart* parts, GreedyPart* out);
+// Whether every one of n floats is finite; host function.
+bool all_finite_f32(const float* x, size_t n);
 int decode_embed(hl_ctx* ctx, const float* table, const float* positions, const long long* state, void* out, int dtype, int dim);
 
 struct AdamPlan;

@@ -121,6 +121,57 @@ double max_of(const double* x, size_t n, bool* all) {
   return level == 2 ? max_avx512(x, n, all) : level == 1 ? max_avx2(x, n, all) : max_plain(x, n, all);
 }
 
+// x[i] = src[i] / by; by 1.0 leaves the value as it is
+HL_INLINE void widen_body(const float* src, double by, double* x, size_t n) {
+  typedef float Narrow __attribute__((vector_size(4 * LANES)));
+  const size_t whole = n / LANES * LANES;
+  for (size_t i = 0; i < whole; i += LANES) {
+    Narrow f;
+    __builtin_memcpy(&f, src + i, sizeof f);
+    Lanes v = __builtin_convertvector(f, Lanes);
+    v /= by;
+    __builtin_memcpy(x + i, &v, sizeof v);
+  }
+  for (size_t i = whole; i < n; ++i) x[i] = (double)src[i] / by;
+}
+void widen_plain(const float* src, double by, double* x, size_t n) { widen_body(src, by, x, n); }
+HL_AVX512 void widen_avx512(const float* src, double by, double* x, size_t n) { widen_body(src, by, x, n); }
+// the first index at or after i whose value is larger than `least`; n when there is none (no NaN compares as larger)
+HL_INLINE size_t next_above_body(const double* x, size_t i, size_t n, double least) {
+  for (; i + 4 * LANES <= n; i += 4 * LANES) {
+    Words any = {0};
+    for (int u = 0; u < 4; ++u) {
+      Lanes v;
+      load_lanes(&v, x + i + u * LANES);
+      any |= v > least;
+    }
+    int64_t bits = 0;
+    for (int j = 0; j < LANES; ++j) bits |= any[j];
+    if (bits) break;
+  }
+  for (; i < n; ++i)
+    if (x[i] > least) break;
+  return i;
+}
+size_t next_above_plain(const double* x, size_t i, size_t n, double least) { return next_above_body(x, i, n, least); }
+HL_AVX512 size_t next_above_avx512(const double* x, size_t i, size_t n, double least) { return next_above_body(x, i, n, least); }
+HL_INLINE bool finite_body(const float* x, size_t n) {
+  typedef int32_t Bits __attribute__((vector_size(64)));
+  const size_t whole = n / 16 * 16;
+  Bits bad = {0};
+  for (size_t i = 0; i < whole; i += 16) {
+    Bits b;
+    __builtin_memcpy(&b, x + i, sizeof b);
+    bad |= (b & 0x7f800000) == 0x7f800000;
+  }
+  int32_t any = 0;
+  for (int j = 0; j < 16; ++j) any |= bad[j];
+  for (size_t i = whole; i < n; ++i) any |= !std::isfinite(x[i]);
+  return any == 0;
+}
+bool finite_plain(const float* x, size_t n) { return finite_body(x, n); }
+HL_AVX512 bool finite_avx512(const float* x, size_t n) { return finite_body(x, n); }
+
 struct Candidate {
   double value;
   long long token;
@@ -212,6 +263,7 @@ size_t ranked_prefix(std::vector<Candidate>& c, double mass) {
 }
 
 }  // namespace
+bool all_finite_f32(const float* x, size_t n) { return vector_level() == 2 ? finite_avx512(x, n) : finite_plain(x, n); }
 }  // namespace hl
 
 extern "C" int hl_sample_token(const void* logits, int dtype, long long vocab, const int64_t* context, long long n_context,
@@ -224,15 +276,18 @@ extern "C" int hl_sample_token(const void* logits, int dtype, long long vocab, c
   const size_t n = (size_t)vocab, padded = (n + LANES - 1) / LANES * LANES;
   static thread_local std::vector<double> x, p;  // grown to the largest vocabulary seen
   if (x.size() < padded) { x.resize(padded); p.resize(padded); }
-  if (dtype == HL_F32) {
+  const bool penalties = o->repetition_penalty > 1.0 || o->frequency_penalty != 0.0 || o->presence_penalty != 0.0;
+  if (dtype == HL_F32) {  // divided by the temperature on the way when nothing comes between
     const float* src = static_cast<const float*>(logits);
-    for (size_t i = 0; i < n; ++i) x[i] = (double)src[i];
+    const double by = !penalties && o->temperature > 0.0 ? o->temperature : 1.0;
+    if (vector_level() == 2) widen_avx512(src, by, x.data(), n);
+    else widen_plain(src, by, x.data(), n);
   } else {
     const double* src = static_cast<const double*>(logits);
     for (size_t i = 0; i < n; ++i) x[i] = src[i];
   }
   for (size_t i = n; i < padded; ++i) x[i] = -INFINITY;
-  if (o->repetition_penalty > 1.0 || o->frequency_penalty != 0.0 || o->presence_penalty != 0.0) {
+  if (penalties) {
     std::vector<int64_t> seen(context, context + n_context);  // sorted, so that a token's occurrences stand together
     std::sort(seen.begin(), seen.end());
     HL_REQUIRE(seen.empty() || seen[0] >= 0, "hl_sample_token: negative token id in the context");
@@ -244,7 +299,7 @@ extern "C" int hl_sample_token(const void* logits, int dtype, long long vocab, c
       v -= o->presence_penalty;
     }
   }
-  if (o->temperature > 0.0) {
+  if (o->temperature > 0.0 && (penalties || dtype != HL_F32)) {
     if (vector_level() == 2) divide_avx512(x.data(), o->temperature, padded);
     else divide_plain(x.data(), o->temperature, padded);
   }
@@ -260,7 +315,12 @@ extern "C" int hl_sample_token(const void* logits, int dtype, long long vocab, c
       std::make_heap(kept.begin(), kept.end(), ranks_before);
       double least = kept.front().value;
       for (size_t i = k; i < n; ++i) {  // a later index loses a tie, so only a larger value (or the first after a NaN) gets in
-        if (!(x[i] > least) && !(std::isnan(least) && !std::isnan(x[i]))) continue;
+        if (!std::isnan(least)) {
+          i = vector_level() == 2 ? next_above_avx512(x.data(), i, n, least) : next_above_plain(x.data(), i, n, least);
+          if (i == n) break;
+        } else if (std::isnan(x[i])) {
+          continue;
+        }
         std::pop_heap(kept.begin(), kept.end(), ranks_before);
         kept.back() = Candidate{x[i], (long long)i};
         std::push_heap(kept.begin(), kept.end(), ranks_before);

@@ -13,6 +13,8 @@
 // used as GEMM operands), ordered by the time their gradient becomes final in backward
 // (lm_head first, embeddings last) so that fixed-size buckets of the gradient arena can be
 // all-reduced on the collective stream while backward is still running.
+#include <cmath>
+#include <limits>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -68,7 +70,7 @@ struct GraphKey {
            dynamic == o.dynamic;
   }
 };
-enum { GRAPH_STEP = 0, GRAPH_LOSS = 1, GRAPH_WINDOW = 2, GRAPH_DECODE = 3 };
+enum { GRAPH_STEP = 0, GRAPH_LOSS = 1, GRAPH_WINDOW = 2, GRAPH_DECODE = 3, GRAPH_DECODE_GREEDY = 4 };
 struct GraphEntry {
   GraphKey key{};
   cudaGraphExec_t exec = nullptr;  // null until the sequence has run once plainly
@@ -195,7 +197,9 @@ struct hl_decoder {
   // state of the next one-token step
   int cached = 0;
   long long* decode_state = nullptr;       // device: position, token
+  GreedyPart* greedy = nullptr;            // device: the result, then the blocks' parts
   long long* decode_state_host = nullptr;  // pinned
+  GreedyPart* greedy_host = nullptr;       // pinned
   float* logits_host = nullptr;            // pinned, [vocab], allocated on first use
   GraphCache graphs;
   std::vector<float*> xf;  // residual stream per block input, f32
@@ -443,6 +447,7 @@ int plan_activations(hl_decoder* m, bool measure_only, size_t* bytes_out) {
   m->tokens = carve<int64_t>(cur, N);
   m->targets = carve<int64_t>(cur, N);
   m->decode_state = carve<long long>(cur, 2);
+  m->greedy = carve<GreedyPart>(cur, 1 + greedy_parts(c.vocab));
   m->loss_dev = carve<float>(cur, 4);
   m->norm_dev = carve<float>(cur, 4);
   m->norm_dev64 = carve<double>(cur, 2);
@@ -487,6 +492,7 @@ int plan_activations_f32(hl_decoder* m, bool measure_only, size_t* bytes_out) {
   m->tokens = carve<int64_t>(cur, N);
   m->targets = carve<int64_t>(cur, N);
   m->decode_state = carve<long long>(cur, 2);
+  m->greedy = carve<GreedyPart>(cur, 1 + greedy_parts(c.vocab));
   m->loss_dev = carve<float>(cur, 4);
   m->norm_dev = carve<float>(cur, 4);
   m->norm_dev64 = carve<double>(cur, 2);
@@ -1253,8 +1259,9 @@ bool decode_applicable(const hl_decoder* m) {
 
 int ensure_logits_host(hl_decoder* m) {
   if (!m->logits_host) {
-    HL_CUDA(cudaMallocHost(reinterpret_cast<void**>(&m->logits_host), sizeof(float) * (size_t)m->cfg.vocab + 32));
+    HL_CUDA(cudaMallocHost(reinterpret_cast<void**>(&m->logits_host), sizeof(float) * (size_t)m->cfg.vocab + 64));
     m->decode_state_host = reinterpret_cast<long long*>(m->logits_host + ((m->cfg.vocab + 3) & ~3));
+    m->greedy_host = reinterpret_cast<GreedyPart*>(m->decode_state_host + 2);
   }
   return HL_OK;
 }
@@ -1910,7 +1917,24 @@ int hl_decoder_eval_loss(hl_decoder* m, const int64_t* tokens_dev, const int64_t
   return hl_memcpy_d2h(m->ctx, loss_host, m->loss_dev, sizeof(float));
 }
 
-static int window_logits(hl_decoder* m, const int64_t* window, cudaMemcpyKind kind, int window_len, float* logits_host) {
+// The row of logits that a pass left in m->logits, or with `greedy` only the choice out of it, on its way to the host.
+static int queue_result(hl_decoder* m, bool greedy) {
+  hl_ctx* ctx = m->ctx;
+  if (greedy) {
+    HL_TRY(decode_greedy(ctx, m->logits, m->cfg.vocab, m->greedy + 1, m->greedy));
+    HL_CUDA(cudaMemcpyAsync(m->greedy_host, m->greedy, sizeof(GreedyPart), cudaMemcpyDeviceToHost, ctx->stream));
+  } else {
+    HL_CUDA(cudaMemcpyAsync(m->logits_host, m->logits, sizeof(float) * (size_t)m->cfg.vocab, cudaMemcpyDeviceToHost, ctx->stream));
+  }
+  return HL_OK;
+}
+static int finish_result(hl_decoder* m, bool greedy) {
+  HL_CUDA(cudaStreamSynchronize(m->ctx->stream));
+  m->ctx->counters.d2h_bytes += greedy ? sizeof(GreedyPart) : sizeof(float) * (size_t)m->cfg.vocab;
+  return HL_OK;
+}
+
+static int run_window(hl_decoder* m, const int64_t* window, cudaMemcpyKind kind, int window_len, bool greedy) {
   HL_REQUIRE(window_len >= 1, "next_token_logits requires at least one token");
   HL_REQUIRE(window_len <= m->cfg.context, "hl_decoder_next_token_logits: the window is longer than the model's context");
   hl_ctx* ctx = m->ctx;
@@ -1921,9 +1945,12 @@ static int window_logits(hl_decoder* m, const int64_t* window, cudaMemcpyKind ki
     HL_TRY(run_graphed(m, GRAPH_WINDOW, [m]() { return m->cfg.precision == HL_PRECISION_AMP_BF16 ? forward(m, true) : forward_f32(m, true); }));
     m->cached = 0;
   }
-  HL_CUDA(cudaMemcpyAsync(m->logits_host, m->logits, sizeof(float) * (size_t)m->cfg.vocab, cudaMemcpyDeviceToHost, ctx->stream));
-  HL_CUDA(cudaStreamSynchronize(ctx->stream));
-  ctx->counters.d2h_bytes += sizeof(float) * (size_t)m->cfg.vocab;
+  HL_TRY(queue_result(m, greedy));
+  return finish_result(m, greedy);
+}
+
+static int window_logits(hl_decoder* m, const int64_t* window, cudaMemcpyKind kind, int window_len, float* logits_host) {
+  HL_TRY(run_window(m, window, kind, window_len, false));
   memcpy(logits_host, m->logits_host, sizeof(float) * (size_t)m->cfg.vocab);
   return HL_OK;
 }
@@ -1942,8 +1969,8 @@ int hl_decoder_prefill(hl_decoder* m, const int64_t* window_host, int window_len
 
 int hl_decoder_cached_positions(hl_decoder* m) { return m ? m->cached : 0; }
 
-int hl_decoder_decode_next(hl_decoder* m, int64_t token, float* logits_host) {
-  HL_REQUIRE(m && logits_host, "hl_decoder_decode_next: null argument");
+// One position behind the cached ones.
+static int run_next(hl_decoder* m, int64_t token, bool greedy) {
   HL_REQUIRE(m->cached > 0, "hl_decoder_decode_next: no window is cached (call hl_decoder_prefill)");
   HL_REQUIRE(m->cached < m->cfg.context, "hl_decoder_decode_next: the context is full");
   HL_REQUIRE(token >= 0 && token < m->cfg.vocab, "hl_decoder_decode_next: token id out of range");
@@ -1952,7 +1979,7 @@ int hl_decoder_decode_next(hl_decoder* m, int64_t token, float* logits_host) {
   m->decode_state_host[1] = token;
   const int position = m->cached;
   m->cached = 0;  // until this step has succeeded
-  auto queue = [m, ctx]() -> int {
+  auto queue = [m, ctx, greedy]() -> int {
     HL_CUDA(cudaMemcpyAsync(m->decode_state, m->decode_state_host, 2 * sizeof(long long), cudaMemcpyHostToDevice, ctx->stream));
     {
       const int n = m->N;
@@ -1961,16 +1988,47 @@ int hl_decoder_decode_next(hl_decoder* m, int64_t token, float* logits_host) {
       m->N = n;
       HL_TRY(rc);
     }
-    HL_CUDA(cudaMemcpyAsync(m->logits_host, m->logits, sizeof(float) * (size_t)m->cfg.vocab, cudaMemcpyDeviceToHost, ctx->stream));
-    return HL_OK;
+    return queue_result(m, greedy);
   };
-  HL_TRY(run_graphed(m, GRAPH_DECODE, queue));  // position and token are read from memory: the same sequence every time
-  HL_CUDA(cudaStreamSynchronize(ctx->stream));
+  HL_TRY(run_graphed(m, greedy ? GRAPH_DECODE_GREEDY : GRAPH_DECODE, queue));  // position and token are read from memory: the same sequence every time
+  HL_TRY(finish_result(m, greedy));
   ctx->counters.h2d_bytes += 2 * sizeof(long long);
-  ctx->counters.d2h_bytes += sizeof(float) * (size_t)m->cfg.vocab;
-  memcpy(logits_host, m->logits_host, sizeof(float) * (size_t)m->cfg.vocab);
   m->cached = position + 1;
   return HL_OK;
+}
+
+int hl_decoder_decode_next(hl_decoder* m, int64_t token, float* logits_host) {
+  HL_REQUIRE(m && logits_host, "hl_decoder_decode_next: null argument");
+  HL_TRY(run_next(m, token, false));
+  memcpy(logits_host, m->logits_host, sizeof(float) * (size_t)m->cfg.vocab);
+  return HL_OK;
+}
+
+int hl_decoder_generate_token(hl_decoder* m, const int64_t* tokens, long long length, int appended, const hl_sampling_options* o,
+                              double draw, int64_t* token, double* probability, double* log_probability) {
+  HL_REQUIRE(m && tokens && o && token && probability && log_probability, "hl_decoder_generate_token: null argument");
+  HL_REQUIRE(length >= 1, "next_token_logits requires at least one token");
+  // without penalties and filters the choice at temperature 0 is the row's last maximum
+  const bool greedy = o->temperature == 0.0 && o->top_k <= 0 && !(o->top_p > 0.0 && o->top_p < 1.0) &&
+                      !(o->repetition_penalty > 1.0) && o->frequency_penalty == 0.0 && o->presence_penalty == 0.0;
+  const int context = m->cfg.context;
+  if (appended && length <= context && m->cached == length - 1) {
+    HL_TRY(run_next(m, tokens[length - 1], greedy));
+  } else {
+    const int window = (int)std::min<long long>(length, context);
+    HL_TRY(run_window(m, tokens + (length - window), cudaMemcpyHostToDevice, window, greedy));
+    m->cached = decode_applicable(m) ? window : 0;
+  }
+  if (greedy) {
+    const GreedyPart& g = *m->greedy_host;
+    HL_REQUIRE(g.index >= 0, "non-finite generation logits");
+    *token = g.index;
+    *probability = 1.0 / g.sum;
+    *log_probability = std::log(std::max(*probability, std::numeric_limits<double>::min()));
+    return HL_OK;
+  }
+  HL_REQUIRE(all_finite_f32(m->logits_host, (size_t)m->cfg.vocab), "non-finite generation logits");
+  return hl_sample_token(m->logits_host, HL_F32, m->cfg.vocab, tokens, length, o, draw, token, probability, log_probability);
 }
 
 int hl_decoder_loss(hl_decoder* m, float* loss_host) {

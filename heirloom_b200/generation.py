@@ -5,8 +5,8 @@ follow src/nn.rs:1595-1751 statement by statement (repetition, frequency and pre
 temperature, top-k, top-p, greedy at temperature 0); `evaluate_token_loss` walks the token stream in
 windows of `context` tokens like src/memory_transformer.rs:1813-1912; `generate` is
 src/memory_transformer.rs:1730-1769.  The model work (full-window forward, loss) runs on the GPU
-through `hl_decoder_eval_loss` / `hl_decoder_prefill` / `hl_decoder_decode_next`; sampling is host arithmetic over one
-row of logits, as in the reference, in native code.
+through `hl_decoder_eval_loss` / `hl_decoder_generate_token`; sampling is host arithmetic over one row of logits, as in the
+reference, in native code, except for the plain maximum, which the device picks.
 """
 from __future__ import annotations
 
@@ -163,10 +163,14 @@ class _SamplingOptions(ctypes.Structure):
                                                "presence_penalty")] + [("top_k", ctypes.c_longlong)]
 
 
+def _sampling_options(o: GenerationOptions) -> _SamplingOptions:
+    return _SamplingOptions(o.temperature, 0.0 if o.top_p is None else o.top_p, o.repetition_penalty, o.frequency_penalty,
+                            o.presence_penalty, 0 if o.top_k is None else o.top_k)
+
+
 def _sample(logits: np.ndarray, context: np.ndarray, o: GenerationOptions, rng: HeirloomRng) -> Tuple[int, float, float]:
     """`hl_sample_token` on a contiguous f32 or f64 row; `context` is an int64 vector."""
-    options = _SamplingOptions(o.temperature, 0.0 if o.top_p is None else o.top_p, o.repetition_penalty, o.frequency_penalty,
-                               o.presence_penalty, 0 if o.top_k is None else o.top_k)
+    options = _sampling_options(o)
     draw = rng.uniform_f32() if o.temperature != 0.0 else 0.0
     token, p, log_p = ctypes.c_int64(), ctypes.c_double(), ctypes.c_double()
     check(load().hl_sample_token(ctypes.c_void_p(logits.ctypes.data), ctypes.c_int(F32 if logits.dtype == np.float32 else F64),
@@ -197,22 +201,22 @@ def generate(model, prefix: Sequence[int], options: GenerationOptions, rng: Heir
     options.validate()
     if len(prefix) == 0:
         raise HeirloomError("generation prefix must contain at least one token")
-    length, context, cached = len(prefix), model.cfg.context, False
+    length = len(prefix)
     tokens = np.empty(length + options.max_new_tokens, np.int64)
     tokens[:length] = prefix
     steps: List[GeneratedTokenStep] = []
     reason = "max_new_tokens"
-    for _ in range(options.max_new_tokens):
+    native = _sampling_options(options)
+    for step in range(options.max_new_tokens):
         # While everything fits in the context the window only grows at its end: its keys and values stay on the device and
         # a step computes one position.  Past the context every position shifts, and the whole window is run again.
-        if cached and length <= context:
-            logits = model.decode_next(int(tokens[length - 1]))
-        else:
-            logits = model.prefill(tokens[max(0, length - context):length])
-        cached = length < context and model.cached_positions == length
-        if not np.isfinite(logits).all():
-            raise HeirloomError("non-finite generation logits")
-        token, p, logp = _sample(logits, tokens[:length], options, rng)
+        state = rng.state
+        draw = rng.uniform_f32() if options.temperature != 0.0 else 0.0
+        try:
+            token, p, logp = model.generate_token(tokens, length, step > 0, native, draw)
+        except HeirloomError:
+            rng.state = state  # no token, no number drawn
+            raise
         tokens[length] = token
         length += 1
         steps.append(GeneratedTokenStep(token, p, logp))

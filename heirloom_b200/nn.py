@@ -8,7 +8,7 @@ state-dict order, `loss`/`backward`/`step`, and a one-call `train_step`.  All ar
 from __future__ import annotations
 
 import ctypes
-from ctypes import POINTER, Structure, byref, c_char_p, c_float, c_int, c_longlong, c_size_t, c_void_p
+from ctypes import POINTER, Structure, byref, c_char_p, c_double, c_float, c_int, c_int64, c_longlong, c_size_t, c_void_p
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Tuple
 
@@ -220,6 +220,13 @@ class DecoderLm:
         out = np.empty(self.cfg.vocab, np.float32)
         check(self._lib.hl_decoder_decode_next(self.handle, c_longlong(token), c_void_p(out.ctypes.data)))
         return out
+
+    def generate_token(self, tokens: np.ndarray, length: int, appended: bool, options, draw: float) -> Tuple[int, float, float]:
+        """One step of a generation loop over the first `length` of an int64 host vector (`hl_decoder_generate_token`)."""
+        token, p, log_p = c_int64(), c_double(), c_double()
+        check(self._lib.hl_decoder_generate_token(self.handle, c_void_p(tokens.ctypes.data), c_longlong(length), c_int(appended),
+                                                  byref(options), c_double(draw), byref(token), byref(p), byref(log_p)))
+        return token.value, p.value, log_p.value
 
     @property
     def cached_positions(self) -> int:

@@ -566,6 +566,13 @@ typedef struct {
 int hl_sample_token(const void* logits, int dtype, long long vocab, const int64_t* context, long long n_context,
                     const hl_sampling_options* options, double draw, int64_t* token, double* probability,
                     double* log_probability);
+/* One step of a generation loop in one call (src/memory_transformer.rs:1730-1769): the logits after `tokens` (host memory, the
+ * last `context` of them), then hl_sample_token over them.  `appended`: tokens[0 .. length-1) are the ones that the last call
+ * worked on, so that only the new position is computed while the context is not full.  Without penalties and filters at
+ * temperature 0 the choice is made on the device. */
+int hl_decoder_generate_token(hl_decoder* model, const int64_t* tokens, long long length, int appended,
+                              const hl_sampling_options* options, double draw, int64_t* token, double* probability,
+                              double* log_probability);
 
 #ifdef __cplusplus
 }

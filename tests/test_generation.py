@@ -181,3 +181,28 @@ def test_one_token_steps_equal_the_full_window(heads, memory):
         with pytest.raises(Exception, match="no window is cached"):
             model.decode_next(0)
         model.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("vocab", [8, 2048, 2056, 50304])
+def test_the_device_picks_the_greedy_token_that_sampling_picks(vocab):
+    """The last maximum and its probability, the row cut into blocks of 2048 logits: the same token as the host's sampling of
+    the same logits, the probability to the rounding of two f64 sums of `vocab` terms; ties go to the last index."""
+    from heirloom_b200 import nn
+    from tests.gpu_util import ctx
+    c = ctx()
+    model = nn.DecoderLm(c, nn.DecoderConfig(vocab=vocab, d_model=64, n_layers=1, n_heads=1, d_ff=64, context=4, batch=1))
+    rng = np.random.default_rng(vocab)
+    for tied in (False, True):
+        state = {n: rng.standard_normal(s) * 0.3 for n, s in model.parameter_shapes().items()}
+        if tied:
+            state = {n: v * (0.0 if n.startswith("lm_head") else 1.0) for n, v in state.items()}
+        model.load_state_dict(state)
+        tokens = rng.integers(0, vocab, 4)
+        options = gen.GenerationOptions.greedy(1, -1)
+        for n in (1, 2, 4):
+            got = model.generate_token(tokens, n, n == 2, gen._sampling_options(options), 0.0)
+            want = gen.sample_token(gen.next_token_logits(model, tokens[:n]), tokens[:n], options, gen.HeirloomRng(0))
+            assert got[0] == want[0] and (not tied or got[0] == vocab - 1)
+            assert got[1] == pytest.approx(want[1], rel=vocab * 2e-16 + 1e-14)
+    model.close()
