@@ -199,31 +199,54 @@ decode_gemv_kernel(const GemvArgs a) {
 
 // Row *pos of the q/k/v rows against rows 0 .. *pos: a cluster of eight CTAs per head, each over an eighth of the keys; their
 // maxima, sums and weighted values are pushed into CTA 0's shared memory.  Eight lanes take a key, sixteen bytes each.
+//
+// Bound by latency: a few hundred bytes of keys a thread behind a chain of dependent steps.  Only the newest row comes from the
+// kernel before this one, so the older keys and values are on their way into shared memory (`staged`, where they fit) while
+// that one still runs, and the chain that is left starts at the query (12 heads of 64 at 500 positions: 9.8 us before).
+__device__ __forceinline__ void cp_async16(void* shared, const void* global) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(shared)), "l"(global) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 constexpr int DA_CTAS = 8;
 constexpr int DA_THREADS = 128;
 constexpr int DA_SLOTS = DA_THREADS / 8;  // keys at a time
 template <typename T, typename Acc>
 __global__ void __launch_bounds__(DA_THREADS)
 decode_attention_kernel(const T* __restrict__ qkv, long long ld, int channels, const long long* __restrict__ pos,
-                        T* __restrict__ out, int hd, int chunk_cap) {
+                        T* __restrict__ out, int hd, int chunk_cap, bool staged) {
   extern __shared__ double da_smem[];
-  Acc* q = reinterpret_cast<Acc*>(da_smem);  // [hd]
+  T* kept = reinterpret_cast<T*>(da_smem);   // staged: [2][chunk_cap][hd] keys, then values
+  Acc* q = reinterpret_cast<Acc*>(kept + (staged ? (size_t)2 * chunk_cap * hd : 0));  // [hd]
   Acc* s = q + hd;                           // [chunk_cap] scores, then weights
   Acc* part = s + chunk_cap;                 // [DA_SLOTS][hd] weighted values per key slot
   Acc* all = part + DA_SLOTS * hd;           // CTA 0: [DA_CTAS][hd + 2] weighted values, maximum, sum of every CTA
   __shared__ Acc red[32];
   cg::cluster_group cluster = cg::this_cluster();
   pdl_trigger();
-  cluster.sync();  // CTA 0 has started: its shared memory may be written
   const int rank = (int)(blockIdx.x % DA_CTAS), h = (int)(blockIdx.x / DA_CTAS);
   const T* base = qkv + (long long)h * hd;
   const int sub = threadIdx.x & 7, slot = threadIdx.x >> 3;
   constexpr int PN = Pack<T>::N;
   const bool vec = hd % PN == 0 && channels % PN == 0 && ld % PN == 0;
-  pdl_wait();
+  // The position was copied here before the step's first kernel started, the rows below it before the step.
   const long long t = *pos;
   const int keys = (int)t + 1, chunk = (keys + DA_CTAS - 1) / DA_CTAS;
   const int k0 = min(keys, rank * chunk), k1 = min(keys, k0 + chunk);
+  const int units = hd / PN;  // 16-byte pieces of a row
+  auto stage = [&](int key, int u) {
+#pragma unroll
+    for (int kv = 0; kv < 2; ++kv)
+      cp_async16(kept + ((size_t)kv * chunk_cap + (key - k0)) * hd + u * PN, base + (1 + kv) * channels + (long long)key * ld + u * PN);
+  };
+  if (staged)
+    for (int key = k0 + slot; key < min(k1, (int)t); key += DA_SLOTS)
+      for (int u = sub; u < units; u += 8) stage(key, u);
+  cluster.sync();  // CTA 0 has started: its shared memory may be written
+  pdl_wait();
+  if (staged) {
+    if (k1 == keys && k1 > k0 && (int)threadIdx.x < units) stage((int)t, threadIdx.x);
+    cp_async_wait_all();
+  }
   for (int c = threadIdx.x; c < hd; c += DA_THREADS) q[c] = (Acc)as_f32(base[t * ld + c]);
   __syncthreads();
   const Acc scale = (Acc)1 / sqrt((Acc)hd);
@@ -232,7 +255,7 @@ decode_attention_kernel(const T* __restrict__ qkv, long long ld, int channels, c
   for (int key = k0 + slot; key - slot < k1; key += DA_SLOTS) {
     Acc dot = 0;
     if (key < k1) {
-      const T* kr = base + channels + (long long)key * ld;
+      const T* kr = staged ? kept + (size_t)(key - k0) * hd : base + channels + (long long)key * ld;
       if (vec) {
         for (int c = sub * PN; c < hd; c += 8 * PN) {
           float kv[PN];
@@ -269,7 +292,8 @@ decode_attention_kernel(const T* __restrict__ qkv, long long ld, int channels, c
 #pragma unroll 4
       for (int key = k0 + slot; key < k1; key += DA_SLOTS) {
         float vv[PN];
-        Pack<T>::unpack(*reinterpret_cast<const uint4*>(base + 2 * channels + (long long)key * ld + c), vv);
+        const T* vr = staged ? kept + ((size_t)chunk_cap + (key - k0)) * hd : base + 2 * channels + (long long)key * ld;
+        Pack<T>::unpack(*reinterpret_cast<const uint4*>(vr + c), vv);
         const Acc w = s[key - k0];
 #pragma unroll
         for (int e = 0; e < PN; ++e) acc[e] += w * (Acc)vv[e];
@@ -435,18 +459,31 @@ size_t decode_attention_smem(int dtype, int hd, int context) {
   return acc * ((size_t)hd + (size_t)ceil_div(context, DA_CTAS) + (size_t)DA_SLOTS * hd + (size_t)DA_CTAS * (hd + 2));
 }
 
-int decode_attention(hl_ctx* ctx, const void* qkv, int dtype, long long ld, const long long* pos, void* out, int channels,
-                     int n_heads, int context) {
+template <typename T, typename Acc>
+int launch_decode_attention(hl_ctx* ctx, const T* qkv, long long ld, const long long* pos, T* out, int channels, int n_heads, int context) {
   const int hd = channels / n_heads, cap = ceil_div(context, DA_CTAS);
-  const size_t smem = decode_attention_smem(dtype, hd, context);
-  if (dtype == HL_BF16)
-    HL_CUDA(launch_pdl(decode_attention_kernel<__nv_bfloat16, float>, n_heads * DA_CTAS, DA_THREADS, smem, ctx->stream, DA_CTAS,
-                       (const __nv_bfloat16*)qkv, ld, channels, pos, (__nv_bfloat16*)out, hd, cap));
-  else
-    HL_CUDA(launch_pdl(decode_attention_kernel<float, double>, n_heads * DA_CTAS, DA_THREADS, smem, ctx->stream, DA_CTAS,
-                       (const float*)qkv, ld, channels, pos, (float*)out, hd, cap));
+  size_t smem = decode_attention_smem(sizeof(T) == 2 ? HL_BF16 : HL_F32, hd, context);
+  const size_t rows = sizeof(T) * 2 * (size_t)cap * hd;
+  // staged while two CTAs still fit on an SM; longer contexts read keys and values where they lie
+  const bool staged = smem + rows <= 110 * 1024 && hd % Pack<T>::N == 0 && channels % Pack<T>::N == 0 && ld % Pack<T>::N == 0 &&
+                      (reinterpret_cast<uintptr_t>(qkv) & 15) == 0;
+  if (staged) smem += rows;
+  auto kern = decode_attention_kernel<T, Acc>;
+  static bool configured = false;
+  if (!configured) {
+    HL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024));
+    configured = true;
+  }
+  HL_CUDA(launch_pdl(kern, n_heads * DA_CTAS, DA_THREADS, smem, ctx->stream, DA_CTAS, qkv, ld, channels, pos, out, hd, cap, staged));
   count_launch(ctx);
   return HL_OK;
+}
+
+int decode_attention(hl_ctx* ctx, const void* qkv, int dtype, long long ld, const long long* pos, void* out, int channels,
+                     int n_heads, int context) {
+  return dtype == HL_BF16 ? launch_decode_attention<__nv_bfloat16, float>(ctx, (const __nv_bfloat16*)qkv, ld, pos, (__nv_bfloat16*)out,
+                                                                          channels, n_heads, context)
+                          : launch_decode_attention<float, double>(ctx, (const float*)qkv, ld, pos, (float*)out, channels, n_heads, context);
 }
 
 int decode_greedy(hl_ctx* ctx, const float* logits, int vocab, GreedyPart* parts, GreedyPart* out) {
