@@ -15,6 +15,11 @@ namespace {
 
 namespace cg = cooperative_groups;
 
+__device__ __forceinline__ void cp_async16(void* shared, const void* global) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(shared)), "l"(global) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 constexpr int GV_WARPS = 8;
 constexpr int GV_THREADS = GV_WARPS * 32;
 
@@ -73,30 +78,43 @@ template <int N> __device__ __forceinline__ void load_x(const __nv_bfloat16* p, 
 // out = epilogue(W · x + bias).  WT/XT/OT: weights, input, output; Acc: float on the bf16 route, double where the f32
 // route's sums are f64.  The values are rounded where the full-window kernels round them.  A lane holds the same 32 elements
 // of x and of the weight row, so that a row needs no shared memory and a layer norm two warp sums; rows longer than 1024
-// are shared by several warps.
+// are shared by several warps.  Three CTAs an SM (two with f64 sums): with gamma and beta in registers there were two (one),
+// and half of the loads that the memory wants in flight (50304 x 768: 30 -> 26 us; a step of the GPT-sized model 3.1 -> 2.8 ms
+// for a prefix of 500 and 8 tokens).
 template <typename WT, typename XT, typename OT, typename Acc>
-__global__ void __launch_bounds__(GV_THREADS)
+__global__ void __launch_bounds__(GV_THREADS, sizeof(WT) == 2 ? 3 : 2)
 decode_gemv_kernel(const GemvArgs a) {
   constexpr int PN = Pack<WT>::N, STEP = 32 * PN, U = GV_SPAN / STEP;
   __shared__ Acc parts[GV_WARPS];
+  __shared__ __align__(16) float affine[2][GV_SPAN];  // gamma and beta, here before the input row is
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wpr = a.warps_per_row, part = warp % wpr, k = a.k;
   const int row_step = gridDim.x * (GV_WARPS / wpr);
   const int spans = (k + GV_SPAN * wpr - 1) / (GV_SPAN * wpr);  // how often the warps of a row move on
   const XT* x = static_cast<const XT*>(a.x);
   auto column = [&](int span, int u) { return (span * wpr + part) * GV_SPAN + u * STEP + lane * PN; };
+  // Weights on their way: the next span of this row or of the warp's next one.
   uint4 raw[U];
-  auto fetch = [&](int row, int span) {
-    const WT* w = static_cast<const WT*>(a.w) + (size_t)row * k;
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int c = column(span, u);
-      raw[u] = c < k ? __ldg(reinterpret_cast<const uint4*>(w + c)) : make_uint4(0, 0, 0, 0);
-    }
-  };
   int row = blockIdx.x * (GV_WARPS / wpr) + warp / wpr;
+  int fetch_row = row, fetch_span = 0;
+  auto fetch = [&]() {
+    if (fetch_row < a.n) {
+      const WT* w = static_cast<const WT*>(a.w) + (size_t)fetch_row * k;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int c = column(fetch_span, u);
+        raw[u] = c < k ? __ldg(reinterpret_cast<const uint4*>(w + c)) : make_uint4(0, 0, 0, 0);
+      }
+    }
+    if (++fetch_span == spans) { fetch_span = 0; fetch_row += row_step; }
+  };
   // weights and bias do not depend on any kernel of the step
-  if (a.vec && row < a.n) fetch(row, 0);
+  if (a.vec) fetch();
+  if (a.gamma)
+    for (int c = threadIdx.x * 4; c < k; c += GV_THREADS * 4) {
+      cp_async16(&affine[0][c], a.gamma + c);
+      cp_async16(&affine[1][c], a.beta + c);
+    }
   float bias = a.bias && row < a.n ? __ldg(a.bias + row) : 0.f;
   pdl_trigger();
   pdl_wait();
@@ -119,12 +137,11 @@ decode_gemv_kernel(const GemvArgs a) {
   };
   if (a.vec) load_span(0);
   if (a.gamma) {  // one span, one warp per row
-    float g[U][PN], b[U][PN];
+    cp_async_wait_all();
+    __syncthreads();
     Acc sum = 0;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int c = column(0, u);
-      if (c < k) { load_x(a.gamma + c, g[u]); load_x(a.beta + c, b[u]); }
 #pragma unroll
       for (int e = 0; e < PN; ++e) sum += (Acc)xv[u][e];
     }
@@ -139,10 +156,13 @@ decode_gemv_kernel(const GemvArgs a) {
     const Acc rstd = (Acc)1 / sqrt(warp_sum(sq) / (Acc)k + (Acc)1e-5f);
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (column(0, u) < k) {
+      if (const int c = column(0, u); c < k) {
+        float g[PN], b[PN];
+        load_x(&affine[0][c], g);
+        load_x(&affine[1][c], b);
 #pragma unroll
         for (int e = 0; e < PN; ++e) {
-          const float y = (float)(((Acc)xv[u][e] - mean) * rstd * (Acc)g[u][e] + (Acc)b[u][e]);
+          const float y = (float)(((Acc)xv[u][e] - mean) * rstd * (Acc)g[e] + (Acc)b[e]);
           xv[u][e] = sizeof(XT) == 2 ? bf16_round(y) : y;
         }
       }
@@ -155,9 +175,7 @@ decode_gemv_kernel(const GemvArgs a) {
         uint4 now[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) now[u] = raw[u];
-        // the next weights, of this row or of the warp's next one, travel while these are multiplied
-        if (span + 1 < spans) fetch(row, span + 1);
-        else if (row + row_step < a.n) fetch(row + row_step, 0);
+        fetch();  // travels while these are multiplied
         if (spans > 1) load_span(span);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -203,10 +221,6 @@ decode_gemv_kernel(const GemvArgs a) {
 // Bound by latency: a few hundred bytes of keys a thread behind a chain of dependent steps.  Only the newest row comes from the
 // kernel before this one, so the older keys and values are on their way into shared memory (`staged`, where they fit) while
 // that one still runs, and the chain that is left starts at the query (12 heads of 64 at 500 positions: 9.8 us before).
-__device__ __forceinline__ void cp_async16(void* shared, const void* global) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(shared)), "l"(global) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 constexpr int DA_CTAS = 8;
 constexpr int DA_THREADS = 128;
 constexpr int DA_SLOTS = DA_THREADS / 8;  // keys at a time
@@ -220,7 +234,7 @@ decode_attention_kernel(const T* __restrict__ qkv, long long ld, int channels, c
   Acc* s = q + hd;                           // [chunk_cap] scores, then weights
   Acc* part = s + chunk_cap;                 // [DA_SLOTS][hd] weighted values per key slot
   Acc* all = part + DA_SLOTS * hd;           // CTA 0: [DA_CTAS][hd + 2] weighted values, maximum, sum of every CTA
-  __shared__ Acc red[32];
+  __shared__ Acc red[32], slot_sums[DA_SLOTS];
   cg::cluster_group cluster = cg::this_cluster();
   pdl_trigger();
   const int rank = (int)(blockIdx.x % DA_CTAS), h = (int)(blockIdx.x / DA_CTAS);
@@ -245,9 +259,9 @@ decode_attention_kernel(const T* __restrict__ qkv, long long ld, int channels, c
   pdl_wait();
   if (staged) {
     if (k1 == keys && k1 > k0 && (int)threadIdx.x < units) stage((int)t, threadIdx.x);
-    cp_async_wait_all();
   }
   for (int c = threadIdx.x; c < hd; c += DA_THREADS) q[c] = (Acc)as_f32(base[t * ld + c]);
+  if (staged) cp_async_wait_all();
   __syncthreads();
   const Acc scale = (Acc)1 / sqrt((Acc)hd);
   Acc mx = -INFINITY;
@@ -277,24 +291,21 @@ decode_attention_kernel(const T* __restrict__ qkv, long long ld, int channels, c
     }
   }
   mx = block_max(mx, red, (Acc)-INFINITY);
-  Acc sum = 0;
-  for (int i = threadIdx.x; i < k1 - k0; i += DA_THREADS) {
-    const Acc e = exp(s[i] - mx);
-    s[i] = e;
-    sum += e;
-  }
-  sum = block_sum(sum, red);
+  Acc weights = 0;  // sum over this slot's keys
+  // every lane of a key takes the exponential again: cheaper than a pass and a barrier of their own
   if (vec) {
     for (int c = sub * PN; c < hd; c += 8 * PN) {
       Acc acc[PN];
 #pragma unroll
       for (int e = 0; e < PN; ++e) acc[e] = 0;
+      weights = 0;
 #pragma unroll 4
       for (int key = k0 + slot; key < k1; key += DA_SLOTS) {
         float vv[PN];
         const T* vr = staged ? kept + ((size_t)chunk_cap + (key - k0)) * hd : base + 2 * channels + (long long)key * ld;
         Pack<T>::unpack(*reinterpret_cast<const uint4*>(vr + c), vv);
-        const Acc w = s[key - k0];
+        const Acc w = exp(s[key - k0] - mx);
+        weights += w;
 #pragma unroll
         for (int e = 0; e < PN; ++e) acc[e] += w * (Acc)vv[e];
       }
@@ -304,10 +315,16 @@ decode_attention_kernel(const T* __restrict__ qkv, long long ld, int channels, c
   } else {
     for (int c = sub; c < hd; c += 8) {
       Acc acc = 0;
-      for (int key = k0 + slot; key < k1; key += DA_SLOTS) acc += s[key - k0] * (Acc)as_f32(base[2 * channels + (long long)key * ld + c]);
+      weights = 0;
+      for (int key = k0 + slot; key < k1; key += DA_SLOTS) {
+        const Acc w = exp(s[key - k0] - mx);
+        weights += w;
+        acc += w * (Acc)as_f32(base[2 * channels + (long long)key * ld + c]);
+      }
       part[slot * hd + c] = acc;
     }
   }
+  if (sub == 0) slot_sums[slot] = weights;
   __syncthreads();
   Acc* mine = cluster.map_shared_rank(all, 0) + rank * (hd + 2);
   for (int c = threadIdx.x; c < hd; c += DA_THREADS) {
@@ -316,7 +333,13 @@ decode_attention_kernel(const T* __restrict__ qkv, long long ld, int channels, c
     for (int i = 0; i < DA_SLOTS; ++i) v += part[i * hd + c];
     mine[c] = v;
   }
-  if (threadIdx.x == 0) { mine[hd] = mx; mine[hd + 1] = sum; }
+  if (threadIdx.x == 0) {
+    Acc sum = 0;
+#pragma unroll
+    for (int i = 0; i < DA_SLOTS; ++i) sum += slot_sums[i];
+    mine[hd] = mx;
+    mine[hd + 1] = sum;
+  }
   cluster.sync();
   if (rank != 0) return;
   Acc m = -INFINITY, l = 0, f[DA_CTAS];
