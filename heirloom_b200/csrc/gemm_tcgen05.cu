@@ -91,6 +91,8 @@ struct GemmParams {
   unsigned sk_seq;          // this launch's number
   unsigned* sched;          // dynamic tile order: a counter that every processed tile advances by one; null: round-robin
   unsigned sched_base;      // the counter's value when this launch starts (the host adds each launch's tile count)
+  bool skip_c;              // bias + GELU: only the second output is wanted
+  GemmRowStats row_stats;   // SPEC_ROW_STATS
   long long ld_aux_in;
   const float* bias;
   const void* aux_in;
@@ -201,7 +203,10 @@ __device__ __forceinline__ bool get_item(const GemmParams& p, int local, WorkIte
 // tiles whose epilogue (SPEC / 2) and output type (SPEC & 1: bf16) are fixed at compile time, so that an epilogue warp
 // runs straight-line code of its own variant only (the step's short-contraction products are bound by their epilogue);
 // SPEC_PARTIAL: equal splits of the contraction whose raw f32 sums go to the scratch of the second kernel.
+// SPEC_ROW_STATS: bias, and no output but, per row and 128 columns, the maximum and the sum of exponentials below it, and the
+// row's value at its target column (a loss that wants no gradient reads nothing else of the logits).
 constexpr int SPEC_PARTIAL = 16;
+constexpr int SPEC_ROW_STATS = 32;
 template <bool A_MN, bool B_MN, bool PAIR, int SPEC>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -408,9 +413,9 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     // bytes halve the requests of 64-byte rows: 16384 x 3072 x 768 with bias and GELU spent 16 of its 81 us on its stores.
     uint8_t* staging = staging_base + size_t(ew) * (EPI_TILES * EPI_TILE_BYTES);
     int stage_sel = 0;
-    const int epi = SPEC == SPEC_PARTIAL ? HL_EPI_NONE : SPEC >= 0 ? SPEC / 2 : p.epilogue;
+    const int epi = SPEC == SPEC_PARTIAL ? HL_EPI_NONE : SPEC == SPEC_ROW_STATS ? HL_EPI_BIAS : SPEC >= 0 ? SPEC / 2 : p.epilogue;
     const bool partial = SPEC == SPEC_PARTIAL ? true : SPEC >= 0 ? false : p.partial_out != 0;
-    const bool out_bf16 = SPEC == SPEC_PARTIAL ? false : SPEC >= 0 ? (SPEC & 1) != 0 : (!partial && p.out_dtype == HL_BF16);
+    const bool out_bf16 = SPEC == SPEC_PARTIAL || SPEC == SPEC_ROW_STATS ? false : SPEC >= 0 ? (SPEC & 1) != 0 : (!partial && p.out_dtype == HL_BF16);
     const bool need_aux = !partial && (epi == HL_EPI_BIAS_RESIDUAL || epi == HL_EPI_DGELU);
     const bool need_bias = !partial && p.bias != nullptr;
     bool ok = true;
@@ -496,6 +501,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       const bool row_ok = row < p.m;
       const int half_col0 = n_tile * BN + half * 128;
       auto fetch_aux = [&](int chunk, uint4 (&dst)[4]) { fetch_aux_of(w, chunk, dst); };
+      long long target = -1;  // this row's target, counted from the warp's first column
+      if (SPEC == SPEC_ROW_STATS && row_ok) target = __ldg(p.row_stats.targets + row) - half_col0;
       if (!tc05::mbar_wait(&tail->tmem_full[buf], buf_phase, abort_flag, p.wait_limit_ns)) { ok = false; break; }
       tc05::tc_fence_after_sync();
       const uint32_t taddr_row = tmem_base + (uint32_t)(buf * BN) + ((uint32_t)(lane_group * 32) << 16);
@@ -656,7 +663,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             for (int i = 0; i < 4; ++i) words[i] = pack_bf16x2(v[i].x, v[i].y);
           }
           if (out_bf16) {
-            put4(tile, ODD * 4 + g, words);
+            if (!(epi == HL_EPI_BIAS_GELU && p.skip_c)) put4(tile, ODD * 4 + g, words);
           } else {
             const uint32_t f[8] = {__float_as_uint(v[0].x), __float_as_uint(v[0].y), __float_as_uint(v[1].x), __float_as_uint(v[1].y),
                                    __float_as_uint(v[2].x), __float_as_uint(v[2].y), __float_as_uint(v[3].x), __float_as_uint(v[3].y)};
@@ -664,6 +671,44 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             put4(tile, g * 2 + 1, f + 4);
           }
         }
+      };
+      float top = -INFINITY, below = 0.f;  // of this row's columns so far: maximum (times log2 e) and sum of exponentials
+      auto gather = [&](auto sub_odd, int sub, const uint32_t (&acc_bits)[32]) {
+        constexpr int ODD = decltype(sub_odd)::value;
+        constexpr float kLog2e = 1.4426950408889634f;
+        float2 v[16];
+        float mx = -INFINITY;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          const bool in = half_col0 + sub * 32 + g * 8 < p.n;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 b = *reinterpret_cast<const float2*>(bias_tile + ODD * 32 + g * 8 + i * 2);
+            const float2 x = add2(make_float2(__uint_as_float(acc_bits[g * 8 + i * 2]), __uint_as_float(acc_bits[g * 8 + i * 2 + 1])), b);
+            v[g * 4 + i] = in ? x : both(-INFINITY);
+            mx = fmaxf(mx, fmaxf(v[g * 4 + i].x, v[g * 4 + i].y));
+          }
+        }
+        const long long at = target - sub * 32;
+        const bool mine = at >= 0 && at < 32;
+        if (__any_sync(0xffffffffu, mine)) {
+          float z = 0.f;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            if (at == i * 2) z = v[i].x;
+            if (at == i * 2 + 1) z = v[i].y;
+          }
+          if (mine) p.row_stats.target_logit[row] = z;
+        }
+        const float next = fmaxf(top, mx * kLog2e);
+        float2 sums = make_float2(below * ex2_fast(top - next), 0.f);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float2 e = fma2(v[i], both(kLog2e), both(-next));
+          sums = add2(sums, make_float2(ex2_fast(e.x), ex2_fast(e.y)));
+        }
+        top = next;
+        below = sums.x + sums.y;
       };
       // 64 columns at a time, the accumulator's next 32 on their way while the current ones are worked on.  Columns beyond
       // the matrix edge are skipped (the test is uniform across the warp).
@@ -706,8 +751,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           released = true;
           if (!aux_tma) ask_next();
         }
-        process(std::integral_constant<int, 0>{}, sub, acc0, aux_a);
-        if (!out_bf16) store_tile(&map_c, tile, col0);
+        if constexpr (SPEC == SPEC_ROW_STATS) {
+          gather(std::integral_constant<int, 0>{}, sub, acc0);
+        } else {
+          process(std::integral_constant<int, 0>{}, sub, acc0, aux_a);
+          if (!out_bf16) store_tile(&map_c, tile, col0);
+        }
         if (second) {
           if (!kAhead) load_acc(sub + 1, acc1);
           tc05::tmem_ld_wait();
@@ -727,14 +776,18 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
               for (int q = 0; q < 4; ++q) { aux_a[q] = aux_b[q]; aux_b[q] = keep[q]; }
             }
           }
-          process(std::integral_constant<int, 1>{}, sub + 1, acc1, aux_b);
-          if (!out_bf16) store_tile(&map_c, tile, col0 + 32);
+          if constexpr (SPEC == SPEC_ROW_STATS) {
+            gather(std::integral_constant<int, 1>{}, sub + 1, acc1);
+          } else {
+            process(std::integral_constant<int, 1>{}, sub + 1, acc1, aux_b);
+            if (!out_bf16) store_tile(&map_c, tile, col0 + 32);
+          }
         } else if (!aux_tma) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) aux_a[q] = aux_b[q];
         }
         if (out_bf16) {
-          store_tile(&map_c, tile, col0);  // columns past the edge are clipped
+          if (!(epi == HL_EPI_BIAS_GELU && p.skip_c)) store_tile(&map_c, tile, col0);  // columns past the edge are clipped
           if (epi == HL_EPI_BIAS_GELU && !partial) {
             tile = free_tile();
 #pragma unroll
@@ -747,6 +800,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           }
         }
       }
+      if (SPEC == SPEC_ROW_STATS && row_ok && half_col0 < p.n)
+        p.row_stats.parts[(size_t)(n_tile * 2 + half) * p.m + row] = make_float2(top, below);
       if (!released) acc_read();
       if (!ok) break;
       if (have_next == -2) {  // no chunk of this half lies inside the matrix
@@ -954,8 +1009,15 @@ static int check_gemm(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const v
   return HL_OK;
 }
 
+// Whole tiles (of the whole contraction or of equal splits of it; not the dealt-out k blocks) can run on CTA pairs
+// with 256-row tiles.
+static bool pair_form(const hl_ctx* ctx, const hl_gemm_desc* d, const GemmPlan& plan, int sms) {
+  return plan.sk_tiles == 0 && d->m > BM && sms >= 2 && ctx->gemm_skip_kblock < 0 && pairs_enabled(d, plan.splits, sms);
+}
+
 int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, void* c, const float* bias,
-                  const void* aux_in, void* aux_out, float* workspace, size_t workspace_bytes, unsigned* stream_flags) {
+                  const void* aux_in, void* aux_out, float* workspace, size_t workspace_bytes, unsigned* stream_flags,
+                  const GemmRowStats* row_stats) {
   int rc = check_gemm(ctx, d, a, b, c, bias, aux_in, aux_out);
   if (rc != HL_OK) return rc;
   const bool a_mn = d->a_layout == HL_MN_MAJOR, b_mn = d->b_layout == HL_MN_MAJOR;
@@ -966,10 +1028,8 @@ int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void*
   const int sms = persistent_sms(ctx);
   const GemmPlan plan = gemm_plan(d, sms);
   const GemmSmallPlan small = small_plan(ctx, d, plan, sms);
-  if (small.splits > 0) return gemm_small_run(ctx, d, small, a, b, c, bias, aux_in, aux_out);
-  // Whole tiles (of the whole contraction or of equal splits of it; not the dealt-out k blocks) can run on CTA pairs
-  // with 256-row tiles.
-  const bool pair = plan.sk_tiles == 0 && d->m > BM && sms >= 2 && ctx->gemm_skip_kblock < 0 && pairs_enabled(d, plan.splits, sms);
+  if (small.splits > 0 && !row_stats) return gemm_small_run(ctx, d, small, a, b, c, bias, aux_in, aux_out);
+  const bool pair = pair_form(ctx, d, plan, sms);
   GemmParams p{};
   p.m = d->m; p.n = d->n; p.k = d->k;
   p.m_tiles = ceil_div(d->m, pair ? 2 * BM : BM);
@@ -1012,6 +1072,8 @@ int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void*
   p.k_blocks_per_split = ceil_div(p.k_blocks, splits);
   p.epilogue = d->epilogue;
   p.out_dtype = d->out_dtype;
+  p.skip_c = ctx->forward_only;
+  if (row_stats) p.row_stats = *row_stats;
   p.ld_aux_in = ld_aux_in;
   p.bias = bias; p.aux_in = aux_in;
   p.status = ctx->status_dev;
@@ -1068,7 +1130,8 @@ int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void*
   constexpr int kBias = HL_EPI_BIAS * 2, kGelu = HL_EPI_BIAS_GELU * 2, kResidual = HL_EPI_BIAS_RESIDUAL * 2,
                 kDgelu = HL_EPI_DGELU * 2, kNone = HL_EPI_NONE * 2;
   bool launched = true;
-  if (!a_mn && !b_mn && !pair && spec == kBias + 1) rc = launch_variant<false, false, false, kBias + 1>(ctx, ma, mb, mc, maux, p, grid);
+  if (row_stats) rc = launch_variant<false, false, true, SPEC_ROW_STATS>(ctx, ma, mb, mc, maux, p, grid);
+  else if (!a_mn && !b_mn && !pair && spec == kBias + 1) rc = launch_variant<false, false, false, kBias + 1>(ctx, ma, mb, mc, maux, p, grid);
   else if (!a_mn && !b_mn && !pair && spec == kBias) rc = launch_variant<false, false, false, kBias>(ctx, ma, mb, mc, maux, p, grid);
   else if (!a_mn && !b_mn && !pair && spec == kGelu + 1) rc = launch_variant<false, false, false, kGelu + 1>(ctx, ma, mb, mc, maux, p, grid);
   else if (!a_mn && !b_mn && !pair && spec == kResidual + 1) rc = launch_variant<false, false, false, kResidual + 1>(ctx, ma, mb, mc, maux, p, grid);
@@ -1138,6 +1201,16 @@ int gemm_bf16_ctx(hl_ctx* ctx, const hl_gemm_desc* desc, const void* a, const vo
 }  // namespace hl
 
 namespace hl {
+bool gemm_bf16_row_stats(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, const float* bias, const GemmRowStats& stats,
+                         void* unused_c, int* rc) {
+  const int sms = persistent_sms(ctx);
+  const GemmPlan plan = gemm_plan(d, sms);
+  if (d->epilogue != HL_EPI_BIAS || d->out_dtype != HL_F32 || d->a_layout != HL_K_MAJOR || d->b_layout != HL_K_MAJOR ||
+      plan.splits != 1 || small_plan(ctx, d, plan, sms).splits > 0 || !pair_form(ctx, d, plan, sms))
+    return false;
+  *rc = gemm_bf16_run(ctx, d, a, b, unused_c, bias, nullptr, nullptr, nullptr, 0, nullptr, &stats);
+  return true;
+}
 bool gemm_bf16_small_applies(hl_ctx* ctx, const hl_gemm_desc* d) {
   const int sms = persistent_sms(ctx);
   return small_plan(ctx, d, gemm_plan(d, sms), sms).splits > 0;

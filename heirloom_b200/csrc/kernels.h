@@ -14,8 +14,22 @@ struct GemmPlan {
   size_t sk_slot_bytes;  // scratch for the raw accumulators of partly finished tiles
 };
 GemmPlan gemm_plan(const hl_gemm_desc* d, int sm_count);
+// For a cross-entropy loss without gradients: per 128 columns (n in all, `parts` is [ceil(n/128)][m]) and row the maximum times
+// log2(e) and the sum of 2^(x log2(e) - that), and the row's value at its target (nothing when it is out of range).
+struct GemmRowStats {
+  float2* parts;
+  float* target_logit;  // [m]
+  const int64_t* targets;
+};
 int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, void* c, const float* bias,
-                  const void* aux_in, void* aux_out, float* workspace, size_t workspace_bytes, unsigned* stream_flags);
+                  const void* aux_in, void* aux_out, float* workspace, size_t workspace_bytes, unsigned* stream_flags,
+                  const GemmRowStats* row_stats = nullptr);
+// The product with bias of which only those are wanted; false when this shape has no such form and nothing was done.
+// `unused_c`: any memory of the result's size.
+bool gemm_bf16_row_stats(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, const float* bias, const GemmRowStats& stats,
+                         void* unused_c, int* rc);
+// The mean loss out of them.
+int row_stats_loss(hl_ctx* ctx, const GemmRowStats& stats, int rows, int classes, float* row_loss, float* loss_dev);
 // Products that leave most of the chip idle in 128 x 256 tiles (gemm_small.cu): how many CTAs share the contraction of one of
 // its 128 x bn tiles (0: not one of them), and whether a CTA has the SM's shared memory to itself.
 struct GemmSmallPlan {

@@ -458,6 +458,52 @@ cross_entropy_online_kernel(const float* __restrict__ logits, long long ld, cons
   mean_when_last(row_loss, rows, mean);
 }
 
+// Row losses out of the maxima and sums that the head's product left per 128 columns: 32 rows a block, a warp takes every
+// eighth part of them.  Reads rows x classes/16 bytes where the logits would be rows x 4 x classes, which are not written either
+// (8192 x 50304: 690 us of product and 300 of loss before).
+__global__ void __launch_bounds__(256)
+row_stats_loss_kernel(const GemmRowStats stats, int rows, int parts, int classes, float* __restrict__ row_loss, int* __restrict__ status,
+                      const MeanLoss mean) {
+  pdl_begin();
+  __shared__ float tops[8][33], sums[8][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int row = blockIdx.x * 32 + lane;
+  float top = -INFINITY, sum = 0.f;
+  if (row < rows) {
+    for (int p0 = warp; p0 < parts; p0 += 64) {
+      float2 v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        v[u] = p0 + u * 8 < parts ? stats.parts[(size_t)(p0 + u * 8) * rows + row] : make_float2(-INFINITY, 0.f);
+      float next = top;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) next = fmaxf(next, v[u].x);
+      sum *= ex2_fast(top - next);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) sum += v[u].y * ex2_fast(v[u].x - next);
+      top = next;
+    }
+  }
+  tops[warp][lane] = top;
+  sums[warp][lane] = sum;
+  __syncthreads();
+  if (warp == 0 && row < rows) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) top = fmaxf(top, tops[w][lane]);
+    sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) sum += sums[w][lane] * ex2_fast(tops[w][lane] - top);
+    const long long target = stats.targets[row];
+    if (target < 0 || target >= classes) {
+      atomicExch(status + ST_BAD_INDEX, 1);
+      row_loss[row] = 0.f;
+    } else {
+      row_loss[row] = -stats.target_logit[row] + top * 0.6931471805599453f + logf(sum);
+    }
+  }
+  mean_when_last(row_loss, rows, mean);
+}
+
 }  // namespace
 
 int layer_norm_forward_impl(hl_ctx* ctx, const void* x, int x_dtype, const float* gamma, const float* beta, void* y,
@@ -490,6 +536,16 @@ int layer_norm_forward_impl(hl_ctx* ctx, const void* x, int x_dtype, const float
   else return fail("hl_layer_norm_forward: dtypes must be f32 or bf16");
 #undef HL_LN_FWD
   HL_LAUNCH_CHECK("layer_norm_fwd_kernel");
+  count_launch(ctx);
+  return HL_OK;
+}
+
+int row_stats_loss(hl_ctx* ctx, const GemmRowStats& stats, int rows, int classes, float* row_loss, float* loss_dev) {
+  const int parts = ceil_div(classes, 128);
+  ProfileScope prof(ctx, HL_PROF_LOSS, (double)rows * parts * 8.0);
+  const MeanLoss mean{loss_dev, nullptr, ctx->gemm_sched + 8};  // a word of the context's zeroed counters
+  pdl(row_stats_loss_kernel, ceil_div(rows, 32), 256, 0, ctx->stream)(stats, rows, parts, classes, row_loss, ctx->status_dev, mean);
+  HL_LAUNCH_CHECK("row_stats_loss_kernel");
   count_launch(ctx);
   return HL_OK;
 }

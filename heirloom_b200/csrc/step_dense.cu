@@ -628,9 +628,16 @@ int decode_head(hl_decoder* m, const void* x, int dtype) {
   return decode_gemv(m->ctx, g);
 }
 
-// `last_only`: nothing is read but the logits of the last position, which go to row 0 of m->logits.
-int forward(hl_decoder* m, bool last_only = false) {
+// What a forward pass is for: logits and activations for the backward pass, the logits of the last position alone (they go to
+// row 0 of m->logits), or the mean loss alone (to m->loss_dev).
+enum class Forward { all, last_position, loss };
+int forward(hl_decoder* m, Forward what = Forward::all) {
   hl_ctx* ctx = m->ctx;
+  struct Only {  // no backward pass follows
+    hl_ctx* c;
+    ~Only() { c->forward_only = false; }
+  } only{ctx};
+  ctx->forward_only = what != Forward::all;
   const hl_decoder_config& c = m->cfg;
   const int N = m->N, d = c.d_model, F = c.d_ff, V = c.vocab, B = c.batch, T = c.context, H = c.n_heads;
   const Gemm g{m};
@@ -678,11 +685,29 @@ int forward(hl_decoder* m, bool last_only = false) {
                  P + o.b2, a.r, d));
   }
   m->cached = 0;
-  if (last_only) return decode_head(m, m->x[c.n_layers] + (size_t)(N - 1) * d, HL_BF16);
+  if (what == Forward::last_position) return decode_head(m, m->x[c.n_layers] + (size_t)(N - 1) * d, HL_BF16);
   HL_TRY(layer_norm_forward_impl(ctx, m->x[c.n_layers], HL_BF16, P + m->off_lnf_g, P + m->off_lnf_b, m->z, HL_BF16, m->meanf,
                                  m->rstdf, N, d, 1e-5f));
+  if (what == Forward::loss) {
+    // maxima and sums of the logits without the logits, in the buffer that would hold them
+    hl_gemm_desc desc{};
+    desc.m = N; desc.n = V; desc.k = d;
+    desc.a_layout = desc.b_layout = HL_K_MAJOR;
+    desc.lda = desc.ldb = d; desc.ldc = V;
+    desc.epilogue = HL_EPI_BIAS; desc.out_dtype = HL_F32;
+    const size_t parts = (size_t)ceil_div(V, 128) * N;
+    const GemmRowStats stats{reinterpret_cast<float2*>(m->logits), m->logits + 2 * parts, m->targets};
+    int rc = HL_OK;
+    if (2 * parts + 2 * (size_t)N <= (size_t)N * V &&
+        gemm_bf16_row_stats(ctx, &desc, m->z, W + m->off_head_w, P + m->off_head_b, stats, m->logits, &rc)) {
+      HL_TRY(rc);
+      return row_stats_loss(ctx, stats, N, V, m->logits + 2 * parts + N, m->loss_dev);
+    }
+  }
   HL_TRY(g.run(N, V, d, m->z, d, HL_K_MAJOR, W + m->off_head_w, d, HL_K_MAJOR, m->logits, V, HL_F32, HL_EPI_BIAS,
                P + m->off_head_b));
+  if (what == Forward::loss)
+    return cross_entropy_impl(ctx, m->logits, V, m->targets, N, V, 1.0f, m->loss_dev, nullptr, nullptr, HL_BF16, V);
   return HL_OK;
 }
 
@@ -1907,8 +1932,8 @@ int hl_decoder_eval_loss(hl_decoder* m, const int64_t* tokens_dev, const int64_t
   {
     ScopedShape shape(m, sequences, m->cfg.context);
     HL_TRY(run_graphed(m, GRAPH_LOSS, [m]() -> int {
-      if (m->cfg.precision == HL_PRECISION_AMP_BF16) HL_TRY(forward(m));
-      else HL_TRY(forward_f32(m));
+      if (m->cfg.precision == HL_PRECISION_AMP_BF16) return forward(m, Forward::loss);
+      HL_TRY(forward_f32(m));
       return cross_entropy_impl(m->ctx, m->logits, m->cfg.vocab, m->targets, m->N, m->cfg.vocab, 1.0f, m->loss_dev, nullptr,
                                 nullptr, HL_BF16, m->cfg.vocab);
     }));
@@ -1942,7 +1967,7 @@ static int run_window(hl_decoder* m, const int64_t* window, cudaMemcpyKind kind,
   HL_CUDA(cudaMemcpyAsync(m->tokens, window, sizeof(int64_t) * window_len, kind, ctx->stream));
   {
     ScopedShape shape(m, 1, window_len);
-    HL_TRY(run_graphed(m, GRAPH_WINDOW, [m]() { return m->cfg.precision == HL_PRECISION_AMP_BF16 ? forward(m, true) : forward_f32(m, true); }));
+    HL_TRY(run_graphed(m, GRAPH_WINDOW, [m]() { return m->cfg.precision == HL_PRECISION_AMP_BF16 ? forward(m, Forward::last_position) : forward_f32(m, true); }));
     m->cached = 0;
   }
   HL_TRY(queue_result(m, greedy));

@@ -4,6 +4,7 @@ import math
 
 import numpy as np
 import pytest
+import torch
 
 from heirloom_b200 import generation as gen
 from oracle import heirloom_oracle as ho
@@ -205,4 +206,28 @@ def test_the_device_picks_the_greedy_token_that_sampling_picks(vocab):
             want = gen.sample_token(gen.next_token_logits(model, tokens[:n]), tokens[:n], options, gen.HeirloomRng(0))
             assert got[0] == want[0] and (not tied or got[0] == vocab - 1)
             assert got[1] == pytest.approx(want[1], rel=vocab * 2e-16 + 1e-14)
+    model.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,vocab", [(13, 5000), (12, 8200), (20, 3208)])
+def test_evaluation_loss_equals_the_training_pass_loss(batch, vocab):
+    """The head's product that leaves maxima and sums per 128 columns, against the logits and the loss kernel of a training
+    pass on the same tokens: last rows and columns ragged (1300 x 5000, 1200 x 8200, 2000 x 3208), one sequence of it, targets in
+    the first and last column.  Both add f32 exponentials of the same f32 logits: a few ulps of the loss."""
+    from heirloom_b200 import nn
+    from tests.gpu_util import ctx
+    c = ctx()
+    model = nn.DecoderLm(c, nn.DecoderConfig(vocab=vocab, d_model=128, n_layers=1, n_heads=2, d_ff=128, context=100, batch=batch))
+    rng = np.random.default_rng(vocab)
+    model.load_state_dict({n: rng.standard_normal(s) * 0.2 for n, s in model.parameter_shapes().items()})
+    x = torch.from_numpy(rng.integers(0, vocab, (batch, 100))).cuda()
+    y = torch.from_numpy(rng.integers(0, vocab, (batch, 100))).cuda()
+    y[0, :2] = torch.tensor([0, vocab - 1])
+    model.forward_backward(x, y)
+    want = model.loss()
+    for _ in range(3):  # plain, captured, replayed
+        assert model.eval_loss_device(x, y) == pytest.approx(want, rel=2e-6)
+    whole = [model.eval_loss_device(x[i:i + 1], y[i:i + 1]) for i in range(batch)]
+    assert np.mean(whole) == pytest.approx(want, rel=2e-6)
     model.close()
