@@ -10,55 +10,57 @@
 //
 // Layout: q, k, v are bf16 row-major [B*T, *] views with heads interleaved along the channel
 // dimension (column h*hd + j, as src/tensor.rs:5156-5177), so they may live side by side in
-// one fused [B*T, 3C] projection buffer.  One CTA owns 128 query rows of one (batch, head).
+// one fused [B*T, 3C] projection buffer.  A work item is 128 query rows of one (batch, head).
 //
-// Pipeline: key tiles of 64; two S buffers and the O accumulator in tensor memory and two P buffers in
-// shared memory.  Four softmax warps (one per tensor-memory lane group, a thread per query row) work
-// on tile j while the tensor cores run P·V of tile j-1 and Q·Kᵀ of tile j+1.  P is formed against a
-// reference maximum that a row raises only when its maximum has grown by more than 2^8; the row then
-// rescales its O in place (tensor-memory load, multiply, store) between two P·V products.  The CTA
-// is sized (192 threads, 98 KB of shared memory, 256 tensor-memory columns) so that two of them share
-// an SM and one's start-up and drain overlap the other's work.
+// Pipeline: key tiles of 64; two S buffers and the O accumulator in tensor memory, P in shared memory.  Four softmax warps (one
+// per tensor-memory lane group, a thread per query row) work on tile j while the tensor cores run P·V of tile j-1 and Q·Kᵀ of
+// tile j+1.  P is formed against a reference maximum that a row raises only when its maximum has grown by more than 2^8; the row
+// then rescales its O in place (tensor-memory load, multiply, store) between two P·V products.
+//
+// Two persistent CTAs share an SM (192 threads, 112 KB of shared memory, 256 tensor-memory columns each), so that one's tensor
+// work and waits lie under the other's exponentials, and each goes through its items without a gap: while the softmax warps
+// write one item's result, the next one's first scores are being formed.  With a CTA per item (B16 H12 T1024: 69 us) 29 us were
+// starts and ends of CTAs; heads of 128 channels had one CTA an SM and nothing to hide a warp's chain under (B4 H12 T4096: 311 us).
 #include "common.cuh"
 #include "tc05.cuh"
 
 namespace hl {
 namespace {
 
-constexpr int FA_BM = 128;   // query rows per CTA
+constexpr int FA_BM = 128;   // query rows per item
 constexpr int FA_BN = 64;    // keys per tile
-constexpr int FA_KV_STAGES = 3;
 constexpr int FA_P_BYTES = FA_BM * FA_BN * 2;   // 16 KB: 128 rows of 64 keys, one 128-byte line each
 constexpr int FA_SOFTMAX_WARPS = 4;
 constexpr int FA_THREADS = (FA_SOFTMAX_WARPS + 2) * 32;  // + TMA warp + MMA warp
 constexpr int FA_TMEM_COLS = 256;  // S: 2 x 64 columns, O: head_dim columns (allocations are powers of two)
 
 // Sizes that depend on the head dimension (64 or 128).  Operands wider than one 128-byte swizzle row are kept as
-// blocks of 64 channels side by side: a Q block is [128 rows x 128 bytes], a K or V block [64 keys x 128 bytes].
+// blocks of 64 channels side by side: a Q block is [128 rows x 128 bytes], a K or V block [64 keys x 128 bytes].  A head of 64
+// has room for the next item's Q and a second P; one of 128 for neither at two CTAs an SM.
 template <int HD>
 struct FaSizes {
   static_assert(HD == 64 || HD == 128, "head_dim 64 or 128");
   static constexpr int BLOCKS = HD / 64;
+  static constexpr int Q_BUFS = HD == 64 ? 2 : 1, P_BUFS = HD == 64 ? 2 : 1, KV_STAGES = HD == 64 ? 3 : 2;
   static constexpr int Q_BLOCK = FA_BM * 128;            // 16 KB
   static constexpr int KV_BLOCK = FA_BN * 128;           // 8 KB
   static constexpr int Q_BYTES = BLOCKS * Q_BLOCK;
   static constexpr int KV_BYTES = BLOCKS * KV_BLOCK;
-  static constexpr int SMEM_DATA = Q_BYTES + 2 * FA_KV_STAGES * KV_BYTES + 2 * FA_P_BYTES;  // 96 KB / 160 KB
-  static constexpr int SMEM_BYTES = SMEM_DATA + 2048;    // barriers in front, alignment slack
-  static constexpr int CTAS_PER_SM = HD == 64 ? 2 : 1;
-  static_assert(CTAS_PER_SM * (SMEM_BYTES + 1024) <= 228 * 1024, "shared memory per SM");
+  static constexpr int SMEM_DATA = Q_BUFS * Q_BYTES + 2 * KV_STAGES * KV_BYTES + P_BUFS * FA_P_BYTES;  // 112 KB
+  static constexpr int SMEM_BYTES = SMEM_DATA + 256;     // barriers behind the tiles
+  static_assert(2 * (SMEM_BYTES + 1024) <= 228 * 1024, "shared memory per SM");
   static_assert(2 * FA_BN + HD <= FA_TMEM_COLS, "tensor memory columns");
 };
 
 struct FaShared {
-  uint64_t q_full;
-  uint64_t k_full[FA_KV_STAGES], k_empty[FA_KV_STAGES];
-  uint64_t v_full[FA_KV_STAGES], v_empty[FA_KV_STAGES];
+  uint64_t q_full[2], q_empty[2];
+  uint64_t k_full[3], k_empty[3];
+  uint64_t v_full[3], v_empty[3];
   uint64_t s_full[2], p_full[2], o_full[2];
   uint32_t tmem_base;
   int abort_flag;
 };
-static_assert(sizeof(FaShared) + 1023 <= 2048, "front matter must fit the slack");
+static_assert(sizeof(FaShared) <= 256, "barriers outgrow their place");
 
 struct FaParams {
   int B, T, H;
@@ -69,43 +71,54 @@ struct FaParams {
   int* status;
 };
 
+// The items of a CTA, longest walks first; rounds over the CTAs alternate direction, which evens out their totals.  Every warp
+// role advances an identical copy.
+struct FaItem {
+  int local, q0, b, h, n_tiles;  // n_tiles: key tiles of 64 up to and including the diagonal; 0: no more items
+};
+__device__ __forceinline__ FaItem fa_item(int local, const FaParams& p) {
+  const int nq = (p.T + FA_BM - 1) / FA_BM, heads = p.B * p.H;
+  const int grid = (int)gridDim.x, cta = (int)blockIdx.x;
+  const int item = local * grid + ((local & 1) ? grid - 1 - cta : cta);
+  FaItem it{local, 0, 0, 0, 0};
+  if (item >= nq * heads) return it;
+  const int qi = nq - 1 - item / heads, bh = item % heads;
+  it.q0 = qi * FA_BM;
+  it.b = bh / p.H;
+  it.h = bh % p.H;
+  it.n_tiles = 2 * (qi + 1);
+  return it;
+}
+
 template <int HD>
-__global__ void __launch_bounds__(FA_THREADS, FaSizes<HD>::CTAS_PER_SM)
+__global__ void __launch_bounds__(FA_THREADS, 2)
 flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                            const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
                            const FaParams p) {
   using Z = FaSizes<HD>;
-  constexpr int FA_HD = HD;
-  constexpr int FA_Q_BYTES = Z::Q_BYTES, FA_KV_BYTES = Z::KV_BYTES, FA_SMEM_DATA = Z::SMEM_DATA, FA_SMEM_BYTES = Z::SMEM_BYTES;
-  extern __shared__ uint8_t fa_smem_raw[];
-  const uintptr_t raw = reinterpret_cast<uintptr_t>(fa_smem_raw);
-  uint8_t* tiles = reinterpret_cast<uint8_t*>((raw + sizeof(FaShared) + 1023) & ~uintptr_t(1023));
-  FaShared* sh = reinterpret_cast<FaShared*>(fa_smem_raw);
-  const bool layout_ok = (tiles + FA_SMEM_DATA) <= (fa_smem_raw + FA_SMEM_BYTES);
-  uint8_t* sq = tiles;
-  uint8_t* sk = sq + FA_Q_BYTES;
+  constexpr int FA_HD = HD, FA_KV_STAGES = Z::KV_STAGES;
+  constexpr int FA_Q_BYTES = Z::Q_BYTES, FA_KV_BYTES = Z::KV_BYTES;
+  extern __shared__ __align__(1024) uint8_t fa_smem[];  // swizzled tiles want 1024 bytes; checked below
+  uint8_t* sq = fa_smem;                          // [Q_BUFS]
+  uint8_t* sk = sq + Z::Q_BUFS * FA_Q_BYTES;
   uint8_t* sv = sk + FA_KV_STAGES * FA_KV_BYTES;
-  uint8_t* sp = sv + FA_KV_STAGES * FA_KV_BYTES;  // two P buffers
+  uint8_t* sp = sv + FA_KV_STAGES * FA_KV_BYTES;  // [P_BUFS]
+  FaShared* sh = reinterpret_cast<FaShared*>(fa_smem + Z::SMEM_DATA);
+  const bool layout_ok = (tc05::smem_u32(fa_smem) & 1023u) == 0;
   volatile int* abort_flag = &sh->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nq = (p.T + FA_BM - 1) / FA_BM;
-  const int bh = blockIdx.x % (p.B * p.H);
-  const int qi = nq - 1 - blockIdx.x / (p.B * p.H);  // heavy (late) query tiles are scheduled first
-  const int b = bh / p.H, h = bh % p.H;
-  const int q0 = qi * FA_BM;
-  const int n_tiles = 2 * (qi + 1);  // key tiles of 64 up to and including the diagonal
-  const int row_base = b * p.T;  // first row of this batch in the [B*T, *] views
 
   if (threadIdx.x == 0) {
-    tc05::mbar_init(&sh->q_full, 1);
-    for (int s = 0; s < FA_KV_STAGES; ++s) {
+    for (int s = 0; s < 3; ++s) {
       tc05::mbar_init(&sh->k_full[s], 1);
       tc05::mbar_init(&sh->k_empty[s], 1);
       tc05::mbar_init(&sh->v_full[s], 1);
       tc05::mbar_init(&sh->v_empty[s], 1);
     }
     for (int i = 0; i < 2; ++i) {
+      tc05::mbar_init(&sh->q_full[i], 1);
+      tc05::mbar_init(&sh->q_empty[i], FA_SOFTMAX_WARPS);
       tc05::mbar_init(&sh->s_full[i], 1);
       tc05::mbar_init(&sh->p_full[i], FA_SOFTMAX_WARPS);
       tc05::mbar_init(&sh->o_full[i], 1);
@@ -130,25 +143,34 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       tc05::tma_prefetch_desc(&map_q);
       tc05::tma_prefetch_desc(&map_k);
       tc05::tma_prefetch_desc(&map_v);
-      tc05::mbar_arrive_expect_tx(&sh->q_full, FA_Q_BYTES);
-#pragma unroll
-      for (int blk = 0; blk < Z::BLOCKS; ++blk)
-        tc05::tma_load_2d(sq + blk * Z::Q_BLOCK, &map_q, &sh->q_full, h * FA_HD + blk * 64, row_base + q0);
-      for (int j = 0; j < n_tiles; ++j) {
-        const int s = j % FA_KV_STAGES;
-        const uint32_t ph = (uint32_t)(j / FA_KV_STAGES) & 1u;
-        if (!tc05::mbar_wait(&sh->k_empty[s], ph ^ 1u, abort_flag)) break;
-        tc05::mbar_arrive_expect_tx(&sh->k_full[s], FA_KV_BYTES);
+      bool ok = true;
+      int g = 0;  // key tiles loaded so far
+      for (FaItem it = fa_item(0, p); ok && it.n_tiles > 0; it = fa_item(it.local + 1, p)) {
+        const int row_base = it.b * p.T;  // first row of this batch in the [B*T, *] views
+        const int qb = it.local % Z::Q_BUFS;
+        if (!tc05::mbar_wait(&sh->q_empty[qb], ((uint32_t)(it.local / Z::Q_BUFS) & 1u) ^ 1u, abort_flag)) break;
+        tc05::mbar_arrive_expect_tx(&sh->q_full[qb], FA_Q_BYTES);
 #pragma unroll
         for (int blk = 0; blk < Z::BLOCKS; ++blk)
-          tc05::tma_load_2d(sk + s * FA_KV_BYTES + blk * Z::KV_BLOCK, &map_k, &sh->k_full[s], h * FA_HD + blk * 64,
-                            row_base + j * FA_BN);
-        if (!tc05::mbar_wait(&sh->v_empty[s], ph ^ 1u, abort_flag)) break;
-        tc05::mbar_arrive_expect_tx(&sh->v_full[s], FA_KV_BYTES);
+          tc05::tma_load_2d(sq + qb * FA_Q_BYTES + blk * Z::Q_BLOCK, &map_q, &sh->q_full[qb], it.h * FA_HD + blk * 64, row_base + it.q0);
+        for (int j = 0; j < it.n_tiles; ++j, ++g) {
+          const int s = g % FA_KV_STAGES;
+          const uint32_t ph = (uint32_t)(g / FA_KV_STAGES) & 1u;
+          ok = tc05::mbar_wait(&sh->k_empty[s], ph ^ 1u, abort_flag);
+          if (!ok) break;
+          tc05::mbar_arrive_expect_tx(&sh->k_full[s], FA_KV_BYTES);
 #pragma unroll
-        for (int blk = 0; blk < Z::BLOCKS; ++blk)
-          tc05::tma_load_2d(sv + s * FA_KV_BYTES + blk * Z::KV_BLOCK, &map_v, &sh->v_full[s], h * FA_HD + blk * 64,
-                            row_base + j * FA_BN);
+          for (int blk = 0; blk < Z::BLOCKS; ++blk)
+            tc05::tma_load_2d(sk + s * FA_KV_BYTES + blk * Z::KV_BLOCK, &map_k, &sh->k_full[s], it.h * FA_HD + blk * 64,
+                              row_base + j * FA_BN);
+          ok = tc05::mbar_wait(&sh->v_empty[s], ph ^ 1u, abort_flag);
+          if (!ok) break;
+          tc05::mbar_arrive_expect_tx(&sh->v_full[s], FA_KV_BYTES);
+#pragma unroll
+          for (int blk = 0; blk < Z::BLOCKS; ++blk)
+            tc05::tma_load_2d(sv + s * FA_KV_BYTES + blk * Z::KV_BLOCK, &map_v, &sh->v_full[s], it.h * FA_HD + blk * 64,
+                              row_base + j * FA_BN);
+        }
       }
     }
   } else if (warp == FA_SOFTMAX_WARPS + 1) {
@@ -156,71 +178,94 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     if (tc05::elect_one() && !*abort_flag) {
       constexpr uint32_t idesc_qk = tc05::instr_desc_bf16_f32(FA_BM, FA_BN, false, false);
       constexpr uint32_t idesc_pv = tc05::instr_desc_bf16_f32(FA_BM, FA_HD, false, true);
-      const uint32_t aq = tc05::smem_u32(sq);
-      auto issue_qk = [&](int j) -> bool {  // S[j & 1] = Q · K(j)ᵀ
-        const int s = j % FA_KV_STAGES;
-        if (!tc05::mbar_wait(&sh->k_full[s], (uint32_t)(j / FA_KV_STAGES) & 1u, abort_flag)) return false;
+      // Q·Kᵀ runs two tiles ahead of P·V, into the next item where this one ends.
+      FaItem qi = fa_item(0, p);
+      int qj = 0, qg = 0;  // the next scores: tile of the item, tile of the CTA
+      auto issue_qk = [&]() -> bool {  // S[qg & 1] = Q · K(qj)ᵀ
+        if (qi.n_tiles == 0) return true;
+        const int qb = qi.local % Z::Q_BUFS, s = qg % FA_KV_STAGES;
+        if (qj == 0 && !tc05::mbar_wait(&sh->q_full[qb], (uint32_t)(qi.local / Z::Q_BUFS) & 1u, abort_flag)) return false;
+        if (!tc05::mbar_wait(&sh->k_full[s], (uint32_t)(qg / FA_KV_STAGES) & 1u, abort_flag)) return false;
         tc05::tc_fence_after_sync();
-        const uint32_t ak = tc05::smem_u32(sk + s * FA_KV_BYTES);
+        const uint32_t aq = tc05::smem_u32(sq + qb * FA_Q_BYTES), ak = tc05::smem_u32(sk + s * FA_KV_BYTES);
 #pragma unroll
         for (int ks = 0; ks < FA_HD / 16; ++ks)  // 16 channels a step; four steps per 64-channel block
-          tc05::umma_ss(tmem_s0 + (uint32_t)((j & 1) * FA_BN),
+          tc05::umma_ss(tmem_s0 + (uint32_t)((qg & 1) * FA_BN),
                         tc05::smem_desc_sw128(aq + (ks / 4) * Z::Q_BLOCK + (ks % 4) * 32, 16, 1024),
                         tc05::smem_desc_sw128(ak + (ks / 4) * Z::KV_BLOCK + (ks % 4) * 32, 16, 1024), idesc_qk,
                         ks > 0 ? 1u : 0u);
         tc05::umma_commit(&sh->k_empty[s]);
-        tc05::umma_commit(&sh->s_full[j & 1]);
+        tc05::umma_commit(&sh->s_full[qg & 1]);
+        ++qg;
+        if (++qj == qi.n_tiles) {
+          qi = fa_item(qi.local + 1, p);
+          qj = 0;
+        }
         return true;
       };
-      bool ok = tc05::mbar_wait(&sh->q_full, 0, abort_flag);
-      if (ok) ok = issue_qk(0);
-      if (ok && n_tiles > 1) ok = issue_qk(1);
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        // P(j) is in shared memory, which also means S(j) has been read out of tensor memory
-        if (!tc05::mbar_wait(&sh->p_full[j & 1], (uint32_t)(j >> 1) & 1u, abort_flag)) break;
-        tc05::tc_fence_after_sync();
-        const int s = j % FA_KV_STAGES;
-        if (!tc05::mbar_wait(&sh->v_full[s], (uint32_t)(j / FA_KV_STAGES) & 1u, abort_flag)) break;
-        tc05::tc_fence_after_sync();
-        const uint32_t av = tc05::smem_u32(sv + s * FA_KV_BYTES);
-        const uint32_t ap = tc05::smem_u32(sp + (j & 1) * FA_P_BYTES);
+      bool ok = issue_qk();
+      // A single Q buffer is overwritten once the item's result has left through it, which the softmax warps do after the last
+      // P·V: the scores of the next item then wait until those have been issued.
+      auto may_run_ahead = [&](bool last_of_item) { return Z::Q_BUFS == 2 || qj > 0 || last_of_item; };
+      int ahead = 1;  // scores issued beyond the tile at hand
+      int g = 0;
+      for (FaItem it = fa_item(0, p); ok && it.n_tiles > 0; it = fa_item(it.local + 1, p)) {
+        for (int j = 0; j < it.n_tiles && ok; ++j, ++g) {
+          while (ok && ahead < 2 && qi.n_tiles > 0 && may_run_ahead(false)) {
+            ok = issue_qk();
+            ++ahead;
+          }
+          if (!ok) break;
+          // P(g) is in shared memory, which also means S(g) has been read out of tensor memory and, in an item's first tile, the
+          // last item's O as well
+          if (!tc05::mbar_wait(&sh->p_full[g % Z::P_BUFS], (uint32_t)(g / Z::P_BUFS) & 1u, abort_flag)) { ok = false; break; }
+          tc05::tc_fence_after_sync();
+          const int s = g % FA_KV_STAGES;
+          if (!tc05::mbar_wait(&sh->v_full[s], (uint32_t)(g / FA_KV_STAGES) & 1u, abort_flag)) { ok = false; break; }
+          tc05::tc_fence_after_sync();
+          const uint32_t av = tc05::smem_u32(sv + s * FA_KV_BYTES);
+          const uint32_t ap = tc05::smem_u32(sp + (g % Z::P_BUFS) * FA_P_BYTES);
 #pragma unroll
-        for (int ks = 0; ks < FA_BN / 16; ++ks) {
-          // A = P: [128 rows x 64 keys], K-major; B = V: rows are keys (MN-major), 16 keys per step
-          const uint64_t da = tc05::smem_desc_sw128(ap + ks * 32, 16, 1024);
-          const uint64_t db = tc05::smem_desc_sw128(av + ks * (16 * 128), Z::KV_BLOCK, 1024);  // channel blocks KV_BLOCK apart
-          tc05::umma_ss(tmem_o0, da, db, idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);  // O accumulates over the key tiles
+          for (int ks = 0; ks < FA_BN / 16; ++ks) {
+            // A = P: [128 rows x 64 keys], K-major; B = V: rows are keys (MN-major), 16 keys per step
+            const uint64_t da = tc05::smem_desc_sw128(ap + ks * 32, 16, 1024);
+            const uint64_t db = tc05::smem_desc_sw128(av + ks * (16 * 128), Z::KV_BLOCK, 1024);  // channel blocks KV_BLOCK apart
+            tc05::umma_ss(tmem_o0, da, db, idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);  // O accumulates over the key tiles
+          }
+          tc05::umma_commit(&sh->v_empty[s]);
+          tc05::umma_commit(&sh->o_full[g % Z::P_BUFS]);
+          --ahead;
+          if (ahead < 1 && qi.n_tiles > 0) {  // a single Q buffer, at the end of an item
+            ok = issue_qk();
+            ++ahead;
+          }
         }
-        tc05::umma_commit(&sh->v_empty[s]);
-        tc05::umma_commit(&sh->o_full[j & 1]);
-        if (j + 2 < n_tiles && !issue_qk(j + 2)) break;
       }
     }
   } else {
     // -------------------------------------------------------------------------- softmax warps
     const int r = warp * 32 + lane;     // query row within the tile == tensor-memory lane
-    const int t = q0 + r;               // query position within the batch
     const uint32_t lane_sel = (uint32_t)(warp * 32) << 16;
     // O accumulates in tensor memory against a reference maximum m_ref that is only raised when a row's maximum has
     // grown by more than 2^8 since: P = 2^(s - m_ref) then stays below 256, which costs bf16 nothing (same relative
     // precision) and f32 sums nothing, and O is rescaled in place a few times per row instead of once per tile.
     constexpr float kRaise = 8.0f;
+    bool ok = !*abort_flag;
+    bool stored = false;  // this warp's rows of the last item are on their way out of its Q buffer
+    int g = 0;            // key tiles done so far
+
+    for (FaItem it = fa_item(0, p); ok && it.n_tiles > 0; it = fa_item(it.local + 1, p)) {
+    const int n_tiles = it.n_tiles, t = it.q0 + r;  // query position within the batch
     float m_ref = -INFINITY;   // reference maximum, in log2 units
     float l_run = 0.f;         // row sum, scaled to m_ref
-    bool ok = !*abort_flag;
-
-    for (int j = 0; j < n_tiles && ok; ++j) {
-      // P·V of tile j-2 has finished: its P buffer is free for this tile
-      if (j >= 2) {
-        if (!tc05::mbar_wait(&sh->o_full[j & 1], (uint32_t)((j - 2) >> 1) & 1u, abort_flag)) { ok = false; break; }
-      }
-      if (!tc05::mbar_wait(&sh->s_full[j & 1], (uint32_t)(j >> 1) & 1u, abort_flag)) { ok = false; break; }
+    for (int j = 0; j < n_tiles && ok; ++j, ++g) {
+      if (!tc05::mbar_wait(&sh->s_full[g & 1], (uint32_t)(g >> 1) & 1u, abort_flag)) { ok = false; break; }
       tc05::tc_fence_after_sync();
       const bool diag = (j >= n_tiles - 2);  // the two tiles that hold keys q0 .. q0+127
       const int key0 = j * FA_BN;
       uint32_t sb[FA_BN];
-      tc05::tmem_ld_32x32b_x32(tmem_s0 + (uint32_t)((j & 1) * FA_BN) + lane_sel, *reinterpret_cast<uint32_t(*)[32]>(&sb[0]));
-      tc05::tmem_ld_32x32b_x32(tmem_s0 + (uint32_t)((j & 1) * FA_BN) + lane_sel + 32, *reinterpret_cast<uint32_t(*)[32]>(&sb[32]));
+      tc05::tmem_ld_32x32b_x32(tmem_s0 + (uint32_t)((g & 1) * FA_BN) + lane_sel, *reinterpret_cast<uint32_t(*)[32]>(&sb[0]));
+      tc05::tmem_ld_32x32b_x32(tmem_s0 + (uint32_t)((g & 1) * FA_BN) + lane_sel + 32, *reinterpret_cast<uint32_t(*)[32]>(&sb[32]));
       tc05::tmem_ld_wait();
       // maximum of the raw scores (the scale is positive); masked entries become -inf
       float m_tile = -INFINITY;
@@ -244,7 +289,7 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       } else if (__any_sync(0xffffffffu, raise)) {
         // rows of this warp rescale their O in place; P·V of tile j-1 must have landed, and P·V of tile j is not
         // issued before this warp has handed over P(j)
-        if (!tc05::mbar_wait(&sh->o_full[(j - 1) & 1], (uint32_t)((j - 1) >> 1) & 1u, abort_flag)) { ok = false; break; }
+        if (!tc05::mbar_wait(&sh->o_full[(g - 1) % Z::P_BUFS], (uint32_t)((g - 1) / Z::P_BUFS) & 1u, abort_flag)) { ok = false; break; }
         tc05::tc_fence_after_sync();
         const float a = raise ? ex2_fast(m_ref - m_new) : 1.0f;
         if (raise) m_ref = m_new;
@@ -261,17 +306,20 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         tc05::tmem_st_wait();
       }
       const float neg_m = -m_ref;
-      uint8_t* line = sp + (j & 1) * FA_P_BYTES + r * 128;
+      // the P·V that read this P buffer has finished
+      if (g >= Z::P_BUFS && !tc05::mbar_wait(&sh->o_full[g % Z::P_BUFS], (uint32_t)((g - Z::P_BUFS) / Z::P_BUFS) & 1u, abort_flag)) { ok = false; break; }
+      uint8_t* line = sp + (g % Z::P_BUFS) * FA_P_BYTES + r * 128;
       float l_tile = 0.f;
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
         uint32_t w[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float p0 = ex2_fast(fmaf(__uint_as_float(sb[q * 8 + 2 * e]), p.scale_log2, neg_m));
-          const float p1 = ex2_fast(fmaf(__uint_as_float(sb[q * 8 + 2 * e + 1]), p.scale_log2, neg_m));
-          l_tile += p0 + p1;
-          w[e] = pack_bf16x2(p0, p1);
+          const float2 x = fma2(make_float2(__uint_as_float(sb[q * 8 + 2 * e]), __uint_as_float(sb[q * 8 + 2 * e + 1])),
+                                both(p.scale_log2), both(neg_m));
+          const float2 pr = make_float2(ex2_fast(x.x), ex2_fast(x.y));
+          l_tile += pr.x + pr.y;
+          w[e] = pack_bf16x2(pr.x, pr.y);
         }
         *reinterpret_cast<uint4*>(line + ((q ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
       }
@@ -279,12 +327,19 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       tc05::fence_proxy_async_smem();
       tc05::tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) tc05::mbar_arrive(&sh->p_full[j & 1]);
+      if (lane == 0) {
+        tc05::mbar_arrive(&sh->p_full[g % Z::P_BUFS]);
+        if (stored) {  // the last item's rows have left its Q buffer
+          tc05::tma_store_wait_read();
+          tc05::mbar_arrive(&sh->q_empty[(it.local - 1) % Z::Q_BUFS]);
+        }
+      }
+      if (Z::Q_BUFS == 2) stored = false;
     }
-    if (ok) {  // the last P·V has landed
-      ok = tc05::mbar_wait(&sh->o_full[(n_tiles - 1) & 1], (uint32_t)((n_tiles - 1) >> 1) & 1u, abort_flag);
-      tc05::tc_fence_after_sync();
-    }
+    if (!ok) break;
+    ok = tc05::mbar_wait(&sh->o_full[(g - 1) % Z::P_BUFS], (uint32_t)((g - 1) / Z::P_BUFS) & 1u, abort_flag);  // the last P·V
+    tc05::tc_fence_after_sync();
+    uint8_t* so = sq + (it.local % Z::Q_BUFS) * FA_Q_BYTES;
     if (ok) {
       // O leaves through the Q tile's shared memory (every product that read Q has finished): a warp stages its 32
       // rows per 64-channel block (128-byte rows, 128-byte swizzle) and its lane 0 sends them with one TMA store, whole
@@ -296,7 +351,7 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         uint32_t ob[32];
         tc05::tmem_ld_32x32b_x32(tmem_o0 + lane_sel + hb * 32, ob);
         tc05::tmem_ld_wait();
-        uint8_t* line = sq + (hb / 2) * Z::Q_BLOCK + r * 128;
+        uint8_t* line = so + (hb / 2) * Z::Q_BLOCK + r * 128;
 #pragma unroll
         for (int i = 0; i < 32; i += 8) {
           uint4 o;
@@ -313,15 +368,21 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       if (lane == 0) {
 #pragma unroll
         for (int blk = 0; blk < Z::BLOCKS; ++blk)
-          tc05::tma_store_3d(&map_o, sq + blk * Z::Q_BLOCK + warp * (32 * 128), h * FA_HD + blk * 64, q0 + warp * 32, b);
+          tc05::tma_store_3d(&map_o, so + blk * Z::Q_BLOCK + warp * (32 * 128), it.h * FA_HD + blk * 64, it.q0 + warp * 32, it.b);
         tc05::tma_store_commit();
-        tc05::tma_store_wait_all();
+        if (Z::Q_BUFS == 1) {  // the next item's Q waits for it
+          tc05::tma_store_wait_read();
+          tc05::mbar_arrive(&sh->q_empty[0]);
+        }
       }
+      stored = Z::Q_BUFS == 2;
     }
     if (ok && t < p.T) {
       // natural-log log-sum-exp of the scaled scores
-      p.lse[((size_t)b * p.H + h) * p.T + t] = (m_ref + log2f(l_run)) * 0.6931471805599453f;
+      p.lse[((size_t)it.b * p.H + it.h) * p.T + t] = (m_ref + log2f(l_run)) * 0.6931471805599453f;
     }
+    }
+    if (lane == 0) tc05::tma_store_wait_all();  // the results have landed before shared memory goes
   }
 
   tc05::tc_fence_before_sync();
@@ -372,7 +433,7 @@ int flash_attention_forward_impl(hl_ctx* ctx, const void* q, const void* k, cons
   p.lse = lse;
   p.scale_log2 = (1.0f / sqrtf((float)head_dim)) * 1.4426950408889634f;
   p.status = ctx->status_dev;
-  const int nq = ceil_div(time, FA_BM);
+  const int grid = std::min(ceil_div(time, FA_BM) * batch * n_heads, 2 * persistent_sms(ctx));
   // causal algorithmic work: QK^T and PV over the lower triangle
   ProfileScope prof(ctx, HL_PROF_ATTENTION_FWD, 2.0 * batch * n_heads * (double)time * time * head_dim);
   if (head_dim == 64) {
@@ -381,14 +442,14 @@ int flash_attention_forward_impl(hl_ctx* ctx, const void* q, const void* k, cons
       HL_CUDA(cudaFuncSetAttribute(flash_attention_fwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, FaSizes<64>::SMEM_BYTES));
       configured = true;
     }
-    pdl(flash_attention_fwd_kernel<64>, nq * batch * n_heads, FA_THREADS, FaSizes<64>::SMEM_BYTES, ctx->stream)(mq, mk, mv, mo, p);
+    pdl(flash_attention_fwd_kernel<64>, grid, FA_THREADS, FaSizes<64>::SMEM_BYTES, ctx->stream)(mq, mk, mv, mo, p);
   } else {
     static bool configured = false;
     if (!configured) {
       HL_CUDA(cudaFuncSetAttribute(flash_attention_fwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, FaSizes<128>::SMEM_BYTES));
       configured = true;
     }
-    pdl(flash_attention_fwd_kernel<128>, nq * batch * n_heads, FA_THREADS, FaSizes<128>::SMEM_BYTES, ctx->stream)(mq, mk, mv, mo, p);
+    pdl(flash_attention_fwd_kernel<128>, grid, FA_THREADS, FaSizes<128>::SMEM_BYTES, ctx->stream)(mq, mk, mv, mo, p);
   }
   HL_LAUNCH_CHECK("flash_attention_fwd_kernel");
   count_launch(ctx);

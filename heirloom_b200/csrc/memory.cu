@@ -45,24 +45,26 @@ __global__ void topk_rows_kernel(const float* __restrict__ scores, int64_t* __re
 // rounded multiply and add, j ascending (src/memory_transformer.rs:2029-2034) -------------------------
 // Block tile 64 tokens x 128 keys, thread tile 8 tokens x 4 keys; the contraction walks in slices of 64 that are
 // staged in shared memory (queries as [j][token], keys as [j][key]), so a step of the inner loop is three 16-byte
-// shared-memory loads for 32 multiplies and 32 adds.  Every accumulator still sees j = 0, 1, 2, ... in order.
+// shared-memory loads for 32 multiplies and 32 adds, two an instruction.  Every accumulator still sees j = 0, 1, 2, ... in
+// order.  Bound by the multiplies and adds, which may not be fused: 118 us for 16384 x 512 x 256.
 constexpr int SS_T = 64;   // tokens per block
 constexpr int SS_K = 128;  // keys per block
 constexpr int SS_J = 64;   // contraction slice
 __global__ void __launch_bounds__(256)
 side_scores_kernel(const float* __restrict__ query, long long ld_q, int q_off, const float* __restrict__ keys,
-                   float* __restrict__ out, int tokens, int side, int half_dim) {
+                   float* __restrict__ out, int tokens, int side, int half_dim, float minus_zero) {
   pdl_begin();
+  // A product is formed as q*k + (-0), which rounds like q*k alone.  The compiler fuses a packed multiply and add; it cannot
+  // know this addend.
+  const float2 zero = both(minus_zero);
   __shared__ __align__(16) float sq[SS_J][SS_T];
   __shared__ __align__(16) float sk[SS_J][SS_K];
   const int t0 = blockIdx.y * SS_T, k0 = blockIdx.x * SS_K;
   const int ty = threadIdx.x >> 5;  // 8 token groups of 8 tokens
   const int tx = threadIdx.x & 31;  // 32 key groups of 4 keys
-  float acc[8][4];
+  float2 acc[8][2];
 #pragma unroll
-  for (int a = 0; a < 8; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
+  for (int a = 0; a < 8; ++a) acc[a][0] = acc[a][1] = both(0.f);
   // 16-byte loads need four-element granularity everywhere an address is formed
   const bool vec = (half_dim % 4) == 0 && (ld_q % 4) == 0 && (q_off % 4) == 0 &&
                    ((reinterpret_cast<uintptr_t>(query) | reinterpret_cast<uintptr_t>(keys)) & 15) == 0;
@@ -101,11 +103,11 @@ side_scores_kernel(const float* __restrict__ query, long long ld_q, int q_off, c
       const float4 qb = *reinterpret_cast<const float4*>(&sq[j][ty * 8 + 4]);
       const float4 kv = *reinterpret_cast<const float4*>(&sk[j][tx * 4]);
       const float qv[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-      const float kk4[4] = {kv.x, kv.y, kv.z, kv.w};
 #pragma unroll
-      for (int a = 0; a < 8; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = __fadd_rn(acc[a][b], __fmul_rn(qv[a], kk4[b]));
+      for (int a = 0; a < 8; ++a) {
+        acc[a][0] = add2(acc[a][0], fma2(both(qv[a]), make_float2(kv.x, kv.y), zero));
+        acc[a][1] = add2(acc[a][1], fma2(both(qv[a]), make_float2(kv.z, kv.w), zero));
+      }
     }
     __syncthreads();
   }
@@ -116,7 +118,7 @@ side_scores_kernel(const float* __restrict__ query, long long ld_q, int q_off, c
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       const int kk = k0 + tx * 4 + b;
-      if (kk < side) out[(size_t)t * side + kk] = acc[a][b];
+      if (kk < side) out[(size_t)t * side + kk] = (b & 1) ? acc[a][b >> 1].y : acc[a][b >> 1].x;
     }
   }
 }
@@ -484,7 +486,8 @@ __global__ void selected_scores_bwd_kernel(const int64_t* __restrict__ idx, cons
 // dK = Wᵀ·Q with W[t, row] = sum of the g[t,k] whose slot maps to `row`: a CTA owns a block of tokens, 256 rows
 // and 64 columns of one table; per slice of 32 tokens it builds W in shared memory (one warp per token, its
 // duplicates added in slot order), multiplies with an 8 x 8 register tile per thread (two CTAs per SM), and clears the entries it
-// set.  The CTA's tile goes out as a partial result that fold_key_partials_kernel adds up in block order, so the
+// set.  The slots and queries of the next slice are fetched during the product (read where they were needed, the building took
+// two thirds of the time: 16384 tokens, 32 of 2 x 512 rows of 256: 386 us).  The CTA's tile goes out as a partial result that fold_key_partials_kernel adds up in block order, so the
 // result does not depend on scheduling.
 constexpr int DK_COLS = 64;    // columns per CTA
 constexpr int DK_ROWS = 256;   // table rows per CTA
@@ -503,50 +506,73 @@ product_key_dkeys_kernel(const int64_t* __restrict__ idx, const float* __restric
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tr = threadIdx.x >> 3;  // 32 row groups of 8 rows
   const int tc = threadIdx.x & 7;   // 8 column groups of 8 columns
-  float acc[8][8];
+  float2 acc[8][4];
 #pragma unroll
   for (int a = 0; a < 8; ++a)
 #pragma unroll
-    for (int b = 0; b < 8; ++b) acc[a][b] = 0.f;
+    for (int b = 0; b < 4; ++b) acc[a][b] = both(0.f);
   for (int i = threadIdx.x; i < DK_TOKENS * DK_ROWS; i += 256) w_tile[i] = 0.f;
   const int t_begin = blockIdx.x * tokens_per_block, t_end = min(tokens, t_begin + tokens_per_block);
+  // What a slice is built from travels while the slice before it is multiplied: eight query values a thread, and of each of
+  // its warp's four tokens one selected slot a lane (more than 32 slots: the rest is read when it is needed).
+  constexpr int TW = DK_TOKENS / 8, QV = DK_TOKENS * DK_COLS / 256;
+  float next_q[QV], next_g[TW];
+  int next_row[TW];
+  const unsigned side32 = (unsigned)side;
+  auto row_of = [&](long long slot) -> int {  // within this CTA's rows, -1 outside
+    if (slot < 0 || slot >= slots) return -1;
+    const unsigned s32 = (unsigned)slot;
+    const int row = (int)(table ? s32 % side32 : s32 / side32) - r0;
+    return row < 0 || row >= DK_ROWS ? -1 : row;
+  };
+  auto fetch = [&](int t0) {
+#pragma unroll
+    for (int i = 0; i < QV; ++i) {
+      const int t = (i * 256 + (int)threadIdx.x) / DK_COLS, c = (int)threadIdx.x % DK_COLS;
+      next_q[i] = (t0 + t < t_end && c0 + c < half) ? query[(size_t)(t0 + t) * ld_q + (table ? half : 0) + c0 + c] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < TW; ++i) {
+      const int t = t0 + warp + i * 8;
+      const bool in = t < t_end && lane < top_k;
+      next_row[i] = row_of(in ? idx[(size_t)t * top_k + lane] : -1);
+      next_g[i] = in ? grad_scores[(size_t)t * top_k + lane] : 0.f;
+    }
+  };
+  // Lanes whose slots share a table row add their gradients one after the other in slot order (round r = the lane's rank among
+  // its duplicates), so a row's sum is formed in the same order on every run.
+  auto add_row = [&](int t, int row, float g) {
+    const unsigned same = __match_any_sync(0xffffffffu, row);
+    const int rank = row < 0 ? -1 : __popc(same & ((1u << lane) - 1u));
+    const int rounds = __reduce_max_sync(0xffffffffu, rank) + 1;
+    for (int r = 0; r < rounds; ++r) {
+      if (rank == r) w_tile[t * DK_ROWS + row] += g;
+      __syncwarp();
+    }
+  };
+  fetch(t_begin);
   for (int t0 = t_begin; t0 < t_end; t0 += DK_TOKENS) {
-    __syncthreads();  // the previous slice's product is done (and, first time, the tile is zero)
-    // this slice's query columns
-    for (int i = threadIdx.x; i < DK_TOKENS * DK_COLS; i += 256) {
-      const int t = i / DK_COLS, c = i % DK_COLS;
-      q_tile[i] = (t0 + t < t_end && c0 + c < half) ? query[(size_t)(t0 + t) * ld_q + (table ? half : 0) + c0 + c] : 0.f;
+    __syncthreads();  // the previous slice's product is done and its entries are cleared (first time: the tile is zero)
+    int rows_set[TW];
+#pragma unroll
+    for (int i = 0; i < QV; ++i) q_tile[i * 256 + threadIdx.x] = next_q[i];
+#pragma unroll
+    for (int i = 0; i < TW; ++i) {
+      rows_set[i] = next_row[i];
+      add_row(warp + i * 8, next_row[i], next_g[i]);
     }
-    // W rows: warp w builds tokens w, w+8, ...  Each lane takes one selected slot; lanes whose slots share a table
-    // row add their gradients one after the other in slot order (round r = the lane's rank among its duplicates),
-    // so a row's sum is formed in the same order on every run.
-    for (int t = warp; t < DK_TOKENS; t += 8) {
-      if (t0 + t >= t_end) break;
-      for (int k0 = 0; k0 < top_k; k0 += 32) {
-        int row = -1;
-        float g = 0.f;
-        if (k0 + lane < top_k) {
-          const long long slot = idx[(size_t)(t0 + t) * top_k + k0 + lane];
-          if (slot >= 0 && slot < slots) {
-            const unsigned s32 = (unsigned)slot, side32 = (unsigned)side;
-            row = (int)(table ? s32 % side32 : s32 / side32) - r0;
-            g = grad_scores[(size_t)(t0 + t) * top_k + k0 + lane];
-            if (row < 0 || row >= DK_ROWS) row = -1;
-          }
+    if (top_k > 32)
+      for (int t = warp; t < DK_TOKENS && t0 + t < t_end; t += 8)
+        for (int k = 32 + lane; k - lane < top_k; k += 32) {
+          const bool in = k < top_k;
+          add_row(t, row_of(in ? idx[(size_t)(t0 + t) * top_k + k] : -1), in ? grad_scores[(size_t)(t0 + t) * top_k + k] : 0.f);
         }
-        const unsigned same = __match_any_sync(0xffffffffu, row);
-        const int rank = row < 0 ? -1 : __popc(same & ((1u << lane) - 1u));
-        const int rounds = __reduce_max_sync(0xffffffffu, rank) + 1;
-        for (int r = 0; r < rounds; ++r) {
-          if (rank == r) w_tile[t * DK_ROWS + row] += g;
-          __syncwarp();
-        }
-      }
-    }
+    if (t0 + DK_TOKENS < t_end) fetch(t0 + DK_TOKENS);
     __syncthreads();
     const int tn = min(DK_TOKENS, t_end - t0);
     for (int t = 0; t < tn; ++t) {
-      float wv[8], qv[8];
+      float wv[8];
+      float2 qv[4];
 #pragma unroll
       for (int a = 0; a < 8; a += 4) {
         const float4 x = *reinterpret_cast<const float4*>(&w_tile[t * DK_ROWS + tr * 8 + a]);
@@ -555,25 +581,25 @@ product_key_dkeys_kernel(const int64_t* __restrict__ idx, const float* __restric
 #pragma unroll
       for (int b = 0; b < 8; b += 4) {
         const float4 x = *reinterpret_cast<const float4*>(&q_tile[t * DK_COLS + tc * 8 + b]);
-        qv[b] = x.x; qv[b + 1] = x.y; qv[b + 2] = x.z; qv[b + 3] = x.w;
+        qv[b / 2] = make_float2(x.x, x.y);
+        qv[b / 2 + 1] = make_float2(x.z, x.w);
       }
 #pragma unroll
       for (int a = 0; a < 8; ++a)
 #pragma unroll
-        for (int b = 0; b < 8; ++b) acc[a][b] = fmaf(wv[a], qv[b], acc[a][b]);
+        for (int b = 0; b < 4; ++b) acc[a][b] = fma2(both(wv[a]), qv[b], acc[a][b]);
     }
     __syncthreads();
     // clear what this slice set
-    for (int t = warp; t < DK_TOKENS; t += 8) {
-      if (t0 + t >= t_end) break;
-      for (int k = lane; k < top_k; k += 32) {
-        const long long slot = idx[(size_t)(t0 + t) * top_k + k];
-        if (slot < 0 || slot >= slots) continue;
-        const unsigned s32 = (unsigned)slot, side32 = (unsigned)side;
-        const int row = (int)(table ? s32 % side32 : s32 / side32) - r0;
-        if (row >= 0 && row < DK_ROWS) w_tile[t * DK_ROWS + row] = 0.f;
-      }
-    }
+#pragma unroll
+    for (int i = 0; i < TW; ++i)
+      if (rows_set[i] >= 0) w_tile[(warp + i * 8) * DK_ROWS + rows_set[i]] = 0.f;
+    if (top_k > 32)
+      for (int t = warp; t < DK_TOKENS && t0 + t < t_end; t += 8)
+        for (int k = 32 + lane; k < top_k; k += 32) {
+          const int row = row_of(idx[(size_t)(t0 + t) * top_k + k]);
+          if (row >= 0) w_tile[t * DK_ROWS + row] = 0.f;
+        }
   }
   // partial[block][table][side][half]
   float* dst = partial + ((size_t)blockIdx.x * 2 + table) * side * half;
@@ -584,7 +610,7 @@ product_key_dkeys_kernel(const int64_t* __restrict__ idx, const float* __restric
 #pragma unroll
     for (int b = 0; b < 8; ++b) {
       const int c = c0 + tc * 8 + b;
-      if (c < half) dst[(size_t)row * half + c] = acc[a][b];
+      if (c < half) dst[(size_t)row * half + c] = (b & 1) ? acc[a][b / 2].y : acc[a][b / 2].x;
     }
   }
 }
@@ -1088,9 +1114,9 @@ int hl_product_key_side_scores_f32(hl_ctx* ctx, const float* query, long long ld
   HL_REQUIRE(ld_query >= key_dim, "hl_product_key_side_scores_f32: query row stride smaller than key_dim");
   const int half = key_dim / 2;
   dim3 grid(ceil_div(side, SS_K), ceil_div(tokens, SS_T));
-  pdl(side_scores_kernel, grid, 256, 0, ctx->stream)(query, ld_query, 0, left_keys, left_scores, tokens, side, half);
+  pdl(side_scores_kernel, grid, 256, 0, ctx->stream)(query, ld_query, 0, left_keys, left_scores, tokens, side, half, -0.0f);
   HL_LAUNCH_CHECK("side_scores_kernel");
-  pdl(side_scores_kernel, grid, 256, 0, ctx->stream)(query, ld_query, half, right_keys, right_scores, tokens, side, half);
+  pdl(side_scores_kernel, grid, 256, 0, ctx->stream)(query, ld_query, half, right_keys, right_scores, tokens, side, half, -0.0f);
   HL_LAUNCH_CHECK("side_scores_kernel");
   count_launch(ctx, 2);
   return HL_OK;
