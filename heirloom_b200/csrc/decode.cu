@@ -227,7 +227,7 @@ constexpr int DA_SLOTS = DA_THREADS / 8;  // keys at a time
 template <typename T, typename Acc>
 __global__ void __launch_bounds__(DA_THREADS)
 decode_attention_kernel(const T* __restrict__ qkv, long long ld, int channels, const long long* __restrict__ pos,
-                        T* __restrict__ out, int hd, int chunk_cap, bool staged) {
+                        T* __restrict__ out, int hd, int chunk_cap, bool staged, bool settled) {
   extern __shared__ double da_smem[];
   T* kept = reinterpret_cast<T*>(da_smem);   // staged: [2][chunk_cap][hd] keys, then values
   Acc* q = reinterpret_cast<Acc*>(kept + (staged ? (size_t)2 * chunk_cap * hd : 0));  // [hd]
@@ -242,7 +242,7 @@ decode_attention_kernel(const T* __restrict__ qkv, long long ld, int channels, c
   const int sub = threadIdx.x & 7, slot = threadIdx.x >> 3;
   constexpr int PN = Pack<T>::N;
   const bool vec = hd % PN == 0 && channels % PN == 0 && ld % PN == 0;
-  // The position was copied here before the step's first kernel started, the rows below it before the step.
+  // The position was copied here before the first kernel of the sequence started.
   const long long t = *pos;
   const int keys = (int)t + 1, chunk = (keys + DA_CTAS - 1) / DA_CTAS;
   const int k0 = min(keys, rank * chunk), k1 = min(keys, k0 + chunk);
@@ -252,6 +252,7 @@ decode_attention_kernel(const T* __restrict__ qkv, long long ld, int channels, c
     for (int kv = 0; kv < 2; ++kv)
       cp_async16(kept + ((size_t)kv * chunk_cap + (key - k0)) * hd + u * PN, base + (1 + kv) * channels + (long long)key * ld + u * PN);
   };
+  if (!settled) pdl_wait();  // the rows below the position come from the predecessor as well
   if (staged)
     for (int key = k0 + slot; key < min(k1, (int)t); key += DA_SLOTS)
       for (int u = sub; u < units; u += 8) stage(key, u);
@@ -483,7 +484,8 @@ size_t decode_attention_smem(int dtype, int hd, int context) {
 }
 
 template <typename T, typename Acc>
-int launch_decode_attention(hl_ctx* ctx, const T* qkv, long long ld, const long long* pos, T* out, int channels, int n_heads, int context) {
+int launch_decode_attention(hl_ctx* ctx, const T* qkv, long long ld, const long long* pos, T* out, int channels, int n_heads, int context,
+                            bool settled) {
   const int hd = channels / n_heads, cap = ceil_div(context, DA_CTAS);
   size_t smem = decode_attention_smem(sizeof(T) == 2 ? HL_BF16 : HL_F32, hd, context);
   const size_t rows = sizeof(T) * 2 * (size_t)cap * hd;
@@ -497,16 +499,17 @@ int launch_decode_attention(hl_ctx* ctx, const T* qkv, long long ld, const long 
     HL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024));
     configured = true;
   }
-  HL_CUDA(launch_pdl(kern, n_heads * DA_CTAS, DA_THREADS, smem, ctx->stream, DA_CTAS, qkv, ld, channels, pos, out, hd, cap, staged));
+  HL_CUDA(launch_pdl(kern, n_heads * DA_CTAS, DA_THREADS, smem, ctx->stream, DA_CTAS, qkv, ld, channels, pos, out, hd, cap, staged,
+                     settled));
   count_launch(ctx);
   return HL_OK;
 }
 
 int decode_attention(hl_ctx* ctx, const void* qkv, int dtype, long long ld, const long long* pos, void* out, int channels,
-                     int n_heads, int context) {
+                     int n_heads, int context, bool settled) {
   return dtype == HL_BF16 ? launch_decode_attention<__nv_bfloat16, float>(ctx, (const __nv_bfloat16*)qkv, ld, pos, (__nv_bfloat16*)out,
-                                                                          channels, n_heads, context)
-                          : launch_decode_attention<float, double>(ctx, (const float*)qkv, ld, pos, (float*)out, channels, n_heads, context);
+                                                                          channels, n_heads, context, settled)
+                          : launch_decode_attention<float, double>(ctx, (const float*)qkv, ld, pos, (float*)out, channels, n_heads, context, settled);
 }
 
 int decode_greedy(hl_ctx* ctx, const float* logits, int vocab, GreedyPart* parts, GreedyPart* out) {

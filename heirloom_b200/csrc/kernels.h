@@ -146,8 +146,9 @@ struct DecodeGemv {
 };
 int decode_gemv(hl_ctx* ctx, const DecodeGemv& g);
 size_t decode_attention_smem(int dtype, int head_dim, int context);
+// `settled`: the rows below the position were written before this sequence of launches began.
 int decode_attention(hl_ctx* ctx, const void* qkv, int dtype, long long ld, const long long* pos, void* out, int channels,
-                     int n_heads, int context);
+                     int n_heads, int context, bool settled);
 // The last maximum of a row of logits and the sum of exponentials below it, without taking the row to the host.  `parts` has
 // room for greedy_parts(vocab) entries.
 struct GreedyPart {

@@ -628,6 +628,52 @@ int decode_head(hl_decoder* m, const void* x, int dtype) {
   return decode_gemv(m->ctx, g);
 }
 
+// A matrix-vector product of one row, in the model's precision, behind a layer norm when one is given.
+DecodeGemv row_gemv(const hl_decoder* m, const void* x, size_t w, size_t b, void* out, int n, int k, int epilogue, const void* residual,
+                    size_t ln_g, size_t ln_b) {
+  const bool amp = m->cfg.precision == HL_PRECISION_AMP_BF16;
+  DecodeGemv g{};
+  g.x = x; g.x_dtype = amp ? HL_BF16 : HL_F32;
+  g.w = amp ? (const void*)(m->shadow + w) : (const void*)(m->params + w);
+  g.w_dtype = g.x_dtype;
+  g.bias = m->params + b;
+  g.out = out; g.out_dtype = g.x_dtype;
+  g.n = n; g.k = k; g.epilogue = epilogue; g.residual = residual;
+  if (ln_g) { g.gamma = m->params + ln_g; g.beta = m->params + ln_b; }
+  return g;
+}
+
+// Attention and feed-forward of block l for the row whose position stands in m->decode_state, `x` being its input row; the
+// result goes to row 0 of the block's output.  The block's q/k/v rows are there, `settled`: but for this row, since before
+// the sequence of launches began.
+int row_block(hl_decoder* m, int l, const void* x, bool settled) {
+  hl_ctx* ctx = m->ctx;
+  const hl_decoder_config& c = m->cfg;
+  const LayerOffsets& o = m->lo[l];
+  const int d = c.d_model, F = c.d_ff;
+  const bool amp = c.precision == HL_PRECISION_AMP_BF16;
+  void *next, *qkv, *att, *r, *g;
+  if (amp) { next = m->x[l + 1]; qkv = m->la[l].qkv; att = m->la[l].o; r = m->la[l].r; g = m->la[l].g; }
+  else { next = m->xf[l + 1]; qkv = m->lf[l].qkv; att = m->lf[l].o; r = m->lf[l].r; g = m->lf[l].g; }
+  HL_TRY(decode_attention(ctx, qkv, amp ? HL_BF16 : HL_F32, 3 * d, m->decode_state, att, d, c.n_heads, c.context, settled));
+  HL_TRY(decode_gemv(ctx, row_gemv(m, att, o.wo, o.bo, r, d, d, GV_RESIDUAL, x, 0, 0)));
+  if (o.is_memory) return HL_OK;
+  HL_TRY(decode_gemv(ctx, row_gemv(m, r, o.w1, o.b1, g, F, d, GV_GELU, nullptr, o.ln2g, o.ln2b)));
+  return decode_gemv(ctx, row_gemv(m, g, o.w2, o.b2, next, d, F, GV_RESIDUAL, r, 0, 0));
+}
+
+bool decode_applicable(const hl_decoder* m) {
+  const hl_decoder_config& c = m->cfg;
+  const int dt = c.precision == HL_PRECISION_AMP_BF16 ? HL_BF16 : HL_F32;
+  return decode_attention_smem(dt, c.d_model / c.n_heads, c.context) <= 48 * 1024;
+}
+// The last block of a pass that wants its last position only: behind the q/k/v product nothing but that row is worked on (a
+// window of 500 of the GPT-sized model: 24 us less, 64 rows of four f32 blocks: 26).  Memory blocks keep all rows: their routing
+// is read by others.
+bool last_block_by_row(const hl_decoder* m, int l) {
+  return l == m->cfg.n_layers - 1 && !m->lo[l].is_memory && decode_applicable(m);
+}
+
 // What a forward pass is for: logits and activations for the backward pass, the logits of the last position alone (they go to
 // row 0 of m->logits), or the mean loss alone (to m->loss_dev).
 enum class Forward { all, last_position, loss };
@@ -650,6 +696,11 @@ int forward(hl_decoder* m, Forward what = Forward::all) {
     LayerActs& a = m->la[l];
     HL_TRY(layer_norm_forward_impl(ctx, m->x[l], HL_BF16, P + o.ln1g, P + o.ln1b, a.a, HL_BF16, a.mean1, a.rstd1, N, d, 1e-5f));
     HL_TRY(g.run(N, 3 * d, d, a.a, d, HL_K_MAJOR, W + o.wqkv, d, HL_K_MAJOR, a.qkv, 3 * d, HL_BF16, HL_EPI_BIAS, P + o.bqkv));
+    if (what == Forward::last_position && last_block_by_row(m, l)) {
+      HL_TRY(row_block(m, l, m->x[l] + (size_t)(N - 1) * d, false));
+      m->cached = 0;
+      return decode_head(m, m->x[l + 1], HL_BF16);
+    }
     if (m->flash_ok) HL_TRY(flash_attention_forward_impl(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, 3 * d, a.o, d, a.lse, B, T, H, d / H));
     else HL_TRY(attention_f64_forward(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, HL_BF16, 3 * d, a.o, d, m->fa_probs, B, T, d, H));
     HL_TRY(g.run(N, d, d, a.o, d, HL_K_MAJOR, W + o.wo, d, HL_K_MAJOR, a.r, d, HL_BF16, HL_EPI_BIAS_RESIDUAL, P + o.bo,
@@ -1052,6 +1103,11 @@ int forward_f32(hl_decoder* m, bool last_only = false) {
     hl_decoder::F32Layer& a = m->lf[l];
     HL_TRY(layer_norm_forward_impl(ctx, m->xf[l], HL_F32, P + o.ln1g, P + o.ln1b, a.a, HL_F32, nullptr, nullptr, N, d, 1e-5f));
     HL_TRY(forward_f32_gemm(m, linear_f32(a.a, P + o.wqkv, P + o.bqkv, a.qkv, N, d, 3 * d)));
+    if (last_only && last_block_by_row(m, l)) {
+      HL_TRY(row_block(m, l, m->xf[l] + (size_t)(N - 1) * d, false));
+      m->cached = 0;
+      return decode_head(m, m->xf[l + 1], HL_F32);
+    }
     HL_TRY(attention_f64_forward(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, HL_F32, 3 * d, a.o, d, a.probs, B, T, d, H));
     HL_TRY(forward_f32_gemm(m, linear_f32(a.o, P + o.wo, P + o.bo, a.r, N, d, d, F64_RESIDUAL, m->xf[l])));
     HL_TRY(layer_norm_forward_impl(ctx, a.r, HL_F32, P + o.ln2g, P + o.ln2b, a.c, HL_F32, nullptr, nullptr, N, d, 1e-5f));
@@ -1224,35 +1280,24 @@ int run_graphed(hl_decoder* m, int kind, F queue) {
 int decode_step(hl_decoder* m) {
   hl_ctx* ctx = m->ctx;
   const hl_decoder_config& c = m->cfg;
-  const int d = c.d_model, F = c.d_ff;
+  const int d = c.d_model;
   const bool amp = c.precision == HL_PRECISION_AMP_BF16;
   const int dt = amp ? HL_BF16 : HL_F32;
   const float* P = m->params;
-  auto weight = [&](size_t off) -> const void* { return amp ? (const void*)(m->shadow + off) : (const void*)(P + off); };
   auto gemv = [&](const void* x, size_t w, size_t b, void* out, int n, int k, int epilogue = GV_STORE, const void* residual = nullptr,
-                  size_t ln_g = 0, size_t ln_b = 0) {
-    DecodeGemv g{};
-    g.x = x; g.x_dtype = dt;
-    g.w = weight(w); g.w_dtype = dt;
-    g.bias = P + b;
-    g.out = out; g.out_dtype = dt;
-    g.n = n; g.k = k; g.epilogue = epilogue; g.residual = residual;
-    if (ln_g) { g.gamma = P + ln_g; g.beta = P + ln_b; }
-    return g;
-  };
+                  size_t ln_g = 0, size_t ln_b = 0) { return row_gemv(m, x, w, b, out, n, k, epilogue, residual, ln_g, ln_b); };
   HL_TRY(decode_embed(ctx, P + m->off_tok, P + m->off_pos, m->decode_state, amp ? (void*)m->x[0] : (void*)m->xf[0], dt, d));
   for (int l = 0; l < c.n_layers; ++l) {
     const LayerOffsets& o = m->lo[l];
-    void *x, *next, *qkv, *att, *r, *g;
-    if (amp) { x = m->x[l]; next = m->x[l + 1]; qkv = m->la[l].qkv; att = m->la[l].o; r = m->la[l].r; g = m->la[l].g; }
-    else { x = m->xf[l]; next = m->xf[l + 1]; qkv = m->lf[l].qkv; att = m->lf[l].o; r = m->lf[l].r; g = m->lf[l].g; }
+    void *x, *next, *qkv, *r;
+    if (amp) { x = m->x[l]; next = m->x[l + 1]; qkv = m->la[l].qkv; r = m->la[l].r; }
+    else { x = m->xf[l]; next = m->xf[l + 1]; qkv = m->lf[l].qkv; r = m->lf[l].r; }
     // the attention output, r and g rows may lie over cached positions' rows: only the q/k/v rows are kept
     DecodeGemv q = gemv(x, o.wqkv, o.bqkv, qkv, 3 * d, d, GV_STORE, nullptr, o.ln1g, o.ln1b);
     q.out_row = m->decode_state;
     q.ld_out = 3 * d;
     HL_TRY(decode_gemv(ctx, q));
-    HL_TRY(decode_attention(ctx, qkv, dt, 3 * d, m->decode_state, att, d, c.n_heads, c.context));
-    HL_TRY(decode_gemv(ctx, gemv(att, o.wo, o.bo, r, d, d, GV_RESIDUAL, x)));
+    HL_TRY(row_block(m, l, x, true));
     if (o.is_memory) {
       MemoryActs& ma = m->ma[l];
       const int kd = m->mem.key_dim, vd = m->mem.value_dim;
@@ -1268,18 +1313,9 @@ int decode_step(hl_decoder* m) {
       HL_TRY(project(r, dt, o.wg_m, o.bg_m, ma.gate, HL_F32, vd, d, GV_GELU, nullptr, true));
       HL_TRY(hl_binary_f32(ctx, HL_MUL, ma.weighted, ma.gate, ma.mv, (size_t)vd));
       HL_TRY(project(ma.mv, HL_F32, o.wout_m, o.bout_m, next, dt, d, vd, GV_RESIDUAL, r, false));
-    } else {
-      HL_TRY(decode_gemv(ctx, gemv(r, o.w1, o.b1, g, F, d, GV_GELU, nullptr, o.ln2g, o.ln2b)));
-      HL_TRY(decode_gemv(ctx, gemv(g, o.w2, o.b2, next, d, F, GV_RESIDUAL, r)));
     }
   }
   return decode_head(m, amp ? (const void*)m->x[c.n_layers] : (const void*)m->xf[c.n_layers], dt);
-}
-
-bool decode_applicable(const hl_decoder* m) {
-  const hl_decoder_config& c = m->cfg;
-  const int dt = c.precision == HL_PRECISION_AMP_BF16 ? HL_BF16 : HL_F32;
-  return decode_attention_smem(dt, c.d_model / c.n_heads, c.context) <= 48 * 1024;
 }
 
 int ensure_logits_host(hl_decoder* m) {
@@ -1967,7 +2003,11 @@ static int run_window(hl_decoder* m, const int64_t* window, cudaMemcpyKind kind,
   HL_CUDA(cudaMemcpyAsync(m->tokens, window, sizeof(int64_t) * window_len, kind, ctx->stream));
   {
     ScopedShape shape(m, 1, window_len);
-    HL_TRY(run_graphed(m, GRAPH_WINDOW, [m]() { return m->cfg.precision == HL_PRECISION_AMP_BF16 ? forward(m, Forward::last_position) : forward_f32(m, true); }));
+    m->decode_state_host[0] = window_len - 1;
+    HL_TRY(run_graphed(m, GRAPH_WINDOW, [m]() -> int {
+      HL_CUDA(cudaMemcpyAsync(m->decode_state, m->decode_state_host, sizeof(long long), cudaMemcpyHostToDevice, m->ctx->stream));
+      return m->cfg.precision == HL_PRECISION_AMP_BF16 ? forward(m, Forward::last_position) : forward_f32(m, true);
+    }));
     m->cached = 0;
   }
   HL_TRY(queue_result(m, greedy));
