@@ -71,6 +71,18 @@ void fold_batch_add(FoldBatch* batch, const float* partial, int blocks, int tota
                     float* o2);
 int fold_batch_flush(hl_ctx* ctx, FoldBatch* batch);
 
+// Weight gradients of several layers in one launch (gemm_group.cu): dw[n_out, n_in] = dyᵀ · x and, when db is given, its column
+// sums, dy and x bf16 with one row per token.  `sums`: device memory, gemm_group_sums() floats for every product with a db.
+struct WeightGradJob {
+  const __nv_bfloat16 *dy, *x;
+  int n_out, n_in;
+  float *dw, *db;
+};
+constexpr int kMaxGroupJobs = 70;
+int gemm_group_tiles(int n_out, int n_in);
+size_t gemm_group_sums(int n_out, int n_in);
+int gemm_group_run(hl_ctx* ctx, const WeightGradJob* jobs, int count, int tokens, float* sums, FoldBatch* fold);
+
 int bias_grad_impl(hl_ctx* ctx, const void* grad_out, int dtype, float* grad_bias, int rows, int cols,
                    FoldBatch* defer = nullptr);
 

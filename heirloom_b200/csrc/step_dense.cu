@@ -127,6 +127,10 @@ struct hl_decoder {
   bool fork_ok = false;
   cudaStream_t side_stream = nullptr;
   cudaEvent_t fork_event = nullptr, join_event = nullptr;
+  // ... or, where the products fill the chip, collected for `group_layers` layers (0: not) and run by one launch.
+  int group_layers = 0;
+  std::vector<WeightGradJob> wgrads;
+  float* group_sums = nullptr;
   bool forked = false;  // work has been queued on the side stream since the last join
   FoldBatch fold;  // column reductions of one block's backward, folded by one launch before its buckets are flushed
   float* loss_dev = nullptr;
@@ -382,6 +386,30 @@ void plan_memory_buffers(hl_decoder* m, uint8_t*& cur) {
 // thousand tokens needs.  Above it the products fill the chip and the copies would be gigabytes.
 constexpr size_t kForkBytes = size_t(256) << 20;
 
+// Weight gradients of how many layers one launch takes (0: each for itself).  As many as leave the fewest waves of tiles over the
+// whole backward pass (the head's product goes with the first group), the fewest layers among those: each has its own copy of
+// the gradients that the products read, which kGroupBytes bounds.
+constexpr size_t kGroupBytes = size_t(1) << 30;
+int plan_group_layers(const hl_decoder* m) {
+  const hl_decoder_config& c = m->cfg;
+  const int d = c.d_model, F = c.d_ff, L = c.n_layers, pairs = std::max(1, m->ctx->sm_count / 2);
+  if (d % 8 != 0 || F % 8 != 0 || c.vocab % 8 != 0) return 0;
+  const size_t per_layer = (size_t)m->N * (F + 5 * d) * 2;
+  const int most = (int)std::min<size_t>({(size_t)L, std::max<size_t>(1, kGroupBytes / per_layer), (size_t)(kMaxGroupJobs - 1) / 4});
+  const int attention = gemm_group_tiles(3 * d, d) + gemm_group_tiles(d, d), ffn = gemm_group_tiles(F, d) + gemm_group_tiles(d, F);
+  int best = 0, best_waves = 0;
+  for (int g = 1; g <= most; ++g) {
+    int waves = 0;
+    for (int top = L; top > 0; top -= g) {
+      int tiles = top == L ? gemm_group_tiles(c.vocab, d) : 0;
+      for (int l = std::max(0, top - g); l < top; ++l) tiles += attention + (m->lo[l].is_memory ? 0 : ffn);
+      waves += ceil_div(tiles, pairs);
+    }
+    if (best == 0 || waves < best_waves) { best = g; best_waves = waves; }
+  }
+  return best;
+}
+
 int plan_activations(hl_decoder* m, bool measure_only, size_t* bytes_out) {
   const hl_decoder_config& c = m->cfg;
   const size_t N = (size_t)m->N, d = c.d_model, F = c.d_ff, V = c.vocab, L = c.n_layers;
@@ -416,17 +444,25 @@ int plan_activations(hl_decoder* m, bool measure_only, size_t* bytes_out) {
   m->dob = carve<__nv_bfloat16>(cur, N * d);
   m->dxb0 = carve<__nv_bfloat16>(cur, N * d);  // gradient of the embeddings' sum: written like a block output's, read by nobody
   m->fork_ok = N * (F + 5 * d) * 2 * L <= kForkBytes;
-  for (size_t l = 0; l < L; ++l) {
-    LayerActs& a = m->la[l];
-    if (l > 0 && !m->fork_ok) {
-      a.dy = m->la[0].dy; a.dh = m->la[0].dh; a.dr = m->la[0].dr; a.dqkv = m->la[0].dqkv;
-      continue;
+  m->group_layers = m->fork_ok ? 0 : plan_group_layers(m);
+  {
+    // one set of gradients per layer, per layer of a group, or for all; a group's last layer writes the next one's dy already
+    const size_t sets = m->fork_ok ? L : std::max(1, m->group_layers), dy_sets = m->fork_ok ? L : std::min(L, sets + (m->group_layers > 0));
+    for (size_t i = 0; i < L; ++i) {  // the order of the backward pass
+      LayerActs& a = m->la[L - 1 - i];
+      a.dy = i < dy_sets ? carve<__nv_bfloat16>(cur, N * d) : m->la[L - 1 - i % dy_sets].dy;
+      if (i >= sets) {
+        const LayerActs& first = m->la[L - 1 - i % sets];
+        a.dh = first.dh; a.dr = first.dr; a.dqkv = first.dqkv;
+        continue;
+      }
+      a.dh = carve<__nv_bfloat16>(cur, N * F);
+      a.dr = carve<__nv_bfloat16>(cur, N * d);
+      a.dqkv = carve<__nv_bfloat16>(cur, N * 3 * d);
     }
-    a.dy = carve<__nv_bfloat16>(cur, N * d);
-    a.dh = carve<__nv_bfloat16>(cur, N * F);
-    a.dr = carve<__nv_bfloat16>(cur, N * d);
-    a.dqkv = carve<__nv_bfloat16>(cur, N * 3 * d);
   }
+  if (m->group_layers > 0)  // biases of the head, of fc1 and of qkv
+    m->group_sums = carve<float>(cur, gemm_group_sums(V, d) + m->group_layers * (gemm_group_sums(F, d) + gemm_group_sums(3 * d, d)));
   if (!m->flash_ok) {
     m->fa_probs = carve<float>(cur, (size_t)c.batch * c.n_heads * c.context * c.context);
   }
@@ -548,6 +584,14 @@ int join_side(hl_decoder* m) {
   return HL_OK;
 }
 
+// Collected weight gradients are not final when their layer is done, so not while buckets of them are being exchanged.
+bool grouping(const hl_decoder* m) { return m->group_layers > 0 && !nccl_active(m->ctx); }
+int run_weight_gradients(hl_decoder* m) {
+  const int rc = gemm_group_run(m->ctx, m->wgrads.data(), (int)m->wgrads.size(), m->N, m->group_sums, &m->fold);
+  m->wgrads.clear();
+  return rc;
+}
+
 // dw[n_out, n_in] = dyᵀ · x and, when asked for, db = column sums of dy (both bf16, one row per token)
 int weight_gradient(hl_decoder* m, const __nv_bfloat16* dy, int n_out, const __nv_bfloat16* x, int n_in, float* dw, float* db) {
   hl_gemm_desc d{};
@@ -555,6 +599,10 @@ int weight_gradient(hl_decoder* m, const __nv_bfloat16* dy, int n_out, const __n
   d.a_layout = HL_MN_MAJOR; d.b_layout = HL_MN_MAJOR;
   d.lda = n_out; d.ldb = n_in; d.ldc = n_in;
   d.epilogue = HL_EPI_NONE; d.out_dtype = HL_F32;
+  if (grouping(m)) {
+    m->wgrads.push_back(WeightGradJob{dy, x, n_out, n_in, dw, db});
+    return HL_OK;
+  }
   bool done = false;
   if (gemm_bf16_small_applies(m->ctx, &d)) {
     // no scratch arena on this path, so it may run on either stream
@@ -931,6 +979,7 @@ int backward(hl_decoder* m) {
   const __nv_bfloat16* W = m->shadow;
   float* G = m->grads;
   m->next_bucket = 0;
+  m->wgrads.clear();
   if (m->comm_pending) {  // a previous step's collectives were never consumed: finish them before its gradients are overwritten
     HL_CUDA(cudaStreamWaitEvent(m->ctx->stream, m->comm_done, 0));
     m->comm_pending = false;
@@ -1034,6 +1083,7 @@ int backward(hl_decoder* m) {
     HL_TRY(layer_norm_backward_impl(ctx, m->x[l], HL_BF16, P + o.ln1g, m->dtmp, a.mean1, a.rstd1, dx, dx_next, l > 0 ? m->la[l - 1].dy : m->dxb0,
                                     G + o.ln1g, G + o.ln1b, l > 0 ? G + m->lo[l - 1].out_bias() : nullptr, N, d, fb));
     std::swap(dx, dx_next);
+    if (grouping(m) && (l == 0 || (c.n_layers - l) % m->group_layers == 0)) HL_TRY(run_weight_gradients(m));
     HL_TRY(finished(o.ln1b + d));
   }
   // embeddings: scatter-add into zeroed tables

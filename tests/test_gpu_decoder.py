@@ -164,3 +164,33 @@ def test_amp_route_tracks_the_oracle_loss_trace_for_200_steps():
     print("amp 200-step trace: worst relative loss deviation", rel.max(), "at step", int(rel.argmax()))
     assert rel.max() <= 0.01, (rel.max(), int(rel.argmax()))
     assert losses[-1] < 4.6
+
+
+def test_collected_weight_gradients_equal_those_of_two_half_batches():
+    """18000 tokens: the weight gradients of several layers in one launch, ragged in every size (960/320/1000 by 320/1000 in tiles of
+    256 by 256, 282 token blocks of 64).  9000 tokens: each product for itself.  The loss is a mean, so that the two halves'
+    gradients are exactly twice as large in every bf16 rounding.  What differs is the order of f32 sums: 2^-24 relative per
+    addition, at random over 18000 of them 8e-6, times ten for what cancels in a sum; and, below the last block, bf16 values of
+    the residual stream's gradient that such a difference tips over (2^-8 of a value, for fewer than one in a hundred)."""
+    from heirloom_b200 import nn
+    c = ctx()
+    rng = np.random.default_rng(5)
+    x = torch.from_numpy(rng.integers(0, 1000, (18, 1000))).cuda()
+    y = torch.from_numpy(rng.integers(0, 1000, (18, 1000))).cuda()
+    state, grads = None, []
+    for part in (slice(0, 18), slice(0, 9), slice(9, 18)):
+        model = nn.DecoderLm(c, nn.DecoderConfig(vocab=1000, d_model=320, n_layers=3, n_heads=5, d_ff=1000, context=1000,
+                                                 batch=len(range(18)[part])))
+        if state is None:
+            state = {n: (np.ones(s) if ".ln" in n or n.startswith("ln_f") else rng.standard_normal(s) * 0.05)
+                     for n, s in model.parameter_shapes().items()}
+        model.load_state_dict(state)
+        model.forward_backward(x[part].contiguous(), y[part].contiguous())
+        grads.append({n: model.grad(n).astype(np.float64) for n in state})
+        model.close()
+    for name, whole in grads[0].items():
+        if name.endswith("k_proj.bias"):
+            continue  # the exact gradient is zero
+        halves = (grads[1][name] + grads[2][name]) / 2
+        tipped = 0 if name.startswith(("lm_head", "ln_f", "block.2")) else 2 ** -8 * 0.1 * (4 if "embedding" in name else 2)
+        assert np.linalg.norm(whole - halves) <= (2 ** -24 * np.sqrt(18000) * 10 + tipped) * np.linalg.norm(halves), name
