@@ -31,8 +31,15 @@ struct GsSizes {
   static constexpr int LD = BN + 4;                                 // accumulator rows in shared memory: conflict-free writes
   static_assert((GS_BM * LD + GS_BM) * 4 <= DATA, "the accumulator reuses the stages");
   static constexpr int ONES = 2048;                                 // 16 x 64 bf16 of 1.0: the right operand of the row sums
-  static constexpr int SMEM = DATA + 1024 + ONES + 256;
-  static constexpr int CTAS_PER_SM = SMEM <= 113 * 1024 ? 2 : 1;
+  static constexpr int TAIL = DATA + ONES;                          // barriers
+  // The residual or pre-activation rows of the tile: a place of their own where one CTA has the SM, else in the stages, behind the
+  // accumulator.
+  static constexpr int CTAS_PER_SM = DATA <= 104 * 1024 ? 2 : 1;
+  static constexpr int AUX = CTAS_PER_SM == 1 ? TAIL + 256 : ((GS_BM * LD + GS_BM) * 4 + 15) / 16 * 16;
+  static constexpr int AUX_BYTES = GS_BM * BN * 2;
+  static constexpr int SMEM = CTAS_PER_SM == 1 ? AUX + AUX_BYTES : TAIL + 256;  // base aligned to 1024 bytes, as the kernel checks
+  static_assert(CTAS_PER_SM == 1 || AUX + AUX_BYTES <= DATA, "the rows fit behind the accumulator");
+  static_assert(CTAS_PER_SM * (SMEM + 1024) <= 228 * 1024, "shared memory budget");
 };
 
 struct GsParams {
@@ -63,9 +70,8 @@ template <bool A_MN, bool B_MN, int BN, int STAGES>
 __global__ void __launch_bounds__(GS_THREADS, (GsSizes<BN, STAGES>::CTAS_PER_SM))
 gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GsParams p) {
   using Z = GsSizes<BN, STAGES>;
-  extern __shared__ uint8_t gs_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gs_raw) + 1023) & ~uintptr_t(1023));
-  GsTail* tail = reinterpret_cast<GsTail*>(smem + Z::DATA + Z::ONES);
+  extern __shared__ __align__(1024) uint8_t smem[];
+  GsTail* tail = reinterpret_cast<GsTail*>(smem + Z::TAIL);
   volatile int* abort_flag = &tail->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)blockIdx.x % p.splits, tile = (int)blockIdx.x / p.splits;
@@ -78,7 +84,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       tc05::mbar_init(&tail->empty[s], 1);
     }
     tc05::mbar_init(&tail->done, 1);
-    tail->abort_flag = 0;
+    tail->abort_flag = (tc05::smem_u32(smem) & 1023u) == 0 ? 0 : 1;
     tc05::fence_barrier_init();
     tc05::tma_prefetch_desc(&map_a);
     tc05::tma_prefetch_desc(&map_b);
@@ -100,8 +106,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   pdl_trigger();
   pdl_wait();
 
-  // This thread's four columns, and the rows it finishes of this CTA's share of the tile; the first residual or
-  // pre-activation rows are requested here, before the roles' loops.
+  // This thread's four columns, and the rows it finishes of this CTA's share of the tile.
   constexpr int QUADS = BN / 4, ROWS_PER_PASS = GS_THREADS / QUADS;
   const int rows_mine = GS_BM / p.splits, row_first = rank * rows_mine;
   const int quad = threadIdx.x % QUADS, sub = threadIdx.x / QUADS;
@@ -110,15 +115,17 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const bool need_aux = p.epilogue == HL_EPI_BIAS_RESIDUAL || p.epilogue == HL_EPI_DGELU;
   float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
   if (p.bias && col_ok) bias = __ldg(reinterpret_cast<const float4*>(p.bias + col));
-  // one pass ahead; a rolled loop, because a CTA that lands on an SM which has not run this kernel yet pays for every cache
-  // line of its code
-  auto fetch_aux = [&](int i) {
-    const int r = sub + i * ROWS_PER_PASS, row = m0 + row_first + r;
-    return need_aux && r < rows_mine && row < p.m && col_ok
-               ? *reinterpret_cast<const uint2*>(p.aux_in + (size_t)row * p.ld_aux_in + col)
-               : make_uint2(0u, 0u);
+  // All of them are requested at once, beside the contraction or right behind it: row by row in the loop below, a load's latency
+  // per eight rows, they took 8 of 23 us (4096 x 512 x 2048 with residual).
+  auto fetch_aux = [&]() {
+    for (int i = threadIdx.x; i < rows_mine * (BN / 8); i += GS_THREADS) {
+      const int r = i / (BN / 8), u = i % (BN / 8), row = m0 + row_first + r, c = n0 + u * 8;
+      if (row < p.m && c < p.n)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc05::smem_u32(smem + Z::AUX + i * 16)),
+                     "l"(p.aux_in + (size_t)row * p.ld_aux_in + c) : "memory");
+    }
   };
-  uint2 aux = fetch_aux(0);
+  if (need_aux && Z::CTAS_PER_SM == 1) fetch_aux();
 
   if (warp == 0) {
     if (tc05::elect_one()) {
@@ -177,6 +184,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   if (have) ok = tc05::mbar_wait(&tail->done, 0, abort_flag, p.wait_limit_ns);
   __syncthreads();  // every role has left its loop: nothing reads or writes the stages any more
   tc05::tc_fence_after_sync();
+  if (need_aux && Z::CTAS_PER_SM == 2) fetch_aux();
   float* acc = reinterpret_cast<float*>(smem);
   {
     const int lg = warp & 3, half = warp >> 2, r = lg * 32 + lane;
@@ -205,6 +213,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
     acc_sums[warp * 32 + lane] = have ? __uint_as_float(bits[0]) : 0.f;
   }
+  if (need_aux) asm volatile("cp.async.wait_all;" ::: "memory");
   tc05::tc_fence_before_sync();
   cg::cluster_group cluster = cg::this_cluster();
   if (p.splits > 1) cluster.sync(); else __syncthreads();
@@ -212,12 +221,11 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     tc05::tc_fence_after_sync();
     tc05::tmem_dealloc(tmem, 2 * BN);
   }
+  // a rolled loop, because a CTA that lands on an SM which has not run this kernel yet pays for every cache line of its code
 #pragma unroll 1
   for (int i = 0; i * ROWS_PER_PASS < rows_mine; ++i) {
     const int r = sub + i * ROWS_PER_PASS;
     const int row = m0 + row_first + r;
-    const uint2 aux_now = aux;
-    aux = fetch_aux(i + 1);
     if (r >= rows_mine || row >= p.m || !col_ok) continue;
     float* at = acc + (row_first + r) * Z::LD + quad * 4;
     float v[4];
@@ -241,6 +249,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       g.y = pack_bf16x2(gelu_fwd_fast(v[2]), gelu_fwd_fast(v[3]));
       *reinterpret_cast<uint2*>(p.aux_out + (size_t)row * p.ld_aux_out + col) = g;
     } else if (need_aux) {
+      const uint2 aux_now = *reinterpret_cast<const uint2*>(smem + Z::AUX + (r * BN + quad * 4) * 2);
       const float2 a0 = unpack_bf16x2(aux_now.x), a1 = unpack_bf16x2(aux_now.y);
       const float a[4] = {a0.x, a0.y, a1.x, a1.y};
 #pragma unroll
