@@ -289,141 +289,211 @@ int launch_f64_gemm(hl_ctx* ctx, const F64Gemm* problems, int count) {
 // q, k, v, out: rows of [B*T, *] with heads interleaved along the channels (column h*hd + j, as
 // src/tensor.rs:5156-5177) and a row stride each, f32 or bf16 (widened exactly).  probs: [B,H,T,T].
 //
-// One CTA of four warps per 16 query rows of one (batch, head); the rows' scores against every visible key stay in shared
+// One CTA of eight warps per 16 query rows of one (batch, head); the rows' scores against every visible key stay in shared
 // memory as f64, so each score is formed once (a lane per key walking the channels formed it three times, from
-// uncoalesced rows).  The first bound is latency: two passes over the keys in tiles of 32.
-// Measured at B16 H4 T64 hd32: forward 76 -> 9 us, backward 66 -> 15 us.
-constexpr int AT_THREADS = 128;
+// uncoalesced rows).  Bound by latency: a few thousand multiply-adds a CTA behind global loads, reductions and f64 exponentials.
+// So everything a CTA reads is requested at once and stays (`resident`, wherever keys and values fit: T 128 up to 96
+// channels), the rows of a warp go through the softmax side by side, and every warp has several chains of products.
+// B16 H4 T64 hd32, one after the other as a user calls them: forward 76 us at first, then 9 with the keys in tiles of 32 behind
+// two barriers each.
+constexpr int AT_WARPS = 8;
+constexpr int AT_THREADS = AT_WARPS * 32;
 constexpr int AT_Q = 16;   // query rows (or key rows) per CTA
-constexpr int AT_K = 32;   // keys (or queries) per tile
-constexpr int AT_GROUPS = 4;  // 8-channel groups per warp and pass: 128 channels at a time
+constexpr int AT_K = 32;   // keys (or queries) per tile where they do not all fit
+constexpr int AT_UNITS = 4;   // (8 channels, 8 rows) units per warp and pass: 128 channels at a time
+constexpr int AT_ROWS = AT_Q / AT_WARPS;  // rows of a warp in the softmax
 
 __host__ __device__ inline int at_ld(int n) { return (n + 15) / 16 * 16 + 4; }  // 4 mod 16 doubles: conflict-free fragments
 
-// rows [r0, r0 + ROWS) of a head's [T, hd] slice, widened, zero past T and past hd
-template <int ROWS, typename T>
-__device__ __forceinline__ void at_load(double* dst, int ld, const T* src, long long ld_src, int r0, int T_, int hd) {
-  const int width = ld - 4;
-  for (int e = threadIdx.x; e < ROWS * width; e += AT_THREADS) {
+__device__ __forceinline__ void at_widen4(const float* p, double (&v)[4]) {
+  const float4 t = *reinterpret_cast<const float4*>(p);
+  v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+}
+__device__ __forceinline__ void at_widen4(const __nv_bfloat16* p, double (&v)[4]) {
+  const uint2 t = *reinterpret_cast<const uint2*>(p);
+  const float2 a = unpack_bf16x2(t.x), b = unpack_bf16x2(t.y);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+
+// rows [r0, r0 + rows) of a head's [T, hd] slice, widened, zero past T.  Columns past hd are left alone: they only reach results
+// that are not stored.  Four elements a load where rows allow it, several loads in flight.
+template <typename T>
+__device__ __forceinline__ void at_load(double* dst, int ld, const T* src, long long ld_src, int r0, int rows, int T_, int hd) {
+  if (hd % 4 == 0 && ld_src % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & (4 * sizeof(T) - 1)) == 0) {
+    const int pieces = hd / 4, dr = AT_THREADS / pieces, dc = AT_THREADS % pieces;
+    int r = (int)threadIdx.x / pieces, c = (int)threadIdx.x % pieces;
+    while (r < rows) {
+      double v[4][4];
+      int at[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        at[u] = r < rows ? r * ld + c * 4 : -1;
+        if (r < rows && r0 + r < T_) {
+          at_widen4(src + (long long)(r0 + r) * ld_src + c * 4, v[u]);
+        } else {
+          v[u][0] = v[u][1] = v[u][2] = v[u][3] = 0.0;
+        }
+        r += dr;
+        c += dc;
+        if (c >= pieces) { c -= pieces; ++r; }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (at[u] >= 0) {
+          *reinterpret_cast<double2*>(dst + at[u]) = make_double2(v[u][0], v[u][1]);
+          *reinterpret_cast<double2*>(dst + at[u] + 2) = make_double2(v[u][2], v[u][3]);
+        }
+    }
+    return;
+  }
+  const int width = (hd + 3) / 4 * 4;  // the contraction goes in steps of four channels
+  for (int e = threadIdx.x; e < rows * width; e += AT_THREADS) {
     const int r = e / width, c = e % width;
     dst[r * ld + c] = (r0 + r < T_ && c < hd) ? widen(src[(long long)(r0 + r) * ld_src + c]) : 0.0;
   }
 }
 
-// S[16][keys] = scale * X · Yᵀ over the key tiles [0, n_keys): X in sx, tiles of Y through sy
+// S[16][keys] = scale * X · Yᵀ over the keys [0, n_keys): X in sx, Y in sy, all of it or (not resident) through it in tiles
 template <typename T>
 __device__ __forceinline__ void at_scores(double* ss, int ld_s, const double* sx, double* sy, int ld, const T* y,
-                                          long long ld_y, int n_keys, int T_, int hd, double scale) {
+                                          long long ld_y, int n_keys, int T_, int hd, double scale, bool resident) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fr = lane >> 2, fk = lane & 3;
-  for (int key0 = 0; key0 < n_keys; key0 += AT_K) {
-    __syncthreads();
-    at_load<AT_K>(sy, ld, y, ld_y, key0, T_, hd);
-    __syncthreads();
-    double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-    const double* pa = sx + fr * ld + fk;
-    const double* pb = sy + (warp * 8 + fr) * ld + fk;
-    for (int c = 0; c < hd; c += 4) {
-      const double b = pb[c];
-      dmma(acc[0], pa[c], b);
-      dmma(acc[1], pa[8 * ld + c], b);
+  const int tile = resident ? n_keys : AT_K;
+  for (int key0 = 0; key0 < n_keys; key0 += tile) {
+    if (!resident) {
+      __syncthreads();
+      at_load(sy, ld, y, ld_y, key0, AT_K, T_, hd);
+      __syncthreads();
     }
+    for (int k8 = warp * 8; k8 < tile; k8 += AT_WARPS * 8) {
+      double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+      const double* pa = sx + fr * ld + fk;
+      const double* pb = sy + (k8 + fr) * ld + fk;
+#pragma unroll 4
+      for (int c = 0; c < hd; c += 4) {
+        const double b = pb[c];
+        dmma(acc[0], pa[c], b);
+        dmma(acc[1], pa[8 * ld + c], b);
+      }
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      double* d = ss + (i * 8 + fr) * ld_s + key0 + warp * 8 + 2 * fk;
-      d[0] = acc[i][0] * scale;
-      d[1] = acc[i][1] * scale;
+      for (int i = 0; i < 2; ++i) {
+        double* d = ss + (i * 8 + fr) * ld_s + key0 + k8 + 2 * fk;
+        d[0] = acc[i][0] * scale;
+        d[1] = acc[i][1] * scale;
+      }
     }
   }
   __syncthreads();
 }
 
-// out rows = W[16][n_keys] · Y: W in sw (f64), tiles of Y through sy
+// out rows = W[16][n_keys] · Y: W in sw (f64), Y in sy as above
 template <typename T, typename OT>
 __device__ __forceinline__ void at_weighted(const double* sw, int ld_s, double* sy, int ld, const T* y, long long ld_y,
-                                            OT* out, long long ld_out, int t0, int n_keys, int T_, int hd) {
+                                            OT* out, long long ld_out, int t0, int n_keys, int T_, int hd, bool resident) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fr = lane >> 2, fk = lane & 3;
-  const int groups = (hd + 7) / 8;
-  for (int g0 = 0; g0 < groups; g0 += 4 * AT_GROUPS) {
-    double acc[AT_GROUPS][2][2];
+  const int units = (hd + 7) / 8 * 2;  // unit: 8 channels (u / 2) of 8 rows (u % 2)
+  const int tile = resident ? n_keys : AT_K;
+  for (int u0 = 0; u0 < units; u0 += AT_WARPS * AT_UNITS) {
+    double acc[AT_UNITS][2][2];  // even and odd steps apart
 #pragma unroll
-    for (int i = 0; i < AT_GROUPS; ++i) acc[i][0][0] = acc[i][0][1] = acc[i][1][0] = acc[i][1][1] = 0.0;
-    for (int key0 = 0; key0 < n_keys; key0 += AT_K) {
-      __syncthreads();
-      at_load<AT_K>(sy, ld, y, ld_y, key0, T_, hd);
-      __syncthreads();
-      const double* pa = sw + fr * ld_s + key0 + fk;
+    for (int i = 0; i < AT_UNITS; ++i) acc[i][0][0] = acc[i][0][1] = acc[i][1][0] = acc[i][1][1] = 0.0;
+    for (int key0 = 0; key0 < n_keys; key0 += tile) {
+      __syncthreads();  // W is complete, and nothing reads the last tile any more
+      if (!resident) {
+        at_load(sy, ld, y, ld_y, key0, AT_K, T_, hd);
+        __syncthreads();
+      }
+      for (int kk = 0; kk < tile; kk += 8) {
 #pragma unroll
-      for (int kk = 0; kk < AT_K; kk += 4) {
-        const double a0 = pa[kk], a1 = pa[8 * ld_s + kk];
-#pragma unroll
-        for (int i = 0; i < AT_GROUPS; ++i) {
-          const int grp = g0 + i * 4 + warp;
-          if (grp < groups) {
-            const double b = sy[(kk + fk) * ld + grp * 8 + fr];
-            dmma(acc[i][0], a0, b);
-            dmma(acc[i][1], a1, b);
+        for (int i = 0; i < AT_UNITS; ++i) {
+          const int u = u0 + i * AT_WARPS + warp;
+          if (u < units) {
+            const double* pa = sw + ((u & 1) * 8 + fr) * ld_s + key0 + kk + fk;
+            const double* pb = sy + (kk + fk) * ld + (u >> 1) * 8 + fr;
+            dmma(acc[i][0], pa[0], pb[0]);
+            dmma(acc[i][1], pa[4], pb[4 * ld]);
           }
         }
       }
     }
 #pragma unroll
-    for (int i = 0; i < AT_GROUPS; ++i) {
-      const int c = (g0 + i * 4 + warp) * 8 + 2 * fk;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int t = t0 + h * 8 + fr;
-        if (t < T_) {
-          if (c < hd) narrow(out + (long long)t * ld_out + c, acc[i][h][0]);
-          if (c + 1 < hd) narrow(out + (long long)t * ld_out + c + 1, acc[i][h][1]);
-        }
+    for (int i = 0; i < AT_UNITS; ++i) {
+      const int u = u0 + i * AT_WARPS + warp, t = t0 + (u & 1) * 8 + fr, c = (u >> 1) * 8 + 2 * fk;
+      if (u < units && t < T_) {
+        if (c < hd) narrow(out + (long long)t * ld_out + c, acc[i][0][0] + acc[i][1][0]);
+        if (c + 1 < hd) narrow(out + (long long)t * ld_out + c + 1, acc[i][0][1] + acc[i][1][1]);
       }
     }
   }
 }
 
-// softmax of the visible part of each row, rounded to f32: into probs (zero past the diagonal) and back into ss
-__device__ __forceinline__ void at_softmax(double* ss, int ld_s, float* probs, int t0, int n_keys, int T_) {
+// softmax of the visible part of each row, rounded to f32: into probs (zero past the diagonal), into ss and, when given, into
+// sp[16][n_keys].  A warp's rows side by side.
+__device__ __forceinline__ void at_softmax(double* ss, int ld_s, float* sp, float* probs, int t0, int n_keys, int T_) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int r = warp; r < AT_Q; r += 4) {
-    const int t = t0 + r;
-    if (t >= T_) break;  // its rows of ss are multiplied but never stored
-    double* row = ss + r * ld_s;
-    double mx = -INFINITY;
-    for (int s = lane; s <= t; s += 32) mx = max(mx, row[s]);
-    mx = warp_max(mx);
-    double sum = 0.0;
-    for (int s = lane; s <= t; s += 32) {
-      const double e = exp(row[s] - mx);
-      row[s] = e;
-      sum += e;
+  const int last = min(t0 + AT_Q, T_);
+  double mx[AT_ROWS], sum[AT_ROWS];
+#pragma unroll
+  for (int i = 0; i < AT_ROWS; ++i) mx[i] = -INFINITY;
+  for (int s = lane; s < last; s += 32)
+#pragma unroll
+    for (int i = 0; i < AT_ROWS; ++i) {
+      const int r = i * AT_WARPS + warp;
+      if (s <= t0 + r) mx[i] = max(mx[i], ss[r * ld_s + s]);
     }
-    sum = warp_sum(sum);
-    float* pr = probs + (size_t)t * T_;
-    for (int s = lane; s < max(n_keys, T_); s += 32) {
-      const float p = s <= t ? (float)(row[s] / sum) : 0.f;
-      if (s < n_keys) row[s] = (double)p;
-      if (s < T_) pr[s] = p;
+#pragma unroll
+  for (int i = 0; i < AT_ROWS; ++i) mx[i] = warp_max(mx[i]);
+#pragma unroll
+  for (int i = 0; i < AT_ROWS; ++i) sum[i] = 0.0;
+  for (int s = lane; s < last; s += 32)
+#pragma unroll
+    for (int i = 0; i < AT_ROWS; ++i) {
+      const int r = i * AT_WARPS + warp;
+      if (s <= t0 + r) {
+        const double e = exp(ss[r * ld_s + s] - mx[i]);
+        ss[r * ld_s + s] = e;
+        sum[i] += e;
+      }
     }
-  }
-  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < AT_ROWS; ++i) sum[i] = warp_sum(sum[i]);
+  for (int s = lane; s < max(n_keys, T_); s += 32)
+#pragma unroll
+    for (int i = 0; i < AT_ROWS; ++i) {
+      const int r = i * AT_WARPS + warp, t = t0 + r;  // rows past T: multiplied as zeros, never stored
+      const float p = s <= t && t < T_ ? (float)(ss[r * ld_s + s] / sum[i]) : 0.f;
+      if (s < n_keys) {
+        ss[r * ld_s + s] = (double)p;
+        if (sp) sp[r * n_keys + s] = p;
+      }
+      if (s < T_ && t < T_) probs[(size_t)t * T_ + s] = p;
+    }
 }
 
 template <typename T>
 __global__ void __launch_bounds__(AT_THREADS)
 attention_f64_fwd_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, long long ld_qkv,
-                         T* __restrict__ out, long long ld_out, float* __restrict__ probs, int T_, int H, int hd, unsigned heads) {
+                         T* __restrict__ out, long long ld_out, float* __restrict__ probs, int T_, int H, int hd, unsigned heads,
+                         bool resident) {
   pdl_begin();
   extern __shared__ double at_smem[];
-  const int ld = at_ld(hd), ld_s = at_ld((T_ + AT_K - 1) / AT_K * AT_K);
-  double *sx = at_smem, *sy = sx + AT_Q * ld, *ss = sy + AT_K * ld;
+  const int step = resident ? 8 : AT_K, padded = (T_ + step - 1) / step * step;
+  const int ld = at_ld(hd), ld_s = at_ld(padded);
+  double *sx = at_smem, *ss = sx + AT_Q * ld, *sk = ss + AT_Q * ld_s, *sv = resident ? sk + (size_t)padded * ld : sk;
   const int bh = (int)(blockIdx.x % heads), h = bh % H, b = bh / H;
   const int t0 = ((T_ - 1) / AT_Q - (int)(blockIdx.x / heads)) * AT_Q;  // the longest rows first
-  const int n_keys = (min(T_, t0 + AT_Q) + AT_K - 1) / AT_K * AT_K;
+  const int n_keys = (min(T_, t0 + AT_Q) + step - 1) / step * step;
   const long long head = (long long)b * T_ * ld_qkv + (long long)h * hd;
-  at_load<AT_Q>(sx, ld, q + head, ld_qkv, t0, T_, hd);
-  at_scores(ss, ld_s, sx, sy, ld, k + head, ld_qkv, n_keys, T_, hd, 1.0 / sqrt((double)hd));
-  at_softmax(ss, ld_s, probs + (size_t)bh * T_ * T_, t0, n_keys, T_);
-  at_weighted(ss, ld_s, sy, ld, v + head, ld_qkv, out + (long long)b * T_ * ld_out + (long long)h * hd, ld_out, t0, n_keys, T_, hd);
+  at_load(sx, ld, q + head, ld_qkv, t0, AT_Q, T_, hd);
+  if (resident) {
+    at_load(sk, ld, k + head, ld_qkv, 0, n_keys, T_, hd);
+    at_load(sv, ld, v + head, ld_qkv, 0, n_keys, T_, hd);
+    __syncthreads();
+  }
+  at_scores(ss, ld_s, sx, sk, ld, k + head, ld_qkv, n_keys, T_, hd, 1.0 / sqrt((double)hd), resident);
+  at_softmax(ss, ld_s, nullptr, probs + (size_t)bh * T_ * T_, t0, n_keys, T_);
+  at_weighted(ss, ld_s, sv, ld, v + head, ld_qkv, out + (long long)b * T_ * ld_out + (long long)h * hd, ld_out, t0, n_keys, T_, hd,
+              resident);
 }
 
 // Per 16 query rows: (the probabilities again, when they were not kept,) dP, dS (to the f32 scratch) and dQ.
@@ -431,56 +501,84 @@ template <typename T, bool RECOMPUTE>
 __global__ void __launch_bounds__(AT_THREADS)
 attention_f64_bwd_rows_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v, long long ld_qkv,
                               float* __restrict__ probs, const T* __restrict__ dout, long long ld_dout,
-                              float* __restrict__ ds, T* __restrict__ dq, long long ld_dqkv, int T_, int H, int hd, unsigned heads) {
+                              float* __restrict__ ds, T* __restrict__ dq, long long ld_dqkv, int T_, int H, int hd, unsigned heads,
+                              bool resident) {
   pdl_begin();
   extern __shared__ double at_smem[];
-  const int ld = at_ld(hd), ld_s = at_ld((T_ + AT_K - 1) / AT_K * AT_K);
-  double *sx = at_smem, *sy = sx + AT_Q * ld, *ss = sy + AT_K * ld;
+  const int step = resident ? 8 : AT_K, padded = (T_ + step - 1) / step * step;
+  const int ld = at_ld(hd), ld_s = at_ld(padded);
+  double *sx = at_smem, *sg = sx + AT_Q * ld, *ss = sg + AT_Q * ld, *sk = ss + AT_Q * ld_s;
+  double* sv = resident ? sk + (size_t)padded * ld : sk;
+  // [16][n_keys] probabilities; where shared memory is short they are read from (or back from) memory, by the lanes that wrote them
+  float* sp = resident ? reinterpret_cast<float*>(sv + (size_t)padded * ld) : nullptr;
   const int bh = (int)(blockIdx.x % heads), h = bh % H, b = bh / H;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t0 = ((T_ - 1) / AT_Q - (int)(blockIdx.x / heads)) * AT_Q;
-  const int n_keys = (min(T_, t0 + AT_Q) + AT_K - 1) / AT_K * AT_K;
+  const int n_keys = (min(T_, t0 + AT_Q) + step - 1) / step * step;
   const long long head = (long long)b * T_ * ld_qkv + (long long)h * hd;
   const double scale = 1.0 / sqrt((double)hd);
   float* pb = probs + (size_t)bh * T_ * T_;
   float* db = ds + (size_t)bh * T_ * T_;
   if constexpr (RECOMPUTE) {
-    at_load<AT_Q>(sx, ld, q + head, ld_qkv, t0, T_, hd);
-    at_scores(ss, ld_s, sx, sy, ld, k + head, ld_qkv, n_keys, T_, hd, scale);
-    at_softmax(ss, ld_s, pb, t0, n_keys, T_);  // read back below by the same warps' lanes: row r by warp r % 4
-  }
-  at_load<AT_Q>(sx, ld, dout + (long long)b * T_ * ld_dout + (long long)h * hd, ld_dout, t0, T_, hd);
-  at_scores(ss, ld_s, sx, sy, ld, v + head, ld_qkv, n_keys, T_, hd, 1.0);  // dP
-  for (int r = warp; r < AT_Q; r += 4) {
-    const int t = t0 + r;
-    if (t >= T_) break;
-    double* row = ss + r * ld_s;
-    const float* pr = pb + (size_t)t * T_;
-    float* dr = db + (size_t)t * T_;
-    double dot = 0.0;
-    for (int s = lane; s <= t; s += 32) dot += row[s] * (double)pr[s];
-    dot = warp_sum(dot);
-    for (int s = lane; s < n_keys; s += 32) {  // the column pass reads no further than this row's last tile
-      const float d = s <= t ? (float)((double)pr[s] * (row[s] - dot) * scale) : 0.f;
-      row[s] = (double)d;
-      if (s < T_) dr[s] = d;
+    at_load(sx, ld, q + head, ld_qkv, t0, AT_Q, T_, hd);
+  } else if (resident) {
+    for (int e = threadIdx.x; e < AT_Q * n_keys; e += AT_THREADS) {
+      const int r = e / n_keys, s = e % n_keys;
+      sp[e] = t0 + r < T_ && s <= t0 + r ? pb[(size_t)(t0 + r) * T_ + s] : 0.f;
     }
   }
-  at_weighted(ss, ld_s, sy, ld, k + head, ld_qkv, dq + (long long)b * T_ * ld_dqkv + (long long)h * hd, ld_dqkv, t0, n_keys, T_, hd);
+  at_load(sg, ld, dout + (long long)b * T_ * ld_dout + (long long)h * hd, ld_dout, t0, AT_Q, T_, hd);
+  if (resident) {
+    at_load(sk, ld, k + head, ld_qkv, 0, n_keys, T_, hd);
+    at_load(sv, ld, v + head, ld_qkv, 0, n_keys, T_, hd);
+    __syncthreads();
+  }
+  if constexpr (RECOMPUTE) {
+    at_scores(ss, ld_s, sx, sk, ld, k + head, ld_qkv, n_keys, T_, hd, scale, resident);
+    at_softmax(ss, ld_s, sp, pb, t0, n_keys, T_);
+    __syncthreads();  // ss is written again
+  }
+  at_scores(ss, ld_s, sg, sv, ld, v + head, ld_qkv, n_keys, T_, hd, 1.0, resident);  // dP
+  auto prob = [&](int r, int s) {  // s <= t0 + r
+    return resident ? sp[r * n_keys + s] : t0 + r < T_ ? pb[(size_t)(t0 + r) * T_ + s] : 0.f;
+  };
+  double dot[AT_ROWS];
+#pragma unroll
+  for (int i = 0; i < AT_ROWS; ++i) dot[i] = 0.0;
+  for (int s = lane; s < n_keys; s += 32)
+#pragma unroll
+    for (int i = 0; i < AT_ROWS; ++i) {
+      const int r = i * AT_WARPS + warp;
+      if (s <= t0 + r) dot[i] += ss[r * ld_s + s] * (double)prob(r, s);
+    }
+#pragma unroll
+  for (int i = 0; i < AT_ROWS; ++i) dot[i] = warp_sum(dot[i]);
+  for (int s = lane; s < n_keys; s += 32)  // the column pass reads no further than this row's last tile
+#pragma unroll
+    for (int i = 0; i < AT_ROWS; ++i) {
+      const int r = i * AT_WARPS + warp, t = t0 + r;
+      const float d = s <= t && t < T_ ? (float)((double)prob(r, s) * (ss[r * ld_s + s] - dot[i]) * scale) : 0.f;
+      ss[r * ld_s + s] = (double)d;
+      if (s < T_ && t < T_) db[(size_t)t * T_ + s] = d;
+    }
+  at_weighted(ss, ld_s, sk, ld, k + head, ld_qkv, dq + (long long)b * T_ * ld_dqkv + (long long)h * hd, ld_dqkv, t0, n_keys, T_, hd,
+              resident);
 }
 
-// Per 16 key rows: dK[s] = sum_{t>=s} dS[t,s] Q[t], dV[s] = sum_{t>=s} P[t,s] dO[t]; fixed order.
+// Per 16 key rows: dK[s] = sum_{t>=s} dS[t,s] Q[t], dV[s] = sum_{t>=s} P[t,s] dO[t]; fixed order.  The queries go through shared
+// memory `tile` at a time, all of them at once where they fit.
 template <typename T>
 __global__ void __launch_bounds__(AT_THREADS)
 attention_f64_bwd_cols_kernel(const T* __restrict__ q, long long ld_qkv, const float* __restrict__ probs,
                               const float* __restrict__ ds, const T* __restrict__ dout, long long ld_dout,
-                              T* __restrict__ dk, T* __restrict__ dv, long long ld_dqkv, int T_, int H, int hd, unsigned heads) {
+                              T* __restrict__ dk, T* __restrict__ dv, long long ld_dqkv, int T_, int H, int hd, unsigned heads,
+                              int tile) {
   pdl_begin();
   extern __shared__ double at_smem[];
-  constexpr int CH = 4 * AT_GROUPS * 8;  // channels of one pass
+  constexpr int CH = AT_WARPS * AT_UNITS / 2 * 8;  // channels of one pass
   const int ld = at_ld(min(hd, CH));
   constexpr int LDW = AT_Q + 4;
-  double *sq = at_smem, *sdo = sq + AT_K * ld, *swd = sdo + AT_K * ld, *swp = swd + AT_K * LDW;
+  double *sq = at_smem, *sdo = sq + (size_t)tile * ld, *swd = sdo + (size_t)tile * ld, *swp = swd + tile * LDW;
   const int bh = (int)(blockIdx.x % heads), h = bh % H, b = bh / H;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fr = lane >> 2, fk = lane & 3;
   const int s0 = (int)(blockIdx.x / heads) * AT_Q;
@@ -488,58 +586,52 @@ attention_f64_bwd_cols_kernel(const T* __restrict__ q, long long ld_qkv, const f
   const float* db = ds + (size_t)bh * T_ * T_;
   const T* qh = q + (long long)b * T_ * ld_qkv + (long long)h * hd;
   const T* gh = dout + (long long)b * T_ * ld_dout + (long long)h * hd;
-  const int groups = (hd + 7) / 8;
-  for (int g0 = 0; g0 < groups; g0 += 4 * AT_GROUPS) {
-    double ak[AT_GROUPS][2][2], av[AT_GROUPS][2][2];
+  for (int c0 = 0; c0 < hd; c0 += CH) {
+    const int width = min(hd - c0, CH), units = (width + 7) / 8 * 2;  // unit: 8 channels (u / 2) of 8 key rows (u % 2)
+    double ak[AT_UNITS][2][2], av[AT_UNITS][2][2];  // even and odd steps apart
 #pragma unroll
-    for (int i = 0; i < AT_GROUPS; ++i)
+    for (int i = 0; i < AT_UNITS; ++i)
 #pragma unroll
       for (int j = 0; j < 2; ++j) ak[i][j][0] = ak[i][j][1] = av[i][j][0] = av[i][j][1] = 0.0;
-    for (int t0 = s0 / AT_K * AT_K; t0 < T_; t0 += AT_K) {
+    for (int t0 = s0 / AT_K * AT_K; t0 < T_; t0 += tile) {
+      const int rows = min(tile, (T_ - t0 + 7) / 8 * 8);
       __syncthreads();
-      at_load<AT_K>(sq, ld, qh + g0 * 8, ld_qkv, t0, T_, hd - g0 * 8);
-      at_load<AT_K>(sdo, ld, gh + g0 * 8, ld_dout, t0, T_, hd - g0 * 8);
-      for (int e = threadIdx.x; e < AT_K * AT_Q; e += AT_THREADS) {
+      for (int e = threadIdx.x; e < rows * AT_Q; e += AT_THREADS) {
         const int r = e / AT_Q, c = e % AT_Q;
         const bool in = t0 + r < T_ && s0 + c <= t0 + r;
         const size_t at = (size_t)(t0 + r) * T_ + s0 + c;
         swd[r * LDW + c] = in ? (double)db[at] : 0.0;
         swp[r * LDW + c] = in ? (double)pb[at] : 0.0;
       }
+      at_load(sq, ld, qh + c0, ld_qkv, t0, rows, T_, width);
+      at_load(sdo, ld, gh + c0, ld_dout, t0, rows, T_, width);
       __syncthreads();
+      for (int kk = 0; kk < rows; kk += 8) {
 #pragma unroll
-      for (int kk = 0; kk < AT_K; kk += 4) {
-        const double* wd = swd + (kk + fk) * LDW + fr;
-        const double* wp = swp + (kk + fk) * LDW + fr;
-        const double d0 = wd[0], d1 = wd[8], p0 = wp[0], p1 = wp[8];
+        for (int i = 0; i < AT_UNITS; ++i) {
+          const int u = i * AT_WARPS + warp;
+          if (u < units) {
 #pragma unroll
-        for (int i = 0; i < AT_GROUPS; ++i) {
-          const int grp = g0 + i * 4 + warp;
-          if (grp < groups) {
-            const double bq = sq[(kk + fk) * ld + (grp - g0) * 8 + fr], bo = sdo[(kk + fk) * ld + (grp - g0) * 8 + fr];
-            dmma(ak[i][0], d0, bq);
-            dmma(ak[i][1], d1, bq);
-            dmma(av[i][0], p0, bo);
-            dmma(av[i][1], p1, bo);
+            for (int j = 0; j < 2; ++j) {
+              const int r = kk + j * 4 + fk, w = r * LDW + (u & 1) * 8 + fr, x = r * ld + (u >> 1) * 8 + fr;
+              dmma(ak[i][j], swd[w], sq[x]);
+              dmma(av[i][j], swp[w], sdo[x]);
+            }
           }
         }
       }
     }
 #pragma unroll
-    for (int i = 0; i < AT_GROUPS; ++i) {
-      const int c = (g0 + i * 4 + warp) * 8 + 2 * fk;
+    for (int i = 0; i < AT_UNITS; ++i) {
+      const int u = i * AT_WARPS + warp, s = s0 + (u & 1) * 8 + fr, c = (u >> 1) * 8 + 2 * fk;
+      if (u < units && s < T_) {
+        const long long at = ((long long)b * T_ + s) * ld_dqkv + (long long)h * hd + c0 + c;
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int s = s0 + j * 8 + fr;
-        if (s < T_) {
-          const long long at = ((long long)b * T_ + s) * ld_dqkv + (long long)h * hd + c;
-#pragma unroll
-          for (int e = 0; e < 2; ++e)
-            if (c + e < hd) {
-              narrow(dk + at + e, ak[i][j][e]);
-              narrow(dv + at + e, av[i][j][e]);
-            }
-        }
+        for (int e = 0; e < 2; ++e)
+          if (c + e < width) {
+            narrow(dk + at + e, ak[i][0][e] + ak[i][1][e]);
+            narrow(dv + at + e, av[i][0][e] + av[i][1][e]);
+          }
       }
     }
   }
@@ -616,10 +708,20 @@ __global__ void attention_f64_bwd_long_rows_kernel(const T* __restrict__ k, cons
 }
 
 constexpr size_t kAttentionSmem = 227 * 1024;
-size_t at_rows_smem(int T, int hd) {
-  return sizeof(double) * ((size_t)(AT_Q + AT_K) * at_ld(hd) + (size_t)AT_Q * at_ld(ceil_div(T, AT_K) * AT_K));
+// A row kernel's shared memory; `resident`: keys and values of the whole head in it.
+size_t at_rows_smem(int T, int hd, bool backward, bool resident) {
+  const int step = resident ? 8 : AT_K, padded = ceil_div(T, step) * step;
+  return sizeof(double) * ((size_t)((backward ? 2 : 1) * AT_Q + (resident ? 2 * padded : AT_K)) * at_ld(hd) + (size_t)AT_Q * at_ld(padded)) +
+         (backward && resident ? sizeof(float) * AT_Q * (size_t)padded : 0);
 }
-size_t at_cols_smem(int hd) { return sizeof(double) * (2 * (size_t)AT_K * at_ld(std::min(hd, 32 * AT_GROUPS)) + 2 * (size_t)AT_K * (AT_Q + 4)); }
+// Queries that the column kernel holds at a time, a multiple of eight: all of them, or what leaves room for two CTAs an SM.
+int at_cols_tile(int T, int hd, size_t* smem) {
+  const size_t row = sizeof(double) * (2 * (size_t)at_ld(std::min(hd, AT_WARPS * AT_UNITS / 2 * 8)) + 2 * (AT_Q + 4));
+  const int most = std::max(AT_K, (int)(112 * 1024 / row) / 8 * 8);
+  const int tile = std::min(ceil_div(T, 8) * 8, most);
+  *smem = row * tile;
+  return tile;
+}
 
 template <typename K>
 int at_configure(K kern) {
@@ -631,7 +733,8 @@ template <typename T>
 int attention_forward_t(hl_ctx* ctx, const T* q, const T* k, const T* v, long long ld_qkv, T* out, long long ld_out,
                         float* probs, int B, int Tn, int C, int H) {
   const int hd = C / H;
-  const size_t smem = at_rows_smem(Tn, hd);
+  const bool resident = at_rows_smem(Tn, hd, false, true) <= kAttentionSmem;
+  const size_t smem = at_rows_smem(Tn, hd, false, resident);
   const long long heads = (long long)B * H;
   if (smem <= kAttentionSmem) {
     static bool configured = false;
@@ -641,7 +744,7 @@ int attention_forward_t(hl_ctx* ctx, const T* q, const T* k, const T* v, long lo
       configured = true;
     }
     pdl(attention_f64_fwd_kernel<T>, (unsigned)(ceil_div(Tn, AT_Q) * heads), AT_THREADS, smem, ctx->stream)(
-        q, k, v, ld_qkv, out, ld_out, probs, Tn, H, hd, (unsigned)heads);
+        q, k, v, ld_qkv, out, ld_out, probs, Tn, H, hd, (unsigned)heads, resident);
     HL_LAUNCH_CHECK("attention_f64_fwd_kernel");
   } else {
     pdl(attention_f64_fwd_rows_kernel<T>, (unsigned)ceil_div_ll(heads * Tn, 4), 128, 0, ctx->stream)(q, k, v, ld_qkv, out, ld_out,
@@ -660,7 +763,10 @@ int attention_backward_t(hl_ctx* ctx, const T* q, const T* k, const T* v, long l
   int rc = ensure_workspace(ctx, sizeof(float) * (size_t)heads * Tn * Tn);
   if (rc != HL_OK) return rc;
   float* ds = reinterpret_cast<float*>(ctx->workspace);
-  const size_t rows = at_rows_smem(Tn, hd), cols = at_cols_smem(hd);
+  const bool resident = at_rows_smem(Tn, hd, true, true) <= kAttentionSmem;
+  const size_t rows = at_rows_smem(Tn, hd, true, resident);
+  size_t cols = 0;
+  const int tile = at_cols_tile(Tn, hd, &cols);
   static bool configured = false;
   if (!configured) {
     if ((rc = at_configure(attention_f64_bwd_rows_kernel<T, RECOMPUTE>)) != HL_OK) return rc;
@@ -669,7 +775,7 @@ int attention_backward_t(hl_ctx* ctx, const T* q, const T* k, const T* v, long l
   }
   if (rows <= kAttentionSmem) {
     pdl(attention_f64_bwd_rows_kernel<T, RECOMPUTE>, (unsigned)(ceil_div(Tn, AT_Q) * heads), AT_THREADS, rows, ctx->stream)(
-        q, k, v, ld_qkv, probs, dout, ld_dout, ds, dq, ld_dqkv, Tn, H, hd, (unsigned)heads);
+        q, k, v, ld_qkv, probs, dout, ld_dout, ds, dq, ld_dqkv, Tn, H, hd, (unsigned)heads, resident);
     HL_LAUNCH_CHECK("attention_f64_bwd_rows_kernel");
   } else {
     if (RECOMPUTE) {  // the output goes where dQ will be written
@@ -680,7 +786,7 @@ int attention_backward_t(hl_ctx* ctx, const T* q, const T* k, const T* v, long l
     HL_LAUNCH_CHECK("attention_f64_bwd_long_rows_kernel");
   }
   pdl(attention_f64_bwd_cols_kernel<T>, (unsigned)(ceil_div(Tn, AT_Q) * heads), AT_THREADS, cols, ctx->stream)(
-      q, ld_qkv, probs, ds, dout, ld_dout, dk, dv, ld_dqkv, Tn, H, hd, (unsigned)heads);
+      q, ld_qkv, probs, ds, dout, ld_dout, dk, dv, ld_dqkv, Tn, H, hd, (unsigned)heads, tile);
   HL_LAUNCH_CHECK("attention_f64_bwd_cols_kernel");
   count_launch(ctx, 2);
   return HL_OK;

@@ -300,7 +300,7 @@ def test_matmul_f32_strided_tiles_and_shared_contractions(m, n, k):
     assert_close("accumulate", host(out), base.astype(np.float64) + a.astype(np.float64) @ b.astype(np.float64), rtol=2 ** -23, atol=1e-30)
 
 
-@pytest.mark.parametrize("B,T,H,hd", [(1, 1, 1, 16), (2, 16, 3, 24), (1, 33, 2, 8), (1, 130, 1, 200), (1, 1700, 1, 16)])
+@pytest.mark.parametrize("B,T,H,hd", [(1, 1, 1, 16), (2, 16, 3, 24), (1, 33, 2, 8), (1, 130, 1, 200), (1, 1700, 1, 16), (2, 128, 1, 64), (1, 209, 2, 36), (1, 1000, 1, 32)])
 def test_attention_f32_tiles(B, T, H, hd):
     """Edges of the 16-row and 32-key tiles, head sizes that are no multiple of a fragment or longer than a pass, and a
     sequence whose scores do not fit in shared memory."""
