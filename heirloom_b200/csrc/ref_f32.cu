@@ -29,13 +29,20 @@ __device__ __forceinline__ void narrow(float* p, double v) { *p = (float)v; }
 __device__ __forceinline__ void narrow(__nv_bfloat16* p, double v) { *p = __float2bfloat16_rn((float)v); }  // through f32
 
 // ---- strided matmul --------------------------------------------------------------------------------
-// One CTA of eight warps per TM x TN output tile (32 x 32, or 64 x 64 when those fill the chip), k in steps of 32.  Steps are
-// copied ahead as f32 by cp.async (four bytes a copy: any stride, zero fill at the edges), each thread widens the elements
-// it copied itself into one of two f64 buffers, and one barrier a step separates widening from multiplying.  Shared rows
-// are padded so that a half warp's fragment (4 rows x 4 k) falls into 16 different 8-byte banks whichever index is
-// contiguous.  At these sizes a step is bound by its instruction count (a generic addressing version issued 976 a warp
-// and step for 32 products), so the four combinations of contiguous indices are compiled apart, with one pointer per
-// operand and immediate offsets, and the small tile's warps come in two groups that take half of every step's k each.
+// One CTA of eight warps per TM x TN output tile: 64 x 64 when those fill the chip, else 32 x 32.
+//
+// The large tile goes through k in steps of 32, copied ahead as f32 by cp.async (four bytes a copy: any stride, zero fill at the
+// edges); each thread widens the elements it copied itself into one of two f64 buffers, and one barrier a step separates
+// widening from multiplying.  Shared rows are padded so that a half warp's fragment (4 rows x 4 k) falls into 16 different
+// 8-byte banks whichever index is contiguous, and the four combinations of contiguous indices are compiled apart.
+//
+// The small tile is for products that take microseconds, where steps, barriers and instructions counted for more than the
+// multiply-adds (1024 x 512 x 128: 3.7 us of those, 14.6 us in steps as above).  Four groups of two warps take 32 of every 128 k
+// each, a warp 32 rows by 16 columns of all of the tile, so that its fragments come straight from memory, sixteen bytes a load
+// and all of them in flight, are widened in registers and meet the other groups' sums once, at the end.  Which k, row or column
+// stands in which place of a fragment is free as long as both operands, or the result, agree; it is chosen so that what a
+// lane needs is contiguous.
+//
 // Small outputs with a long contraction (weight gradients) are shared by the CTAs of a cluster: each takes a part of k,
 // and the parts are added in rank order through distributed shared memory, so the result does not depend on timing.
 // Two independent products may share a launch (an input gradient beside its weight gradient).
@@ -61,7 +68,6 @@ __device__ __forceinline__ void copy_async4(float* dst_shared, const float* src,
                "r"(in ? 4 : 0)
                : "memory");
 }
-constexpr int f64_depth(int tm) { return tm == 32 ? 4 : 2; }
 
 // One operand of a tile, ROWS x 32 a step.  KM: the contraction index is contiguous in memory.
 template <int ROWS, bool KM>
@@ -106,17 +112,17 @@ struct F64Operand {
 
 template <int TM, int TN>
 struct F64Tile {
-  static constexpr int WK = TM == 32 ? 2 : 1;              // groups of warps along k
-  static constexpr int WM = TM == 32 ? 2 : 4, WN = 2;      // warps along the tile
-  static_assert(WK * WM * WN * 32 == F64_THREADS, "eight warps");
+  static constexpr int WK = 1;                             // groups of warps along k
+  static constexpr int WM = 4, WN = 2;                     // warps along the tile
+  static_assert(WM * WN * 32 == F64_THREADS, "eight warps");
   static constexpr int FM = TM / (8 * WM), FN = TN / (8 * WN);  // 8 x 8 fragments per warp
   static constexpr int A_ELEMS = TM * (F64_BK + 4), B_ELEMS = TN * (F64_BK + 4);  // either layout fits
   static_assert(F64_BK * (TM + 4) <= A_ELEMS && F64_BK * (TN + 4) <= B_ELEMS, "both layouts share the buffers");
   static constexpr int LDC = TN + 2;
-  static constexpr int PART = TM * LDC + TM;               // one group's sums: the tile and the row sums
-  static_assert(WK * PART <= 2 * (A_ELEMS + B_ELEMS), "the output tile reuses the operand buffers");
+  static constexpr int PART = TM * LDC + TM;               // the tile's sums and the row sums
+  static_assert(PART <= 2 * (A_ELEMS + B_ELEMS), "the output tile reuses the operand buffers");
   static constexpr int RAW = (TM + TN) * F64_BK;           // one copied step, in the order the threads copied it
-  static constexpr int DEPTH = f64_depth(TM);
+  static constexpr int DEPTH = 2;
   static constexpr size_t SMEM = sizeof(double) * 2 * (A_ELEMS + B_ELEMS) + sizeof(float) * DEPTH * RAW;
 };
 
@@ -140,10 +146,8 @@ __device__ __forceinline__ void f64_tile_sums(const F64Gemm& g, double* smem, in
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  const int group = warp / (Z::WM * Z::WN), within = warp % (Z::WM * Z::WN);
-  const int wm = within / Z::WN * (Z::FM * 8), wn = within % Z::WN * (Z::FN * 8);
+  const int wm = warp / Z::WN * (Z::FM * 8), wn = warp % Z::WN * (Z::FN * 8);
   const int fr = lane >> 2, fk = lane & 3;
-  constexpr int KG = F64_BK / Z::WK;  // this group's part of a step
   double acc[Z::FM][Z::FN][2], rs[Z::FM][2];
 #pragma unroll
   for (int i = 0; i < Z::FM; ++i) {
@@ -162,10 +166,10 @@ __device__ __forceinline__ void f64_tile_sums(const F64Gemm& g, double* smem, in
     ob.widen_into(buf + Z::A_ELEMS, src + OA::PER_THREAD * F64_THREADS);
     request(step + Z::DEPTH);
     __syncthreads();
-    const double* sa = buf + (wm + fr) * OA::ROW + (group * KG + fk) * OA::K;
-    const double* sb = buf + Z::A_ELEMS + (wn + fr) * OB::ROW + (group * KG + fk) * OB::K;
+    const double* sa = buf + (wm + fr) * OA::ROW + fk * OA::K;
+    const double* sb = buf + Z::A_ELEMS + (wn + fr) * OB::ROW + fk * OB::K;
 #pragma unroll
-    for (int kk = 0; kk < KG; kk += 4) {
+    for (int kk = 0; kk < F64_BK; kk += 4) {
       double fa[Z::FM], fb[Z::FN];
 #pragma unroll
       for (int i = 0; i < Z::FM; ++i) fa[i] = sa[i * 8 * OA::ROW + kk * OA::K];
@@ -182,7 +186,7 @@ __device__ __forceinline__ void f64_tile_sums(const F64Gemm& g, double* smem, in
     }
   }
   __syncthreads();
-  double* sc = smem + group * Z::PART;
+  double* sc = smem;
 #pragma unroll
   for (int i = 0; i < Z::FM; ++i) {
 #pragma unroll
@@ -195,8 +199,108 @@ __device__ __forceinline__ void f64_tile_sums(const F64Gemm& g, double* smem, in
   }
 }
 
+template <>
+struct F64Tile<32, 32> {
+  static constexpr int WK = 4, LDC = 34, PART = 32 * LDC + 32;
+  static constexpr size_t SMEM = sizeof(double) * WK * PART;
+};
+
+// Up to four values, zero past `left`; `vec`: they are contiguous and start on their size.
+__device__ __forceinline__ float4 load_upto4(const float* p, long long stride, int left, bool vec) {
+  if (left >= 4 && vec) return __ldg(reinterpret_cast<const float4*>(p));
+  return make_float4(left > 0 ? __ldg(p) : 0.f, left > 1 ? __ldg(p + stride) : 0.f, left > 2 ? __ldg(p + 2 * stride) : 0.f,
+                     left > 3 ? __ldg(p + 3 * stride) : 0.f);
+}
+// Fragments of 8 * F rows (of A; columns of B) and sixteen k: v[i][s] is this lane's element of fragment i in step s.  Lane (fr,
+// fk) stands for k = k0 + 4 fk + s and, with the contraction contiguous (KM), for row i * 8 + fr, else for row fr * F + i.
+template <int F, bool KM>
+__device__ __forceinline__ void load_fragments(float (&v)[F][4], const float* base, long long row_stride, long long k_stride, int row0,
+                                               int rows, int k0, int k_end, bool vec) {
+  const int lane = threadIdx.x & 31, fr = lane >> 2, k = k0 + 4 * (lane & 3);
+  if constexpr (KM) {
+#pragma unroll
+    for (int i = 0; i < F; ++i) {
+      const int row = row0 + i * 8 + fr;
+      const float4 t = load_upto4(base + row * row_stride + k, 1, row < rows ? k_end - k : 0, vec);
+      v[i][0] = t.x; v[i][1] = t.y; v[i][2] = t.z; v[i][3] = t.w;
+    }
+  } else {
+    const int row = row0 + fr * F;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int left = k + s < k_end ? rows - row : 0;
+      const float* p = base + row * row_stride + (k + s) * k_stride;
+      if constexpr (F == 4) {
+        const float4 t = load_upto4(p, row_stride, left, vec);
+        v[0][s] = t.x; v[1][s] = t.y; v[2][s] = t.z; v[3][s] = t.w;
+      } else {
+        static_assert(F == 2, "two or four fragments");
+        float2 t;
+        if (left >= 2 && vec) t = __ldg(reinterpret_cast<const float2*>(p));
+        else t = make_float2(left > 0 ? __ldg(p) : 0.f, left > 1 ? __ldg(p + row_stride) : 0.f);
+        v[0][s] = t.x; v[1][s] = t.y;
+      }
+    }
+  }
+}
+
+// The 32 x 32 tile: this warp's sums over its group's k, to the group's place in shared memory.
+template <bool A_KM, bool B_KM>
+__device__ __forceinline__ void f64_small_sums(const F64Gemm& g, double* smem, int row0, int col0, int kt0, int kt1, bool sums) {
+  using Z = F64Tile<32, 32>;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, fr = lane >> 2, fk = lane & 3;
+  const int group = warp >> 1, wn = (warp & 1) * 16;
+  // one index contiguous, strides along the other that keep sixteen bytes
+  const bool vec_a = (A_KM || g.a_row == 1) && ((A_KM ? g.a_row : g.a_col) & 3) == 0 && (reinterpret_cast<uintptr_t>(g.a) & 15) == 0;
+  const bool vec_b = (B_KM || g.b_col == 1) && ((B_KM ? g.b_col : g.b_row) & 3) == 0 && (reinterpret_cast<uintptr_t>(g.b) & 15) == 0;
+  double acc[4][2][2], rs[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    rs[i] = 0.0;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  }
+  const int k_end = min(g.k, kt1 * F64_BK);
+  for (int kt = kt0 + group; kt < kt1; kt += Z::WK) {
+    float a[2][4][4], b[2][2][4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      load_fragments<4, A_KM>(a[h], g.a, g.a_row, g.a_col, row0, g.m, kt * F64_BK + h * 16, k_end, vec_a);
+      load_fragments<2, B_KM>(b[h], g.b, g.b_col, g.b_row, col0 + wn, g.n, kt * F64_BK + h * 16, k_end, vec_b);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const double b0 = (double)b[h][0][s], b1 = (double)b[h][1][s];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const double av = (double)a[h][i][s];
+          dmma(acc[i][0], av, b0);
+          dmma(acc[i][1], av, b1);
+          if (sums) rs[i] += av;  // row sums of A: a bias gradient rides on its weight gradient
+        }
+      }
+  }
+  double* sc = smem + group * Z::PART;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = A_KM ? i * 8 + fr : fr * 4 + i;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) sc[row * Z::LDC + wn + (B_KM ? j * 8 + 2 * fk + e : (2 * fk + e) * 2 + j)] = acc[i][j][e];
+    if (sums && wn == 0) {
+      double t = rs[i];
+      t += __shfl_xor_sync(0xffffffffu, t, 1);
+      t += __shfl_xor_sync(0xffffffffu, t, 2);
+      if (fk == 0) sc[32 * Z::LDC + row] = t;
+    }
+  }
+}
+
 template <int TM, int TN>
-__global__ void __launch_bounds__(F64_THREADS, TM == 32 ? 3 : 2)
+__global__ void __launch_bounds__(F64_THREADS, 2)
 f64_gemm_kernel(const F64Jobs jobs) {
   pdl_begin();
   using Z = F64Tile<TM, TN>;
@@ -212,7 +316,15 @@ f64_gemm_kernel(const F64Jobs jobs) {
   const int row0 = (tile / jb.tiles_n) * TM, col0 = (tile % jb.tiles_n) * TN;
   const int kt0 = rank * jb.k_tiles_per_rank, kt1 = max(kt0, min((g.k + F64_BK - 1) / F64_BK, kt0 + jb.k_tiles_per_rank));
   const bool sums = g.row_sum != nullptr && col0 == 0;
-  if (g.a_col == 1) {
+  if constexpr (TM == 32) {
+    if (g.a_col == 1) {
+      if (g.b_row == 1) f64_small_sums<true, true>(g, f64_smem, row0, col0, kt0, kt1, sums);
+      else f64_small_sums<true, false>(g, f64_smem, row0, col0, kt0, kt1, sums);
+    } else {
+      if (g.b_row == 1) f64_small_sums<false, true>(g, f64_smem, row0, col0, kt0, kt1, sums);
+      else f64_small_sums<false, false>(g, f64_smem, row0, col0, kt0, kt1, sums);
+    }
+  } else if (g.a_col == 1) {
     if (g.b_row == 1) f64_tile_sums<TM, TN, true, true>(g, f64_smem, row0, col0, kt0, kt1, sums);
     else f64_tile_sums<TM, TN, true, false>(g, f64_smem, row0, col0, kt0, kt1, sums);
   } else {
@@ -221,14 +333,22 @@ f64_gemm_kernel(const F64Jobs jobs) {
   }
   const int parts = jb.split;
   cg::cluster_group cluster = cg::this_cluster();
-  if (parts > 1) cluster.sync(); else __syncthreads();
-  auto total = [&](int at) {  // over the CTAs of the cluster and the groups of each, in order
-    double v = 0.0;
-    for (int p = 0; p < parts; ++p) {
-      const double* s = parts > 1 ? cluster.map_shared_rank(f64_smem + at, p) : f64_smem + at;
+  __syncthreads();
+  auto groups = [&](int at) {  // the sums of this CTA's groups of warps, in order
+    double v = f64_smem[at];
 #pragma unroll
-      for (int w = 0; w < Z::WK; ++w) v += s[w * Z::PART];
-    }
+    for (int w = 1; w < Z::WK; ++w) v += f64_smem[w * Z::PART + at];
+    return v;
+  };
+  if (parts > 1) {
+    if (Z::WK > 1)  // added up before the other CTAs of the cluster read them
+      for (int at = tid; at < Z::PART; at += F64_THREADS) f64_smem[at] = groups(at);
+    cluster.sync();
+  }
+  auto total = [&](int at) {  // over the CTAs of the cluster, in order
+    if (parts == 1) return groups(at);
+    double v = 0.0;
+    for (int p = 0; p < parts; ++p) v += *cluster.map_shared_rank(f64_smem + at, p);
     return v;
   };
   for (int e = rank * F64_THREADS + tid; e < TM * TN; e += parts * F64_THREADS) {
