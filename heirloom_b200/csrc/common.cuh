@@ -63,7 +63,7 @@ struct hl_ctx {
   int comm_sms = 0;                    // how many they leave when asked to (0 = none); set when the communicator is made
   cudaStream_t stream = nullptr;       // compute stream
   cudaStream_t comm_stream = nullptr;  // collective stream
-  int* status_dev = nullptr;           // hl::ST_SLOTS ints
+  int* status_dev = nullptr;           // hl::ST_SLOTS ints: status_host as the device sees it
   int* status_host = nullptr;          // pinned mirror
   void* workspace = nullptr;           // grow-only scratch (split-K partials, reductions)
   size_t workspace_bytes = 0;

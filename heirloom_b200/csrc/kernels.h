@@ -177,8 +177,15 @@ int decode_embed(hl_ctx* ctx, const float* table, const float* positions, const 
 struct AdamPlan;
 int adam_plan_create(hl_ctx* ctx, const hl_adamw_tensor* tensors, int count, AdamPlan** out);
 void adam_plan_destroy(AdamPlan* plan);
-int adam_plan_step(hl_ctx* ctx, AdamPlan* plan, const hl_adamw_params* hp);
-int adam_plan_step_range(hl_ctx* ctx, AdamPlan* plan, const hl_adamw_params* hp, int first, int count);
+// Clipping by the global norm on the device: hp's clip_scale times min(1, limit / norm), norm the square root of *sum_sq times
+// scale * scale.  Nothing is updated when that sum is not a finite non-negative number.
+struct AdamClip {
+  const float* sum_sq;  // device, null: no clipping
+  double scale, limit;
+};
+int adam_plan_step(hl_ctx* ctx, AdamPlan* plan, const hl_adamw_params* hp, const AdamClip& clip = AdamClip{nullptr, 0.0, 0.0});
+int adam_plan_step_range(hl_ctx* ctx, AdamPlan* plan, const hl_adamw_params* hp, int first, int count,
+                         const AdamClip& clip = AdamClip{nullptr, 0.0, 0.0});
 int adam_plan_chunk_elements(const AdamPlan* plan);
 int adam_plan_chunk_count(const AdamPlan* plan);
 

@@ -4,7 +4,7 @@
 // weights the next step's GEMMs read.
 #include <vector>
 
-#include "common.cuh"
+#include "kernels.h"
 
 namespace hl {
 namespace {
@@ -44,8 +44,19 @@ __device__ __forceinline__ void adamw_element(float& p, float g, float& m, float
 }
 
 __global__ void __launch_bounds__(ADAM_THREADS)
-adamw_chunks_kernel(const AdamChunk* __restrict__ chunks, const hl_adamw_params hp) {
+adamw_chunks_kernel(const AdamChunk* __restrict__ chunks, hl_adamw_params hp, const AdamClip clip) {
   pdl_begin();
+  if (clip.sum_sq) {
+    __shared__ float factor;
+    if (threadIdx.x == 0) {
+      const double sum = (double)*clip.sum_sq * clip.scale * clip.scale;
+      const double norm = sqrt(sum);
+      factor = !(sum >= 0.0) || sum > 1e300 ? -1.f : norm > clip.limit ? (float)(clip.limit / (norm + 1e-12)) : 1.f;
+    }
+    __syncthreads();
+    if (factor < 0.f) return;
+    hp.clip_scale = factor * hp.clip_scale;
+  }
   const AdamChunk ch = chunks[blockIdx.x];
   const unsigned int n4 = ch.n / 4;
   for (unsigned int i = threadIdx.x; i < n4; i += blockDim.x) {
@@ -148,21 +159,21 @@ int adam_plan_chunk_count(const AdamPlan* plan) { return plan->count; }
 
 // Chunks [first, first + count) of the table: lets a caller update the part of a gradient arena whose
 // all-reduce has finished while the rest is still in flight.
-int adam_plan_step_range(hl_ctx* ctx, AdamPlan* plan, const hl_adamw_params* hp, int first, int count) {
+int adam_plan_step_range(hl_ctx* ctx, AdamPlan* plan, const hl_adamw_params* hp, int first, int count, const AdamClip& clip) {
   int rc = validate(hp, "hl_adamw_multi");
   if (rc != HL_OK) return rc;
   HL_REQUIRE(first >= 0 && count >= 0 && first + count <= plan->count, "adamw plan: chunk range out of bounds");
   if (count == 0) return HL_OK;
   // 28 bytes per parameter (read p, g, m, v; write p, m, v) plus 2 for the bf16 shadow
   ProfileScope prof(ctx, HL_PROF_OPTIMIZER, 30.0 * (double)plan->elements * ((double)count / (double)plan->count));
-  pdl(adamw_chunks_kernel, count, ADAM_THREADS, 0, ctx->stream)(plan->chunks_dev + first, *hp);
+  pdl(adamw_chunks_kernel, count, ADAM_THREADS, 0, ctx->stream)(plan->chunks_dev + first, *hp, clip);
   HL_LAUNCH_CHECK("adamw_chunks_kernel");
   count_launch(ctx);
   return HL_OK;
 }
 
-int adam_plan_step(hl_ctx* ctx, AdamPlan* plan, const hl_adamw_params* hp) {
-  return adam_plan_step_range(ctx, plan, hp, 0, plan->count);
+int adam_plan_step(hl_ctx* ctx, AdamPlan* plan, const hl_adamw_params* hp, const AdamClip& clip) {
+  return adam_plan_step_range(ctx, plan, hp, 0, plan->count, clip);
 }
 
 }  // namespace hl

@@ -1417,16 +1417,25 @@ int optimizer_step(hl_decoder* m) {
   if (m->opt.clip_norm > 0.f) HL_TRY(wait_for_collectives(m));  // the global norm needs every averaged gradient
   const int world = nccl_world(ctx);
   const float inv_world = 1.0f / (float)world;  // sum then scale by 1/world (src/nn.rs:2100-2117)
+  // Global gradient norm after averaging; forces one device-to-host read like the reference.  Without collectives the factor is
+  // worked out on the device, so that the update does not wait for the host to have read the norm.
+  const bool on_device = m->opt.clip_norm > 0.f && !m->comm_pending;
   double clip = 1.0;
-  if (m->opt.clip_norm > 0.f) {
-    // global gradient norm after averaging; forces one device-to-host read like the reference
-    HL_TRY(hl_sum_squares_f32(ctx, m->grads, m->arena, m->norm_dev));
+  double sum_sq = 0.0;
+  auto read_norm = [&]() -> int {
     HL_CUDA(cudaMemcpyAsync(m->norm_host, m->norm_dev, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     HL_CUDA(cudaStreamSynchronize(ctx->stream));
-    const double sum_sq = (double)m->norm_host[0] * (double)inv_world * (double)inv_world;
+    sum_sq = (double)m->norm_host[0] * (double)inv_world * (double)inv_world;
     if (!(sum_sq >= 0.0) || sum_sq > 1e300) return fail("non-finite or negative global gradient sum-of-squares");
-    const double norm = sqrt(sum_sq);
-    if (norm > (double)m->opt.clip_norm) clip = (double)m->opt.clip_norm / (norm + 1e-12);
+    return HL_OK;
+  };
+  if (m->opt.clip_norm > 0.f) {
+    HL_TRY(hl_sum_squares_f32(ctx, m->grads, m->arena, m->norm_dev));
+    if (!on_device) {
+      HL_TRY(read_norm());
+      const double norm = sqrt(sum_sq);
+      if (norm > (double)m->opt.clip_norm) clip = (double)m->opt.clip_norm / (norm + 1e-12);
+    }
   }
   m->step += 1;
   hl_adamw_params hp{};
@@ -1435,6 +1444,12 @@ int optimizer_step(hl_decoder* m) {
   hp.clip_scale = (float)clip * inv_world;
   hp.bias_correction1 = (float)(1.0 - pow((double)m->opt.beta1, (double)m->step));
   hp.bias_correction2 = (float)(1.0 - pow((double)m->opt.beta2, (double)m->step));
+  if (on_device) {
+    HL_TRY(adam_plan_step(ctx, m->plan, &hp, AdamClip{m->norm_dev, (double)inv_world, (double)m->opt.clip_norm}));
+    const int rc = read_norm();
+    if (rc != HL_OK) m->step -= 1;  // nothing was updated
+    return rc;
+  }
   if (!m->comm_pending) return adam_plan_step(ctx, m->plan, &hp);
   // Collectives still in flight: update the arena in groups of buckets, each group as soon as its last
   // all-reduce has finished, so the update of the early buckets overlaps the reduction of the late ones.
