@@ -31,11 +31,11 @@ GPT = dict(vocab=50304, d_model=768, n_layers=12, n_heads=12, d_ff=3072, context
 MICRO_BATCH = 16
 METRIC = "train tokens/s (GPT-124M-shaped bf16 step)"
 DATASHEET_BF16_TFLOPS = 2250.0
-# dram__bytes_read.sum + dram__bytes_write.sum per GEMM launch, averaged over the launches of two training steps
+# dram__bytes_read.sum + dram__bytes_write.sum per GEMM launch, averaged over the GEMM launches of one training step
 # in a one-pass ncu launch list of this command (summary kept under profiles/), and the first 16 hex digits of the
 # SHA-256 of the GEMM source the capture ran with: a kernel changed since then gets no traffic figure, not a stale one.
-GEMM_DRAM_BYTES_PER_LAUNCH = 153.7e6
-GEMM_SOURCE_AT_CAPTURE = "6a10afcb74c80bde"
+GEMM_DRAM_BYTES_PER_LAUNCH = 239.1e6
+GEMM_SOURCE_AT_CAPTURE = "64ddc78a321a5734"
 
 
 def gemm_traffic():
