@@ -206,16 +206,21 @@ reduce_partial_kernel(const float* __restrict__ x, size_t n, bool vec, double* _
   if (threadIdx.x == 0) partial[blockIdx.x] = acc;
 }
 
-__global__ void reduce_final_kernel(const double* __restrict__ partial, int count, double scale, float* __restrict__ out) {
+__global__ void reduce_final_kernel(const double* __restrict__ partial, int count, double scale, float* __restrict__ out,
+                                    float* __restrict__ out_host) {
   pdl_begin();
   __shared__ double sm[32];
   double acc = 0.0;
   for (int i = threadIdx.x; i < count; i += blockDim.x) acc += partial[i];
   acc = block_sum(acc, sm);
-  if (threadIdx.x == 0) out[0] = (float)(acc * scale);
+  if (threadIdx.x == 0) {
+    out[0] = (float)(acc * scale);
+    if (out_host) out_host[0] = (float)(acc * scale);
+  }
 }
 
-int reduce_impl(hl_ctx* ctx, const float* x, size_t n, float* out_dev, int mode, double scale) {
+// `out_host`: pinned memory that gets the result as well, or null.
+int reduce_impl(hl_ctx* ctx, const float* x, size_t n, float* out_dev, int mode, double scale, float* out_host = nullptr) {
   HL_REQUIRE(ctx && out_dev && (x || n == 0), "reduction: null argument");
   const int blocks = (int)std::min<size_t>(std::max<size_t>((n + 4095) / 4096, 1), (size_t)ctx->sm_count * 8);
   const bool vec = aligned16(x);
@@ -225,13 +230,17 @@ int reduce_impl(hl_ctx* ctx, const float* x, size_t n, float* out_dev, int mode,
   if (mode == 1) pdl(reduce_partial_kernel<1>, blocks, 256, 0, ctx->stream).streaming(4.0 * n)(x, n, vec, partial);
   else pdl(reduce_partial_kernel<0>, blocks, 256, 0, ctx->stream).streaming(4.0 * n)(x, n, vec, partial);
   HL_LAUNCH_CHECK("reduce_partial_kernel");
-  pdl(reduce_final_kernel, 1, 256, 0, ctx->stream)(partial, blocks, scale, out_dev);
+  pdl(reduce_final_kernel, 1, 256, 0, ctx->stream)(partial, blocks, scale, out_dev, out_host);
   HL_LAUNCH_CHECK("reduce_final_kernel");
   count_launch(ctx, 2);
   return HL_OK;
 }
 
 }  // namespace
+
+int sum_squares_impl(hl_ctx* ctx, const float* x, size_t n, float* out_dev, float* out_host) {
+  return reduce_impl(ctx, x, n, out_dev, 1, 1.0, out_host);
+}
 
 int bias_grad_impl(hl_ctx* ctx, const void* grad_out, int dtype, float* grad_bias, int rows, int cols, FoldBatch* defer) {
   HL_REQUIRE(ctx && grad_out && grad_bias, "hl_bias_grad: null argument");

@@ -177,6 +177,8 @@ int decode_embed(hl_ctx* ctx, const float* table, const float* positions, const 
 struct AdamPlan;
 int adam_plan_create(hl_ctx* ctx, const hl_adamw_tensor* tensors, int count, AdamPlan** out);
 void adam_plan_destroy(AdamPlan* plan);
+// hl_sum_squares_f32 whose result goes to pinned host memory as well.
+int sum_squares_impl(hl_ctx* ctx, const float* x, size_t n, float* out_dev, float* out_host);
 // Clipping by the global norm on the device: hp's clip_scale times min(1, limit / norm), norm the square root of *sum_sq times
 // scale * scale.  Nothing is updated when that sum is not a finite non-negative number.
 struct AdamClip {

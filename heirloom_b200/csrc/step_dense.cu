@@ -127,6 +127,8 @@ struct hl_decoder {
   bool fork_ok = false;
   cudaStream_t side_stream = nullptr;
   cudaEvent_t fork_event = nullptr, join_event = nullptr;
+  cudaEvent_t zero_event = nullptr;  // the scattered gradients have been zeroed there
+  bool zeroed = false;
   // ... or, where the products fill the chip, collected for `group_layers` layers (0: not) and run by one launch.
   int group_layers = 0;
   std::vector<WeightGradJob> wgrads;
@@ -584,6 +586,38 @@ int join_side(hl_decoder* m) {
   return HL_OK;
 }
 
+int zero_memory_table_grads(hl_decoder* m) {
+  if (!m->has_memory) return HL_OK;
+  const size_t count = m->off_val + (size_t)m->mem.slots * m->mem.value_dim - m->off_kl;
+  HL_CUDA(cudaMemsetAsync(m->grads + m->off_kl, 0, sizeof(float) * count, m->ctx->stream));
+  return HL_OK;
+}
+
+bool beside(const hl_decoder* m) { return m->side_stream && !nccl_active(m->ctx) && !m->ctx->profiler; }
+
+// Gradients that are sums over scattered rows (embeddings, memory tables) start at zero: zeroed beside the forward pass, which
+// does not look at them, so that 20 MB or 540 MB of them do not stand between two kernels of the backward pass.
+int zero_tables(hl_decoder* m) {
+  HL_TRY(zero_memory_table_grads(m));
+  HL_CUDA(cudaMemsetAsync(m->grads + m->off_pos, 0, sizeof(float) * (m->arena - m->off_pos), m->ctx->stream));
+  return HL_OK;
+}
+int zero_tables_beside(hl_decoder* m) {
+  m->zeroed = beside(m);
+  if (!m->zeroed) return HL_OK;
+  SideStream side(m);
+  HL_TRY(side.rc);
+  HL_TRY(zero_tables(m));
+  HL_CUDA(cudaEventRecord(m->zero_event, m->ctx->stream));
+  return HL_OK;
+}
+// Before the first of those gradients is added to.
+int tables_are_zero(hl_decoder* m) {
+  if (!m->zeroed) return zero_tables(m);
+  HL_CUDA(cudaStreamWaitEvent(m->ctx->stream, m->zero_event, 0));
+  return HL_OK;
+}
+
 // Collected weight gradients are not final when their layer is done, so not while buckets of them are being exchanged.
 bool grouping(const hl_decoder* m) { return m->group_layers > 0 && !nccl_active(m->ctx); }
 int run_weight_gradients(hl_decoder* m) {
@@ -649,14 +683,6 @@ int memory_core_backward(hl_decoder* m, int l, const float* dweighted) {
   HL_TRY(hl_softmax_rows_backward_f32(ctx, a.weights, m->m_dw, m->m_dscores, N, k));
   return hl_memory_selected_scores_backward(ctx, a.idx, a.query, kd, P + m->off_kl, P + m->off_kr, m->m_dscores, m->m_dq, kd,
                                             G + m->off_kl, G + m->off_kr, N, k, side, kd, m->mem.slots);
-}
-
-// Table gradients are sums over scattered rows: they start every backward at zero.
-int zero_memory_table_grads(hl_decoder* m) {
-  if (!m->has_memory) return HL_OK;
-  const size_t count = m->off_val + (size_t)m->mem.slots * m->mem.value_dim - m->off_kl;
-  HL_CUDA(cudaMemsetAsync(m->grads + m->off_kl, 0, sizeof(float) * count, m->ctx->stream));
-  return HL_OK;
 }
 
 // Attention for head sizes the tcgen05 kernels are not built for (they take head_dim 64 and 128): the f32 kernels read the
@@ -984,9 +1010,9 @@ int backward(hl_decoder* m) {
     HL_CUDA(cudaStreamWaitEvent(m->ctx->stream, m->comm_done, 0));
     m->comm_pending = false;
   }
-  HL_TRY(zero_memory_table_grads(m));
   // loss and dlogits = (softmax - onehot)/N in bf16, the operand precision of the next GEMMs
   HL_TRY(cross_entropy_impl(ctx, m->logits, V, m->targets, N, V, 1.0f, m->loss_dev, nullptr, m->dlogits, HL_BF16, V, m->loss_host));
+  if (m->has_memory) HL_TRY(tables_are_zero(m));
   FoldBatch* fb = &m->fold;
   fb->n = 0;
   fb->used = 0;
@@ -1086,8 +1112,13 @@ int backward(hl_decoder* m) {
     if (grouping(m) && (l == 0 || (c.n_layers - l) % m->group_layers == 0)) HL_TRY(run_weight_gradients(m));
     HL_TRY(finished(o.ln1b + d));
   }
-  // embeddings: scatter-add into zeroed tables
-  HL_CUDA(cudaMemsetAsync(G + m->off_pos, 0, sizeof(float) * (m->arena - m->off_pos), ctx->stream));
+  // embeddings: scatter-add into zeroed tables, the last column sums folded beside them
+  if (!m->has_memory) HL_TRY(tables_are_zero(m));
+  if (beside(m)) {
+    SideStream side(m);
+    HL_TRY(side.rc);
+    HL_TRY(fold_batch_flush(ctx, fb));
+  }
   HL_TRY(hl_embedding_backward(ctx, dx, m->tokens, G + m->off_tok, V, G + m->off_pos, T, N, d));
   HL_TRY(join_side(m));
   HL_TRY(finished(m->arena));
@@ -1202,7 +1233,7 @@ int backward_f32(hl_decoder* m) {
     return flush_buckets(m, done);
   };
   HL_TRY(cross_entropy_impl(ctx, m->logits, V, m->targets, N, V, 1.0f, m->loss_dev, nullptr, m->dlogits_f, HL_F32, V, m->loss_host));
-  HL_TRY(zero_memory_table_grads(m));
+  if (m->has_memory) HL_TRY(tables_are_zero(m));
   float* dx = m->d_a;       // gradient of the residual stream
   float* dx_next = m->d_b;
   HL_TRY(linear_backward_f32(m, m->zf, P + m->off_head_w, m->dlogits_f, m->d_c, G + m->off_head_w, G + m->off_head_b, N, d, V));
@@ -1242,8 +1273,14 @@ int backward_f32(hl_decoder* m) {
     std::swap(dx, dx_next);
     HL_TRY(finished(o.ln1b + d));
   }
-  HL_CUDA(cudaMemsetAsync(G + m->off_pos, 0, sizeof(float) * (m->arena - m->off_pos), ctx->stream));
+  if (!m->has_memory) HL_TRY(tables_are_zero(m));
+  if (beside(m)) {
+    SideStream side(m);
+    HL_TRY(side.rc);
+    HL_TRY(fold_batch_flush(ctx, fb));
+  }
   HL_TRY(hl_embedding_backward(ctx, dx, m->tokens, G + m->off_tok, V, G + m->off_pos, T, N, d));
+  HL_TRY(join_side(m));
   HL_TRY(finished(m->arena));
   if (nccl_active(ctx)) {
     if (m->has_memory || m->sparse_tok_exchange) {
@@ -1423,14 +1460,13 @@ int optimizer_step(hl_decoder* m) {
   double clip = 1.0;
   double sum_sq = 0.0;
   auto read_norm = [&]() -> int {
-    HL_CUDA(cudaMemcpyAsync(m->norm_host, m->norm_dev, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     HL_CUDA(cudaStreamSynchronize(ctx->stream));
     sum_sq = (double)m->norm_host[0] * (double)inv_world * (double)inv_world;
     if (!(sum_sq >= 0.0) || sum_sq > 1e300) return fail("non-finite or negative global gradient sum-of-squares");
     return HL_OK;
   };
   if (m->opt.clip_norm > 0.f) {
-    HL_TRY(hl_sum_squares_f32(ctx, m->grads, m->arena, m->norm_dev));
+    HL_TRY(sum_squares_impl(ctx, m->grads, m->arena, m->norm_dev, m->norm_host));
     if (!on_device) {
       HL_TRY(read_norm());
       const double norm = sqrt(sum_sq);
@@ -1614,10 +1650,11 @@ static int decoder_create_impl(hl_ctx* ctx, const hl_decoder_config* cfg, const 
     e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
     if (e != cudaSuccess) { *ev = nullptr; return fail_cuda(e, "cudaEventCreate(row exchange)"); }
   }
-  if (m->fork_ok) {
+  {
     e = cudaStreamCreateWithFlags(&m->side_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&m->fork_event, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&m->join_event, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&m->zero_event, cudaEventDisableTiming);
     if (e != cudaSuccess) return cleanup(fail_cuda(e, "cudaStreamCreate(side)"));
   }
   e = cudaEventCreateWithFlags(&m->comm_done, cudaEventDisableTiming);
@@ -1641,6 +1678,7 @@ void hl_decoder_destroy(hl_decoder* m) {
   if (m->comm_done) cudaEventDestroy(m->comm_done);
   if (m->side_stream) cudaStreamDestroy(m->side_stream);
   if (m->fork_event) cudaEventDestroy(m->fork_event);
+  if (m->zero_event) cudaEventDestroy(m->zero_event);
   if (m->join_event) cudaEventDestroy(m->join_event);
   for (cudaEvent_t ev : {m->rows_known, m->tok_count_ready, m->val_count_ready}) if (ev) cudaEventDestroy(ev);
   for (auto ev : m->wait_begin) cudaEventDestroy(ev);
@@ -1752,6 +1790,7 @@ int hl_decoder_forward_backward(hl_decoder* m, const int64_t* tokens_dev, const 
   if (targets_dev != m->targets)
     HL_CUDA(cudaMemcpyAsync(m->targets, targets_dev, sizeof(int64_t) * m->N, cudaMemcpyDeviceToDevice, m->ctx->stream));
   HL_TRY(run_graphed(m, GRAPH_STEP, [m]() -> int {
+    HL_TRY(zero_tables_beside(m));
     HL_TRY(prepare_token_rows(m));  // data parallel: the union of the ranks' token rows forms while forward runs
     if (m->cfg.precision == HL_PRECISION_AMP_BF16) {
       HL_TRY(forward(m));
