@@ -51,9 +51,14 @@ constexpr int SS_T = 64;   // tokens per block
 constexpr int SS_K = 128;  // keys per block
 constexpr int SS_J = 64;   // contraction slice
 __global__ void __launch_bounds__(256)
-side_scores_kernel(const float* __restrict__ query, long long ld_q, int q_off, const float* __restrict__ keys,
-                   float* __restrict__ out, int tokens, int side, int half_dim, float minus_zero) {
+side_scores_kernel(const float* __restrict__ query, long long ld_q, const float* __restrict__ left_keys,
+                   const float* __restrict__ right_keys, float* __restrict__ left_out, float* __restrict__ right_out, int tokens,
+                   int side, int half_dim, float minus_zero) {
   pdl_begin();
+  const bool right = blockIdx.z == 1;
+  const float* keys = right ? right_keys : left_keys;
+  float* out = right ? right_out : left_out;
+  const int q_off = right ? half_dim : 0;
   // A product is formed as q*k + (-0), which rounds like q*k alone.  The compiler fuses a packed multiply and add; it cannot
   // know this addend.
   const float2 zero = both(minus_zero);
@@ -98,7 +103,7 @@ side_scores_kernel(const float* __restrict__ query, long long ld_q, int q_off, c
     }
     __syncthreads();
     const int jn = min(SS_J, half_dim - j0);
-    for (int j = 0; j < jn; ++j) {
+    auto step = [&](int j) {
       const float4 qa = *reinterpret_cast<const float4*>(&sq[j][ty * 8]);
       const float4 qb = *reinterpret_cast<const float4*>(&sq[j][ty * 8 + 4]);
       const float4 kv = *reinterpret_cast<const float4*>(&sk[j][tx * 4]);
@@ -108,6 +113,12 @@ side_scores_kernel(const float* __restrict__ query, long long ld_q, int q_off, c
         acc[a][0] = add2(acc[a][0], fma2(both(qv[a]), make_float2(kv.x, kv.y), zero));
         acc[a][1] = add2(acc[a][1], fma2(both(qv[a]), make_float2(kv.z, kv.w), zero));
       }
+    };
+    if (jn == SS_J) {
+#pragma unroll 8
+      for (int j = 0; j < SS_J; ++j) step(j);
+    } else {
+      for (int j = 0; j < jn; ++j) step(j);
     }
     __syncthreads();
   }
@@ -1113,12 +1124,13 @@ int hl_product_key_side_scores_f32(hl_ctx* ctx, const float* query, long long ld
   HL_REQUIRE(key_dim % 2 == 0, "product-key memory lookup requires even memory_key_dim, got " + std::to_string(key_dim));
   HL_REQUIRE(ld_query >= key_dim, "hl_product_key_side_scores_f32: query row stride smaller than key_dim");
   const int half = key_dim / 2;
-  dim3 grid(ceil_div(side, SS_K), ceil_div(tokens, SS_T));
-  pdl(side_scores_kernel, grid, 256, 0, ctx->stream)(query, ld_query, 0, left_keys, left_scores, tokens, side, half, -0.0f);
+  // Both tables in one launch: a second one would come in while the first runs, and its blocks, four to an SM, would sit on the few
+  // SMs that the first one leaves over (2048 tokens: 72 us a table instead of 43).
+  dim3 grid(ceil_div(side, SS_K), ceil_div(tokens, SS_T), 2);
+  pdl(side_scores_kernel, grid, 256, 0, ctx->stream)(query, ld_query, left_keys, right_keys, left_scores, right_scores, tokens, side,
+                                                     half, -0.0f);
   HL_LAUNCH_CHECK("side_scores_kernel");
-  pdl(side_scores_kernel, grid, 256, 0, ctx->stream)(query, ld_query, half, right_keys, right_scores, tokens, side, half, -0.0f);
-  HL_LAUNCH_CHECK("side_scores_kernel");
-  count_launch(ctx, 2);
+  count_launch(ctx);
   return HL_OK;
 }
 
