@@ -70,7 +70,8 @@ struct GraphKey {
            dynamic == o.dynamic;
   }
 };
-enum { GRAPH_STEP = 0, GRAPH_LOSS = 1, GRAPH_WINDOW = 2, GRAPH_DECODE = 3, GRAPH_DECODE_GREEDY = 4 };
+enum { GRAPH_STEP = 0, GRAPH_LOSS = 1, GRAPH_WINDOW = 2, GRAPH_DECODE = 3, GRAPH_DECODE_GREEDY = 4,
+       GRAPH_WINDOW_TO_HOST = 5 };
 struct GraphEntry {
   GraphKey key{};
   cudaGraphExec_t exec = nullptr;  // null until the sequence has run once plainly
@@ -203,7 +204,8 @@ struct hl_decoder {
   // state of the next one-token step
   int cached = 0;
   long long* decode_state = nullptr;       // device: position, token
-  GreedyPart* greedy = nullptr;            // device: the result, then the blocks' parts
+  float* row_logits = nullptr;             // where the logits of a single row go; null: m->logits
+  GreedyPart* greedy = nullptr;            // device: the blocks' parts
   long long* decode_state_host = nullptr;  // pinned
   GreedyPart* greedy_host = nullptr;       // pinned
   float* logits_host = nullptr;            // pinned, [vocab], allocated on first use
@@ -485,7 +487,7 @@ int plan_activations(hl_decoder* m, bool measure_only, size_t* bytes_out) {
   m->tokens = carve<int64_t>(cur, N);
   m->targets = carve<int64_t>(cur, N);
   m->decode_state = carve<long long>(cur, 2);
-  m->greedy = carve<GreedyPart>(cur, 1 + greedy_parts(c.vocab));
+  m->greedy = carve<GreedyPart>(cur, greedy_parts(c.vocab));
   m->loss_dev = carve<float>(cur, 4);
   m->norm_dev = carve<float>(cur, 4);
   m->norm_dev64 = carve<double>(cur, 2);
@@ -530,7 +532,7 @@ int plan_activations_f32(hl_decoder* m, bool measure_only, size_t* bytes_out) {
   m->tokens = carve<int64_t>(cur, N);
   m->targets = carve<int64_t>(cur, N);
   m->decode_state = carve<long long>(cur, 2);
-  m->greedy = carve<GreedyPart>(cur, 1 + greedy_parts(c.vocab));
+  m->greedy = carve<GreedyPart>(cur, greedy_parts(c.vocab));
   m->loss_dev = carve<float>(cur, 4);
   m->norm_dev = carve<float>(cur, 4);
   m->norm_dev64 = carve<double>(cur, 2);
@@ -697,7 +699,7 @@ int decode_head(hl_decoder* m, const void* x, int dtype) {
   g.w = dtype == HL_BF16 ? (const void*)(m->shadow + m->off_head_w) : (const void*)(m->params + m->off_head_w);
   g.w_dtype = dtype;
   g.bias = m->params + m->off_head_b;
-  g.out = m->logits; g.out_dtype = HL_F32;
+  g.out = m->row_logits ? m->row_logits : m->logits; g.out_dtype = HL_F32;
   g.n = m->cfg.vocab; g.k = m->cfg.d_model;
   return decode_gemv(m->ctx, g);
 }
@@ -2083,14 +2085,20 @@ int hl_decoder_eval_loss(hl_decoder* m, const int64_t* tokens_dev, const int64_t
 }
 
 // The row of logits that a pass left in m->logits, or with `greedy` only the choice out of it, on its way to the host.
+// A short row is written to pinned memory by the product itself, and so is the choice: no copy behind the last kernel.
+constexpr int kDirectVocab = 4096;
+struct RowTarget {
+  hl_decoder* m;
+  RowTarget(hl_decoder* model, bool greedy) : m(model) {
+    m->row_logits = !greedy && m->cfg.vocab <= kDirectVocab ? m->logits_host : nullptr;
+  }
+  ~RowTarget() { m->row_logits = nullptr; }
+};
 static int queue_result(hl_decoder* m, bool greedy) {
   hl_ctx* ctx = m->ctx;
-  if (greedy) {
-    HL_TRY(decode_greedy(ctx, m->logits, m->cfg.vocab, m->greedy + 1, m->greedy));
-    HL_CUDA(cudaMemcpyAsync(m->greedy_host, m->greedy, sizeof(GreedyPart), cudaMemcpyDeviceToHost, ctx->stream));
-  } else {
+  if (greedy) return decode_greedy(ctx, m->logits, m->cfg.vocab, m->greedy, m->greedy_host);
+  if (!m->row_logits)
     HL_CUDA(cudaMemcpyAsync(m->logits_host, m->logits, sizeof(float) * (size_t)m->cfg.vocab, cudaMemcpyDeviceToHost, ctx->stream));
-  }
   return HL_OK;
 }
 static int finish_result(hl_decoder* m, bool greedy) {
@@ -2104,11 +2112,12 @@ static int run_window(hl_decoder* m, const int64_t* window, cudaMemcpyKind kind,
   HL_REQUIRE(window_len <= m->cfg.context, "hl_decoder_next_token_logits: the window is longer than the model's context");
   hl_ctx* ctx = m->ctx;
   HL_TRY(ensure_logits_host(m));
+  const RowTarget target(m, greedy);
   HL_CUDA(cudaMemcpyAsync(m->tokens, window, sizeof(int64_t) * window_len, kind, ctx->stream));
   {
     ScopedShape shape(m, 1, window_len);
     m->decode_state_host[0] = window_len - 1;
-    HL_TRY(run_graphed(m, GRAPH_WINDOW, [m]() -> int {
+    HL_TRY(run_graphed(m, target.m->row_logits ? GRAPH_WINDOW_TO_HOST : GRAPH_WINDOW, [m]() -> int {
       HL_CUDA(cudaMemcpyAsync(m->decode_state, m->decode_state_host, sizeof(long long), cudaMemcpyHostToDevice, m->ctx->stream));
       return m->cfg.precision == HL_PRECISION_AMP_BF16 ? forward(m, Forward::last_position) : forward_f32(m, true);
     }));
@@ -2148,6 +2157,7 @@ static int run_next(hl_decoder* m, int64_t token, bool greedy) {
   m->decode_state_host[1] = token;
   const int position = m->cached;
   m->cached = 0;  // until this step has succeeded
+  const RowTarget target(m, greedy);
   auto queue = [m, ctx, greedy]() -> int {
     HL_CUDA(cudaMemcpyAsync(m->decode_state, m->decode_state_host, 2 * sizeof(long long), cudaMemcpyHostToDevice, ctx->stream));
     {
