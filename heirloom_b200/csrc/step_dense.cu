@@ -199,6 +199,7 @@ struct hl_decoder {
   // f32 route (reference f32 semantics: f32 tensors, f64 accumulation inside every op)
   struct F32Layer {
     float *a, *qkv, *probs, *o, *r, *c, *h, *g;
+    float *dy, *dr, *dqkv, *dwide;  // gradients of the block output, r, qkv and h; shared by the layers unless forked
   };
   // generation: how many positions of sequence 0 have their keys and values in the activation buffers (0: none) and the
   // state of the next one-token step
@@ -212,7 +213,7 @@ struct hl_decoder {
   GraphCache graphs;
   std::vector<float*> xf;  // residual stream per block input, f32
   std::vector<F32Layer> lf;
-  float *zf = nullptr, *dlogits_f = nullptr, *d_a = nullptr, *d_b = nullptr, *d_c = nullptr, *d_qkv = nullptr, *d_wide = nullptr;
+  float *zf = nullptr, *dlogits_f = nullptr, *d_a = nullptr, *d_c = nullptr;
 };
 
 namespace hl {
@@ -519,10 +520,19 @@ int plan_activations_f32(hl_decoder* m, bool measure_only, size_t* bytes_out) {
   m->logits = carve<float>(cur, N * V);
   m->dlogits_f = carve<float>(cur, N * V);
   m->d_a = carve<float>(cur, N * d);
-  m->d_b = carve<float>(cur, N * d);
   m->d_c = carve<float>(cur, N * d);
-  m->d_qkv = carve<float>(cur, N * 3 * d);
-  m->d_wide = carve<float>(cur, N * F);
+  m->fork_ok = !m->has_memory && N * (F + 5 * d) * sizeof(float) * L <= kForkBytes;  // (memory blocks share theirs)
+  for (size_t l = 0; l < L; ++l) {
+    hl_decoder::F32Layer& a = m->lf[l];
+    if (l > 0 && !m->fork_ok) {
+      a.dy = m->lf[0].dy; a.dr = m->lf[0].dr; a.dqkv = m->lf[0].dqkv; a.dwide = m->lf[0].dwide;
+      continue;
+    }
+    a.dy = m->fork_ok ? carve<float>(cur, N * d) : m->d_a;
+    a.dr = carve<float>(cur, N * d);
+    a.dqkv = carve<float>(cur, N * 3 * d);
+    a.dwide = carve<float>(cur, N * F);
+  }
   plan_memory_buffers(m, cur);
   // partial rows of a full batch of layer norms' parameter gradients (at most two CTAs per SM, two sums each)
   m->fold.capacity = (size_t)FoldBatch::kMaxJobs * (2 * (size_t)m->ctx->sm_count * 2 * d + 64);
@@ -1170,6 +1180,12 @@ int linear_backward_f32(hl_decoder* m, const float* x, const float* w, const flo
   g[1].out = dw; g[1].o_row = in; g[1].o_col = 1;
   g[1].m = out; g[1].n = in; g[1].k = rows;
   g[1].row_sum = db;
+  if (m->fork_ok && beside(m)) {  // the weight gradient beside whatever follows on the chain
+    HL_TRY(f64_gemm_run(m->ctx, g, 1));
+    SideStream side(m);
+    HL_TRY(side.rc);
+    return f64_gemm_run(m->ctx, g + 1, 1);
+  }
   return f64_gemm_run(m->ctx, g, 2);
 }
 
@@ -1236,8 +1252,7 @@ int backward_f32(hl_decoder* m) {
   };
   HL_TRY(cross_entropy_impl(ctx, m->logits, V, m->targets, N, V, 1.0f, m->loss_dev, nullptr, m->dlogits_f, HL_F32, V, m->loss_host));
   if (m->has_memory) HL_TRY(tables_are_zero(m));
-  float* dx = m->d_a;       // gradient of the residual stream
-  float* dx_next = m->d_b;
+  float* dx = m->lf[c.n_layers - 1].dy;  // gradient of the residual stream
   HL_TRY(linear_backward_f32(m, m->zf, P + m->off_head_w, m->dlogits_f, m->d_c, G + m->off_head_w, G + m->off_head_b, N, d, V));
   HL_TRY(layer_norm_backward_impl(ctx, m->xf[c.n_layers], HL_F32, P + m->off_lnf_g, m->d_c, nullptr, nullptr, nullptr, dx,
                                   nullptr, G + m->off_lnf_g, G + m->off_lnf_b, nullptr, N, d, fb));
@@ -1259,20 +1274,21 @@ int backward_f32(hl_decoder* m) {
       HL_TRY(linear_backward_f32(m, a.c, P + o.wq_m, m->m_dq, m->d_c, G + o.wq_m, G + o.bq_m, N, d, kd, F64_ACCUMULATE));
     } else {
       // y = r + fc2(gelu(fc1(ln2 r)))
-      HL_TRY(linear_backward_f32(m, a.g, P + o.w2, dx, m->d_wide, G + o.w2, G + o.b2, N, F, d, F64_DGELU, a.h));
-      HL_TRY(linear_backward_f32(m, a.c, P + o.w1, m->d_wide, m->d_c, G + o.w1, G + o.b1, N, d, F));
+      HL_TRY(linear_backward_f32(m, a.g, P + o.w2, dx, a.dwide, G + o.w2, G + o.b2, N, F, d, F64_DGELU, a.h));
+      HL_TRY(linear_backward_f32(m, a.c, P + o.w1, a.dwide, m->d_c, G + o.w1, G + o.b1, N, d, F));
     }
-    HL_TRY(layer_norm_backward_impl(ctx, a.r, HL_F32, P + o.ln2g, m->d_c, nullptr, nullptr, dx, dx_next, nullptr, G + o.ln2g,
+    HL_TRY(layer_norm_backward_impl(ctx, a.r, HL_F32, P + o.ln2g, m->d_c, nullptr, nullptr, dx, a.dr, nullptr, G + o.ln2g,
                                     G + o.ln2b, nullptr, N, d, fb));
-    std::swap(dx, dx_next);  // dL/dr
+    dx = a.dr;
     // r = x + out_proj(attention(q, k, v))
     HL_TRY(linear_backward_f32(m, a.o, P + o.wo, dx, m->d_c, G + o.wo, G + o.bo, N, d, d));
-    HL_TRY(attention_f64_backward(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, HL_F32, 3 * d, a.probs, m->d_c, d, m->d_qkv,
-                                  m->d_qkv + d, m->d_qkv + 2 * d, 3 * d, B, T, d, H));
-    HL_TRY(linear_backward_f32(m, a.a, P + o.wqkv, m->d_qkv, m->d_c, G + o.wqkv, G + o.bqkv, N, d, 3 * d));
+    HL_TRY(attention_f64_backward(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, HL_F32, 3 * d, a.probs, m->d_c, d, a.dqkv,
+                                  a.dqkv + d, a.dqkv + 2 * d, 3 * d, B, T, d, H));
+    HL_TRY(linear_backward_f32(m, a.a, P + o.wqkv, a.dqkv, m->d_c, G + o.wqkv, G + o.bqkv, N, d, 3 * d));
+    float* dx_next = l > 0 ? m->lf[l - 1].dy : m->d_a;
     HL_TRY(layer_norm_backward_impl(ctx, m->xf[l], HL_F32, P + o.ln1g, m->d_c, nullptr, nullptr, dx, dx_next, nullptr,
                                     G + o.ln1g, G + o.ln1b, nullptr, N, d, fb));
-    std::swap(dx, dx_next);
+    dx = dx_next;
     HL_TRY(finished(o.ln1b + d));
   }
   if (!m->has_memory) HL_TRY(tables_are_zero(m));
