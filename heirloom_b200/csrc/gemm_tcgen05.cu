@@ -1010,8 +1010,10 @@ static int check_gemm(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const v
 }
 
 // Whole tiles (of the whole contraction or of equal splits of it; not the dealt-out k blocks) can run on CTA pairs
-// with 256-row tiles.
+// with 256-row tiles.  Not an f32 result that reads bf16 rows (dGELU): a pair's epilogue works in the staging tile those rows
+// came into, and 64 columns of f32 results take twice that tile, over rows that have not been read yet.
 static bool pair_form(const hl_ctx* ctx, const hl_gemm_desc* d, const GemmPlan& plan, int sms) {
+  if (d->epilogue == HL_EPI_DGELU && d->out_dtype == HL_F32) return false;
   return plan.sk_tiles == 0 && d->m > BM && sms >= 2 && ctx->gemm_skip_kblock < 0 && pairs_enabled(d, plan.splits, sms);
 }
 

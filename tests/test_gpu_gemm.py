@@ -253,6 +253,25 @@ def test_tiles_handed_out_by_a_counter_give_the_same_bits_as_round_robin(monkeyp
     c.sync()
 
 
+@pytest.mark.parametrize("m,n,k", [(2500, 1544, 200), (4100, 776, 2104)])
+@pytest.mark.parametrize("b_mn", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_dgelu_epilogue_at_sizes_of_the_persistent_kernels(m, n, k, b_mn, dtype):
+    """C = acc * gelu'(h) with ragged rows and columns, too large for the small-product kernel, into both result types.  Bounds: the
+    f32 accumulation (2e-6 sqrt(k) of the largest product) times |gelu'| <= 1.13, the hardware tanh in gelu' (2e-3), and for a bf16
+    result half a step of it."""
+    from heirloom_b200 import cuda
+    c = ctx()
+    rng = np.random.default_rng(m + n)
+    a, b, da, db = operands(rng, m, n, k, False, b_mn)
+    h = ho.bf16_round(rng.standard_normal((m, n)) * 2.0)
+    out = cuda.gemm_bf16(c, da, db, m, n, k, cuda.K_MAJOR, cuda.MN_MAJOR if b_mn else cuda.K_MAJOR, epilogue=cuda.EPI_DGELU,
+                         aux_in=dev(h, torch.bfloat16), out_dtype=dtype)
+    acc = a @ b
+    want = acc * ho.gelu_backward(h, np.ones_like(h))
+    assert_close("dgelu", host(out), want, atol=(2e-3 + 2.3e-6 * np.sqrt(k)) * np.abs(acc).max(), rtol=0.0 if dtype is torch.float32 else 2 ** -8)
+
+
 PAIR_SCRIPT = r"""
 import numpy as np, torch
 from oracle import heirloom_oracle as ho
