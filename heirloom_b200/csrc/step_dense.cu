@@ -1320,11 +1320,13 @@ int backward_f32(hl_decoder* m) {
 template <typename F>
 int run_graphed(hl_decoder* m, int kind, F queue) {
   hl_ctx* ctx = m->ctx;
-  // collectives and per-kernel timing are host work of the step; the test hook changes a launch's arguments
-  if (nccl_active(ctx) || ctx->profiler || ctx->gemm_skip_kblock >= 0 || m->comm_pending) return queue();
   auto setting = [](const char* name) { const char* e = getenv(name); return e ? e[0] : '\0'; };
+  const char dynamic = setting("HEIRLOOM_GEMM_DYNAMIC");
+  // Collectives and per-kernel timing are host work of the step; the test hook changes a launch's arguments; and a launch that
+  // draws its tiles from the counter carries the counter's value, which no two launches share.
+  if (nccl_active(ctx) || ctx->profiler || ctx->gemm_skip_kblock >= 0 || m->comm_pending || dynamic == '1') return queue();
   const GraphKey key{kind, m->cfg.batch, m->cfg.context, ctx->workspace, ctx->workspace_bytes, ctx->wait_limit_ns, ctx->faults,
-                     setting("HEIRLOOM_GEMM_PAIRS"), setting("HEIRLOOM_GEMM_DYNAMIC")};
+                     setting("HEIRLOOM_GEMM_PAIRS"), dynamic};
   std::vector<GraphEntry>& entries = m->graphs.entries;
   GraphEntry* entry = nullptr;
   for (GraphEntry& e : entries)

@@ -194,3 +194,41 @@ def test_collected_weight_gradients_equal_those_of_two_half_batches():
         halves = (grads[1][name] + grads[2][name]) / 2
         tipped = 0 if name.startswith(("lm_head", "ln_f", "block.2")) else 2 ** -8 * 0.1 * (4 if "embedding" in name else 2)
         assert np.linalg.norm(whole - halves) <= (2 ** -24 * np.sqrt(18000) * 10 + tipped) * np.linalg.norm(halves), name
+
+
+def test_training_with_tiles_from_a_counter_equals_training_without(monkeypatch):
+    """HEIRLOOM_GEMM_DYNAMIC=1 over five training steps, more than the plain, the captured and a replayed pass would take: every
+    tile of the head's product (256 of 128 x 256, single CTAs) is computed in each of them.  Which CTA computes a
+    tile changes no bits; the products that the small-product kernel takes without the setting round alike but sum in another
+    order, which bf16 activations and AdamW's first steps turn into 1e-2 of a gradient at most."""
+    from heirloom_b200 import cuda, nn
+    c = ctx()
+    rng = np.random.default_rng(0)
+    tokens = torch.from_numpy(rng.integers(0, 4096, (5, 2, 16, 128))).cuda()
+    monkeypatch.setenv("HEIRLOOM_GEMM_PAIRS", "0")
+    state, runs = None, []
+    for dynamic in "01":
+        monkeypatch.setenv("HEIRLOOM_GEMM_DYNAMIC", dynamic)
+        model = nn.DecoderLm(c, nn.DecoderConfig(vocab=4096, d_model=128, n_layers=1, n_heads=2, d_ff=256, context=128, batch=16))
+        if state is None:
+            state = {n: (np.ones(s) if ".ln" in n or n.startswith("ln_f") else rng.standard_normal(s) * 0.05)
+                     for n, s in model.parameter_shapes().items()}
+        model.load_state_dict(state)
+        model.set_optimizer(lr=1e-2, weight_decay=0.0)
+        steps = []
+        for x, y in tokens:
+            model.forward_backward(x, y)
+            steps.append((model.loss(), model.grad("lm_head.weight")))
+            model.optimizer_step()
+        runs.append(steps)
+        model.close()
+    for step, ((want, want_grad), (got, got_grad)) in enumerate(zip(*runs)):
+        assert got == pytest.approx(want, rel=1e-3), step
+        assert np.linalg.norm(got_grad - want_grad) <= 2e-2 * np.linalg.norm(want_grad), step
+    # the host still knows the counter: an eager product computes all of its tiles as well
+    a = torch.randn(4096, 320, device="cuda").bfloat16()
+    b = torch.randn(2048, 320, device="cuda").bfloat16()
+    out = cuda.gemm_bf16(c, a, b, 4096, 2048, 320, out_dtype=torch.float32)
+    c.sync()
+    want = a.double() @ b.double().t()
+    assert (out.double() - want).abs().max() <= 2e-6 * np.sqrt(320) * want.abs().max()
