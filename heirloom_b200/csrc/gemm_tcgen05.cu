@@ -701,10 +701,11 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           if (mine) p.row_stats.target_logit[row] = z;
         }
         const float next = fmaxf(top, mx * kLog2e);
-        float2 sums = make_float2(below * ex2_fast(top - next), 0.f);
+        const float base = next == -INFINITY ? 0.f : next;  // all masked so far (-inf, or so low that log2 e times it is): sums of 0
+        float2 sums = make_float2(below * ex2_fast(top - base), 0.f);
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const float2 e = fma2(v[i], both(kLog2e), both(-next));
+          const float2 e = fma2(v[i], both(kLog2e), both(-base));
           sums = add2(sums, make_float2(ex2_fast(e.x), ex2_fast(e.y)));
         }
         top = next;

@@ -478,9 +478,10 @@ row_stats_loss_kernel(const GemmRowStats stats, int rows, int parts, int classes
       float next = top;
 #pragma unroll
       for (int u = 0; u < 8; ++u) next = fmaxf(next, v[u].x);
-      sum *= ex2_fast(top - next);
+      const float base = next == -INFINITY ? 0.f : next;  // nothing but masked columns so far
+      sum *= ex2_fast(top - base);
 #pragma unroll
-      for (int u = 0; u < 8; ++u) sum += v[u].y * ex2_fast(v[u].x - next);
+      for (int u = 0; u < 8; ++u) sum += v[u].y * ex2_fast(v[u].x - base);
       top = next;
     }
   }

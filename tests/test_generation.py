@@ -231,3 +231,26 @@ def test_evaluation_loss_equals_the_training_pass_loss(batch, vocab):
     whole = [model.eval_loss_device(x[i:i + 1], y[i:i + 1]) for i in range(batch)]
     assert np.mean(whole) == pytest.approx(want, rel=2e-6)
     model.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("masked", [-np.inf, -3.4e38])
+@pytest.mark.parametrize("vocab,columns", [(5000, np.arange(384, 416)), (5000, np.arange(2048)), (16384, np.arange(16384).reshape(-1, 8, 128)[:8, 1])])
+def test_evaluation_loss_with_masked_words(vocab, columns, masked):
+    """Words switched off by their head bias: the first 32 columns of a block of 128, sixteen whole blocks, and the 2nd, 10th, ... 58th
+    block of 128, which are what one warp of the loss kernel reads first.  They carry no probability; the loss is the training pass's."""
+    from heirloom_b200 import nn
+    from tests.gpu_util import ctx
+    c = ctx()
+    model = nn.DecoderLm(c, nn.DecoderConfig(vocab=vocab, d_model=128, n_layers=1, n_heads=2, d_ff=128, context=128, batch=32))
+    rng = np.random.default_rng(vocab)
+    state = {n: rng.standard_normal(s) * 0.2 for n, s in model.parameter_shapes().items()}
+    columns = columns.reshape(-1)
+    state["lm_head.bias"][columns] = masked
+    model.load_state_dict(state)
+    x = torch.from_numpy(rng.integers(0, vocab, (32, 128))).cuda()
+    y = torch.from_numpy(rng.choice(np.setdiff1d(np.arange(vocab), columns), (32, 128))).cuda()
+    model.forward_backward(x, y)
+    want, got = model.loss(), model.eval_loss_device(x, y)
+    model.close()
+    assert math.isfinite(want) and got == pytest.approx(want, rel=2e-6)
