@@ -2099,7 +2099,9 @@ int hl_decoder_eval_loss(hl_decoder* m, const int64_t* tokens_dev, const int64_t
     }));
     m->cached = 0;
   }
-  return hl_memcpy_d2h(m->ctx, loss_host, m->loss_dev, sizeof(float));
+  HL_CUDA(cudaMemcpyAsync(loss_host, m->loss_dev, sizeof(float), cudaMemcpyDeviceToHost, m->ctx->stream));
+  m->ctx->counters.d2h_bytes += sizeof(float);
+  return hl_ctx_sync(m->ctx);  // an id out of range or an expired wait: no loss
 }
 
 // The row of logits that a pass left in m->logits, or with `greedy` only the choice out of it, on its way to the host.
@@ -2119,8 +2121,10 @@ static int queue_result(hl_decoder* m, bool greedy) {
     HL_CUDA(cudaMemcpyAsync(m->logits_host, m->logits, sizeof(float) * (size_t)m->cfg.vocab, cudaMemcpyDeviceToHost, ctx->stream));
   return HL_OK;
 }
+// With the status words: a pass that gave up or met an id out of range has no result, and the graphs that hold its launches have to
+// be told (their launch numbers repeat, and a number that was not read stays behind).
 static int finish_result(hl_decoder* m, bool greedy) {
-  HL_CUDA(cudaStreamSynchronize(m->ctx->stream));
+  HL_TRY(hl_ctx_sync(m->ctx));
   m->ctx->counters.d2h_bytes += greedy ? sizeof(GreedyPart) : sizeof(float) * (size_t)m->cfg.vocab;
   return HL_OK;
 }

@@ -254,3 +254,50 @@ def test_evaluation_loss_with_masked_words(vocab, columns, masked):
     want, got = model.loss(), model.eval_loss_device(x, y)
     model.close()
     assert math.isfinite(want) and got == pytest.approx(want, rel=2e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [0, 1])
+def test_evaluation_and_generation_report_the_device_status(precision):
+    """Ids past the vocabulary, and products whose pipeline wait runs out (the bound shortened, one block left out, which the
+    GEMM returns from with its status): an error from the call itself, a fourth and a fifth time too (plain, captured and replayed
+    passes), nothing left for the next call, and the next passes are right."""
+    from heirloom_b200 import nn
+    from heirloom_b200._lib import HeirloomError
+    from tests.gpu_util import ctx
+    c = ctx()
+    model = nn.DecoderLm(c, nn.DecoderConfig(vocab=64, d_model=64, n_layers=2, n_heads=1, d_ff=128, context=16, batch=2, precision=precision))
+    rng = np.random.default_rng(3)
+    model.load_state_dict({n: rng.standard_normal(s) * 0.2 for n, s in model.parameter_shapes().items()})
+    good = torch.from_numpy(rng.integers(0, 64, (2, 16))).cuda()
+    bad = good.clone()
+    bad[1, 7] = 64
+    calls = [(lambda ids: model.eval_loss_device(ids, good), good, bad), (lambda ids: model.eval_loss_device(good, ids), good, bad),
+             (lambda ids: gen.next_token_logits(model, ids), [3, 63], [3, 64]),
+             (lambda ids: gen.generate_greedy(model, ids, 3, 10 ** 9), [3, 63], [3, 64]),
+             (lambda ids: model.prefill(np.array(ids, np.int64)), [3, 63], [3, 64])]
+    outcomes = []
+
+    def attempt(call, ids):
+        try:
+            return np.asarray(call(ids))
+        except HeirloomError as e:
+            return str(e)
+
+    for call, right, wrong in calls:
+        want = attempt(call, right)
+        errors = [attempt(call, wrong) for _ in range(5)]
+        outcomes.append((want, errors, attempt(call, right)))
+    if precision == nn.PRECISION_AMP_BF16:  # the f32 route's products have no waits
+        for call, right, _ in calls[:4]:
+            want = attempt(call, right)
+            c.set_test_hooks(wait_limit_ns=200_000, gemm_skip_kblock=0)
+            try:
+                error = attempt(call, right)
+            finally:
+                c.set_test_hooks(0, -1)
+            outcomes.append((want, [error], attempt(call, right)))
+    model.close()
+    for want, errors, after in outcomes:
+        assert all(isinstance(e, str) and ("out-of-range index" in e or "wait expired" in e) for e in errors), errors
+        assert not isinstance(want, str) and np.array_equal(after, want)
