@@ -1325,6 +1325,10 @@ int run_graphed(hl_decoder* m, int kind, F queue) {
   // Collectives and per-kernel timing are host work of the step; the test hook changes a launch's arguments; and a launch that
   // draws its tiles from the counter carries the counter's value, which no two launches share.
   if (nccl_active(ctx) || ctx->profiler || ctx->gemm_skip_kblock >= 0 || m->comm_pending || dynamic == '1') return queue();
+  // A caller that captures the context's stream gets the launches themselves.
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  HL_CUDA(cudaStreamIsCapturing(ctx->stream, &capturing));
+  if (capturing != cudaStreamCaptureStatusNone) return queue();
   const GraphKey key{kind, m->cfg.batch, m->cfg.context, ctx->workspace, ctx->workspace_bytes, ctx->wait_limit_ns, ctx->faults,
                      setting("HEIRLOOM_GEMM_PAIRS"), dynamic};
   std::vector<GraphEntry>& entries = m->graphs.entries;

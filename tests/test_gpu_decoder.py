@@ -232,3 +232,62 @@ def test_training_with_tiles_from_a_counter_equals_training_without(monkeypatch)
     c.sync()
     want = a.double() @ b.double().t()
     assert (out.double() - want).abs().max() <= 2e-6 * np.sqrt(320) * want.abs().max()
+
+
+def test_a_caller_may_capture_the_step():
+    """Forward, backward and AdamW inside a capture of the context's stream that the caller began, after one and three passes of its
+    own: a step each, whose replay leaves the parameters of a step that was not captured (scatter-adds and dQ reductions have
+    no fixed order: 1e-6 of a parameter's scale, and where a gradient is noise AdamW's step of at most lr)."""
+    import ctypes
+    from heirloom_b200 import nn
+    c = ctx()
+    rt = ctypes.CDLL("libcudart.so.12")
+    c.lib.hl_ctx_stream.restype = ctypes.c_void_p
+    stream = ctypes.c_void_p(c.lib.hl_ctx_stream(c.handle))
+    rng = np.random.default_rng(0)
+    x = torch.from_numpy(rng.integers(0, 256, (4, 64))).cuda()
+    y = torch.from_numpy(rng.integers(0, 256, (4, 64))).cuda()
+    torch.cuda.synchronize()
+    for precision in (nn.PRECISION_AMP_BF16, nn.PRECISION_F32):
+        state = None
+        for passes in (1, 3):
+            results = []
+            for captured in (False, True):
+                model = nn.DecoderLm(c, nn.DecoderConfig(vocab=256, d_model=128, n_layers=2, n_heads=2, d_ff=256, context=64, batch=4,
+                                                         precision=precision))
+                if state is None:
+                    state = {n: (np.ones(s) if ".ln" in n or n.startswith("ln_f") else rng.standard_normal(s) * 0.05)
+                             for n, s in model.parameter_shapes().items()}
+                model.load_state_dict(state)
+                model.set_optimizer(lr=1e-3)
+                for _ in range(passes):
+                    model.forward_backward(x, y)
+                c.sync()
+                error = None
+                if captured:
+                    graph, exe = ctypes.c_void_p(), ctypes.c_void_p()
+                    assert rt.cudaStreamBeginCapture(stream, 2) == 0  # relaxed
+                    try:
+                        model.train_step_device(x, y)
+                    except Exception as e:
+                        error = e
+                    ended = rt.cudaStreamEndCapture(stream, ctypes.byref(graph))
+                    if error is None and ended == 0:
+                        assert rt.cudaGraphInstantiate(ctypes.byref(exe), graph, ctypes.c_ulonglong(0)) == 0
+                        assert rt.cudaGraphLaunch(exe, stream) == 0
+                    c.sync()
+                    if exe:
+                        rt.cudaGraphExecDestroy(exe)
+                    if graph:
+                        rt.cudaGraphDestroy(graph)
+                    error = error or (ended or None)
+                else:
+                    model.train_step_device(x, y)
+                    c.sync()
+                results.append({n: model.parameter(n) for n in state})
+                model.close()
+                assert error is None, (precision, passes, error)
+            for n in state:
+                if not n.endswith("k_proj.bias"):  # its exact gradient is zero
+                    diff = np.abs(results[1][n] - results[0][n])
+                    assert np.mean(diff > 1e-6 * max(1.0, np.abs(results[0][n]).max())) <= 0.01 and diff.max() <= 2.1e-3, (precision, passes, n)
