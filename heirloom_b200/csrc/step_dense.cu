@@ -75,6 +75,7 @@ enum { GRAPH_STEP = 0, GRAPH_LOSS = 1, GRAPH_WINDOW = 2, GRAPH_DECODE = 3, GRAPH
 struct GraphEntry {
   GraphKey key{};
   cudaGraphExec_t exec = nullptr;  // null until the sequence has run once plainly
+  bool plain = false;              // it could not be captured
   Counters counts{};               // what a replay adds to the context's counters
   unsigned long long used = 0;
 };
@@ -1316,6 +1317,29 @@ int backward_f32(hl_decoder* m) {
   return HL_OK;
 }
 
+// The launches of `queue` as a graph on the device, or false with nothing queued and no error left behind (a device without memory
+// for it, say).
+template <typename F>
+bool capture_pass(hl_decoder* m, F queue, cudaGraphExec_t* exec) {
+  hl_ctx* ctx = m->ctx;
+  cudaGraph_t graph = nullptr;
+  bool ok = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+  if (ok) {
+    ok = queue() == HL_OK;
+    ok = cudaStreamEndCapture(ctx->stream, &graph) == cudaSuccess && ok;
+  }
+  ok = ok && cudaGraphInstantiate(exec, graph, 0) == cudaSuccess;
+  ok = ok && cudaGraphUpload(*exec, ctx->stream) == cudaSuccess;
+  if (graph) cudaGraphDestroy(graph);
+  if (!ok) {
+    if (*exec) cudaGraphExecDestroy(*exec);
+    *exec = nullptr;
+    m->forked = false;  // what was forked ended with the capture
+    cudaGetLastError();
+  }
+  return ok;
+}
+
 // Queues the launches of `queue` on the compute stream, from the second time on as a graph.
 template <typename F>
 int run_graphed(hl_decoder* m, int kind, F queue) {
@@ -1352,22 +1376,13 @@ int run_graphed(hl_decoder* m, int kind, F queue) {
     return HL_OK;
   }
   entry->used = ++m->graphs.clock;
+  if (entry->plain) return queue();
   if (!entry->exec) {
     const Counters before = ctx->counters;
-    cudaGraph_t graph = nullptr;
-    HL_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-    const int rc = queue();
-    const cudaError_t ended = cudaStreamEndCapture(ctx->stream, &graph);
-    if (rc != HL_OK) {
-      if (graph) cudaGraphDestroy(graph);
-      return rc;
-    }
-    HL_CUDA(ended);
-    const cudaError_t made = cudaGraphInstantiate(&entry->exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (made != cudaSuccess) {
-      entry->exec = nullptr;
-      return fail_cuda(made, "cudaGraphInstantiate");
+    if (!capture_pass(m, queue, &entry->exec)) {  // what cannot be captured runs as it did the first time, now and from now on
+      entry->plain = true;
+      ctx->counters = before;
+      return queue();
     }
     Counters& c = entry->counts;
     c.launches = ctx->counters.launches - before.launches;

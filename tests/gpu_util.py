@@ -1,4 +1,6 @@
 """Helpers shared by the GPU parity tests."""
+import contextlib
+
 import numpy as np
 import pytest
 import torch
@@ -35,3 +37,23 @@ def assert_close(name, got, want, atol=0.0, rtol=0.0):
     if not np.all(err <= bound):
         i = np.unravel_index(np.argmax(err - bound), err.shape)
         raise AssertionError(f"{name}: max violation at {i}: got {got[i]!r} want {want[i]!r} (err {err[i]:.3e})")
+
+
+@contextlib.contextmanager
+def full_device(leave=0):
+    """All but about `leave` bytes (and a megabyte) of the device's memory taken."""
+    held = [] if leave == 0 else [torch.empty(leave, dtype=torch.uint8, device="cuda")]
+    size = 1 << 34
+    while size >= 1 << 20:
+        try:
+            held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+        except torch.OutOfMemoryError:
+            size >>= 1
+    if leave:
+        held.pop(0)
+        torch.cuda.empty_cache()
+    try:
+        yield
+    finally:
+        held.clear()
+        torch.cuda.empty_cache()

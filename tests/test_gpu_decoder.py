@@ -1,10 +1,12 @@
 """Step-level parity of the decoder executor (amp-bf16 route) against the oracle's AMP restatement."""
+import contextlib
+
 import numpy as np
 import pytest
 import torch
 
 from oracle import heirloom_oracle as ho
-from tests.gpu_util import ctx
+from tests.gpu_util import ctx, full_device
 
 pytestmark = pytest.mark.gpu
 
@@ -291,3 +293,36 @@ def test_a_caller_may_capture_the_step():
                 if not n.endswith("k_proj.bias"):  # its exact gradient is zero
                     diff = np.abs(results[1][n] - results[0][n])
                     assert np.mean(diff > 1e-6 * max(1.0, np.abs(results[0][n]).max())) <= 0.01 and diff.max() <= 2.1e-3, (precision, passes, n)
+
+
+def test_passes_run_on_a_device_without_memory_for_their_graphs():
+    """Six models of twelve layers, no memory left on the device: more graphs than fit into what the driver still has.  A pass that
+    cannot be captured runs plainly, every time, with the same losses as in a device with room."""
+    from heirloom_b200 import nn
+    c = ctx()
+    rng = np.random.default_rng(0)
+    x = torch.from_numpy(rng.integers(0, 256, (4, 64))).cuda()
+    runs = []
+    for full in (False, True):
+        rng = np.random.default_rng(1)
+        models = []
+        for _ in range(6):
+            model = nn.DecoderLm(c, nn.DecoderConfig(vocab=256, d_model=128, n_layers=12, n_heads=2, d_ff=256, context=64, batch=4))
+            model.load_state_dict({n: rng.standard_normal(s) * 0.05 for n, s in model.parameter_shapes().items()})
+            model.forward_backward(x, x)
+            model.eval_loss_device(x, x)
+            models.append(model)
+        c.sync()
+        losses = []
+        with full_device() if full else contextlib.nullcontext():
+            for model in models:
+                for _ in range(3):
+                    try:
+                        model.forward_backward(x, x)
+                        losses += [model.loss(), model.eval_loss_device(x, x)]
+                    except Exception as e:
+                        losses.append(str(e))
+        for model in models:
+            model.close()
+        runs.append(losses)
+    assert runs[0] == runs[1]
