@@ -21,6 +21,7 @@ int fail(const std::string& msg) {
 }
 int fail_cuda(cudaError_t e, const char* what) {
   g_last_error = std::string("CUDA error in ") + what + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")";
+  cudaGetLastError();  // reported here, not by the launch check of whatever comes next
   return HL_ERR_CUDA;
 }
 

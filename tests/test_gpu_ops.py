@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from oracle import heirloom_oracle as ho
-from tests.gpu_util import assert_close, ctx, dev, host
+from tests.gpu_util import assert_close, ctx, dev, full_device, host
 
 pytestmark = pytest.mark.gpu
 F32_TOL = dict(atol=1e-6, rtol=2e-6)
@@ -406,3 +406,23 @@ def test_arange_and_concat_of_index_vectors():
     assert np.array_equal(host(got), np.concatenate([host(t) for t in parts]))
     with pytest.raises(HeirloomError, match="at least one input"):
         cuda.concat_i64(c, [])
+
+
+def test_an_allocation_that_failed_is_reported_once():
+    """A product whose split contraction wants 268 MB of scratch raises on a full device; the call after it does not."""
+    from heirloom_b200 import cuda
+    from heirloom_b200._lib import HeirloomError
+    a, b = torch.ones(4096, 512, device="cuda").bfloat16(), torch.ones(2048, 512, device="cuda").bfloat16()
+    out = torch.empty(4096, 2048, device="cuda")
+    cuda.gemm_bf16(ctx(), a[:256], b[:256], 256, 256, 512, out_dtype=torch.float32, split_k=8)  # the kernel is on the device
+    ctx().sync()
+    c = cuda.Context(0)  # no scratch yet
+    with full_device():
+        with pytest.raises(HeirloomError, match="out of memory"):
+            cuda.gemm_bf16(c, a, b, 4096, 2048, 512, out_dtype=torch.float32, split_k=8, out=out)
+    try:
+        cuda.gemm_bf16(c, a, b, 4096, 2048, 512, out_dtype=torch.float32, split_k=8, out=out)
+        c.sync()
+    finally:
+        c.close()
+    assert (out == 512.0).all()
