@@ -785,7 +785,6 @@ int forward(hl_decoder* m, Forward what = Forward::all) {
     HL_TRY(g.run(N, 3 * d, d, a.a, d, HL_K_MAJOR, W + o.wqkv, d, HL_K_MAJOR, a.qkv, 3 * d, HL_BF16, HL_EPI_BIAS, P + o.bqkv));
     if (what == Forward::last_position && last_block_by_row(m, l)) {
       HL_TRY(row_block(m, l, m->x[l] + (size_t)(N - 1) * d, false));
-      m->cached = 0;
       return decode_head(m, m->x[l + 1], HL_BF16);
     }
     if (m->flash_ok) HL_TRY(flash_attention_forward_impl(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, 3 * d, a.o, d, a.lse, B, T, H, d / H));
@@ -822,7 +821,6 @@ int forward(hl_decoder* m, Forward what = Forward::all) {
     HL_TRY(g.run(N, d, F, a.g, F, HL_K_MAJOR, W + o.w2, F, HL_K_MAJOR, m->x[l + 1], d, HL_BF16, HL_EPI_BIAS_RESIDUAL,
                  P + o.b2, a.r, d));
   }
-  m->cached = 0;
   if (what == Forward::last_position) return decode_head(m, m->x[c.n_layers] + (size_t)(N - 1) * d, HL_BF16);
   HL_TRY(layer_norm_forward_impl(ctx, m->x[c.n_layers], HL_BF16, P + m->off_lnf_g, P + m->off_lnf_b, m->z, HL_BF16, m->meanf,
                                  m->rstdf, N, d, 1e-5f));
@@ -1205,7 +1203,6 @@ int forward_f32(hl_decoder* m, bool last_only = false) {
     HL_TRY(forward_f32_gemm(m, linear_f32(a.a, P + o.wqkv, P + o.bqkv, a.qkv, N, d, 3 * d)));
     if (last_only && last_block_by_row(m, l)) {
       HL_TRY(row_block(m, l, m->xf[l] + (size_t)(N - 1) * d, false));
-      m->cached = 0;
       return decode_head(m, m->xf[l + 1], HL_F32);
     }
     HL_TRY(attention_f64_forward(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, HL_F32, 3 * d, a.o, d, a.probs, B, T, d, H));
@@ -1224,7 +1221,6 @@ int forward_f32(hl_decoder* m, bool last_only = false) {
       HL_TRY(forward_f32_gemm(m, linear_f32(a.g, P + o.w2, P + o.b2, m->xf[l + 1], N, F, d, F64_RESIDUAL, a.r)));
     }
   }
-  m->cached = 0;
   if (last_only) return decode_head(m, m->xf[c.n_layers] + (size_t)(N - 1) * d, HL_F32);
   HL_TRY(layer_norm_forward_impl(ctx, m->xf[c.n_layers], HL_F32, P + m->off_lnf_g, P + m->off_lnf_b, m->zf, HL_F32, nullptr,
                                  nullptr, N, d, 1e-5f));
@@ -1828,6 +1824,7 @@ int hl_decoder_forward_backward(hl_decoder* m, const int64_t* tokens_dev, const 
     HL_CUDA(cudaMemcpyAsync(m->tokens, tokens_dev, sizeof(int64_t) * m->N, cudaMemcpyDeviceToDevice, m->ctx->stream));
   if (targets_dev != m->targets)
     HL_CUDA(cudaMemcpyAsync(m->targets, targets_dev, sizeof(int64_t) * m->N, cudaMemcpyDeviceToDevice, m->ctx->stream));
+  m->cached = 0;  // the pass overwrites the cached rows from its first kernel on, whether or not it gets to its end
   HL_TRY(run_graphed(m, GRAPH_STEP, [m]() -> int {
     HL_TRY(zero_tables_beside(m));
     HL_TRY(prepare_token_rows(m));  // data parallel: the union of the ranks' token rows forms while forward runs
@@ -1840,7 +1837,6 @@ int hl_decoder_forward_backward(hl_decoder* m, const int64_t* tokens_dev, const 
     HL_TRY(prepare_value_rows(m));
     return backward_f32(m);
   }));
-  m->cached = 0;
   m->launches_last_step = m->ctx->counters.launches - before;
   return HL_OK;
 }
@@ -2110,13 +2106,13 @@ int hl_decoder_eval_loss(hl_decoder* m, const int64_t* tokens_dev, const int64_t
   HL_CUDA(cudaMemcpyAsync(m->targets, targets_dev, sizeof(int64_t) * n, cudaMemcpyDeviceToDevice, m->ctx->stream));
   {
     ScopedShape shape(m, sequences, m->cfg.context);
+    m->cached = 0;
     HL_TRY(run_graphed(m, GRAPH_LOSS, [m]() -> int {
       if (m->cfg.precision == HL_PRECISION_AMP_BF16) return forward(m, Forward::loss);
       HL_TRY(forward_f32(m));
       return cross_entropy_impl(m->ctx, m->logits, m->cfg.vocab, m->targets, m->N, m->cfg.vocab, 1.0f, m->loss_dev, nullptr,
                                 nullptr, HL_BF16, m->cfg.vocab);
     }));
-    m->cached = 0;
   }
   HL_CUDA(cudaMemcpyAsync(loss_host, m->loss_dev, sizeof(float), cudaMemcpyDeviceToHost, m->ctx->stream));
   m->ctx->counters.d2h_bytes += sizeof(float);
@@ -2157,12 +2153,12 @@ static int run_window(hl_decoder* m, const int64_t* window, cudaMemcpyKind kind,
   HL_CUDA(cudaMemcpyAsync(m->tokens, window, sizeof(int64_t) * window_len, kind, ctx->stream));
   {
     ScopedShape shape(m, 1, window_len);
+    m->cached = 0;
     m->decode_state_host[0] = window_len - 1;
     HL_TRY(run_graphed(m, target.m->row_logits ? GRAPH_WINDOW_TO_HOST : GRAPH_WINDOW, [m]() -> int {
       HL_CUDA(cudaMemcpyAsync(m->decode_state, m->decode_state_host, sizeof(long long), cudaMemcpyHostToDevice, m->ctx->stream));
       return m->cfg.precision == HL_PRECISION_AMP_BF16 ? forward(m, Forward::last_position) : forward_f32(m, true);
     }));
-    m->cached = 0;
   }
   HL_TRY(queue_result(m, greedy));
   return finish_result(m, greedy);

@@ -301,3 +301,28 @@ def test_evaluation_and_generation_report_the_device_status(precision):
     for want, errors, after in outcomes:
         assert all(isinstance(e, str) and ("out-of-range index" in e or "wait expired" in e) for e in errors), errors
         assert not isinstance(want, str) and np.array_equal(after, want)
+
+
+@pytest.mark.gpu
+def test_a_pass_that_ends_in_an_error_leaves_no_cache():
+    """A training pass that runs out of memory in its first block (its fc2 product, 20 x 4 tiles over a contraction of 12288, deals out
+    k blocks and wants 19 MB of scratch), after it has overwritten the block's q/k/v rows of a cached window."""
+    from heirloom_b200 import cuda, nn
+    from tests.gpu_util import ctx, full_device
+    ctx()
+    c = cuda.Context(0)  # no scratch yet
+    model = nn.DecoderLm(c, nn.DecoderConfig(vocab=64, d_model=1024, n_layers=1, n_heads=16, d_ff=12288, context=128, batch=20))
+    rng = np.random.default_rng(0)
+    model.load_state_dict({n: rng.standard_normal(s) * 0.02 for n, s in model.parameter_shapes().items()})
+    x = torch.from_numpy(rng.integers(0, 64, (20, 128))).cuda()
+    model.prefill(rng.integers(0, 64, 8))
+    raised = False
+    with full_device():
+        try:
+            model.forward_backward(x, x)
+        except Exception as e:
+            raised = "memory" in str(e)
+    cached = model.cached_positions
+    model.close()
+    c.close()
+    assert raised and cached == 0
