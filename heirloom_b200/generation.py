@@ -164,8 +164,9 @@ class _SamplingOptions(ctypes.Structure):
 
 
 def _sampling_options(o: GenerationOptions) -> _SamplingOptions:
+    # any number type is taken (ctypes wants Python's own); a top_k beyond 64 bits filters nothing
     return _SamplingOptions(o.temperature, 0.0 if o.top_p is None else o.top_p, o.repetition_penalty, o.frequency_penalty,
-                            o.presence_penalty, 0 if o.top_k is None else o.top_k)
+                            o.presence_penalty, 0 if o.top_k is None else min(int(o.top_k), 2 ** 63 - 1))
 
 
 def _sample(logits: np.ndarray, context: np.ndarray, o: GenerationOptions, rng: HeirloomRng) -> Tuple[int, float, float]:

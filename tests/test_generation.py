@@ -93,6 +93,17 @@ def test_native_sampling_follows_the_stated_rules(n):
             assert logp == pytest.approx(math.log(max(p, np.finfo(np.float64).tiny))) and a.state == b.state
 
 
+def test_sampling_options_of_any_number_type():
+    """NumPy integers and floats, and a top_k past 64 bits, are the options that Python's own numbers are."""
+    logits = np.random.default_rng(0).standard_normal(50)
+    for kind in (np.int64, np.int32, np.uint8):
+        o = gen.GenerationOptions(1, 0, temperature=np.float32(0.5), top_k=kind(3), top_p=np.float64(0.75), repetition_penalty=np.float32(1.25))
+        want = gen.GenerationOptions(1, 0, temperature=0.5, top_k=3, top_p=0.75, repetition_penalty=1.25)
+        assert gen.sample_token(logits, [1], o, gen.HeirloomRng(4)) == gen.sample_token(logits, [1], want, gen.HeirloomRng(4))
+    assert gen.sample_token(logits, [], gen.GenerationOptions(1, 0, temperature=1.0, top_k=2 ** 64 + 1), gen.HeirloomRng(9)) == \
+        gen.sample_token(logits, [], gen.GenerationOptions(1, 0, temperature=1.0), gen.HeirloomRng(9))
+
+
 def test_option_validation_messages():
     for kwargs, text in ((dict(temperature=-1.0), "temperature must be non-negative"), (dict(top_k=0), "top_k must be greater than zero"),
                          (dict(top_p=0.0), "top_p must be in"), (dict(repetition_penalty=0.5), "at least 1.0"),
