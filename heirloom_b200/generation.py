@@ -203,8 +203,8 @@ def generate(model, prefix: Sequence[int], options: GenerationOptions, rng: Heir
     if len(prefix) == 0:
         raise HeirloomError("generation prefix must contain at least one token")
     length = len(prefix)
-    tokens = np.empty(length + options.max_new_tokens, np.int64)
-    tokens[:length] = prefix
+    tokens = np.empty(length + min(options.max_new_tokens, 1024), np.int64)  # grows with what is generated, max_new_tokens may be "until eos"
+    tokens[:length] = [int(t) for t in prefix]
     steps: List[GeneratedTokenStep] = []
     reason = "max_new_tokens"
     native = _sampling_options(options)
@@ -218,6 +218,8 @@ def generate(model, prefix: Sequence[int], options: GenerationOptions, rng: Heir
         except HeirloomError:
             rng.state = state  # no token, no number drawn
             raise
+        if length == len(tokens):
+            tokens = np.concatenate([tokens, np.empty(length, np.int64)])
         tokens[length] = token
         length += 1
         steps.append(GeneratedTokenStep(token, p, logp))

@@ -104,6 +104,22 @@ def test_sampling_options_of_any_number_type():
         gen.sample_token(logits, [], gen.GenerationOptions(1, 0, temperature=1.0), gen.HeirloomRng(9))
 
 
+class Counting:
+    """A model whose next token is the count of tokens so far."""
+    def generate_token(self, tokens, length, appended, options, draw):
+        assert tokens[:length].tolist() == list(range(length)) and appended == (length > 3)
+        return length, 1.0, 0.0
+
+
+def test_generation_until_eos_has_no_bound_on_its_tokens():
+    """The token array grows with what is generated: a max_new_tokens that no memory would hold, an end after 2500 tokens; and a prefix of
+    one-element tensors."""
+    out = gen.generate(Counting(), [torch.tensor(0), np.int32(1), 2], gen.GenerationOptions(2 ** 60, 2499), gen.HeirloomRng(0))
+    assert out.finish_reason == "eos" and out.tokens == list(range(2500)) and out.new_token_count == 2497
+    out = gen.generate(Counting(), range(3), gen.GenerationOptions(1500, -1), gen.HeirloomRng(0))
+    assert out.finish_reason == "max_new_tokens" and out.tokens == list(range(1503))
+
+
 def test_option_validation_messages():
     for kwargs, text in ((dict(temperature=-1.0), "temperature must be non-negative"), (dict(top_k=0), "top_k must be greater than zero"),
                          (dict(top_p=0.0), "top_p must be in"), (dict(repetition_penalty=0.5), "at least 1.0"),
