@@ -198,6 +198,16 @@ def next_token_logits(model, tokens: Sequence[int]) -> np.ndarray:
     return out.astype(np.float64)
 
 
+def _generates_natively(model) -> bool:
+    """Whether a step may be one call into the library: not for a model of the caller's own that only gives logits, nor where the
+    caller has put something in front of the library's logits."""
+    from .nn import DecoderLm
+    logits = getattr(model, "next_token_logits_device", None)
+    if isinstance(model, DecoderLm):
+        return getattr(logits, "__func__", None) is DecoderLm.next_token_logits_device
+    return logits is None
+
+
 def generate(model, prefix: Sequence[int], options: GenerationOptions, rng: HeirloomRng) -> GenerationOutput:
     options.validate()
     if len(prefix) == 0:
@@ -207,17 +217,20 @@ def generate(model, prefix: Sequence[int], options: GenerationOptions, rng: Heir
     tokens[:length] = [int(t) for t in prefix]
     steps: List[GeneratedTokenStep] = []
     reason = "max_new_tokens"
-    native = _sampling_options(options)
+    native = _sampling_options(options) if _generates_natively(model) else None
     for step in range(options.max_new_tokens):
         # While everything fits in the context the window only grows at its end: its keys and values stay on the device and
         # a step computes one position.  Past the context every position shifts, and the whole window is run again.
-        state = rng.state
-        draw = rng.uniform_f32() if options.temperature != 0.0 else 0.0
-        try:
-            token, p, logp = model.generate_token(tokens, length, step > 0, native, draw)
-        except HeirloomError:
-            rng.state = state  # no token, no number drawn
-            raise
+        if native is None:
+            token, p, logp = _sample(next_token_logits(model, tokens[:length]), tokens[:length], options, rng)
+        else:
+            state = rng.state
+            draw = rng.uniform_f32() if options.temperature != 0.0 else 0.0
+            try:
+                token, p, logp = model.generate_token(tokens, length, step > 0, native, draw)
+            except HeirloomError:
+                rng.state = state  # no token, no number drawn
+                raise
         if length == len(tokens):
             tokens = np.concatenate([tokens, np.empty(length, np.int64)])
         tokens[length] = token

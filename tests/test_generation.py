@@ -120,6 +120,54 @@ def test_generation_until_eos_has_no_bound_on_its_tokens():
     assert out.finish_reason == "max_new_tokens" and out.tokens == list(range(1503))
 
 
+class OwnLogits:
+    """A model that is not the library's: the token after the last one, modulo 7, gets most of the probability."""
+    class cfg:
+        context = 4
+
+    def next_token_logits_device(self, window):
+        out = np.zeros(7, np.float32)
+        out[(int(window[-1]) + 1) % 7] = 5.0
+        return out
+
+
+def test_generation_over_a_model_that_only_gives_logits(monkeypatch):
+    monkeypatch.setattr(torch.Tensor, "cuda", lambda self: self)
+    out = gen.generate(OwnLogits(), [2, 3], gen.GenerationOptions(9, 10 ** 9), gen.HeirloomRng(0))
+    assert out.tokens == [2, 3, 4, 5, 6, 0, 1, 2, 3, 4, 5]
+    out = gen.generate(OwnLogits(), [2], gen.GenerationOptions(3, 10 ** 9, temperature=1.0, top_k=1), gen.HeirloomRng(7))
+    rng = gen.HeirloomRng(7)
+    [rng.uniform_f32() for _ in range(3)]
+    assert out.tokens == [2, 3, 4, 5] and out.rng_state == rng.state
+
+
+@pytest.mark.gpu
+def test_generation_asks_an_overridden_method_for_the_logits():
+    """A subclass, and an instance, that bans a token in next_token_logits_device: generate follows it."""
+    from heirloom_b200 import nn
+    from tests.gpu_util import ctx
+
+    class Banning(nn.DecoderLm):
+        def next_token_logits_device(self, window):
+            out = super().next_token_logits_device(window)
+            out[banned] = -100.0
+            return out
+
+    models = []
+    for kind in (nn.DecoderLm, Banning, nn.DecoderLm):
+        model = kind(ctx(), nn.DecoderConfig(vocab=64, d_model=64, n_layers=1, n_heads=1, d_ff=64, context=8, batch=1))
+        rng = np.random.default_rng(1)
+        model.load_state_dict({n: rng.standard_normal(s) * 0.3 for n, s in model.parameter_shapes().items()})
+        models.append(model)
+    banned = gen.generate_greedy(models[0], [1, 2], 1, -1)[-1]
+    plain = models[2].next_token_logits_device
+    models[2].next_token_logits_device = lambda window: np.where(np.arange(64) == banned, np.float32(-100.0), plain(window))
+    chains = [gen.generate_greedy(m, [1, 2], 6, -1) for m in models]
+    for m in models:
+        m.close()
+    assert banned in chains[0] and banned not in chains[1][2:] and chains[1] == chains[2]
+
+
 def test_option_validation_messages():
     for kwargs, text in ((dict(temperature=-1.0), "temperature must be non-negative"), (dict(top_k=0), "top_k must be greater than zero"),
                          (dict(top_p=0.0), "top_p must be in"), (dict(repetition_penalty=0.5), "at least 1.0"),
