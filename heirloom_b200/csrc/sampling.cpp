@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <exception>
 #include <limits>
 #include <string>
 #include <vector>
@@ -264,18 +265,16 @@ size_t ranked_prefix(std::vector<Candidate>& c, double mass) {
 
 }  // namespace
 bool all_finite_f32(const float* x, size_t n) { return vector_level() == 2 ? finite_avx512(x, n) : finite_plain(x, n); }
-}  // namespace hl
 
-extern "C" int hl_sample_token(const void* logits, int dtype, long long vocab, const int64_t* context, long long n_context,
-                               const hl_sampling_options* o, double draw, int64_t* token, double* probability,
-                               double* log_probability) {
-  using namespace hl;
+namespace {
+int sample_token(const void* logits, int dtype, long long vocab, const int64_t* context, long long n_context, const hl_sampling_options* o,
+                 double draw, int64_t* token, double* probability, double* log_probability) {
   HL_REQUIRE(logits && o && token && probability && log_probability && (context || n_context == 0), "hl_sample_token: null argument");
   HL_REQUIRE(vocab > 0 && n_context >= 0, "hl_sample_token: requires at least one logit");
   HL_REQUIRE(dtype == HL_F32 || dtype == HL_F64, "hl_sample_token: logits must be f32 or f64");
   const size_t n = (size_t)vocab, padded = (n + LANES - 1) / LANES * LANES;
   static thread_local std::vector<double> x, p;  // grown to the largest vocabulary seen
-  if (x.size() < padded) { x.resize(padded); p.resize(padded); }
+  if (p.size() < padded) { x.resize(padded); p.resize(padded); }
   const bool penalties = o->repetition_penalty > 1.0 || o->frequency_penalty != 0.0 || o->presence_penalty != 0.0;
   if (dtype == HL_F32) {  // divided by the temperature on the way when nothing comes between
     const float* src = static_cast<const float*>(logits);
@@ -400,4 +399,16 @@ extern "C" int hl_sample_token(const void* logits, int dtype, long long vocab, c
   *probability = prob;
   *log_probability = std::log(std::max(prob, std::numeric_limits<double>::min()));
   return HL_OK;
+}
+}  // namespace
+}  // namespace hl
+
+extern "C" int hl_sample_token(const void* logits, int dtype, long long vocab, const int64_t* context, long long n_context,
+                               const hl_sampling_options* o, double draw, int64_t* token, double* probability,
+                               double* log_probability) {
+  try {
+    return hl::sample_token(logits, dtype, vocab, context, n_context, o, draw, token, probability, log_probability);
+  } catch (const std::exception& e) {  // memory for the row's working copies; callers in C cannot catch it
+    return hl::fail(std::string("hl_sample_token: ") + e.what());
+  }
 }

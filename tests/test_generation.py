@@ -168,6 +168,29 @@ def test_generation_asks_an_overridden_method_for_the_logits():
     assert banned in chains[0] and banned not in chains[1][2:] and chains[1] == chains[2]
 
 
+HUGE_ROW = """
+import ctypes
+from heirloom_b200 import _lib, generation as gen
+lib = _lib.load()
+o = gen._sampling_options(gen.GenerationOptions(1, 0))
+row, t, p, lp = (ctypes.c_double * 8)(), ctypes.c_int64(), ctypes.c_double(), ctypes.c_double()
+for vocab in (1 << 60, 1 << 50):
+    rc = lib.hl_sample_token(row, 2, ctypes.c_longlong(vocab), None, ctypes.c_longlong(0), ctypes.byref(o), ctypes.c_double(0.0),
+                             ctypes.byref(t), ctypes.byref(p), ctypes.byref(lp))
+    assert rc != 0
+print(lib.hl_last_error().decode())
+"""
+
+
+def test_a_row_that_no_memory_holds_is_an_error_and_no_abort():
+    import subprocess
+    import sys
+    from pathlib import Path
+    res = subprocess.run([sys.executable, "-c", HUGE_ROW], cwd=str(Path(__file__).resolve().parents[1]), capture_output=True, text=True,
+                         timeout=120)
+    assert res.returncode == 0 and "hl_sample_token" in res.stdout, (res.returncode, res.stdout, res.stderr)
+
+
 def test_option_validation_messages():
     for kwargs, text in ((dict(temperature=-1.0), "temperature must be non-negative"), (dict(top_k=0), "top_k must be greater than zero"),
                          (dict(top_p=0.0), "top_p must be in"), (dict(repetition_penalty=0.5), "at least 1.0"),
