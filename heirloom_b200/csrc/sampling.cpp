@@ -30,7 +30,8 @@ HL_INLINE void load_lanes(Lanes* v, const double* p) { __builtin_memcpy(v, p, si
 // *y = e^*x for *x <= 0: x = n ln2 + r, |r| <= ln2/2, the Taylor polynomial of degree 13 (its remainder is 4e-18 of e^r) and
 // n added to the exponent.  Below -708 the result is 0; those terms are 1e-308 of the largest one.
 HL_INLINE void exp_lanes(const Lanes* x, Lanes* y) {
-  constexpr double kLog2e = 1.4426950408889634074, kLn2Hi = 6.93147180369123816490e-01, kLn2Lo = 1.90821492927058770002e-10;
+  // ln2 in two parts (Cody and Waite): rounded to f32, so that its product with a whole number below 2^29 is exact, and the rest
+  constexpr double kLog2e = 1.4426950408889634074, kLn2Hi = 0.693147182464599609375, kLn2Lo = -1.904654299957768e-09;
   constexpr double kShift = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer in the low bits
   const Words tiny = *x < -708.0;
   const Lanes zero = *x * 0.0;
