@@ -174,6 +174,10 @@ int decode_greedy(hl_ctx* ctx, const float* logits, int vocab, GreedyPart* parts
 bool all_finite_f32(const float* x, size_t n);
 int decode_embed(hl_ctx* ctx, const float* table, const float* positions, const long long* state, void* out, int dtype, int dim);
 
+// hl_product_key_topk_from_side_scores whose choices go to rows *kept_row and on of `kept` as well (null: nowhere else).
+int product_key_topk_impl(hl_ctx* ctx, const float* left_scores, const float* right_scores, int64_t* out, int tokens, int side, int top_k,
+                          int beam, int64_t* kept, const long long* kept_row);
+
 struct AdamPlan;
 int adam_plan_create(hl_ctx* ctx, const hl_adamw_tensor* tensors, int count, AdamPlan** out);
 void adam_plan_destroy(AdamPlan* plan);

@@ -158,7 +158,8 @@ __device__ __forceinline__ float okey_value(unsigned k) {
 template <int PER_LANE>
 __global__ void __launch_bounds__(128)
 product_key_topk_kernel(const float* __restrict__ left, const float* __restrict__ right, int64_t* __restrict__ out,
-                        int tokens, int side, int top_k, int beam, int* __restrict__ status) {
+                        int tokens, int side, int top_k, int beam, int* __restrict__ status, int64_t* __restrict__ kept,
+                        const long long* __restrict__ kept_row) {
   pdl_begin();
   __shared__ unsigned s_hist[4][256];
   __shared__ unsigned s_key[4][32];
@@ -290,7 +291,11 @@ product_key_topk_kernel(const float* __restrict__ left, const float* __restrict_
   for (int r = 0; r < top_k; ++r) {
     const unsigned m = __reduce_max_sync(full, head_key);
     if (m == 0u) {
-      if (lane == 0) { atomicExch(status + ST_BAD_ARGUMENT, 1); out[(size_t)token * top_k + r] = 0; }
+      if (lane == 0) {
+        atomicExch(status + ST_BAD_ARGUMENT, 1);
+        out[(size_t)token * top_k + r] = 0;
+        if (kept) kept[(*kept_row + token) * top_k + r] = 0;
+      }
       continue;
     }
     const unsigned bs = __reduce_min_sync(full, head_key == m ? head_slot : 0xffffffffu);
@@ -298,7 +303,10 @@ product_key_topk_kernel(const float* __restrict__ left, const float* __restrict_
       used |= 1u << head_j;
       advance();
     }
-    if (lane == 0) out[(size_t)token * top_k + r] = (long long)bs;
+    if (lane == 0) {
+      out[(size_t)token * top_k + r] = (long long)bs;
+      if (kept) kept[(*kept_row + token) * top_k + r] = (long long)bs;
+    }
   }
 }
 
@@ -1113,6 +1121,26 @@ int check_memory_dims(int tokens, int top_k, int dim, const char* who) {
 
 using namespace hl;
 
+namespace hl {
+int product_key_topk_impl(hl_ctx* ctx, const float* left_scores, const float* right_scores, int64_t* out, int tokens, int side, int top_k,
+                          int beam, int64_t* kept, const long long* kept_row) {
+  HL_REQUIRE(ctx && left_scores && right_scores && out, "hl_product_key_topk_from_side_scores: null argument");
+  HL_REQUIRE(tokens > 0 && side > 0, "hl_product_key_topk_from_side_scores: requires non-zero tokens/side");
+  HL_REQUIRE(side <= 2048, "hl_product_key_topk_from_side_scores: side must be at most 2048");
+  HL_REQUIRE(beam > 0 && beam <= 32 && beam <= side, "hl_product_key_topk_from_side_scores: beam must be in [1, min(32, side)]");
+  HL_REQUIRE(top_k > 0 && top_k <= beam * beam, "hl_product_key_topk_from_side_scores: top_k must be in [1, beam^2]");
+  if (side <= 512)
+    pdl(product_key_topk_kernel<16>, ceil_div(tokens, 4), 128, 0, ctx->stream)(left_scores, right_scores, out, tokens, side,
+                                                                              top_k, beam, ctx->status_dev, kept, kept_row);
+  else
+    pdl(product_key_topk_kernel<PK_MAX_PER_LANE>, ceil_div(tokens, 4), 128, 0, ctx->stream)(
+        left_scores, right_scores, out, tokens, side, top_k, beam, ctx->status_dev, kept, kept_row);
+  HL_LAUNCH_CHECK("product_key_topk_kernel");
+  count_launch(ctx);
+  return HL_OK;
+}
+}  // namespace hl
+
 extern "C" {
 
 int hl_topk_rows_f32(hl_ctx* ctx, const float* scores, int64_t* out, int rows, int cols, int k) {
@@ -1146,20 +1174,7 @@ int hl_product_key_side_scores_f32(hl_ctx* ctx, const float* query, long long ld
 
 int hl_product_key_topk_from_side_scores(hl_ctx* ctx, const float* left_scores, const float* right_scores, int64_t* out,
                                          int tokens, int side, int top_k, int beam) {
-  HL_REQUIRE(ctx && left_scores && right_scores && out, "hl_product_key_topk_from_side_scores: null argument");
-  HL_REQUIRE(tokens > 0 && side > 0, "hl_product_key_topk_from_side_scores: requires non-zero tokens/side");
-  HL_REQUIRE(side <= 2048, "hl_product_key_topk_from_side_scores: side must be at most 2048");
-  HL_REQUIRE(beam > 0 && beam <= 32 && beam <= side, "hl_product_key_topk_from_side_scores: beam must be in [1, min(32, side)]");
-  HL_REQUIRE(top_k > 0 && top_k <= beam * beam, "hl_product_key_topk_from_side_scores: top_k must be in [1, beam^2]");
-  if (side <= 512)
-    pdl(product_key_topk_kernel<16>, ceil_div(tokens, 4), 128, 0, ctx->stream)(left_scores, right_scores, out, tokens, side,
-                                                                              top_k, beam, ctx->status_dev);
-  else
-    pdl(product_key_topk_kernel<PK_MAX_PER_LANE>, ceil_div(tokens, 4), 128, 0, ctx->stream)(
-        left_scores, right_scores, out, tokens, side, top_k, beam, ctx->status_dev);
-  HL_LAUNCH_CHECK("product_key_topk_kernel");
-  count_launch(ctx);
-  return HL_OK;
+  return hl::product_key_topk_impl(ctx, left_scores, right_scores, out, tokens, side, top_k, beam, nullptr, nullptr);
 }
 
 int hl_product_key_split_rows(hl_ctx* ctx, const int64_t* rows, int64_t* left, int64_t* right, long long n, int side) {

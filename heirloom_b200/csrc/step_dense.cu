@@ -196,6 +196,7 @@ struct hl_decoder {
   int* m_union_count = nullptr;      // device count of them
   int* m_union_count_host = nullptr; // pinned mirror
   int union_n = -1;                  // rows in the union after the last exchange, -1 before any
+  int64_t* decode_idx = nullptr;  // selections of a one-token step
   int64_t *m_sel_all = nullptr, *m_sel_left = nullptr, *m_sel_right = nullptr;  // concatenated selections of all memory blocks
   // f32 route (reference f32 semantics: f32 tensors, f64 accumulation inside every op)
   struct F32Layer {
@@ -386,6 +387,7 @@ void plan_memory_buffers(hl_decoder* m, uint8_t*& cur) {
   m->m_sel_all = carve<int64_t>(cur, all);
   m->m_sel_left = carve<int64_t>(cur, all);
   m->m_sel_right = carve<int64_t>(cur, all);
+  m->decode_idx = carve<int64_t>(cur, k);
 }
 
 // Operand copies of a step whose weight gradients may run beside the chain of input gradients: what a model of a few
@@ -667,20 +669,23 @@ int weight_gradient(hl_decoder* m, const __nv_bfloat16* dy, int n_out, const __n
 // ---- memory feed-forward core (both routes): lookup, re-scoring, softmax, weighted value -----------
 // query [N, key_dim] f32 is already in ma[l].query (MemoryFeedForward::forward_named,
 // src/memory_transformer.rs:742-781).
-int memory_core_forward(hl_decoder* m, int l) {
+// In a one-token step the block's selections of the window stay, with this position's in the position's row, as a full-window
+// pass would leave them: they are read by others.
+int memory_core_forward(hl_decoder* m, int l, bool one_token = false) {
   hl_ctx* ctx = m->ctx;
   MemoryActs& a = m->ma[l];
+  int64_t* idx = one_token ? m->decode_idx : a.idx;
   const float* P = m->params;
   const int N = m->N, kd = m->mem.key_dim, vd = m->mem.value_dim, k = m->mem.top_k, side = m->side;
   const int beam = std::min(side, std::max(k, (int)ceil(sqrt((double)k))));  // product_key_beam, :2014-2016
   // timed as one family ("other" in the per-kernel profile); work = table rows gathered, in bytes
   ProfileScope prof(ctx, HL_PROF_OTHER, (double)N * k * (double)(kd + vd) * 4.0 + 2.0 * (double)N * side * 4.0);
   HL_TRY(hl_product_key_side_scores_f32(ctx, a.query, kd, P + m->off_kl, P + m->off_kr, m->m_ls, m->m_rs, N, side, kd));
-  HL_TRY(hl_product_key_topk_from_side_scores(ctx, m->m_ls, m->m_rs, a.idx, N, side, k, beam));
-  HL_TRY(hl_memory_selected_scores_forward(ctx, a.idx, a.query, kd, P + m->off_kl, P + m->off_kr, m->m_scores, N, k, side, kd,
+  HL_TRY(product_key_topk_impl(ctx, m->m_ls, m->m_rs, idx, N, side, k, beam, one_token ? a.idx : nullptr, m->decode_state));
+  HL_TRY(hl_memory_selected_scores_forward(ctx, idx, a.query, kd, P + m->off_kl, P + m->off_kr, m->m_scores, N, k, side, kd,
                                            m->mem.slots));
   HL_TRY(hl_softmax_rows_f32(ctx, m->m_scores, a.weights, N, k));
-  return hl_memory_weighted_value_forward(ctx, a.idx, a.weights, P + m->off_val, a.weighted, N, k, m->mem.slots, vd);
+  return hl_memory_weighted_value_forward(ctx, idx, a.weights, P + m->off_val, a.weighted, N, k, m->mem.slots, vd);
 }
 
 // dweighted -> m_dq (gradient of the query) and the table gradients (added into the arena).
@@ -1431,7 +1436,7 @@ int decode_step(hl_decoder* m) {
         return decode_gemv(ctx, p);
       };
       HL_TRY(project(r, dt, o.wq_m, o.bq_m, ma.query, HL_F32, kd, d, GV_STORE, nullptr, true));
-      HL_TRY(memory_core_forward(m, l));
+      HL_TRY(memory_core_forward(m, l, true));
       HL_TRY(project(r, dt, o.wg_m, o.bg_m, ma.gate, HL_F32, vd, d, GV_GELU, nullptr, true));
       HL_TRY(hl_binary_f32(ctx, HL_MUL, ma.weighted, ma.gate, ma.mv, (size_t)vd));
       HL_TRY(project(ma.mv, HL_F32, o.wout_m, o.bout_m, next, dt, d, vd, GV_RESIDUAL, r, false));

@@ -424,3 +424,43 @@ def test_a_pass_that_ends_in_an_error_leaves_no_cache():
     model.close()
     c.close()
     assert raised and cached == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("memory_layers", [(0, 1), (0,)])
+def test_routing_after_one_token_steps_is_the_window_s(memory_layers):
+    """selected_indices and memory_access_counts after a window of five tokens and seven one-token steps, and after generate, are what
+    the last full-window pass over the same tokens leaves (f32 queries to the rounding of f64 sums: no near-ties here)."""
+    from heirloom_b200 import nn
+    from tests.gpu_util import ctx
+    c = ctx()
+    mem = dict(memory_layers=memory_layers, slots=64, key_dim=32, value_dim=32, top_k=4)
+    model = nn.DecoderLm(c, nn.DecoderConfig(vocab=72, d_model=128, n_layers=2, n_heads=2, d_ff=200, context=16, batch=1,
+                                             precision=nn.PRECISION_F32), nn.MemoryConfig(**mem))
+    rng = np.random.default_rng(5)
+    model.load_state_dict({n: (np.ones(s) if ".ln" in n or n.startswith("ln_f") else rng.standard_normal(s) * 0.3)
+                           for n, s in model.parameter_shapes().items()})
+    read = lambda: ([model.selected_indices(l).copy() for l in memory_layers], model.memory_access_counts().row_counts)
+    stream = rng.integers(0, 72, 12)
+    gen.next_token_logits(model, stream)
+    want = read()
+    gen.next_token_logits(model, rng.integers(0, 72, 16))
+    model.prefill(stream[:5])
+    for t in stream[5:]:
+        model.decode_next(int(t))
+    got = [a[:12] for a in read()[0]]
+    out = gen.generate_greedy(model, stream[:3], 9, -1)
+    after = [a[:11] for a in read()[0]]
+    gen.next_token_logits(model, out[:11])
+    window = [a[:11] for a in read()[0]]
+    gen.next_token_logits(model, stream)
+    model.prefill(stream[:5])
+    for t in stream[5:]:
+        model.decode_next(int(t))
+    counts = read()[1]
+    gen.next_token_logits(model, stream)
+    want_counts = read()[1]
+    model.close()
+    assert all(np.array_equal(g, w[:12]) for g, w in zip(got, want[0]))
+    assert all(np.array_equal(g, w) for g, w in zip(after, window))
+    assert np.array_equal(counts, want_counts)
