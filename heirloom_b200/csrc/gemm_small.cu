@@ -29,13 +29,14 @@ struct GsSizes {
   static constexpr int STAGE_BYTES = GS_A_BYTES + BN * GS_BK * 2;   // 24 / 32 KB
   static constexpr int DATA = STAGES * STAGE_BYTES;
   static constexpr int LD = BN + 4;                                 // accumulator rows in shared memory: conflict-free writes
-  static_assert((GS_BM * LD + GS_BM) * 4 <= DATA, "the accumulator reuses the stages");
-  static constexpr int ONES = 2048;                                 // 16 x 64 bf16 of 1.0: the right operand of the row sums
-  static constexpr int TAIL = DATA + ONES;                          // barriers
+  static constexpr int SUMS = GS_BM * LD * 4;                       // behind it the row sums of the two halves of every k block
+  static constexpr int ACC_BYTES = SUMS + 2 * GS_BM * 8;
+  static_assert(ACC_BYTES <= DATA && ACC_BYTES % 16 == 0, "the accumulator reuses the stages");
+  static constexpr int TAIL = DATA;                                 // barriers
   // The residual or pre-activation rows of the tile: a place of their own where one CTA has the SM, else in the stages, behind the
   // accumulator.
   static constexpr int CTAS_PER_SM = DATA <= 104 * 1024 ? 2 : 1;
-  static constexpr int AUX = CTAS_PER_SM == 1 ? TAIL + 256 : ((GS_BM * LD + GS_BM) * 4 + 15) / 16 * 16;
+  static constexpr int AUX = CTAS_PER_SM == 1 ? TAIL + 256 : ACC_BYTES;
   static constexpr int AUX_BYTES = GS_BM * BN * 2;
   static constexpr int SMEM = CTAS_PER_SM == 1 ? AUX + AUX_BYTES : TAIL + 256;  // base aligned to 1024 bytes, as the kernel checks
   static_assert(CTAS_PER_SM == 1 || AUX + AUX_BYTES <= DATA, "the rows fit behind the accumulator");
@@ -56,7 +57,7 @@ struct GsParams {
   long long ldc;
   __nv_bfloat16* aux_out;
   long long ld_aux_out;
-  float* row_sum;  // [m] or null: sum over the contraction of A's rows
+  float* row_sum;  // [m] or null: sum over the contraction of A's rows (A MN-major)
   int* status;
 };
 
@@ -78,10 +79,16 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const int m0 = (tile % p.m_tiles) * GS_BM, n0 = (tile / p.m_tiles) * BN;
   const int kb0 = rank * p.k_blocks_per_rank, kb1 = min(p.k_blocks, kb0 + p.k_blocks_per_rank);
 
+  // Row sums (a bias gradient beside its weight gradient): in the tiles of the first column four warps that have nothing to do
+  // until the epilogue add up A's stages as they pass, four values in f32, the rest in f64, which is no further off than column sums by
+  // themselves: 16384 tokens 5.8e-8 of the terms' magnitudes at most, those 4.2e-7, and 1.7e-5 when they were a product with a block
+  // of ones, whose f32 sums the tensor core cuts off at every step.  (256-token model's step 186 -> 179 us without those products.)
+  const bool sums = A_MN && p.row_sum != nullptr && n0 == 0;
+  constexpr int SUM_WARP0 = 4, SUM_WARPS = 4;
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       tc05::mbar_init(&tail->full[s], 1);
-      tc05::mbar_init(&tail->empty[s], 1);
+      tc05::mbar_init(&tail->empty[s], sums ? 1 + SUM_WARPS : 1);
     }
     tc05::mbar_init(&tail->done, 1);
     tail->abort_flag = (tc05::smem_u32(smem) & 1023u) == 0 ? 0 : 1;
@@ -89,16 +96,10 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     tc05::tma_prefetch_desc(&map_a);
     tc05::tma_prefetch_desc(&map_b);
   }
-  // Row sums (a bias gradient beside its weight gradient): the tiles of the first column multiply A by a block of ones as
-  // well, sixteen more columns of tensor memory.
-  const bool sums = p.row_sum != nullptr && n0 == 0;
   if (warp == 1) {
-    tc05::tmem_alloc(&tail->tmem_base, 2 * BN);
+    tc05::tmem_alloc(&tail->tmem_base, BN);
     tc05::tmem_relinquish();
   }
-  if (sums && threadIdx.x >= 128)
-    reinterpret_cast<uint4*>(smem + Z::DATA)[threadIdx.x - 128] = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
-  tc05::fence_proxy_async_smem();
   tc05::tc_fence_before_sync();
   __syncthreads();
   tc05::tc_fence_after_sync();
@@ -155,8 +156,6 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   } else if (warp == 1) {
     if (tc05::elect_one()) {
       constexpr uint32_t idesc = tc05::instr_desc_bf16_f32(GS_BM, BN, A_MN, B_MN);
-      constexpr uint32_t idesc_sums = tc05::instr_desc_bf16_f32(GS_BM, 16, A_MN, false);
-      const uint64_t ones = tc05::smem_desc_sw128(tc05::smem_u32(smem + Z::DATA), 16, 1024);
       bool ok = true;
       for (int kb = kb0; kb < kb1; ++kb) {
         const int i = kb - kb0, stage = i % STAGES;
@@ -170,11 +169,33 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           const uint64_t db = B_MN ? tc05::smem_desc_sw128(sb + ks * (16 * 128), GS_BK * 128, 1024)
                                    : tc05::smem_desc_sw128(sb + ks * 32, 16, 1024);
           tc05::umma_ss(tmem, da, db, idesc, (i > 0 || ks > 0) ? 1u : 0u);
-          if (sums) tc05::umma_ss(tmem + BN, da, ones, idesc_sums, (i > 0 || ks > 0) ? 1u : 0u);
         }
         tc05::umma_commit(&tail->empty[stage]);
       }
       if (ok) tc05::umma_commit(&tail->done);
+    }
+  }
+  // This lane's two rows of A (columns in memory: a stage holds two blocks of 64, token by token, 128-byte swizzle), over 32 of a
+  // stage's 64 tokens; tokens past the end are zeros.
+  double row_sum[2] = {0.0, 0.0};
+  const int sum_block = warp & 1, sum_half = (warp >> 1) & 1;
+  if (sums && warp >= SUM_WARP0) {
+    for (int kb = kb0; kb < kb1; ++kb) {
+      const int i = kb - kb0, stage = i % STAGES;
+      if (!tc05::mbar_wait(&tail->full[stage], (uint32_t)(i / STAGES) & 1u, abort_flag, p.wait_limit_ns)) break;
+      const uint8_t* block = smem + stage * Z::STAGE_BYTES + sum_block * (GS_BK * 128);
+#pragma unroll 4
+      for (int t = sum_half * 32; t < sum_half * 32 + 32; t += 4) {
+        float2 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          v[u] = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(block + (t + u) * 128 + (((lane >> 2) ^ ((t + u) & 7)) << 4) + (lane & 3) * 4));
+        const float2 four = add2(add2(v[0], v[1]), add2(v[2], v[3]));
+        row_sum[0] += (double)four.x;
+        row_sum[1] += (double)four.y;
+      }
+      __syncwarp();
+      if (lane == 0) tc05::mbar_arrive(&tail->empty[stage]);
     }
   }
 
@@ -204,22 +225,16 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         *reinterpret_cast<uint4*>(acc + r * Z::LD + c0 + i) = make_uint4(bits[i], bits[i + 1], bits[i + 2], bits[i + 3]);
     }
   }
-  float* acc_sums = acc + GS_BM * Z::LD;
-  if (sums && warp < 4) {
-    uint32_t bits[8];
-    if (have) {
-      tc05::tmem_ld_32x32b_x8(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)BN, bits);
-      tc05::tmem_ld_wait();
-    }
-    acc_sums[warp * 32 + lane] = have ? __uint_as_float(bits[0]) : 0.f;
-  }
+  double* acc_sums = reinterpret_cast<double*>(smem + Z::SUMS);  // [half][row]
+  if (sums && warp >= SUM_WARP0)
+    *reinterpret_cast<double2*>(acc_sums + sum_half * GS_BM + sum_block * 64 + lane * 2) = make_double2(row_sum[0], row_sum[1]);
   if (need_aux) asm volatile("cp.async.wait_all;" ::: "memory");
   tc05::tc_fence_before_sync();
   cg::cluster_group cluster = cg::this_cluster();
   if (p.splits > 1) cluster.sync(); else __syncthreads();
   if (warp == 1) {
     tc05::tc_fence_after_sync();
-    tc05::tmem_dealloc(tmem, 2 * BN);
+    tc05::tmem_dealloc(tmem, BN);
   }
   // a rolled loop, because a CTA that lands on an SM which has not run this kernel yet pays for every cache line of its code
 #pragma unroll 1
@@ -263,10 +278,11 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       *reinterpret_cast<float4*>(static_cast<float*>(p.c) + (size_t)row * p.ldc + col) = make_float4(v[0], v[1], v[2], v[3]);
   }
   if (sums && threadIdx.x < rows_mine && m0 + row_first + (int)threadIdx.x < p.m) {
-    float v = 0.f;
-    float* at = acc_sums + row_first + threadIdx.x;
-    for (int s = 0; s < p.splits; ++s) v += p.splits > 1 ? *cluster.map_shared_rank(at, s) : *at;
-    p.row_sum[m0 + row_first + threadIdx.x] = v;
+    double v = 0.0;
+    double* at = acc_sums + row_first + threadIdx.x;
+    for (int s = 0; s < p.splits; ++s)
+      for (int half = 0; half < 2; ++half) v += p.splits > 1 ? *cluster.map_shared_rank(at + half * GS_BM, s) : at[half * GS_BM];
+    p.row_sum[m0 + row_first + threadIdx.x] = (float)v;
   }
   if (p.splits > 1) cluster.sync();  // no CTA leaves while another still reads its sums
   if (!ok || *abort_flag) {

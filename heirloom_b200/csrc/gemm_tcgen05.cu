@@ -1224,7 +1224,7 @@ int gemm_bf16_row_sums(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const 
   if (rc != HL_OK) return rc;
   const int sms = persistent_sms(ctx);
   const GemmSmallPlan small = small_plan(ctx, d, gemm_plan(d, sms), sms);
-  if (small.splits == 0) return HL_OK;
+  if (small.splits == 0 || d->a_layout != HL_MN_MAJOR) return HL_OK;
   *done = true;
   return gemm_small_run(ctx, d, small, a, b, c, nullptr, nullptr, nullptr, row_sum);
 }

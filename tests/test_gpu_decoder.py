@@ -326,3 +326,29 @@ def test_passes_run_on_a_device_without_memory_for_their_graphs():
             model.close()
         runs.append(losses)
     assert runs[0] == runs[1]
+
+
+@pytest.mark.parametrize("batch,d_model,d_ff,layers", [(3, 64, 8, 1), (16, 64, 8, 1), (100, 128, 256, 1)])
+def test_bias_gradients_of_many_tokens_are_column_sums(batch, d_model, d_ff, layers):
+    """The head's bias gradient beside its weight gradient, against the f64 sums of the same bf16 dlogits (3072, 16384 and 102400 tokens
+    of one logit row each, made by the same loss kernel).  Four values at a time are added in f32, two roundings, the rest in
+    f64, rounded once as a part and once as the result: 4 x 2^-24 of the terms' magnitudes."""
+    from heirloom_b200 import cuda, nn
+    c = ctx()
+    vocab, time = 64, 1024
+    rng = np.random.default_rng(batch)
+    model = nn.DecoderLm(c, nn.DecoderConfig(vocab=vocab, d_model=d_model, n_layers=layers, n_heads=d_model // 64, d_ff=d_ff, context=time,
+                                             batch=batch))
+    state = {n: np.zeros(s, np.float32) for n, s in model.parameter_shapes().items()}  # every token's logits are the head's bias
+    state["lm_head.bias"] = rng.standard_normal(vocab).astype(np.float32) * 3
+    model.load_state_dict(state)
+    x = torch.from_numpy(rng.integers(0, vocab, (batch, time))).cuda()
+    y = torch.from_numpy(rng.integers(0, vocab, (batch, time))).cuda()
+    model.forward_backward(x, y)
+    got = model.grad("lm_head.bias").astype(np.float64)
+    model.close()
+    logits = torch.from_numpy(np.tile(state["lm_head.bias"], (batch * time, 1))).cuda()
+    _, dlogits = cuda.cross_entropy(c, logits, y.reshape(-1), dlogits_dtype=torch.bfloat16)
+    c.sync()
+    want, magnitude = dlogits.double().sum(0).cpu().numpy(), dlogits.double().abs().sum(0).cpu().numpy()
+    assert (np.abs(got - want) <= 4 * 2.0 ** -24 * magnitude).all(), (np.abs(got - want) / magnitude).max()
