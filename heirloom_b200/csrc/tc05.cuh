@@ -238,6 +238,13 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr) {
                : "memory");
 }
 
+// The same for the barriers at this address in both CTAs of the pair.
+__device__ __forceinline__ void umma_commit_pair_both(const uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+               "h"((uint16_t)3)
+               : "memory");
+}
+
 // Tensor-memory load: this warp's 32 lanes x 32 consecutive f32 columns; thread t gets lane
 // (warp%4)*32+t.  taddr = (lane << 16) | column.
 __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&r)[32]) {

@@ -328,11 +328,13 @@ def test_passes_run_on_a_device_without_memory_for_their_graphs():
     assert runs[0] == runs[1]
 
 
-@pytest.mark.parametrize("batch,d_model,d_ff,layers", [(3, 64, 8, 1), (16, 64, 8, 1), (100, 128, 256, 1)])
-def test_bias_gradients_of_many_tokens_are_column_sums(batch, d_model, d_ff, layers):
-    """The head's bias gradient beside its weight gradient, against the f64 sums of the same bf16 dlogits (3072, 16384 and 102400 tokens
-    of one logit row each, made by the same loss kernel).  Four values at a time are added in f32, two roundings, the rest in
-    f64, rounded once as a part and once as the result: 4 x 2^-24 of the terms' magnitudes."""
+@pytest.mark.parametrize("batch,d_model,d_ff,layers,roundings", [(3, 64, 8, 1, 4), (16, 64, 8, 1, 4), (100, 128, 256, 1, 4),
+                                                                (16, 128, 512, 12, 12), (5, 768, 3072, 5, 12)])
+def test_bias_gradients_of_many_tokens_are_column_sums(batch, d_model, d_ff, layers, roundings):
+    """The head's bias gradient beside its weight gradient, against the f64 sums of the same bf16 dlogits (3072 to 102400 tokens of one
+    logit row each, made by the same loss kernel); a product of its own, and one of a group of layers' (the last two).  Four values
+    at a time are added in f32, two roundings (in a group eight such sums one after the other, eight more), the rest in
+    f64, rounded once as a part and once as the result: that many times 2^-24 of the terms' magnitudes."""
     from heirloom_b200 import cuda, nn
     c = ctx()
     vocab, time = 64, 1024
@@ -351,4 +353,4 @@ def test_bias_gradients_of_many_tokens_are_column_sums(batch, d_model, d_ff, lay
     _, dlogits = cuda.cross_entropy(c, logits, y.reshape(-1), dlogits_dtype=torch.bfloat16)
     c.sync()
     want, magnitude = dlogits.double().sum(0).cpu().numpy(), dlogits.double().abs().sum(0).cpu().numpy()
-    assert (np.abs(got - want) <= 4 * 2.0 ** -24 * magnitude).all(), (np.abs(got - want) / magnitude).max()
+    assert (np.abs(got - want) <= roundings * 2.0 ** -24 * magnitude).all(), (np.abs(got - want) / magnitude).max()
