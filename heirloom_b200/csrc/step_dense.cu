@@ -126,6 +126,7 @@ struct hl_decoder {
   int64_t *tokens = nullptr, *targets = nullptr;
   // Weight gradients beside the backward's chain of input gradients (they depend on it, nothing depends on them): on a second
   // stream, reading operands that every layer has its own copy of.
+  bool lean = false;  // neither of the two below: no copies of operands
   bool fork_ok = false;
   cudaStream_t side_stream = nullptr;
   cudaEvent_t fork_event = nullptr, join_event = nullptr;
@@ -451,8 +452,8 @@ int plan_activations(hl_decoder* m, bool measure_only, size_t* bytes_out) {
   m->dtmp = carve<float>(cur, N * d);
   m->dob = carve<__nv_bfloat16>(cur, N * d);
   m->dxb0 = carve<__nv_bfloat16>(cur, N * d);  // gradient of the embeddings' sum: written like a block output's, read by nobody
-  m->fork_ok = N * (F + 5 * d) * 2 * L <= kForkBytes;
-  m->group_layers = m->fork_ok ? 0 : plan_group_layers(m);
+  m->fork_ok = !m->lean && N * (F + 5 * d) * 2 * L <= kForkBytes;
+  m->group_layers = m->lean || m->fork_ok ? 0 : plan_group_layers(m);
   {
     // one set of gradients per layer, per layer of a group, or for all; a group's last layer writes the next one's dy already
     const size_t sets = m->fork_ok ? L : std::max(1, m->group_layers), dy_sets = m->fork_ok ? L : std::min(L, sets + (m->group_layers > 0));
@@ -524,7 +525,7 @@ int plan_activations_f32(hl_decoder* m, bool measure_only, size_t* bytes_out) {
   m->dlogits_f = carve<float>(cur, N * V);
   m->d_a = carve<float>(cur, N * d);
   m->d_c = carve<float>(cur, N * d);
-  m->fork_ok = !m->has_memory && N * (F + 5 * d) * sizeof(float) * L <= kForkBytes;  // (memory blocks share theirs)
+  m->fork_ok = !m->lean && !m->has_memory && N * (F + 5 * d) * sizeof(float) * L <= kForkBytes;  // (memory blocks share theirs)
   for (size_t l = 0; l < L; ++l) {
     hl_decoder::F32Layer& a = m->lf[l];
     if (l > 0 && !m->fork_ok) {
@@ -1644,11 +1645,32 @@ static int decoder_create_impl(hl_ctx* ctx, const hl_decoder_config* cfg, const 
   HL_ALLOC(m->v, fb)
   HL_ALLOC(m->shadow, sizeof(__nv_bfloat16) * m->arena)
   size_t act = 0;
-  if (amp) plan_activations(m, true, &act); else plan_activations_f32(m, true, &act);
+  auto plan = [&](bool measure_only) { if (amp) plan_activations(m, measure_only, &act); else plan_activations_f32(m, measure_only, &act); };
+  // Copies of operands for weight gradients beside or behind the backward pass (up to 256 MB, or a gigabyte) are only made where the
+  // device has a gigabyte left behind them and behind the attention's scratch, so that a model fits wherever it did without them;
+  // and not beside a communicator, which uses none of them.
+  m->lean = nccl_active(ctx);
+  plan(true);
+  if (m->fork_ok || m->group_layers > 0) {
+    const size_t scores = (size_t)cfg->batch * cfg->n_heads * cfg->context * cfg->context * sizeof(float);
+    const size_t behind = kGroupBytes + (amp && m->flash_ok ? flash_attention_backward_scratch_bytes(cfg->batch, cfg->context, cfg->n_heads,
+                                                                                                    cfg->d_model / cfg->n_heads) : scores);
+    size_t free_bytes = 0, total_bytes = 0;
+    e = cudaMemGetInfo(&free_bytes, &total_bytes);
+    if (e != cudaSuccess) return cleanup(fail_cuda(e, "cudaMemGetInfo"));
+    if (free_bytes < act + behind || cudaMalloc(reinterpret_cast<void**>(&m->act_arena), act) != cudaSuccess) {
+      cudaGetLastError();
+      m->act_arena = nullptr;
+      m->lean = true;
+      plan(true);
+    }
+  }
   m->act_bytes = act;
-  HL_ALLOC(m->act_arena, act)
+  if (!m->act_arena) {
+    HL_ALLOC(m->act_arena, act)
+  }
 #undef HL_ALLOC
-  if (amp) plan_activations(m, false, &act); else plan_activations_f32(m, false, &act);
+  plan(false);
   cudaMemsetAsync(m->params, 0, fb, ctx->stream);
   cudaMemsetAsync(m->grads, 0, fb, ctx->stream);
   cudaMemsetAsync(m->m, 0, fb, ctx->stream);

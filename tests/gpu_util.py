@@ -41,7 +41,10 @@ def assert_close(name, got, want, atol=0.0, rtol=0.0):
 
 @contextlib.contextmanager
 def full_device(leave=0):
-    """All but about `leave` bytes (and a megabyte) of the device's memory taken."""
+    """All but about `leave` bytes (and a megabyte) of the device's memory taken, what the driver's pool holds for stream-ordered
+    allocations included."""
+    import ctypes
+    runtime, pooled = ctypes.CDLL("libcudart.so.12"), []
     held = [] if leave == 0 else [torch.empty(leave, dtype=torch.uint8, device="cuda")]
     size = 1 << 34
     while size >= 1 << 20:
@@ -49,11 +52,21 @@ def full_device(leave=0):
             held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
         except torch.OutOfMemoryError:
             size >>= 1
+    while True:
+        block = ctypes.c_void_p()
+        if runtime.cudaMallocAsync(ctypes.byref(block), ctypes.c_size_t(1 << 20), None) != 0:
+            runtime.cudaGetLastError()
+            break
+        pooled.append(block)
     if leave:
         held.pop(0)
         torch.cuda.empty_cache()
+    torch.cuda.synchronize()
     try:
         yield
     finally:
         held.clear()
+        for block in pooled:
+            runtime.cudaFreeAsync(block, None)
+        torch.cuda.synchronize()
         torch.cuda.empty_cache()
