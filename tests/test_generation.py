@@ -408,11 +408,17 @@ def test_a_pass_that_ends_in_an_error_leaves_no_cache():
     from heirloom_b200 import cuda, nn
     from tests.gpu_util import ctx, full_device
     ctx()
-    c = cuda.Context(0)  # no scratch yet
-    model = nn.DecoderLm(c, nn.DecoderConfig(vocab=64, d_model=1024, n_layers=1, n_heads=16, d_ff=12288, context=128, batch=20))
     rng = np.random.default_rng(0)
-    model.load_state_dict({n: rng.standard_normal(s) * 0.02 for n, s in model.parameter_shapes().items()})
     x = torch.from_numpy(rng.integers(0, 64, (20, 128))).cuda()
+    for warm in (True, False):  # a kernel whose first launch finds no memory stays unusable in its process: all of them run once before
+        c = cuda.Context(0)  # no scratch yet
+        model = nn.DecoderLm(c, nn.DecoderConfig(vocab=64, d_model=1024, n_layers=1, n_heads=16, d_ff=12288, context=128, batch=20))
+        model.load_state_dict({n: rng.standard_normal(s) * 0.02 for n, s in model.parameter_shapes().items()})
+        if warm:
+            model.forward_backward(x, x)
+            c.sync()
+            model.close()
+            c.close()
     model.prefill(rng.integers(0, 64, 8))
     raised = False
     with full_device():
