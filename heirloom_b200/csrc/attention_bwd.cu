@@ -574,11 +574,7 @@ int flash_attention_backward_impl(hl_ctx* ctx, const void* q, const void* k, con
     if ((rc = make_tensor_map(&mdv, HL_BF16, 3, dv, dims, strides, box, 64)) != HL_OK) return rc;
   }
   if (head_dim == 64) {
-    static bool configured = false;
-    if (!configured) {
-      HL_CUDA(cudaFuncSetAttribute(flash_attention_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FB_SMEM_BYTES));
-      configured = true;
-    }
+    HL_ALLOW_SHARED(ctx, FB_SMEM_BYTES, flash_attention_bwd_kernel);
     const int grid = std::min(nq * batch * n_heads, persistent_sms(ctx));
     pdl(flash_attention_bwd_kernel, grid, FB_THREADS, FB_SMEM_BYTES, ctx->stream)(mq, mk, mv, mdo, mdq, mdk, mdv, p);
   } else {

@@ -423,11 +423,7 @@ flash_attention_bwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
 
 int launch_attention_bwd128(hl_ctx* ctx, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
                             const CUtensorMap& mdq, const CUtensorMap& mdk, const CUtensorMap& mdv, const FbParams& p) {
-  static bool configured = false;
-  if (!configured) {
-    HL_CUDA(cudaFuncSetAttribute(flash_attention_bwd128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FW_SMEM));
-    configured = true;
-  }
+  HL_ALLOW_SHARED(ctx, FW_SMEM, flash_attention_bwd128_kernel);
   const int items = ceil_div(p.T, FW_BN) * p.B * p.H;
   pdl(flash_attention_bwd128_kernel, std::min(items, persistent_sms(ctx)), FW_THREADS, FW_SMEM, ctx->stream)(mq, mk, mv, mdo, mdq, mdk,
                                                                                                           mdv, p);

@@ -437,18 +437,10 @@ int flash_attention_forward_impl(hl_ctx* ctx, const void* q, const void* k, cons
   // causal algorithmic work: QK^T and PV over the lower triangle
   ProfileScope prof(ctx, HL_PROF_ATTENTION_FWD, 2.0 * batch * n_heads * (double)time * time * head_dim);
   if (head_dim == 64) {
-    static bool configured = false;
-    if (!configured) {
-      HL_CUDA(cudaFuncSetAttribute(flash_attention_fwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, FaSizes<64>::SMEM_BYTES));
-      configured = true;
-    }
+    HL_ALLOW_SHARED(ctx, FaSizes<64>::SMEM_BYTES, flash_attention_fwd_kernel<64>);
     pdl(flash_attention_fwd_kernel<64>, grid, FA_THREADS, FaSizes<64>::SMEM_BYTES, ctx->stream)(mq, mk, mv, mo, p);
   } else {
-    static bool configured = false;
-    if (!configured) {
-      HL_CUDA(cudaFuncSetAttribute(flash_attention_fwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, FaSizes<128>::SMEM_BYTES));
-      configured = true;
-    }
+    HL_ALLOW_SHARED(ctx, FaSizes<128>::SMEM_BYTES, flash_attention_fwd_kernel<128>);
     pdl(flash_attention_fwd_kernel<128>, grid, FA_THREADS, FaSizes<128>::SMEM_BYTES, ctx->stream)(mq, mk, mv, mo, p);
   }
   HL_LAUNCH_CHECK("flash_attention_fwd_kernel");

@@ -10,6 +10,7 @@
 #include <utility>
 #include <algorithm>
 #include "../../include/heirloom_b200.h"
+#include "per_device.h"
 
 namespace hl {
 
@@ -28,6 +29,15 @@ int fail_cuda(cudaError_t e, const char* what);
 #define HL_REQUIRE(cond, msg)                                             \
   do {                                                                    \
     if (!(cond)) return ::hl::fail(std::string(msg));                     \
+  } while (0)
+
+// Lets a kernel have that much dynamic shared memory on the context's device.
+#define HL_ALLOW_SHARED(ctx, bytes, ...)                                                                            \
+  do {                                                                                                              \
+    static ::hl::PerDevice _allowed;                                                                                \
+    HL_CUDA(_allowed.once((ctx)->device, [&] {                                                                      \
+      return cudaFuncSetAttribute(__VA_ARGS__, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes));          \
+    }));                                                                                                            \
   } while (0)
 
 #define HL_LAUNCH_CHECK(name)                                             \
@@ -126,6 +136,24 @@ cudaError_t launch_pdl_split(int shared_percent, void (*kernel)(P...), dim3 grid
 template <typename... P, typename... A>
 cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, A&&... args) {
   return launch_pdl_split(-1, kernel, grid, block, smem, stream, cluster, std::forward<A>(args)...);
+}
+
+// How many clusters of a kernel the current device holds at once; 0 when it cannot be told.
+template <typename... P>
+int resident_clusters(void (*kernel)(P...), int cluster, int threads, size_t smem) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(cluster * 1024));
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)cluster; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess) return n;
+  cudaGetLastError();
+  return 0;
 }
 
 constexpr double kStreamingBytes = 16e6;

@@ -494,11 +494,7 @@ int launch_decode_attention(hl_ctx* ctx, const T* qkv, long long ld, const long 
                       (reinterpret_cast<uintptr_t>(qkv) & 15) == 0;
   if (staged) smem += rows;
   auto kern = decode_attention_kernel<T, Acc>;
-  static bool configured = false;
-  if (!configured) {
-    HL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024));
-    configured = true;
-  }
+  HL_ALLOW_SHARED(ctx, 110 * 1024, kern);
   HL_CUDA(launch_pdl(kern, n_heads * DA_CTAS, DA_THREADS, smem, ctx->stream, DA_CTAS, qkv, ld, channels, pos, out, hd, cap, staged,
                      settled));
   count_launch(ctx);

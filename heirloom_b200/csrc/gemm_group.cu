@@ -331,23 +331,10 @@ int gemm_group_run(hl_ctx* ctx, const WeightGradJob* jobs, int count, int tokens
   p.k_blocks = ceil_div(tokens, GG_BK);
   p.wait_limit_ns = ctx->wait_limit_ns ? ctx->wait_limit_ns : tc05::kWaitLimitNs;
   p.status = ctx->status_dev;
-  static int resident_pairs = 0;  // a GPC with an odd number of SMs leaves one out
-  if (resident_pairs == 0) {
-    HL_CUDA(cudaFuncSetAttribute(gemm_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GG_SMEM));
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(ctx->sm_count & ~1));
-    cfg.blockDim = dim3(GG_THREADS);
-    cfg.dynamicSmemBytes = GG_SMEM;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    HL_CUDA(cudaOccupancyMaxActiveClusters(&n, gemm_group_kernel, &cfg));
-    HL_REQUIRE(n > 0, "gemm_group: no CTA pair fits on this device");
-    resident_pairs = n;
-  }
+  HL_ALLOW_SHARED(ctx, GG_SMEM, gemm_group_kernel);
+  static PerDevice pairs;  // a GPC with an odd number of SMs leaves one out
+  const int resident_pairs = pairs.value(ctx->device, [&] { return resident_clusters(gemm_group_kernel, 2, GG_THREADS, GG_SMEM); });
+  HL_REQUIRE(resident_pairs > 0, "gemm_group: no CTA pair fits on this device");
   {
     ProfileScope prof(ctx, HL_PROF_GEMM, flops);
     HL_CUDA(launch_pdl(gemm_group_kernel, (unsigned)(2 * std::min({p.tiles, resident_pairs, std::max(1, persistent_sms(ctx) / 2)})), GG_THREADS, GG_SMEM, ctx->stream, 2, p));

@@ -295,11 +295,7 @@ template <bool A_MN, bool B_MN, int BN, int STAGES>
 int launch_small(hl_ctx* ctx, const CUtensorMap& ma, const CUtensorMap& mb, const GsParams& p, int grid) {
   using Z = GsSizes<BN, STAGES>;
   auto kern = gemm_small_kernel<A_MN, B_MN, BN, STAGES>;
-  static bool configured = false;
-  if (!configured) {
-    HL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Z::SMEM));
-    configured = true;
-  }
+  HL_ALLOW_SHARED(ctx, Z::SMEM, kern);
   HL_CUDA(launch_pdl(kern, (unsigned)grid, GS_THREADS, Z::SMEM, ctx->stream, p.splits, ma, mb, p));
   count_launch(ctx);
   ctx->counters.gemm_tcgen05_launches += 1;
@@ -329,36 +325,25 @@ int launch_majors(hl_ctx* ctx, bool a_mn, bool b_mn, const CUtensorMap& ma, cons
 namespace {
 // CTAs of one wave of clusters of `splits`: a cluster sits in one GPC, so clusters of four and eight leave SMs over.  Asked of
 // the driver once per form; form 0 deep, 1 narrow, 2 wide.
-int wave_ctas(int form, int splits, int sm_count) {
-  static int clusters[3][4] = {};
+int wave_ctas(int form, int splits, int device, int sm_count) {
+  static PerDevice clusters[3][4];
   const int at = splits == 1 ? 0 : splits == 2 ? 1 : splits == 4 ? 2 : 3;
   if (at == 0) return sm_count * (form == 1 ? 2 : 1);
-  int& c = clusters[form][at];
-  if (c == 0) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(splits * 1024));
-    cfg.blockDim = dim3(GS_THREADS);
-    cfg.dynamicSmemBytes = form == 0 ? GsSizes<64, 8>::SMEM : form == 1 ? GsSizes<64, 4>::SMEM : GsSizes<128, 6>::SMEM;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = (unsigned)splits; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+  const int n = clusters[form][at].value(device, [&] {
+    const size_t smem = form == 0 ? GsSizes<64, 8>::SMEM : form == 1 ? GsSizes<64, 4>::SMEM : GsSizes<128, 6>::SMEM;
     auto ask = [&](auto kern) {
-      int n = 0;
-      const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) == cudaSuccess &&
-                      cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess;
+      const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
       if (!ok) cudaGetLastError();
-      return ok && n > 0 ? n : 1;
+      return ok ? std::max(1, resident_clusters(kern, splits, GS_THREADS, smem)) : 1;
     };
-    c = form == 0 ? ask(gemm_small_kernel<true, true, 64, 8>)
-                  : form == 1 ? ask(gemm_small_kernel<true, true, 64, 4>) : ask(gemm_small_kernel<true, true, 128, 6>);
-  }
-  return std::min(c * splits, sm_count * (form == 1 ? 2 : 1));
+    return form == 0 ? ask(gemm_small_kernel<true, true, 64, 8>)
+                     : form == 1 ? ask(gemm_small_kernel<true, true, 64, 4>) : ask(gemm_small_kernel<true, true, 128, 6>);
+  });
+  return std::min(n * splits, sm_count * (form == 1 ? 2 : 1));
 }
 }  // namespace
 
-GemmSmallPlan gemm_small_plan(const hl_gemm_desc* d, const GemmPlan& big, int sm_count) {
+GemmSmallPlan gemm_small_plan(const hl_gemm_desc* d, const GemmPlan& big, int device, int sm_count) {
   const int kb = ceil_div(d->k, GS_BK), m_tiles = ceil_div(d->m, GS_BM);
   const long long narrow = (long long)m_tiles * ceil_div(d->n, 64), wide = (long long)m_tiles * ceil_div(d->n, 128);
   const long long tiles = (long long)m_tiles * ceil_div(d->n, 256);
@@ -375,9 +360,9 @@ GemmSmallPlan gemm_small_plan(const hl_gemm_desc* d, const GemmPlan& big, int sm
     auto take = [&](float t, int bn, bool deep) {
       if (t < best) { best = t; plan = GemmSmallPlan{s, bn, deep}; }
     };
-    if (narrow * s <= wave_ctas(0, s, sm_count)) take(3.0f + 0.17f * steps + shared, 64, true);
-    else if (narrow * s <= wave_ctas(1, s, sm_count)) take(3.0f + 0.34f * steps + shared, 64, false);
-    if (wide * s <= wave_ctas(2, s, sm_count)) take(4.4f + 0.21f * steps + (s > 1 ? 2.5f : 0.f), 128, false);
+    if (narrow * s <= wave_ctas(0, s, device, sm_count)) take(3.0f + 0.17f * steps + shared, 64, true);
+    else if (narrow * s <= wave_ctas(1, s, device, sm_count)) take(3.0f + 0.34f * steps + shared, 64, false);
+    if (wide * s <= wave_ctas(2, s, device, sm_count)) take(4.4f + 0.21f * steps + (s > 1 ? 2.5f : 0.f), 128, false);
   }
   return plan;
 }

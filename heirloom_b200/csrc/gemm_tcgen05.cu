@@ -856,29 +856,12 @@ template <bool A_MN, bool B_MN, bool PAIR, int SPEC = -1>
 int launch_variant(hl_ctx* ctx, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc,
                    const CUtensorMap& maux, const GemmParams& p, int grid) {
   auto kern = gemm_bf16_tcgen05_kernel<A_MN, B_MN, PAIR, SPEC>;
-  static bool configured = false;
-  if (!configured) {
-    HL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM_BYTES));
-    configured = true;
-  }
+  HL_ALLOW_SHARED(ctx, GEMM_SMEM_BYTES, kern);
   if (PAIR) {
     // `grid` CTAs in clusters of two neighbouring SMs; no more pairs than can be resident at once (a GPC with an odd number of free SMs leaves one out)
-    static int resident_pairs = 0;
-    if (resident_pairs == 0) {
-      cudaLaunchConfig_t cfg{};
-      cfg.gridDim = dim3((unsigned)grid);
-      cfg.blockDim = dim3(GEMM_THREADS);
-      cfg.dynamicSmemBytes = GEMM_SMEM_BYTES;
-      cudaLaunchAttribute attr{};
-      attr.id = cudaLaunchAttributeClusterDimension;
-      attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-      cfg.attrs = &attr;
-      cfg.numAttrs = 1;
-      int n = 0;
-      HL_CUDA(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
-      HL_REQUIRE(n > 0, "hl_gemm_bf16: no CTA pair fits on this device");
-      resident_pairs = n;
-    }
+    static PerDevice pairs;
+    const int resident_pairs = pairs.value(ctx->device, [&] { return resident_clusters(kern, 2, GEMM_THREADS, GEMM_SMEM_BYTES); });
+    HL_REQUIRE(resident_pairs > 0, "hl_gemm_bf16: no CTA pair fits on this device");
     HL_CUDA(launch_pdl(kern, (unsigned)std::min(grid, 2 * resident_pairs), GEMM_THREADS, GEMM_SMEM_BYTES, ctx->stream, 2, ma, mb, mc,
                        maux, p));
   } else {
@@ -911,7 +894,7 @@ GemmSmallPlan small_plan(const hl_ctx* ctx, const hl_gemm_desc* d, const GemmPla
   auto forced = [](const char* name) { const char* e = getenv(name); return e && e[0] == '1'; };
   if (d->split_k > 0 || ctx->gemm_skip_kblock >= 0 || forced("HEIRLOOM_GEMM_PAIRS") || forced("HEIRLOOM_GEMM_DYNAMIC"))
     return GemmSmallPlan{0, 0, false};
-  return gemm_small_plan(d, plan, sms);
+  return gemm_small_plan(d, plan, ctx->device, sms);
 }
 
 }  // namespace

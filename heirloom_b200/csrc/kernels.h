@@ -36,7 +36,7 @@ struct GemmSmallPlan {
   int splits, bn;
   bool deep;
 };
-GemmSmallPlan gemm_small_plan(const hl_gemm_desc* d, const GemmPlan& big, int sm_count);
+GemmSmallPlan gemm_small_plan(const hl_gemm_desc* d, const GemmPlan& big, int device, int sm_count);
 int gemm_small_run(hl_ctx* ctx, const hl_gemm_desc* d, const GemmSmallPlan& plan, const void* a, const void* b, void* c,
                    const float* bias, const void* aux_in, void* aux_out, float* row_sum = nullptr);
 // The GEMM with its scratch taken from (and grown in) the context.

@@ -591,11 +591,7 @@ int layer_norm_backward_impl(hl_ctx* ctx, const void* x, int x_dtype, const floa
 #define HL_LN_BWD(XT, ACC, J)                                                                                          \
   do {                                                                                                                 \
     auto k = layer_norm_bwd_kernel<XT, ACC, J>;                                                                        \
-    static bool configured = false;                                                                                    \
-    if (!configured) {                                                                                                 \
-      HL_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(float) * LNB_WARPS * 2 * LNB_MAXJ * 128))); \
-      configured = true;                                                                                               \
-    }                                                                                                                  \
+    HL_ALLOW_SHARED(ctx, sizeof(float) * LNB_WARPS * 2 * LNB_MAXJ * 128, k);                                            \
     pdl(k, blocks, LNB_WARPS * 32, smem, ctx->stream)((const XT*)x, gamma, dy, mean, rstd, residual_grad, dx_f32,       \
                                                      (__nv_bfloat16*)dx_bf16, partial, rows, features, rows_per_block, \
                                                      1e-5f);                                                           \

@@ -372,11 +372,7 @@ template <int TM, int TN>
 int launch_f64_gemm(hl_ctx* ctx, const F64Gemm* problems, int count) {
   constexpr size_t smem = F64Tile<TM, TN>::SMEM;
   auto kern = f64_gemm_kernel<TM, TN>;
-  static bool configured = false;
-  if (!configured) {
-    HL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
-  }
+  HL_ALLOW_SHARED(ctx, smem, kern);
   F64Jobs jobs{};
   jobs.count = count;
   // A contraction longer than 256 is shared as long as its tiles leave SMs idle; eight CTAs is the largest portable cluster.
@@ -843,12 +839,6 @@ int at_cols_tile(int T, int hd, size_t* smem) {
   return tile;
 }
 
-template <typename K>
-int at_configure(K kern) {
-  HL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttentionSmem));
-  return HL_OK;
-}
-
 template <typename T>
 int attention_forward_t(hl_ctx* ctx, const T* q, const T* k, const T* v, long long ld_qkv, T* out, long long ld_out,
                         float* probs, int B, int Tn, int C, int H) {
@@ -857,12 +847,7 @@ int attention_forward_t(hl_ctx* ctx, const T* q, const T* k, const T* v, long lo
   const size_t smem = at_rows_smem(Tn, hd, false, resident);
   const long long heads = (long long)B * H;
   if (smem <= kAttentionSmem) {
-    static bool configured = false;
-    if (!configured) {
-      int rc = at_configure(attention_f64_fwd_kernel<T>);
-      if (rc != HL_OK) return rc;
-      configured = true;
-    }
+    HL_ALLOW_SHARED(ctx, kAttentionSmem, attention_f64_fwd_kernel<T>);
     pdl(attention_f64_fwd_kernel<T>, (unsigned)(ceil_div(Tn, AT_Q) * heads), AT_THREADS, smem, ctx->stream)(
         q, k, v, ld_qkv, out, ld_out, probs, Tn, H, hd, (unsigned)heads, resident);
     HL_LAUNCH_CHECK("attention_f64_fwd_kernel");
@@ -887,12 +872,8 @@ int attention_backward_t(hl_ctx* ctx, const T* q, const T* k, const T* v, long l
   const size_t rows = at_rows_smem(Tn, hd, true, resident);
   size_t cols = 0;
   const int tile = at_cols_tile(Tn, hd, &cols);
-  static bool configured = false;
-  if (!configured) {
-    if ((rc = at_configure(attention_f64_bwd_rows_kernel<T, RECOMPUTE>)) != HL_OK) return rc;
-    if ((rc = at_configure(attention_f64_bwd_cols_kernel<T>)) != HL_OK) return rc;
-    configured = true;
-  }
+  HL_ALLOW_SHARED(ctx, kAttentionSmem, attention_f64_bwd_rows_kernel<T, RECOMPUTE>);
+  HL_ALLOW_SHARED(ctx, kAttentionSmem, attention_f64_bwd_cols_kernel<T>);
   if (rows <= kAttentionSmem) {
     pdl(attention_f64_bwd_rows_kernel<T, RECOMPUTE>, (unsigned)(ceil_div(Tn, AT_Q) * heads), AT_THREADS, rows, ctx->stream)(
         q, k, v, ld_qkv, probs, dout, ld_dout, ds, dq, ld_dqkv, Tn, H, hd, (unsigned)heads, resident);
