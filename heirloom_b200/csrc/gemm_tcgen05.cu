@@ -1025,7 +1025,7 @@ int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void*
   p.b_kb_wrap = d->b_k_period > 0 ? d->b_k_period / BK : 0;
   p.wait_limit_ns = ctx->wait_limit_ns ? ctx->wait_limit_ns : tc05::kWaitLimitNs;
   p.skip_kblock = ctx->gemm_skip_kblock;
-// Panels of up to sixteen tile columns: A streams past B's columns, which stay in L2.  One column after the other would read
+  // Panels of up to sixteen tile columns: A streams past B's columns, which stay in L2.  One column after the other would read
   // an A of 25 MB again for each of them while the results push it out of L2 (16384 x 3072 x 768: 81 us, now 77).
   p.panel_w = std::min(p.n_tiles, 16);
   const int splits = plan.splits;
@@ -1109,7 +1109,10 @@ int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void*
   const int total = p.m_tiles * p.n_tiles * p.splits;
   const int grid = pair ? 2 * min(total, sms / 2) : plan.sk_tiles > 0 ? sms : min(total, sms);
   ProfileScope prof(ctx, HL_PROF_GEMM, 2.0 * (double)d->m * (double)d->n * (double)d->k);
-  // The training step's products with whole tiles have kernels of their own, compiled for one epilogue and output type.
+  // Whole-tile products have kernels compiled for one epilogue and output type where a training step or an evaluation runs them (operand
+  // order, pairing and epilogue as they occur there): the generic kernel carries every epilogue behind run-time branches in its
+  // column loop and is bound by instruction supply (fc1 forward 105 us, its own kernel 87; out_proj forward 36 and 30;
+  // lm_head forward 1363 and 1295).  Everything else takes the generic kernels below.
   const bool simple = splits == 1 && plan.sk_tiles == 0;
   const int spec = simple ? d->epilogue * 2 + (d->out_dtype == HL_BF16 ? 1 : 0)
                           : (splits > 1 && plan.sk_tiles == 0) ? SPEC_PARTIAL : -1;
@@ -1221,7 +1224,9 @@ extern "C" int hl_gemm_bf16(hl_ctx* ctx, const hl_gemm_desc* desc, const void* a
 extern "C" int hl_gemm_bf16_plan(hl_ctx* ctx, const hl_gemm_desc* desc, int* splits, int* dealt_tiles, size_t* scratch_bytes) {
   if (!ctx || !desc) return hl::fail("hl_gemm_bf16_plan: null argument");
   if (desc->m <= 0 || desc->n <= 0 || desc->k <= 0) return hl::fail("hl_gemm_bf16_plan: m, n, k must be positive");
-  const hl::GemmPlan plan = hl::gemm_plan(desc, ctx->sm_count);
+  hl::GemmPlan plan = hl::gemm_plan(desc, ctx->sm_count);
+  const hl::GemmSmallPlan small = hl::small_plan(ctx, desc, plan, ctx->sm_count);
+  if (small.splits > 0) plan = hl::GemmPlan{small.splits, 0, 0, 0, 0};  // shared within a cluster, no scratch
   if (splits) *splits = plan.splits;
   if (dealt_tiles) *dealt_tiles = plan.sk_tiles;
   if (scratch_bytes) *scratch_bytes = std::max(plan.splitk_bytes, plan.sk_slot_bytes);

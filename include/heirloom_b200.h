@@ -279,7 +279,7 @@ int hl_gemm_bf16(hl_ctx* ctx, const hl_gemm_desc* desc, const void* a, const voi
                  const float* bias, const void* aux_in, void* aux_out);
 
 /* How hl_gemm_bf16 would cut this shape on this context's GPU: the number of equal splits of the contraction
- * (1 = none), the number of output tiles whose k blocks are dealt out over the CTAs (0 = none), and the scratch
+ * (1 = none; the splits of a product of few tiles are shared within a cluster and need no scratch), the number of output tiles whose k blocks are dealt out over the CTAs (0 = none), and the scratch
  * bytes the launch needs.  Pure host arithmetic; lets a caller check a shape against a scratch budget before the
  * step starts (the reference's shape-support predicates play this role, heirloom-kernels/src/cuda.rs:3761-3900). */
 int hl_gemm_bf16_plan(hl_ctx* ctx, const hl_gemm_desc* desc, int* splits, int* dealt_tiles, size_t* scratch_bytes);

@@ -272,6 +272,22 @@ def test_dgelu_epilogue_at_sizes_of_the_persistent_kernels(m, n, k, b_mn, dtype)
     assert_close("dgelu", host(out), want, atol=(2e-3 + 2.3e-6 * np.sqrt(k)) * np.abs(acc).max(), rtol=0.0 if dtype is torch.float32 else 2 ** -8)
 
 
+@pytest.mark.parametrize("m,n,k", [(500, 768, 3072), (128, 128, 256), (512, 768, 16384), (1280, 2048, 12288), (4096, 2048, 512)])
+def test_the_plan_is_what_the_product_does(m, n, k):
+    """hl_gemm_bf16_plan's scratch bytes against what a context without scratch allocates for the product (rounded up to megabytes, and
+    a flag array once for dealt tiles): none for products of few tiles, which share their contraction within a cluster."""
+    from heirloom_b200 import cuda
+    ctx()
+    c = cuda.Context(0)
+    a, b = torch.zeros(m, k, dtype=torch.bfloat16, device="cuda"), torch.zeros(n, k, dtype=torch.bfloat16, device="cuda")
+    splits, dealt, need = cuda.gemm_bf16_plan(c, m, n, k)
+    cuda.gemm_bf16(c, a, b, m, n, k, out_dtype=torch.float32)
+    c.sync()
+    allocated = int(c.counters().allocated_bytes)
+    c.close()
+    assert (allocated > 0) == (need > 0) and need <= allocated <= need + (2 << 20) and splits >= 1, (splits, dealt, need, allocated)
+
+
 PAIR_SCRIPT = r"""
 import numpy as np, torch
 from oracle import heirloom_oracle as ho
