@@ -704,10 +704,6 @@ int memory_core_backward(hl_decoder* m, int l, const float* dweighted) {
                                             G + m->off_kl, G + m->off_kr, N, k, side, kd, m->mem.slots);
 }
 
-// Attention for head sizes the tcgen05 kernels are not built for (they take head_dim 64 and 128): the f32 kernels read the
-// bf16 q, k, v (widened exactly) and round to bf16 where the flash route stores bf16.  Probabilities are not kept per
-// layer, the backward forms them again.
-
 // Final layer norm and head of one row of the residual stream: the logits in row 0 of m->logits.
 int decode_head(hl_decoder* m, const void* x, int dtype) {
   DecodeGemv g{};
@@ -794,6 +790,8 @@ int forward(hl_decoder* m, Forward what = Forward::all) {
       return decode_head(m, m->x[l + 1], HL_BF16);
     }
     if (m->flash_ok) HL_TRY(flash_attention_forward_impl(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, 3 * d, a.o, d, a.lse, B, T, H, d / H));
+    // head sizes other than 64 and 128: the f64 kernels read the bf16 rows (widened exactly) and round to bf16 where the flash route
+    // stores bf16; the backward pass forms the probabilities again
     else HL_TRY(attention_f64_forward(ctx, a.qkv, a.qkv + d, a.qkv + 2 * d, HL_BF16, 3 * d, a.o, d, m->fa_probs, B, T, d, H));
     HL_TRY(g.run(N, d, d, a.o, d, HL_K_MAJOR, W + o.wo, d, HL_K_MAJOR, a.r, d, HL_BF16, HL_EPI_BIAS_RESIDUAL, P + o.bo,
                  m->x[l], d));
@@ -1495,37 +1493,24 @@ int optimizer_step(hl_decoder* m) {
   if (m->opt.clip_norm > 0.f) HL_TRY(wait_for_collectives(m));  // the global norm needs every averaged gradient
   const int world = nccl_world(ctx);
   const float inv_world = 1.0f / (float)world;  // sum then scale by 1/world (src/nn.rs:2100-2117)
-  // Global gradient norm after averaging; forces one device-to-host read like the reference.  Without collectives the factor is
-  // worked out on the device, so that the update does not wait for the host to have read the norm.
-  const bool on_device = m->opt.clip_norm > 0.f && !m->comm_pending;
-  double clip = 1.0;
-  double sum_sq = 0.0;
-  auto read_norm = [&]() -> int {
-    HL_CUDA(cudaStreamSynchronize(ctx->stream));
-    sum_sq = (double)m->norm_host[0] * (double)inv_world * (double)inv_world;
-    if (!(sum_sq >= 0.0) || sum_sq > 1e300) return fail("non-finite or negative global gradient sum-of-squares");
-    return HL_OK;
-  };
-  if (m->opt.clip_norm > 0.f) {
-    HL_TRY(sum_squares_impl(ctx, m->grads, m->arena, m->norm_dev, m->norm_host));
-    if (!on_device) {
-      HL_TRY(read_norm());
-      const double norm = sqrt(sum_sq);
-      if (norm > (double)m->opt.clip_norm) clip = (double)m->opt.clip_norm / (norm + 1e-12);
-    }
-  }
+  // The norm of the averaged gradients: the clipping factor is worked out on the device, so that the update does not wait for the host
+  // to have read the norm, which it does like the reference, to refuse a step whose norm is not finite.
+  const bool clipped = m->opt.clip_norm > 0.f;
+  if (clipped) HL_TRY(sum_squares_impl(ctx, m->grads, m->arena, m->norm_dev, m->norm_host));
   m->step += 1;
   hl_adamw_params hp{};
   hp.lr = m->opt.lr; hp.beta1 = m->opt.beta1; hp.beta2 = m->opt.beta2; hp.eps = m->opt.eps;
   hp.weight_decay = m->opt.weight_decay;
-  hp.clip_scale = (float)clip * inv_world;
+  hp.clip_scale = inv_world;
   hp.bias_correction1 = (float)(1.0 - pow((double)m->opt.beta1, (double)m->step));
   hp.bias_correction2 = (float)(1.0 - pow((double)m->opt.beta2, (double)m->step));
-  if (on_device) {
+  if (clipped) {  // every collective has been waited for
     HL_TRY(adam_plan_step(ctx, m->plan, &hp, AdamClip{m->norm_dev, (double)inv_world, (double)m->opt.clip_norm}));
-    const int rc = read_norm();
-    if (rc != HL_OK) m->step -= 1;  // nothing was updated
-    return rc;
+    HL_CUDA(cudaStreamSynchronize(ctx->stream));
+    const double sum_sq = (double)m->norm_host[0] * (double)inv_world * (double)inv_world;
+    if (sum_sq >= 0.0 && sum_sq <= 1e300) return HL_OK;
+    m->step -= 1;  // nothing was updated
+    return fail("non-finite or negative global gradient sum-of-squares");
   }
   if (!m->comm_pending) return adam_plan_step(ctx, m->plan, &hp);
   // Collectives still in flight: update the arena in groups of buckets, each group as soon as its last

@@ -1,5 +1,6 @@
 """Step-level parity of the decoder executor (amp-bf16 route) against the oracle's AMP restatement."""
 import contextlib
+import math
 
 import numpy as np
 import pytest
@@ -391,3 +392,62 @@ def test_a_model_without_room_for_operand_copies_is_created_without_them(batch, 
     for n in state:
         if not n.endswith("k_proj.bias"):
             assert np.linalg.norm(runs[1][1][n] - runs[0][1][n]) <= 1e-2 * np.linalg.norm(runs[0][1][n]), n
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_clipping_by_the_global_norm_of_a_dense_step(precision):
+    """The factor is worked out on the device: parameters and moments of a step with a limit below the norm are those of the oracle's
+    update with the f64 factor, a limit above it changes nothing, and a norm that is not finite is an error that leaves
+    parameters, moments and the step count as they were; the next step is right again."""
+    from heirloom_b200 import nn
+    from heirloom_b200._lib import HeirloomError
+    c = ctx()
+    rng = np.random.default_rng(2)
+    x = torch.from_numpy(rng.integers(0, 64, (4, 32))).cuda()
+    y = torch.from_numpy(rng.integers(0, 64, (4, 32))).cuda()
+    model = nn.DecoderLm(c, nn.DecoderConfig(vocab=64, d_model=64, n_layers=2, n_heads=1, d_ff=128, context=32, batch=4, precision=precision))
+    state = {n: (np.ones(s) if ".ln" in n or n.startswith("ln_f") else rng.standard_normal(s) * 0.1)
+             for n, s in model.parameter_shapes().items()}
+    before = {n: v.astype(np.float32) for n, v in state.items()}
+
+    def stepped(limit):
+        model.load_state_dict(state)
+        model.set_optimizer(lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.01, clip_norm=limit)
+        for n in state:
+            model.set_moments(n, np.zeros_like(before[n]), np.zeros_like(before[n]))
+        model.set_optimizer_steps(0)
+        model.forward_backward(x, y)
+        grads = {n: model.grad(n) for n in state}
+        error = None
+        try:
+            model.optimizer_step()
+            c.sync()
+        except HeirloomError as e:
+            error = str(e)
+        return grads, {n: (model.parameter(n),) + model.moments(n) for n in state}, model.optimizer_steps, error
+
+    grads, free, steps, error = stepped(None)
+    norm = math.sqrt(sum(float((g.astype(np.float64) ** 2).sum()) for g in grads.values()))
+    results = {limit: stepped(limit) for limit in (norm * 0.25, norm * 4.0)}
+    broken = dict(state, **{"lm_head.bias": np.full_like(state["lm_head.bias"], np.nan)})
+    model.load_state_dict(broken)
+    model.set_optimizer(lr=1e-3, clip_norm=1.0)
+    model.set_optimizer_steps(5)
+    model.forward_backward(x, y)
+    kept = {n: (model.parameter(n),) + model.moments(n) for n in state}
+    with pytest.raises(HeirloomError, match="non-finite or negative global gradient"):
+        model.optimizer_step()
+    after, count = {n: (model.parameter(n),) + model.moments(n) for n in state}, model.optimizer_steps
+    again = stepped(norm * 0.25)
+    model.close()
+    assert error is None and steps == 1 and count == 5
+    assert all(np.array_equal(a, b, equal_nan=True) for n in state for a, b in zip(kept[n], after[n]))
+    for limit, (g, got, _, error) in list(results.items()) + [(norm * 0.25, again)]:
+        assert error is None
+        own = math.sqrt(sum(float((v.astype(np.float64) ** 2).sum()) for v in g.values()))
+        factor = min(1.0, limit / (own + 1e-12)) if own > limit else 1.0
+        for n in state:
+            # AdamW's first moment of a first step is (1 - beta1) x (factor x gradient + decay x parameter) with f32 constants: f32
+            # roundings of a few terms
+            want = float(np.float32(1) - np.float32(0.9)) * (factor * g[n].astype(np.float64) + float(np.float32(0.01)) * before[n])
+            assert np.abs(got[n][1] - want).max() <= 4 * 2.0 ** -24 * (np.abs(0.1 * factor * g[n]).max() + np.abs(1e-3 * before[n]).max()) + 1e-12, n
