@@ -206,12 +206,12 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       bool ok = issue_qk();
       // A single Q buffer is overwritten once the item's result has left through it, which the softmax warps do after the last
       // P·V: the scores of the next item then wait until those have been issued.
-      auto may_run_ahead = [&](bool last_of_item) { return Z::Q_BUFS == 2 || qj > 0 || last_of_item; };
+      auto may_run_ahead = [&]() { return Z::Q_BUFS == 2 || qj > 0; };
       int ahead = 1;  // scores issued beyond the tile at hand
       int g = 0;
       for (FaItem it = fa_item(0, p); ok && it.n_tiles > 0; it = fa_item(it.local + 1, p)) {
         for (int j = 0; j < it.n_tiles && ok; ++j, ++g) {
-          while (ok && ahead < 2 && qi.n_tiles > 0 && may_run_ahead(false)) {
+          while (ok && ahead < 2 && qi.n_tiles > 0 && may_run_ahead()) {
             ok = issue_qk();
             ++ahead;
           }

@@ -408,7 +408,7 @@ int launch_f64_gemm(hl_ctx* ctx, const F64Gemm* problems, int count) {
 // One CTA of eight warps per 16 query rows of one (batch, head); the rows' scores against every visible key stay in shared
 // memory as f64, so each score is formed once (a lane per key walking the channels formed it three times, from
 // uncoalesced rows).  Bound by latency: a few thousand multiply-adds a CTA behind global loads, reductions and f64 exponentials.
-// So everything a CTA reads is requested at once and stays (`resident`, wherever keys and values fit: T 128 up to 96
+// So everything a CTA reads is requested at once and stays (`resident`, wherever keys and values fit: T 128 up to 80
 // channels), the rows of a warp go through the softmax side by side, and every warp has several chains of products.
 // B16 H4 T64 hd32, one after the other as a user calls them: forward 76 us at first, then 9 with the keys in tiles of 32 behind
 // two barriers each.
