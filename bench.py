@@ -33,21 +33,21 @@ METRIC = "train tokens/s (GPT-124M-shaped bf16 step)"
 DATASHEET_BF16_TFLOPS = 2250.0
 # dram__bytes_read.sum + dram__bytes_write.sum per GEMM launch, averaged over the GEMM launches of one training step
 # in a one-pass ncu launch list of this command (summary kept under profiles/), and the first 16 hex digits of the
-# SHA-256 of the GEMM source the capture ran with: a kernel changed since then gets no traffic figure, not a stale one.
-GEMM_DRAM_BYTES_PER_LAUNCH = 239.1e6
-GEMM_SOURCE_AT_CAPTURE = "64ddc78a321a5734"
+# SHA-256 of the GEMM sources the capture ran with: kernels changed since then get no traffic figure, not a stale one.
+GEMM_DRAM_BYTES_PER_LAUNCH = 229.4e6
+GEMM_SOURCE_AT_CAPTURE = "64f87fa126bbc822"
 
 
 def gemm_traffic():
     """(bytes per launch or None, note)."""
     import hashlib
-    src = ROOT / "heirloom_b200" / "csrc" / "gemm_tcgen05.cu"
+    sources = [ROOT / "heirloom_b200" / "csrc" / name for name in ("gemm_tcgen05.cu", "gemm_group.cu", "gemm_small.cu")]
     try:
-        now = hashlib.sha256(src.read_bytes()).hexdigest()[:16]
+        now = hashlib.sha256(b"".join(src.read_bytes() for src in sources)).hexdigest()[:16]
     except OSError:
         return None, "GEMM source not found beside the library: capture cannot be matched to it"
     if now != GEMM_SOURCE_AT_CAPTURE:
-        return None, "gemm_tcgen05.cu changed since the ncu capture (" + GEMM_SOURCE_AT_CAPTURE + " -> " + now + "): re-capture"
+        return None, "the GEMM sources changed since the ncu capture (" + GEMM_SOURCE_AT_CAPTURE + " -> " + now + "): re-capture"
     return GEMM_DRAM_BYTES_PER_LAUNCH, "ncu launch list of this command, profiles/bench_step_launch_list.md"
 
 
