@@ -93,6 +93,8 @@ class LmEvalMetrics:
     perplexity: float
 
 
+# The rules of sampling, written out in NumPy.  `sample_token` and `generate` follow them natively; these are for callers who
+# want a single rule, and for the tests that hold the native code to them.
 def softmax_logits(logits: np.ndarray) -> np.ndarray:
     finite = np.isfinite(logits)
     if not finite.any():
