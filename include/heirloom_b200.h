@@ -516,7 +516,8 @@ long long hl_decoder_optimizer_steps(hl_decoder* model);
 int hl_decoder_set_moments(hl_decoder* model, int index, const float* m_host, const float* v_host, long long numel);
 int hl_decoder_set_optimizer_steps(hl_decoder* model, long long steps);
 /* Forward only, no gradients (the loss inside evaluate_token_loss, src/memory_transformer.rs:1813-1912):
- * mean cross-entropy over `sequences` (1..batch) rows of `context` tokens; the value is copied to the host. */
+ * mean cross-entropy over `sequences` (1..batch) rows of `context` tokens; the value is copied to the host.  An id out of
+ * range or an expired wait is an error of this call, as it is of the generation calls below. */
 int hl_decoder_eval_loss(hl_decoder* model, const int64_t* tokens_dev, const int64_t* targets_dev, int sequences,
                          float* loss_host);
 /* next_token_logits (src/memory_transformer.rs:1930-1984): one window of 1..context tokens, full-window
