@@ -1633,17 +1633,25 @@ static int decoder_create_impl(hl_ctx* ctx, const hl_decoder_config* cfg, const 
   auto plan = [&](bool measure_only) { if (amp) plan_activations(m, measure_only, &act); else plan_activations_f32(m, measure_only, &act); };
   // Copies of operands for weight gradients beside or behind the backward pass (up to 256 MB, or a gigabyte) are only made where the
   // device has a gigabyte left behind them and behind the attention's scratch, so that a model fits wherever it did without them;
-  // and not beside a communicator, which uses none of them.
+  // and not beside a communicator, which uses none of them.  Asking for the free memory takes a millisecond, a fifth of a small
+  // model's creation: copies below 32 MB, a block of the driver's pool, are made where their allocation succeeds.
+  m->lean = true;
+  plan(true);
+  const size_t without = act;
   m->lean = nccl_active(ctx);
   plan(true);
-  if (m->fork_ok || m->group_layers > 0) {
-    const size_t scores = (size_t)cfg->batch * cfg->n_heads * cfg->context * cfg->context * sizeof(float);
-    const size_t behind = kGroupBytes + (amp && m->flash_ok ? flash_attention_backward_scratch_bytes(cfg->batch, cfg->context, cfg->n_heads,
-                                                                                                    cfg->d_model / cfg->n_heads) : scores);
-    size_t free_bytes = 0, total_bytes = 0;
-    e = cudaMemGetInfo(&free_bytes, &total_bytes);
-    if (e != cudaSuccess) return cleanup(fail_cuda(e, "cudaMemGetInfo"));
-    if (free_bytes < act + behind || cudaMalloc(reinterpret_cast<void**>(&m->act_arena), act) != cudaSuccess) {
+  if (act > without) {
+    bool room = true;
+    if (act - without >= (size_t(32) << 20)) {
+      const size_t scores = (size_t)cfg->batch * cfg->n_heads * cfg->context * cfg->context * sizeof(float);
+      const size_t behind = kGroupBytes + (amp && m->flash_ok ? flash_attention_backward_scratch_bytes(cfg->batch, cfg->context, cfg->n_heads,
+                                                                                                      cfg->d_model / cfg->n_heads) : scores);
+      size_t free_bytes = 0, total_bytes = 0;
+      e = cudaMemGetInfo(&free_bytes, &total_bytes);
+      if (e != cudaSuccess) return cleanup(fail_cuda(e, "cudaMemGetInfo"));
+      room = free_bytes >= act + behind;
+    }
+    if (!room || cudaMalloc(reinterpret_cast<void**>(&m->act_arena), act) != cudaSuccess) {
       cudaGetLastError();
       m->act_arena = nullptr;
       m->lean = true;
