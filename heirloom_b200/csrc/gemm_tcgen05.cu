@@ -204,9 +204,12 @@ __device__ __forceinline__ bool get_item(const GemmParams& p, int local, WorkIte
 // runs straight-line code of its own variant only (the step's short-contraction products are bound by their epilogue);
 // SPEC_PARTIAL: equal splits of the contraction whose raw f32 sums go to the scratch of the second kernel.
 // SPEC_ROW_STATS: bias, and no output but, per row and 128 columns, the maximum and the sum of exponentials below it, and the
-// row's value at its target column (a loss that wants no gradient reads nothing else of the logits).
+// row's value at its target column (a loss reads nothing else of the logits).
+// SPEC_LOSS_GRADIENT: bias, then the gradient of the loss in bf16, out of the row's maximum and sum: with SPEC_ROW_STATS before it
+// the logits are formed twice and never stored.  Rule and figures: gemm_bf16_row_stats below.
 constexpr int SPEC_PARTIAL = 16;
 constexpr int SPEC_ROW_STATS = 32;
+constexpr int SPEC_LOSS_GRADIENT = 34;
 template <bool A_MN, bool B_MN, bool PAIR, int SPEC>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -413,9 +416,11 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     // bytes halve the requests of 64-byte rows: 16384 x 3072 x 768 with bias and GELU spent 16 of its 81 us on its stores.
     uint8_t* staging = staging_base + size_t(ew) * (EPI_TILES * EPI_TILE_BYTES);
     int stage_sel = 0;
-    const int epi = SPEC == SPEC_PARTIAL ? HL_EPI_NONE : SPEC == SPEC_ROW_STATS ? HL_EPI_BIAS : SPEC >= 0 ? SPEC / 2 : p.epilogue;
+    constexpr bool kLoss = SPEC == SPEC_ROW_STATS || SPEC == SPEC_LOSS_GRADIENT;
+    const int epi = SPEC == SPEC_PARTIAL ? HL_EPI_NONE : kLoss ? HL_EPI_BIAS : SPEC >= 0 ? SPEC / 2 : p.epilogue;
     const bool partial = SPEC == SPEC_PARTIAL ? true : SPEC >= 0 ? false : p.partial_out != 0;
-    const bool out_bf16 = SPEC == SPEC_PARTIAL || SPEC == SPEC_ROW_STATS ? false : SPEC >= 0 ? (SPEC & 1) != 0 : (!partial && p.out_dtype == HL_BF16);
+    const bool out_bf16 = SPEC == SPEC_LOSS_GRADIENT ? true : SPEC == SPEC_PARTIAL || SPEC == SPEC_ROW_STATS ? false
+                          : SPEC >= 0 ? (SPEC & 1) != 0 : (!partial && p.out_dtype == HL_BF16);
     const bool need_aux = !partial && (epi == HL_EPI_BIAS_RESIDUAL || epi == HL_EPI_DGELU);
     const bool need_bias = !partial && p.bias != nullptr;
     bool ok = true;
@@ -502,7 +507,9 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       const int half_col0 = n_tile * BN + half * 128;
       auto fetch_aux = [&](int chunk, uint4 (&dst)[4]) { fetch_aux_of(w, chunk, dst); };
       long long target = -1;  // this row's target, counted from the warp's first column
-      if (SPEC == SPEC_ROW_STATS && row_ok) target = __ldg(p.row_stats.targets + row) - half_col0;
+      if (kLoss && row_ok) target = __ldg(p.row_stats.targets + row) - half_col0;
+      float2 row_top = make_float2(0.f, 0.f);  // its maximum, and grad_scale over its sum
+      if (SPEC == SPEC_LOSS_GRADIENT && row_ok) row_top = __ldg(p.row_stats.rows + row);
       if (!tc05::mbar_wait(&tail->tmem_full[buf], buf_phase, abort_flag, p.wait_limit_ns)) { ok = false; break; }
       tc05::tc_fence_after_sync();
       const uint32_t taddr_row = tmem_base + (uint32_t)(buf * BN) + ((uint32_t)(lane_group * 32) << 16);
@@ -618,6 +625,9 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         } else if (!out_bf16 || !ODD) {
           tile = free_tile();
         }
+        // of the loss's gradient: where in these 32 columns the row's target stands, and whether any of the warp's rows has one here
+        const long long at = SPEC == SPEC_LOSS_GRADIENT ? target - sub * 32 : -1;
+        const bool any_target = SPEC == SPEC_LOSS_GRADIENT && __any_sync(0xffffffffu, at >= 0 && at < 32);
 #pragma unroll
         for (int g = 0; g < 4; ++g) {  // groups of 8 columns
           float2 v[4];
@@ -629,6 +639,20 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             const float4 b1 = *reinterpret_cast<const float4*>(bias_tile + ODD * 32 + g * 8 + 4);
             v[0] = add2(v[0], make_float2(b0.x, b0.y)); v[1] = add2(v[1], make_float2(b0.z, b0.w));
             v[2] = add2(v[2], make_float2(b1.x, b1.y)); v[3] = add2(v[3], make_float2(b1.z, b1.w));
+          }
+          if constexpr (SPEC == SPEC_LOSS_GRADIENT) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float2 e = fma2(v[i], both(1.4426950408889634f), both(-row_top.x));
+              v[i] = mul2(make_float2(ex2_fast(e.x), ex2_fast(e.y)), both(row_top.y));
+            }
+            if (any_target) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                if (at == g * 8 + i * 2) v[i].x -= p.row_stats.grad_scale;
+                if (at == g * 8 + i * 2 + 1) v[i].y -= p.row_stats.grad_scale;
+              }
+            }
           }
           if (epi == HL_EPI_BIAS_GELU && !partial) {
             // h = bf16(acc + bias) is the main output; g = bf16(gelu(h)) the second one
@@ -1119,7 +1143,8 @@ int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void*
   constexpr int kBias = HL_EPI_BIAS * 2, kGelu = HL_EPI_BIAS_GELU * 2, kResidual = HL_EPI_BIAS_RESIDUAL * 2,
                 kDgelu = HL_EPI_DGELU * 2, kNone = HL_EPI_NONE * 2;
   bool launched = true;
-  if (row_stats) rc = launch_variant<false, false, true, SPEC_ROW_STATS>(ctx, ma, mb, mc, maux, p, grid);
+  if (row_stats && d->out_dtype == HL_F32) rc = launch_variant<false, false, true, SPEC_ROW_STATS>(ctx, ma, mb, mc, maux, p, grid);
+  else if (row_stats) rc = launch_variant<false, false, true, SPEC_LOSS_GRADIENT>(ctx, ma, mb, mc, maux, p, grid);
   else if (!a_mn && !b_mn && !pair && spec == kBias + 1) rc = launch_variant<false, false, false, kBias + 1>(ctx, ma, mb, mc, maux, p, grid);
   else if (!a_mn && !b_mn && !pair && spec == kBias) rc = launch_variant<false, false, false, kBias>(ctx, ma, mb, mc, maux, p, grid);
   else if (!a_mn && !b_mn && !pair && spec == kGelu + 1) rc = launch_variant<false, false, false, kGelu + 1>(ctx, ma, mb, mc, maux, p, grid);
@@ -1199,6 +1224,12 @@ bool gemm_bf16_row_stats(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, cons
     return false;
   *rc = gemm_bf16_run(ctx, d, a, b, unused_c, bias, nullptr, nullptr, nullptr, 0, nullptr, &stats);
   return true;
+}
+int gemm_bf16_loss_gradient(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, const float* bias, const GemmRowStats& stats,
+                            void* dlogits) {
+  hl_gemm_desc g = *d;  // the same plan and pairs: neither reads the result's type
+  g.out_dtype = HL_BF16;
+  return gemm_bf16_run(ctx, &g, a, b, dlogits, bias, nullptr, nullptr, nullptr, 0, nullptr, &stats);
 }
 bool gemm_bf16_small_applies(hl_ctx* ctx, const hl_gemm_desc* d) {
   const int sms = persistent_sms(ctx);

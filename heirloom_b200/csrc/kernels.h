@@ -14,12 +14,14 @@ struct GemmPlan {
   size_t sk_slot_bytes;  // scratch for the raw accumulators of partly finished tiles
 };
 GemmPlan gemm_plan(const hl_gemm_desc* d, int sm_count);
-// For a cross-entropy loss without gradients: per 128 columns (n in all, `parts` is [ceil(n/128)][m]) and row the maximum times
+// For a cross-entropy loss without stored logits: per 128 columns (n in all, `parts` is [ceil(n/128)][m]) and row the maximum times
 // log2(e) and the sum of 2^(x log2(e) - that), and the row's value at its target (nothing when it is out of range).
 struct GemmRowStats {
   float2* parts;
   float* target_logit;  // [m]
   const int64_t* targets;
+  float2* rows;         // [m] the whole row's maximum (in the same unit) and grad_scale over its sum; null without a gradient
+  float grad_scale;
 };
 int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, void* c, const float* bias,
                   const void* aux_in, void* aux_out, float* workspace, size_t workspace_bytes, unsigned* stream_flags,
@@ -28,8 +30,12 @@ int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void*
 // `unused_c`: any memory of the result's size.
 bool gemm_bf16_row_stats(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, const float* bias, const GemmRowStats& stats,
                          void* unused_c, int* rc);
-// The mean loss out of them.
-int row_stats_loss(hl_ctx* ctx, const GemmRowStats& stats, int rows, int classes, float* row_loss, float* loss_dev);
+// The mean loss out of them, and `rows` where it is wanted.  `loss_host` may be null.
+int row_stats_loss(hl_ctx* ctx, const GemmRowStats& stats, int rows, int classes, float* row_loss, float* loss_dev, float* loss_host = nullptr);
+// The same product again (call it where gemm_bf16_row_stats returned true), its result turned into the loss's gradient in bf16 on
+// its way out: (2^(x log2(e) - maximum) - [column is the target] * sum) * grad_scale / sum.
+int gemm_bf16_loss_gradient(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, const float* bias, const GemmRowStats& stats,
+                            void* dlogits);
 // Products that leave most of the chip idle in 128 x 256 tiles (gemm_small.cu): how many CTAs share the contraction of one of
 // its 128 x bn tiles (0: not one of them), and whether a CTA has the SM's shared memory to itself.
 struct GemmSmallPlan {

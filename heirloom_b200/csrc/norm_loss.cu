@@ -495,6 +495,7 @@ row_stats_loss_kernel(const GemmRowStats stats, int rows, int parts, int classes
 #pragma unroll
     for (int w = 0; w < 8; ++w) sum += sums[w][lane] * ex2_fast(tops[w][lane] - top);
     const long long target = stats.targets[row];
+    if (stats.rows) stats.rows[row] = make_float2(top, stats.grad_scale / sum);
     if (target < 0 || target >= classes) {
       atomicExch(status + ST_BAD_INDEX, 1);
       row_loss[row] = 0.f;
@@ -541,10 +542,10 @@ int layer_norm_forward_impl(hl_ctx* ctx, const void* x, int x_dtype, const float
   return HL_OK;
 }
 
-int row_stats_loss(hl_ctx* ctx, const GemmRowStats& stats, int rows, int classes, float* row_loss, float* loss_dev) {
+int row_stats_loss(hl_ctx* ctx, const GemmRowStats& stats, int rows, int classes, float* row_loss, float* loss_dev, float* loss_host) {
   const int parts = ceil_div(classes, 128);
   ProfileScope prof(ctx, HL_PROF_LOSS, (double)rows * parts * 8.0);
-  const MeanLoss mean{loss_dev, nullptr, ctx->gemm_sched + 8};  // a word of the context's zeroed counters
+  const MeanLoss mean{loss_dev, loss_host, ctx->gemm_sched + 8};  // a word of the context's zeroed counters
   pdl(row_stats_loss_kernel, ceil_div(rows, 32), 256, 0, ctx->stream)(stats, rows, parts, classes, row_loss, ctx->status_dev, mean);
   HL_LAUNCH_CHECK("row_stats_loss_kernel");
   count_launch(ctx);

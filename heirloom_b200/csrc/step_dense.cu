@@ -208,6 +208,7 @@ struct hl_decoder {
   // state of the next one-token step
   int cached = 0;
   long long* decode_state = nullptr;       // device: position, token
+  bool head_twice = false;                 // this pass left the head's row sums instead of its logits
   float* row_logits = nullptr;             // where the logits of a single row go; null: m->logits
   GreedyPart* greedy = nullptr;            // device: the blocks' parts
   long long* decode_state_host = nullptr;  // pinned
@@ -763,6 +764,36 @@ bool last_block_by_row(const hl_decoder* m, int l) {
   return l == m->cfg.n_layers - 1 && !m->lo[l].is_memory && decode_applicable(m);
 }
 
+// The head's product as gemm_bf16_row_stats takes it; its results lie in the logits' buffer.
+struct HeadStats {
+  hl_gemm_desc desc{};
+  GemmRowStats stats{};
+  float* row_loss;
+  bool fits;
+  explicit HeadStats(const hl_decoder* m) {
+    const size_t N = (size_t)m->N, V = (size_t)m->cfg.vocab, parts = (size_t)ceil_div(m->cfg.vocab, 128) * N;
+    desc.m = m->N; desc.n = m->cfg.vocab; desc.k = m->cfg.d_model;
+    desc.a_layout = desc.b_layout = HL_K_MAJOR;
+    desc.lda = desc.ldb = m->cfg.d_model; desc.ldc = m->cfg.vocab;
+    desc.epilogue = HL_EPI_BIAS; desc.out_dtype = HL_F32;
+    stats.parts = reinterpret_cast<float2*>(m->logits);
+    stats.rows = stats.parts + parts;
+    stats.target_logit = m->logits + 2 * (parts + N);
+    stats.targets = m->targets;
+    stats.grad_scale = 1.0f / (float)m->N;
+    row_loss = stats.target_logit + N;
+    fits = 2 * parts + 4 * N <= N * V;
+  }
+};
+// Whether a training step forms the logits twice, for the row sums and for their gradient, instead of storing them in f32 for the
+// loss kernel to read and turn into the gradient: 2 d flop an element (d is at most 1024 here) against eight bytes.  Bound by the
+// tensor core then instead of by the copy rate; a step under the power cap gains least, since the flop cost power as well.  Step
+// before / after, us: 4096 x 32000 x 512 2460 / 2392, 16384 x 32000 x 512 10330 / 10110, 16384 x 50304 x 768 17280 / 17260,
+// 16384 x 32000 x 64 1644 / 1419, 8192 x 2000 x 512 2700 / 2652, 1024 x 32000 x 512 1541 / 1533, 1024 x 8000 x 512 1277 / 1276.
+// Below 1024 rows the logits stay in L2 and the second product's start costs what it saves: 512 x 32000 x 512 1308 / 1311.
+constexpr int kHeadTwiceRows = 1024;
+bool head_twice_pays(const hl_decoder* m) { return m->N >= kHeadTwiceRows; }
+
 // What a forward pass is for: logits and activations for the backward pass, the logits of the last position alone (they go to
 // row 0 of m->logits), or the mean loss alone (to m->loss_dev).
 enum class Forward { all, last_position, loss };
@@ -828,20 +859,15 @@ int forward(hl_decoder* m, Forward what = Forward::all) {
   if (what == Forward::last_position) return decode_head(m, m->x[c.n_layers] + (size_t)(N - 1) * d, HL_BF16);
   HL_TRY(layer_norm_forward_impl(ctx, m->x[c.n_layers], HL_BF16, P + m->off_lnf_g, P + m->off_lnf_b, m->z, HL_BF16, m->meanf,
                                  m->rstdf, N, d, 1e-5f));
-  if (what == Forward::loss) {
+  m->head_twice = false;
+  if (what == Forward::loss || head_twice_pays(m)) {
     // maxima and sums of the logits without the logits, in the buffer that would hold them
-    hl_gemm_desc desc{};
-    desc.m = N; desc.n = V; desc.k = d;
-    desc.a_layout = desc.b_layout = HL_K_MAJOR;
-    desc.lda = desc.ldb = d; desc.ldc = V;
-    desc.epilogue = HL_EPI_BIAS; desc.out_dtype = HL_F32;
-    const size_t parts = (size_t)ceil_div(V, 128) * N;
-    const GemmRowStats stats{reinterpret_cast<float2*>(m->logits), m->logits + 2 * parts, m->targets};
+    const HeadStats h(m);
     int rc = HL_OK;
-    if (2 * parts + 2 * (size_t)N <= (size_t)N * V &&
-        gemm_bf16_row_stats(ctx, &desc, m->z, W + m->off_head_w, P + m->off_head_b, stats, m->logits, &rc)) {
+    if (h.fits && gemm_bf16_row_stats(ctx, &h.desc, m->z, W + m->off_head_w, P + m->off_head_b, h.stats, m->logits, &rc)) {
       HL_TRY(rc);
-      return row_stats_loss(ctx, stats, N, V, m->logits + 2 * parts + N, m->loss_dev);
+      m->head_twice = what == Forward::all;  // the backward pass takes the loss, and forms the logits again for its gradient
+      return m->head_twice ? HL_OK : row_stats_loss(ctx, h.stats, N, V, h.row_loss, m->loss_dev);
     }
   }
   HL_TRY(g.run(N, V, d, m->z, d, HL_K_MAJOR, W + m->off_head_w, d, HL_K_MAJOR, m->logits, V, HL_F32, HL_EPI_BIAS,
@@ -1026,7 +1052,13 @@ int backward(hl_decoder* m) {
     m->comm_pending = false;
   }
   // loss and dlogits = (softmax - onehot)/N in bf16, the operand precision of the next GEMMs
-  HL_TRY(cross_entropy_impl(ctx, m->logits, V, m->targets, N, V, 1.0f, m->loss_dev, nullptr, m->dlogits, HL_BF16, V, m->loss_host));
+  if (m->head_twice) {
+    const HeadStats h(m);
+    HL_TRY(row_stats_loss(ctx, h.stats, N, V, h.row_loss, m->loss_dev, m->loss_host));
+    HL_TRY(gemm_bf16_loss_gradient(ctx, &h.desc, m->z, W + m->off_head_w, P + m->off_head_b, h.stats, m->dlogits));
+  } else {
+    HL_TRY(cross_entropy_impl(ctx, m->logits, V, m->targets, N, V, 1.0f, m->loss_dev, nullptr, m->dlogits, HL_BF16, V, m->loss_host));
+  }
   if (m->has_memory) HL_TRY(tables_are_zero(m));
   FoldBatch* fb = &m->fold;
   fb->n = 0;

@@ -451,3 +451,40 @@ def test_clipping_by_the_global_norm_of_a_dense_step(precision):
             # roundings of a few terms
             want = float(np.float32(1) - np.float32(0.9)) * (factor * g[n].astype(np.float64) + float(np.float32(0.01)) * before[n])
             assert np.abs(got[n][1] - want).max() <= 4 * 2.0 ** -24 * (np.abs(0.1 * factor * g[n]).max() + np.abs(1e-3 * before[n]).max()) + 1e-12, n
+
+
+@pytest.mark.parametrize("context,vocab,masked", [(103, 8200, False), (128, 5000, False), (128, 5000, True), (103, 16384, True)])
+def test_head_of_many_rows_equals_the_head_that_stores_its_logits(context, vocab, masked):
+    """From 1024 rows on the logits are formed twice instead of stored (1030 and 1280 rows, ragged last columns): loss and head
+    gradients are the average of those of two halves below that, in whose scale the same bf16 values are a factor of two larger.
+    A gradient of a row may round the other way (a few of a column's, each at most 2^-8 of 1 / rows); masked columns have none."""
+    from heirloom_b200 import nn
+    kw = dict(vocab=vocab, d_model=128, n_layers=1, n_heads=2, d_ff=128, context=context)
+    rng = np.random.default_rng(vocab)
+    c = ctx()
+    whole, half = nn.DecoderLm(c, nn.DecoderConfig(batch=10, **kw)), nn.DecoderLm(c, nn.DecoderConfig(batch=5, **kw))
+    state = {n: rng.standard_normal(s) * 0.2 for n, s in whole.parameter_shapes().items()}
+    off = np.arange(300, 700) if masked else np.arange(0)
+    state["lm_head.bias"][off] = -np.inf
+    x = torch.from_numpy(rng.integers(0, vocab, (10, context))).cuda()
+    y = torch.from_numpy(rng.choice(np.setdiff1d(np.arange(vocab), off), (10, context))).cuda()
+    y[0, :2] = torch.tensor([0, vocab - 1])
+    for m in (whole, half):
+        m.load_state_dict(state)
+    names = ("lm_head.bias", "lm_head.weight")
+    want, loss = {n: 0.0 for n in names}, 0.0
+    for part in range(2):
+        half.forward_backward(x[part * 5:part * 5 + 5].contiguous(), y[part * 5:part * 5 + 5].contiguous())
+        loss += half.loss() / 2
+        for n in names:
+            want[n] = want[n] + half.grad(n).astype(np.float64) / 2
+    for _ in range(3):  # plain, captured, replayed
+        whole.forward_backward(x, y)
+        assert whole.loss() == pytest.approx(loss, rel=2e-6)
+        rounding = 2.0 ** -8 / (10 * context)
+        bias, weight = (whole.grad(n).astype(np.float64) for n in names)
+        assert np.abs(bias - want["lm_head.bias"]).max() <= 8 * rounding
+        assert np.abs(weight - want["lm_head.weight"]).max() <= 8 * rounding * 4.0  # |z| of a layer norm of gamma 0.2: below 4
+        assert not bias[off].any() and not weight[off].any()
+    whole.close()
+    half.close()
