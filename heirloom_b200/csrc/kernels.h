@@ -180,6 +180,19 @@ int decode_greedy(hl_ctx* ctx, const float* logits, int vocab, GreedyPart* parts
 bool all_finite_f32(const float* x, size_t n);
 int decode_embed(hl_ctx* ctx, const float* table, const float* positions, const long long* state, void* out, int dtype, int dim);
 
+// Half-key gradients of the product-key form on the tensor cores (memory_keys.cu): *partial is where in the scratch the sums
+// [shares][2][side][half] end up, one per share of the tokens.  Shares: 0 where this form does not apply.
+struct KeyGradient {
+  const int64_t* idx;         // [tokens][top_k]
+  const float* query;         // [tokens][2 * half], row stride ld_query
+  long long ld_query;
+  const float* grad_scores;   // [tokens][top_k]
+  int tokens, top_k, side, half, slots;
+};
+int key_gradient_shares(const hl_ctx* ctx, const KeyGradient& k);
+size_t key_gradient_bytes(const KeyGradient& k, int shares);
+int key_gradient_run(hl_ctx* ctx, const KeyGradient& k, int shares, void* scratch, float** partial);
+
 // hl_product_key_topk_from_side_scores whose choices go to rows *kept_row and on of `kept` as well (null: nowhere else).
 int product_key_topk_impl(hl_ctx* ctx, const float* left_scores, const float* right_scores, int64_t* out, int tokens, int side, int top_k,
                           int beam, int64_t* kept, const long long* kept_row);

@@ -506,7 +506,8 @@ __global__ void selected_scores_bwd_kernel(const int64_t* __restrict__ idx, cons
 // and 64 columns of one table; per slice of 32 tokens it builds W in shared memory (one warp per token, its
 // duplicates added in slot order), multiplies with an 8 x 8 register tile per thread (two CTAs per SM), and clears the entries it
 // set.  The slots and queries of the next slice are fetched during the product (read where they were needed, the building took
-// two thirds of the time: 16384 tokens, 32 of 2 x 512 rows of 256: 386 us).  The CTA's tile goes out as a partial result that fold_key_partials_kernel adds up in block order, so the
+// two thirds of the time: 16384 tokens, 32 of 2 x 512 rows of 256: 386 us).  From 2048 tokens on key_gradient_run (memory_keys.cu)
+// takes its place where it can.  The CTA's tile goes out as a partial result that fold_key_partials_kernel adds up in block order, so the
 // result does not depend on scheduling.
 constexpr int DK_COLS = 64;    // columns per CTA
 constexpr int DK_ROWS = 256;   // table rows per CTA
@@ -1217,23 +1218,33 @@ int hl_memory_selected_scores_backward(hl_ctx* ctx, const int64_t* indices, cons
   count_launch(ctx);
   if (side > 0 && (grad_left_or_keys || grad_right_keys)) {
     const int half = key_dim / 2;
-    const size_t smem = sizeof(float) * (size_t)DK_TOKENS * (DK_ROWS + DK_COLS);
+    const KeyGradient keys{indices, query, ld_query, grad_scores, tokens, top_k, side, half, slots};
+    int token_blocks = key_gradient_shares(ctx, keys);
+    // the tensor-core form's scratch holds the queries' pieces as well: where the device has no room for them, the f32 form
+    const bool tensor = token_blocks > 0 && ensure_workspace(ctx, key_gradient_bytes(keys, token_blocks)) == HL_OK;
     const int col_blocks = ceil_div(half, DK_COLS), row_blocks = ceil_div(side, DK_ROWS);
-    const int token_blocks =
-        std::max(1, std::min(ceil_div(tokens, 64), std::max(1, (2 * ctx->sm_count) / (2 * col_blocks * row_blocks))));
-    const int tokens_per_block = ceil_div(tokens, token_blocks);
-    rc = ensure_workspace(ctx, sizeof(float) * (size_t)token_blocks * 2 * side * half);
-    if (rc != HL_OK) return rc;
+    if (!tensor) {
+      token_blocks = std::max(1, std::min(ceil_div(tokens, 64), std::max(1, (2 * ctx->sm_count) / (2 * col_blocks * row_blocks))));
+      rc = ensure_workspace(ctx, sizeof(float) * (size_t)token_blocks * 2 * side * half);
+      if (rc != HL_OK) return rc;
+    }
     float* partial = reinterpret_cast<float*>(ctx->workspace);
-    HL_CUDA(cudaFuncSetAttribute(product_key_dkeys_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    pdl(product_key_dkeys_kernel, dim3(token_blocks, col_blocks * row_blocks, 2), 256, smem, ctx->stream)(
-        indices, query, ld_query, grad_scores, partial, tokens, top_k, side, half, slots, tokens_per_block, col_blocks);
-    HL_LAUNCH_CHECK("product_key_dkeys_kernel");
+    if (tensor) {
+      rc = key_gradient_run(ctx, keys, token_blocks, ctx->workspace, &partial);
+      if (rc != HL_OK) return rc;
+    } else {
+      const size_t smem = sizeof(float) * (size_t)DK_TOKENS * (DK_ROWS + DK_COLS);
+      HL_ALLOW_SHARED(ctx, smem, product_key_dkeys_kernel);
+      pdl(product_key_dkeys_kernel, dim3(token_blocks, col_blocks * row_blocks, 2), 256, smem, ctx->stream)(
+          indices, query, ld_query, grad_scores, partial, tokens, top_k, side, half, slots, ceil_div(tokens, token_blocks), col_blocks);
+      HL_LAUNCH_CHECK("product_key_dkeys_kernel");
+      count_launch(ctx);
+    }
     const size_t total = 2 * (size_t)side * half;
     pdl(fold_key_partials_kernel, (unsigned)((total + 255) / 256), 256, 0, ctx->stream)(partial, grad_left_or_keys, grad_right_keys,
                                                                                        token_blocks, side, half);
     HL_LAUNCH_CHECK("fold_key_partials_kernel");
-    count_launch(ctx, 2);
+    count_launch(ctx);
   }
   return HL_OK;
 }

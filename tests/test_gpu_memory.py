@@ -147,6 +147,32 @@ def test_memory_layer_forward_backward_random():
     assert_close("dright", host(dr), dro, atol=1e-4, rtol=1e-4)
 
 
+@pytest.mark.parametrize("tokens,top_k,side,key_dim", [(2048, 32, 130, 128), (2049, 5, 100, 320), (3000, 32, 512, 512), (2500, 1, 7, 16), (2048, 33, 64, 64)])
+def test_half_key_gradients_of_many_tokens(tokens, top_k, side, key_dim):
+    """Ragged rows (130 = 128 + 2), columns (160 = 2.5 chunks, 8) and last stages; the last case has too many slots for the tensor-core form.
+    Slots repeat within a token, some are out of range.  f32 sums of exact products: 2^-20 of the terms' magnitudes covers both forms
+    (3e-7 measured).  The same bits every time."""
+    from heirloom_b200 import cuda
+    c = ctx()
+    gen = torch.Generator(device="cuda").manual_seed(tokens + side)
+    idx = torch.randint(0, side * side, (tokens, top_k), generator=gen, device="cuda")
+    idx[::3, -1] = idx[::3, 0]
+    idx[5, 0], idx[6, 0] = -1, side * side
+    q, kl, kr = (torch.randn(s, generator=gen, device="cuda") for s in ((tokens, key_dim), (side, key_dim // 2), (side, key_dim // 2)))
+    g = torch.randn(tokens, top_k, generator=gen, device="cuda") * 10.0 ** torch.randint(-6, 3, (tokens, 1), generator=gen, device="cuda")
+    torch.cuda.synchronize()
+    _, dl, dr = cuda.memory_selected_scores_backward(c, idx, q, kl, kr, g)
+    c.sync()
+    good = (idx >= 0) & (idx < side * side)
+    for rows, got, part in ((idx // side, dl, q[:, :key_dim // 2]), (idx % side, dr, q[:, key_dim // 2:])):
+        w = torch.zeros(tokens, side, dtype=torch.float64, device="cuda").scatter_add_(1, rows.where(good, 0), g.double() * good)
+        want, size = w.t() @ part.double(), w.abs().t() @ part.double().abs()
+        assert ((got.double() - want).abs() <= size * 2.0 ** -20).all()
+    again = cuda.memory_selected_scores_backward(c, idx, q, kl, kr, g)
+    c.sync()
+    assert torch.equal(again[1], dl) and torch.equal(again[2], dr)
+
+
 @pytest.mark.parametrize("key", ["sparse_adamw_unique_rows", "sparse_adamw_row_mask"])
 def test_sparse_adamw_known_answers(golden, key):
     from heirloom_b200 import cuda
