@@ -342,6 +342,23 @@ __device__ __forceinline__ float2 gelu_grad_fast2(float2 x) {
   return fma2(mul2(mul2(x, both(0.5f)), sech2), dinner, fma2(t, both(0.5f), both(0.5f)));
 }
 
+// Eight f32 values as three bf16 pieces each, sixteen bytes a piece: hi = bf16(x), mid = bf16(x - hi), lo = bf16(x - hi - mid).  The
+// differences are exact, so that hi + mid + lo == x whenever the three 8-bit mantissas reach the last bit of x.
+__device__ __forceinline__ void split8_bf16(const float (&x)[8], uint4 (&piece)[3]) {
+  uint32_t w[3][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float a = x[2 * i], b = x[2 * i + 1];
+    w[0][i] = pack_bf16x2(a, b);
+    a -= __uint_as_float(w[0][i] << 16);
+    b -= __uint_as_float(w[0][i] & 0xFFFF0000u);
+    w[1][i] = pack_bf16x2(a, b);
+    w[2][i] = pack_bf16x2(a - __uint_as_float(w[1][i] << 16), b - __uint_as_float(w[1][i] & 0xFFFF0000u));
+  }
+#pragma unroll
+  for (int p = 0; p < 3; ++p) piece[p] = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+}
+
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll

@@ -180,6 +180,28 @@ int decode_greedy(hl_ctx* ctx, const float* logits, int vocab, GreedyPart* parts
 bool all_finite_f32(const float* x, size_t n);
 int decode_embed(hl_ctx* ctx, const float* table, const float* positions, const long long* state, void* out, int dtype, int dim);
 
+// bf16 pieces of f32 values (elementwise.cu): piece number id[j] of row r goes to out + r * ld + j * piece, for j < n; all multiples
+// of 8 elements.  Pieces as split8_bf16 forms them.
+struct PieceDest {
+  __nv_bfloat16* out;
+  long long ld, piece;
+  int n, id[3];
+};
+// One below the other, [pieces * rows][cols], or side by side, rows of `ld` elements; the pieces in the order given.
+inline PieceDest pieces_stacked(__nv_bfloat16* out, long long rows, int cols, int n, int i0, int i1, int i2 = 0) {
+  return PieceDest{out, cols, rows * cols, n, {i0, i1, i2}};
+}
+inline PieceDest pieces_beside(__nv_bfloat16* out, long long ld, int cols, int n, int i0, int i1, int i2 = 0) {
+  return PieceDest{out, ld, cols, n, {i0, i1, i2}};
+}
+// src [rows][cols], read once.  `b` may be empty (n = 0).  cols a multiple of 8, everything on 16 bytes.
+int split_pieces(hl_ctx* ctx, const float* src, long long rows, int cols, const PieceDest& a, const PieceDest& b = PieceDest{});
+// gate = gelu(gpre), mv = weighted * gate and mv's pieces; and backward: dweighted = dmv * gate, dgpre = gelu'(gpre) dmv weighted and
+// its pieces.  Rounded to f32 after every operation, gelu in f64, as the single ops round.
+int memory_gate_forward(hl_ctx* ctx, const float* gpre, const float* weighted, float* gate, float* mv, long long rows, int cols, const PieceDest& a);
+int memory_gate_backward(hl_ctx* ctx, const float* dmv, const float* gate, const float* weighted, const float* gpre, float* dweighted, float* dgpre,
+                         long long rows, int cols, const PieceDest& a, const PieceDest& b);
+
 // Half-key gradients of the product-key form on the tensor cores (memory_keys.cu): *partial is where in the scratch the sums
 // [shares][2][side][half] end up, one per share of the tokens.  Shares: 0 where this form does not apply.
 struct KeyGradient {

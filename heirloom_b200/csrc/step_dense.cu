@@ -174,12 +174,11 @@ struct hl_decoder {
   AdamPlan *plan_tables = nullptr, *plan_no_values = nullptr;  // the memory tables alone; everything but the value table
   std::vector<MemoryActs> ma;  // indexed by layer; empty entries for dense layers
   float *m_ls = nullptr, *m_rs = nullptr, *m_scores = nullptr, *m_dmv = nullptr, *m_dweighted = nullptr, *m_dgate = nullptr,
-        *m_dgpre = nullptr, *m_dw = nullptr, *m_dscores = nullptr, *m_dq = nullptr, *m_dc2 = nullptr;
-  __nv_bfloat16 *m_dgpre_b = nullptr, *m_dq_b = nullptr;
+        *m_dgpre = nullptr, *m_dw = nullptr, *m_dscores = nullptr, *m_dq = nullptr;
   // amp route, backward of the three memory projections at f32 accuracy: bf16 pieces of the f32 operands, side by
   // side along the columns where the contraction runs along a row, one below the other where it runs down the rows
-  __nv_bfloat16 *p_dx_side = nullptr, *p_dx_rows = nullptr, *p_mv_rows = nullptr, *p_dg_side = nullptr, *p_dg_rows = nullptr,
-                *p_dq_side = nullptr, *p_dq_rows = nullptr, *p_wout_rows = nullptr, *p_wg_rows = nullptr, *p_wq_rows = nullptr;
+  __nv_bfloat16 *p_dx_side = nullptr, *p_dx_rows = nullptr, *p_mv_rows = nullptr, *p_dg_rows = nullptr, *p_dq_rows = nullptr,
+                *p_dc_side = nullptr, *p_wout_rows = nullptr, *p_wc_rows = nullptr;
   unsigned char* m_row_flags = nullptr;
   unsigned char *smft_value_mask = nullptr, *smft_left_mask = nullptr, *smft_right_mask = nullptr;  // [slots], [side], [side]
   bool smft_on = false;  // the sparse-rows step filters its rows through the three masks
@@ -363,20 +362,15 @@ void plan_memory_buffers(hl_decoder* m, uint8_t*& cur) {
   m->m_dw = carve<float>(cur, N * k);
   m->m_dscores = carve<float>(cur, N * k);
   m->m_dq = carve<float>(cur, N * kd);
-  m->m_dc2 = carve<float>(cur, N * d);
-  m->m_dgpre_b = carve<__nv_bfloat16>(cur, N * vd);
-  m->m_dq_b = carve<__nv_bfloat16>(cur, N * kd);
   if (m->cfg.precision == HL_PRECISION_AMP_BF16) {
     m->p_dx_side = carve<__nv_bfloat16>(cur, N * 2 * d);
     m->p_dx_rows = carve<__nv_bfloat16>(cur, 2 * N * d);
     m->p_mv_rows = carve<__nv_bfloat16>(cur, 3 * N * vd);
-    m->p_dg_side = carve<__nv_bfloat16>(cur, N * 2 * vd);
     m->p_dg_rows = carve<__nv_bfloat16>(cur, 3 * N * vd);
-    m->p_dq_side = carve<__nv_bfloat16>(cur, N * 2 * kd);
+    m->p_dc_side = carve<__nv_bfloat16>(cur, N * 3 * (vd + kd));
     m->p_dq_rows = carve<__nv_bfloat16>(cur, 3 * N * kd);
     m->p_wout_rows = carve<__nv_bfloat16>(cur, 3 * d * vd);
-    m->p_wg_rows = carve<__nv_bfloat16>(cur, 3 * vd * d);
-    m->p_wq_rows = carve<__nv_bfloat16>(cur, 3 * kd * d);
+    m->p_wc_rows = carve<__nv_bfloat16>(cur, 3 * (vd + kd) * d);
   }
   m->m_row_flags = carve<unsigned char>(cur, (size_t)m->mem.slots);
   m->smft_value_mask = carve<unsigned char>(cur, (size_t)m->mem.slots);
@@ -844,9 +838,7 @@ int forward(hl_decoder* m, Forward what = Forward::all) {
       HL_TRY(memory_core_forward(m, l));
       HL_TRY(g.run(N, vd, 3 * d, a.c, d, HL_K_MAJOR, ma.wg3, 3 * d, HL_K_MAJOR, ma.gpre, vd, HL_F32, HL_EPI_BIAS, P + o.bg_m,
                    nullptr, 0, nullptr, 0, d));
-      HL_TRY(hl_gelu(ctx, ma.gpre, ma.gate, HL_F32, (size_t)N * vd));
-      HL_TRY(hl_binary_f32(ctx, HL_MUL, ma.weighted, ma.gate, ma.mv, (size_t)N * vd));
-      HL_TRY(hl_split_bf16_f32(ctx, ma.mv, ma.mv_b, N, vd, HL_SPLIT_HI_LO));
+      HL_TRY(memory_gate_forward(ctx, ma.gpre, ma.weighted, ma.gate, ma.mv, N, vd, pieces_beside(ma.mv_b, 2 * vd, vd, 2, 0, 1)));
       HL_TRY(g.run(N, d, 3 * vd, ma.mv_b, 2 * vd, HL_K_MAJOR, ma.wout3, 3 * vd, HL_K_MAJOR, m->x[l + 1], d, HL_BF16,
                    HL_EPI_BIAS_RESIDUAL, P + o.bout_m, a.r, d, nullptr, 0, 2 * vd));
       continue;
@@ -1092,41 +1084,36 @@ int backward(hl_decoder* m) {
       // every product stays on the tensor cores with its f32 operands as bf16 pieces: hi*hi + lo*hi + hi*lo in one
       // f32 accumulation (the dropped lo*lo term is 2^-16 relative), or hi + mid + lo (exact) against the block input,
       // which is bf16-exact.  `side`: pieces along the columns, for operands contracted along their rows' direction;
-      // `rows`: pieces one below the other, for operands contracted down their rows.
+      // `rows`: pieces one below the other, for operands contracted down their rows.  The gradients of the two projections
+      // that read c are one product: their pieces stand side by side (hi, lo, hi), and so do the weights' (hi, hi, lo).
       const int ROWS = HL_SPLIT_STACK_ROWS;
       const float* dy = dx;  // dL/dy of this block, f32
       // out_proj: dW = dy^T mv, dmv = dy W
-      HL_TRY(hl_split_bf16_f32(ctx, dy, m->p_dx_rows, N, d, HL_SPLIT_HI_LO | ROWS));
+      HL_TRY(split_pieces(ctx, dy, N, d, pieces_stacked(m->p_dx_rows, N, d, 2, 0, 1), pieces_beside(m->p_dx_side, 2 * d, d, 2, 0, 1)));
       HL_TRY(hl_split_bf16_f32(ctx, ma.mv, m->p_mv_rows, N, vd, HL_SPLIT_HI_HI_LO | ROWS));
       HL_TRY(g.run(d, vd, 3 * N, m->p_dx_rows, d, HL_MN_MAJOR, m->p_mv_rows, vd, HL_MN_MAJOR, G + o.wout_m, vd, HL_F32,
                    HL_EPI_NONE, nullptr, nullptr, 0, nullptr, 0, 2 * N));
-      HL_TRY(hl_split_bf16_f32(ctx, dy, m->p_dx_side, N, d, HL_SPLIT_HI_LO));
       HL_TRY(hl_split_bf16_f32(ctx, P + o.wout_m, m->p_wout_rows, d, vd, HL_SPLIT_HI_HI_LO | ROWS));
       HL_TRY(g.run(N, vd, 3 * d, m->p_dx_side, 2 * d, HL_K_MAJOR, m->p_wout_rows, vd, HL_MN_MAJOR, m->m_dmv, vd, HL_F32,
                    HL_EPI_NONE, nullptr, nullptr, 0, nullptr, 0, 2 * d));
-      HL_TRY(hl_binary_f32(ctx, HL_MUL, m->m_dmv, ma.gate, m->m_dweighted, nv));
-      HL_TRY(hl_binary_f32(ctx, HL_MUL, m->m_dmv, ma.weighted, m->m_dgate, nv));
-      HL_TRY(hl_gelu_backward(ctx, ma.gpre, m->m_dgate, m->m_dgpre, HL_F32, nv));
-      // gate_proj: dW = dgpre^T c (c is bf16-exact: three exact pieces of dgpre, c read three times), dc = dgpre W
-      HL_TRY(hl_split_bf16_f32(ctx, m->m_dgpre, m->p_dg_rows, N, vd, HL_SPLIT_HI_MID_LO | ROWS));
+      // gate_proj: dW = dgpre^T c (c is bf16-exact: three exact pieces of dgpre, c read three times)
+      const int both = 3 * (vd + kd);
+      HL_TRY(memory_gate_backward(ctx, m->m_dmv, ma.gate, ma.weighted, ma.gpre, m->m_dweighted, m->m_dgpre, N, vd,
+                                  pieces_stacked(m->p_dg_rows, N, vd, 3, 0, 1, 2), pieces_beside(m->p_dc_side, both, vd, 3, 0, 1, 0)));
       HL_TRY(g.run(vd, d, 3 * N, m->p_dg_rows, vd, HL_MN_MAJOR, a.c, d, HL_MN_MAJOR, G + o.wg_m, d, HL_F32, HL_EPI_NONE,
                    nullptr, nullptr, 0, nullptr, 0, 0, N));
       HL_TRY(bias_grad_impl(ctx, m->m_dgpre, HL_F32, G + o.bg_m, N, vd, fb));
-      HL_TRY(hl_split_bf16_f32(ctx, m->m_dgpre, m->p_dg_side, N, vd, HL_SPLIT_HI_LO));
-      HL_TRY(hl_split_bf16_f32(ctx, P + o.wg_m, m->p_wg_rows, vd, d, HL_SPLIT_HI_HI_LO | ROWS));
-      HL_TRY(g.run(N, d, 3 * vd, m->p_dg_side, 2 * vd, HL_K_MAJOR, m->p_wg_rows, d, HL_MN_MAJOR, m->dtmp, d, HL_F32,
-                   HL_EPI_NONE, nullptr, nullptr, 0, nullptr, 0, 2 * vd));
       HL_TRY(memory_core_backward(m, l, m->m_dweighted));
-      // query_proj: dW = dq^T c, dc += dq W
-      HL_TRY(hl_split_bf16_f32(ctx, m->m_dq, m->p_dq_rows, N, kd, HL_SPLIT_HI_MID_LO | ROWS));
+      // query_proj: dW = dq^T c
+      HL_TRY(split_pieces(ctx, m->m_dq, N, kd, pieces_stacked(m->p_dq_rows, N, kd, 3, 0, 1, 2),
+                          pieces_beside(m->p_dc_side + 3 * vd, both, kd, 3, 0, 1, 0)));
       HL_TRY(g.run(kd, d, 3 * N, m->p_dq_rows, kd, HL_MN_MAJOR, a.c, d, HL_MN_MAJOR, G + o.wq_m, d, HL_F32, HL_EPI_NONE,
                    nullptr, nullptr, 0, nullptr, 0, 0, N));
       HL_TRY(bias_grad_impl(ctx, m->m_dq, HL_F32, G + o.bq_m, N, kd, fb));
-      HL_TRY(hl_split_bf16_f32(ctx, m->m_dq, m->p_dq_side, N, kd, HL_SPLIT_HI_LO));
-      HL_TRY(hl_split_bf16_f32(ctx, P + o.wq_m, m->p_wq_rows, kd, d, HL_SPLIT_HI_HI_LO | ROWS));
-      HL_TRY(g.run(N, d, 3 * kd, m->p_dq_side, 2 * kd, HL_K_MAJOR, m->p_wq_rows, d, HL_MN_MAJOR, m->m_dc2, d, HL_F32,
-                   HL_EPI_NONE, nullptr, nullptr, 0, nullptr, 0, 2 * kd));
-      HL_TRY(hl_binary_f32(ctx, HL_ADD, m->dtmp, m->m_dc2, m->dtmp, (size_t)N * d));
+      // dc = dgpre Wg + dq Wq
+      HL_TRY(hl_split_bf16_f32(ctx, P + o.wg_m, m->p_wc_rows, vd, d, HL_SPLIT_HI_HI_LO | ROWS));
+      HL_TRY(hl_split_bf16_f32(ctx, P + o.wq_m, m->p_wc_rows + (size_t)3 * vd * d, kd, d, HL_SPLIT_HI_HI_LO | ROWS));
+      HL_TRY(g.run(N, d, both, m->p_dc_side, both, HL_K_MAJOR, m->p_wc_rows, d, HL_MN_MAJOR, m->dtmp, d, HL_F32));
     } else {
     // y = r + fc2(gelu(fc1(c)));   dx is dL/dy (f32), a.dy its bf16 operand copy
     HL_TRY(weight_gradient(m, a.dy, d, a.g, F, G + o.w2, nullptr));

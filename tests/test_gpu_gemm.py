@@ -144,6 +144,28 @@ def test_split_pieces_rebuild_the_f32_value_exactly():
     assert np.array_equal(r[:, :72], p[:, :72]) and np.array_equal(r[:, 72:], p[:, 72:144])
 
 
+@pytest.mark.parametrize("rows,cols,shift", [(3, 8, 0), (5, 24, 0), (7, 20, 0), (5, 24, 1), (1, 1, 0), (4099, 64, 0)])
+@pytest.mark.parametrize("stacked", [0, 4])
+def test_pieces_of_any_row_length_and_alignment(rows, cols, shift, stacked):
+    """Rows of eights on sixteen bytes take eight values a thread, all others one; both leave the same pieces, also of values whose pieces
+    vanish or are subnormal, side by side and stacked."""
+    from heirloom_b200 import cuda
+    c = ctx()
+    gen = torch.Generator(device="cuda").manual_seed(rows * cols)
+    flat = torch.randn(rows * cols + shift, generator=gen, device="cuda") * 10.0 ** torch.randint(-40, 30, (rows * cols + shift,), generator=gen, device="cuda")
+    x = flat[shift:].view(rows, cols)
+    hi = x.to(torch.bfloat16)
+    mid = (x - hi.float()).to(torch.bfloat16)
+    lo = (x - hi.float() - mid.float()).to(torch.bfloat16)
+    torch.cuda.synchronize()
+    for mode, want in ((cuda.SPLIT_HI_MID_LO, (hi, mid, lo)), (cuda.SPLIT_HI_HI_LO, (hi, hi, mid)), (cuda.SPLIT_HI_LO, (hi, mid))):
+        out = torch.full((len(want) * rows * cols,), 7.0, dtype=torch.bfloat16, device="cuda")
+        torch.cuda.synchronize()
+        cuda.check(c.lib.hl_split_bf16_f32(c.handle, cuda._p(x), cuda._p(out), cuda.c_longlong(rows), cuda.c_int(cols), cuda.c_int(mode | stacked)))
+        c.sync()
+        assert torch.equal(out.view(-1), torch.cat(want, 0 if stacked else 1).reshape(-1))
+
+
 @pytest.mark.parametrize("m,n,k", [(300, 264, 128), (1024, 512, 512)])
 def test_gemm_with_a_repeated_operand_reaches_f32_accuracy(m, n, k):
     """x [m,k] bf16-exact against an f32 weight [n,k]: one accumulation over the weight's three bf16 pieces, the input
