@@ -13,7 +13,7 @@
 //
 // A CTA takes 128 rows of one table, all columns and a share of the tokens.  A stage of 32 tokens: the queries' pieces by TMA; of
 // W, eight warps put the entries of four tokens each into a tile that is zero otherwise, and take them out again before the tile
-// is used next (slots that share a row are added in slot order first, so the result does not depend on scheduling).  The same warps
+// is used next (slots that share a row are added first, in a fixed order).  The same warps
 // empty the accumulators, beside the small products of the next stage.  A stage's twelve instructions of 128 x 256 x 16 take 1536
 // cycles; bound by those warps (some 5000 cycles a stage; eight of them took 6000): 86 us for the size above, 16 more for the
 // queries' pieces.
@@ -223,24 +223,30 @@ key_gradient_kernel(const __grid_constant__ CUtensorMap map_q, const int64_t* __
           g[i] = next_g[i];
         }
         if (s + 1 < stages) fetch(t_begin + (s + 1) * KG_TOKENS);
-        // the first lane of those whose slots share a row adds the others' values in slot order
-        unsigned others[KG_TW], any = 0;
+        // The first lane of those whose slots share a row gets the sum of all: every lane holds the sum from itself up to the one
+        // that its pointer names, adds that one's and takes over its pointer.  A token's slots share few rows (a handful for 32 slots):
+        // five rounds at most where adding one after the other took up to thirty.
+        int next[KG_TW];
+        bool any = false;
 #pragma unroll
         for (int i = 0; i < KG_TW; ++i) {
-          const unsigned same = __match_any_sync(0xffffffffu, row[i]);
-          const bool leads = row[i] >= 0 && (same & ((1u << lane) - 1u)) == 0;
-          others[i] = leads ? same & ~(1u << lane) : 0u;
-          if (!leads) row[i] = -1;
-          any |= others[i];
+          const unsigned same = __match_any_sync(0xffffffffu, row[i]), above = same & ~((2u << lane) - 1u);
+          next[i] = row[i] >= 0 && above != 0 ? __ffs(above) - 1 : -1;
+          if ((same & ((1u << lane) - 1u)) != 0) row[i] = -1;
+          any |= next[i] >= 0;
         }
-        while (__any_sync(0xffffffffu, any != 0)) {
-          any = 0;
+        while (__any_sync(0xffffffffu, any)) {
+          any = false;
 #pragma unroll
-          for (int i = 0; i < KG_TW; ++i) {  // (a lane whose value is taken leads nothing, so that value is still its own)
-            const float v = __shfl_sync(0xffffffffu, g[i], others[i] ? __ffs(others[i]) - 1 : lane);
-            if (others[i]) g[i] += v;
-            others[i] &= others[i] - 1;
-            any |= others[i];
+          for (int i = 0; i < KG_TW; ++i) {
+            const int from = next[i] >= 0 ? next[i] : lane;
+            const float v = __shfl_sync(0xffffffffu, g[i], from);
+            const int further = __shfl_sync(0xffffffffu, next[i], from);
+            if (next[i] >= 0) {
+              g[i] += v;
+              next[i] = further;
+            }
+            any |= next[i] >= 0;
           }
         }
         if (!tc05::mbar_wait(&bars->empty[st], ((uint32_t)(s / KG_STAGES) & 1u) ^ 1u, abort_flag, wait_limit_ns)) { ok = false; break; }
