@@ -543,7 +543,12 @@ int flash_attention_backward_impl(hl_ctx* ctx, const void* q, const void* k, con
   CUtensorMap mq, mk, mv, mdo;
   int rc;
   // boxes of 64 channels (one 128-byte swizzle row); a head of 128 channels takes two boxes per tile and tiles of 64 keys
-  const uint32_t key_rows = head_dim == 64 ? FB_BN : 64;
+  // With keys as rows a tile is 128 keys: half the tiles of the 64-key kernel, each some 15 % longer than one of those.  So it wins where
+  // the tiles' number bounds the pass (all of them over the SMs), and loses where the longest walk does: heads (n + 1) / 2 walks of n
+  // tiles against 0.6 SMs.  Whole call with 64 and with 128 keys, us: B16 H6 T1024 (5.8 walks an SM) 188 / 126; B2 H4 T2048 (0.46) 53 / 57,
+  // B3 H5 T777 (0.41) 31.1 / 32.7, B1 H8 T512 (0.14) 22.1 / 22.8.
+  const bool transposed = head_dim == 128 && 5ll * batch * n_heads * (ceil_div(time, FB_BM) + 1) >= 6ll * ctx->sm_count;
+  const uint32_t key_rows = head_dim == 64 || transposed ? FB_BN : 64;
   if ((rc = make_tensor_map_bf16_2d(&mq, q, (uint64_t)C, rows, (uint64_t)ld_qkv, 64, FB_BM)) != HL_OK) return rc;
   if ((rc = make_tensor_map_bf16_2d(&mk, k, (uint64_t)C, rows, (uint64_t)ld_qkv, 64, key_rows)) != HL_OK) return rc;
   if ((rc = make_tensor_map_bf16_2d(&mv, v, (uint64_t)C, rows, (uint64_t)ld_qkv, 64, key_rows)) != HL_OK) return rc;
@@ -569,11 +574,14 @@ int flash_attention_backward_impl(hl_ctx* ctx, const void* q, const void* k, con
   {
     const uint64_t dims[3] = {(uint64_t)C, (uint64_t)time, (uint64_t)batch};
     const uint64_t strides[2] = {(uint64_t)ld_dqkv * 2, (uint64_t)time * (uint64_t)ld_dqkv * 2};
-    const uint32_t box[3] = {32, 32, 1};
-    if ((rc = make_tensor_map(&mdk, HL_BF16, 3, dk, dims, strides, box, 64)) != HL_OK) return rc;
-    if ((rc = make_tensor_map(&mdv, HL_BF16, 3, dv, dims, strides, box, 64)) != HL_OK) return rc;
+    const uint32_t wide = transposed ? 64 : 32;
+    const uint32_t box[3] = {wide, 32, 1};
+    if ((rc = make_tensor_map(&mdk, HL_BF16, 3, dk, dims, strides, box, (int)wide * 2)) != HL_OK) return rc;
+    if ((rc = make_tensor_map(&mdv, HL_BF16, 3, dv, dims, strides, box, (int)wide * 2)) != HL_OK) return rc;
   }
-  if (head_dim == 64) {
+  if (transposed) {
+    if ((rc = launch_attention_bwd_t(ctx, mq, mk, mv, mdo, mdq, mdk, mdv, p)) != HL_OK) return rc;
+  } else if (head_dim == 64) {
     HL_ALLOW_SHARED(ctx, FB_SMEM_BYTES, flash_attention_bwd_kernel);
     const int grid = std::min(nq * batch * n_heads, persistent_sms(ctx));
     pdl(flash_attention_bwd_kernel, grid, FB_THREADS, FB_SMEM_BYTES, ctx->stream)(mq, mk, mv, mdo, mdq, mdk, mdv, p);

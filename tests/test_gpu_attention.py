@@ -80,3 +80,10 @@ def test_flash_backward_at_the_edges_of_its_key_tiles(B, T, H):
     """Heads of 128 channels walk tiles of 64 keys against query tiles of 128: the last key tile absent, full or one row deep,
     and enough items that a CTA takes several.  (A single position's dQ and dK are exactly zero: nothing to scale a bound by.)"""
     test_flash_backward_matches_oracle(B, T, H, 128)
+
+
+@pytest.mark.parametrize("B,T,H", [(90, 2, 1), (45, 64, 2), (30, 129, 2), (60, 200, 1), (24, 600, 2)])
+def test_flash_backward_with_keys_as_rows(B, T, H):
+    """Heads of 128 channels with enough walks for every SM take tiles of 128 keys: a tile almost empty, half full, a second one of one
+    row, ragged, and several items a CTA with a ragged last tile."""
+    test_flash_backward_matches_oracle(B, T, H, 128)
