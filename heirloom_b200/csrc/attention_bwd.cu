@@ -549,10 +549,15 @@ int flash_attention_backward_impl(hl_ctx* ctx, const void* q, const void* k, con
   // B3 H5 T777 (0.41) 31.1 / 32.7, B1 H8 T512 (0.14) 22.1 / 22.8.
   const bool transposed = head_dim == 128 && 5ll * batch * n_heads * (ceil_div(time, FB_BM) + 1) >= 6ll * ctx->sm_count;
   const uint32_t key_rows = head_dim == 64 || transposed ? FB_BN : 64;
-  if ((rc = make_tensor_map_bf16_2d(&mq, q, (uint64_t)C, rows, (uint64_t)ld_qkv, 64, FB_BM)) != HL_OK) return rc;
-  if ((rc = make_tensor_map_bf16_2d(&mk, k, (uint64_t)C, rows, (uint64_t)ld_qkv, 64, key_rows)) != HL_OK) return rc;
-  if ((rc = make_tensor_map_bf16_2d(&mv, v, (uint64_t)C, rows, (uint64_t)ld_qkv, 64, key_rows)) != HL_OK) return rc;
-  if ((rc = make_tensor_map_bf16_2d(&mdo, dout, (uint64_t)C, rows, (uint64_t)ld_dout, 64, FB_BM)) != HL_OK) return rc;
+  auto operand_map = [&](CUtensorMap* map, const void* base, long long ld, uint32_t box_rows) {
+    if (transposed)  // [batch][time][channels]: rows past `time` are zeros
+      return make_tensor_map_bf16_3d(map, base, (uint64_t)C, (uint64_t)time, (uint64_t)batch, (uint64_t)ld, (uint64_t)ld * (uint64_t)time, 64, box_rows, 1);
+    return make_tensor_map_bf16_2d(map, base, (uint64_t)C, rows, (uint64_t)ld, 64, box_rows);
+  };
+  if ((rc = operand_map(&mq, q, ld_qkv, FB_BM)) != HL_OK) return rc;
+  if ((rc = operand_map(&mk, k, ld_qkv, key_rows)) != HL_OK) return rc;
+  if ((rc = operand_map(&mv, v, ld_qkv, key_rows)) != HL_OK) return rc;
+  if ((rc = operand_map(&mdo, dout, ld_dout, FB_BM)) != HL_OK) return rc;
   FbParams p{};
   p.B = batch; p.T = time; p.H = n_heads;
   p.lse = lse; p.delta = delta;

@@ -14,7 +14,7 @@ struct FbParams {
   int* status;
 };
 
-// Heads of 128 channels.  Keys as rows (attention_bwd_t.cu): boxes of 64 channels by 128 rows in mq, mk, mv and mdo, of 32 f32 channels by
+// Heads of 128 channels.  Keys as rows (attention_bwd_t.cu): boxes of 64 channels by 128 rows by one batch entry in mq, mk, mv and mdo, of 32 f32 channels by
 // 32 rows in mdq, of 64 channels by 32 keys in mdk and mdv.
 int launch_attention_bwd_t(hl_ctx* ctx, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
                            const CUtensorMap& mdq, const CUtensorMap& mdk, const CUtensorMap& mdv, const FbParams& p);

@@ -122,30 +122,31 @@ flash_attention_bwd_t_kernel(const __grid_constant__ CUtensorMap map_q, const __
       tc05::tma_prefetch_desc(&map_k);
       tc05::tma_prefetch_desc(&map_v);
       tc05::tma_prefetch_desc(&map_do);
-      auto load = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int col, int row) {
+      // rows past T are zeros, also where another batch entry follows
+      auto load = [&](uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int col, int row, int b) {
 #pragma unroll
-        for (int blk = 0; blk < BT_HD / 64; ++blk) tc05::tma_load_2d(dst + blk * BT_CHUNK, map, bar, col + blk * 64, row);
+        for (int blk = 0; blk < BT_HD / 64; ++blk) tc05::tma_load_3d(dst + blk * BT_CHUNK, map, bar, col + blk * 64, row, b);
       };
       int g = 0;
       for (BtCursor c = first; c.valid(); c = bt_next(c, p), ++g) {
-        const int row_base = c.b * p.T, col = c.h * BT_HD, qrow = row_base + c.q0(), s = g % BT_Q_STAGES;
+        const int col = c.h * BT_HD, s = g % BT_Q_STAGES;
 #pragma unroll
         for (int blk = 0; blk < BT_HD / 64; ++blk) {
-          tc05::tma_prefetch_l2_2d(&map_q, col + blk * 64, qrow);
-          tc05::tma_prefetch_l2_2d(&map_do, col + blk * 64, qrow);
+          tc05::tma_prefetch_l2_3d(&map_q, col + blk * 64, c.q0(), c.b);
+          tc05::tma_prefetch_l2_3d(&map_do, col + blk * 64, c.q0(), c.b);
         }
         if (c.it == 0) {
           if (!tc05::mbar_wait(&tail->kv_empty, ((uint32_t)c.local & 1u) ^ 1u, abort_flag)) break;
           tc05::mbar_arrive_expect_tx(&tail->kv_full, 2 * BT_OPERAND);
-          load(sk, &map_k, &tail->kv_full, col, row_base + c.kj * BT_TILE);
-          load(sv, &map_v, &tail->kv_full, col, row_base + c.kj * BT_TILE);
+          load(sk, &map_k, &tail->kv_full, col, c.kj * BT_TILE, c.b);
+          load(sv, &map_v, &tail->kv_full, col, c.kj * BT_TILE, c.b);
         }
         if (!tc05::mbar_wait(&tail->q_empty[s], ((uint32_t)(g / BT_Q_STAGES) & 1u) ^ 1u, abort_flag)) break;
         tc05::mbar_arrive_expect_tx(&tail->q_full[s], BT_OPERAND);
-        load(sq + s * BT_OPERAND, &map_q, &tail->q_full[s], col, qrow);
+        load(sq + s * BT_OPERAND, &map_q, &tail->q_full[s], col, c.q0(), c.b);
         if (!tc05::mbar_wait(&tail->do_empty, ((uint32_t)g & 1u) ^ 1u, abort_flag)) break;
         tc05::mbar_arrive_expect_tx(&tail->do_full, BT_OPERAND);
-        load(sdo, &map_do, &tail->do_full, col, qrow);
+        load(sdo, &map_do, &tail->do_full, col, c.q0(), c.b);
       }
     }
   } else if (warp == BT_SOFTMAX_WARPS + BT_DRAIN_WARPS + 1) {

@@ -87,3 +87,27 @@ def test_flash_backward_with_keys_as_rows(B, T, H):
     """Heads of 128 channels with enough walks for every SM take tiles of 128 keys: a tile almost empty, half full, a second one of one
     row, ragged, and several items a CTA with a ragged last tile."""
     test_flash_backward_matches_oracle(B, T, H, 128)
+
+
+def test_rows_of_the_next_batch_entry_stay_out_of_a_tile():
+    """192 positions leave 64 rows of the last 128-row tile empty: what the next entry holds there, infinities and NaN here, reaches none
+    of this one's gradients."""
+    from heirloom_b200 import cuda
+    c = ctx()
+    B, T, H = 60, 192, 1
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    qkv, go = (torch.randn(B * T, n * 128, generator=gen, device="cuda").to(torch.bfloat16) for n in (3, 1))
+    q, k, v = qkv.split(128, dim=1)
+    torch.cuda.synchronize()
+    out, lse = cuda.flash_attention_forward(c, q, k, v, B, T, H)
+    c.sync()
+    def run():
+        torch.cuda.synchronize()
+        return host(cuda.flash_attention_backward(c, q, k, v, out, go, lse, B, T, H)).reshape(B, T, -1)
+    want = run()
+    qkv.view(B, T, -1)[1::2, :64] = float("nan")
+    go.view(B, T, -1)[1::2, :64] = float("inf")
+    got = run()
+    # the clean entries: the same products; dQ is summed by reductions in any order, in f32, and rounded to bf16
+    assert np.isfinite(got[::2]).all()
+    assert_close("clean entries", got[::2], want[::2], atol=np.abs(want).max() * 2 ** -8)
