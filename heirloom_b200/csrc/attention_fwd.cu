@@ -146,13 +146,12 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       bool ok = true;
       int g = 0;  // key tiles loaded so far
       for (FaItem it = fa_item(0, p); ok && it.n_tiles > 0; it = fa_item(it.local + 1, p)) {
-        const int row_base = it.b * p.T;  // first row of this batch in the [B*T, *] views
         const int qb = it.local % Z::Q_BUFS;
         if (!tc05::mbar_wait(&sh->q_empty[qb], ((uint32_t)(it.local / Z::Q_BUFS) & 1u) ^ 1u, abort_flag)) break;
         tc05::mbar_arrive_expect_tx(&sh->q_full[qb], FA_Q_BYTES);
 #pragma unroll
         for (int blk = 0; blk < Z::BLOCKS; ++blk)
-          tc05::tma_load_2d(sq + qb * FA_Q_BYTES + blk * Z::Q_BLOCK, &map_q, &sh->q_full[qb], it.h * FA_HD + blk * 64, row_base + it.q0);
+          tc05::tma_load_3d(sq + qb * FA_Q_BYTES + blk * Z::Q_BLOCK, &map_q, &sh->q_full[qb], it.h * FA_HD + blk * 64, it.q0, it.b);
         for (int j = 0; j < it.n_tiles; ++j, ++g) {
           const int s = g % FA_KV_STAGES;
           const uint32_t ph = (uint32_t)(g / FA_KV_STAGES) & 1u;
@@ -161,15 +160,15 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
           tc05::mbar_arrive_expect_tx(&sh->k_full[s], FA_KV_BYTES);
 #pragma unroll
           for (int blk = 0; blk < Z::BLOCKS; ++blk)
-            tc05::tma_load_2d(sk + s * FA_KV_BYTES + blk * Z::KV_BLOCK, &map_k, &sh->k_full[s], it.h * FA_HD + blk * 64,
-                              row_base + j * FA_BN);
+            tc05::tma_load_3d(sk + s * FA_KV_BYTES + blk * Z::KV_BLOCK, &map_k, &sh->k_full[s], it.h * FA_HD + blk * 64,
+                              j * FA_BN, it.b);
           ok = tc05::mbar_wait(&sh->v_empty[s], ph ^ 1u, abort_flag);
           if (!ok) break;
           tc05::mbar_arrive_expect_tx(&sh->v_full[s], FA_KV_BYTES);
 #pragma unroll
           for (int blk = 0; blk < Z::BLOCKS; ++blk)
-            tc05::tma_load_2d(sv + s * FA_KV_BYTES + blk * Z::KV_BLOCK, &map_v, &sh->v_full[s], it.h * FA_HD + blk * 64,
-                              row_base + j * FA_BN);
+            tc05::tma_load_3d(sv + s * FA_KV_BYTES + blk * Z::KV_BLOCK, &map_v, &sh->v_full[s], it.h * FA_HD + blk * 64,
+                              j * FA_BN, it.b);
         }
       }
     }
@@ -411,13 +410,17 @@ int flash_attention_forward_impl(hl_ctx* ctx, const void* q, const void* k, cons
   HL_REQUIRE(((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
                reinterpret_cast<uintptr_t>(out)) & 15) == 0,
              "hl_flash_attention_forward: pointers must be 16-byte aligned");
-  const uint64_t rows = (uint64_t)batch * time, cols = (uint64_t)n_heads * head_dim;
+  const uint64_t cols = (uint64_t)n_heads * head_dim;
   CUtensorMap mq, mk, mv;
   int rc;
-  // boxes of 64 channels (one 128-byte swizzle row); wider heads take several boxes per tile
-  if ((rc = make_tensor_map_bf16_2d(&mq, q, cols, rows, (uint64_t)ld_qkv, 64, FA_BM)) != HL_OK) return rc;
-  if ((rc = make_tensor_map_bf16_2d(&mk, k, cols, rows, (uint64_t)ld_qkv, 64, FA_BN)) != HL_OK) return rc;
-  if ((rc = make_tensor_map_bf16_2d(&mv, v, cols, rows, (uint64_t)ld_qkv, 64, FA_BN)) != HL_OK) return rc;
+  // boxes of 64 channels (one 128-byte swizzle row); wider heads take several boxes per tile.  [batch][time][channels], so that
+  // rows past `time` are zeros: a masked P of zero times another batch entry's infinity would be NaN.
+  auto operand_map = [&](CUtensorMap* map, const void* base, uint32_t box_rows) {
+    return make_tensor_map_bf16_3d(map, base, cols, (uint64_t)time, (uint64_t)batch, (uint64_t)ld_qkv, (uint64_t)ld_qkv * (uint64_t)time, 64, box_rows, 1);
+  };
+  if ((rc = operand_map(&mq, q, FA_BM)) != HL_OK) return rc;
+  if ((rc = operand_map(&mk, k, FA_BN)) != HL_OK) return rc;
+  if ((rc = operand_map(&mv, v, FA_BN)) != HL_OK) return rc;
   // the output as [batch][time][channels], so that a tile's rows past `time` are clipped; boxes of 64 channels by 32 rows
   CUtensorMap mo;
   {

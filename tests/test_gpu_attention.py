@@ -111,3 +111,21 @@ def test_rows_of_the_next_batch_entry_stay_out_of_a_tile():
     # the clean entries: the same products; dQ is summed by reductions in any order, in f32, and rounded to bf16
     assert np.isfinite(got[::2]).all()
     assert_close("clean entries", got[::2], want[::2], atol=np.abs(want).max() * 2 ** -8)
+
+
+@pytest.mark.parametrize("B,T,H,hd", [(60, 192, 1, 128), (4, 72, 1, 128), (4, 192, 2, 64), (60, 100, 1, 64), (4, 40, 1, 64)])
+def test_rows_of_the_next_batch_entry_stay_out_of_a_forward_tile(B, T, H, hd):
+    """The same of the output and the rows' statistics, which are the same bits."""
+    from heirloom_b200 import cuda
+    c = ctx()
+    C = H * hd
+    qkv = torch.randn(B * T, 3 * C, generator=torch.Generator(device="cuda").manual_seed(9), device="cuda").to(torch.bfloat16)
+    q, k, v = qkv.split(C, dim=1)
+    def run():
+        torch.cuda.synchronize()
+        out, lse = cuda.flash_attention_forward(c, q, k, v, B, T, H)
+        return host(out).reshape(B, T, -1), host(lse)
+    want = run()
+    qkv.view(B, T, -1)[1::2, :T // 3] = float("nan")
+    got = run()
+    assert all(np.array_equal(g[::2], w[::2]) for g, w in zip(got, want))
