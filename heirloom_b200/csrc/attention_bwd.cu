@@ -147,23 +147,22 @@ flash_attention_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       tc05::tma_prefetch_desc(&map_do);
       int g = 0;  // query tiles loaded so far
       for (FbCursor c = first; c.valid(); c = fb_next(c, p), ++g) {
-        const int row_base = c.b * p.T;
         if (c.it == 0) {
           const int kb = c.local % FB_KV_BUFFERS;
           if (!tc05::mbar_wait(&bars->kv_empty[kb], ((uint32_t)(c.local / FB_KV_BUFFERS) & 1u) ^ 1u, abort_flag)) break;
           tc05::mbar_arrive_expect_tx(&bars->kv_full[kb], 2 * FB_TILE_BYTES);
-          tc05::tma_load_2d(sk + kb * FB_TILE_BYTES, &map_k, &bars->kv_full[kb], c.h * FB_HD, row_base + c.kj * FB_BN);
-          tc05::tma_load_2d(sv + kb * FB_TILE_BYTES, &map_v, &bars->kv_full[kb], c.h * FB_HD, row_base + c.kj * FB_BN);
+          tc05::tma_load_3d(sk + kb * FB_TILE_BYTES, &map_k, &bars->kv_full[kb], c.h * FB_HD, c.kj * FB_BN, c.b);
+          tc05::tma_load_3d(sv + kb * FB_TILE_BYTES, &map_v, &bars->kv_full[kb], c.h * FB_HD, c.kj * FB_BN, c.b);
         }
         const int s = g % FB_Q_STAGES;
-        const int qrow = row_base + (c.kj + c.it) * FB_BM;
+        const int qrow = (c.kj + c.it) * FB_BM;
         // the stage frees only when the tile two back has been consumed: have L2 fetch the tile in the meantime
-        tc05::tma_prefetch_l2_2d(&map_q, c.h * FB_HD, qrow);
-        tc05::tma_prefetch_l2_2d(&map_do, c.h * FB_HD, qrow);
+        tc05::tma_prefetch_l2_3d(&map_q, c.h * FB_HD, qrow, c.b);
+        tc05::tma_prefetch_l2_3d(&map_do, c.h * FB_HD, qrow, c.b);
         if (!tc05::mbar_wait(&bars->q_empty[s], ((uint32_t)(g / FB_Q_STAGES) & 1u) ^ 1u, abort_flag)) break;
         tc05::mbar_arrive_expect_tx(&bars->q_full[s], 2 * FB_TILE_BYTES);
-        tc05::tma_load_2d(sq + s * FB_TILE_BYTES, &map_q, &bars->q_full[s], c.h * FB_HD, qrow);
-        tc05::tma_load_2d(sdo + s * FB_TILE_BYTES, &map_do, &bars->q_full[s], c.h * FB_HD, qrow);
+        tc05::tma_load_3d(sq + s * FB_TILE_BYTES, &map_q, &bars->q_full[s], c.h * FB_HD, qrow, c.b);
+        tc05::tma_load_3d(sdo + s * FB_TILE_BYTES, &map_do, &bars->q_full[s], c.h * FB_HD, qrow, c.b);
       }
     }
   } else if (warp == FB_SOFTMAX_WARPS + 1) {
@@ -549,10 +548,9 @@ int flash_attention_backward_impl(hl_ctx* ctx, const void* q, const void* k, con
   // B3 H5 T777 (0.41) 31.1 / 32.7, B1 H8 T512 (0.14) 22.1 / 22.8.
   const bool transposed = head_dim == 128 && 5ll * batch * n_heads * (ceil_div(time, FB_BM) + 1) >= 6ll * ctx->sm_count;
   const uint32_t key_rows = head_dim == 64 || transposed ? FB_BN : 64;
+  // [batch][time][channels], so that rows past `time` are zeros: another batch entry's infinity there would meet a P of zero
   auto operand_map = [&](CUtensorMap* map, const void* base, long long ld, uint32_t box_rows) {
-    if (transposed)  // [batch][time][channels]: rows past `time` are zeros
-      return make_tensor_map_bf16_3d(map, base, (uint64_t)C, (uint64_t)time, (uint64_t)batch, (uint64_t)ld, (uint64_t)ld * (uint64_t)time, 64, box_rows, 1);
-    return make_tensor_map_bf16_2d(map, base, (uint64_t)C, rows, (uint64_t)ld, 64, box_rows);
+    return make_tensor_map_bf16_3d(map, base, (uint64_t)C, (uint64_t)time, (uint64_t)batch, (uint64_t)ld, (uint64_t)ld * (uint64_t)time, 64, box_rows, 1);
   };
   if ((rc = operand_map(&mq, q, ld_qkv, FB_BM)) != HL_OK) return rc;
   if ((rc = operand_map(&mk, k, ld_qkv, key_rows)) != HL_OK) return rc;

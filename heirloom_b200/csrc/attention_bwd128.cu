@@ -130,13 +130,13 @@ flash_attention_bwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
       tc05::tma_prefetch_desc(&map_do);
       int g = 0;  // query tiles loaded so far
       for (FwCursor c = first; c.valid(); c = fw_next(c, p), ++g) {
-        const int row_base = c.b * p.T, col = c.h * FW_HD;
+        const int col = c.h * FW_HD;
         const int s = g % FW_STAGES;
-        const int qrow = row_base + c.q_tile() * FW_BM;
+        const int qrow = c.q_tile() * FW_BM;
 #pragma unroll
         for (int blk = 0; blk < 2; ++blk) {
-          tc05::tma_prefetch_l2_2d(&map_q, col + blk * 64, qrow);
-          tc05::tma_prefetch_l2_2d(&map_do, col + blk * 64, qrow);
+          tc05::tma_prefetch_l2_3d(&map_q, col + blk * 64, qrow, c.b);
+          tc05::tma_prefetch_l2_3d(&map_do, col + blk * 64, qrow, c.b);
         }
         if (c.it == 0) {
           // one K/V buffer: free once the previous item's last products have been committed
@@ -144,16 +144,16 @@ flash_attention_bwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
           tc05::mbar_arrive_expect_tx(&bars->kv_full, 2 * FW_KV_BYTES);
 #pragma unroll
           for (int blk = 0; blk < 2; ++blk) {
-            tc05::tma_load_2d(sk + blk * FW_KV_BLOCK, &map_k, &bars->kv_full, col + blk * 64, row_base + c.kj * FW_BN);
-            tc05::tma_load_2d(sv + blk * FW_KV_BLOCK, &map_v, &bars->kv_full, col + blk * 64, row_base + c.kj * FW_BN);
+            tc05::tma_load_3d(sk + blk * FW_KV_BLOCK, &map_k, &bars->kv_full, col + blk * 64, c.kj * FW_BN, c.b);
+            tc05::tma_load_3d(sv + blk * FW_KV_BLOCK, &map_v, &bars->kv_full, col + blk * 64, c.kj * FW_BN, c.b);
           }
         }
         if (!tc05::mbar_wait(&bars->q_empty[s], ((uint32_t)(g / FW_STAGES) & 1u) ^ 1u, abort_flag)) break;
         tc05::mbar_arrive_expect_tx(&bars->q_full[s], 2 * FW_Q_BYTES);
 #pragma unroll
         for (int blk = 0; blk < 2; ++blk) {
-          tc05::tma_load_2d(sq + s * FW_Q_BYTES + blk * FW_Q_BLOCK, &map_q, &bars->q_full[s], col + blk * 64, qrow);
-          tc05::tma_load_2d(sdo + s * FW_Q_BYTES + blk * FW_Q_BLOCK, &map_do, &bars->q_full[s], col + blk * 64, qrow);
+          tc05::tma_load_3d(sq + s * FW_Q_BYTES + blk * FW_Q_BLOCK, &map_q, &bars->q_full[s], col + blk * 64, qrow, c.b);
+          tc05::tma_load_3d(sdo + s * FW_Q_BYTES + blk * FW_Q_BLOCK, &map_do, &bars->q_full[s], col + blk * 64, qrow, c.b);
         }
       }
     }

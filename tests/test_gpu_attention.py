@@ -89,15 +89,16 @@ def test_flash_backward_with_keys_as_rows(B, T, H):
     test_flash_backward_matches_oracle(B, T, H, 128)
 
 
-def test_rows_of_the_next_batch_entry_stay_out_of_a_tile():
-    """192 positions leave 64 rows of the last 128-row tile empty: what the next entry holds there, infinities and NaN here, reaches none
-    of this one's gradients."""
+@pytest.mark.parametrize("B,T,H,hd", [(60, 192, 1, 128), (2, 192, 2, 128), (4, 72, 1, 128), (4, 192, 2, 64), (60, 100, 1, 64), (4, 40, 1, 64)])
+def test_rows_of_the_next_batch_entry_stay_out_of_a_tile(B, T, H, hd):
+    """Positions that are no multiple of a tile leave rows of the last tile empty: what the next entry holds there, infinities and NaN
+    here, reaches none of this one's gradients (the first case takes keys as rows, the next two queries as rows)."""
     from heirloom_b200 import cuda
     c = ctx()
-    B, T, H = 60, 192, 1
+    C = H * hd
     gen = torch.Generator(device="cuda").manual_seed(9)
-    qkv, go = (torch.randn(B * T, n * 128, generator=gen, device="cuda").to(torch.bfloat16) for n in (3, 1))
-    q, k, v = qkv.split(128, dim=1)
+    qkv, go = (torch.randn(B * T, n * C, generator=gen, device="cuda").to(torch.bfloat16) for n in (3, 1))
+    q, k, v = qkv.split(C, dim=1)
     torch.cuda.synchronize()
     out, lse = cuda.flash_attention_forward(c, q, k, v, B, T, H)
     c.sync()
@@ -105,8 +106,8 @@ def test_rows_of_the_next_batch_entry_stay_out_of_a_tile():
         torch.cuda.synchronize()
         return host(cuda.flash_attention_backward(c, q, k, v, out, go, lse, B, T, H)).reshape(B, T, -1)
     want = run()
-    qkv.view(B, T, -1)[1::2, :64] = float("nan")
-    go.view(B, T, -1)[1::2, :64] = float("inf")
+    qkv.view(B, T, -1)[1::2, :T // 3] = float("nan")
+    go.view(B, T, -1)[1::2, :T // 3] = float("inf")
     got = run()
     # the clean entries: the same products; dQ is summed by reductions in any order, in f32, and rounded to bf16
     assert np.isfinite(got[::2]).all()
