@@ -33,7 +33,12 @@ constexpr int KG_THREADS = (KG_WARPS + 2) * 32;
 constexpr int KG_CHUNK = KG_TOKENS * 128;            // 64 rows or columns of a stage: 4 KB
 constexpr int KG_W_PIECE = 2 * KG_CHUNK;
 constexpr int KG_TW = KG_TOKENS / KG_WARPS;          // tokens of a warp in a stage
+constexpr int KG_SPLIT_BLOCKS = 1184;                // at most, of the kernel that cuts up the queries: eight an SM
 static_assert(KG_SMALL % KG_GROUP == 0, "the small products' accumulator is emptied at the end of a group");
+// Pieces rebuild a value only where all three are finite, and an infinity times a piece of either sign is NaN.  So where any score
+// gradient or query is this large, infinite or NaN, the sums are f32 products of the values themselves, zeros of W included, on the
+// same CTAs (some ten times as slow); below it no product or sum of up to 2^27 terms overflows.
+constexpr float kWide = 0x1p47f;
 
 template <int NC>
 struct KgLayout {  // NC: 64-column chunks
@@ -53,7 +58,8 @@ static_assert(sizeof(KgBarriers) <= 256, "barriers outgrow their place");
 
 template <int NC>
 __global__ void __launch_bounds__(KG_THREADS, 1)
-key_gradient_kernel(const __grid_constant__ CUtensorMap map_q, const int64_t* __restrict__ idx, const float* __restrict__ grad_scores,
+key_gradient_kernel(const __grid_constant__ CUtensorMap map_q, const int64_t* __restrict__ idx, const float* __restrict__ query,
+                    long long ld_query, const float* __restrict__ grad_scores, const int* __restrict__ wide_blocks, int n_wide_blocks,
                     float* __restrict__ partial, int tokens, int top_k, int side, int half, int slots, int tokens_per_block,
                     int* __restrict__ status, unsigned long long wait_limit_ns) {
   extern __shared__ __align__(1024) uint8_t kg_smem[];
@@ -64,10 +70,6 @@ key_gradient_kernel(const __grid_constant__ CUtensorMap map_q, const int64_t* __
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int table = blockIdx.z, r0 = blockIdx.y * KG_ROWS;
   const int t_begin = min(tokens, (int)blockIdx.x * tokens_per_block), t_end = min(tokens, t_begin + tokens_per_block);
-  const int stages = (t_end - t_begin + KG_TOKENS - 1) / KG_TOKENS;
-  // at the end of which stages the accumulators are emptied
-  auto ends_group = [&](int s) { return s % KG_GROUP == KG_GROUP - 1 || s == stages - 1; };
-  auto ends_small = [&](int s) { return s % KG_SMALL == KG_SMALL - 1 || s == stages - 1; };
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < KG_STAGES; ++i) {
@@ -94,6 +96,13 @@ key_gradient_kernel(const __grid_constant__ CUtensorMap map_q, const int64_t* __
   tc05::tc_fence_after_sync();
   const uint32_t tmem_large = bars->tmem_base, tmem_small = tmem_large + 256;
   pdl_begin();
+  int found = 0;
+  for (int i = threadIdx.x; i < n_wide_blocks; i += KG_THREADS) found |= __ldcg(wide_blocks + i);
+  const bool wide = __syncthreads_or(found) != 0;
+  const int stages = wide ? 0 : (t_end - t_begin + KG_TOKENS - 1) / KG_TOKENS;
+  // at the end of which stages the accumulators are emptied
+  auto ends_group = [&](int s) { return s % KG_GROUP == KG_GROUP - 1 || s == stages - 1; };
+  auto ends_small = [&](int s) { return s % KG_SMALL == KG_SMALL - 1 || s == stages - 1; };
 
   if (warp == KG_WARPS + 1) {
     // ------------------------------------------------------------------ queries
@@ -152,17 +161,17 @@ key_gradient_kernel(const __grid_constant__ CUtensorMap map_q, const int64_t* __
       const int row = (int)(table ? (unsigned)slot % side32 : (unsigned)slot / side32) - r0;
       return slot < 0 || row < 0 || row >= KG_ROWS ? -1 : row;
     };
-    int next_slot[KG_TW];  // -1: none, or none of the table
+    auto slot_of = [&](int t, int& slot, float& g) {  // this lane's of token t; -1: none, or none of the table
+      const bool in = t < t_end && lane < top_k;
+      const long long at = in ? __ldg(idx + (size_t)t * top_k + lane) : -1;
+      slot = at >= 0 && at < slots ? (int)at : -1;
+      g = in ? __ldg(grad_scores + (size_t)t * top_k + lane) : 0.f;
+    };
+    int next_slot[KG_TW];
     float next_g[KG_TW];
     auto fetch = [&](int t0) {  // of the stage whose first token is t0
 #pragma unroll
-      for (int i = 0; i < KG_TW; ++i) {
-        const int t = t0 + warp + i * KG_WARPS;
-        const bool in = t < t_end && lane < top_k;
-        const long long slot = in ? __ldg(idx + (size_t)t * top_k + lane) : -1;
-        next_slot[i] = slot >= 0 && slot < slots ? (int)slot : -1;
-        next_g[i] = in ? __ldg(grad_scores + (size_t)t * top_k + lane) : 0.f;
-      }
+      for (int i = 0; i < KG_TW; ++i) slot_of(t0 + warp + i * KG_WARPS, next_slot[i], next_g[i]);
     };
     const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
     const int col0 = (warp >> 2) * (N / 4);  // this thread's columns of its row
@@ -199,9 +208,7 @@ key_gradient_kernel(const __grid_constant__ CUtensorMap map_q, const int64_t* __
 #pragma unroll
       for (int j = 0; j < KG_TW; ++j) placed[i][j] = -1;
     auto put = [&](uint8_t* at, float x) {
-      // the largest f32 values round up to infinity in bf16: they are held at the largest bf16 value, the rest follows in the second piece
-      constexpr float kMost = 3.3895313892515355e38f;
-      const __nv_bfloat16 hi = __float2bfloat16_rn(fminf(fmaxf(x, -kMost), kMost));
+      const __nv_bfloat16 hi = __float2bfloat16_rn(x);
       const float rest = x - __bfloat162float(hi);
       const __nv_bfloat16 mid = __float2bfloat16_rn(rest);
       *reinterpret_cast<__nv_bfloat16*>(at) = hi;
@@ -209,6 +216,29 @@ key_gradient_kernel(const __grid_constant__ CUtensorMap map_q, const int64_t* __
       *reinterpret_cast<__nv_bfloat16*>(at + 2 * KG_W_PIECE) = __float2bfloat16_rn(rest - __bfloat162float(mid));
     };
     bool ok = !*abort_flag;
+    if (wide) {
+      for (int t = t_begin; t < t_end; ++t) {
+        int slot;
+        float g, w = 0.f;  // w: this thread's row of W, the token's slots in order
+        slot_of(t, slot, g);
+        const int of = row_of(slot);
+        for (int j = 0; j < top_k; ++j) {
+          const int at = __shfl_sync(0xffffffffu, of, j);
+          const float more = __shfl_sync(0xffffffffu, g, j);
+          if (at == (warp & 3) * 32 + lane) w += more;
+        }
+        const float* q = query + (size_t)t * ld_query + table * half + col0;
+#pragma unroll
+        for (int i = 0; i < N / 4; i += 4)
+          if (col0 + i < half) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(q + i));
+            sum[i] = fmaf(w, v.x, sum[i]);
+            sum[i + 1] = fmaf(w, v.y, sum[i + 1]);
+            sum[i + 2] = fmaf(w, v.z, sum[i + 2]);
+            sum[i + 3] = fmaf(w, v.w, sum[i + 3]);
+          }
+      }
+    }
     if (ok && stages > 0) fetch(t_begin);
     for (int s0 = 0; ok && s0 < stages; s0 += KG_STAGES) {
 #pragma unroll
@@ -292,9 +322,13 @@ key_gradient_kernel(const __grid_constant__ CUtensorMap map_q, const int64_t* __
   }
 }
 
-// The queries' three pieces, one below the other: eight values a thread.
-__global__ void split_queries_kernel(const float* __restrict__ query, long long ld, uint4* __restrict__ out, int tokens, int dim) {
+// The queries' three pieces, one below the other: eight values a thread; and for each block whether it met a wide value.
+__global__ void split_queries_kernel(const float* __restrict__ query, long long ld, uint4* __restrict__ out, int tokens, int dim,
+                                     const float* __restrict__ grad_scores, size_t scores, int* __restrict__ wide_blocks) {
   pdl_begin();
+  bool wide = false;
+  auto look = [&](float x) { wide |= !(fabsf(x) < kWide); };  // NaN too
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < scores; i += (size_t)gridDim.x * blockDim.x) look(__ldg(grad_scores + i));
   const size_t per_piece = (size_t)tokens * dim / 8;
   const int groups = dim / 8;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < per_piece; i += (size_t)gridDim.x * blockDim.x) {
@@ -302,28 +336,24 @@ __global__ void split_queries_kernel(const float* __restrict__ query, long long 
     const float4* src = reinterpret_cast<const float4*>(query + (size_t)t * ld + c * 8);
     const float4 a = __ldg(src), b = __ldg(src + 1);
     const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    uint32_t w[3][4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      constexpr float kMost = 3.3895313892515355e38f;
-      float lo = x[2 * j], hi = x[2 * j + 1];
-      w[0][j] = pack_bf16x2(fminf(fmaxf(lo, -kMost), kMost), fminf(fmaxf(hi, -kMost), kMost));
-      lo -= __uint_as_float(w[0][j] << 16);
-      hi -= __uint_as_float(w[0][j] & 0xFFFF0000u);
-      w[1][j] = pack_bf16x2(lo, hi);
-      w[2][j] = pack_bf16x2(lo - __uint_as_float(w[1][j] << 16), hi - __uint_as_float(w[1][j] & 0xFFFF0000u));
-    }
+    for (int j = 0; j < 8; ++j) look(x[j]);
+    uint4 piece[3];
+    split8_bf16(x, piece);
 #pragma unroll
-    for (int p = 0; p < 3; ++p) out[p * per_piece + i] = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+    for (int p = 0; p < 3; ++p) out[p * per_piece + i] = piece[p];
   }
+  const int any = __syncthreads_or(wide);
+  if (threadIdx.x == 0) wide_blocks[blockIdx.x] = any;
 }
 
 template <int NC>
-int launch_key_gradient(hl_ctx* ctx, const KeyGradient& k, const CUtensorMap& map_q, int shares, float* partial) {
+int launch_key_gradient(hl_ctx* ctx, const KeyGradient& k, const CUtensorMap& map_q, const int* wide_blocks, int n_wide_blocks, int shares,
+                        float* partial) {
   HL_ALLOW_SHARED(ctx, KgLayout<NC>::SMEM, key_gradient_kernel<NC>);
   const int tokens_per_block = ceil_div(ceil_div(k.tokens, shares), KG_TOKENS) * KG_TOKENS;
   pdl(key_gradient_kernel<NC>, dim3(shares, ceil_div(k.side, KG_ROWS), 2), KG_THREADS, KgLayout<NC>::SMEM, ctx->stream)(
-      map_q, k.idx, k.grad_scores, partial, k.tokens, k.top_k, k.side, k.half, k.slots, tokens_per_block, ctx->status_dev,
+      map_q, k.idx, k.query, k.ld_query, k.grad_scores, wide_blocks, n_wide_blocks, partial, k.tokens, k.top_k, k.side, k.half, k.slots, tokens_per_block, ctx->status_dev,
       ctx->wait_limit_ns ? ctx->wait_limit_ns : tc05::kWaitLimitNs);
   HL_LAUNCH_CHECK("key_gradient_kernel");
   count_launch(ctx);
@@ -347,24 +377,28 @@ int key_gradient_shares(const hl_ctx* ctx, const KeyGradient& k) {
   return std::max(1, std::min(ceil_div(k.tokens, 2 * KG_TOKENS), ctx->sm_count / tiles));
 }
 
-size_t key_gradient_bytes(const KeyGradient& k, int shares) { return query_bytes(k) + sizeof(float) * (size_t)shares * 2 * k.side * k.half; }
+size_t key_gradient_bytes(const KeyGradient& k, int shares) {
+  return query_bytes(k) + sizeof(int) * KG_SPLIT_BLOCKS + sizeof(float) * (size_t)shares * 2 * k.side * k.half;
+}
 
 int key_gradient_run(hl_ctx* ctx, const KeyGradient& k, int shares, void* scratch, float** partial) {
-  *partial = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + query_bytes(k));
+  int* wide_blocks = reinterpret_cast<int*>(static_cast<uint8_t*>(scratch) + query_bytes(k));
+  *partial = reinterpret_cast<float*>(wide_blocks + KG_SPLIT_BLOCKS);
   const int dim = 2 * k.half;
   const size_t groups = (size_t)k.tokens * dim / 8;
-  pdl(split_queries_kernel, (unsigned)std::min<size_t>((groups + 255) / 256, (size_t)ctx->sm_count * 8), 256, 0, ctx->stream)(
-      k.query, k.ld_query, static_cast<uint4*>(scratch), k.tokens, dim);
+  const int blocks = (int)std::min<size_t>((groups + 255) / 256, KG_SPLIT_BLOCKS);
+  pdl(split_queries_kernel, (unsigned)blocks, 256, 0, ctx->stream)(k.query, k.ld_query, static_cast<uint4*>(scratch), k.tokens, dim, k.grad_scores,
+                                                                   (size_t)k.tokens * k.top_k, wide_blocks);
   HL_LAUNCH_CHECK("split_queries_kernel");
   count_launch(ctx);
   CUtensorMap map_q;
   const int rc = make_tensor_map_bf16_3d(&map_q, scratch, (uint64_t)dim, (uint64_t)k.tokens, 3, (uint64_t)dim, (uint64_t)dim * k.tokens, 64, KG_TOKENS, 1);
   if (rc != HL_OK) return rc;
   switch (ceil_div(k.half, 64)) {
-    case 1: return launch_key_gradient<1>(ctx, k, map_q, shares, *partial);
-    case 2: return launch_key_gradient<2>(ctx, k, map_q, shares, *partial);
-    case 3: return launch_key_gradient<3>(ctx, k, map_q, shares, *partial);
-    default: return launch_key_gradient<4>(ctx, k, map_q, shares, *partial);
+    case 1: return launch_key_gradient<1>(ctx, k, map_q, wide_blocks, blocks, shares, *partial);
+    case 2: return launch_key_gradient<2>(ctx, k, map_q, wide_blocks, blocks, shares, *partial);
+    case 3: return launch_key_gradient<3>(ctx, k, map_q, wide_blocks, blocks, shares, *partial);
+    default: return launch_key_gradient<4>(ctx, k, map_q, wide_blocks, blocks, shares, *partial);
   }
 }
 

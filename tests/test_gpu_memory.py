@@ -173,6 +173,40 @@ def test_half_key_gradients_of_many_tokens(tokens, top_k, side, key_dim):
     assert torch.equal(again[1], dl) and torch.equal(again[2], dr)
 
 
+@pytest.mark.parametrize("top_k", [4, 33])
+@pytest.mark.parametrize("what,value", [("score", np.inf), ("score", -np.inf), ("score", np.nan), ("score", 3.4e38), ("score", 1e37), ("query", np.inf),
+                                        ("query", np.nan), ("query", 3.4e38), ("query", -1e30), ("both", 1e38)])
+def test_half_key_gradients_of_values_that_pieces_cannot_hold(top_k, what, value):
+    """Infinities, NaN and values whose products overflow reach the same places as in a dense product of W and the queries, zeros of W
+    included, in either form (33 slots a token: the f32 one).  f32 sums: 2^-20 of the terms' magnitudes where those stay finite."""
+    from heirloom_b200 import cuda
+    c = ctx()
+    tokens, side, key_dim = 2050, 130, 48
+    gen = torch.Generator(device="cuda").manual_seed(top_k)
+    idx = torch.randint(0, side * side, (tokens, top_k), generator=gen, device="cuda")
+    q, kl, kr, g = (torch.randn(s, generator=gen, device="cuda") for s in ((tokens, key_dim), (side, key_dim // 2), (side, key_dim // 2), (tokens, top_k)))
+    q[70, 5] = 0.0
+    if what in ("score", "both"):
+        g[70, 2] = value
+    if what == "query":
+        q[2049, 7] = q[3, key_dim - 2] = value
+    if what == "both":
+        q[70, 4], q[70, key_dim - 1] = value, -value
+    torch.cuda.synchronize()
+    _, dl, dr = cuda.memory_selected_scores_backward(c, idx, q, kl, kr, g)
+    c.sync()
+    for rows, got, part in ((idx // side, dl, q[:, :key_dim // 2]), (idx % side, dr, q[:, key_dim // 2:])):
+        w = torch.zeros(tokens, side, dtype=torch.float64, device="cuda").scatter_add_(1, rows, g.double())
+        terms = w.t()[:, :, None] * part.double()[None]  # [side, tokens, half]
+        want, size = terms.sum(1), terms.abs().sum(1)
+        overflow = want.abs() > torch.finfo(torch.float32).max
+        want = torch.where(overflow, want.sign() * float("inf"), want)
+        assert torch.equal(got.isnan(), want.isnan())
+        assert torch.equal(got.double()[want.isinf()], want[want.isinf()])
+        fine = want.isfinite()
+        assert ((got.double() - want)[fine].abs() <= size[fine] * 2.0 ** -20).all()
+
+
 @pytest.mark.parametrize("key", ["sparse_adamw_unique_rows", "sparse_adamw_row_mask"])
 def test_sparse_adamw_known_answers(golden, key):
     from heirloom_b200 import cuda
