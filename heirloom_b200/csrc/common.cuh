@@ -185,6 +185,8 @@ PdlLauncher<P...> pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, 
 }
 
 int ensure_workspace(hl_ctx* ctx, size_t bytes);
+// For a form that can be done without: false, with the arena as it was, where the device has no room for the larger one beside it.
+bool try_workspace(hl_ctx* ctx, size_t bytes);
 inline void count_launch(hl_ctx* ctx, unsigned long long n = 1) { ctx->counters.launches += n; }
 // SMs a persistent one-CTA-per-SM kernel should fill: all of them, minus those left to the collective kernels.  A CTA of
 // those kernels takes a whole SM's registers or shared memory, so it cannot start on an SM a collective kernel sits

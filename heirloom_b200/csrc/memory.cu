@@ -1221,7 +1221,7 @@ int hl_memory_selected_scores_backward(hl_ctx* ctx, const int64_t* indices, cons
     const KeyGradient keys{indices, query, ld_query, grad_scores, tokens, top_k, side, half, slots};
     int token_blocks = key_gradient_shares(ctx, keys);
     // the tensor-core form's scratch holds the queries' pieces as well: where the device has no room for them, the f32 form
-    const bool tensor = token_blocks > 0 && ensure_workspace(ctx, key_gradient_bytes(keys, token_blocks)) == HL_OK;
+    const bool tensor = token_blocks > 0 && try_workspace(ctx, key_gradient_bytes(keys, token_blocks));
     const int col_blocks = ceil_div(half, DK_COLS), row_blocks = ceil_div(side, DK_ROWS);
     if (!tensor) {
       token_blocks = std::max(1, std::min(ceil_div(tokens, 64), std::max(1, (2 * ctx->sm_count) / (2 * col_blocks * row_blocks))));

@@ -25,18 +25,39 @@ int fail_cuda(cudaError_t e, const char* what) {
   return HL_ERR_CUDA;
 }
 
+static size_t arena_bytes(size_t bytes) { return (bytes + (size_t(1) << 20) - 1) & ~((size_t(1) << 20) - 1); }
+static void adopt_arena(hl_ctx* ctx, void* arena, size_t bytes) {
+  ctx->workspace = arena;
+  ctx->workspace_bytes = bytes;
+  ctx->counters.allocations += 1;
+  ctx->counters.allocated_bytes += bytes;
+}
+
 int ensure_workspace(hl_ctx* ctx, size_t bytes) {
   if (ctx->workspace_bytes >= bytes) return HL_OK;
   // Grow-only; the old block is released in stream order so kernels still using it finish first.
   if (ctx->workspace) HL_CUDA(cudaFreeAsync(ctx->workspace, ctx->stream));
   ctx->workspace = nullptr;
   ctx->workspace_bytes = 0;
-  size_t rounded = (bytes + (size_t(1) << 20) - 1) & ~((size_t(1) << 20) - 1);
-  HL_CUDA(cudaMallocAsync(&ctx->workspace, rounded, ctx->stream));
-  ctx->workspace_bytes = rounded;
-  ctx->counters.allocations += 1;
-  ctx->counters.allocated_bytes += rounded;
+  void* arena = nullptr;
+  HL_CUDA(cudaMallocAsync(&arena, arena_bytes(bytes), ctx->stream));
+  adopt_arena(ctx, arena, arena_bytes(bytes));
   return HL_OK;
+}
+
+bool try_workspace(hl_ctx* ctx, size_t bytes) {
+  if (ctx->workspace_bytes >= bytes) return true;
+  // within a capture the block would be the graph's own
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return false;
+  void* larger = nullptr;
+  if (cudaMallocAsync(&larger, arena_bytes(bytes), ctx->stream) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (ctx->workspace) cudaFreeAsync(ctx->workspace, ctx->stream);
+  adopt_arena(ctx, larger, arena_bytes(bytes));
+  return true;
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry-point lookup.

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from oracle import heirloom_oracle as ho
-from tests.gpu_util import assert_close, ctx, dev, host
+from tests.gpu_util import assert_close, ctx, dev, full_device, host
 
 pytestmark = pytest.mark.gpu
 I64 = torch.int64
@@ -205,6 +205,39 @@ def test_half_key_gradients_of_values_that_pieces_cannot_hold(top_k, what, value
         assert torch.equal(got.double()[want.isinf()], want[want.isinf()])
         fine = want.isfinite()
         assert ((got.double() - want)[fine].abs() <= size[fine] * 2.0 ** -20).all()
+
+
+def test_half_key_gradients_without_room_for_the_tensor_cores_scratch():
+    """Where the device has no room for the larger scratch, the f32 form runs in the arena that there is: nothing is given back or
+    allocated again, call after call."""
+    from heirloom_b200 import cuda
+    tokens, top_k, side, key_dim = 4096, 8, 256, 512
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    idx = torch.randint(0, side * side, (tokens, top_k), generator=gen, device="cuda")
+    q, kl, kr, g = (torch.randn(s, generator=gen, device="cuda") for s in ((tokens, key_dim), (side, key_dim // 2), (side, key_dim // 2), (tokens, top_k)))
+    wide = torch.cat((idx, torch.full((tokens, 33 - top_k), -1, dtype=torch.int64, device="cuda")), 1)  # too many slots for the tensor-core form
+    g_wide = torch.cat((g, torch.zeros(tokens, 33 - top_k, device="cuda")), 1)
+    torch.cuda.synchronize()
+    cuda.memory_selected_scores_backward(ctx(), idx, q, kl, kr, g)  # the kernels are on the device
+    ctx().sync()
+    c = cuda.Context(0)
+    try:
+        want = cuda.memory_selected_scores_backward(c, wide, q, kl, kr, g_wide)
+        c.sync()
+        before = c.counters().allocations
+        outs = [[torch.zeros_like(t) for t in want] for _ in range(2)]  # from here on nothing is allocated in this process
+        torch.cuda.synchronize()
+        with full_device():
+            for out in outs:
+                cuda.check(c.lib.hl_memory_selected_scores_backward(
+                    c.handle, cuda._p(idx), cuda._p(q), cuda.c_longlong(key_dim), cuda._p(kl), cuda._p(kr), cuda._p(g), cuda._p(out[0]),
+                    cuda.c_longlong(key_dim), cuda._p(out[1]), cuda._p(out[2]), cuda.c_int(tokens), cuda.c_int(top_k), cuda.c_int(side),
+                    cuda.c_int(key_dim), cuda.c_int(side * side)))
+            c.sync()
+        assert c.counters().allocations == before
+        assert all(torch.equal(a, b) for out in outs for a, b in zip(out[1:], want[1:]))
+    finally:
+        c.close()
 
 
 @pytest.mark.parametrize("key", ["sparse_adamw_unique_rows", "sparse_adamw_row_mask"])
