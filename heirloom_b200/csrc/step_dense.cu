@@ -367,7 +367,7 @@ void plan_memory_buffers(hl_decoder* m, uint8_t*& cur) {
     m->p_dx_rows = carve<__nv_bfloat16>(cur, 2 * N * d);
     m->p_mv_rows = carve<__nv_bfloat16>(cur, 3 * N * vd);
     m->p_dg_rows = carve<__nv_bfloat16>(cur, 3 * N * vd);
-    m->p_dc_side = carve<__nv_bfloat16>(cur, N * 3 * (vd + kd));
+    m->p_dc_side = carve<__nv_bfloat16>(cur, N * 2 * (vd + kd));
     m->p_dq_rows = carve<__nv_bfloat16>(cur, 3 * N * kd);
     m->p_wout_rows = carve<__nv_bfloat16>(cur, 3 * d * vd);
     m->p_wc_rows = carve<__nv_bfloat16>(cur, 3 * (vd + kd) * d);
@@ -1085,7 +1085,9 @@ int backward(hl_decoder* m) {
       // f32 accumulation (the dropped lo*lo term is 2^-16 relative), or hi + mid + lo (exact) against the block input,
       // which is bf16-exact.  `side`: pieces along the columns, for operands contracted along their rows' direction;
       // `rows`: pieces one below the other, for operands contracted down their rows.  The gradients of the two projections
-      // that read c are one product: their pieces stand side by side (hi, lo, hi), and so do the weights' (hi, hi, lo).
+      // that read c are one product over both: hi*lo and lo*hi of the two, 2^-8 of the rest, come first and hi*hi after them, since the
+      // tensor core's additions truncate what it has added up so far (error against f64 of 16384 x 512 over 2 x 512: 4.5e-6, of it 4.4e-6
+      // the dropped lo*lo; a projection after the other with hi*hi first 6.2e-6, two products added up 5.1e-6).
       const int ROWS = HL_SPLIT_STACK_ROWS;
       const float* dy = dx;  // dL/dy of this block, f32
       // out_proj: dW = dy^T mv, dmv = dy W
@@ -1097,23 +1099,24 @@ int backward(hl_decoder* m) {
       HL_TRY(g.run(N, vd, 3 * d, m->p_dx_side, 2 * d, HL_K_MAJOR, m->p_wout_rows, vd, HL_MN_MAJOR, m->m_dmv, vd, HL_F32,
                    HL_EPI_NONE, nullptr, nullptr, 0, nullptr, 0, 2 * d));
       // gate_proj: dW = dgpre^T c (c is bf16-exact: three exact pieces of dgpre, c read three times)
-      const int both = 3 * (vd + kd);
+      const int both = vd + kd;
       HL_TRY(memory_gate_backward(ctx, m->m_dmv, ma.gate, ma.weighted, ma.gpre, m->m_dweighted, m->m_dgpre, N, vd,
-                                  pieces_stacked(m->p_dg_rows, N, vd, 3, 0, 1, 2), pieces_beside(m->p_dc_side, both, vd, 3, 0, 1, 0)));
+                                  pieces_stacked(m->p_dg_rows, N, vd, 3, 0, 1, 2), PieceDest{m->p_dc_side, 2 * both, both, 2, {0, 1}}));
       HL_TRY(g.run(vd, d, 3 * N, m->p_dg_rows, vd, HL_MN_MAJOR, a.c, d, HL_MN_MAJOR, G + o.wg_m, d, HL_F32, HL_EPI_NONE,
                    nullptr, nullptr, 0, nullptr, 0, 0, N));
       HL_TRY(bias_grad_impl(ctx, m->m_dgpre, HL_F32, G + o.bg_m, N, vd, fb));
       HL_TRY(memory_core_backward(m, l, m->m_dweighted));
       // query_proj: dW = dq^T c
       HL_TRY(split_pieces(ctx, m->m_dq, N, kd, pieces_stacked(m->p_dq_rows, N, kd, 3, 0, 1, 2),
-                          pieces_beside(m->p_dc_side + 3 * vd, both, kd, 3, 0, 1, 0)));
+                          PieceDest{m->p_dc_side + vd, 2 * both, both, 2, {0, 1}}));
       HL_TRY(g.run(kd, d, 3 * N, m->p_dq_rows, kd, HL_MN_MAJOR, a.c, d, HL_MN_MAJOR, G + o.wq_m, d, HL_F32, HL_EPI_NONE,
                    nullptr, nullptr, 0, nullptr, 0, 0, N));
       HL_TRY(bias_grad_impl(ctx, m->m_dq, HL_F32, G + o.bq_m, N, kd, fb));
       // dc = dgpre Wg + dq Wq
-      HL_TRY(hl_split_bf16_f32(ctx, P + o.wg_m, m->p_wc_rows, vd, d, HL_SPLIT_HI_HI_LO | ROWS));
-      HL_TRY(hl_split_bf16_f32(ctx, P + o.wq_m, m->p_wc_rows + (size_t)3 * vd * d, kd, d, HL_SPLIT_HI_HI_LO | ROWS));
-      HL_TRY(g.run(N, d, both, m->p_dc_side, both, HL_K_MAJOR, m->p_wc_rows, d, HL_MN_MAJOR, m->dtmp, d, HL_F32));
+      HL_TRY(split_pieces(ctx, P + o.wg_m, vd, d, PieceDest{m->p_wc_rows, d, (long long)both * d, 3, {1, 0, 0}}));
+      HL_TRY(split_pieces(ctx, P + o.wq_m, kd, d, PieceDest{m->p_wc_rows + (size_t)vd * d, d, (long long)both * d, 3, {1, 0, 0}}));
+      HL_TRY(g.run(N, d, 3 * both, m->p_dc_side, 2 * both, HL_K_MAJOR, m->p_wc_rows, d, HL_MN_MAJOR, m->dtmp, d, HL_F32, HL_EPI_NONE,
+                   nullptr, nullptr, 0, nullptr, 0, 2 * both));
     } else {
     // y = r + fc2(gelu(fc1(c)));   dx is dL/dy (f32), a.dy its bf16 operand copy
     HL_TRY(weight_gradient(m, a.dy, d, a.g, F, G + o.w2, nullptr));

@@ -261,3 +261,42 @@ def test_dense_plus_sparse_values_policy():
         assert np.array_equal(got[~active], p2[~active]), name
         assert np.abs(got[active] - want[active]).max() <= 2e-4, name
     model.close()
+
+
+@pytest.mark.parametrize("key_gradient", [1.0, 0.01])
+def test_the_input_gradient_of_a_memory_blocks_projections_keeps_f32_accuracy(key_gradient):
+    """dc = dgpre Wg + dq Wq leaves out the products of the two low pieces; what its accumulation adds to their error is at most a tenth
+    of it (one projection after the other in one accumulator, the large products first, added two fifths).  2048 equal rows of one
+    position: the biases' gradients are 2048 times a row's dy, dgpre, dq and, in front of the attention, dr = dy + LN'(dc)."""
+    from heirloom_b200 import nn
+    d, rows = 512, 2048
+    model = nn.DecoderLm(ctx(), nn.DecoderConfig(vocab=64, d_model=d, n_layers=1, n_heads=8, d_ff=512, context=1, batch=rows),
+                         nn.MemoryConfig(memory_layers=(0,), slots=1024, key_dim=512, value_dim=512, top_k=8))
+    rng = np.random.default_rng(5)
+    state = {n: (rng.standard_normal(s) * d ** -0.5).astype(np.float32) for n, s in model.parameter_shapes().items()}
+    mem = "block.0.feed_forward.memory."
+    for n in state:
+        if ".ln" in n or n.startswith("ln_f") or "attention" in n:
+            state[n] = np.full_like(state[n], 1.0 if n.endswith("weight") and "attention" not in n else 0.0)  # r is the embedded row
+    state["shared_memory.value"] *= 2e3     # far more comes back through the projections than around them
+    state[mem + "out_proj.weight"] *= 2e3
+    for side in ("left", "right"):
+        state["shared_memory.product_key_" + side] *= 1e-3 * key_gradient  # the routing stays soft
+    model.load_state_dict(state)
+    tokens = torch.full((rows, 1), 7, device="cuda")
+    model.forward_backward(tokens, torch.full((rows, 1), 9, device="cuda"))
+    one = lambda n: model.grad(n).astype(np.float64) / rows
+    dy, dg, dq, dr = one(mem + "out_proj.bias"), one(mem + "gate_proj.bias"), one(mem + "query_proj.bias"), one("block.0.attention.out_proj.bias")
+    r = ho.bf16_round(ho.bf16_round(state["token_embedding.weight"][7]) + ho.bf16_round(state["position_embedding.weight"][0]))
+    hat = (r - r.mean()) / np.sqrt(r.var() + 1e-5)
+    norm = lambda dc: (dc - dc.mean() - hat * (dc * hat).mean()) / np.sqrt(r.var() + 1e-5)
+    high = ho.bf16_round
+    dc, left_out = 0.0, 0.0
+    for g, w in ((dg, state[mem + "gate_proj.weight"].astype(np.float64)), (dq, state[mem + "query_proj.weight"].astype(np.float64))):
+        glo, wlo = high(g - high(g)), high(w - high(w))
+        dc = dc + g @ w
+        left_out = left_out + g @ w - (high(g) @ high(w) + glo @ high(w) + high(g) @ wlo)
+    got, want = dr - dy, norm(dc)
+    assert np.linalg.norm(dy) < 1e-3 * np.linalg.norm(want)
+    assert np.linalg.norm(got - want) <= 1.1 * np.linalg.norm(norm(left_out))
+    model.close()
