@@ -781,12 +781,20 @@ struct HeadStats {
 };
 // Whether a training step forms the logits twice, for the row sums and for their gradient, instead of storing them in f32 for the
 // loss kernel to read and turn into the gradient: 2 d flop an element (d is at most 1024 here) against eight bytes.  Bound by the
-// tensor core then instead of by the copy rate; a step under the power cap gains least, since the flop cost power as well.  Step
-// before / after, us: 4096 x 32000 x 512 2460 / 2392, 16384 x 32000 x 512 10330 / 10110, 16384 x 50304 x 768 17280 / 17260,
-// 16384 x 32000 x 64 1644 / 1419, 8192 x 2000 x 512 2700 / 2652, 1024 x 32000 x 512 1541 / 1533, 1024 x 8000 x 512 1277 / 1276.
-// Below 1024 rows the logits stay in L2 and the second product's start costs what it saves: 512 x 32000 x 512 1308 / 1311.
-constexpr int kHeadTwiceRows = 1024;
-bool head_twice_pays(const hl_decoder* m) { return m->N >= kHeadTwiceRows; }
+// tensor core then instead of by the copy rate.  Step of a one-block model, stored / twice, us, in turn in one process (quartiles 1 to
+// 3 % apart where the power cap acts): d 512, 4096 x 32000 780 / 729, 1024 x 32000 315 / 303; d 768, 16384 x 50304 5293 / 4895,
+// 2048 x 32000 562 / 551; d 1024, 16384 x 32000 4655 / 4316, 1024 x 32000 431 / 428.  In the benchmark step, whose other products
+// draw on the same power, 17280 / 17260.
+// Below 1024 rows the logits stay in L2 and the second product's start costs what it saves: d 768, 512 x 32000 277 / 286.  With few
+// columns they stay there too, and the wider rows are, the more the product costs: d 960, 1024 x 8000 264 / 270, 2048 x 2000 271 / 275,
+// d 832, 1024 x 8000 242 / 245; from 48 MB of logits or 4096 rows on even those gain (d 960, 1536 x 8000 316 / 315, 4096 x 2000
+// 409 / 388), and at d 512 all do (1024 x 8000 187 / 183), up to d 768 as many as lose (2048 x 2000 224 / 227 and 240 / 240).
+constexpr int kHeadTwiceRows = 1024, kHeadTwiceManyRows = 4096, kHeadTwiceWide = 768;
+constexpr long long kHeadTwiceLogits = 12000000;
+bool head_twice_pays(const hl_decoder* m) {
+  return m->N >= kHeadTwiceRows &&
+         (m->N >= kHeadTwiceManyRows || m->cfg.d_model <= kHeadTwiceWide || (long long)m->N * m->cfg.vocab >= kHeadTwiceLogits);
+}
 
 // What a forward pass is for: logits and activations for the backward pass, the logits of the last position alone (they go to
 // row 0 of m->logits), or the mean loss alone (to m->loss_dev).

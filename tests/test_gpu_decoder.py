@@ -488,3 +488,34 @@ def test_head_of_many_rows_equals_the_head_that_stores_its_logits(context, vocab
         assert not bias[off].any() and not weight[off].any()
     whole.close()
     half.close()
+
+
+def _profile_of_a_pass(batch, context, vocab, d_model):
+    """What the profile says that one forward and backward pass of a one-block model worked, by category."""
+    import ctypes
+    from heirloom_b200 import cuda, nn
+    from heirloom_b200._lib import Profile
+    c = ctx()
+    model = nn.DecoderLm(c, nn.DecoderConfig(batch=batch, context=context, vocab=vocab, d_model=d_model, n_layers=1, n_heads=d_model // 64, d_ff=128))
+    rng = np.random.default_rng(0)
+    model.load_state_dict({n: rng.standard_normal(s) * 0.2 for n, s in model.parameter_shapes().items()})
+    x = torch.from_numpy(rng.integers(0, vocab, (batch, context))).cuda()
+    cuda.check(c.lib.hl_profile_enable(c.handle, 1))
+    try:
+        model.forward_backward(x, x)
+        c.sync()
+        p = Profile()
+        cuda.check(c.lib.hl_profile_read(c.handle, ctypes.byref(p)))
+    finally:
+        cuda.check(c.lib.hl_profile_enable(c.handle, 0))
+        model.close()
+    return list(p.work)
+
+
+@pytest.mark.parametrize("batch,vocab,d_model,twice", [(8, 8000, 960, False), (8, 8000, 768, True), (8, 32000, 960, True), (16, 2000, 832, False),
+                                                       (12, 8000, 832, True), (32, 2000, 832, True), (7, 32000, 512, False)])
+def test_which_heads_form_their_logits_twice(batch, vocab, d_model, twice):
+    """Contexts of 128: 1024 rows, or few columns and wide rows, or too few rows.  The loss reads eight bytes for every 128 columns of a row,
+    or all of its logits."""
+    loss = _profile_of_a_pass(batch, 128, vocab, d_model)[4]
+    assert (loss < batch * 128 * vocab) == twice
