@@ -25,8 +25,7 @@ namespace {
 
 constexpr int KG_TOKENS = 32;   // a stage
 constexpr int KG_STAGES = 3;
-constexpr int KG_GROUP = 1;     // stages until the large products' accumulator is emptied
-constexpr int KG_SMALL = 32;    // stages until the small ones' is
+constexpr int KG_SMALL = 32;    // stages until the small products' accumulator is emptied
 constexpr int KG_ROWS = 128;
 constexpr int KG_WARPS = 16;
 constexpr int KG_THREADS = (KG_WARPS + 2) * 32;
@@ -34,7 +33,6 @@ constexpr int KG_CHUNK = KG_TOKENS * 128;            // 64 rows or columns of a 
 constexpr int KG_W_PIECE = 2 * KG_CHUNK;
 constexpr int KG_TW = KG_TOKENS / KG_WARPS;          // tokens of a warp in a stage
 constexpr int KG_SPLIT_BLOCKS = 1184;                // at most, of the kernel that cuts up the queries: eight an SM
-static_assert(KG_SMALL % KG_GROUP == 0, "the small products' accumulator is emptied at the end of a group");
 // Pieces rebuild a value only where all three are finite, and an infinity times a piece of either sign is NaN.  So where any score
 // gradient or query is this large, infinite or NaN, the sums are f32 products of the values themselves, zeros of W included, on the
 // same CTAs (some ten times as slow); below it no product or sum of up to 2^27 terms overflows.
@@ -100,8 +98,7 @@ key_gradient_kernel(const __grid_constant__ CUtensorMap map_q, const int64_t* __
   for (int i = threadIdx.x; i < n_wide_blocks; i += KG_THREADS) found |= __ldcg(wide_blocks + i);
   const bool wide = __syncthreads_or(found) != 0;
   const int stages = wide ? 0 : (t_end - t_begin + KG_TOKENS - 1) / KG_TOKENS;
-  // at the end of which stages the accumulators are emptied
-  auto ends_group = [&](int s) { return s % KG_GROUP == KG_GROUP - 1 || s == stages - 1; };
+  // at the end of which stages the small products' accumulator is emptied; the large ones' is at the end of each
   auto ends_small = [&](int s) { return s % KG_SMALL == KG_SMALL - 1 || s == stages - 1; };
 
   if (warp == KG_WARPS + 1) {
@@ -142,14 +139,13 @@ key_gradient_kernel(const __grid_constant__ CUtensorMap map_q, const int64_t* __
 #pragma unroll
           for (int ks = 0; ks < KG_TOKENS / 16; ++ks) product(tmem_small, kW[pair], kQ[pair], ks, s % KG_SMALL == 0 && pair == 0 && ks == 0 ? 0u : 1u);
         }
-        if (s % KG_GROUP == 0) {
-          if (!tc05::mbar_wait(&bars->large_empty, large ^ 1u, abort_flag, wait_limit_ns)) break;
-          tc05::tc_fence_after_sync();
-        }
+        if (!tc05::mbar_wait(&bars->large_empty, large ^ 1u, abort_flag, wait_limit_ns)) break;
+        tc05::tc_fence_after_sync();
 #pragma unroll
-        for (int ks = 0; ks < KG_TOKENS / 16; ++ks) product(tmem_large, 0, 0, ks, s % KG_GROUP == 0 && ks == 0 ? 0u : 1u);
+        for (int ks = 0; ks < KG_TOKENS / 16; ++ks) product(tmem_large, 0, 0, ks, ks == 0 ? 0u : 1u);
         tc05::umma_commit(&bars->empty[st]);
-        if (ends_group(s)) { tc05::umma_commit(&bars->large_full); large ^= 1u; }
+        tc05::umma_commit(&bars->large_full);
+        large ^= 1u;
         if (ends_small(s)) { tc05::umma_commit(&bars->small_full); small ^= 1u; }
         if (++st == KG_STAGES) { st = 0; phase ^= 1u; }
       }
@@ -198,7 +194,7 @@ key_gradient_kernel(const __grid_constant__ CUtensorMap map_q, const int64_t* __
     };
     uint32_t large = 0, small = 0;
     auto drain_after = [&](int s) -> bool {  // what stage s was the last one of
-      if (ends_group(s) && !drain(&bars->large_full, &bars->large_empty, tmem_large, large)) return false;
+      if (!drain(&bars->large_full, &bars->large_empty, tmem_large, large)) return false;
       return !ends_small(s) || drain(&bars->small_full, &bars->small_empty, tmem_small, small);
     };
     // where this lane's entries of each stage's tile stand (-1: nowhere), so that they can be taken out again

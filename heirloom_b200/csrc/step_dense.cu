@@ -357,7 +357,6 @@ void plan_memory_buffers(hl_decoder* m, uint8_t*& cur) {
   m->m_scores = carve<float>(cur, N * k);
   m->m_dmv = carve<float>(cur, N * vd);
   m->m_dweighted = carve<float>(cur, N * vd);
-  m->m_dgate = carve<float>(cur, N * vd);
   m->m_dgpre = carve<float>(cur, N * vd);
   m->m_dw = carve<float>(cur, N * k);
   m->m_dscores = carve<float>(cur, N * k);
@@ -371,6 +370,8 @@ void plan_memory_buffers(hl_decoder* m, uint8_t*& cur) {
     m->p_dq_rows = carve<__nv_bfloat16>(cur, 3 * N * kd);
     m->p_wout_rows = carve<__nv_bfloat16>(cur, 3 * d * vd);
     m->p_wc_rows = carve<__nv_bfloat16>(cur, 3 * (vd + kd) * d);
+  } else {
+    m->m_dgate = carve<float>(cur, N * vd);
   }
   m->m_row_flags = carve<unsigned char>(cur, (size_t)m->mem.slots);
   m->smft_value_mask = carve<unsigned char>(cur, (size_t)m->mem.slots);
@@ -764,14 +765,14 @@ struct HeadStats {
   GemmRowStats stats{};
   float* row_loss;
   bool fits;
-  explicit HeadStats(const hl_decoder* m) {
+  HeadStats(const hl_decoder* m, bool gradient) {
     const size_t N = (size_t)m->N, V = (size_t)m->cfg.vocab, parts = (size_t)ceil_div(m->cfg.vocab, 128) * N;
     desc.m = m->N; desc.n = m->cfg.vocab; desc.k = m->cfg.d_model;
     desc.a_layout = desc.b_layout = HL_K_MAJOR;
     desc.lda = desc.ldb = m->cfg.d_model; desc.ldc = m->cfg.vocab;
     desc.epilogue = HL_EPI_BIAS; desc.out_dtype = HL_F32;
     stats.parts = reinterpret_cast<float2*>(m->logits);
-    stats.rows = stats.parts + parts;
+    stats.rows = gradient ? stats.parts + parts : nullptr;
     stats.target_logit = m->logits + 2 * (parts + N);
     stats.targets = m->targets;
     stats.grad_scale = 1.0f / (float)m->N;
@@ -862,7 +863,7 @@ int forward(hl_decoder* m, Forward what = Forward::all) {
   m->head_twice = false;
   if (what == Forward::loss || head_twice_pays(m)) {
     // maxima and sums of the logits without the logits, in the buffer that would hold them
-    const HeadStats h(m);
+    const HeadStats h(m, what == Forward::all);
     int rc = HL_OK;
     if (h.fits && gemm_bf16_row_stats(ctx, &h.desc, m->z, W + m->off_head_w, P + m->off_head_b, h.stats, m->logits, &rc)) {
       HL_TRY(rc);
@@ -1053,7 +1054,7 @@ int backward(hl_decoder* m) {
   }
   // loss and dlogits = (softmax - onehot)/N in bf16, the operand precision of the next GEMMs
   if (m->head_twice) {
-    const HeadStats h(m);
+    const HeadStats h(m, true);
     HL_TRY(row_stats_loss(ctx, h.stats, N, V, h.row_loss, m->loss_dev, m->loss_host));
     HL_TRY(gemm_bf16_loss_gradient(ctx, &h.desc, m->z, W + m->off_head_w, P + m->off_head_b, h.stats, m->dlogits));
   } else {
@@ -1087,7 +1088,6 @@ int backward(hl_decoder* m) {
       // y = r + out_proj(weighted * gelu(gate_proj(c))), weighted from the lookup on query_proj(c)
       MemoryActs& ma = m->ma[l];
       const int kd = m->mem.key_dim, vd = m->mem.value_dim;
-      const size_t nv = (size_t)N * vd;
       // The reference runs these three projections in f32 also backward (src/memory_transformer.rs:787-789).  Here
       // every product stays on the tensor cores with its f32 operands as bf16 pieces: hi*hi + lo*hi + hi*lo in one
       // f32 accumulation (the dropped lo*lo term is 2^-16 relative), or hi + mid + lo (exact) against the block input,
