@@ -206,7 +206,7 @@ __device__ __forceinline__ bool get_item(const GemmParams& p, int local, WorkIte
 // SPEC_ROW_STATS: bias, and no output but, per row and 128 columns, the maximum and the sum of exponentials below it, and the
 // row's value at its target column (a loss reads nothing else of the logits).
 // SPEC_LOSS_GRADIENT: bias, then the gradient of the loss in bf16, out of the row's maximum and sum: with SPEC_ROW_STATS before it
-// the logits are formed twice and never stored.  Rule and figures: gemm_bf16_row_stats below.
+// the logits are formed twice and never stored.  Rule and figures: head_twice_pays in step_dense.cu.
 constexpr int SPEC_PARTIAL = 16;
 constexpr int SPEC_ROW_STATS = 32;
 constexpr int SPEC_LOSS_GRADIENT = 34;
@@ -1132,7 +1132,8 @@ int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void*
 
   const int total = p.m_tiles * p.n_tiles * p.splits;
   const int grid = pair ? 2 * min(total, sms / 2) : plan.sk_tiles > 0 ? sms : min(total, sms);
-  ProfileScope prof(ctx, HL_PROF_GEMM, 2.0 * (double)d->m * (double)d->n * (double)d->k);
+  const bool again = row_stats && d->out_dtype == HL_BF16;  // the product of gemm_bf16_row_stats once more: time, but no work that was asked for
+  ProfileScope prof(ctx, HL_PROF_GEMM, again ? 0.0 : 2.0 * (double)d->m * (double)d->n * (double)d->k);
   // Whole-tile products have kernels compiled for one epilogue and output type where a training step or an evaluation runs them (operand
   // order, pairing and epilogue as they occur there): the generic kernel carries every epilogue behind run-time branches in its
   // column loop and is bound by instruction supply (fc1 forward 105 us, its own kernel 87; out_proj forward 36 and 30;

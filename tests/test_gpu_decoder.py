@@ -512,6 +512,12 @@ def _profile_of_a_pass(batch, context, vocab, d_model):
     return list(p.work)
 
 
+def test_the_heads_second_product_counts_as_time_and_not_as_work():
+    """Rates are made of what a step needs: with 1030 rows, whose logits are formed twice, the profile reports the products' flop of two
+    passes of 515."""
+    assert _profile_of_a_pass(10, 103, 8200, 128)[0] == 2 * _profile_of_a_pass(5, 103, 8200, 128)[0]
+
+
 @pytest.mark.parametrize("batch,vocab,d_model,twice", [(8, 8000, 960, False), (8, 8000, 768, True), (8, 32000, 960, True), (16, 2000, 832, False),
                                                        (12, 8000, 832, True), (32, 2000, 832, True), (7, 32000, 512, False)])
 def test_which_heads_form_their_logits_twice(batch, vocab, d_model, twice):
