@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(KG_THREADS, 1)
 key_gradient_kernel(const __grid_constant__ CUtensorMap map_q, const int64_t* __restrict__ idx, const float* __restrict__ query,
                     long long ld_query, const float* __restrict__ grad_scores, const int* __restrict__ wide_blocks, int n_wide_blocks,
                     float* __restrict__ partial, int tokens, int top_k, int side, int half, int slots, int tokens_per_block,
-                    int* __restrict__ status, unsigned long long wait_limit_ns) {
+                    int* __restrict__ status, unsigned long long wait_limit_ns, int skip_stage) {
   extern __shared__ __align__(1024) uint8_t kg_smem[];
   using L = KgLayout<NC>;
   constexpr int N = NC * 64;
@@ -109,6 +109,7 @@ key_gradient_kernel(const __grid_constant__ CUtensorMap map_q, const int64_t* __
       uint32_t phase = 0;
       for (int s = 0; s < stages; ++s) {
         if (!tc05::mbar_wait(&bars->empty[st], phase ^ 1u, abort_flag, wait_limit_ns)) break;
+        if (s == skip_stage) break;  // test hook: this stage never fills
         tc05::mbar_arrive_expect_tx(&bars->full[st], 3 * L::Q_PIECE);
         uint8_t* q = kg_smem + st * L::STAGE + 3 * KG_W_PIECE;
         for (int p = 0; p < 3; ++p)
@@ -349,8 +350,8 @@ int launch_key_gradient(hl_ctx* ctx, const KeyGradient& k, const CUtensorMap& ma
   HL_ALLOW_SHARED(ctx, KgLayout<NC>::SMEM, key_gradient_kernel<NC>);
   const int tokens_per_block = ceil_div(ceil_div(k.tokens, shares), KG_TOKENS) * KG_TOKENS;
   pdl(key_gradient_kernel<NC>, dim3(shares, ceil_div(k.side, KG_ROWS), 2), KG_THREADS, KgLayout<NC>::SMEM, ctx->stream)(
-      map_q, k.idx, k.query, k.ld_query, k.grad_scores, wide_blocks, n_wide_blocks, partial, k.tokens, k.top_k, k.side, k.half, k.slots, tokens_per_block, ctx->status_dev,
-      ctx->wait_limit_ns ? ctx->wait_limit_ns : tc05::kWaitLimitNs);
+      map_q, k.idx, k.query, k.ld_query, k.grad_scores, wide_blocks, n_wide_blocks, partial, k.tokens, k.top_k, k.side, k.half, k.slots,
+      tokens_per_block, ctx->status_dev, ctx->wait_limit_ns ? ctx->wait_limit_ns : tc05::kWaitLimitNs, ctx->gemm_skip_kblock);
   HL_LAUNCH_CHECK("key_gradient_kernel");
   count_launch(ctx);
   return HL_OK;

@@ -453,13 +453,14 @@ def test_clipping_by_the_global_norm_of_a_dense_step(precision):
             assert np.abs(got[n][1] - want).max() <= 4 * 2.0 ** -24 * (np.abs(0.1 * factor * g[n]).max() + np.abs(1e-3 * before[n]).max()) + 1e-12, n
 
 
-@pytest.mark.parametrize("context,vocab,masked", [(103, 8200, False), (128, 5000, False), (128, 5000, True), (103, 16384, True)])
-def test_head_of_many_rows_equals_the_head_that_stores_its_logits(context, vocab, masked):
+@pytest.mark.parametrize("context,vocab,masked,d_model", [(103, 8200, False, 128), (128, 5000, False, 128), (128, 5000, True, 128), (103, 16384, True, 128),
+                                                          (128, 4104, False, 320), (103, 12000, True, 1024)])
+def test_head_of_many_rows_equals_the_head_that_stores_its_logits(context, vocab, masked, d_model):
     """From 1024 rows on the logits are formed twice instead of stored (1030 and 1280 rows, ragged last columns): loss and head
     gradients are the average of those of two halves below that, in whose scale the same bf16 values are a factor of two larger.
     A gradient of a row may round the other way (a few of a column's, each at most 2^-8 of 1 / rows); masked columns have none."""
     from heirloom_b200 import nn
-    kw = dict(vocab=vocab, d_model=128, n_layers=1, n_heads=2, d_ff=128, context=context)
+    kw = dict(vocab=vocab, d_model=d_model, n_layers=1, n_heads=d_model // 64, d_ff=128, context=context)
     rng = np.random.default_rng(vocab)
     c = ctx()
     whole, half = nn.DecoderLm(c, nn.DecoderConfig(batch=10, **kw)), nn.DecoderLm(c, nn.DecoderConfig(batch=5, **kw))

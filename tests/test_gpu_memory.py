@@ -147,9 +147,11 @@ def test_memory_layer_forward_backward_random():
     assert_close("dright", host(dr), dro, atol=1e-4, rtol=1e-4)
 
 
-@pytest.mark.parametrize("tokens,top_k,side,key_dim", [(2048, 32, 130, 128), (2049, 5, 100, 320), (3000, 32, 512, 512), (2500, 1, 7, 16), (2048, 33, 64, 64)])
+@pytest.mark.parametrize("tokens,top_k,side,key_dim", [(2048, 32, 130, 128), (2049, 5, 100, 320), (3000, 32, 512, 512), (2500, 1, 7, 16), (2048, 33, 64, 64),
+                                                       (4200, 8, 2048, 64), (9000, 4, 2048, 512)])
 def test_half_key_gradients_of_many_tokens(tokens, top_k, side, key_dim):
-    """Ragged rows (130 = 128 + 2), columns (160 = 2.5 chunks, 8) and last stages; the last case has too many slots for the tensor-core form.
+    """Ragged rows (130 = 128 + 2), columns (160 = 2.5 chunks, 8) and last stages; one case has too many slots for the tensor-core form, and
+    with 2048 rows a CTA walks 33 and 71 stages, past the 32 after which the small products' accumulator is emptied, once and twice.
     Slots repeat within a token, some are out of range.  f32 sums of exact products: 2^-20 of the terms' magnitudes covers both forms
     (3e-7 measured).  The same bits every time."""
     from heirloom_b200 import cuda
@@ -238,6 +240,72 @@ def test_half_key_gradients_without_room_for_the_tensor_cores_scratch():
         assert all(torch.equal(a, b) for out in outs for a, b in zip(out[1:], want[1:]))
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("stage", [0, 4])
+def test_a_half_key_gradient_whose_wait_runs_out_reports_it_and_the_next_call_is_right(stage):
+    """A stage of tokens that the test hook keeps from arriving: every role leaves, and the next synchronisation reports the status."""
+    from heirloom_b200 import cuda
+    from heirloom_b200._lib import HeirloomError
+    c = ctx()
+    gen = torch.Generator(device="cuda").manual_seed(stage)
+    idx = torch.randint(0, 900 * 900, (4096, 8), generator=gen, device="cuda")  # eight to fifteen stages a CTA
+    q, kl, kr, g = (torch.randn(s, generator=gen, device="cuda") for s in ((4096, 128), (900, 64), (900, 64), (4096, 8)))
+    torch.cuda.synchronize()
+    want = cuda.memory_selected_scores_backward(c, idx, q, kl, kr, g)
+    c.sync()
+    c.set_test_hooks(wait_limit_ns=200_000, gemm_skip_kblock=stage)
+    try:
+        cuda.memory_selected_scores_backward(c, idx, q, kl, kr, g)
+        with pytest.raises(HeirloomError, match="bounded pipeline wait expired"):
+            c.sync()
+    finally:
+        c.set_test_hooks(0, -1)
+    again = cuda.memory_selected_scores_backward(c, idx, q, kl, kr, g)
+    c.sync()
+    assert all(torch.equal(a, w) for a, w in zip(again, want))
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (37, 64), (4096, 520)])
+def test_the_fused_gate_rounds_as_the_single_ops(rows, cols):
+    """gelu, products and pieces of a memory block's gate in one pass, forward and backward: the bits of an op after the other."""
+    import ctypes
+    from heirloom_b200 import cuda
+    c = ctx()
+
+    class Dest(ctypes.Structure):
+        _fields_ = [("out", ctypes.c_void_p), ("ld", ctypes.c_longlong), ("piece", ctypes.c_longlong), ("n", ctypes.c_int), ("id", ctypes.c_int * 3)]
+
+    forward = c.lib["_ZN2hl19memory_gate_forwardEP6hl_ctxPKfS3_PfS4_xiRKNS_9PieceDestE"]  # no entry point of the C header
+    backward = c.lib["_ZN2hl20memory_gate_backwardEP6hl_ctxPKfS3_S3_S3_PfS4_xiRKNS_9PieceDestES7_"]
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    gpre, weighted, dmv = (torch.randn(rows, cols, generator=gen, device="cuda") * 3 for _ in range(3))
+    new = lambda *shape, dtype=torch.float32: torch.full(shape, 7.0, dtype=dtype, device="cuda")
+    gate, mv, dweighted, dgpre = (new(rows, cols) for _ in range(4))
+    beside, stacked = new(rows, 2 * cols + 8, dtype=torch.bfloat16), new(3 * rows, cols, dtype=torch.bfloat16)
+    side = Dest(beside.data_ptr(), 2 * cols + 8, cols, 2, (ctypes.c_int * 3)(0, 1, 0))
+    rest = Dest(stacked.data_ptr(), cols, rows * cols, 3, (ctypes.c_int * 3)(0, 1, 2))
+
+    def pieces(x):
+        hi = x.to(torch.bfloat16)
+        mid = (x - hi.float()).to(torch.bfloat16)
+        return hi, mid, (x - hi.float() - mid.float()).to(torch.bfloat16)
+
+    torch.cuda.synchronize()
+    cuda.check(forward(c.handle, cuda._p(gpre), cuda._p(weighted), cuda._p(gate), cuda._p(mv), cuda.c_longlong(rows), cuda.c_int(cols), ctypes.byref(side)))
+    want_gate = cuda.gelu(c, gpre)
+    want_mv = cuda.binary_f32(c, 2, weighted, want_gate)
+    c.sync()
+    assert torch.equal(gate, want_gate) and torch.equal(mv, want_mv)
+    assert torch.equal(beside[:, :2 * cols], torch.cat(pieces(mv)[:2], 1)) and (beside[:, 2 * cols:] == 7).all()
+    cuda.check(backward(c.handle, cuda._p(dmv), cuda._p(gate), cuda._p(weighted), cuda._p(gpre), cuda._p(dweighted), cuda._p(dgpre),
+                        cuda.c_longlong(rows), cuda.c_int(cols), ctypes.byref(rest), ctypes.byref(side)))
+    want_dweighted = cuda.binary_f32(c, 2, dmv, gate)
+    want_dgpre = cuda.gelu_backward(c, gpre, cuda.binary_f32(c, 2, dmv, weighted))
+    c.sync()
+    assert torch.equal(dweighted, want_dweighted) and torch.equal(dgpre, want_dgpre)
+    assert torch.equal(stacked, torch.cat(pieces(dgpre), 0))
+    assert torch.equal(beside[:, :2 * cols], torch.cat(pieces(dgpre)[:2], 1)) and (beside[:, 2 * cols:] == 7).all()
 
 
 @pytest.mark.parametrize("key", ["sparse_adamw_unique_rows", "sparse_adamw_row_mask"])
