@@ -203,7 +203,8 @@ int memory_gate_backward(hl_ctx* ctx, const float* dmv, const float* gate, const
                          long long rows, int cols, const PieceDest& a, const PieceDest& b);
 
 // Half-key gradients of the product-key form on the tensor cores (memory_keys.cu): *partial is where in the scratch the sums
-// [shares][2][side][half] end up, one per share of the tokens.  Shares: 0 where this form does not apply.
+// [shares][2][side][half] end up, one per share of the tokens.  Shares: 0 where this form does not apply.  The scratch's first word is
+// zero before the call.
 struct KeyGradient {
   const int64_t* idx;         // [tokens][top_k]
   const float* query;         // [tokens][2 * half], row stride ld_query

@@ -420,8 +420,9 @@ __global__ void selected_scores_bwd_kernel(const int64_t* __restrict__ idx, cons
                                            const float* __restrict__ left, const float* __restrict__ right,
                                            const float* __restrict__ grad_scores, float* __restrict__ dq, long long ld_dq,
                                            float* __restrict__ dleft, float* __restrict__ dright, int tokens, int top_k,
-                                           int side, int key_dim, int slots) {
+                                           int side, int key_dim, int slots, int* __restrict__ clear) {
   pdl_begin();
+  if (clear && blockIdx.x == 0 && threadIdx.x == 0) *clear = 0;  // a word that the kernels behind this one set and read
   const int lane = threadIdx.x & 31;
   const int token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (token >= tokens) return;
@@ -1211,17 +1212,18 @@ int hl_memory_selected_scores_backward(hl_ctx* ctx, const int64_t* indices, cons
   int rc = check_memory_dims(tokens, top_k, key_dim, "hl_memory_selected_scores_backward");
   if (rc != HL_OK) return rc;
   HL_REQUIRE(side == 0 || (right_keys && key_dim % 2 == 0), "hl_memory_selected_scores_backward: product-key mode needs both half tables");
+  const int half = key_dim / 2;
+  const KeyGradient keys{indices, query, ld_query, grad_scores, tokens, top_k, side, half, slots};
+  const bool half_keys = side > 0 && (grad_left_or_keys || grad_right_keys);
+  int token_blocks = half_keys ? key_gradient_shares(ctx, keys) : 0;
+  // the tensor-core form's scratch holds the queries' pieces as well: where the device has no room for them, the f32 form
+  const bool tensor = token_blocks > 0 && try_workspace(ctx, key_gradient_bytes(keys, token_blocks));
   pdl(selected_scores_bwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream)(
       indices, query, ld_query, left_or_keys, right_keys, grad_scores, grad_query, ld_grad_query, grad_left_or_keys,
-      grad_right_keys, tokens, top_k, side, key_dim, slots);
+      grad_right_keys, tokens, top_k, side, key_dim, slots, tensor ? static_cast<int*>(ctx->workspace) : nullptr);
   HL_LAUNCH_CHECK("selected_scores_bwd_kernel");
   count_launch(ctx);
-  if (side > 0 && (grad_left_or_keys || grad_right_keys)) {
-    const int half = key_dim / 2;
-    const KeyGradient keys{indices, query, ld_query, grad_scores, tokens, top_k, side, half, slots};
-    int token_blocks = key_gradient_shares(ctx, keys);
-    // the tensor-core form's scratch holds the queries' pieces as well: where the device has no room for them, the f32 form
-    const bool tensor = token_blocks > 0 && try_workspace(ctx, key_gradient_bytes(keys, token_blocks));
+  if (half_keys) {
     const int col_blocks = ceil_div(half, DK_COLS), row_blocks = ceil_div(side, DK_ROWS);
     if (!tensor) {
       token_blocks = std::max(1, std::min(ceil_div(tokens, 64), std::max(1, (2 * ctx->sm_count) / (2 * col_blocks * row_blocks))));

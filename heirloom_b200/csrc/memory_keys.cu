@@ -32,7 +32,6 @@ constexpr int KG_THREADS = (KG_WARPS + 2) * 32;
 constexpr int KG_CHUNK = KG_TOKENS * 128;            // 64 rows or columns of a stage: 4 KB
 constexpr int KG_W_PIECE = 2 * KG_CHUNK;
 constexpr int KG_TW = KG_TOKENS / KG_WARPS;          // tokens of a warp in a stage
-constexpr int KG_SPLIT_BLOCKS = 1184;                // at most, of the kernel that cuts up the queries: eight an SM
 // Pieces rebuild a value only where all three are finite, and an infinity times a piece of either sign is NaN.  So where any score
 // gradient or query is this large, infinite or NaN, the sums are f32 products of the values themselves, zeros of W included, on the
 // same CTAs (some ten times as slow); below it no product or sum of up to 2^27 terms overflows.
@@ -57,7 +56,7 @@ static_assert(sizeof(KgBarriers) <= 256, "barriers outgrow their place");
 template <int NC>
 __global__ void __launch_bounds__(KG_THREADS, 1)
 key_gradient_kernel(const __grid_constant__ CUtensorMap map_q, const int64_t* __restrict__ idx, const float* __restrict__ query,
-                    long long ld_query, const float* __restrict__ grad_scores, const int* __restrict__ wide_blocks, int n_wide_blocks,
+                    long long ld_query, const float* __restrict__ grad_scores, const int* __restrict__ wide_seen,
                     float* __restrict__ partial, int tokens, int top_k, int side, int half, int slots, int tokens_per_block,
                     int* __restrict__ status, unsigned long long wait_limit_ns, int skip_stage) {
   extern __shared__ __align__(1024) uint8_t kg_smem[];
@@ -94,9 +93,7 @@ key_gradient_kernel(const __grid_constant__ CUtensorMap map_q, const int64_t* __
   tc05::tc_fence_after_sync();
   const uint32_t tmem_large = bars->tmem_base, tmem_small = tmem_large + 256;
   pdl_begin();
-  int found = 0;
-  for (int i = threadIdx.x; i < n_wide_blocks; i += KG_THREADS) found |= __ldcg(wide_blocks + i);
-  const bool wide = __syncthreads_or(found) != 0;
+  const bool wide = __ldcg(wide_seen) != 0;
   const int stages = wide ? 0 : (t_end - t_begin + KG_TOKENS - 1) / KG_TOKENS;
   // at the end of which stages the small products' accumulator is emptied; the large ones' is at the end of each
   auto ends_small = [&](int s) { return s % KG_SMALL == KG_SMALL - 1 || s == stages - 1; };
@@ -319,9 +316,9 @@ key_gradient_kernel(const __grid_constant__ CUtensorMap map_q, const int64_t* __
   }
 }
 
-// The queries' three pieces, one below the other: eight values a thread; and for each block whether it met a wide value.
+// The queries' three pieces, one below the other: eight values a thread; and whether any value is too wide for pieces.
 __global__ void split_queries_kernel(const float* __restrict__ query, long long ld, uint4* __restrict__ out, int tokens, int dim,
-                                     const float* __restrict__ grad_scores, size_t scores, int* __restrict__ wide_blocks) {
+                                     const float* __restrict__ grad_scores, size_t scores, int* __restrict__ wide_seen) {
   pdl_begin();
   bool wide = false;
   auto look = [&](float x) { wide |= !(fabsf(x) < kWide); };  // NaN too
@@ -340,23 +337,22 @@ __global__ void split_queries_kernel(const float* __restrict__ query, long long 
 #pragma unroll
     for (int p = 0; p < 3; ++p) out[p * per_piece + i] = piece[p];
   }
-  const int any = __syncthreads_or(wide);
-  if (threadIdx.x == 0) wide_blocks[blockIdx.x] = any;
+  if (wide) *wide_seen = 1;
 }
 
 template <int NC>
-int launch_key_gradient(hl_ctx* ctx, const KeyGradient& k, const CUtensorMap& map_q, const int* wide_blocks, int n_wide_blocks, int shares,
-                        float* partial) {
+int launch_key_gradient(hl_ctx* ctx, const KeyGradient& k, const CUtensorMap& map_q, const int* wide_seen, int shares, float* partial) {
   HL_ALLOW_SHARED(ctx, KgLayout<NC>::SMEM, key_gradient_kernel<NC>);
   const int tokens_per_block = ceil_div(ceil_div(k.tokens, shares), KG_TOKENS) * KG_TOKENS;
   pdl(key_gradient_kernel<NC>, dim3(shares, ceil_div(k.side, KG_ROWS), 2), KG_THREADS, KgLayout<NC>::SMEM, ctx->stream)(
-      map_q, k.idx, k.query, k.ld_query, k.grad_scores, wide_blocks, n_wide_blocks, partial, k.tokens, k.top_k, k.side, k.half, k.slots,
-      tokens_per_block, ctx->status_dev, ctx->wait_limit_ns ? ctx->wait_limit_ns : tc05::kWaitLimitNs, ctx->gemm_skip_kblock);
+      map_q, k.idx, k.query, k.ld_query, k.grad_scores, wide_seen, partial, k.tokens, k.top_k, k.side, k.half, k.slots, tokens_per_block,
+      ctx->status_dev, ctx->wait_limit_ns ? ctx->wait_limit_ns : tc05::kWaitLimitNs, ctx->gemm_skip_kblock);
   HL_LAUNCH_CHECK("key_gradient_kernel");
   count_launch(ctx);
   return HL_OK;
 }
 
+constexpr size_t kWideWordBytes = 256;  // in front of the pieces: the word that says whether a value is too wide for them
 size_t query_bytes(const KeyGradient& k) { return ((size_t)k.tokens * k.half * 2 * 3 * sizeof(__nv_bfloat16) + 255) & ~size_t(255); }
 
 }  // namespace
@@ -375,27 +371,27 @@ int key_gradient_shares(const hl_ctx* ctx, const KeyGradient& k) {
 }
 
 size_t key_gradient_bytes(const KeyGradient& k, int shares) {
-  return query_bytes(k) + sizeof(int) * KG_SPLIT_BLOCKS + sizeof(float) * (size_t)shares * 2 * k.side * k.half;
+  return kWideWordBytes + query_bytes(k) + sizeof(float) * (size_t)shares * 2 * k.side * k.half;
 }
 
 int key_gradient_run(hl_ctx* ctx, const KeyGradient& k, int shares, void* scratch, float** partial) {
-  int* wide_blocks = reinterpret_cast<int*>(static_cast<uint8_t*>(scratch) + query_bytes(k));
-  *partial = reinterpret_cast<float*>(wide_blocks + KG_SPLIT_BLOCKS);
+  int* wide_seen = static_cast<int*>(scratch);
+  uint8_t* pieces = static_cast<uint8_t*>(scratch) + kWideWordBytes;
+  *partial = reinterpret_cast<float*>(pieces + query_bytes(k));
   const int dim = 2 * k.half;
   const size_t groups = (size_t)k.tokens * dim / 8;
-  const int blocks = (int)std::min<size_t>((groups + 255) / 256, KG_SPLIT_BLOCKS);
-  pdl(split_queries_kernel, (unsigned)blocks, 256, 0, ctx->stream)(k.query, k.ld_query, static_cast<uint4*>(scratch), k.tokens, dim, k.grad_scores,
-                                                                   (size_t)k.tokens * k.top_k, wide_blocks);
+  pdl(split_queries_kernel, (unsigned)std::min<size_t>((groups + 255) / 256, (size_t)ctx->sm_count * 8), 256, 0, ctx->stream)(
+      k.query, k.ld_query, reinterpret_cast<uint4*>(pieces), k.tokens, dim, k.grad_scores, (size_t)k.tokens * k.top_k, wide_seen);
   HL_LAUNCH_CHECK("split_queries_kernel");
   count_launch(ctx);
   CUtensorMap map_q;
-  const int rc = make_tensor_map_bf16_3d(&map_q, scratch, (uint64_t)dim, (uint64_t)k.tokens, 3, (uint64_t)dim, (uint64_t)dim * k.tokens, 64, KG_TOKENS, 1);
+  const int rc = make_tensor_map_bf16_3d(&map_q, pieces, (uint64_t)dim, (uint64_t)k.tokens, 3, (uint64_t)dim, (uint64_t)dim * k.tokens, 64, KG_TOKENS, 1);
   if (rc != HL_OK) return rc;
   switch (ceil_div(k.half, 64)) {
-    case 1: return launch_key_gradient<1>(ctx, k, map_q, wide_blocks, blocks, shares, *partial);
-    case 2: return launch_key_gradient<2>(ctx, k, map_q, wide_blocks, blocks, shares, *partial);
-    case 3: return launch_key_gradient<3>(ctx, k, map_q, wide_blocks, blocks, shares, *partial);
-    default: return launch_key_gradient<4>(ctx, k, map_q, wide_blocks, blocks, shares, *partial);
+    case 1: return launch_key_gradient<1>(ctx, k, map_q, wide_seen, shares, *partial);
+    case 2: return launch_key_gradient<2>(ctx, k, map_q, wide_seen, shares, *partial);
+    case 3: return launch_key_gradient<3>(ctx, k, map_q, wide_seen, shares, *partial);
+    default: return launch_key_gradient<4>(ctx, k, map_q, wide_seen, shares, *partial);
   }
 }
 
