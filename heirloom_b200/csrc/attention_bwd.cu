@@ -541,10 +541,10 @@ int flash_attention_backward_impl(hl_ctx* ctx, const void* q, const void* k, con
   }
   CUtensorMap mq, mk, mv, mdo;
   int rc;
-  // boxes of 64 channels (one 128-byte swizzle row); a head of 128 channels takes two boxes per tile and tiles of 64 keys
-  // With keys as rows a tile is 128 keys: half the tiles of the 64-key kernel, each some 15 % longer than one of those.  So it wins where
+  // boxes of 64 channels (one 128-byte swizzle row); a head of 128 channels takes two boxes per tile, and tiles of 128 keys as rows or of
+  // 64 keys with queries as rows.  Keys as rows are half the tiles of the 64-key kernel, each some 15 % longer than one of those: so it wins where
   // the tiles' number bounds the pass (all of them over the SMs), and loses where the longest walk does: heads (n + 1) / 2 walks of n
-  // tiles against 0.6 SMs.  Whole call with 64 and with 128 keys, us: B16 H6 T1024 (5.8 walks an SM) 188 / 126; B2 H4 T2048 (0.46) 53 / 57,
+  // tiles against 0.6 SMs.  Whole call with 64 and with 128 keys, us: B16 H6 T1024 (2.9 walks an SM) 188 / 126; B2 H4 T2048 (0.46) 53 / 57,
   // B3 H5 T777 (0.41) 31.1 / 32.7, B1 H8 T512 (0.14) 22.1 / 22.8.
   const bool transposed = head_dim == 128 && 5ll * batch * n_heads * (ceil_div(time, FB_BM) + 1) >= 6ll * ctx->sm_count;
   const uint32_t key_rows = head_dim == 64 || transposed ? FB_BN : 64;

@@ -7,7 +7,8 @@
 // keys, every product runs on all 128 rows of the tensor core and tensor memory holds S and dP (64 columns each), dVᵀ and
 // dKᵀ (64 each) and two dQ tiles (128 each), so each of the five products is formed once.  A 128-key tile had room for one
 // stage and one half of the head at a time: S and dP were formed twice, and every tile waited for its own loads (B4 H12 T4096:
-// 1334 us then, 931 us now).  Bound by shared memory: a product 64 columns wide reads its 128 rows of A for half the work of a
+// 1334 us then, 931 us with 64; such sizes take keys as rows now, 632 us for the whole call, and this kernel the few or short heads
+// whose longest walk bounds the pass: B2 H4 T2048 53 us against 57).  Bound by shared memory: a product 64 columns wide reads its 128 rows of A for half the work of a
 // full tile, which makes the five products worth nine halves, and by the softmax warps' chain that runs beside them.
 #include "attention_bwd.cuh"
 #include "tc05.cuh"

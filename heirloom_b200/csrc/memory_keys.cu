@@ -12,11 +12,12 @@
 // 64 tokens deep it was 2.2e-7, 2.4e-7 and 2.1e-7.
 //
 // A CTA takes 128 rows of one table, all columns and a share of the tokens.  A stage of 32 tokens: the queries' pieces by TMA; of
-// W, eight warps put the entries of four tokens each into a tile that is zero otherwise, and take them out again before the tile
+// W, sixteen warps put the entries of two tokens each into a tile that is zero otherwise, and take them out again before the tile
 // is used next (slots that share a row are added first, in a fixed order).  The same warps
 // empty the accumulators, beside the small products of the next stage.  A stage's twelve instructions of 128 x 256 x 16 take 1536
-// cycles; bound by those warps (some 5000 cycles a stage; eight of them took 6000): 86 us for the size above, 16 more for the
-// queries' pieces.
+// cycles; bound by those warps' chain of loads, exchanges and stores, some 5400 cycles a stage (tensor pipe 33 % active, instructions
+// issued in 31 % of the cycles): 83 us for the size above, 16 more for the queries' pieces.  Eighteen warps leave a thread 96
+// registers, of which the kernel for 256 columns spills 484 bytes.
 #include "kernels.h"
 #include "tc05.cuh"
 
