@@ -180,6 +180,45 @@ int decode_greedy(hl_ctx* ctx, const float* logits, int vocab, GreedyPart* parts
 bool all_finite_f32(const float* x, size_t n);
 int decode_embed(hl_ctx* ctx, const float* table, const float* positions, const long long* state, void* out, int dtype, int dim);
 
+// The same in two kernels a block (decode_block.cu).  A row of the residual stream that no kernel has written yet: base + bias + the
+// sum of `parts` rows, or what base holds (n = 0), or the embedding of the state's token (n = 0, base null).  The kernel that takes
+// it also writes it to `keep`, where given.  Rows and `keep` are of the model's type, parts f32 on the bf16 route and f64 on the f32 one.
+struct DecodeRow {
+  const void* base;
+  const void* parts;  // [n][d]
+  int n;
+  const float* bias;
+  const float *table, *positions;
+  const long long* state;
+  void* keep;
+};
+struct DecodeBlock {
+  int dtype, d, heads, hidden, context;
+  const long long* state;  // device: position, token
+  DecodeRow x;
+  bool window;             // the q/k/v rows, this position's as well, come from the predecessor: x.base is only the residual
+  const float *ln1_gamma, *ln1_beta;
+  const void* wqkv;        // [3 d][d]
+  const float* bqkv;
+  void* qkv;               // rows of 3 d, those below the position settled before this sequence of launches began unless `window`
+  const void* wo;
+  const float* bo;
+  const float *ln2_gamma, *ln2_beta;
+  const void *w1, *w2;
+  const float *b1, *b2;
+  void *attention_parts, *feed_forward_parts;  // decode_block_parts_bytes each
+};
+bool decode_block_applies(int dtype, int d, int heads, int hidden, int context);
+size_t decode_block_parts_bytes(int d);
+// *after: the row behind the block's attention, behind its feed-forward (`x` needs a `keep`).
+int decode_attention_block(hl_ctx* ctx, const DecodeBlock& b, DecodeRow* after);
+int decode_feed_forward(hl_ctx* ctx, const DecodeBlock& b, const DecodeRow& x, DecodeRow* after);
+// Writes the row to its `keep`.
+int decode_row(hl_ctx* ctx, const DecodeRow& r, int dtype, int d);
+// Final layer norm and head.
+int decode_head_row(hl_ctx* ctx, const DecodeRow& x, int dtype, const float* gamma, const float* beta, const void* w, const float* bias,
+                    float* out, int n, int d);
+
 // bf16 pieces of f32 values (elementwise.cu): piece number id[j] of row r goes to out + r * ld + j * piece, for j < n; all multiples
 // of 8 elements.  Pieces as split8_bf16 forms them.
 struct PieceDest {

@@ -207,6 +207,7 @@ struct hl_decoder {
   // state of the next one-token step
   int cached = 0;
   long long* decode_state = nullptr;       // device: position, token
+  void* row_parts[2] = {};                 // device: what clusters add to the row, of attention and of the feed-forward
   bool head_twice = false;                 // this pass left the head's row sums instead of its logits
   float* row_logits = nullptr;             // where the logits of a single row go; null: m->logits
   GreedyPart* greedy = nullptr;            // device: the blocks' parts
@@ -488,6 +489,8 @@ int plan_activations(hl_decoder* m, bool measure_only, size_t* bytes_out) {
   m->tokens = carve<int64_t>(cur, N);
   m->targets = carve<int64_t>(cur, N);
   m->decode_state = carve<long long>(cur, 2);
+  m->row_parts[0] = carve<uint8_t>(cur, decode_block_parts_bytes(c.d_model));
+  m->row_parts[1] = carve<uint8_t>(cur, decode_block_parts_bytes(c.d_model));
   m->greedy = carve<GreedyPart>(cur, greedy_parts(c.vocab));
   m->loss_dev = carve<float>(cur, 4);
   m->norm_dev = carve<float>(cur, 4);
@@ -542,6 +545,8 @@ int plan_activations_f32(hl_decoder* m, bool measure_only, size_t* bytes_out) {
   m->tokens = carve<int64_t>(cur, N);
   m->targets = carve<int64_t>(cur, N);
   m->decode_state = carve<long long>(cur, 2);
+  m->row_parts[0] = carve<uint8_t>(cur, decode_block_parts_bytes(c.d_model));
+  m->row_parts[1] = carve<uint8_t>(cur, decode_block_parts_bytes(c.d_model));
   m->greedy = carve<GreedyPart>(cur, greedy_parts(c.vocab));
   m->loss_dev = carve<float>(cur, 4);
   m->norm_dev = carve<float>(cur, 4);
@@ -728,6 +733,46 @@ DecodeGemv row_gemv(const hl_decoder* m, const void* x, size_t w, size_t b, void
   return g;
 }
 
+// Block l for the row whose position stands in m->decode_state, in the two kernels of decode_block.cu.  `x`: its input row; with
+// `window` the block's q/k/v rows are there.  Returns the row behind the block, or behind its attention in front of a memory block.
+bool row_block_fused(const hl_decoder* m) {
+  const hl_decoder_config& c = m->cfg;
+  return decode_block_applies(c.precision == HL_PRECISION_AMP_BF16 ? HL_BF16 : HL_F32, c.d_model, c.n_heads, c.d_ff, c.context);
+}
+int row_block_fused(hl_decoder* m, int l, const DecodeRow& x, bool window, DecodeRow* after) {
+  const hl_decoder_config& c = m->cfg;
+  const LayerOffsets& o = m->lo[l];
+  const bool amp = c.precision == HL_PRECISION_AMP_BF16;
+  const float* P = m->params;
+  auto weight = [&](size_t w) { return amp ? (const void*)(m->shadow + w) : (const void*)(P + w); };
+  DecodeBlock b{};
+  b.dtype = amp ? HL_BF16 : HL_F32;
+  b.d = c.d_model; b.heads = c.n_heads; b.hidden = c.d_ff; b.context = c.context;
+  b.state = m->decode_state;
+  b.x = x;
+  b.x.keep = window ? nullptr : amp ? (void*)m->x[l] : (void*)m->xf[l];
+  b.window = window;
+  b.ln1_gamma = P + o.ln1g; b.ln1_beta = P + o.ln1b;
+  b.wqkv = weight(o.wqkv); b.bqkv = P + o.bqkv;
+  b.qkv = amp ? (void*)m->la[l].qkv : (void*)m->lf[l].qkv;
+  b.wo = weight(o.wo); b.bo = P + o.bo;
+  b.attention_parts = m->row_parts[0]; b.feed_forward_parts = m->row_parts[1];
+  DecodeRow r{};
+  HL_TRY(decode_attention_block(m->ctx, b, &r));
+  r.keep = amp ? (void*)m->la[l].r : (void*)m->lf[l].r;
+  if (o.is_memory) { *after = r; return HL_OK; }
+  b.ln2_gamma = P + o.ln2g; b.ln2_beta = P + o.ln2b;
+  b.w1 = weight(o.w1); b.b1 = P + o.b1;
+  b.w2 = weight(o.w2); b.b2 = P + o.b2;
+  return decode_feed_forward(m->ctx, b, r, after);
+}
+int row_head(hl_decoder* m, const DecodeRow& x) {
+  const bool amp = m->cfg.precision == HL_PRECISION_AMP_BF16;
+  return decode_head_row(m->ctx, x, amp ? HL_BF16 : HL_F32, m->params + m->off_lnf_g, m->params + m->off_lnf_b,
+                         amp ? (const void*)(m->shadow + m->off_head_w) : (const void*)(m->params + m->off_head_w), m->params + m->off_head_b,
+                         m->row_logits ? m->row_logits : m->logits, m->cfg.vocab, m->cfg.d_model);
+}
+
 // Attention and feed-forward of block l for the row whose position stands in m->decode_state, `x` being its input row; the
 // result goes to row 0 of the block's output.  The block's q/k/v rows are there, `settled`: but for this row, since before
 // the sequence of launches began.
@@ -820,6 +865,12 @@ int forward(hl_decoder* m, Forward what = Forward::all) {
     HL_TRY(layer_norm_forward_impl(ctx, m->x[l], HL_BF16, P + o.ln1g, P + o.ln1b, a.a, HL_BF16, a.mean1, a.rstd1, N, d, 1e-5f));
     HL_TRY(g.run(N, 3 * d, d, a.a, d, HL_K_MAJOR, W + o.wqkv, d, HL_K_MAJOR, a.qkv, 3 * d, HL_BF16, HL_EPI_BIAS, P + o.bqkv));
     if (what == Forward::last_position && last_block_by_row(m, l)) {
+      if (row_block_fused(m)) {
+        DecodeRow x{}, after{};
+        x.base = m->x[l] + (size_t)(N - 1) * d;
+        HL_TRY(row_block_fused(m, l, x, true, &after));
+        return row_head(m, after);
+      }
       HL_TRY(row_block(m, l, m->x[l] + (size_t)(N - 1) * d, false));
       return decode_head(m, m->x[l + 1], HL_BF16);
     }
@@ -1236,6 +1287,12 @@ int forward_f32(hl_decoder* m, bool last_only = false) {
     HL_TRY(layer_norm_forward_impl(ctx, m->xf[l], HL_F32, P + o.ln1g, P + o.ln1b, a.a, HL_F32, nullptr, nullptr, N, d, 1e-5f));
     HL_TRY(forward_f32_gemm(m, linear_f32(a.a, P + o.wqkv, P + o.bqkv, a.qkv, N, d, 3 * d)));
     if (last_only && last_block_by_row(m, l)) {
+      if (row_block_fused(m)) {
+        DecodeRow x{}, after{};
+        x.base = m->xf[l] + (size_t)(N - 1) * d;
+        HL_TRY(row_block_fused(m, l, x, true, &after));
+        return row_head(m, after);
+      }
       HL_TRY(row_block(m, l, m->xf[l] + (size_t)(N - 1) * d, false));
       return decode_head(m, m->xf[l + 1], HL_F32);
     }
@@ -1442,18 +1499,26 @@ int decode_step(hl_decoder* m) {
   const float* P = m->params;
   auto gemv = [&](const void* x, size_t w, size_t b, void* out, int n, int k, int epilogue = GV_STORE, const void* residual = nullptr,
                   size_t ln_g = 0, size_t ln_b = 0) { return row_gemv(m, x, w, b, out, n, k, epilogue, residual, ln_g, ln_b); };
-  HL_TRY(decode_embed(ctx, P + m->off_tok, P + m->off_pos, m->decode_state, amp ? (void*)m->x[0] : (void*)m->xf[0], dt, d));
+  const bool fused = row_block_fused(m);
+  DecodeRow row{};  // fused: the row so far
+  row.table = P + m->off_tok; row.positions = P + m->off_pos; row.state = m->decode_state;
+  if (!fused) HL_TRY(decode_embed(ctx, P + m->off_tok, P + m->off_pos, m->decode_state, amp ? (void*)m->x[0] : (void*)m->xf[0], dt, d));
   for (int l = 0; l < c.n_layers; ++l) {
     const LayerOffsets& o = m->lo[l];
     void *x, *next, *qkv, *r;
     if (amp) { x = m->x[l]; next = m->x[l + 1]; qkv = m->la[l].qkv; r = m->la[l].r; }
     else { x = m->xf[l]; next = m->xf[l + 1]; qkv = m->lf[l].qkv; r = m->lf[l].r; }
-    // the attention output, r and g rows may lie over cached positions' rows: only the q/k/v rows are kept
-    DecodeGemv q = gemv(x, o.wqkv, o.bqkv, qkv, 3 * d, d, GV_STORE, nullptr, o.ln1g, o.ln1b);
-    q.out_row = m->decode_state;
-    q.ld_out = 3 * d;
-    HL_TRY(decode_gemv(ctx, q));
-    HL_TRY(row_block(m, l, x, true));
+    if (fused) {
+      HL_TRY(row_block_fused(m, l, row, false, &row));
+      if (o.is_memory) HL_TRY(decode_row(ctx, row, dt, d));
+    } else {
+      // the attention output, r and g rows may lie over cached positions' rows: only the q/k/v rows are kept
+      DecodeGemv q = gemv(x, o.wqkv, o.bqkv, qkv, 3 * d, d, GV_STORE, nullptr, o.ln1g, o.ln1b);
+      q.out_row = m->decode_state;
+      q.ld_out = 3 * d;
+      HL_TRY(decode_gemv(ctx, q));
+      HL_TRY(row_block(m, l, x, true));
+    }
     if (o.is_memory) {
       MemoryActs& ma = m->ma[l];
       const int kd = m->mem.key_dim, vd = m->mem.value_dim;
@@ -1469,8 +1534,11 @@ int decode_step(hl_decoder* m) {
       HL_TRY(project(r, dt, o.wg_m, o.bg_m, ma.gate, HL_F32, vd, d, GV_GELU, nullptr, true));
       HL_TRY(hl_binary_f32(ctx, HL_MUL, ma.weighted, ma.gate, ma.mv, (size_t)vd));
       HL_TRY(project(ma.mv, HL_F32, o.wout_m, o.bout_m, next, dt, d, vd, GV_RESIDUAL, r, false));
+      row = DecodeRow{};
+      row.base = next;
     }
   }
+  if (fused) return row_head(m, row);
   return decode_head(m, amp ? (const void*)m->x[c.n_layers] : (const void*)m->xf[c.n_layers], dt);
 }
 

@@ -283,6 +283,36 @@ def test_one_token_steps_equal_the_full_window(heads, memory):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("d_model,heads,d_ff,context,prefix", [
+    (16, 1, 8, 9, 1),          # the smallest: half a step of the contraction, one CTA with hidden units
+    (48, 3, 200, 40, 30),      # heads of 16 channels, a slice of hidden units that is cut short
+    (1024, 16, 4096, 24, 17),  # the widest row (f32: too much shared memory, kernels of their own)
+    (256, 2, 776, 1024, 1000), # a thread's second key
+    (128, 1, 64, 1030, 1021),  # contexts beyond that: kernels of their own
+    (64, 8, 64, 19, 10),       # heads of 8 channels: kernels of their own
+])
+def test_one_token_steps_of_all_sizes_equal_the_full_window(d_model, heads, d_ff, context, prefix):
+    """prefill + decode_next against a full-window pass, on both sides of every limit of the kernels that take a block in two
+    launches; the tolerances of the test above (the sums are as long or shorter, or grow with the row as the logits do)."""
+    from heirloom_b200 import nn
+    from tests.gpu_util import ctx
+    c = ctx()
+    stream = np.random.default_rng(d_model).integers(0, 72, context)
+    for precision, tol in ((nn.PRECISION_F32, 2e-6), (nn.PRECISION_AMP_BF16, 3e-2)):
+        model = nn.DecoderLm(c, nn.DecoderConfig(vocab=72, d_model=d_model, n_layers=2, n_heads=heads, d_ff=d_ff, context=context, batch=1,
+                                                 precision=precision))
+        rng = np.random.default_rng(heads)
+        model.load_state_dict({n: (np.ones(s) if ".ln" in n or n.startswith("ln_f") else rng.standard_normal(s) * (0.1 if len(s) == 1 else s[-1] ** -0.5))
+                               for n, s in ((n, s) for n, s in model.parameter_shapes().items())})
+        lengths = range(prefix, min(context, prefix + 8) + 1)
+        got = [model.prefill(stream[:prefix])] + [model.decode_next(int(stream[n - 1])) for n in lengths[1:]]
+        for n, logits in zip(lengths, got):
+            want = gen.next_token_logits(model, stream[:n])
+            assert np.abs(logits - want).max() <= tol * max(1.0, np.abs(want).max()), (precision, n)
+        model.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("vocab", [8, 2048, 2056, 50304])
 def test_the_device_picks_the_greedy_token_that_sampling_picks(vocab):
     """The last maximum and its probability, the row cut into blocks of 2048 logits: the same token as the host's sampling of
