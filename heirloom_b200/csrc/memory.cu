@@ -320,8 +320,91 @@ __global__ void split_rows_kernel(const int64_t* __restrict__ rows, int64_t* __r
   right[i] = r % side;
 }
 
+// Sums over the warp's lanes of eight values a lane: value 4 b4 + 2 b3 + b2 in the lanes whose bits 4, 3 and 2 are these (a lane keeps
+// the half of its values that its bit names and gives the other half away: 9 exchanges instead of 40).
+__device__ __forceinline__ double sum8_over_lanes(double (&v)[8]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int d = 16, n = 4; n >= 1; d >>= 1, n >>= 1) {
+    const bool upper = (lane & d) != 0;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const double send = upper ? v[i] : v[i + n], keep = upper ? v[i + n] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
+    }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+__device__ __forceinline__ int sum8_index() { return (threadIdx.x & 31) >> 2; }  // which of the eight a lane holds then
+
+// The kernels that gather table rows (selected scores and weighted value, forward and backward) are bound by how many rows are on
+// their way: by L2 for many tokens (16384 tokens of 32 rows of 2 KB: 50 to 100 us a kernel), and for few by latency, since with a warp
+// a token, a row after the other, 2048 tokens keep a tenth of the memory busy.  So a warp takes eight rows at a time, and where
+// columns do not meet, 128 of the columns only.  Scores, their gradient and value at 2048 tokens 21, 31 and 37 -> 13, 12 and 21 us, at 16384 tokens
+// 100, 67 and 51 -> 64, 61 and 53.
+constexpr int GATHER = 8;
+__device__ __forceinline__ float4 row_piece(const float* table, long long row, int dim, int piece, bool on) {
+  return on && row >= 0 ? __ldg(reinterpret_cast<const float4*>(table + (size_t)row * dim) + piece) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
 // ---- selected scores: score[t,k] = q_L . K_L[idx/side] + q_R . K_R[idx%side]  (src/tensor.rs:3593-3769).
-// `exact` mode (side == 0): score = q . K[idx] over key_dim (src/tensor.rs:3465-3548). One warp per token. ---
+// Product-key form, key_dim up to 128 U, sixteen-byte rows: a CTA of four warps a token, eight of every 32 slots each; the query sits
+// in registers.  A lane's share (at most 4 U products) is summed in f32, the 32 shares in f64: f64 multiply-adds run at a
+// fraction of the f32 rate.
+template <int U>
+__global__ void __launch_bounds__(128)
+selected_scores_rows_kernel(const int64_t* __restrict__ idx, const float* __restrict__ query, long long ld_q,
+                            const float* __restrict__ left, const float* __restrict__ right, float* __restrict__ scores, int top_k,
+                            int side, int key_dim, int slots, int* __restrict__ status) {
+  pdl_begin();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const size_t token = blockIdx.x;
+  const int half = key_dim / 2, groups = key_dim / 4, half_groups = half / 4;
+  float4 qv[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int gi = u * 32 + lane;
+    qv[u] = gi < groups ? *reinterpret_cast<const float4*>(query + token * ld_q + gi * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  for (int k0 = warp * GATHER; k0 < top_k; k0 += 32) {
+    int my_li = -1, my_ri = 0;
+    if (lane < GATHER && k0 + lane < top_k) {
+      const long long slot = idx[token * top_k + k0 + lane];
+      if (slot >= 0 && slot < slots) {
+        my_li = (int)((unsigned)slot / (unsigned)side);
+        my_ri = (int)((unsigned)slot % (unsigned)side);
+      } else {
+        atomicExch(status + ST_BAD_INDEX, 1);
+      }
+    }
+    double part[GATHER];
+#pragma unroll
+    for (int k = 0; k < GATHER; ++k) {
+      const int li = __shfl_sync(0xffffffffu, my_li, k), ri = __shfl_sync(0xffffffffu, my_ri, k);
+      float acc = 0.f;
+      if (li >= 0) {
+        const float4* lrow = reinterpret_cast<const float4*>(left + (size_t)li * half);
+        const float4* rrow = reinterpret_cast<const float4*>(right + (size_t)ri * half);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int gi = u * 32 + lane;
+          if (gi < groups) {
+            const float4 kv = gi < half_groups ? __ldg(lrow + gi) : __ldg(rrow + (gi - half_groups));
+            acc = fmaf(qv[u].x, kv.x, acc); acc = fmaf(qv[u].y, kv.y, acc);
+            acc = fmaf(qv[u].z, kv.z, acc); acc = fmaf(qv[u].w, kv.w, acc);
+          }
+        }
+      }
+      part[k] = (double)acc;
+    }
+    const double sum = sum8_over_lanes(part);
+    const int k = k0 + sum8_index();
+    if ((lane & 3) == 0 && k < top_k) scores[token * top_k + k] = (float)sum;
+  }
+}
+
+// The same for any sizes, and in `exact` mode (side == 0): score = q . K[idx] over key_dim (src/tensor.rs:3465-3548).  A warp a token.
 __global__ void selected_scores_fwd_kernel(const int64_t* __restrict__ idx, const float* __restrict__ query, long long ld_q,
                                            const float* __restrict__ left, const float* __restrict__ right,
                                            float* __restrict__ scores, int tokens, int top_k, int side, int key_dim,
@@ -332,67 +415,6 @@ __global__ void selected_scores_fwd_kernel(const int64_t* __restrict__ idx, cons
   if (token >= tokens) return;
   const int half = side > 0 ? key_dim / 2 : key_dim;
   const float* q = query + (size_t)token * ld_q;
-  if (side > 0 && half % 4 == 0 && key_dim <= 1024 && (ld_q % 4) == 0 &&
-      ((reinterpret_cast<uintptr_t>(query) | reinterpret_cast<uintptr_t>(left) | reinterpret_cast<uintptr_t>(right)) & 15) == 0) {
-    // product-key form: the query sits in registers (a lane owns up to 8 four-column groups); slots are split into
-    // their half-table rows once per 32 and handed around by shuffles; 32 per-lane partial dots are then summed
-    // across the warp by a transposing butterfly (31 exchanges instead of 32 five-step reductions).
-    const int groups = key_dim / 4, half_groups = half / 4;
-    float4 qv[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int gi = u * 32 + lane;
-      qv[u] = gi < groups ? *reinterpret_cast<const float4*>(q + gi * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    for (int k0 = 0; k0 < top_k; k0 += 32) {
-      int my_li = -1, my_ri = 0;
-      if (k0 + lane < top_k) {
-        const long long slot = idx[(size_t)token * top_k + k0 + lane];
-        if (slot >= 0 && slot < slots) {
-          my_li = (int)((unsigned)slot / (unsigned)side);
-          my_ri = (int)((unsigned)slot % (unsigned)side);
-        } else {
-          atomicExch(status + ST_BAD_INDEX, 1);
-        }
-      }
-      double part[32];
-#pragma unroll
-      for (int k = 0; k < 32; ++k) {
-        const int li = __shfl_sync(0xffffffffu, my_li, k);
-        const int ri = __shfl_sync(0xffffffffu, my_ri, k);
-        // a lane's share (at most 32 products) is summed in f32, the 32 shares in f64: f64 multiply-adds run at a
-        // fraction of the f32 rate and were the busiest pipe of this kernel
-        float acc = 0.f;
-        if (li >= 0) {
-          const float4* lrow = reinterpret_cast<const float4*>(left + (size_t)li * half);
-          const float4* rrow = reinterpret_cast<const float4*>(right + (size_t)ri * half);
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int gi = u * 32 + lane;
-            if (gi < groups) {
-              const float4 kv = gi < half_groups ? __ldg(lrow + gi) : __ldg(rrow + (gi - half_groups));
-              acc = fmaf(qv[u].x, kv.x, acc); acc = fmaf(qv[u].y, kv.y, acc);
-              acc = fmaf(qv[u].z, kv.z, acc); acc = fmaf(qv[u].w, kv.w, acc);
-            }
-          }
-        }
-        part[k] = (double)acc;
-      }
-      // after the step with distance d, a lane keeps the half of its values whose index has the same d-bit as the lane
-#pragma unroll
-      for (int d = 16; d >= 1; d >>= 1) {
-        const bool upper = (lane & d) != 0;
-#pragma unroll
-        for (int i = 0; i < d; ++i) {
-          const double send = upper ? part[i] : part[i + d];
-          const double keep = upper ? part[i + d] : part[i];
-          part[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
-        }
-      }
-      if (k0 + lane < top_k) scores[(size_t)token * top_k + k0 + lane] = (float)part[0];
-    }
-    return;
-  }
   for (int k = 0; k < top_k; ++k) {
     const long long slot = idx[(size_t)token * top_k + k];
     if (slot < 0 || slot >= slots) {
@@ -414,8 +436,55 @@ __global__ void selected_scores_fwd_kernel(const int64_t* __restrict__ idx, cons
   }
 }
 
-// dq[t,:] = sum_k g[t,k] * [K_L[li]; K_R[ri]]; dK_L[li,:] += g[t,k] q_L[t]; dK_R[ri,:] += g[t,k] q_R[t]
-// (src/tensor/autograd.rs:2386-2494).  Key gradients use f32 atomics like the reference.
+// dq[t,:] = sum_k g[t,k] * [K_L[li]; K_R[ri]] of the product-key form, sixteen-byte rows: a warp a token and 128 columns.
+__global__ void __launch_bounds__(128)
+selected_query_gradient_kernel(const int64_t* __restrict__ idx, const float* __restrict__ left, const float* __restrict__ right,
+                               const float* __restrict__ grad_scores, float* __restrict__ dq, long long ld_dq, int tokens, int top_k,
+                               int side, int key_dim, int slots, int* __restrict__ clear) {
+  pdl_begin();
+  if (clear && blockIdx.x == 0 && threadIdx.x == 0) *clear = 0;  // a word that the kernels behind this one set and read
+  const int lane = threadIdx.x & 31, slices = (key_dim + 127) / 128, w = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int token = w / slices, gi = (w - token * slices) * 32 + lane, half = key_dim / 2;
+  if (token >= tokens) return;
+  const bool on = gi < key_dim / 4, in_left = gi < half / 4;
+  const float* table = in_left ? left : right;
+  const int piece = in_left ? gi : gi - half / 4;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k0 = 0; k0 < top_k; k0 += 32) {
+    int my_li = -1, my_ri = -1;
+    float my_g = 0.f;
+    if (k0 + lane < top_k) {
+      const long long slot = idx[(size_t)token * top_k + k0 + lane];
+      if (slot >= 0 && slot < slots) {
+        my_li = (int)((unsigned)slot / (unsigned)side);
+        my_ri = (int)((unsigned)slot % (unsigned)side);
+        my_g = grad_scores[(size_t)token * top_k + k0 + lane];
+      }
+    }
+    for (int k = 0; k < min(32, top_k - k0); k += GATHER) {
+      float4 v[GATHER];
+      float g[GATHER];
+      bool there[GATHER];
+#pragma unroll
+      for (int j = 0; j < GATHER; ++j) {
+        const int li = __shfl_sync(0xffffffffu, my_li, k + j), ri = __shfl_sync(0xffffffffu, my_ri, k + j);
+        g[j] = __shfl_sync(0xffffffffu, my_g, k + j);
+        there[j] = li >= 0;
+        v[j] = row_piece(table, in_left ? li : ri, half, piece, on);
+      }
+#pragma unroll
+      for (int j = 0; j < GATHER; ++j)
+        if (there[j]) {
+          acc.x = fmaf(g[j], v[j].x, acc.x); acc.y = fmaf(g[j], v[j].y, acc.y);
+          acc.z = fmaf(g[j], v[j].z, acc.z); acc.w = fmaf(g[j], v[j].w, acc.w);
+        }
+    }
+  }
+  if (on) *reinterpret_cast<float4*>(dq + (size_t)token * ld_dq + gi * 4) = acc;
+}
+
+// The same for any sizes, and in `exact` mode with dK[idx,:] += g[t,k] q[t]
+// (src/tensor/autograd.rs:2386-2494).  Those key gradients use f32 atomics like the reference.
 __global__ void selected_scores_bwd_kernel(const int64_t* __restrict__ idx, const float* __restrict__ query, long long ld_q,
                                            const float* __restrict__ left, const float* __restrict__ right,
                                            const float* __restrict__ grad_scores, float* __restrict__ dq, long long ld_dq,
@@ -429,63 +498,18 @@ __global__ void selected_scores_bwd_kernel(const int64_t* __restrict__ idx, cons
   const int half = side > 0 ? key_dim / 2 : key_dim;
   const float* q = query + (size_t)token * ld_q;
   if (dq) {
-    if (side > 0 && half % 4 == 0 && key_dim <= 1024 && (ld_dq % 4) == 0 &&
-        ((reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(left) | reinterpret_cast<uintptr_t>(right)) & 15) == 0) {
-      // product-key form: a lane owns up to 8 four-column groups of the query gradient; slots and score gradients are
-      // read once per 32 and handed around by shuffles, table rows come in with 16-byte loads
-      float4 acc[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-      const int groups = key_dim / 4, half_groups = half / 4;
-      for (int k0 = 0; k0 < top_k; k0 += 32) {
-        int my_li = -1, my_ri = 0;
-        float my_g = 0.f;
-        if (k0 + lane < top_k) {
-          const long long slot = idx[(size_t)token * top_k + k0 + lane];
-          if (slot >= 0 && slot < slots) {
-            my_li = (int)((unsigned)slot / (unsigned)side);
-            my_ri = (int)((unsigned)slot % (unsigned)side);
-            my_g = grad_scores[(size_t)token * top_k + k0 + lane];
-          }
-        }
-        const int n = min(32, top_k - k0);
-        for (int k = 0; k < n; ++k) {
-          const int li = __shfl_sync(0xffffffffu, my_li, k);
-          const int ri = __shfl_sync(0xffffffffu, my_ri, k);
-          const float g = __shfl_sync(0xffffffffu, my_g, k);
-          if (li < 0) continue;
-          const float4* lrow = reinterpret_cast<const float4*>(left + (size_t)li * half);
-          const float4* rrow = reinterpret_cast<const float4*>(right + (size_t)ri * half);
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int gi = u * 32 + lane;
-            if (gi < groups) {
-              const float4 kv = gi < half_groups ? __ldg(lrow + gi) : __ldg(rrow + (gi - half_groups));
-              acc[u].x = fmaf(g, kv.x, acc[u].x); acc[u].y = fmaf(g, kv.y, acc[u].y);
-              acc[u].z = fmaf(g, kv.z, acc[u].z); acc[u].w = fmaf(g, kv.w, acc[u].w);
-            }
-          }
-        }
+    for (int j = lane; j < key_dim; j += 32) {
+      double acc = 0.0;
+      for (int k = 0; k < top_k; ++k) {
+        const long long slot = idx[(size_t)token * top_k + k];
+        if (slot < 0 || slot >= slots) continue;
+        const double g = (double)grad_scores[(size_t)token * top_k + k];
+        float kv;
+        if (side > 0) kv = j < half ? left[(size_t)(slot / side) * half + j] : right[(size_t)(slot % side) * half + (j - half)];
+        else kv = left[(size_t)slot * key_dim + j];
+        acc += g * (double)kv;
       }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int gi = u * 32 + lane;
-        if (gi < groups) *reinterpret_cast<float4*>(dq + (size_t)token * ld_dq + gi * 4) = acc[u];
-      }
-    } else {
-      for (int j = lane; j < key_dim; j += 32) {
-        double acc = 0.0;
-        for (int k = 0; k < top_k; ++k) {
-          const long long slot = idx[(size_t)token * top_k + k];
-          if (slot < 0 || slot >= slots) continue;
-          const double g = (double)grad_scores[(size_t)token * top_k + k];
-          float kv;
-          if (side > 0) kv = j < half ? left[(size_t)(slot / side) * half + j] : right[(size_t)(slot % side) * half + (j - half)];
-          else kv = left[(size_t)slot * key_dim + j];
-          acc += g * (double)kv;
-        }
-        dq[(size_t)token * ld_dq + j] = (float)acc;
-      }
+      dq[(size_t)token * ld_dq + j] = (float)acc;
     }
   }
   if (side > 0) return;  // the half-key gradients of the product-key form come from product_key_dkeys_kernel
@@ -683,7 +707,48 @@ __global__ void softmax_rows_bwd_kernel(const float* __restrict__ y, const float
 }
 
 // ---- weighted value: out[t,:] = sum_k w[t,k] V[idx[t,k],:] (* gate[t,:] when given)  (src/tensor.rs:3771-3900).
-// One warp per token, 128-bit row gathers. ------------------------------------------------------------
+// A warp a token and 128 columns; at most top_k products a column in f32 (f64 multiply-adds run at a fraction of the f32 rate).
+__global__ void __launch_bounds__(128)
+weighted_value_rows_kernel(const int64_t* __restrict__ idx, const float* __restrict__ weights, const float* __restrict__ values,
+                           float* __restrict__ out, int tokens, int top_k, int rows, int dim, int* __restrict__ status) {
+  pdl_begin();
+  const int lane = threadIdx.x & 31, slices = (dim + 127) / 128, w = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int token = w / slices, gi = (w - token * slices) * 32 + lane;
+  if (token >= tokens) return;
+  const bool on = gi < dim / 4;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k0 = 0; k0 < top_k; k0 += 32) {
+    int my_row = -1;
+    float my_w = 0.f;
+    if (k0 + lane < top_k) {
+      const long long r = idx[(size_t)token * top_k + k0 + lane];
+      my_w = weights[(size_t)token * top_k + k0 + lane];
+      if (r < 0 || r >= rows) atomicExch(status + ST_BAD_INDEX, 1);
+      else my_row = (int)r;
+    }
+    for (int k = 0; k < min(32, top_k - k0); k += GATHER) {
+      float4 v[GATHER];
+      float wt[GATHER];
+      bool there[GATHER];
+#pragma unroll
+      for (int j = 0; j < GATHER; ++j) {
+        const int r = __shfl_sync(0xffffffffu, my_row, k + j);
+        wt[j] = __shfl_sync(0xffffffffu, my_w, k + j);
+        there[j] = r >= 0;
+        v[j] = row_piece(values, r, dim, gi, on);
+      }
+#pragma unroll
+      for (int j = 0; j < GATHER; ++j)
+        if (there[j]) {
+          acc.x = fmaf(wt[j], v[j].x, acc.x); acc.y = fmaf(wt[j], v[j].y, acc.y);
+          acc.z = fmaf(wt[j], v[j].z, acc.z); acc.w = fmaf(wt[j], v[j].w, acc.w);
+        }
+    }
+  }
+  if (on) reinterpret_cast<float4*>(out + (size_t)token * dim)[gi] = acc;
+}
+
+// The same for rows of more than 1024.
 __global__ void weighted_value_fwd_kernel(const int64_t* __restrict__ idx, const float* __restrict__ weights,
                                           const float* __restrict__ values, float* __restrict__ out, int tokens, int top_k,
                                           int rows, int dim, int* __restrict__ status) {
@@ -691,45 +756,6 @@ __global__ void weighted_value_fwd_kernel(const int64_t* __restrict__ idx, const
   const int lane = threadIdx.x & 31;
   const int token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (token >= tokens) return;
-  if (dim <= 1024) {
-    // slots and weights are read once per 32 and handed around by shuffles; a lane owns up to 8 four-column groups and
-    // sums its at most top_k products per column in f32 (f64 multiply-adds run at a fraction of the f32 rate)
-    const int groups = dim / 4;
-    float4 acc[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int k0 = 0; k0 < top_k; k0 += 32) {
-      long long my_row = -1;
-      float my_w = 0.f;
-      if (k0 + lane < top_k) {
-        my_row = idx[(size_t)token * top_k + k0 + lane];
-        my_w = weights[(size_t)token * top_k + k0 + lane];
-        if (my_row < 0 || my_row >= rows) { atomicExch(status + ST_BAD_INDEX, 1); my_row = -1; }
-      }
-      const int n = min(32, top_k - k0);
-      for (int k = 0; k < n; ++k) {
-        const long long r = __shfl_sync(0xffffffffu, my_row, k);
-        const float w = __shfl_sync(0xffffffffu, my_w, k);
-        if (r < 0) continue;
-        const float4* row = reinterpret_cast<const float4*>(values + (size_t)r * dim);
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int gi = u * 32 + lane;
-          if (gi < groups) {
-            const float4 v = __ldg(row + gi);
-            acc[u].x = fmaf(w, v.x, acc[u].x); acc[u].y = fmaf(w, v.y, acc[u].y);
-            acc[u].z = fmaf(w, v.z, acc[u].z); acc[u].w = fmaf(w, v.w, acc[u].w);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int gi = u * 32 + lane;
-      if (gi < groups) reinterpret_cast<float4*>(out + (size_t)token * dim)[gi] = acc[u];
-    }
-    return;
-  }
   for (int c = lane * 4; c < dim; c += 128) {
     double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
     for (int k = 0; k < top_k; ++k) {
@@ -744,7 +770,62 @@ __global__ void weighted_value_fwd_kernel(const int64_t* __restrict__ idx, const
 }
 
 // dw[t,k] = dout[t] . V[idx[t,k]];  dV[idx[t,k],:] += w[t,k] dout[t,:] (f32 atomics, repeats accumulate)
-// (src/tensor/autograd.rs:2263-2323).
+// (src/tensor/autograd.rs:2263-2323).  Rows of up to 1024: a warp a token and 128 columns, the warps of a token in one CTA, which adds
+// up their parts of dw; f64 sums.
+constexpr int VB_WARPS = 8;  // rows of up to 1024
+__global__ void weighted_value_bwd_rows_kernel(const int64_t* __restrict__ idx, const float* __restrict__ weights,
+                                               const float* __restrict__ values, const float* __restrict__ grad_out,
+                                               float* __restrict__ dweights, float* __restrict__ dvalues, int top_k, int rows, int dim) {
+  pdl_begin();
+  __shared__ double parts[VB_WARPS][32];
+  const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5, slices = blockDim.x >> 5, gi = slice * 32 + lane;
+  const size_t token = blockIdx.x;
+  const bool on = gi < dim / 4;
+  const float4 g = on ? reinterpret_cast<const float4*>(grad_out + token * dim)[gi] : make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k0 = 0; k0 < top_k; k0 += 32) {
+    int my_row = -1;
+    float my_w = 0.f;
+    if (k0 + lane < top_k) {
+      const long long r = idx[token * top_k + k0 + lane];
+      my_w = weights[token * top_k + k0 + lane];
+      if (r >= 0 && r < rows) my_row = (int)r;
+    }
+    const int n = min(32, top_k - k0);
+    for (int k = 0; k < n; k += GATHER) {
+      float4 v[GATHER];
+      int row[GATHER];
+#pragma unroll
+      for (int j = 0; j < GATHER; ++j) {
+        row[j] = __shfl_sync(0xffffffffu, my_row, k + j);
+        if (dweights) v[j] = row_piece(values, row[j], dim, gi, on);
+      }
+      if (dvalues)
+#pragma unroll
+        for (int j = 0; j < GATHER; ++j) {
+          const float w = __shfl_sync(0xffffffffu, my_w, k + j);
+          if (on && row[j] >= 0)
+            atomicAdd(reinterpret_cast<float4*>(dvalues + (size_t)row[j] * dim) + gi, make_float4(w * g.x, w * g.y, w * g.z, w * g.w));
+        }
+      if (dweights) {
+        double dot[GATHER];
+#pragma unroll
+        for (int j = 0; j < GATHER; ++j) dot[j] = (double)g.x * v[j].x + (double)g.y * v[j].y + (double)g.z * v[j].z + (double)g.w * v[j].w;
+        const double sum = sum8_over_lanes(dot);
+        if ((lane & 3) == 0) parts[slice][k + sum8_index()] = sum;
+      }
+    }
+    if (dweights) {
+      __syncthreads();
+      if (slice == 0 && lane < n && my_row >= 0) {
+        double sum = 0.0;
+        for (int i = 0; i < slices; ++i) sum += parts[i][lane];
+        dweights[token * top_k + k0 + lane] = (float)sum;
+      }
+      __syncthreads();
+    }
+  }
+}
+// The same for longer rows, a warp a token.
 __global__ void weighted_value_bwd_kernel(const int64_t* __restrict__ idx, const float* __restrict__ weights,
                                           const float* __restrict__ values, const float* __restrict__ grad_out,
                                           float* __restrict__ dweights, float* __restrict__ dvalues, int tokens, int top_k,
@@ -930,7 +1011,9 @@ radix_scatter_kernel(const int* __restrict__ keys, const int* __restrict__ vals,
   }
 }
 
-template <int VPL>  // 16-byte pieces of a row per lane: dim <= VPL * 128
+// A warp a chunk of CHUNK events, VPL 16-byte pieces of a row a lane (dim <= VPL * 128).  Columns shared by several warps, as above, were
+// slower here (16384 tokens of 32 slots 105 -> 220 us): what a run of equal rows costs to follow is paid by each.
+template <int VPL, int CHUNK>
 __global__ void __launch_bounds__(128)
 weighted_value_bwd_sorted_kernel(const int* __restrict__ keys, const int* __restrict__ events,
                                  const float* __restrict__ weights, const float* __restrict__ values,
@@ -938,16 +1021,17 @@ weighted_value_bwd_sorted_kernel(const int* __restrict__ keys, const int* __rest
                                  float* __restrict__ dvalues, long long n, int top_k, int rows, int dim) {
   pdl_begin();
   const int lane = threadIdx.x & 31;
-  const long long base = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32;
+  const long long base = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * CHUNK;
   if (base >= n) return;
   const int groups = dim / 4;
   int my_key = rows, my_event = 0;
   float my_w = 0.f;
-  if (base + lane < n) {
+  if (lane < CHUNK && base + lane < n) {
     my_key = keys[base + lane];
     my_event = events[base + lane];
     if (my_key < rows) my_w = weights[my_event];
   }
+  const int my_token = my_event / top_k;
   float4 acc[VPL], vrow[VPL];
 #pragma unroll
   for (int u = 0; u < VPL; ++u) acc[u] = vrow[u] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -961,38 +1045,39 @@ weighted_value_bwd_sorted_kernel(const int* __restrict__ keys, const int* __rest
       acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
   };
-  for (int i = 0; i < 32; ++i) {
-    const int key = __shfl_sync(0xffffffffu, my_key, i);
-    if (key >= rows) break;  // sorted: nothing valid follows
-    const int event = __shfl_sync(0xffffffffu, my_event, i);
-    const float w = __shfl_sync(0xffffffffu, my_w, i);
-    if (key != cur) {
-      flush();
-      cur = key;
-      if (dweights) {
+  for (int i0 = 0; i0 < CHUNK; i0 += GATHER) {
+    if (__shfl_sync(0xffffffffu, my_key, i0) >= rows) break;  // sorted: nothing valid follows
+    double dot[GATHER];
 #pragma unroll
-        for (int u = 0; u < VPL; ++u) {
-          const int gi = u * 32 + lane;
-          if (gi < groups) vrow[u] = __ldg(reinterpret_cast<const float4*>(values + (size_t)key * dim) + gi);
+    for (int j = 0; j < GATHER; ++j) {
+      const int key = __shfl_sync(0xffffffffu, my_key, i0 + j), token = __shfl_sync(0xffffffffu, my_token, i0 + j);
+      const float w = __shfl_sync(0xffffffffu, my_w, i0 + j);
+      dot[j] = 0.0;
+      if (key >= rows) continue;
+      if (key != cur) {
+        flush();
+        cur = key;
+        if (dweights) {
+#pragma unroll
+          for (int u = 0; u < VPL; ++u) vrow[u] = row_piece(values, key, dim, u * 32 + lane, u * 32 + lane < groups);
         }
       }
-    }
-    const float4* go = reinterpret_cast<const float4*>(grad_out + (size_t)(event / top_k) * dim);
-    float share = 0.f;  // this lane's part of the dot product in f32, the 32 parts are summed in f64
+      float share = 0.f;  // this lane's part of the dot product in f32, the 32 parts are summed in f64
 #pragma unroll
-    for (int u = 0; u < VPL; ++u) {
-      const int gi = u * 32 + lane;
-      if (gi < groups) {
-        const float4 g = __ldg(go + gi);
+      for (int u = 0; u < VPL; ++u) {
+        const float4 g = row_piece(grad_out, token, dim, u * 32 + lane, u * 32 + lane < groups);
         share = fmaf(g.x, vrow[u].x, share); share = fmaf(g.y, vrow[u].y, share);
         share = fmaf(g.z, vrow[u].z, share); share = fmaf(g.w, vrow[u].w, share);
         acc[u].x = fmaf(w, g.x, acc[u].x); acc[u].y = fmaf(w, g.y, acc[u].y);
         acc[u].z = fmaf(w, g.z, acc[u].z); acc[u].w = fmaf(w, g.w, acc[u].w);
       }
+      dot[j] = (double)share;
     }
     if (dweights) {
-      const double dot = warp_sum((double)share);
-      if (lane == 0) dweights[event] = (float)dot;
+      const double sum = sum8_over_lanes(dot);
+      const int at = i0 + sum8_index();
+      const int event = __shfl_sync(0xffffffffu, my_event, at), key = __shfl_sync(0xffffffffu, my_key, at);
+      if ((lane & 3) == 0 && key < rows) dweights[event] = (float)sum;
     }
   }
   flush();
@@ -1113,6 +1198,12 @@ __global__ void move_rows_kernel(const float* __restrict__ src, const int64_t* _
   }
 }
 
+// Half-table rows and a row of queries (or their gradient) `ld` apart that the sixteen-byte forms take.
+bool rows_of_16_bytes(int key_dim, long long ld, const void* query, const void* left, const void* right) {
+  return key_dim % 8 == 0 && key_dim <= 1024 && ld % 4 == 0 &&
+         ((reinterpret_cast<uintptr_t>(query) | reinterpret_cast<uintptr_t>(left) | reinterpret_cast<uintptr_t>(right)) & 15) == 0;
+}
+
 int check_memory_dims(int tokens, int top_k, int dim, const char* who) {
   HL_REQUIRE(tokens > 0 && top_k > 0 && dim > 0, std::string(who) + ": requires non-zero tokens/top_k/dim");
   return HL_OK;
@@ -1196,9 +1287,19 @@ int hl_memory_selected_scores_forward(hl_ctx* ctx, const int64_t* indices, const
   if (rc != HL_OK) return rc;
   HL_REQUIRE(side == 0 || (right_keys && key_dim % 2 == 0 && (long long)side * side == slots),
              "hl_memory_selected_scores_forward: product-key mode needs both half tables, even key_dim and square slots");
-  pdl(selected_scores_fwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream).streaming(4.0 * tokens * top_k * key_dim)(indices, query, ld_query, left_or_keys, right_keys,
-                                                                           scores, tokens, top_k, side, key_dim, slots,
-                                                                           ctx->status_dev);
+  if (side > 0 && rows_of_16_bytes(key_dim, ld_query, query, left_or_keys, right_keys)) {
+    auto launch = [&](auto kern) {
+      pdl(kern, tokens, 128, 0, ctx->stream).streaming(4.0 * tokens * top_k * key_dim)(indices, query, ld_query, left_or_keys, right_keys, scores,
+                                                                                      top_k, side, key_dim, slots, ctx->status_dev);
+    };
+    if (key_dim <= 128) launch(selected_scores_rows_kernel<1>);
+    else if (key_dim <= 256) launch(selected_scores_rows_kernel<2>);
+    else if (key_dim <= 512) launch(selected_scores_rows_kernel<4>);
+    else launch(selected_scores_rows_kernel<8>);
+  } else {
+    pdl(selected_scores_fwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream).streaming(4.0 * tokens * top_k * key_dim)(
+        indices, query, ld_query, left_or_keys, right_keys, scores, tokens, top_k, side, key_dim, slots, ctx->status_dev);
+  }
   HL_LAUNCH_CHECK("selected_scores_fwd_kernel");
   count_launch(ctx);
   return HL_OK;
@@ -1218,9 +1319,14 @@ int hl_memory_selected_scores_backward(hl_ctx* ctx, const int64_t* indices, cons
   int token_blocks = half_keys ? key_gradient_shares(ctx, keys) : 0;
   // the tensor-core form's scratch holds the queries' pieces as well: where the device has no room for them, the f32 form
   const bool tensor = token_blocks > 0 && try_workspace(ctx, key_gradient_bytes(keys, token_blocks));
-  pdl(selected_scores_bwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream)(
-      indices, query, ld_query, left_or_keys, right_keys, grad_scores, grad_query, ld_grad_query, grad_left_or_keys,
-      grad_right_keys, tokens, top_k, side, key_dim, slots, tensor ? static_cast<int*>(ctx->workspace) : nullptr);
+  int* clear = tensor ? static_cast<int*>(ctx->workspace) : nullptr;
+  if (side > 0 && grad_query && rows_of_16_bytes(key_dim, ld_grad_query, grad_query, left_or_keys, right_keys))
+    pdl(selected_query_gradient_kernel, (unsigned)ceil_div_ll((long long)tokens * ceil_div(key_dim, 128), 4), 128, 0, ctx->stream)(
+        indices, left_or_keys, right_keys, grad_scores, grad_query, ld_grad_query, tokens, top_k, side, key_dim, slots, clear);
+  else
+    pdl(selected_scores_bwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream)(
+        indices, query, ld_query, left_or_keys, right_keys, grad_scores, grad_query, ld_grad_query, grad_left_or_keys,
+        grad_right_keys, tokens, top_k, side, key_dim, slots, clear);
   HL_LAUNCH_CHECK("selected_scores_bwd_kernel");
   count_launch(ctx);
   if (half_keys) {
@@ -1275,8 +1381,12 @@ int hl_memory_weighted_value_forward(hl_ctx* ctx, const int64_t* indices, const 
   int rc = check_memory_dims(tokens, top_k, dim, "hl_memory_weighted_value_forward");
   if (rc != HL_OK) return rc;
   HL_REQUIRE(rows > 0 && dim % 4 == 0, "hl_memory_weighted_value_forward: non-zero rows/row_dim, row_dim a multiple of 4");
-  pdl(weighted_value_fwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream)(indices, weights, values, out, tokens, top_k, rows,
-                                                                          dim, ctx->status_dev);
+  if (dim <= 1024)
+    pdl(weighted_value_rows_kernel, (unsigned)ceil_div_ll((long long)tokens * ceil_div(dim, 128), 4), 128, 0, ctx->stream)(
+        indices, weights, values, out, tokens, top_k, rows, dim, ctx->status_dev);
+  else
+    pdl(weighted_value_fwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream)(indices, weights, values, out, tokens, top_k, rows, dim,
+                                                                            ctx->status_dev);
   HL_LAUNCH_CHECK("weighted_value_fwd_kernel");
   count_launch(ctx);
   return HL_OK;
@@ -1320,19 +1430,25 @@ int hl_memory_weighted_value_backward(hl_ctx* ctx, const int64_t* indices, const
     }
     const int *keys = keys_a, *ev = ev_a;  // the last pass's output
     count_launch(ctx, 3 * passes);
-    const unsigned blocks = (unsigned)ceil_div_ll(ceil_div_ll(n, 32), 4);
-    if (dim <= 512)
-      pdl(weighted_value_bwd_sorted_kernel<4>, blocks, 128, 0, ctx->stream)(keys, ev, weights, values, grad_out, grad_weights,
-                                                                           grad_values, n, top_k, rows, dim);
-    else
-      pdl(weighted_value_bwd_sorted_kernel<8>, blocks, 128, 0, ctx->stream)(keys, ev, weights, values, grad_out, grad_weights,
-                                                                           grad_values, n, top_k, rows, dim);
+    auto launch = [&](auto kern, int chunk) {
+      pdl(kern, (unsigned)ceil_div_ll(ceil_div_ll(n, chunk), 4), 128, 0, ctx->stream)(keys, ev, weights, values, grad_out, grad_weights, grad_values,
+                                                                                      n, top_k, rows, dim);
+    };
+    // Short chunks where the warps of long ones would not fill the chip, us a call with its sort, long / short: 65536 events 210 / 200 and
+    // 155 / 145 (many and few distinct rows), 131072 260 / 265 and 180 / 180, 524288 375 / 380 and 240 / 255.
+    const bool few = n < 100000;
+    if (dim <= 512) few ? launch(weighted_value_bwd_sorted_kernel<4, 8>, 8) : launch(weighted_value_bwd_sorted_kernel<4, 32>, 32);
+    else few ? launch(weighted_value_bwd_sorted_kernel<8, 8>, 8) : launch(weighted_value_bwd_sorted_kernel<8, 32>, 32);
     HL_LAUNCH_CHECK("weighted_value_bwd_sorted_kernel");
     count_launch(ctx, 2);
     return HL_OK;
   }
-  pdl(weighted_value_bwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream)(indices, weights, values, grad_out, grad_weights,
-                                                                          grad_values, tokens, top_k, rows, dim);
+  if (dim <= 1024)
+    pdl(weighted_value_bwd_rows_kernel, tokens, 32 * ceil_div(dim, 128), 0, ctx->stream)(indices, weights, values, grad_out, grad_weights,
+                                                                                        grad_values, top_k, rows, dim);
+  else
+    pdl(weighted_value_bwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream)(indices, weights, values, grad_out, grad_weights, grad_values,
+                                                                            tokens, top_k, rows, dim);
   HL_LAUNCH_CHECK("weighted_value_bwd_kernel");
   count_launch(ctx);
   return HL_OK;

@@ -434,3 +434,38 @@ def test_row_ordered_value_backward_reports_a_bad_index_and_zeroes_its_weight_gr
     good = np.ones_like(idx, bool); good[5, 3] = good[100, 0] = False
     want_dw = np.einsum("td,tkd->tk", go.astype(np.float64), vals[np.clip(idx, 0, rows - 1)].astype(np.float64))
     assert np.allclose(got[good], want_dw[good], rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("tokens,top_k,side,key_dim,dim", [(37, 5, 9, 16, 4), (65, 33, 20, 136, 132), (41, 40, 16, 512, 512), (20, 32, 16, 1024, 1024),
+                                                           (9, 7, 12, 1032, 1028), (30, 9, 10, 12, 8), (6400, 16, 40, 256, 260), (3200, 33, 30, 264, 640)])
+def test_gathers_at_the_edges_of_their_forms(tokens, top_k, side, key_dim, dim):
+    """Rows of one piece to more than a warp's, slots that fill no group of eight, forms for any size, few and many events of the value
+    backward.  Bounds: f32 sums of at most 64 products (or top_k of them, or an event's run), so 2^-24 sqrt of that many of the terms'
+    magnitudes, times a few."""
+    from heirloom_b200 import cuda
+    c = ctx()
+    rng = np.random.default_rng(tokens + key_dim)
+    q = rng.standard_normal((tokens, key_dim)).astype(np.float32)
+    kl, kr = (rng.standard_normal((side, key_dim // 2)).astype(np.float32) for _ in range(2))
+    vals = rng.standard_normal((side * side, dim)).astype(np.float32)
+    idx = rng.integers(0, side * side, (tokens, top_k))
+    idx[:, 1] = idx[:, 0]
+    idx[-1, -1] = side * side - 1
+    w = rng.random((tokens, top_k)).astype(np.float32)
+    g = rng.standard_normal((tokens, top_k)).astype(np.float32)
+    go = rng.standard_normal((tokens, dim)).astype(np.float32)
+    di = dev(idx, I64)
+    keys = np.concatenate([kl[idx // side], kr[idx % side]], axis=2).astype(np.float64)
+    assert_close("scores", host(cuda.memory_selected_scores_forward(c, di, dev(q), dev(kl), dev(kr))), np.einsum("td,tkd->tk", q.astype(np.float64), keys),
+                 atol=4e-6 * np.sqrt(key_dim), rtol=1e-6)
+    dq, _, _ = cuda.memory_selected_scores_backward(c, di, dev(q), dev(kl), dev(kr), dev(g))
+    assert_close("dq", host(dq), np.einsum("tk,tkd->td", g.astype(np.float64), keys), atol=4e-6 * np.sqrt(top_k), rtol=1e-6)
+    picked = vals[idx].astype(np.float64)
+    assert_close("value", host(cuda.memory_weighted_value_forward(c, di, dev(w), dev(vals))), np.einsum("tk,tkd->td", w.astype(np.float64), picked),
+                 atol=4e-6 * np.sqrt(top_k), rtol=1e-6)
+    dw, dv = cuda.memory_weighted_value_backward(c, di, dev(w), dev(vals), dev(go))
+    assert_close("dw", host(dw), np.einsum("td,tkd->tk", go.astype(np.float64), picked), atol=4e-6 * np.sqrt(dim), rtol=1e-6)
+    want = np.zeros((side * side, dim))
+    np.add.at(want, idx.reshape(-1), (w[..., None].astype(np.float64) * go[:, None, :]).reshape(-1, dim))
+    run = np.bincount(idx.reshape(-1)).max()
+    assert_close("dv", host(dv), want, atol=1e-6 * np.sqrt(run) * 4 + 2e-7 * run, rtol=1e-6)
