@@ -138,11 +138,14 @@ side_scores_kernel(const float* __restrict__ query, long long ld_q, const float*
 // kernels.ptx:2121-2262): top-`beam` per side (desc score, asc index), beam^2 f32 sums, top-k by
 // (desc sum, asc slot).  One warp per token; side <= 2048, beam <= 32, top_k <= beam*beam.
 //
-// The selection never walks the side scores one winner at a time.  Scores become order-preserving 32-bit keys held
-// in registers; the beam-th largest key is found by a four-pass radix select over a per-warp histogram; the chosen
-// entries are compacted in index order (which settles ties at the threshold), sorted across the lanes, and the
-// final top-k merges the 32 sorted rows `left[i] + right[.]` with one pointer per lane: a round is two warp
-// reductions, and only the winning lane advances. ---------------------------------------------------------------
+// A warp a token, and everything it does is a chain of dependent steps, so what counts is their number (2048 tokens: 50 -> 22 us, 16384
+// tokens 141 -> 81).  Scores become order-preserving 32-bit keys held in registers, all loaded at once.  The 32nd largest of the lanes'
+// two largest keys is a bound that the beam's keys reach and few others (36 of 512 random ones); those are sorted with their
+// indices.  Of the sums of two sorted beams only those of ranks i and j with (i + 1)(j + 1) <= top_k can be among the top_k, 119 for
+// 32, since as many pairs of lower ranks are no smaller; they are sorted with their slots.  Whatever that does not settle (more than 64
+// keys that reach the bound, top_k above 32, infinities and NaNs in a beam, a pair left out that equals the last one taken) goes the
+// general way: a four-pass radix select over a per-warp histogram, and a merge of the 32 sorted rows `left[i] + right[.]` with
+// one pointer per lane, where a round is two warp reductions and only the winning lane advances. ---------------------------------
 constexpr int PK_MAX_PER_LANE = 64;
 
 // a > b as floats  <=>  okey(a) > okey(b); both zeros share a key, a NaN gets the lowest key 1, 0 means "no entry"
@@ -155,113 +158,165 @@ __device__ __forceinline__ float okey_value(unsigned k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
+// A step of a bitonic sort across the lanes, of N values a lane side by side.
+template <int N, typename V>
+__device__ __forceinline__ void exchange(V (&v)[N], int stride, bool keep_max) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const V other = __shfl_xor_sync(0xffffffffu, v[i], stride);
+    v[i] = keep_max ? (v[i] > other ? v[i] : other) : (v[i] < other ? v[i] : other);
+  }
+}
+// Each v[i] in descending order over the lanes.
+template <int N, typename V>
+__device__ __forceinline__ void sort_lanes(V (&v)[N]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+    for (int stride = size >> 1; stride > 0; stride >>= 1) exchange(v, stride, ((lane & stride) == 0) == ((lane & size) == 0));
+}
+// The 32 largest of two descending vectors, in no order but one that merge_lanes takes.
+template <typename V> __device__ __forceinline__ V upper_half(V a, V b) {
+  const V other = __shfl_sync(0xffffffffu, b, 31 - (threadIdx.x & 31));
+  return a > other ? a : other;
+}
+template <int N, typename V>
+__device__ __forceinline__ void merge_lanes(V (&v)[N]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int stride = 16; stride > 0; stride >>= 1) exchange(v, stride, (lane & stride) == 0);
+}
+
+struct TopkScratch {  // of a warp
+  unsigned hist[256], key[64];
+  int index[64];
+  float rscore[32];
+};
+
+// The beam's keys and indices of one side, sorted across the lanes: key descending, index ascending; zero past the beam.
 template <int PER_LANE>
-__global__ void __launch_bounds__(128)
-product_key_topk_kernel(const float* __restrict__ left, const float* __restrict__ right, int64_t* __restrict__ out,
-                        int tokens, int side, int top_k, int beam, int* __restrict__ status, int64_t* __restrict__ kept,
-                        const long long* __restrict__ kept_row) {
-  pdl_begin();
-  __shared__ unsigned s_hist[4][256];
-  __shared__ unsigned s_key[4][32];
-  __shared__ int s_index[4][32];
-  __shared__ float s_rscore[4][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int token = blockIdx.x * 4 + w;
-  if (token >= tokens) return;
+__device__ __forceinline__ unsigned long long radix_beam(const unsigned (&key)[PER_LANE], int beam, TopkScratch& sc) {
+  const int lane = threadIdx.x & 31;
   const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
-  unsigned l_key = 0u;  // left beam entry `lane` after the sort
-  int l_idx = 0;
-  for (int sd = 0; sd < 2; ++sd) {
-    const float* s = (sd == 0 ? left : right) + (size_t)token * side;
-    unsigned key[PER_LANE];
-#pragma unroll
-    for (int i = 0; i < PER_LANE; ++i) key[i] = (i * 32 + lane < side) ? okey(s[i * 32 + lane]) : 0u;
-    // radix select, 8 bits a pass from the top: afterwards `kstar` is the beam-th largest key and `need` says how
-    // many entries equal to it belong to the beam
-    unsigned kstar = 0u, decided = 0u;
-    int need = beam;
+  // radix select, 8 bits a pass from the top: afterwards `kstar` is the beam-th largest key and `need` says how
+  // many entries equal to it belong to the beam
+  unsigned kstar = 0u, decided = 0u;
+  int need = beam;
 #pragma unroll 1
-    for (int shift = 24; shift >= 0; shift -= 8) {
-      for (int b = lane; b < 256; b += 32) s_hist[w][b] = 0u;
-      __syncwarp();
+  for (int shift = 24; shift >= 0; shift -= 8) {
+    for (int b = lane; b < 256; b += 32) sc.hist[b] = 0u;
+    __syncwarp();
 #pragma unroll
-      for (int i = 0; i < PER_LANE; ++i)
-        if (key[i] != 0u && (key[i] & decided) == kstar) atomicAdd(&s_hist[w][(key[i] >> shift) & 255u], 1u);
-      __syncwarp();
-      unsigned c[8], mine = 0u;  // the lane owns digits 8*lane .. 8*lane+7
+    for (int i = 0; i < PER_LANE; ++i)
+      if (key[i] != 0u && (key[i] & decided) == kstar) atomicAdd(&sc.hist[(key[i] >> shift) & 255u], 1u);
+    __syncwarp();
+    unsigned c[8], mine = 0u;  // the lane owns digits 8*lane .. 8*lane+7
 #pragma unroll
-      for (int b = 0; b < 8; ++b) { c[b] = s_hist[w][lane * 8 + b]; mine += c[b]; }
-      unsigned from_here = mine;  // entries whose digit is in this lane's range or above
+    for (int b = 0; b < 8; ++b) { c[b] = sc.hist[lane * 8 + b]; mine += c[b]; }
+    unsigned from_here = mine;  // entries whose digit is in this lane's range or above
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned y = __shfl_down_sync(full, from_here, o);
-        if (lane + o < 32) from_here += y;
-      }
-      const unsigned above = from_here - mine;
-      const bool here = above < (unsigned)need && from_here >= (unsigned)need;
-      int digit = 0;
-      unsigned over = 0u;
-      if (here) {
-        unsigned run = above;
-        bool found = false;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_down_sync(full, from_here, o);
+      if (lane + o < 32) from_here += y;
+    }
+    const unsigned above = from_here - mine;
+    const bool here = above < (unsigned)need && from_here >= (unsigned)need;
+    int digit = 0;
+    unsigned over = 0u;
+    if (here) {
+      unsigned run = above;
+      bool found = false;
 #pragma unroll
-        for (int b = 7; b >= 0; --b) {
-          if (!found) {
-            if (run + c[b] >= (unsigned)need) { digit = lane * 8 + b; over = run; found = true; }
-            else run += c[b];
-          }
+      for (int b = 7; b >= 0; --b) {
+        if (!found) {
+          if (run + c[b] >= (unsigned)need) { digit = lane * 8 + b; over = run; found = true; }
+          else run += c[b];
         }
       }
-      const unsigned who = __ballot_sync(full, here);
-      const int src = who ? __ffs(who) - 1 : 0;  // who == 0 only with fewer than `beam` entries, which the host rejects
-      digit = __shfl_sync(full, digit, src);
-      over = __shfl_sync(full, over, src);
-      kstar |= (unsigned)digit << shift;
-      decided |= 255u << shift;
-      need -= (int)over;
-      __syncwarp();
     }
-    // compaction in index order: everything above the threshold, and the first `need` entries equal to it
-    int base = 0, eq_seen = 0;
-#pragma unroll
-    for (int i = 0; i < PER_LANE; ++i) {
-      const bool eq = key[i] == kstar && kstar != 0u;
-      const unsigned b_eq = __ballot_sync(full, eq);
-      const bool take = (key[i] > kstar && kstar != 0u) || (eq && eq_seen + __popc(b_eq & below) < need);
-      eq_seen += __popc(b_eq);
-      const unsigned b_take = __ballot_sync(full, take);
-      if (take) {
-        const int pos = base + __popc(b_take & below);
-        if (pos < 32) { s_key[w][pos] = key[i]; s_index[w][pos] = i * 32 + lane; }
-      }
-      base += __popc(b_take);
-    }
-    __syncwarp();
-    // sort the beam across the lanes: key descending, index ascending
-    const bool valid = lane < base && lane < 32;
-    unsigned long long c64 = valid ? ((unsigned long long)s_key[w][lane] << 32) | (0xffffffffu - (unsigned)s_index[w][lane]) : 0ull;
-#pragma unroll
-    for (int size = 2; size <= 32; size <<= 1) {
-#pragma unroll
-      for (int stride = size >> 1; stride > 0; stride >>= 1) {
-        const unsigned long long other = __shfl_xor_sync(full, c64, stride);
-        const bool keep_max = ((lane & stride) == 0) == ((lane & size) == 0);
-        c64 = keep_max ? (c64 > other ? c64 : other) : (c64 < other ? c64 : other);
-      }
-    }
-    const unsigned k_sorted = (unsigned)(c64 >> 32);
-    const int i_sorted = (int)(0xffffffffu - (unsigned)(c64 & 0xffffffffull));
-    __syncwarp();
-    if (sd == 0) {
-      l_key = k_sorted;
-      l_idx = i_sorted;
-    } else {
-      s_key[w][lane] = k_sorted;
-      s_index[w][lane] = i_sorted;
-      s_rscore[w][lane] = okey_value(k_sorted);
-    }
+    const unsigned who = __ballot_sync(full, here);
+    const int src = who ? __ffs(who) - 1 : 0;  // who == 0 only with fewer than `beam` entries, which the host rejects
+    digit = __shfl_sync(full, digit, src);
+    over = __shfl_sync(full, over, src);
+    kstar |= (unsigned)digit << shift;
+    decided |= 255u << shift;
+    need -= (int)over;
     __syncwarp();
   }
+  // compaction in index order: everything above the threshold, and the first `need` entries equal to it
+  int base = 0, eq_seen = 0;
+#pragma unroll
+  for (int i = 0; i < PER_LANE; ++i) {
+    const bool eq = key[i] == kstar && kstar != 0u;
+    const unsigned b_eq = __ballot_sync(full, eq);
+    const bool take = (key[i] > kstar && kstar != 0u) || (eq && eq_seen + __popc(b_eq & below) < need);
+    eq_seen += __popc(b_eq);
+    const unsigned b_take = __ballot_sync(full, take);
+    if (take) {
+      const int pos = base + __popc(b_take & below);
+      if (pos < 32) { sc.key[pos] = key[i]; sc.index[pos] = i * 32 + lane; }
+    }
+    base += __popc(b_take);
+  }
+  __syncwarp();
+  const bool valid = lane < base && lane < 32;
+  unsigned long long v[1] = {valid ? ((unsigned long long)sc.key[lane] << 32) | (0xffffffffu - (unsigned)sc.index[lane]) : 0ull};
+  __syncwarp();
+  sort_lanes(v);
+  return v[0];
+}
+template <int PER_LANE>
+__device__ __forceinline__ unsigned long long beam_of_side(const float* s, int side, int beam, TopkScratch& sc) {
+  const int lane = threadIdx.x & 31;
+  const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
+  float score[PER_LANE];
+#pragma unroll
+  for (int i = 0; i < PER_LANE; ++i) score[i] = s[min(i * 32 + lane, side - 1)];
+  unsigned key[PER_LANE], top[2] = {0u, 0u};
+#pragma unroll
+  for (int i = 0; i < PER_LANE; ++i) {
+    key[i] = i * 32 + lane < side ? okey(score[i]) : 0u;
+    top[1] = max(top[1], min(top[0], key[i]));
+    top[0] = max(top[0], key[i]);
+  }
+  sort_lanes(top);
+  const unsigned bound = max(1u, __reduce_min_sync(full, upper_half(top[0], top[1])));
+  int count = 0;
+#pragma unroll
+  for (int i = 0; i < PER_LANE; ++i) {
+    const unsigned who = __ballot_sync(full, key[i] >= bound);
+    const int at = count + __popc(who & below);
+    if (key[i] >= bound && at < 64) {
+      sc.key[at] = key[i];
+      sc.index[at] = i * 32 + lane;
+    }
+    count += __popc(who);
+  }
+  __syncwarp();
+  if (count > 64) return radix_beam(key, beam, sc);
+  unsigned long long v[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int at = h * 32 + lane;
+    v[h] = at < count ? ((unsigned long long)sc.key[at] << 32) | (0xffffffffu - (unsigned)sc.index[at]) : 0ull;
+  }
+  __syncwarp();
+  sort_lanes(v);
+  unsigned long long best[1] = {upper_half(v[0], v[1])};
+  merge_lanes(best);
+  return lane < beam ? best[0] : 0ull;
+}
+
+// The top_k of all sums of the two beams, the general way.
+__device__ __noinline__ void merge_beams(unsigned l_key, int l_idx, unsigned r_key, int r_idx, int64_t* out, int64_t* kept, int side, int top_k,
+                                         int beam, TopkScratch& sc, int* status) {
+  const int lane = threadIdx.x & 31;
+  const unsigned full = 0xffffffffu;
+  sc.key[lane] = r_key;
+  sc.index[lane] = r_idx;
+  sc.rscore[lane] = okey_value(r_key);
+  __syncwarp();
   // row `lane` of the candidate matrix: left[lane] + right[j], non-increasing in j because the right beam is sorted
   // and f32 addition is monotone.  Equal sums sit next to each other; among them the lowest slot goes first.
   const bool has = lane < beam && l_key != 0u;
@@ -276,12 +331,12 @@ product_key_topk_kernel(const float* __restrict__ left, const float* __restrict_
     const unsigned avail = ~used & beam_mask;
     if (!has || avail == 0u) return;
     const int j = __ffs(avail) - 1;
-    if (s_key[w][j] == 0u) return;
-    const float sum = __fadd_rn(ls, s_rscore[w][j]);
-    int best_ri = s_index[w][j], best_j = j;
+    if (sc.key[j] == 0u) return;
+    const float sum = __fadd_rn(ls, sc.rscore[j]);
+    int best_ri = sc.index[j], best_j = j;
     for (int jj = j + 1; jj < beam; ++jj) {
-      if (s_key[w][jj] == 0u || !(__fadd_rn(ls, s_rscore[w][jj]) == sum)) break;
-      if (!((used >> jj) & 1u) && s_index[w][jj] < best_ri) { best_ri = s_index[w][jj]; best_j = jj; }
+      if (sc.key[jj] == 0u || !(__fadd_rn(ls, sc.rscore[jj]) == sum)) break;
+      if (!((used >> jj) & 1u) && sc.index[jj] < best_ri) { best_ri = sc.index[jj]; best_j = jj; }
     }
     head_key = okey(sum);
     head_slot = (unsigned)(l_idx * side + best_ri);
@@ -293,8 +348,8 @@ product_key_topk_kernel(const float* __restrict__ left, const float* __restrict_
     if (m == 0u) {
       if (lane == 0) {
         atomicExch(status + ST_BAD_ARGUMENT, 1);
-        out[(size_t)token * top_k + r] = 0;
-        if (kept) kept[(*kept_row + token) * top_k + r] = 0;
+        out[r] = 0;
+        if (kept) kept[r] = 0;
       }
       continue;
     }
@@ -304,10 +359,69 @@ product_key_topk_kernel(const float* __restrict__ left, const float* __restrict_
       advance();
     }
     if (lane == 0) {
-      out[(size_t)token * top_k + r] = (long long)bs;
-      if (kept) kept[(*kept_row + token) * top_k + r] = (long long)bs;
+      out[r] = (long long)bs;
+      if (kept) kept[r] = (long long)bs;
     }
   }
+}
+
+template <int PER_LANE>
+__global__ void __launch_bounds__(128)
+product_key_topk_kernel(const float* __restrict__ left, const float* __restrict__ right, int64_t* __restrict__ out,
+                        int tokens, int side, int top_k, int beam, int* __restrict__ status, int64_t* __restrict__ kept,
+                        const long long* __restrict__ kept_row) {
+  pdl_begin();
+  __shared__ TopkScratch scratch[4];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int token = blockIdx.x * 4 + w;
+  if (token >= tokens) return;
+  const unsigned full = 0xffffffffu;
+  TopkScratch& sc = scratch[w];
+  const unsigned long long l = beam_of_side<PER_LANE>(left + (size_t)token * side, side, beam, sc);
+  const unsigned long long r = beam_of_side<PER_LANE>(right + (size_t)token * side, side, beam, sc);
+  const unsigned l_key = (unsigned)(l >> 32), r_key = (unsigned)(r >> 32);
+  const int l_idx = (int)(0xffffffffu - (unsigned)l), r_idx = (int)(0xffffffffu - (unsigned)r);
+  out += (size_t)token * top_k;
+  if (kept) kept += (*kept_row + token) * top_k;
+  const float ls = okey_value(l_key), rs = okey_value(r_key);
+  bool general = top_k > 32 || __any_sync(full, lane < beam && !(isfinite(ls) && isfinite(rs)));
+  if (!general) {
+    const int mine = lane < beam ? min(beam, top_k / (lane + 1)) : 0;  // pairs of left rank `lane`
+    int upto = mine;                                                    // pairs up to and with it
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(full, upto, o);
+      if (lane >= o) upto += y;
+    }
+    const int pairs = __shfl_sync(full, upto, 31);  // at most 119
+    unsigned long long v[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const int c = m * 32 + lane;
+      int i = 0;
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1)
+        if (c >= __shfl_sync(full, upto, i + step - 1)) i += step;
+      const int j = (c - __shfl_sync(full, upto - mine, i)) & 31;
+      const float sum = __fadd_rn(__shfl_sync(full, ls, i), __shfl_sync(full, rs, j));
+      const unsigned slot = (unsigned)(__shfl_sync(full, l_idx, i) * side + __shfl_sync(full, r_idx, j));
+      v[m] = c < pairs ? ((unsigned long long)okey(sum) << 32) | (0xffffffffu - slot) : 0ull;
+    }
+    sort_lanes(v);
+    unsigned long long two[2] = {upper_half(v[0], v[1]), upper_half(v[2], v[3])};
+    merge_lanes(two);
+    unsigned long long best[1] = {upper_half(two[0], two[1])};
+    merge_lanes(best);
+    const unsigned last = (unsigned)(__shfl_sync(full, best[0], top_k - 1) >> 32);
+    const float next = __fadd_rn(ls, __shfl_sync(full, rs, mine & 31));  // the largest of this rank's pairs that were left out
+    general = __any_sync(full, lane < beam && mine < beam && okey(next) == last);
+    if (!general && lane < top_k) {
+      const long long slot = (long long)(0xffffffffu - (unsigned)best[0]);
+      out[lane] = slot;
+      if (kept) kept[lane] = slot;
+    }
+  }
+  if (general) merge_beams(l_key, l_idx, r_key, r_idx, out, kept, side, top_k, beam, sc, status);
 }
 
 __global__ void split_rows_kernel(const int64_t* __restrict__ rows, int64_t* __restrict__ left, int64_t* __restrict__ right,
