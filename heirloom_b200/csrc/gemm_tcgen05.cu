@@ -1232,6 +1232,13 @@ int gemm_bf16_loss_gradient(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, c
   g.out_dtype = HL_BF16;
   return gemm_bf16_run(ctx, &g, a, b, dlogits, bias, nullptr, nullptr, nullptr, 0, nullptr, &stats);
 }
+bool gemm_bf16_scratch(hl_ctx* ctx, const hl_gemm_desc* d, size_t* bytes) {
+  const int sms = persistent_sms(ctx);
+  const GemmPlan plan = gemm_plan(d, sms);
+  const bool small = small_plan(ctx, d, plan, sms).splits > 0;
+  *bytes = small ? 0 : plan.splitk_bytes;
+  return small || plan.sk_tiles == 0;
+}
 bool gemm_bf16_small_applies(hl_ctx* ctx, const hl_gemm_desc* d) {
   const int sms = persistent_sms(ctx);
   return small_plan(ctx, d, gemm_plan(d, sms), sms).splits > 0;

@@ -48,6 +48,8 @@ int gemm_small_run(hl_ctx* ctx, const hl_gemm_desc* d, const GemmSmallPlan& plan
 // The GEMM with its scratch taken from (and grown in) the context.
 int gemm_bf16_ctx(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, void* c, const float* bias,
                   const void* aux_in, void* aux_out);
+// The scratch that gemm_bf16_ctx would take, or false where the product also uses the context's flags, which only one stream may.
+bool gemm_bf16_scratch(hl_ctx* ctx, const hl_gemm_desc* d, size_t* bytes);
 // A plain product with the sums of A's rows over the contraction beside it (a weight gradient and its bias gradient), where
 // that costs no launch of its own; *done tells whether it was one of those, otherwise nothing has been launched.
 bool gemm_bf16_small_applies(hl_ctx* ctx, const hl_gemm_desc* d);
@@ -258,6 +260,15 @@ int key_gradient_run(hl_ctx* ctx, const KeyGradient& k, int shares, void* scratc
 // hl_product_key_topk_from_side_scores whose choices go to rows *kept_row and on of `kept` as well (null: nowhere else).
 int product_key_topk_impl(hl_ctx* ctx, const float* left_scores, const float* right_scores, int64_t* out, int tokens, int side, int top_k,
                           int beam, int64_t* kept, const long long* kept_row);
+
+// hl_memory_weighted_value_backward in two: the (token, slot) events sorted by row, which needs the indices alone, and the rest.  `keys`
+// and `events` lie in value_sort_bytes, half each; rows that do not exist report themselves and zero their grad_weights (may be null).
+bool value_events_ordered(long long n, int rows, int dim);
+size_t value_sort_bytes(long long n);
+size_t value_order_scratch_bytes(long long n);
+int value_sort(hl_ctx* ctx, const int64_t* indices, long long n, int rows, int* keys, int* events, void* scratch, float* grad_weights);
+int weighted_value_backward_ordered(hl_ctx* ctx, const int* keys, const int* events, const float* weights, const float* values,
+                                    const float* grad_out, float* grad_weights, float* grad_values, long long n, int top_k, int rows, int dim);
 
 struct AdamPlan;
 int adam_plan_create(hl_ctx* ctx, const hl_adamw_tensor* tensors, int count, AdamPlan** out);

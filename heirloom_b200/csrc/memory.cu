@@ -1506,6 +1506,65 @@ int hl_memory_weighted_value_forward(hl_ctx* ctx, const int64_t* indices, const 
   return HL_OK;
 }
 
+}  // extern "C" (reopened below)
+
+namespace hl {
+// Row order of a step's (token, slot) events (see weighted_value_bwd_sorted_kernel).
+bool value_events_ordered(long long n, int rows, int dim) { return n >= 32768 && n < (1ll << 31) - 64 && dim <= 1024 && rows < (1 << 30); }
+static size_t value_array_bytes(long long n) { return ((size_t)n * sizeof(int) + 255) & ~size_t(255); }
+size_t value_sort_bytes(long long n) { return 2 * value_array_bytes(n); }
+size_t value_order_scratch_bytes(long long n) {  // keys and events of every other pass; digit counts of every tile, then their totals
+  return 2 * value_array_bytes(n) + (((size_t)RS_DIGITS * ((size_t)ceil_div_ll(n, RS_TILE) + 1) * sizeof(int) + 255) & ~size_t(255));
+}
+int value_sort(hl_ctx* ctx, const int64_t* indices, long long n, int rows, int* keys, int* events, void* scratch, float* grad_weights) {
+  uint8_t* ws = static_cast<uint8_t*>(scratch);
+  const size_t arr = value_array_bytes(n);
+  int *keys_a = keys, *ev_a = events, *keys_b = reinterpret_cast<int*>(ws), *ev_b = reinterpret_cast<int*>(ws + arr);
+  int* hist = reinterpret_cast<int*>(ws + 2 * arr);
+  const int n_tiles = (int)ceil_div_ll(n, RS_TILE);
+  int end_bit = 1;
+  while ((1ll << end_bit) <= rows) ++end_bit;  // the sentinel key `rows` must sort last
+  const int passes = ceil_div(end_bit, RS_BITS);
+  if (passes & 1) {  // so that the last pass writes where the caller wants it
+    std::swap(keys_a, keys_b);
+    std::swap(ev_a, ev_b);
+  }
+  pdl(value_event_keys_kernel, (unsigned)ceil_div_ll(n, 256), 256, 0, ctx->stream)(indices, n, rows, keys_a, ev_a, grad_weights, ctx->status_dev);
+  HL_LAUNCH_CHECK("value_event_keys_kernel");
+  for (int pass = 0; pass < passes; ++pass) {
+    const int shift = pass * RS_BITS;
+    pdl(radix_hist_kernel, n_tiles, RS_THREADS, 0, ctx->stream)(keys_a, n, shift, hist, n_tiles);
+    HL_LAUNCH_CHECK("radix_hist_kernel");
+    int* totals = hist + (size_t)RS_DIGITS * n_tiles;
+    pdl(radix_scan_rows_kernel, RS_DIGITS, RS_THREADS, 0, ctx->stream)(hist, n_tiles, totals);
+    HL_LAUNCH_CHECK("radix_scan_rows_kernel");
+    pdl(radix_scatter_kernel, n_tiles, RS_THREADS, 0, ctx->stream)(keys_a, ev_a, keys_b, ev_b, n, shift, hist, totals, n_tiles);
+    HL_LAUNCH_CHECK("radix_scatter_kernel");
+    std::swap(keys_a, keys_b);
+    std::swap(ev_a, ev_b);
+  }
+  count_launch(ctx, 1 + 3 * passes);
+  return HL_OK;
+}
+int weighted_value_backward_ordered(hl_ctx* ctx, const int* keys, const int* events, const float* weights, const float* values,
+                                    const float* grad_out, float* grad_weights, float* grad_values, long long n, int top_k, int rows, int dim) {
+  auto launch = [&](auto kern, int chunk) {
+    pdl(kern, (unsigned)ceil_div_ll(ceil_div_ll(n, chunk), 4), 128, 0, ctx->stream)(keys, events, weights, values, grad_out, grad_weights,
+                                                                                    grad_values, n, top_k, rows, dim);
+  };
+  // Short chunks where the warps of long ones would not fill the chip, us a call with its sort, long / short: 65536 events 210 / 200 and
+  // 155 / 145 (many and few distinct rows), 131072 260 / 265 and 180 / 180, 524288 375 / 380 and 240 / 255.
+  const bool few = n < 100000;
+  if (dim <= 512) few ? launch(weighted_value_bwd_sorted_kernel<4, 8>, 8) : launch(weighted_value_bwd_sorted_kernel<4, 32>, 32);
+  else few ? launch(weighted_value_bwd_sorted_kernel<8, 8>, 8) : launch(weighted_value_bwd_sorted_kernel<8, 32>, 32);
+  HL_LAUNCH_CHECK("weighted_value_bwd_sorted_kernel");
+  count_launch(ctx);
+  return HL_OK;
+}
+}  // namespace hl
+
+extern "C" {
+
 int hl_memory_weighted_value_backward(hl_ctx* ctx, const int64_t* indices, const float* weights, const float* values,
                                       const float* grad_out, float* grad_weights, float* grad_values, int tokens,
                                       int top_k, int rows, int dim) {
@@ -1514,48 +1573,14 @@ int hl_memory_weighted_value_backward(hl_ctx* ctx, const int64_t* indices, const
   if (rc != HL_OK) return rc;
   HL_REQUIRE(rows > 0 && dim % 4 == 0, "hl_memory_weighted_value_backward: non-zero rows/row_dim, row_dim a multiple of 4");
   const long long n = (long long)tokens * top_k;
-  if (grad_values && n >= 32768 && n < (1ll << 31) - 64 && dim <= 1024 && rows < (1 << 30)) {
-    // row order (see weighted_value_bwd_sorted_kernel).  Scratch: keys and events in and out, and the sort's own space.
-    int end_bit = 1;
-    while ((1ll << end_bit) <= rows) ++end_bit;  // the sentinel key `rows` must sort last
-    const int n_tiles = (int)ceil_div_ll(n, RS_TILE);
-    const size_t arr = ((size_t)n * sizeof(int) + 255) & ~size_t(255);
-    const size_t hist_bytes = ((size_t)RS_DIGITS * (n_tiles + 1) * sizeof(int) + 255) & ~size_t(255);  // rows, then totals
-    rc = ensure_workspace(ctx, 4 * arr + hist_bytes);
+  if (grad_values && value_events_ordered(n, rows, dim)) {
+    rc = ensure_workspace(ctx, value_sort_bytes(n) + value_order_scratch_bytes(n));
     if (rc != HL_OK) return rc;
     uint8_t* ws = reinterpret_cast<uint8_t*>(ctx->workspace);
-    int *keys_a = reinterpret_cast<int*>(ws), *ev_a = reinterpret_cast<int*>(ws + arr);
-    int *keys_b = reinterpret_cast<int*>(ws + 2 * arr), *ev_b = reinterpret_cast<int*>(ws + 3 * arr);
-    int* hist = reinterpret_cast<int*>(ws + 4 * arr);
-    pdl(value_event_keys_kernel, (unsigned)ceil_div_ll(n, 256), 256, 0, ctx->stream)(indices, n, rows, keys_a, ev_a, grad_weights,
-                                                                                     ctx->status_dev);
-    HL_LAUNCH_CHECK("value_event_keys_kernel");
-    int passes = 0;
-    for (int shift = 0; shift < end_bit; shift += RS_BITS, ++passes) {
-      pdl(radix_hist_kernel, n_tiles, RS_THREADS, 0, ctx->stream)(keys_a, n, shift, hist, n_tiles);
-      HL_LAUNCH_CHECK("radix_hist_kernel");
-      int* totals = hist + (size_t)RS_DIGITS * n_tiles;
-      pdl(radix_scan_rows_kernel, RS_DIGITS, RS_THREADS, 0, ctx->stream)(hist, n_tiles, totals);
-      HL_LAUNCH_CHECK("radix_scan_rows_kernel");
-      pdl(radix_scatter_kernel, n_tiles, RS_THREADS, 0, ctx->stream)(keys_a, ev_a, keys_b, ev_b, n, shift, hist, totals, n_tiles);
-      HL_LAUNCH_CHECK("radix_scatter_kernel");
-      std::swap(keys_a, keys_b);
-      std::swap(ev_a, ev_b);
-    }
-    const int *keys = keys_a, *ev = ev_a;  // the last pass's output
-    count_launch(ctx, 3 * passes);
-    auto launch = [&](auto kern, int chunk) {
-      pdl(kern, (unsigned)ceil_div_ll(ceil_div_ll(n, chunk), 4), 128, 0, ctx->stream)(keys, ev, weights, values, grad_out, grad_weights, grad_values,
-                                                                                      n, top_k, rows, dim);
-    };
-    // Short chunks where the warps of long ones would not fill the chip, us a call with its sort, long / short: 65536 events 210 / 200 and
-    // 155 / 145 (many and few distinct rows), 131072 260 / 265 and 180 / 180, 524288 375 / 380 and 240 / 255.
-    const bool few = n < 100000;
-    if (dim <= 512) few ? launch(weighted_value_bwd_sorted_kernel<4, 8>, 8) : launch(weighted_value_bwd_sorted_kernel<4, 32>, 32);
-    else few ? launch(weighted_value_bwd_sorted_kernel<8, 8>, 8) : launch(weighted_value_bwd_sorted_kernel<8, 32>, 32);
-    HL_LAUNCH_CHECK("weighted_value_bwd_sorted_kernel");
-    count_launch(ctx, 2);
-    return HL_OK;
+    int *keys = reinterpret_cast<int*>(ws), *events = reinterpret_cast<int*>(ws + value_sort_bytes(n) / 2);
+    rc = value_sort(ctx, indices, n, rows, keys, events, ws + value_sort_bytes(n), grad_weights);
+    if (rc != HL_OK) return rc;
+    return weighted_value_backward_ordered(ctx, keys, events, weights, values, grad_out, grad_weights, grad_values, n, top_k, rows, dim);
   }
   if (dim <= 1024)
     pdl(weighted_value_bwd_rows_kernel, tokens, 32 * ceil_div(dim, 128), 0, ctx->stream)(indices, weights, values, grad_out, grad_weights,

@@ -48,6 +48,7 @@ struct LayerOffsets {
 struct MemoryActs {
   float *query = nullptr, *weights = nullptr, *weighted = nullptr, *gpre = nullptr, *gate = nullptr, *mv = nullptr;
   int64_t* idx = nullptr;
+  int *sorted_rows = nullptr, *sorted_events = nullptr;  // the selections in row order (value_sort); null: the backward pass sorts them
   __nv_bfloat16* mv_b = nullptr;  // amp route: [N, 2*value_dim] = [hi | lo] pieces of mv
   // amp route: the three projection weights as bf16 pieces along the contraction (hl_split_bf16_f32),
   // rebuilt from the f32 parameters at the start of every forward pass
@@ -131,6 +132,12 @@ struct hl_decoder {
   cudaStream_t side_stream = nullptr;
   cudaEvent_t fork_event = nullptr, join_event = nullptr;
   cudaEvent_t zero_event = nullptr;  // the scattered gradients have been zeroed there
+  cudaEvent_t sort_event = nullptr;  // the selections that the forward pass has left so far are in row order
+  void* sort_scratch = nullptr;      // of those sorts, one at a time
+  bool sorted = false;               // this pass sorts them there
+  // a scratch arena for what runs there, in place of the context's
+  void* side_arena = nullptr;
+  size_t side_arena_bytes = 0;
   bool zeroed = false;
   // ... or, where the products fill the chip, collected for `group_layers` layers (0: not) and run by one launch.
   int group_layers = 0;
@@ -330,6 +337,39 @@ T* carve(uint8_t*& cursor, size_t count) {
   return p;
 }
 
+hl_gemm_desc product(int M, int N, int K, int al, long long lda, int bl, long long ldb, int a_k_period, int b_k_period) {
+  hl_gemm_desc d{};
+  d.m = M; d.n = N; d.k = K;
+  d.a_layout = al; d.b_layout = bl;
+  d.lda = lda; d.ldb = ldb; d.ldc = N;
+  d.out_dtype = HL_F32;
+  d.a_k_period = a_k_period; d.b_k_period = b_k_period;
+  return d;
+}
+// The weight gradients of a memory block's three projections (amp route).
+hl_gemm_desc out_gradient(const hl_decoder* m) {
+  return product(m->cfg.d_model, m->mem.value_dim, 3 * m->N, HL_MN_MAJOR, m->cfg.d_model, HL_MN_MAJOR, m->mem.value_dim, 2 * m->N, 0);
+}
+hl_gemm_desc in_gradient(const hl_decoder* m, int width) {
+  return product(width, m->cfg.d_model, 3 * m->N, HL_MN_MAJOR, width, HL_MN_MAJOR, m->cfg.d_model, 0, m->N);
+}
+KeyGradient key_gradient(const hl_decoder* m) {
+  KeyGradient k{};
+  k.ld_query = m->mem.key_dim;
+  k.tokens = m->N; k.top_k = m->mem.top_k; k.side = m->side; k.half = m->mem.key_dim / 2; k.slots = m->mem.slots;
+  return k;
+}
+// Scratch for what a memory block's backward pass puts on the side stream.
+size_t memory_side_bytes(const hl_decoder* m) {
+  size_t most = 0, bytes = 0;
+  if (m->cfg.precision == HL_PRECISION_AMP_BF16)
+    for (const hl_gemm_desc& d : {out_gradient(m), in_gradient(m, m->mem.value_dim), in_gradient(m, m->mem.key_dim)})
+      if (gemm_bf16_scratch(m->ctx, &d, &bytes)) most = std::max(most, bytes);
+  const KeyGradient k = key_gradient(m);
+  if (const int shares = key_gradient_shares(m->ctx, k)) most = std::max(most, key_gradient_bytes(k, shares));
+  return most;
+}
+
 // Buffers of the memory feed-forward blocks; appended to either route's arena.
 void plan_memory_buffers(hl_decoder* m, uint8_t*& cur) {
   m->tok_flags = carve<unsigned char>(cur, (size_t)m->cfg.vocab);
@@ -352,7 +392,15 @@ void plan_memory_buffers(hl_decoder* m, uint8_t*& cur) {
     a.wq3 = carve<__nv_bfloat16>(cur, kd * 3 * d);
     a.wg3 = carve<__nv_bfloat16>(cur, vd * 3 * d);
     a.wout3 = carve<__nv_bfloat16>(cur, d * 3 * vd);
+    a.sorted_rows = a.sorted_events = nullptr;
+    if (!m->lean && value_events_ordered((long long)(N * k), m->mem.slots, (int)vd)) {
+      a.sorted_rows = reinterpret_cast<int*>(carve<uint8_t>(cur, value_sort_bytes((long long)(N * k))));
+      a.sorted_events = a.sorted_rows + value_sort_bytes((long long)(N * k)) / 2 / sizeof(int);
+    }
   }
+  m->sort_scratch = m->lean ? nullptr : carve<uint8_t>(cur, value_order_scratch_bytes((long long)(N * k)));
+  m->side_arena_bytes = m->lean ? 0 : memory_side_bytes(m);
+  m->side_arena = m->side_arena_bytes ? carve<uint8_t>(cur, m->side_arena_bytes) : nullptr;
   m->m_ls = carve<float>(cur, N * m->side);
   m->m_rs = carve<float>(cur, N * m->side);
   m->m_scores = carve<float>(cur, N * k);
@@ -595,6 +643,17 @@ struct SideStream {
   ~SideStream() { m->ctx->stream = main; }
 };
 
+// The same with a scratch arena of its own.
+struct SideWork : SideStream {
+  explicit SideWork(hl_decoder* model) : SideStream(model) { swap(); }
+  ~SideWork() { swap(); }
+ private:
+  void swap() {
+    std::swap(m->ctx->workspace, m->side_arena);
+    std::swap(m->ctx->workspace_bytes, m->side_arena_bytes);
+  }
+};
+
 int join_side(hl_decoder* m) {
   if (!m->forked) return HL_OK;
   m->forked = false;
@@ -684,6 +743,12 @@ int memory_core_forward(hl_decoder* m, int l, bool one_token = false) {
   ProfileScope prof(ctx, HL_PROF_OTHER, (double)N * k * (double)(kd + vd) * 4.0 + 2.0 * (double)N * side * 4.0);
   HL_TRY(hl_product_key_side_scores_f32(ctx, a.query, kd, P + m->off_kl, P + m->off_kr, m->m_ls, m->m_rs, N, side, kd));
   HL_TRY(product_key_topk_impl(ctx, m->m_ls, m->m_rs, idx, N, side, k, beam, one_token ? a.idx : nullptr, m->decode_state));
+  if (m->sorted && a.sorted_rows) {  // for the backward pass, beside what follows
+    SideStream beside(m);
+    HL_TRY(beside.rc);
+    HL_TRY(value_sort(ctx, idx, (long long)N * k, m->mem.slots, a.sorted_rows, a.sorted_events, m->sort_scratch, nullptr));
+    HL_CUDA(cudaEventRecord(m->sort_event, ctx->stream));
+  }
   HL_TRY(hl_memory_selected_scores_forward(ctx, idx, a.query, kd, P + m->off_kl, P + m->off_kr, m->m_scores, N, k, side, kd,
                                            m->mem.slots));
   HL_TRY(hl_softmax_rows_f32(ctx, m->m_scores, a.weights, N, k));
@@ -698,11 +763,38 @@ int memory_core_backward(hl_decoder* m, int l, const float* dweighted) {
   float* G = m->grads;
   const int N = m->N, kd = m->mem.key_dim, vd = m->mem.value_dim, k = m->mem.top_k, side = m->side;
   ProfileScope prof(ctx, HL_PROF_OTHER, (double)N * k * (double)(kd + 3 * vd) * 4.0);
-  HL_TRY(hl_memory_weighted_value_backward(ctx, a.idx, a.weights, P + m->off_val, dweighted, m->m_dw, G + m->off_val, N, k,
-                                           m->mem.slots, vd));
+  if (m->sorted && a.sorted_rows) {
+    HL_CUDA(cudaStreamWaitEvent(ctx->stream, m->sort_event, 0));
+    HL_TRY(weighted_value_backward_ordered(ctx, a.sorted_rows, a.sorted_events, a.weights, P + m->off_val, dweighted, m->m_dw, G + m->off_val,
+                                           (long long)N * k, k, m->mem.slots, vd));
+  } else {
+    HL_TRY(hl_memory_weighted_value_backward(ctx, a.idx, a.weights, P + m->off_val, dweighted, m->m_dw, G + m->off_val, N, k,
+                                             m->mem.slots, vd));
+  }
   HL_TRY(hl_softmax_rows_backward_f32(ctx, a.weights, m->m_dw, m->m_dscores, N, k));
-  return hl_memory_selected_scores_backward(ctx, a.idx, a.query, kd, P + m->off_kl, P + m->off_kr, m->m_dscores, m->m_dq, kd,
-                                            G + m->off_kl, G + m->off_kr, N, k, side, kd, m->mem.slots);
+  auto scores_backward = [&](float* dq, float* dl, float* dr) {
+    return hl_memory_selected_scores_backward(ctx, a.idx, a.query, kd, P + m->off_kl, P + m->off_kr, m->m_dscores, dq, kd, dl, dr, N, k, side, kd,
+                                              m->mem.slots);
+  };
+  const KeyGradient keys = key_gradient(m);
+  const int shares = beside(m) ? key_gradient_shares(ctx, keys) : 0;
+  if (shares == 0 || key_gradient_bytes(keys, shares) > m->side_arena_bytes) return scores_backward(m->m_dq, G + m->off_kl, G + m->off_kr);
+  {  // nothing in the backward pass waits for the tables' gradients
+    SideWork side_work(m);
+    HL_TRY(side_work.rc);
+    HL_TRY(scores_backward(nullptr, G + m->off_kl, G + m->off_kr));
+  }
+  return scores_backward(m->m_dq, nullptr, nullptr);
+}
+
+// A product on the side stream where its scratch is there, else where everything is.
+int run_beside(hl_decoder* m, const hl_gemm_desc& d, const __nv_bfloat16* a, const __nv_bfloat16* b, float* c) {
+  size_t bytes = 0;
+  if (!beside(m) || !gemm_bf16_scratch(m->ctx, &d, &bytes) || bytes > m->side_arena_bytes)
+    return gemm_bf16_ctx(m->ctx, &d, a, b, c, nullptr, nullptr, nullptr);
+  SideWork side(m);
+  HL_TRY(side.rc);
+  return gemm_bf16_ctx(m->ctx, &d, a, b, c, nullptr, nullptr, nullptr);
 }
 
 // Final layer norm and head of one row of the residual stream: the logits in row 0 of m->logits.
@@ -1121,9 +1213,17 @@ int backward(hl_decoder* m) {
     if (nccl_active(ctx) || done == m->arena) HL_TRY(fold_batch_flush(ctx, fb));
     return flush_buckets(m, done);
   };
-  // lm_head
-  HL_TRY(weight_gradient(m, m->dlogits, V, m->z, d, G + m->off_head_w, G + m->off_head_b));
+  // lm_head.  Its bias gradient, where it is a pass of its own over the logits' gradient, runs beside the two products.
+  const hl_gemm_desc head_gradient = product(V, d, N, HL_MN_MAJOR, V, HL_MN_MAJOR, d, 0, 0);
+  const bool bias_apart = beside(m) && !grouping(m) && !gemm_bf16_small_applies(ctx, &head_gradient);
+  if (bias_apart) {
+    SideStream side(m);
+    HL_TRY(side.rc);
+    HL_TRY(bias_grad_impl(ctx, m->dlogits, HL_BF16, G + m->off_head_b, N, V, fb));
+  }
+  HL_TRY(weight_gradient(m, m->dlogits, V, m->z, d, G + m->off_head_w, bias_apart ? nullptr : G + m->off_head_b));
   HL_TRY(g.run(N, d, V, m->dlogits, V, HL_K_MAJOR, W + m->off_head_w, d, HL_MN_MAJOR, m->dtmp, d, HL_F32));
+  if (bias_apart) HL_TRY(join_side(m));  // its partial sums are folded with the others'
   float* dx = m->dx0;
   float* dx_next = m->dx1;
   // every layer-norm backward also returns the column sums of the gradient it writes: the bias
@@ -1147,13 +1247,13 @@ int backward(hl_decoder* m) {
       // that read c are one product over both: hi*lo and lo*hi of the two, 2^-8 of the rest, come first and hi*hi after them, since the
       // tensor core's additions truncate what it has added up so far (error against f64 of 16384 x 512 over 2 x 512: 4.5e-6, of it 4.4e-6
       // the dropped lo*lo; a projection after the other with hi*hi first 6.2e-6, two products added up 5.1e-6).
+      HL_TRY(join_side(m));  // the block's buffers are those of the one above
       const int ROWS = HL_SPLIT_STACK_ROWS;
       const float* dy = dx;  // dL/dy of this block, f32
       // out_proj: dW = dy^T mv, dmv = dy W
       HL_TRY(split_pieces(ctx, dy, N, d, pieces_stacked(m->p_dx_rows, N, d, 2, 0, 1), pieces_beside(m->p_dx_side, 2 * d, d, 2, 0, 1)));
       HL_TRY(hl_split_bf16_f32(ctx, ma.mv, m->p_mv_rows, N, vd, HL_SPLIT_HI_HI_LO | ROWS));
-      HL_TRY(g.run(d, vd, 3 * N, m->p_dx_rows, d, HL_MN_MAJOR, m->p_mv_rows, vd, HL_MN_MAJOR, G + o.wout_m, vd, HL_F32,
-                   HL_EPI_NONE, nullptr, nullptr, 0, nullptr, 0, 2 * N));
+      HL_TRY(run_beside(m, out_gradient(m), m->p_dx_rows, m->p_mv_rows, G + o.wout_m));
       HL_TRY(hl_split_bf16_f32(ctx, P + o.wout_m, m->p_wout_rows, d, vd, HL_SPLIT_HI_HI_LO | ROWS));
       HL_TRY(g.run(N, vd, 3 * d, m->p_dx_side, 2 * d, HL_K_MAJOR, m->p_wout_rows, vd, HL_MN_MAJOR, m->m_dmv, vd, HL_F32,
                    HL_EPI_NONE, nullptr, nullptr, 0, nullptr, 0, 2 * d));
@@ -1161,15 +1261,13 @@ int backward(hl_decoder* m) {
       const int both = vd + kd;
       HL_TRY(memory_gate_backward(ctx, m->m_dmv, ma.gate, ma.weighted, ma.gpre, m->m_dweighted, m->m_dgpre, N, vd,
                                   pieces_stacked(m->p_dg_rows, N, vd, 3, 0, 1, 2), PieceDest{m->p_dc_side, 2 * both, both, 2, {0, 1}}));
-      HL_TRY(g.run(vd, d, 3 * N, m->p_dg_rows, vd, HL_MN_MAJOR, a.c, d, HL_MN_MAJOR, G + o.wg_m, d, HL_F32, HL_EPI_NONE,
-                   nullptr, nullptr, 0, nullptr, 0, 0, N));
+      HL_TRY(run_beside(m, in_gradient(m, vd), m->p_dg_rows, a.c, G + o.wg_m));
       HL_TRY(bias_grad_impl(ctx, m->m_dgpre, HL_F32, G + o.bg_m, N, vd, fb));
       HL_TRY(memory_core_backward(m, l, m->m_dweighted));
       // query_proj: dW = dq^T c
       HL_TRY(split_pieces(ctx, m->m_dq, N, kd, pieces_stacked(m->p_dq_rows, N, kd, 3, 0, 1, 2),
                           PieceDest{m->p_dc_side + vd, 2 * both, both, 2, {0, 1}}));
-      HL_TRY(g.run(kd, d, 3 * N, m->p_dq_rows, kd, HL_MN_MAJOR, a.c, d, HL_MN_MAJOR, G + o.wq_m, d, HL_F32, HL_EPI_NONE,
-                   nullptr, nullptr, 0, nullptr, 0, 0, N));
+      HL_TRY(run_beside(m, in_gradient(m, kd), m->p_dq_rows, a.c, G + o.wq_m));
       HL_TRY(bias_grad_impl(ctx, m->m_dq, HL_F32, G + o.bq_m, N, kd, fb));
       // dc = dgpre Wg + dq Wq
       HL_TRY(split_pieces(ctx, P + o.wg_m, vd, d, PieceDest{m->p_wc_rows, d, (long long)both * d, 3, {1, 0, 0}}));
@@ -1357,6 +1455,7 @@ int backward_f32(hl_decoder* m) {
       HL_TRY(hl_binary_f32(ctx, HL_MUL, m->m_dmv, ma.weighted, m->m_dgate, nv));
       HL_TRY(hl_gelu_backward(ctx, ma.gpre, m->m_dgate, m->m_dgpre, HL_F32, nv));
       HL_TRY(linear_backward_f32(m, a.c, P + o.wg_m, m->m_dgpre, m->d_c, G + o.wg_m, G + o.bg_m, N, d, vd));
+      HL_TRY(join_side(m));  // its buffers are those of the block above
       HL_TRY(memory_core_backward(m, l, m->m_dweighted));
       // the query path's input gradient is added to the gate path's
       HL_TRY(linear_backward_f32(m, a.c, P + o.wq_m, m->m_dq, m->d_c, G + o.wq_m, G + o.bq_m, N, d, kd, F64_ACCUMULATE));
@@ -1808,6 +1907,7 @@ static int decoder_create_impl(hl_ctx* ctx, const hl_decoder_config* cfg, const 
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&m->fork_event, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&m->join_event, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&m->zero_event, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&m->sort_event, cudaEventDisableTiming);
     if (e != cudaSuccess) return cleanup(fail_cuda(e, "cudaStreamCreate(side)"));
   }
   e = cudaEventCreateWithFlags(&m->comm_done, cudaEventDisableTiming);
@@ -1832,6 +1932,7 @@ void hl_decoder_destroy(hl_decoder* m) {
   if (m->side_stream) cudaStreamDestroy(m->side_stream);
   if (m->fork_event) cudaEventDestroy(m->fork_event);
   if (m->zero_event) cudaEventDestroy(m->zero_event);
+  if (m->sort_event) cudaEventDestroy(m->sort_event);
   if (m->join_event) cudaEventDestroy(m->join_event);
   for (cudaEvent_t ev : {m->rows_known, m->tok_count_ready, m->val_count_ready}) if (ev) cudaEventDestroy(ev);
   for (auto ev : m->wait_begin) cudaEventDestroy(ev);
@@ -1944,6 +2045,11 @@ int hl_decoder_forward_backward(hl_decoder* m, const int64_t* tokens_dev, const 
     HL_CUDA(cudaMemcpyAsync(m->targets, targets_dev, sizeof(int64_t) * m->N, cudaMemcpyDeviceToDevice, m->ctx->stream));
   m->cached = 0;  // the pass overwrites the cached rows from its first kernel on, whether or not it gets to its end
   HL_TRY(run_graphed(m, GRAPH_STEP, [m]() -> int {
+    struct Sorting {  // a backward pass follows
+      hl_decoder* m;
+      ~Sorting() { m->sorted = false; }
+    } sorting{m};
+    m->sorted = beside(m);
     HL_TRY(zero_tables_beside(m));
     HL_TRY(prepare_token_rows(m));  // data parallel: the union of the ranks' token rows forms while forward runs
     if (m->cfg.precision == HL_PRECISION_AMP_BF16) {

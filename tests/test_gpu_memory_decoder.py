@@ -300,3 +300,32 @@ def test_the_input_gradient_of_a_memory_blocks_projections_keeps_f32_accuracy(ke
     assert np.linalg.norm(dy) < 1e-3 * np.linalg.norm(want)
     assert np.linalg.norm(got - want) <= 1.1 * np.linalg.norm(norm(left_out))
     model.close()
+
+
+@pytest.mark.parametrize("precision,limit", [(0, 1e-6), (1, 4e-3)])
+def test_what_runs_beside_the_backward_pass_equals_everything_in_one_stream(precision, limit):
+    """Selections sorted beside the forward pass; weight gradients of the memory projections, half-key gradients and the head's bias
+    gradient beside the backward one, with two memory blocks that share their buffers.  Per-kernel timing keeps all of it in
+    one stream.  Passes that differ only in the order of their atomics: f32 1e-6 of a tensor's scale, bf16 the 4e-3 of whole batches
+    against their parts (an f32 sum in another order flips single bf16 roundings).  The first pass runs plainly, the others as a graph."""
+    from heirloom_b200 import cuda, nn
+    c = ctx()
+    kw, mem = dict(KW, vocab=8200), dict(MEM, top_k=16)
+    model = nn.DecoderLm(c, nn.DecoderConfig(batch=17, precision=nn.PRECISION_AMP_BF16 if precision else nn.PRECISION_F32, **kw), nn.MemoryConfig(**mem))
+    model.load_state_dict(ho.init_memory_parameters(ho.DecoderConfig(**kw), ho.MemoryConfig(**mem), 3))
+    tok = torch.tensor(ho.zipf_tokens(np.random.default_rng(5), kw["vocab"], (17, 129)), device="cuda")
+    x, y = tok[:, :-1].contiguous(), tok[:, 1:].contiguous()
+
+    def gradients():
+        model.forward_backward(x, y)
+        return {n: model.grad(n).astype(np.float64) for n in model.parameter_names() if not n.endswith("k_proj.bias")}
+    cuda.check(c.lib.hl_profile_enable(c.handle, 1))
+    try:
+        want = gradients()
+    finally:
+        cuda.check(c.lib.hl_profile_enable(c.handle, 0))
+    for _ in range(3):
+        for name, g in gradients().items():
+            scale = np.abs(want[name]).max()
+            assert np.abs(g - want[name]).max() <= limit * scale + 1e-12, (name, np.abs(g - want[name]).max() / scale)
+    model.close()
