@@ -235,36 +235,42 @@ fold_partials_kernel(const float* __restrict__ partial, int blocks, int total, f
   }
 }
 
-// The same fold for up to FoldBatch::kMaxJobs reductions in one launch: blockIdx.y picks the job.
+// The same fold for up to FoldBatch::kMaxJobs reductions in one launch, whose blocks follow one another.
 struct FoldJobs {
   FoldJob job[FoldBatch::kMaxJobs];
+  int first[FoldBatch::kMaxJobs + 1];  // block of a job's first 32 columns; behind the last job the number of blocks
 };
-__global__ void __launch_bounds__(FOLD_WARPS * 32)
-fold_batch_kernel(const FoldJobs jobs) {
+// Small CTAs, all resident at once: 32 warps for 32 columns came in two to five waves (20000 columns of 296 rows 10 -> 9 us, 56000 columns
+// of a training step's head and blocks 41 -> 11).
+constexpr int FB_WARPS = 8, FB_LOADS = 16;
+__global__ void __launch_bounds__(FB_WARPS * 32)
+fold_batch_kernel(const __grid_constant__ FoldJobs jobs) {
   pdl_begin();
-  __shared__ double acc[FOLD_WARPS][33];
-  const FoldJob& j = jobs.job[blockIdx.y];
-  if ((int)blockIdx.x * 32 >= j.total) return;
+  __shared__ double acc[FB_WARPS][33];
+  int which = 0;
+  while ((int)blockIdx.x >= jobs.first[which + 1]) ++which;
+  const FoldJob& j = jobs.job[which];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + lane;
+  const int c0 = ((int)blockIdx.x - jobs.first[which]) * 32, c = c0 + lane, total = j.total, blocks = j.blocks;
+  const float* partial = j.partial + c;
   double s = 0.0;
-  if (c < j.total) {
-    for (int b0 = warp; b0 < j.blocks; b0 += FOLD_WARPS * 8) {
-      float v[8];
+  if (c < total) {
+    for (int b0 = warp; b0 < blocks; b0 += FB_WARPS * FB_LOADS) {
+      float v[FB_LOADS];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int b = b0 + u * FOLD_WARPS;
-        v[u] = b < j.blocks ? j.partial[(size_t)b * j.total + c] : 0.f;
+      for (int u = 0; u < FB_LOADS; ++u) {
+        const int b = b0 + u * FB_WARPS;
+        v[u] = b < blocks ? partial[(size_t)b * total] : 0.f;
       }
 #pragma unroll
-      for (int u = 0; u < 8; ++u) s += (double)v[u];
+      for (int u = 0; u < FB_LOADS; ++u) s += (double)v[u];
     }
   }
   acc[warp][lane] = s;
   __syncthreads();
-  if (warp == 0 && c < j.total) {
-#pragma unroll 8
-    for (int w = 1; w < FOLD_WARPS; ++w) s += acc[w][lane];
+  if (warp == 0 && c < total) {
+#pragma unroll
+    for (int w = 1; w < FB_WARPS; ++w) s += acc[w][lane];
     float* dst = c < j.features ? j.o0 : (c < 2 * j.features ? j.o1 : j.o2);
     if (dst) dst[c % j.features] = (float)s;
   }
@@ -330,12 +336,14 @@ void fold_batch_add(FoldBatch* batch, const float* partial, int blocks, int tota
 int fold_batch_flush(hl_ctx* ctx, FoldBatch* batch) {
   if (!batch || batch->n == 0) return HL_OK;
   FoldJobs jobs{};
-  int widest = 0;
+  int blocks = 0;
   for (int i = 0; i < batch->n; ++i) {
     jobs.job[i] = batch->jobs[i];
-    widest = std::max(widest, batch->jobs[i].total);
+    jobs.first[i] = blocks;
+    blocks += ceil_div(batch->jobs[i].total, 32);
   }
-  pdl(fold_batch_kernel, dim3(ceil_div(widest, 32), batch->n), FOLD_WARPS * 32, 0, ctx->stream)(jobs);
+  jobs.first[batch->n] = blocks;
+  pdl(fold_batch_kernel, blocks, FB_WARPS * 32, 0, ctx->stream)(jobs);
   HL_LAUNCH_CHECK("fold_batch_kernel");
   count_launch(ctx);
   batch->n = 0;
