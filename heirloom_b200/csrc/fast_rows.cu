@@ -130,17 +130,51 @@ ln_bwd_bf16_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
   if (active) load8_f32(gamma + c, g);
   const float inv_f = 1.0f / (float)features;
   int parity = 0;
+  // A row's operands are requested while the row before it is worked on, as far as registers allow it: with three or four warps a row the
+  // group's 24 warps keep more on their way without (16384 x 768 33.6 us, 36.7 with it; x 512 26.4 -> 22.2, 4096 x 512 8.4 -> 6.3).
+  constexpr bool AHEAD = WPR <= 2;
+  uint4 next_x = make_uint4(0u, 0u, 0u, 0u);
+  float4 next_dy[2] = {}, next_res[2] = {};
+  float next_mean = 0.f, next_rstd = 0.f;
+  auto fetch = [&](int row) {
+    if (row >= r1) return;
+    next_mean = mean_in[row];
+    next_rstd = rstd_in[row];
+    if (!active) return;
+    const size_t base = (size_t)row * features + c;
+    next_x = *reinterpret_cast<const uint4*>(x + base);
+    next_dy[0] = *reinterpret_cast<const float4*>(dy + base);
+    next_dy[1] = *reinterpret_cast<const float4*>(dy + base + 4);
+    if (residual) {
+      next_res[0] = *reinterpret_cast<const float4*>(residual + base);
+      next_res[1] = *reinterpret_cast<const float4*>(residual + base + 4);
+    }
+  };
+  if constexpr (AHEAD) fetch(r0 + group);
   for (int row = r0 + group; row < r1; row += GROUPS, parity ^= 1) {
     const size_t base = (size_t)row * features + c;
-    float xh[8], d[8], o[8];
+    float xh[8], d[8], o[8], mean, rstd;
+    if constexpr (AHEAD) {
+      unpack8_bf16(next_x, xh);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) { xh[e] = 0.f; d[e] = 0.f; o[e] = 0.f; }
-    if (active) {  // every global read of the row is issued before anything is consumed
-      load8_bf16(x + base, xh);
-      load8_f32(dy + base, d);
-      if (residual) load8_f32(residual + base, o);
+      for (int e = 0; e < 8; ++e) {
+        d[e] = e < 4 ? (&next_dy[0].x)[e] : (&next_dy[1].x)[e - 4];
+        o[e] = e < 4 ? (&next_res[0].x)[e] : (&next_res[1].x)[e - 4];
+      }
+      mean = next_mean;
+      rstd = next_rstd;
+      fetch(row + GROUPS);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) { xh[e] = 0.f; d[e] = 0.f; o[e] = 0.f; }
+      if (active) {  // every global read of the row is issued before anything is consumed
+        load8_bf16(x + base, xh);
+        load8_f32(dy + base, d);
+        if (residual) load8_f32(residual + base, o);
+      }
+      mean = mean_in[row];
+      rstd = rstd_in[row];
     }
-    const float mean = mean_in[row], rstd = rstd_in[row];
     float s1 = 0.f, s2 = 0.f;
     if (active) {
 #pragma unroll
