@@ -261,6 +261,15 @@ int key_gradient_run(hl_ctx* ctx, const KeyGradient& k, int shares, void* scratc
 int product_key_topk_impl(hl_ctx* ctx, const float* left_scores, const float* right_scores, int64_t* out, int tokens, int side, int top_k,
                           int beam, int64_t* kept, const long long* kept_row);
 
+// Side scores and hl_product_key_topk_from_side_scores in one, with the selections of those two, for queries with rows of key_dim: the scores
+// that can be selected are formed exactly, the others on the tensor cores.  `pieces` (product_key_pieces_bytes) come from the tables by
+// product_key_pieces; query_pieces: tokens * 2 * key_dim; the approximate scores: tokens * side each; all on 16 bytes.
+bool product_key_lookup_takes(int side, int key_dim, int beam);
+size_t product_key_pieces_bytes(int side, int key_dim);
+int product_key_pieces(hl_ctx* ctx, const float* left_keys, const float* right_keys, int side, int key_dim, void* pieces);
+int product_key_lookup(hl_ctx* ctx, const float* query, const float* left_keys, const float* right_keys, const void* pieces,
+                       __nv_bfloat16* query_pieces, float* left_approx, float* right_approx, int64_t* out, int tokens, int side, int key_dim,
+                       int top_k, int beam);
 // hl_memory_weighted_value_backward in two: the (token, slot) events sorted by row, which needs the indices alone, and the rest.  `keys`
 // and `events` lie in value_sort_bytes, half each; rows that do not exist report themselves and zero their grad_weights (may be null).
 bool value_events_ordered(long long n, int rows, int dim);

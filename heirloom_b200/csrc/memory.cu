@@ -266,22 +266,33 @@ __device__ __forceinline__ unsigned long long radix_beam(const unsigned (&key)[P
   sort_lanes(v);
   return v[0];
 }
+// The 32nd largest of the lanes' two largest keys, which at least 32 keys reach where there are as many.
 template <int PER_LANE>
-__device__ __forceinline__ unsigned long long beam_of_side(const float* s, int side, int beam, TopkScratch& sc) {
-  const int lane = threadIdx.x & 31;
-  const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
-  float score[PER_LANE];
-#pragma unroll
-  for (int i = 0; i < PER_LANE; ++i) score[i] = s[min(i * 32 + lane, side - 1)];
-  unsigned key[PER_LANE], top[2] = {0u, 0u};
+__device__ __forceinline__ unsigned key_bound(const unsigned (&key)[PER_LANE]) {
+  unsigned top[2] = {0u, 0u};
 #pragma unroll
   for (int i = 0; i < PER_LANE; ++i) {
-    key[i] = i * 32 + lane < side ? okey(score[i]) : 0u;
     top[1] = max(top[1], min(top[0], key[i]));
     top[0] = max(top[0], key[i]);
   }
   sort_lanes(top);
-  const unsigned bound = max(1u, __reduce_min_sync(full, upper_half(top[0], top[1])));
+  return max(1u, __reduce_min_sync(0xffffffffu, upper_half(top[0], top[1])));
+}
+template <int PER_LANE>
+__device__ __forceinline__ void load_scores(const float* s, int side, float (&score)[PER_LANE]) {
+#pragma unroll
+  for (int i = 0; i < PER_LANE; ++i) score[i] = s[min(i * 32 + (int)(threadIdx.x & 31), side - 1)];
+}
+template <int PER_LANE>
+__device__ __forceinline__ unsigned long long beam_of_scores(const float (&score)[PER_LANE], int side, int beam, TopkScratch& sc) {
+  const int lane = threadIdx.x & 31;
+  const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
+  unsigned key[PER_LANE];
+#pragma unroll
+  for (int i = 0; i < PER_LANE; ++i) {
+    key[i] = i * 32 + lane < side ? okey(score[i]) : 0u;
+  }
+  const unsigned bound = key_bound(key);
   int count = 0;
 #pragma unroll
   for (int i = 0; i < PER_LANE; ++i) {
@@ -365,24 +376,13 @@ __device__ __noinline__ void merge_beams(unsigned l_key, int l_idx, unsigned r_k
   }
 }
 
-template <int PER_LANE>
-__global__ void __launch_bounds__(128)
-product_key_topk_kernel(const float* __restrict__ left, const float* __restrict__ right, int64_t* __restrict__ out,
-                        int tokens, int side, int top_k, int beam, int* __restrict__ status, int64_t* __restrict__ kept,
-                        const long long* __restrict__ kept_row) {
-  pdl_begin();
-  __shared__ TopkScratch scratch[4];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int token = blockIdx.x * 4 + w;
-  if (token >= tokens) return;
+// The top_k of all sums of two sorted beams (okey << 32 | ~index, zero past the beam) into `out`, and `kept` where given.
+__device__ __forceinline__ void pick_pairs(unsigned long long l, unsigned long long r, int64_t* out, int64_t* kept, int side, int top_k, int beam,
+                                           TopkScratch& sc, int* status) {
+  const int lane = threadIdx.x & 31;
   const unsigned full = 0xffffffffu;
-  TopkScratch& sc = scratch[w];
-  const unsigned long long l = beam_of_side<PER_LANE>(left + (size_t)token * side, side, beam, sc);
-  const unsigned long long r = beam_of_side<PER_LANE>(right + (size_t)token * side, side, beam, sc);
   const unsigned l_key = (unsigned)(l >> 32), r_key = (unsigned)(r >> 32);
   const int l_idx = (int)(0xffffffffu - (unsigned)l), r_idx = (int)(0xffffffffu - (unsigned)r);
-  out += (size_t)token * top_k;
-  if (kept) kept += (*kept_row + token) * top_k;
   const float ls = okey_value(l_key), rs = okey_value(r_key);
   bool general = top_k > 32 || __any_sync(full, lane < beam && !(isfinite(ls) && isfinite(rs)));
   if (!general) {
@@ -422,6 +422,255 @@ product_key_topk_kernel(const float* __restrict__ left, const float* __restrict_
     }
   }
   if (general) merge_beams(l_key, l_idx, r_key, r_idx, out, kept, side, top_k, beam, sc, status);
+}
+
+template <int PER_LANE>
+__global__ void __launch_bounds__(128)
+product_key_topk_kernel(const float* __restrict__ left, const float* __restrict__ right, int64_t* __restrict__ out,
+                        int tokens, int side, int top_k, int beam, int* __restrict__ status, int64_t* __restrict__ kept,
+                        const long long* __restrict__ kept_row) {
+  pdl_begin();
+  __shared__ TopkScratch scratch[4];
+  const int w = threadIdx.x >> 5;
+  const int token = blockIdx.x * 4 + w;
+  if (token >= tokens) return;
+  TopkScratch& sc = scratch[w];
+  float score[PER_LANE];
+  load_scores(left + (size_t)token * side, side, score);
+  const unsigned long long l = beam_of_scores(score, side, beam, sc);
+  load_scores(right + (size_t)token * side, side, score);
+  const unsigned long long r = beam_of_scores(score, side, beam, sc);
+  pick_pairs(l, r, out + (size_t)token * top_k, kept ? kept + (*kept_row + token) * top_k : nullptr, side, top_k, beam, sc, status);
+}
+
+// ---- the same from queries: side scores that decide nothing are not formed exactly ----------------------------------------
+// Every score is an f32 sum in a fixed order with separately rounded products (side_scores_kernel), 340 us for 16384 tokens and two
+// tables of 512 x 256, of which the selection wants 32 in 512.  So the tensor core forms all of them first out of bf16 pieces, hi * hi +
+// lo * hi + hi * lo, and only what can be among the beam's is formed again as it has to be: with |approximate - exact| <= E, every
+// key of the beam has an approximate score of at least the beam-th largest minus 2 E.  In terms of S, the norm of the token's half
+// query times the largest norm of a half key (sum |q k| <= S): the f32 sum is off by at most 2 half * 2^-24 S, the dropped pieces by
+// 3 * 2^-18 S, and each of the 3 half / 16 tensor-core steps by 17 terms cut off at 2^-23, together less than (5.1e-7 half + 1.2e-5) S.
+// Where S is not within 1e-30 and 1e37 (or a norm below 1e-18: its squares and the pieces of such values lose bits), or more than 64 keys come into
+// question, all scores of that token and side are formed exactly.  The selections are the same bit by bit.  The kernel takes 226 us of the 276,
+// two thirds of the shared memory's rate: rows are staged there for the lanes that walk them; 5 or 6 blocks an SM: 230 and 234.
+constexpr int LK_PER_LANE = 16;          // sides of up to 512
+constexpr int LK_J = 32, LK_LD = LK_J + 4;  // columns of 32 rows in shared memory at a time, and their pitch
+__device__ __forceinline__ const float* shuffle_pointer(const float* p, int lane) {
+  return reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(p), lane));
+}
+// The exact score of the lane's half query (in shared memory) and half key: rows come in whole segments, a lane walks its own (null: none).
+__device__ __forceinline__ float exact_score(const float* key_row, const float* q, int half, float* buf) {
+  const int lane = threadIdx.x & 31;
+  const float* src[8];
+  float4 r[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    src[i] = shuffle_pointer(key_row, i * 4 + (lane >> 3));
+    if (src[i]) r[i] = __ldg(reinterpret_cast<const float4*>(src[i] += (lane & 7) * 4));
+  }
+  float acc = 0.f;
+#pragma unroll 1
+  for (int j0 = 0; j0 < half; j0 += LK_J) {
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (src[i]) *reinterpret_cast<float4*>(buf + (i * 4 + (lane >> 3)) * LK_LD + (lane & 7) * 4) = r[i];
+    __syncwarp();
+    if (j0 + LK_J < half) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (src[i]) r[i] = __ldg(reinterpret_cast<const float4*>(src[i] + j0 + LK_J));
+    }
+    if (!key_row) continue;
+#pragma unroll
+    for (int j = 0; j < LK_J; j += 4) {
+      const float4 k = *reinterpret_cast<const float4*>(buf + lane * LK_LD + j), x = *reinterpret_cast<const float4*>(q + j0 + j);
+      acc = __fadd_rn(acc, __fmul_rn(x.x, k.x));
+      acc = __fadd_rn(acc, __fmul_rn(x.y, k.y));
+      acc = __fadd_rn(acc, __fmul_rn(x.z, k.z));
+      acc = __fadd_rn(acc, __fmul_rn(x.w, k.w));
+    }
+  }
+  __syncwarp();
+  return acc;
+}
+// Indices of the keys whose approximate score is no further than `band` below the beam-th largest; their number, -1 when it is above 64.
+__device__ __forceinline__ int find_candidates(const float* approximate, int side, int beam, float band, int* cand, TopkScratch& sc) {
+  const int lane = threadIdx.x & 31;
+  const unsigned full = 0xffffffffu, below = (1u << lane) - 1u;
+  float score[LK_PER_LANE];
+  unsigned key[LK_PER_LANE];
+  load_scores(approximate, side, score);
+#pragma unroll
+  for (int i = 0; i < LK_PER_LANE; ++i) key[i] = i * 32 + lane < side ? okey(score[i]) : 0u;
+  const unsigned bound = key_bound(key);
+  const float least = bound > 1u ? okey_value(bound) - band : -INFINITY;
+  int count = 0;
+#pragma unroll
+  for (int i = 0; i < LK_PER_LANE; ++i) {
+    const bool take = key[i] != 0u && score[i] >= least;
+    const unsigned who = __ballot_sync(full, take);
+    const int at = count + __popc(who & below);
+    if (take && at < 64) {
+      sc.key[at] = key[i];
+      sc.index[at] = i * 32 + lane;
+    }
+    count += __popc(who);
+  }
+  __syncwarp();
+  if (count > 64 || count < beam) return -1;
+  unsigned v[2] = {lane < count ? sc.key[lane] : 0u, 32 + lane < count ? sc.key[32 + lane] : 0u};
+  unsigned sorted[2] = {v[0], v[1]};
+  sort_lanes(sorted);
+  unsigned best[1] = {upper_half(sorted[0], sorted[1])};
+  merge_lanes(best);
+  const float last = okey_value(__shfl_sync(full, best[0], beam - 1)) - band;
+  int n = 0;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const bool take = v[h] != 0u && okey_value(v[h]) >= last;
+    const unsigned who = __ballot_sync(full, take);
+    if (take) cand[n + __popc(who & below)] = sc.index[h * 32 + lane];
+    n += __popc(who);
+  }
+  __syncwarp();
+  return n;
+}
+// A side's beam out of exact scores of all of its keys.
+__device__ __noinline__ unsigned long long exact_beam(const float* keys, const float* q, int side, int half, int beam, float* buf, TopkScratch& sc) {
+  float score[LK_PER_LANE];
+#pragma unroll
+  for (int i = 0; i < LK_PER_LANE; ++i) score[i] = 0.f;
+#pragma unroll 1
+  for (int i = 0; i < LK_PER_LANE; ++i) {
+    if (i * 32 >= side) break;
+    const float x = exact_score(keys + (size_t)min(i * 32 + (int)(threadIdx.x & 31), side - 1) * half, q, half, buf);
+#pragma unroll
+    for (int u = 0; u < LK_PER_LANE; ++u)
+      if (u == i) score[u] = x;
+  }
+  return beam_of_scores(score, side, beam, sc);
+}
+
+__global__ void __launch_bounds__(128)
+product_key_lookup_kernel(const float* __restrict__ left_approx, const float* __restrict__ right_approx, const float* __restrict__ query,
+                          long long ld_q, const float* __restrict__ left_keys, const float* __restrict__ right_keys,
+                          const float* __restrict__ norms /* largest of either side */, int64_t* __restrict__ out, int tokens, int side, int half,
+                          int top_k, int beam, int* __restrict__ status) {
+  pdl_begin();
+  extern __shared__ __align__(16) float lk_smem[];
+  __shared__ TopkScratch scratch[4];
+  __shared__ int cands[4][2][64];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int token = blockIdx.x * 4 + w;
+  if (token >= tokens) return;
+  TopkScratch& sc = scratch[w];
+  float* q = lk_smem + w * (2 * half + 32 * LK_LD);
+  float* buf = q + 2 * half;
+  float squares[2] = {0.f, 0.f};
+  for (int c = lane * 4; c < 2 * half; c += 128) {
+    const float4 x = *reinterpret_cast<const float4*>(query + (size_t)token * ld_q + c);
+    *reinterpret_cast<float4*>(q + c) = x;
+    const float t = x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
+    if (c < half) squares[0] += t; else squares[1] += t;
+  }
+  int (*cand)[64] = cands[w];
+  int count[2];
+#pragma unroll
+  for (int sd = 0; sd < 2; ++sd) {
+    const float qn = sqrtf(warp_sum(squares[sd])), kn = norms[sd], s = qn * kn;
+    const bool within = qn >= 1e-18f && kn >= 1e-18f && s >= 1e-30f && s <= 1e37f;  // (false for NaN)
+    const float band = 2.f * s * (5.4e-7f * (float)half + 2e-5f);
+    count[sd] = within ? find_candidates((sd ? right_approx : left_approx) + (size_t)token * side, side, beam, band, cand[sd], sc) : -1;
+  }
+  int more[2] = {max(0, count[0] - 32), max(0, count[1] - 32)};  // beyond a warp's lanes
+  if (more[0] + more[1] > 32) {
+    count[more[0] > more[1] ? 0 : 1] = -1;
+    more[more[0] > more[1] ? 0 : 1] = 0;
+  }
+  unsigned long long v[2][2];  // [side]: the first 32 candidates, the rest
+#pragma unroll
+  for (int sd = 0; sd < 2; ++sd) {
+    v[sd][0] = v[sd][1] = 0ull;
+    if (count[sd] < 0) continue;
+    const int mine = lane < count[sd] ? cand[sd][lane] : 0;
+    const float x = exact_score(lane < count[sd] ? (sd ? right_keys : left_keys) + (size_t)mine * half : nullptr, q + sd * half, half, buf);
+    if (lane < count[sd]) v[sd][0] = ((unsigned long long)okey(x) << 32) | (0xffffffffu - (unsigned)mine);
+  }
+  if (more[0] + more[1] > 0) {  // both sides' in one go
+    const int sd = lane < more[0] ? 0 : 1, at = sd ? lane - more[0] : lane;
+    const bool real = lane < more[0] + more[1];
+    const int mine = real ? cand[sd][32 + at] : 0;
+    const float x = exact_score(real ? (sd ? right_keys : left_keys) + (size_t)mine * half : nullptr, q + sd * half, half, buf);
+    const unsigned long long e = ((unsigned long long)okey(x) << 32) | (0xffffffffu - (unsigned)mine);
+    if (real && sd == 0) v[0][1] = e;
+    if (real && sd == 1) v[1][1] = e;
+  }
+  unsigned long long beams[2];
+#pragma unroll
+  for (int sd = 0; sd < 2; ++sd) {
+    if (count[sd] < 0) {
+      beams[sd] = exact_beam(sd ? right_keys : left_keys, q + sd * half, side, half, beam, buf, sc);
+      continue;
+    }
+    if (more[sd] > 0) {
+      sort_lanes(v[sd]);
+      unsigned long long best[1] = {upper_half(v[sd][0], v[sd][1])};
+      merge_lanes(best);
+      beams[sd] = best[0];
+    } else {
+      unsigned long long one[1] = {v[sd][0]};
+      sort_lanes(one);
+      beams[sd] = one[0];
+    }
+    if (lane >= beam) beams[sd] = 0ull;
+  }
+  pick_pairs(beams[0], beams[1], out + (size_t)token * top_k, nullptr, side, top_k, beam, sc, status);
+}
+
+// Operands of the approximate scores.  Queries: row [hi left | lo left | hi right | lo right]; half keys: row [hi | hi | lo], the left
+// table's rows, then the right one's, and the largest norm of either table.
+__global__ void __launch_bounds__(256)
+query_pieces_kernel(const float* __restrict__ query, long long ld_q, __nv_bfloat16* __restrict__ out, int tokens, int half) {
+  pdl_begin();
+  const int per_row = half / 4;  // groups of eight in a row
+  const long long i = blockIdx.x * 256ll + threadIdx.x;
+  const long long t = i / per_row;
+  if (t >= tokens) return;
+  const int c = (int)(i - t * per_row) * 8, sd = c >= half;
+  float x[8];
+  const float4 a = *reinterpret_cast<const float4*>(query + t * ld_q + c), b = *reinterpret_cast<const float4*>(query + t * ld_q + c + 4);
+  x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+  uint4 piece[3];
+  split8_bf16(x, piece);
+  __nv_bfloat16* to = out + t * 4 * half + sd * 2 * half + (c - sd * half);
+  *reinterpret_cast<uint4*>(to) = piece[0];
+  *reinterpret_cast<uint4*>(to + half) = piece[1];
+}
+__global__ void __launch_bounds__(256)
+key_pieces_kernel(const float* __restrict__ left, const float* __restrict__ right, __nv_bfloat16* __restrict__ out, int* __restrict__ norm_bits,
+                  int side, int half) {
+  pdl_begin();
+  const int lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (row >= 2 * side) return;
+  const float* key = row < side ? left + (size_t)row * half : right + (size_t)(row - side) * half;
+  float squares = 0.f;
+  for (int c = lane * 8; c < half; c += 256) {
+    float x[8];
+    const float4 a = __ldg(reinterpret_cast<const float4*>(key + c)), b = __ldg(reinterpret_cast<const float4*>(key + c + 4));
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) squares += x[e] * x[e];
+    uint4 piece[3];
+    split8_bf16(x, piece);
+    __nv_bfloat16* to = out + (size_t)row * 3 * half + c;
+    *reinterpret_cast<uint4*>(to) = piece[0];
+    *reinterpret_cast<uint4*>(to + half) = piece[0];
+    *reinterpret_cast<uint4*>(to + 2 * half) = piece[1];
+  }
+  squares = warp_sum(squares);
+  const float norm = sqrtf(squares);
+  if (lane == 0) atomicMax(norm_bits + (row >= side), norm == norm ? __float_as_int(norm) : 0x7fffffff);  // (a NaN stays one)
 }
 
 __global__ void split_rows_kernel(const int64_t* __restrict__ rows, int64_t* __restrict__ left, int64_t* __restrict__ right,
@@ -1346,6 +1595,48 @@ int product_key_topk_impl(hl_ctx* ctx, const float* left_scores, const float* ri
   count_launch(ctx);
   return HL_OK;
 }
+
+bool product_key_lookup_takes(int side, int key_dim, int beam) {
+  return side % 8 == 0 && side <= 32 * LK_PER_LANE && key_dim % 64 == 0 && key_dim <= 1024 && beam <= 32;
+}
+size_t product_key_pieces_bytes(int side, int key_dim) { return (size_t)3 * side * key_dim * sizeof(__nv_bfloat16) + 256; }
+int product_key_pieces(hl_ctx* ctx, const float* left_keys, const float* right_keys, int side, int key_dim, void* pieces) {
+  int* norms = static_cast<int*>(pieces);
+  HL_CUDA(cudaMemsetAsync(norms, 0, 2 * sizeof(int), ctx->stream));
+  pdl(key_pieces_kernel, ceil_div(2 * side, 8), 256, 0, ctx->stream)(left_keys, right_keys,
+                                                                    reinterpret_cast<__nv_bfloat16*>(static_cast<uint8_t*>(pieces) + 256), norms,
+                                                                    side, key_dim / 2);
+  HL_LAUNCH_CHECK("key_pieces_kernel");
+  count_launch(ctx);
+  return HL_OK;
+}
+int product_key_lookup(hl_ctx* ctx, const float* query, const float* left_keys, const float* right_keys, const void* pieces,
+                       __nv_bfloat16* query_pieces, float* left_approx, float* right_approx, int64_t* out, int tokens, int side, int key_dim,
+                       int top_k, int beam) {
+  const int half = key_dim / 2;
+  pdl(query_pieces_kernel, (unsigned)ceil_div_ll((long long)tokens * (half / 4), 256), 256, 0, ctx->stream)(query, key_dim, query_pieces, tokens, half);
+  HL_LAUNCH_CHECK("query_pieces_kernel");
+  const __nv_bfloat16* keys = reinterpret_cast<const __nv_bfloat16*>(static_cast<const uint8_t*>(pieces) + 256);
+  hl_gemm_desc d{};
+  d.m = tokens; d.n = side; d.k = 3 * half;
+  d.a_layout = d.b_layout = HL_K_MAJOR;
+  d.lda = 4 * half; d.ldb = 3 * half; d.ldc = side;
+  d.out_dtype = HL_F32;
+  d.a_k_period = 2 * half;
+  for (int sd = 0; sd < 2; ++sd) {
+    const int rc = gemm_bf16_ctx(ctx, &d, query_pieces + sd * 2 * half, keys + (size_t)sd * side * 3 * half, sd ? right_approx : left_approx, nullptr,
+                                 nullptr, nullptr);
+    if (rc != HL_OK) return rc;
+  }
+  const size_t smem = sizeof(float) * 4 * (size_t)(2 * half + 32 * LK_LD);
+  HL_ALLOW_SHARED(ctx, sizeof(float) * 4 * (2 * 512 + 32 * LK_LD), product_key_lookup_kernel);
+  pdl(product_key_lookup_kernel, ceil_div(tokens, 4), 128, smem, ctx->stream)(left_approx, right_approx, query, key_dim, left_keys, right_keys,
+                                                                             static_cast<const float*>(pieces), out, tokens, side, half, top_k,
+                                                                             beam, ctx->status_dev);
+  HL_LAUNCH_CHECK("product_key_lookup_kernel");
+  count_launch(ctx, 2);
+  return HL_OK;
+}
 }  // namespace hl
 
 extern "C" {
@@ -1377,6 +1668,16 @@ int hl_product_key_side_scores_f32(hl_ctx* ctx, const float* query, long long ld
   HL_LAUNCH_CHECK("side_scores_kernel");
   count_launch(ctx);
   return HL_OK;
+}
+
+// product_key_pieces and product_key_lookup for a caller that brings all buffers (the step has its own).
+int hl_product_key_lookup(hl_ctx* ctx, const float* query, const float* left_keys, const float* right_keys, void* pieces, void* query_pieces,
+                          float* left_approx, float* right_approx, int64_t* out, int tokens, int side, int key_dim, int top_k, int beam) {
+  if (tokens < 1 || !product_key_lookup_takes(side, key_dim, beam)) return fail("hl_product_key_lookup: sizes of the general form");
+  const int rc = product_key_pieces(ctx, left_keys, right_keys, side, key_dim, pieces);
+  if (rc != HL_OK) return rc;
+  return product_key_lookup(ctx, query, left_keys, right_keys, pieces, static_cast<__nv_bfloat16*>(query_pieces), left_approx, right_approx, out,
+                            tokens, side, key_dim, top_k, beam);
 }
 
 int hl_product_key_topk_from_side_scores(hl_ctx* ctx, const float* left_scores, const float* right_scores, int64_t* out,

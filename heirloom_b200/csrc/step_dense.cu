@@ -134,6 +134,9 @@ struct hl_decoder {
   cudaEvent_t zero_event = nullptr;  // the scattered gradients have been zeroed there
   cudaEvent_t sort_event = nullptr;  // the selections that the forward pass has left so far are in row order
   void* sort_scratch = nullptr;      // of those sorts, one at a time
+  bool lookup = false;               // passes over whole windows select by product_key_lookup
+  void* key_pieces = nullptr;        // of the half keys, made at the start of every pass
+  __nv_bfloat16* query_pieces = nullptr;
   bool sorted = false;               // this pass sorts them there
   // a scratch arena for what runs there, in place of the context's
   void* side_arena = nullptr;
@@ -410,6 +413,10 @@ void plan_memory_buffers(hl_decoder* m, uint8_t*& cur) {
   m->m_dw = carve<float>(cur, N * k);
   m->m_dscores = carve<float>(cur, N * k);
   m->m_dq = carve<float>(cur, N * kd);
+  // Exact scores of all keys and the selection take 421 us a block at 16384 tokens, sides of 512 and keys of 512, the lookup 276; steps with
+  // two blocks, all keys against the lookup: 1102 and 1020 us at 128 tokens of the same tables, 869 and 861 at 2048 tokens, sides of 128 and
+  // keys of 64, 690 and 708 at 512 tokens of these.
+  m->lookup = !m->lean && N * m->side * kd >= (1ull << 24) && product_key_lookup_takes(m->side, (int)kd, (int)k);
   if (m->cfg.precision == HL_PRECISION_AMP_BF16) {
     m->p_dx_side = carve<__nv_bfloat16>(cur, N * 2 * d);
     m->p_dx_rows = carve<__nv_bfloat16>(cur, 2 * N * d);
@@ -419,9 +426,12 @@ void plan_memory_buffers(hl_decoder* m, uint8_t*& cur) {
     m->p_dq_rows = carve<__nv_bfloat16>(cur, 3 * N * kd);
     m->p_wout_rows = carve<__nv_bfloat16>(cur, 3 * d * vd);
     m->p_wc_rows = carve<__nv_bfloat16>(cur, 3 * (vd + kd) * d);
+    m->query_pieces = m->p_dc_side;  // (the backward pass comes later)
   } else {
     m->m_dgate = carve<float>(cur, N * vd);
+    if (m->lookup) m->query_pieces = carve<__nv_bfloat16>(cur, N * 2 * kd);
   }
+  if (m->lookup) m->key_pieces = carve<uint8_t>(cur, product_key_pieces_bytes(m->side, (int)kd));
   m->m_row_flags = carve<unsigned char>(cur, (size_t)m->mem.slots);
   m->smft_value_mask = carve<unsigned char>(cur, (size_t)m->mem.slots);
   m->smft_left_mask = carve<unsigned char>(cur, (size_t)m->side);
@@ -739,10 +749,15 @@ int memory_core_forward(hl_decoder* m, int l, bool one_token = false) {
   const float* P = m->params;
   const int N = m->N, kd = m->mem.key_dim, vd = m->mem.value_dim, k = m->mem.top_k, side = m->side;
   const int beam = std::min(side, std::max(k, (int)ceil(sqrt((double)k))));  // product_key_beam, :2014-2016
+  if (!one_token && m->lookup) {
+    HL_TRY(product_key_lookup(ctx, a.query, P + m->off_kl, P + m->off_kr, m->key_pieces, m->query_pieces, m->m_ls, m->m_rs, idx, N, side, kd, k, beam));
+  } else {
+    ProfileScope prof(ctx, HL_PROF_OTHER, 2.0 * (double)N * side * 4.0);
+    HL_TRY(hl_product_key_side_scores_f32(ctx, a.query, kd, P + m->off_kl, P + m->off_kr, m->m_ls, m->m_rs, N, side, kd));
+    HL_TRY(product_key_topk_impl(ctx, m->m_ls, m->m_rs, idx, N, side, k, beam, one_token ? a.idx : nullptr, m->decode_state));
+  }
   // timed as one family ("other" in the per-kernel profile); work = table rows gathered, in bytes
-  ProfileScope prof(ctx, HL_PROF_OTHER, (double)N * k * (double)(kd + vd) * 4.0 + 2.0 * (double)N * side * 4.0);
-  HL_TRY(hl_product_key_side_scores_f32(ctx, a.query, kd, P + m->off_kl, P + m->off_kr, m->m_ls, m->m_rs, N, side, kd));
-  HL_TRY(product_key_topk_impl(ctx, m->m_ls, m->m_rs, idx, N, side, k, beam, one_token ? a.idx : nullptr, m->decode_state));
+  ProfileScope prof(ctx, HL_PROF_OTHER, (double)N * k * (double)(kd + vd) * 4.0);
   if (m->sorted && a.sorted_rows) {  // for the backward pass, beside what follows
     SideStream beside(m);
     HL_TRY(beside.rc);
@@ -753,6 +768,12 @@ int memory_core_forward(hl_decoder* m, int l, bool one_token = false) {
                                            m->mem.slots));
   HL_TRY(hl_softmax_rows_f32(ctx, m->m_scores, a.weights, N, k));
   return hl_memory_weighted_value_forward(ctx, idx, a.weights, P + m->off_val, a.weighted, N, k, m->mem.slots, vd);
+}
+
+// What every memory block's lookup of a pass reads of the tables, which all of them share.
+int prepare_lookups(hl_decoder* m) {
+  if (!m->lookup) return HL_OK;
+  return product_key_pieces(m->ctx, m->params + m->off_kl, m->params + m->off_kr, m->side, m->mem.key_dim, m->key_pieces);
 }
 
 // dweighted -> m_dq (gradient of the query) and the table gradients (added into the arena).
@@ -951,6 +972,7 @@ int forward(hl_decoder* m, Forward what = Forward::all) {
   const __nv_bfloat16* W = m->shadow;
   if (!m->comm_pending) ctx->reserve_sms = 0;  // nothing of the gradient exchange is in flight during a forward pass
   HL_TRY(hl_embedding_forward(ctx, P + m->off_tok, V, m->tokens, P + m->off_pos, T, m->x[0], HL_BF16, N, d));
+  HL_TRY(prepare_lookups(m));
   for (int l = 0; l < c.n_layers; ++l) {
     const LayerOffsets& o = m->lo[l];
     LayerActs& a = m->la[l];
@@ -1379,6 +1401,7 @@ int forward_f32(hl_decoder* m, bool last_only = false) {
   const int N = m->N, d = c.d_model, F = c.d_ff, V = c.vocab, B = c.batch, T = c.context, H = c.n_heads;
   const float* P = m->params;
   HL_TRY(hl_embedding_forward(ctx, P + m->off_tok, V, m->tokens, P + m->off_pos, T, m->xf[0], HL_F32, N, d));
+  HL_TRY(prepare_lookups(m));
   for (int l = 0; l < c.n_layers; ++l) {
     const LayerOffsets& o = m->lo[l];
     hl_decoder::F32Layer& a = m->lf[l];

@@ -469,3 +469,45 @@ def test_gathers_at_the_edges_of_their_forms(tokens, top_k, side, key_dim, dim):
     np.add.at(want, idx.reshape(-1), (w[..., None].astype(np.float64) * go[:, None, :]).reshape(-1, dim))
     run = np.bincount(idx.reshape(-1)).max()
     assert_close("dv", host(dv), want, atol=1e-6 * np.sqrt(run) * 4 + 2e-7 * run, rtol=1e-6)
+
+
+@pytest.mark.parametrize("tokens,side,key_dim,top_k", [(1, 8, 64, 5), (259, 40, 64, 32), (300, 512, 512, 32), (1001, 256, 192, 16), (257, 504, 1024, 1)])
+@pytest.mark.parametrize("kind", ["random", "ties", "near", "huge", "tiny", "odd"])
+def test_lookup_of_the_step_selects_what_exact_scores_do(tokens, side, key_dim, top_k, kind):
+    """Scores that decide are formed in the order of hl_product_key_side_scores_f32, so the rows are the same, in order; also where many
+    keys tie, lie closer than the approximation tells apart, or are out of its range."""
+    from ctypes import c_int
+
+    from heirloom_b200 import cuda
+    c = ctx()
+    rng = np.random.default_rng(side + key_dim)
+    half = key_dim // 2
+    q = rng.standard_normal((max(tokens, 10), key_dim)).astype(np.float32)
+    keys = [rng.standard_normal((side, half)).astype(np.float32) for _ in range(2)]
+    if kind == "ties":  # 16 distinct keys; whole numbers, whose sums are exact, in the right table
+        keys[0] = keys[0][rng.integers(0, min(side, 16), side)]
+        keys[1], q[:, half:] = rng.integers(-2, 3, keys[1].shape), rng.integers(-2, 3, (len(q), half))
+    elif kind == "near":  # all of the left table within a few units in the last place
+        keys[0] = (keys[0][:1] * (1 + 2e-7 * rng.standard_normal((side, half)))).astype(np.float32)
+    elif kind == "huge":
+        q[::2] *= 1e20
+        q[1::4] *= 1e30
+        keys[1] *= 1e7
+    elif kind == "tiny":
+        q[::2] *= 1e-25
+        q[1::4, :half] = 0
+        keys[1] *= 1e-20
+    elif kind == "odd":
+        q[3, 1], q[5, half], q[8], q[9, 0] = np.inf, -np.inf, 3e38, np.nan
+        keys[0][side - 1, 0] = np.inf
+    beam = min(side, max(top_k, int(np.ceil(np.sqrt(top_k)))))
+    query, left, right = dev(q[:tokens]), dev(keys[0].astype(np.float32)), dev(keys[1].astype(np.float32))
+    want = cuda.product_key_topk_from_side_scores(c, *cuda.product_key_side_scores(c, query, left, right), top_k, beam)
+    got = torch.full_like(want, -1)
+    pieces = torch.empty(6 * side * key_dim + 256, dtype=torch.uint8, device="cuda")
+    query_pieces = torch.empty(tokens, 2 * key_dim, dtype=torch.bfloat16, device="cuda")
+    approx = torch.empty(2, tokens, side, device="cuda")
+    cuda.check(c.lib.hl_product_key_lookup(c.handle, cuda._p(query), cuda._p(left), cuda._p(right), cuda._p(pieces), cuda._p(query_pieces),
+                                           cuda._p(approx[0]), cuda._p(approx[1]), cuda._p(got), c_int(tokens), c_int(side), c_int(key_dim),
+                                           c_int(top_k), c_int(beam)))
+    np.testing.assert_array_equal(host(got), host(want))
