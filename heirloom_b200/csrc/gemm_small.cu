@@ -364,6 +364,11 @@ GemmSmallPlan gemm_small_plan(const hl_gemm_desc* d, const GemmPlan& big, int de
     else if (narrow * s <= wave_ctas(1, s, device, sm_count)) take(3.0f + 0.34f * steps + shared, 64, false);
     if (wide * s <= wave_ctas(2, s, device, sm_count)) take(4.4f + 0.21f * steps + (s > 1 ? 2.5f : 0.f), 128, false);
   }
+  // A weight gradient (both operands down their rows) runs beside the next layer's kernels, and four stages leave these half of the SM:
+  // with up to eight k blocks a CTA a step of 1024 tokens and 256 channels takes 466 us for 494, 384 tokens of 512 channels 1075 for 1088.
+  // With 32 k blocks (2048 tokens of 512 channels) it is 2432 for 2408, and products that the next kernel waits for lose as well (700 tokens
+  // of 192 channels 360 for 345 us).
+  if (plan.deep && d->a_layout == HL_MN_MAJOR && d->b_layout == HL_MN_MAJOR && ceil_div(kb, plan.splits) <= 8) plan.deep = false;
   return plan;
 }
 
