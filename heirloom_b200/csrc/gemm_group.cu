@@ -262,7 +262,7 @@ gemm_group_kernel(const __grid_constant__ GroupParams p) {
         } else {  // all of it is in registers: the next tile may overwrite it
           tc05::tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) tc05::mbar_arrive_cluster(tc05::cluster_map_shared(&sh->tmem_empty, 0));
+          if (lane == 0) tc05::mbar_arrive_cluster_read(tc05::cluster_map_shared(&sh->tmem_empty, 0));
         }
         if (lane == 0) tc05::tma_store_wait_read();
         __syncwarp();

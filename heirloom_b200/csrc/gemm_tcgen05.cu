@@ -427,7 +427,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     WorkItem w;
     // the accumulator buffer goes back to the MMA issuer, which in a pair sits in the even CTA
     auto release_buffer = [&](int buf) {
-      if (PAIR) tc05::mbar_arrive_cluster(tc05::cluster_map_shared(&tail->tmem_empty[buf], 0));
+      if (PAIR) tc05::mbar_arrive_cluster_read(tc05::cluster_map_shared(&tail->tmem_empty[buf], 0));
       else tc05::mbar_arrive(&tail->tmem_empty[buf]);
     };
     // The `local`-th item of this CTA into `dst`: 1 = there is one, 0 = the sequence is over, -1 = a wait ran out.

@@ -208,8 +208,11 @@ __device__ __forceinline__ uint32_t cluster_map_shared(const void* p, uint32_t r
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
   return a;
 }
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
+// An arrival in another CTA that hands over tensor memory this warp has read (tmem_ld_wait, tc_fence_before_sync before it), and nothing that
+// was written to memory.  So it is relaxed: with release at cluster scope it waited 2300 cycles for the warp's stores, once a tile of
+// 5000 to 12000 cycles.
+__device__ __forceinline__ void mbar_arrive_cluster_read(uint32_t bar_cluster_addr) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
 // TMA tile load into this CTA's shared memory whose bytes are counted on a barrier that may live in the peer CTA.
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar_cluster_addr, int c0,
