@@ -74,6 +74,17 @@ constexpr int TAIL_BYTES = 320;
 constexpr size_t GEMM_SMEM_BYTES = GEMM_DATA_BYTES + TAIL_BYTES + size_t(EPI_WARPS) * EPI_BIAS_BYTES;
 static_assert(GEMM_SMEM_BYTES <= 227 * 1024, "shared memory budget");
 
+// n / d for 0 <= n < 2^31 by a multiplication (Granlund and Montgomery 1994, "Division by invariant integers using multiplication"): every
+// warp role divides three times a tile, at some 200 cycles each time.
+struct QuickDiv {
+  uint32_t mul, shift;
+  explicit QuickDiv(uint32_t d = 1) : shift(0) {
+    while ((1ull << shift) < d) ++shift;
+    mul = (uint32_t)(((1ull << 32) * ((1ull << shift) - d)) / d + 1);
+  }
+  __device__ __forceinline__ int operator()(int n) const { return (int)((__umulhi((uint32_t)n, mul) + (uint32_t)n) >> shift); }
+};
+
 struct GemmParams {
   int m, n, k;
   int m_tiles, n_tiles, splits, k_blocks, k_blocks_per_split;
@@ -82,6 +93,7 @@ struct GemmParams {
   int partial_out;  // split-K: raw accumulators go to the [splits][m][n] scratch through map_c
   int dp_tiles, sk_tiles;   // whole-wave tiles, then tiles whose k blocks are dealt out evenly
   int panel_w;              // tile columns per panel of the tile order
+  QuickDiv by_tiles, by_panel, by_width, by_last_width;  // all tiles, those of a panel, a panel's columns, the last panel's
   int a_kb_wrap;            // > 0: A holds this many k blocks and is read again from its start after them
   int b_kb_wrap;            // the same for B
   unsigned long long wait_limit_ns;  // bound of every pipeline wait
@@ -144,7 +156,7 @@ __device__ __forceinline__ bool get_item(const GemmParams& p, int local, WorkIte
   if (p.sk_tiles == 0) {  // tiles (times explicit splits) round-robin, or handed out by a counter (item < 0: local is the item)
     const int item = local < 0 ? -local - 1 : cta + local * grid;
     if (item >= tiles * p.splits) return false;
-    w.split = item / tiles;
+    w.split = p.splits == 1 ? 0 : p.by_tiles(item);
     tile = item - w.split * tiles;
     w.kb0 = w.split * p.k_blocks_per_split;
     w.kb1 = min(p.k_blocks, w.kb0 + p.k_blocks_per_split);
@@ -191,10 +203,10 @@ __device__ __forceinline__ bool get_item(const GemmParams& p, int local, WorkIte
   // run at the same time then share a few A row blocks and a few B column blocks, so each operand
   // byte comes out of DRAM once instead of once per tile column.
   const int per_panel = p.panel_w * p.m_tiles;
-  const int panel = tile / per_panel;
+  const int panel = p.by_panel(tile);
   const int r = tile - panel * per_panel;
   const int width = min(p.panel_w, p.n_tiles - panel * p.panel_w);
-  w.m_tile = r / width;
+  w.m_tile = width == p.panel_w ? p.by_width(r) : p.by_last_width(r);
   w.n_tile = panel * p.panel_w + (r - w.m_tile * width);
   return true;
 }
@@ -1052,6 +1064,10 @@ int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void*
   // Panels of up to sixteen tile columns: A streams past B's columns, which stay in L2.  One column after the other would read
   // an A of 25 MB again for each of them while the results push it out of L2 (16384 x 3072 x 768: 81 us, now 77).
   p.panel_w = std::min(p.n_tiles, 16);
+  p.by_tiles = QuickDiv((uint32_t)(p.m_tiles * p.n_tiles));
+  p.by_panel = QuickDiv((uint32_t)(p.panel_w * p.m_tiles));
+  p.by_width = QuickDiv((uint32_t)p.panel_w);
+  p.by_last_width = QuickDiv((uint32_t)(p.n_tiles % p.panel_w ? p.n_tiles % p.panel_w : p.panel_w));
   const int splits = plan.splits;
   const size_t need = plan.splitk_bytes;
   p.splits = splits;
