@@ -16,6 +16,7 @@
 // A one-token step of the GPT-sized model at 500 positions: 271 -> 225 us (attention kernel 10, feed-forward 6.6, head 20); generation
 // of 8 tokens behind a prefix of 500 2690 -> 2377 us, of 32 with four f32 blocks of 128 channels (24 one-token steps) 3550 -> 3080.
 #include "decode.cuh"
+#include "tc05.cuh"
 
 namespace hl {
 namespace {
@@ -316,7 +317,7 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_attention_block_kernel(c
   const Row<T, Acc> in(a.x, a.gamma, a.beta, a.window ? 0 : d);
   const Acc scale = (Acc)1 / sqrt((Acc)hd);
   const int fresh_at = (int)threadIdx.x / cpc * pitch_fresh + (int)threadIdx.x % cpc;
-  cluster.sync();  // the peers have started: their shared memory may be written
+  tc05::cluster_meet();  // the peers have started: their shared memory may be written
   pdl_wait();
   if (a.window) {
     stage_keys(k1 - k0);
@@ -329,16 +330,16 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_attention_block_kernel(c
     multiply_rows(wqkv, d + PAD, rows, row, d, red);
     __syncthreads();
     float* own = fresh + rank * pitch_fresh;
-    if (const int i = threadIdx.x; i < rows) {
-      const int which = i < cpc ? 0 : i < 2 * cpc ? 1 : 2;
-      const float y = rounded<T>((float)product_of_row(red, rows, i) + bias[i]);
-      own[i] = y;
-      qkv[(long long)t * ld + which * d + rank * cpc + i - which * cpc] = stored<T>(y);
-    }
+    float y = 0.f;
+    if (const int i = threadIdx.x; i < rows) own[i] = y = rounded<T>((float)product_of_row(red, rows, i) + bias[i]);
     __syncthreads();
     if (warp < DB_CTAS && warp != rank) push(cluster, own, own, pitch_fresh * 4, warp);
     cp_async_wait_all();
     cluster.sync();
+    if (const int i = threadIdx.x; i < rows) {  // (in front of the barrier it would wait for these stores)
+      const int which = i < cpc ? 0 : i < 2 * cpc ? 1 : 2;
+      qkv[(long long)t * ld + which * d + rank * cpc + i - which * cpc] = stored<T>(y);
+    }
     if (const int c = threadIdx.x; c < hd) {
       const float* f = fresh + fresh_at;
       q[c] = f[0];
@@ -501,7 +502,7 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_feed_forward_kernel(cons
     for (int i = threadIdx.x; i < d * (units - n); i += DB_THREADS) w2[i / (units - n) * at.pitch2 + n + i % (units - n)] = T(0.f);
   const Row<T, Acc> in(a.x, a.gamma, a.beta, d);
   const unsigned per_share = ((1u << 20) + opc - 1) / opc;  // c / opc = c * per_share >> 20 for c < 1024, opc <= 128
-  cluster.sync();  // the peers have started
+  tc05::cluster_meet();  // the peers have started
   pdl_wait();
   in.form(a.x, d, norm, row);
   cp_async_wait<1>();

@@ -202,6 +202,11 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// Every CTA of the cluster is at this point; nothing that was written is handed over (which would wait for the thread's stores).
+__device__ __forceinline__ void cluster_meet() {
+  asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+  asm volatile("barrier.cluster.wait;" ::: "memory");
+}
 // The address, in the cluster's shared window, of CTA `rank`'s copy of a shared-memory object of this CTA.
 __device__ __forceinline__ uint32_t cluster_map_shared(const void* p, uint32_t rank) {
   uint32_t a;
