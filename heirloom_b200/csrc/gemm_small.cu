@@ -284,7 +284,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       for (int half = 0; half < 2; ++half) v += p.splits > 1 ? *cluster.map_shared_rank(at + half * GS_BM, s) : at[half * GS_BM];
     p.row_sum[m0 + row_first + threadIdx.x] = (float)v;
   }
-  if (p.splits > 1) cluster.sync();  // no CTA leaves while another still reads its sums
+  if (p.splits > 1) tc05::cluster_meet();  // no CTA leaves while another still reads its sums
   if (!ok || *abort_flag) {
     for (int i = 0; i < 2000; ++i) __nanosleep(100);  // copies in flight land before shared memory is released
     if (threadIdx.x == 0) atomicExch(p.status + ST_WAIT_EXPIRED, 1);

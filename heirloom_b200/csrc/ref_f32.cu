@@ -10,6 +10,7 @@
 #include <cooperative_groups.h>
 
 #include "kernels.h"
+#include "tc05.cuh"
 
 namespace hl {
 namespace {
@@ -365,7 +366,7 @@ f64_gemm_kernel(const F64Jobs jobs) {
     g.out[at] = y;
   }
   if (sums && rank == 0 && tid < TM && row0 + tid < g.m) g.row_sum[row0 + tid] = (float)total(TM * Z::LDC + tid);
-  if (parts > 1) cluster.sync();  // no CTA leaves while another still reads its part
+  if (parts > 1) tc05::cluster_meet();  // no CTA leaves while another still reads its part
 }
 
 template <int TM, int TN>
