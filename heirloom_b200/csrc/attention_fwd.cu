@@ -21,6 +21,8 @@
 // work and waits lie under the other's exponentials, and each goes through its items without a gap: while the softmax warps
 // write one item's result, the next one's first scores are being formed.  With a CTA per item (B16 H12 T1024: 69 us) 29 us were
 // starts and ends of CTAs; heads of 128 channels had one CTA an SM and nothing to hide a warp's chain under (B4 H12 T4096: 311 us).
+#include <type_traits>
+
 #include "common.cuh"
 #include "tc05.cuh"
 
@@ -67,6 +69,7 @@ struct FaParams {
   long long ld_out;
   __nv_bfloat16* out;
   float* lse;
+  QuickDiv by_heads, by_h;  // all heads, a batch entry's
   float scale_log2;  // softmax scale times log2(e)
   int* status;
 };
@@ -76,19 +79,20 @@ struct FaParams {
 struct FaItem {
   int local, q0, b, h, n_tiles;  // n_tiles: key tiles of 64 up to and including the diagonal; 0: no more items
 };
-__device__ __forceinline__ FaItem fa_item(int local, const FaParams& p) {
+__device__ __forceinline__ FaItem fa_item(int local, const FaParams& p, int cta, int grid) {
   const int nq = (p.T + FA_BM - 1) / FA_BM, heads = p.B * p.H;
-  const int grid = (int)gridDim.x, cta = (int)blockIdx.x;
   const int item = local * grid + ((local & 1) ? grid - 1 - cta : cta);
   FaItem it{local, 0, 0, 0, 0};
   if (item >= nq * heads) return it;
-  const int qi = nq - 1 - item / heads, bh = item % heads;
+  const int round = p.by_heads(item), qi = nq - 1 - round, bh = item - round * heads;
   it.q0 = qi * FA_BM;
-  it.b = bh / p.H;
-  it.h = bh % p.H;
+  it.b = p.by_h(bh);
+  it.h = bh - it.b * p.H;
   it.n_tiles = 2 * (qi + 1);
   return it;
 }
+
+__device__ __forceinline__ FaItem fa_item(int local, const FaParams& p) { return fa_item(local, p, (int)blockIdx.x, (int)gridDim.x); }
 
 template <int HD>
 __global__ void __launch_bounds__(FA_THREADS, 2)
@@ -396,6 +400,310 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   }
 }
 
+// ---- heads of 64 channels ---------------------------------------------------------------------------------------------------
+// What bounds these is the softmax: 64 exponentials a row and tile are 512 cycles of a scheduler's, the products 256.  A warp's chain (scores,
+// maximum, exponentials, hand-over) takes three times that, so that three warps share a scheduler: one CTA an SM walks three streams
+// of items side by side, each with its own tiles, four softmax warps and a warp whose elected thread queues both loads and products.
+// That thread waits for scores that have been read and P that has been written, and for nothing else: when S(g) has been read, Q·K(g)
+// is done and K(g) can be replaced; when P(g) has been written, P·V(g-1) is done and V(g-1) can.
+// A stream has one S and one O in tensor memory (128 columns), one Q, one P (through which the result leaves), three K, two V: 72 KB.
+constexpr int F3_STREAMS = 3;
+constexpr int F3_THREADS = F3_STREAMS * 5 * 32;
+constexpr int F3_K_STAGES = 3, F3_V_STAGES = 2;
+constexpr int F3_TMEM_COLS = FA_BN + FA_BN / 2 + 64;  // S, P in bf16, O
+static_assert(F3_STREAMS * F3_TMEM_COLS <= 512, "tensor memory columns");
+constexpr int F3_Q_BYTES = FA_BM * 128, F3_KV_BYTES = FA_BN * 128;
+constexpr int F3_O_BYTES = F3_Q_BYTES;
+constexpr int F3_STREAM_BYTES = F3_Q_BYTES + F3_O_BYTES + (F3_K_STAGES + F3_V_STAGES) * F3_KV_BYTES;
+struct F3Shared {
+  uint64_t q_full, k_full[F3_K_STAGES], v_full[F3_V_STAGES], s_full, s_empty, p_full, o_full;
+};
+constexpr int F3_SMEM = F3_STREAMS * F3_STREAM_BYTES + 512;
+static_assert(F3_STREAMS * sizeof(F3Shared) + 8 <= 512 && F3_SMEM <= 227 * 1024, "shared memory budget");
+
+__global__ void __launch_bounds__(F3_THREADS, 1)
+flash_attention_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                             const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o, const FaParams p) {
+  extern __shared__ __align__(1024) uint8_t fa_smem[];  // swizzled tiles want 1024 bytes; checked below
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool control = warp >= F3_STREAMS * 4;
+  const int stream = control ? warp - F3_STREAMS * 4 : warp >> 2;
+  uint8_t* sq = fa_smem + stream * F3_STREAM_BYTES;
+  uint8_t* so = sq + F3_Q_BYTES;
+  uint8_t* sk = so + F3_O_BYTES;
+  uint8_t* sv = sk + F3_K_STAGES * F3_KV_BYTES;
+  F3Shared* all = reinterpret_cast<F3Shared*>(fa_smem + F3_STREAMS * F3_STREAM_BYTES);
+  F3Shared* sh = all + stream;
+  uint32_t* tmem_base = reinterpret_cast<uint32_t*>(all + F3_STREAMS);
+  int* abort_word = reinterpret_cast<int*>(tmem_base + 1);
+  volatile int* abort_flag = abort_word;
+  const bool layout_ok = (tc05::smem_u32(fa_smem) & 1023u) == 0;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < F3_STREAMS; ++i) {
+      tc05::mbar_init(&all[i].q_full, 1);
+      for (int s = 0; s < F3_K_STAGES; ++s) tc05::mbar_init(&all[i].k_full[s], 1);
+      for (int s = 0; s < F3_V_STAGES; ++s) tc05::mbar_init(&all[i].v_full[s], 1);
+      tc05::mbar_init(&all[i].s_full, 1);
+      tc05::mbar_init(&all[i].s_empty, 4);
+      tc05::mbar_init(&all[i].p_full, 4);
+      tc05::mbar_init(&all[i].o_full, 1);
+    }
+    *abort_word = layout_ok ? 0 : 1;
+    tc05::fence_barrier_init();
+  }
+  if (warp == F3_STREAMS * 4) {
+    tc05::tmem_alloc(tmem_base, 512);
+    tc05::tmem_relinquish();
+  }
+  tc05::tc_fence_before_sync();
+  __syncthreads();
+  tc05::tc_fence_after_sync();
+  const uint32_t tmem_s = *tmem_base + (uint32_t)(stream * F3_TMEM_COLS), tmem_p = tmem_s + FA_BN, tmem_o = tmem_p + FA_BN / 2;
+  pdl_begin();  // everything above touches nothing a predecessor wrote
+
+  const int grid = F3_STREAMS * (int)gridDim.x, cta = stream * (int)gridDim.x + (int)blockIdx.x;
+  auto item = [&](int local) { return fa_item(local, p, cta, grid); };
+  if (control) {
+    // -------------------------------------------------------------------------- loads and products of one stream
+    if (tc05::elect_one() && !*abort_flag) {
+      tc05::tma_prefetch_desc(&map_q);
+      tc05::tma_prefetch_desc(&map_k);
+      tc05::tma_prefetch_desc(&map_v);
+      constexpr uint32_t idesc_qk = tc05::instr_desc_bf16_f32(FA_BM, FA_BN, false, false);
+      constexpr uint32_t idesc_pv = tc05::instr_desc_bf16_f32(FA_BM, 64, false, true);
+      // the next tile to load (K, V) or to score, each with its item, its place in the item and its number in the stream
+      struct Cursor {
+        FaItem it;
+        int j, g;
+      };
+      auto advance = [&](Cursor& c) {
+        ++c.g;
+        if (++c.j == c.it.n_tiles) {
+          c.it = item(c.it.local + 1);
+          c.j = 0;
+        }
+      };
+      const FaItem first = item(0);
+      Cursor ck{first, 0, 0}, cv{first, 0, 0}, cs{first, 0, 0};
+      auto load_q = [&](const FaItem& it) {
+        if (it.n_tiles == 0) return;
+        tc05::mbar_arrive_expect_tx(&sh->q_full, F3_Q_BYTES);
+        tc05::tma_load_3d(sq, &map_q, &sh->q_full, it.h * 64, it.q0, it.b);
+      };
+      auto load_k = [&]() {
+        if (ck.it.n_tiles == 0) return;
+        const int s = ck.g % F3_K_STAGES;
+        tc05::mbar_arrive_expect_tx(&sh->k_full[s], F3_KV_BYTES);
+        tc05::tma_load_3d(sk + s * F3_KV_BYTES, &map_k, &sh->k_full[s], ck.it.h * 64, ck.j * FA_BN, ck.it.b);
+        advance(ck);
+      };
+      auto load_v = [&]() {
+        if (cv.it.n_tiles == 0) return;
+        const int s = cv.g % F3_V_STAGES;
+        tc05::mbar_arrive_expect_tx(&sh->v_full[s], F3_KV_BYTES);
+        tc05::tma_load_3d(sv + s * F3_KV_BYTES, &map_v, &sh->v_full[s], cv.it.h * 64, cv.j * FA_BN, cv.it.b);
+        advance(cv);
+      };
+      auto scores = [&]() -> bool {  // S = Q · Kᵀ of the next tile
+        if (cs.it.n_tiles == 0) return true;
+        if (cs.j == 0 && !tc05::mbar_wait(&sh->q_full, (uint32_t)cs.it.local & 1u, abort_flag)) return false;
+        const int s = cs.g % F3_K_STAGES;
+        if (!tc05::mbar_wait(&sh->k_full[s], (uint32_t)(cs.g / F3_K_STAGES) & 1u, abort_flag)) return false;
+        tc05::tc_fence_after_sync();
+        const uint32_t aq = tc05::smem_u32(sq), ak = tc05::smem_u32(sk + s * F3_KV_BYTES);
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+          tc05::umma_ss(tmem_s, tc05::smem_desc_sw128(aq + ks * 32, 16, 1024), tc05::smem_desc_sw128(ak + ks * 32, 16, 1024), idesc_qk, ks > 0 ? 1u : 0u);
+        tc05::umma_commit(&sh->s_full);
+        advance(cs);
+        return true;
+      };
+      load_q(first);
+      load_k();
+      load_v();
+#pragma unroll 1
+      for (int i = 1; i < F3_K_STAGES; ++i) load_k();
+#pragma unroll 1
+      for (int i = 1; i < F3_V_STAGES; ++i) load_v();
+      bool ok = scores();
+      int g = 0;
+      for (FaItem it = first; ok && it.n_tiles > 0; it = item(it.local + 1)) {
+        for (int j = 0; j < it.n_tiles; ++j, ++g) {
+          ok = tc05::mbar_wait(&sh->s_empty, (uint32_t)g & 1u, abort_flag);  // S(g) has been read
+          if (!ok) break;
+          load_k();
+          if (j + 1 == it.n_tiles) load_q(item(it.local + 1));
+          ok = scores();
+          if (!ok) break;
+          // P(g) has been written and, in an item's first tile, the last item's O read
+          ok = tc05::mbar_wait(&sh->p_full, (uint32_t)g & 1u, abort_flag);
+          if (!ok) break;
+          if (g > 0) load_v();  // in the place of V(g - 1)
+          const int s = g % F3_V_STAGES;
+          ok = tc05::mbar_wait(&sh->v_full[s], (uint32_t)(g / F3_V_STAGES) & 1u, abort_flag);
+          if (!ok) break;
+          tc05::tc_fence_after_sync();
+          const uint32_t av = tc05::smem_u32(sv + s * F3_KV_BYTES);
+#pragma unroll
+          for (int ks = 0; ks < FA_BN / 16; ++ks)  // A = P, two keys a column; B = V: rows are keys (MN-major), 16 keys per step
+            tc05::umma_ts(tmem_o, tmem_p + ks * 8, tc05::smem_desc_sw128(av + ks * (16 * 128), F3_KV_BYTES, 1024), idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
+          tc05::umma_commit(&sh->o_full);
+        }
+      }
+    }
+  } else {
+    // -------------------------------------------------------------------------- softmax warps
+    const int rows = warp & 3;          // tensor-memory lanes and query rows of this warp
+    const int r = rows * 32 + lane;     // query row within the tile
+    const uint32_t lane_sel = (uint32_t)(rows * 32) << 16;
+    uint8_t* line = so + r * 128;
+    constexpr float kRaise = 8.0f;      // as above
+    bool ok = !*abort_flag, stored = false;  // stored: this warp has staged rows of an item
+    int g = 0;
+    for (FaItem it = item(0); ok && it.n_tiles > 0; it = item(it.local + 1)) {
+      const int t = it.q0 + r;
+      float m_ref = -INFINITY, l_run = 0.f;
+      for (int j = 0; j < it.n_tiles; ++j, ++g) {
+        const int key0 = j * FA_BN, last_row = it.q0 + rows * 32 + 31;
+        const int halves = key0 > last_row ? 0 : key0 + 32 > last_row ? 1 : 2;  // halves of the tile that any of this warp's rows sees
+        ok = tc05::mbar_wait(&sh->s_full, (uint32_t)g & 1u, abort_flag);
+        if (!ok) break;
+        tc05::tc_fence_after_sync();
+        uint32_t sb[FA_BN];
+        if (halves > 0) tc05::tmem_ld_32x32b_x32(tmem_s + lane_sel, *reinterpret_cast<uint32_t(*)[32]>(&sb[0]));
+        if (halves > 1) tc05::tmem_ld_32x32b_x32(tmem_s + lane_sel + 32, *reinterpret_cast<uint32_t(*)[32]>(&sb[32]));
+        tc05::tmem_ld_wait();
+        tc05::tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) tc05::mbar_arrive(&sh->s_empty);
+        tc05::tmem_ld_fence(sb);
+        if (j >= it.n_tiles - 2) {  // the two tiles that hold keys q0 .. q0 + 127
+#pragma unroll
+          for (int i = 0; i < FA_BN; ++i)
+            if (key0 + i > t) sb[i] = 0xff800000u;
+        }
+        float m_tile;
+        {
+          float mx[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) mx[u] = __uint_as_float(sb[u]);
+#pragma unroll
+          for (int i = 8; i < FA_BN; ++i) mx[i & 7] = fmaxf(mx[i & 7], __uint_as_float(sb[i]));
+          m_tile = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])), fmaxf(fmaxf(mx[4], mx[5]), fmaxf(mx[6], mx[7])));
+        }
+        const float m_new = m_tile * p.scale_log2;    // finite in tile 0: key 0 is visible to every row
+        const bool raise = m_new > m_ref + kRaise;    // always true in tile 0
+        // P·V of the tile before has read P, and O may be rescaled.  Waited for as late as may be.
+        bool landed = g == 0;
+        auto wait_landed = [&]() {
+          if (!landed) ok = tc05::mbar_wait(&sh->o_full, (uint32_t)(g - 1) & 1u, abort_flag);
+          landed = true;
+          tc05::tc_fence_after_sync();
+        };
+        if (j == 0) {
+          m_ref = m_new;
+        } else if (__any_sync(0xffffffffu, raise)) {
+          wait_landed();
+          if (!ok) break;
+          const float a = raise ? ex2_fast(m_ref - m_new) : 1.0f;
+          if (raise) m_ref = m_new;
+          l_run *= a;
+#pragma unroll 1
+          for (int c = 0; c < 64; c += 8) {
+            uint32_t ob[8];
+            tc05::tmem_ld_32x32b_x8(tmem_o + lane_sel + c, ob);
+            tc05::tmem_ld_wait();
+            tc05::tmem_ld_fence(ob);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) ob[k] = __float_as_uint(__uint_as_float(ob[k]) * a);
+            tc05::tmem_st_32x32b_x8(tmem_o + lane_sel + c, ob);
+          }
+          tc05::tmem_st_wait();
+        }
+        const float neg_m = -m_ref;
+        float2 sums[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        auto half = [&](auto which, uint32_t (&w)[2][8]) {  // of P, sixteen keys each
+          constexpr int H = decltype(which)::value;
+          if (halves <= H) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) w[e / 8][e % 8] = 0u;
+            return;
+          }
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            const float2 x = fma2(make_float2(__uint_as_float(sb[H * 32 + 2 * e]), __uint_as_float(sb[H * 32 + 2 * e + 1])), both(p.scale_log2),
+                                  both(neg_m));
+            const float2 pr = make_float2(ex2_fast(x.x), ex2_fast(x.y));
+            sums[e & 1] = add2(sums[e & 1], pr);
+            w[e / 8][e % 8] = pack_bf16x2(pr.x, pr.y);
+          }
+        };
+        uint32_t w[2][8];
+        half(std::integral_constant<int, 0>{}, w);
+        wait_landed();
+        if (!ok) break;
+        tc05::tmem_st_32x32b_x8(tmem_p + lane_sel, w[0]);
+        tc05::tmem_st_32x32b_x8(tmem_p + lane_sel + 8, w[1]);
+        half(std::integral_constant<int, 1>{}, w);
+        tc05::tmem_st_32x32b_x8(tmem_p + lane_sel + 16, w[0]);
+        tc05::tmem_st_32x32b_x8(tmem_p + lane_sel + 24, w[1]);
+        l_run += (sums[0].x + sums[0].y) + (sums[1].x + sums[1].y);
+        tc05::tmem_st_wait();
+        tc05::tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) tc05::mbar_arrive(&sh->p_full);
+      }
+      if (!ok) break;
+      ok = tc05::mbar_wait(&sh->o_full, (uint32_t)(g - 1) & 1u, abort_flag);  // the last P·V
+      if (!ok) break;
+      tc05::tc_fence_after_sync();
+      if (stored) {  // the last item's
+        if (lane == 0) tc05::tma_store_wait_read();
+        __syncwarp();
+      }
+      // A warp stages its 32 rows of O (128-byte rows, 128-byte swizzle) and its lane 0 sends them with one TMA store.  Rows past T are
+      // clipped by the tensor map.
+      const float inv = 1.0f / l_run;
+#pragma unroll
+      for (int hb = 0; hb < 2; ++hb) {
+        uint32_t ob[32];
+        tc05::tmem_ld_32x32b_x32(tmem_o + lane_sel + hb * 32, ob);
+        tc05::tmem_ld_wait();
+        tc05::tmem_ld_fence(ob);
+#pragma unroll
+        for (int i = 0; i < 32; i += 8) {
+          uint4 o;
+          o.x = pack_bf16x2(__uint_as_float(ob[i]) * inv, __uint_as_float(ob[i + 1]) * inv);
+          o.y = pack_bf16x2(__uint_as_float(ob[i + 2]) * inv, __uint_as_float(ob[i + 3]) * inv);
+          o.z = pack_bf16x2(__uint_as_float(ob[i + 4]) * inv, __uint_as_float(ob[i + 5]) * inv);
+          o.w = pack_bf16x2(__uint_as_float(ob[i + 6]) * inv, __uint_as_float(ob[i + 7]) * inv);
+          *reinterpret_cast<uint4*>(line + (((hb * 4 + i / 8) ^ (r & 7)) << 4)) = o;
+        }
+      }
+      tc05::fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        tc05::tma_store_3d(&map_o, so + rows * (32 * 128), it.h * 64, it.q0 + rows * 32, it.b);
+        tc05::tma_store_commit();
+      }
+      stored = true;
+      if (t < p.T) p.lse[((size_t)it.b * p.H + it.h) * p.T + t] = (m_ref + log2f(l_run)) * 0.6931471805599453f;
+    }
+    if (lane == 0) tc05::tma_store_wait_all();  // the results have landed before shared memory goes
+  }
+
+  tc05::tc_fence_before_sync();
+  __syncthreads();
+  if (*abort_flag) {
+    for (int i = 0; i < 2000; ++i) __nanosleep(100);
+    if (threadIdx.x == 0) atomicExch(p.status + (layout_ok ? ST_WAIT_EXPIRED : ST_BAD_ARGUMENT), 1);
+  }
+  if (warp == F3_STREAMS * 4) {
+    tc05::tc_fence_after_sync();
+    tc05::tmem_dealloc(*tmem_base, 512);
+  }
+}
+
 }  // namespace
 
 int flash_attention_forward_impl(hl_ctx* ctx, const void* q, const void* k, const void* v, long long ld_qkv, void* out,
@@ -434,14 +742,17 @@ int flash_attention_forward_impl(hl_ctx* ctx, const void* q, const void* k, cons
   p.ld_out = ld_out;
   p.out = reinterpret_cast<__nv_bfloat16*>(out);
   p.lse = lse;
+  p.by_heads = QuickDiv((uint32_t)(batch * n_heads));
+  p.by_h = QuickDiv((uint32_t)n_heads);
   p.scale_log2 = (1.0f / sqrtf((float)head_dim)) * 1.4426950408889634f;
   p.status = ctx->status_dev;
   const int grid = std::min(ceil_div(time, FA_BM) * batch * n_heads, 2 * persistent_sms(ctx));
   // causal algorithmic work: QK^T and PV over the lower triangle
   ProfileScope prof(ctx, HL_PROF_ATTENTION_FWD, 2.0 * batch * n_heads * (double)time * time * head_dim);
   if (head_dim == 64) {
-    HL_ALLOW_SHARED(ctx, FaSizes<64>::SMEM_BYTES, flash_attention_fwd_kernel<64>);
-    pdl(flash_attention_fwd_kernel<64>, grid, FA_THREADS, FaSizes<64>::SMEM_BYTES, ctx->stream)(mq, mk, mv, mo, p);
+    HL_ALLOW_SHARED(ctx, F3_SMEM, flash_attention_fwd64_kernel);
+    pdl(flash_attention_fwd64_kernel, std::min(ceil_div(time, FA_BM) * batch * n_heads, persistent_sms(ctx)), F3_THREADS, F3_SMEM, ctx->stream)(
+        mq, mk, mv, mo, p);
   } else {
     HL_ALLOW_SHARED(ctx, FaSizes<128>::SMEM_BYTES, flash_attention_fwd_kernel<128>);
     pdl(flash_attention_fwd_kernel<128>, grid, FA_THREADS, FaSizes<128>::SMEM_BYTES, ctx->stream)(mq, mk, mv, mo, p);

@@ -219,6 +219,17 @@ inline size_t dtype_size(int dtype) {
 __host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 __host__ __device__ inline long long ceil_div_ll(long long a, long long b) { return (a + b - 1) / b; }
 
+// n / d for 0 <= n < 2^31 by a multiplication (Granlund and Montgomery 1994, "Division by invariant integers using multiplication"), for divisors known at launch: a division
+// takes some 200 cycles.
+struct QuickDiv {
+  uint32_t mul, shift;
+  explicit QuickDiv(uint32_t d = 1) : shift(0) {
+    while ((1ull << shift) < d) ++shift;
+    mul = (uint32_t)(((1ull << 32) * ((1ull << shift) - d)) / d + 1);
+  }
+  __device__ __forceinline__ int operator()(int n) const { return (int)((__umulhi((uint32_t)n, mul) + (uint32_t)n) >> shift); }
+};
+
 // f32 -> bf16 round-to-nearest-even (same rounding as the reference's storage.rs:440-445).
 __device__ __forceinline__ __nv_bfloat16 to_bf16(float x) { return __float2bfloat16_rn(x); }
 __device__ __forceinline__ float from_bf16(__nv_bfloat16 x) { return __bfloat162float(x); }

@@ -74,17 +74,6 @@ constexpr int TAIL_BYTES = 320;
 constexpr size_t GEMM_SMEM_BYTES = GEMM_DATA_BYTES + TAIL_BYTES + size_t(EPI_WARPS) * EPI_BIAS_BYTES;
 static_assert(GEMM_SMEM_BYTES <= 227 * 1024, "shared memory budget");
 
-// n / d for 0 <= n < 2^31 by a multiplication (Granlund and Montgomery 1994, "Division by invariant integers using multiplication"): every
-// warp role divides three times a tile, at some 200 cycles each time.
-struct QuickDiv {
-  uint32_t mul, shift;
-  explicit QuickDiv(uint32_t d = 1) : shift(0) {
-    while ((1ull << shift) < d) ++shift;
-    mul = (uint32_t)(((1ull << 32) * ((1ull << shift) - d)) / d + 1);
-  }
-  __device__ __forceinline__ int operator()(int n) const { return (int)((__umulhi((uint32_t)n, mul) + (uint32_t)n) >> shift); }
-};
-
 struct GemmParams {
   int m, n, k;
   int m_tiles, n_tiles, splits, k_blocks, k_blocks_per_split;
