@@ -1,6 +1,6 @@
 // Causal flash attention forward on tcgen05: S = Q·Kᵀ and O += P·V are tensor-memory
 // accumulators, K/V tiles stream in by TMA, the online softmax runs in registers and P goes
-// back to the tensor cores through swizzled shared memory.
+// back to the tensor cores through tensor memory.
 //
 // Replaces the reference's attention forward family — materialised [B,H,T,T] scores
 // (src/tensor.rs:4459-4472, tensor_core.ptx:1785-2283) and the mma.sync flash forward that
@@ -12,15 +12,15 @@
 // dimension (column h*hd + j, as src/tensor.rs:5156-5177), so they may live side by side in
 // one fused [B*T, 3C] projection buffer.  A work item is 128 query rows of one (batch, head).
 //
-// Pipeline: key tiles of 64; two S buffers and the O accumulator in tensor memory, P in shared memory.  Four softmax warps (one
-// per tensor-memory lane group, a thread per query row) work on tile j while the tensor cores run P·V of tile j-1 and Q·Kᵀ of
-// tile j+1.  P is formed against a reference maximum that a row raises only when its maximum has grown by more than 2^8; the row
-// then rescales its O in place (tensor-memory load, multiply, store) between two P·V products.
+// Key tiles of 64; S, P (bf16) and the O accumulator in tensor memory.  Softmax warps (one per tensor-memory lane group, a thread per
+// query row) work on tile j while the tensor cores run P·V of tile j-1 and Q·Kᵀ of tile j+1.  P is formed against a reference maximum
+// that a row raises only when its maximum has grown by more than 2^8; the row then rescales its O in place (tensor-memory load,
+// multiply, store) between two P·V products.  P goes to the tensor cores out of tensor memory: through shared memory it was a third
+// of that memory's traffic, which was three quarters of what an SM can do (heads of 128: B4 H12 T4096 211.7 us with it, now 196.6).
 //
-// Two persistent CTAs share an SM (192 threads, 112 KB of shared memory, 256 tensor-memory columns each), so that one's tensor
-// work and waits lie under the other's exponentials, and each goes through its items without a gap: while the softmax warps
-// write one item's result, the next one's first scores are being formed.  With a CTA per item (B16 H12 T1024: 69 us) 29 us were
-// starts and ends of CTAs; heads of 128 channels had one CTA an SM and nothing to hide a warp's chain under (B4 H12 T4096: 311 us).
+// Work items go round persistent streams without a gap, several of them on an SM, so that one's tensor work and waits lie under
+// another's exponentials.  Heads of 128 have room for two, a CTA each (192 threads, 112 KB of shared memory, 256 tensor-memory columns);
+// heads of 64 for three in one CTA (below).  With a CTA per item (heads of 64, B16 H12 T1024: 69 us) 29 us were starts and ends.
 #include <type_traits>
 
 #include "common.cuh"
@@ -31,34 +31,26 @@ namespace {
 
 constexpr int FA_BM = 128;   // query rows per item
 constexpr int FA_BN = 64;    // keys per tile
-constexpr int FA_P_BYTES = FA_BM * FA_BN * 2;   // 16 KB: 128 rows of 64 keys, one 128-byte line each
 constexpr int FA_SOFTMAX_WARPS = 4;
 constexpr int FA_THREADS = (FA_SOFTMAX_WARPS + 2) * 32;  // + TMA warp + MMA warp
 constexpr int FA_TMEM_COLS = 256;  // S: 2 x 64 columns, O: head_dim columns (allocations are powers of two)
 
-// Sizes that depend on the head dimension (64 or 128).  Operands wider than one 128-byte swizzle row are kept as
-// blocks of 64 channels side by side: a Q block is [128 rows x 128 bytes], a K or V block [64 keys x 128 bytes].  A head of 64
-// has room for the next item's Q and a second P; one of 128 for neither at two CTAs an SM.
-template <int HD>
-struct FaSizes {
-  static_assert(HD == 64 || HD == 128, "head_dim 64 or 128");
-  static constexpr int BLOCKS = HD / 64;
-  static constexpr int Q_BUFS = HD == 64 ? 2 : 1, P_BUFS = HD == 64 ? 2 : 1, KV_STAGES = HD == 64 ? 3 : 2;
-  static constexpr int Q_BLOCK = FA_BM * 128;            // 16 KB
-  static constexpr int KV_BLOCK = FA_BN * 128;           // 8 KB
-  static constexpr int Q_BYTES = BLOCKS * Q_BLOCK;
-  static constexpr int KV_BYTES = BLOCKS * KV_BLOCK;
-  static constexpr int SMEM_DATA = Q_BUFS * Q_BYTES + 2 * KV_STAGES * KV_BYTES + P_BUFS * FA_P_BYTES;  // 112 KB
-  static constexpr int SMEM_BYTES = SMEM_DATA + 256;     // barriers behind the tiles
-  static_assert(2 * (SMEM_BYTES + 1024) <= 228 * 1024, "shared memory per SM");
-  static_assert(2 * FA_BN + HD <= FA_TMEM_COLS, "tensor memory columns");
-};
+// Heads of 128 channels.  Operands wider than one 128-byte swizzle row are kept as blocks of 64 channels side by side: a Q block is
+// [128 rows x 128 bytes], a K or V block [64 keys x 128 bytes].
+constexpr int FA_HD = 128, FA_BLOCKS = FA_HD / 64;
+constexpr int FA_K_STAGES = 3, FA_V_STAGES = 2;
+constexpr int FA_Q_BLOCK = FA_BM * 128, FA_KV_BLOCK = FA_BN * 128;
+constexpr int FA_Q_BYTES = FA_BLOCKS * FA_Q_BLOCK, FA_KV_BYTES = FA_BLOCKS * FA_KV_BLOCK;
+constexpr int FA_DATA = FA_Q_BYTES + (FA_K_STAGES + FA_V_STAGES) * FA_KV_BYTES;  // 112 KB
+constexpr int FA_SMEM = FA_DATA + 256;                                           // barriers behind the tiles
+static_assert(2 * (FA_SMEM + 1024) <= 228 * 1024, "shared memory per SM");
+static_assert(2 * FA_BN + FA_HD <= FA_TMEM_COLS, "tensor memory columns");
 
 struct FaShared {
-  uint64_t q_full[2], q_empty[2];
-  uint64_t k_full[3], k_empty[3];
-  uint64_t v_full[3], v_empty[3];
-  uint64_t s_full[2], p_full[2], o_full[2];
+  uint64_t q_full, q_empty;
+  uint64_t k_full[FA_K_STAGES], k_empty[FA_K_STAGES];
+  uint64_t v_full[FA_V_STAGES], v_empty[FA_V_STAGES];
+  uint64_t s_full[2], p_full[2], o_full;
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -94,39 +86,36 @@ __device__ __forceinline__ FaItem fa_item(int local, const FaParams& p, int cta,
 
 __device__ __forceinline__ FaItem fa_item(int local, const FaParams& p) { return fa_item(local, p, (int)blockIdx.x, (int)gridDim.x); }
 
-template <int HD>
 __global__ void __launch_bounds__(FA_THREADS, 2)
-flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                            const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
                            const FaParams p) {
-  using Z = FaSizes<HD>;
-  constexpr int FA_HD = HD, FA_KV_STAGES = Z::KV_STAGES;
-  constexpr int FA_Q_BYTES = Z::Q_BYTES, FA_KV_BYTES = Z::KV_BYTES;
   extern __shared__ __align__(1024) uint8_t fa_smem[];  // swizzled tiles want 1024 bytes; checked below
-  uint8_t* sq = fa_smem;                          // [Q_BUFS]
-  uint8_t* sk = sq + Z::Q_BUFS * FA_Q_BYTES;
-  uint8_t* sv = sk + FA_KV_STAGES * FA_KV_BYTES;
-  uint8_t* sp = sv + FA_KV_STAGES * FA_KV_BYTES;  // [P_BUFS]
-  FaShared* sh = reinterpret_cast<FaShared*>(fa_smem + Z::SMEM_DATA);
+  uint8_t* sq = fa_smem;
+  uint8_t* sk = sq + FA_Q_BYTES;
+  uint8_t* sv = sk + FA_K_STAGES * FA_KV_BYTES;
+  FaShared* sh = reinterpret_cast<FaShared*>(fa_smem + FA_DATA);
   const bool layout_ok = (tc05::smem_u32(fa_smem) & 1023u) == 0;
   volatile int* abort_flag = &sh->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < 3; ++s) {
+    for (int s = 0; s < FA_K_STAGES; ++s) {
       tc05::mbar_init(&sh->k_full[s], 1);
       tc05::mbar_init(&sh->k_empty[s], 1);
+    }
+    for (int s = 0; s < FA_V_STAGES; ++s) {
       tc05::mbar_init(&sh->v_full[s], 1);
       tc05::mbar_init(&sh->v_empty[s], 1);
     }
     for (int i = 0; i < 2; ++i) {
-      tc05::mbar_init(&sh->q_full[i], 1);
-      tc05::mbar_init(&sh->q_empty[i], FA_SOFTMAX_WARPS);
       tc05::mbar_init(&sh->s_full[i], 1);
       tc05::mbar_init(&sh->p_full[i], FA_SOFTMAX_WARPS);
-      tc05::mbar_init(&sh->o_full[i], 1);
     }
+    tc05::mbar_init(&sh->q_full, 1);
+    tc05::mbar_init(&sh->q_empty, FA_SOFTMAX_WARPS);
+    tc05::mbar_init(&sh->o_full, 1);
     sh->abort_flag = layout_ok ? 0 : 1;
     tc05::fence_barrier_init();
   }
@@ -137,7 +126,7 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
   tc05::tc_fence_before_sync();
   __syncthreads();
   tc05::tc_fence_after_sync();
-  const uint32_t tmem_s0 = sh->tmem_base;         // S buffers at +0 and +64
+  const uint32_t tmem_s0 = sh->tmem_base;         // S buffers at +0 and +64, P over the S it is formed from
   const uint32_t tmem_o0 = tmem_s0 + 2 * FA_BN;   // O at +128
   pdl_begin();  // everything above touches nothing a predecessor wrote
 
@@ -150,28 +139,26 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       bool ok = true;
       int g = 0;  // key tiles loaded so far
       for (FaItem it = fa_item(0, p); ok && it.n_tiles > 0; it = fa_item(it.local + 1, p)) {
-        const int qb = it.local % Z::Q_BUFS;
-        if (!tc05::mbar_wait(&sh->q_empty[qb], ((uint32_t)(it.local / Z::Q_BUFS) & 1u) ^ 1u, abort_flag)) break;
-        tc05::mbar_arrive_expect_tx(&sh->q_full[qb], FA_Q_BYTES);
+        if (!tc05::mbar_wait(&sh->q_empty, ((uint32_t)it.local & 1u) ^ 1u, abort_flag)) break;
+        tc05::mbar_arrive_expect_tx(&sh->q_full, FA_Q_BYTES);
 #pragma unroll
-        for (int blk = 0; blk < Z::BLOCKS; ++blk)
-          tc05::tma_load_3d(sq + qb * FA_Q_BYTES + blk * Z::Q_BLOCK, &map_q, &sh->q_full[qb], it.h * FA_HD + blk * 64, it.q0, it.b);
+        for (int blk = 0; blk < FA_BLOCKS; ++blk)
+          tc05::tma_load_3d(sq + blk * FA_Q_BLOCK, &map_q, &sh->q_full, it.h * FA_HD + blk * 64, it.q0, it.b);
         for (int j = 0; j < it.n_tiles; ++j, ++g) {
-          const int s = g % FA_KV_STAGES;
-          const uint32_t ph = (uint32_t)(g / FA_KV_STAGES) & 1u;
-          ok = tc05::mbar_wait(&sh->k_empty[s], ph ^ 1u, abort_flag);
+          const int s = g % FA_K_STAGES, vs = g % FA_V_STAGES;
+          ok = tc05::mbar_wait(&sh->k_empty[s], ((uint32_t)(g / FA_K_STAGES) & 1u) ^ 1u, abort_flag);
           if (!ok) break;
           tc05::mbar_arrive_expect_tx(&sh->k_full[s], FA_KV_BYTES);
 #pragma unroll
-          for (int blk = 0; blk < Z::BLOCKS; ++blk)
-            tc05::tma_load_3d(sk + s * FA_KV_BYTES + blk * Z::KV_BLOCK, &map_k, &sh->k_full[s], it.h * FA_HD + blk * 64,
+          for (int blk = 0; blk < FA_BLOCKS; ++blk)
+            tc05::tma_load_3d(sk + s * FA_KV_BYTES + blk * FA_KV_BLOCK, &map_k, &sh->k_full[s], it.h * FA_HD + blk * 64,
                               j * FA_BN, it.b);
-          ok = tc05::mbar_wait(&sh->v_empty[s], ph ^ 1u, abort_flag);
+          ok = tc05::mbar_wait(&sh->v_empty[vs], ((uint32_t)(g / FA_V_STAGES) & 1u) ^ 1u, abort_flag);
           if (!ok) break;
-          tc05::mbar_arrive_expect_tx(&sh->v_full[s], FA_KV_BYTES);
+          tc05::mbar_arrive_expect_tx(&sh->v_full[vs], FA_KV_BYTES);
 #pragma unroll
-          for (int blk = 0; blk < Z::BLOCKS; ++blk)
-            tc05::tma_load_3d(sv + s * FA_KV_BYTES + blk * Z::KV_BLOCK, &map_v, &sh->v_full[s], it.h * FA_HD + blk * 64,
+          for (int blk = 0; blk < FA_BLOCKS; ++blk)
+            tc05::tma_load_3d(sv + vs * FA_KV_BYTES + blk * FA_KV_BLOCK, &map_v, &sh->v_full[vs], it.h * FA_HD + blk * 64,
                               j * FA_BN, it.b);
         }
       }
@@ -186,16 +173,16 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       int qj = 0, qg = 0;  // the next scores: tile of the item, tile of the CTA
       auto issue_qk = [&]() -> bool {  // S[qg & 1] = Q · K(qj)ᵀ
         if (qi.n_tiles == 0) return true;
-        const int qb = qi.local % Z::Q_BUFS, s = qg % FA_KV_STAGES;
-        if (qj == 0 && !tc05::mbar_wait(&sh->q_full[qb], (uint32_t)(qi.local / Z::Q_BUFS) & 1u, abort_flag)) return false;
-        if (!tc05::mbar_wait(&sh->k_full[s], (uint32_t)(qg / FA_KV_STAGES) & 1u, abort_flag)) return false;
+        const int s = qg % FA_K_STAGES;
+        if (qj == 0 && !tc05::mbar_wait(&sh->q_full, (uint32_t)qi.local & 1u, abort_flag)) return false;
+        if (!tc05::mbar_wait(&sh->k_full[s], (uint32_t)(qg / FA_K_STAGES) & 1u, abort_flag)) return false;
         tc05::tc_fence_after_sync();
-        const uint32_t aq = tc05::smem_u32(sq + qb * FA_Q_BYTES), ak = tc05::smem_u32(sk + s * FA_KV_BYTES);
+        const uint32_t aq = tc05::smem_u32(sq), ak = tc05::smem_u32(sk + s * FA_KV_BYTES);
 #pragma unroll
         for (int ks = 0; ks < FA_HD / 16; ++ks)  // 16 channels a step; four steps per 64-channel block
           tc05::umma_ss(tmem_s0 + (uint32_t)((qg & 1) * FA_BN),
-                        tc05::smem_desc_sw128(aq + (ks / 4) * Z::Q_BLOCK + (ks % 4) * 32, 16, 1024),
-                        tc05::smem_desc_sw128(ak + (ks / 4) * Z::KV_BLOCK + (ks % 4) * 32, 16, 1024), idesc_qk,
+                        tc05::smem_desc_sw128(aq + (ks / 4) * FA_Q_BLOCK + (ks % 4) * 32, 16, 1024),
+                        tc05::smem_desc_sw128(ak + (ks / 4) * FA_KV_BLOCK + (ks % 4) * 32, 16, 1024), idesc_qk,
                         ks > 0 ? 1u : 0u);
         tc05::umma_commit(&sh->k_empty[s]);
         tc05::umma_commit(&sh->s_full[qg & 1]);
@@ -207,9 +194,9 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         return true;
       };
       bool ok = issue_qk();
-      // A single Q buffer is overwritten once the item's result has left through it, which the softmax warps do after the last
-      // P·V: the scores of the next item then wait until those have been issued.
-      auto may_run_ahead = [&]() { return Z::Q_BUFS == 2 || qj > 0; };
+      // Q is overwritten once the item's result has left through its place, which the softmax warps do after the last P·V: the scores of
+      // the next item wait until those have been issued.
+      auto may_run_ahead = [&]() { return qj > 0; };
       int ahead = 1;  // scores issued beyond the tile at hand
       int g = 0;
       for (FaItem it = fa_item(0, p); ok && it.n_tiles > 0; it = fa_item(it.local + 1, p)) {
@@ -219,26 +206,24 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             ++ahead;
           }
           if (!ok) break;
-          // P(g) is in shared memory, which also means S(g) has been read out of tensor memory and, in an item's first tile, the
-          // last item's O as well
-          if (!tc05::mbar_wait(&sh->p_full[g % Z::P_BUFS], (uint32_t)(g / Z::P_BUFS) & 1u, abort_flag)) { ok = false; break; }
+          // P(g) stands in S(g)'s columns and, in an item's first tile, the last item's O has been read.  The scores two tiles on take the
+          // same columns; they are queued behind the product that reads P.
+          if (!tc05::mbar_wait(&sh->p_full[g & 1], (uint32_t)(g >> 1) & 1u, abort_flag)) { ok = false; break; }
           tc05::tc_fence_after_sync();
-          const int s = g % FA_KV_STAGES;
-          if (!tc05::mbar_wait(&sh->v_full[s], (uint32_t)(g / FA_KV_STAGES) & 1u, abort_flag)) { ok = false; break; }
+          const int s = g % FA_V_STAGES;
+          if (!tc05::mbar_wait(&sh->v_full[s], (uint32_t)(g / FA_V_STAGES) & 1u, abort_flag)) { ok = false; break; }
           tc05::tc_fence_after_sync();
           const uint32_t av = tc05::smem_u32(sv + s * FA_KV_BYTES);
-          const uint32_t ap = tc05::smem_u32(sp + (g % Z::P_BUFS) * FA_P_BYTES);
 #pragma unroll
           for (int ks = 0; ks < FA_BN / 16; ++ks) {
-            // A = P: [128 rows x 64 keys], K-major; B = V: rows are keys (MN-major), 16 keys per step
-            const uint64_t da = tc05::smem_desc_sw128(ap + ks * 32, 16, 1024);
-            const uint64_t db = tc05::smem_desc_sw128(av + ks * (16 * 128), Z::KV_BLOCK, 1024);  // channel blocks KV_BLOCK apart
-            tc05::umma_ss(tmem_o0, da, db, idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);  // O accumulates over the key tiles
+            // A = P, two keys a column; B = V: rows are keys (MN-major), 16 keys per step, channel blocks FA_KV_BLOCK apart
+            const uint64_t db = tc05::smem_desc_sw128(av + ks * (16 * 128), FA_KV_BLOCK, 1024);
+            tc05::umma_ts(tmem_o0, tmem_s0 + (uint32_t)((g & 1) * FA_BN + ks * 8), db, idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
           }
           tc05::umma_commit(&sh->v_empty[s]);
-          tc05::umma_commit(&sh->o_full[g % Z::P_BUFS]);
+          tc05::umma_commit(&sh->o_full);
           --ahead;
-          if (ahead < 1 && qi.n_tiles > 0) {  // a single Q buffer, at the end of an item
+          if (ahead < 1 && qi.n_tiles > 0) {  // at the end of an item
             ok = issue_qk();
             ++ahead;
           }
@@ -254,7 +239,6 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     // precision) and f32 sums nothing, and O is rescaled in place a few times per row instead of once per tile.
     constexpr float kRaise = 8.0f;
     bool ok = !*abort_flag;
-    bool stored = false;  // this warp's rows of the last item are on their way out of its Q buffer
     int g = 0;            // key tiles done so far
 
     for (FaItem it = fa_item(0, p); ok && it.n_tiles > 0; it = fa_item(it.local + 1, p)) {
@@ -292,7 +276,7 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       } else if (__any_sync(0xffffffffu, raise)) {
         // rows of this warp rescale their O in place; P·V of tile j-1 must have landed, and P·V of tile j is not
         // issued before this warp has handed over P(j)
-        if (!tc05::mbar_wait(&sh->o_full[(g - 1) % Z::P_BUFS], (uint32_t)((g - 1) / Z::P_BUFS) & 1u, abort_flag)) { ok = false; break; }
+        if (!tc05::mbar_wait(&sh->o_full, (uint32_t)(g - 1) & 1u, abort_flag)) { ok = false; break; }
         tc05::tc_fence_after_sync();
         const float a = raise ? ex2_fast(m_ref - m_new) : 1.0f;
         if (raise) m_ref = m_new;
@@ -309,40 +293,30 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         tc05::tmem_st_wait();
       }
       const float neg_m = -m_ref;
-      // the P·V that read this P buffer has finished
-      if (g >= Z::P_BUFS && !tc05::mbar_wait(&sh->o_full[g % Z::P_BUFS], (uint32_t)((g - Z::P_BUFS) / Z::P_BUFS) & 1u, abort_flag)) { ok = false; break; }
-      uint8_t* line = sp + (g % Z::P_BUFS) * FA_P_BYTES + r * 128;
-      float l_tile = 0.f;
+      const uint32_t tp = tmem_s0 + (uint32_t)((g & 1) * FA_BN) + lane_sel;
+      float2 sums[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        uint32_t w[4];
+      for (int q = 0; q < 4; ++q) {  // sixteen keys
+        uint32_t w[8];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 x = fma2(make_float2(__uint_as_float(sb[q * 8 + 2 * e]), __uint_as_float(sb[q * 8 + 2 * e + 1])),
+        for (int e = 0; e < 8; ++e) {
+          const float2 x = fma2(make_float2(__uint_as_float(sb[q * 16 + 2 * e]), __uint_as_float(sb[q * 16 + 2 * e + 1])),
                                 both(p.scale_log2), both(neg_m));
           const float2 pr = make_float2(ex2_fast(x.x), ex2_fast(x.y));
-          l_tile += pr.x + pr.y;
+          sums[e & 1] = add2(sums[e & 1], pr);
           w[e] = pack_bf16x2(pr.x, pr.y);
         }
-        *reinterpret_cast<uint4*>(line + ((q ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        tc05::tmem_st_32x32b_x8(tp + q * 8, w);
       }
-      l_run += l_tile;
-      tc05::fence_proxy_async_smem();
+      l_run += (sums[0].x + sums[0].y) + (sums[1].x + sums[1].y);
+      tc05::tmem_st_wait();
       tc05::tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) {
-        tc05::mbar_arrive(&sh->p_full[g % Z::P_BUFS]);
-        if (stored) {  // the last item's rows have left its Q buffer
-          tc05::tma_store_wait_read();
-          tc05::mbar_arrive(&sh->q_empty[(it.local - 1) % Z::Q_BUFS]);
-        }
-      }
-      if (Z::Q_BUFS == 2) stored = false;
+      if (lane == 0) tc05::mbar_arrive(&sh->p_full[g & 1]);
     }
     if (!ok) break;
-    ok = tc05::mbar_wait(&sh->o_full[(g - 1) % Z::P_BUFS], (uint32_t)((g - 1) / Z::P_BUFS) & 1u, abort_flag);  // the last P·V
+    ok = tc05::mbar_wait(&sh->o_full, (uint32_t)(g - 1) & 1u, abort_flag);  // the last P·V
     tc05::tc_fence_after_sync();
-    uint8_t* so = sq + (it.local % Z::Q_BUFS) * FA_Q_BYTES;
     if (ok) {
       // O leaves through the Q tile's shared memory (every product that read Q has finished): a warp stages its 32
       // rows per 64-channel block (128-byte rows, 128-byte swizzle) and its lane 0 sends them with one TMA store, whole
@@ -354,7 +328,7 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         uint32_t ob[32];
         tc05::tmem_ld_32x32b_x32(tmem_o0 + lane_sel + hb * 32, ob);
         tc05::tmem_ld_wait();
-        uint8_t* line = so + (hb / 2) * Z::Q_BLOCK + r * 128;
+        uint8_t* line = sq + (hb / 2) * FA_Q_BLOCK + r * 128;
 #pragma unroll
         for (int i = 0; i < 32; i += 8) {
           uint4 o;
@@ -370,15 +344,12 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
       __syncwarp();
       if (lane == 0) {
 #pragma unroll
-        for (int blk = 0; blk < Z::BLOCKS; ++blk)
-          tc05::tma_store_3d(&map_o, so + blk * Z::Q_BLOCK + warp * (32 * 128), it.h * FA_HD + blk * 64, it.q0 + warp * 32, it.b);
+        for (int blk = 0; blk < FA_BLOCKS; ++blk)
+          tc05::tma_store_3d(&map_o, sq + blk * FA_Q_BLOCK + warp * (32 * 128), it.h * FA_HD + blk * 64, it.q0 + warp * 32, it.b);
         tc05::tma_store_commit();
-        if (Z::Q_BUFS == 1) {  // the next item's Q waits for it
-          tc05::tma_store_wait_read();
-          tc05::mbar_arrive(&sh->q_empty[0]);
-        }
+        tc05::tma_store_wait_read();  // the next item's Q waits for it
+        tc05::mbar_arrive(&sh->q_empty);
       }
-      stored = Z::Q_BUFS == 2;
     }
     if (ok && t < p.T) {
       // natural-log log-sum-exp of the scaled scores
@@ -403,10 +374,12 @@ flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
 // ---- heads of 64 channels ---------------------------------------------------------------------------------------------------
 // What bounds these is the softmax: 64 exponentials a row and tile are 512 cycles of a scheduler's, the products 256.  A warp's chain (scores,
 // maximum, exponentials, hand-over) takes three times that, so that three warps share a scheduler: one CTA an SM walks three streams
-// of items side by side, each with its own tiles, four softmax warps and a warp whose elected thread queues both loads and products.
+// of items side by side, each with its own tiles, four softmax warps and a warp whose elected thread queues both loads and products
+// (B16 H12 T1024: two CTAs of four softmax warps 62.8 us, three streams 58.3, P in tensor memory 55.2, its place waited for when half of
+// P has been formed 52.5; B4 H12 T4096 175.5, 176.5, 164.5, 153.7).
 // That thread waits for scores that have been read and P that has been written, and for nothing else: when S(g) has been read, Q·K(g)
 // is done and K(g) can be replaced; when P(g) has been written, P·V(g-1) is done and V(g-1) can.
-// A stream has one S and one O in tensor memory (128 columns), one Q, one P (through which the result leaves), three K, two V: 72 KB.
+// A stream has S, P and O in tensor memory (160 columns), and Q, a place for the result, three K and two V in shared memory: 72 KB.
 constexpr int F3_STREAMS = 3;
 constexpr int F3_THREADS = F3_STREAMS * 5 * 32;
 constexpr int F3_K_STAGES = 3, F3_V_STAGES = 2;
@@ -754,8 +727,8 @@ int flash_attention_forward_impl(hl_ctx* ctx, const void* q, const void* k, cons
     pdl(flash_attention_fwd64_kernel, std::min(ceil_div(time, FA_BM) * batch * n_heads, persistent_sms(ctx)), F3_THREADS, F3_SMEM, ctx->stream)(
         mq, mk, mv, mo, p);
   } else {
-    HL_ALLOW_SHARED(ctx, FaSizes<128>::SMEM_BYTES, flash_attention_fwd_kernel<128>);
-    pdl(flash_attention_fwd_kernel<128>, grid, FA_THREADS, FaSizes<128>::SMEM_BYTES, ctx->stream)(mq, mk, mv, mo, p);
+    HL_ALLOW_SHARED(ctx, FA_SMEM, flash_attention_fwd128_kernel);
+    pdl(flash_attention_fwd128_kernel, grid, FA_THREADS, FA_SMEM, ctx->stream)(mq, mk, mv, mo, p);
   }
   HL_LAUNCH_CHECK("flash_attention_fwd_kernel");
   count_launch(ctx);

@@ -223,7 +223,7 @@ __host__ __device__ inline long long ceil_div_ll(long long a, long long b) { ret
 // takes some 200 cycles.
 struct QuickDiv {
   uint32_t mul, shift;
-  explicit QuickDiv(uint32_t d = 1) : shift(0) {
+  QuickDiv(uint32_t d = 1) : shift(0) {
     while ((1ull << shift) < d) ++shift;
     mul = (uint32_t)(((1ull << 32) * ((1ull << shift) - d)) / d + 1);
   }
