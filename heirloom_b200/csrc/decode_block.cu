@@ -142,12 +142,33 @@ __device__ __forceinline__ Acc sum_of_warps(const Acc* red, int rows, int r) {
   return s;
 }
 
-// `bytes` (whole sixteens) of this CTA's shared memory to the same place in a peer's, by one warp.  A store to a peer takes its turn
-// whatever its width: 96 of 32 bytes held a kernel up for 3300 cycles.
-__device__ __forceinline__ void push(cg::cluster_group& cluster, void* to, const void* from, int bytes, int peer) {
+// What the peers of a cluster send arrives on barriers that count its bytes: a barrier of the cluster behind the stores cost a release,
+// that is, waiting for every store's answer, and the barrier's own way there and back.
+struct Mail {
+  uint64_t arrived[2];
+  int abort_flag;
+  __device__ __forceinline__ void open(int bytes0, int bytes1) {  // by one thread, before the cluster meets
+    tc05::mbar_init(&arrived[0], 1);
+    tc05::mbar_init(&arrived[1], 1);
+    abort_flag = 0;
+    tc05::fence_barrier_init();
+    if (bytes0) tc05::mbar_arrive_expect_tx(&arrived[0], bytes0);
+    if (bytes1) tc05::mbar_arrive_expect_tx(&arrived[1], bytes1);
+  }
+  __device__ __forceinline__ void wait(int i, int* status) {
+    if (!tc05::mbar_wait(&arrived[i], 0, &abort_flag)) *status = 1;
+  }
+};
+// `bytes` (whole sixteens) of this CTA's shared memory into a peer's, by one warp.  A store to a peer takes its turn whatever its width:
+// 96 of 32 bytes held a kernel up for 3300 cycles.
+__device__ __forceinline__ void push(uint64_t* arrived, void* to, const void* from, int bytes, int peer) {
+  const uint32_t there = tc05::cluster_map_shared(to, peer), bar = tc05::cluster_map_shared(arrived, peer);
 #pragma unroll 1
-  for (int b = (threadIdx.x & 31) * 16; b < bytes; b += 32 * 16)
-    *reinterpret_cast<uint4*>(cluster.map_shared_rank(static_cast<char*>(to) + b, peer)) = *reinterpret_cast<const uint4*>(static_cast<const char*>(from) + b);
+  for (int b = (threadIdx.x & 31) * 16; b < bytes; b += 32 * 16) {
+    const uint4 v = *reinterpret_cast<const uint4*>(static_cast<const char*>(from) + b);
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(there + b), "r"(v.x), "r"(v.y),
+                 "r"(v.z), "r"(v.w), "r"(bar) : "memory");
+  }
 }
 
 // The residual stream's row, rounded where the full-window kernels round it, and its layer norm.  Every CTA forms it for itself, a
@@ -268,12 +289,14 @@ struct AttentionArgs {
   void* parts;  // [heads][d]
   int d, hd, cap;
   bool window;
+  int* status;
 };
 
 template <typename T, typename Acc>
 __global__ void __launch_bounds__(DB_THREADS, 2) decode_attention_block_kernel(const __grid_constant__ AttentionArgs a) {
   extern __shared__ __align__(16) unsigned char db_smem[];
   __shared__ Acc norm[2 * DB_WARPS], red_max[DB_WARPS], red_sum[DB_WARPS];
+  __shared__ Mail mail;
   constexpr int PN = Pack<T>::N, PAD = row_pad<T>;
   const int d = a.d, hd = a.hd, cpc = hd / DB_CTAS, opc = d / DB_CTAS, rows = 3 * cpc;
   const AttentionLayout<T, Acc> at(d, hd, a.cap, a.window);
@@ -290,11 +313,11 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_attention_block_kernel(c
   Acc* part = reinterpret_cast<Acc*>(db_smem + at.part);        // [warps][hd]
   Acc* all = reinterpret_cast<Acc*>(db_smem + at.all);          // [CTAs][pitch_all] values, maximum, sum
   T* att = reinterpret_cast<T*>(db_smem + at.att);
-  cg::cluster_group cluster = cg::this_cluster();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rank = (int)(blockIdx.x % DB_CTAS), h = (int)(blockIdx.x / DB_CTAS);
   const long long ld = 3 * d;
   T* qkv = static_cast<T*>(a.qkv) + h * hd;
   pdl_trigger();
+  if (threadIdx.x == 0) mail.open(a.window ? 0 : (DB_CTAS - 1) * pitch_fresh * 4, (DB_CTAS - 1) * pitch_all * (int)sizeof(Acc));
   // The position was copied here before the first kernel of the sequence started.
   const int t = (int)a.state[0], keys = t + 1, chunk = (keys + DB_CTAS - 1) / DB_CTAS;
   const int k0 = min(keys, rank * chunk), k1 = min(keys, k0 + chunk);
@@ -333,10 +356,10 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_attention_block_kernel(c
     float y = 0.f;
     if (const int i = threadIdx.x; i < rows) own[i] = y = rounded<T>((float)product_of_row(red, rows, i) + bias[i]);
     __syncthreads();
-    if (warp < DB_CTAS && warp != rank) push(cluster, own, own, pitch_fresh * 4, warp);
+    if (warp < DB_CTAS && warp != rank) push(&mail.arrived[0], own, own, pitch_fresh * 4, warp);
     cp_async_wait_all();
-    cluster.sync();
-    if (const int i = threadIdx.x; i < rows) {  // (in front of the barrier it would wait for these stores)
+    mail.wait(0, a.status);
+    if (const int i = threadIdx.x; i < rows) {  // (nobody waits for these)
       const int which = i < cpc ? 0 : i < 2 * cpc ? 1 : 2;
       qkv[(long long)t * ld + which * d + rank * cpc + i - which * cpc] = stored<T>(y);
     }
@@ -415,8 +438,8 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_attention_block_kernel(c
   Acc* own = all + rank * pitch_all;
   if (const int c = threadIdx.x; c < hd + 2) own[c] = c == hd ? mx : sum_of_warps(c < hd ? part : red_sum, c < hd ? hd : 1, c < hd ? c : 0);
   __syncthreads();
-  if (warp < DB_CTAS && warp != rank) push(cluster, own, own, pitch_all * sizeof(Acc), warp);
-  cluster.sync();
+  if (warp < DB_CTAS && warp != rank) push(&mail.arrived[1], own, own, pitch_all * sizeof(Acc), warp);
+  mail.wait(1, a.status);
   {
     const Acc* mine = all + (lane & 7) * pitch_all + hd;
     const Acc m = mine[0];
@@ -471,12 +494,14 @@ struct FeedForwardArgs {
   const void* w2;
   void* parts;  // [clusters][d]
   int d, hidden, units;  // units: hidden units a CTA
+  int* status;
 };
 
 template <typename T, typename Acc>
 __global__ void __launch_bounds__(DB_THREADS, 2) decode_feed_forward_kernel(const __grid_constant__ FeedForwardArgs a) {
   extern __shared__ __align__(16) unsigned char db_smem[];
   __shared__ Acc norm[2 * DB_WARPS];
+  __shared__ Mail mail;
   constexpr int PAD = row_pad<T>;
   const int d = a.d, opc = d / DB_CTAS, units = a.units;
   const FeedForwardLayout<T, Acc> at(d, units);
@@ -489,10 +514,10 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_feed_forward_kernel(cons
   const int pitch_sums = at.pitch_sums;
   Acc* outputs = reinterpret_cast<Acc*>(db_smem + at.outputs);  // [CTAs][pitch_sums] this CTA's part of every output, a peer's together
   Acc* sums = reinterpret_cast<Acc*>(db_smem + at.sums);        // [CTAs][pitch_sums] the peers' parts of this CTA's outputs
-  cg::cluster_group cluster = cg::this_cluster();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rank = (int)(blockIdx.x % DB_CTAS);
+  const int warp = threadIdx.x >> 5, rank = (int)(blockIdx.x % DB_CTAS);
   const int first = min(a.hidden, (int)blockIdx.x * units), n = min(units, a.hidden - first);  // n may be 0
   pdl_trigger();
+  if (threadIdx.x == 0) mail.open(DB_CTAS * pitch_sums * (int)sizeof(Acc), 0);
   stage_rows(w1, (d + PAD) * sizeof(T), static_cast<const T*>(a.w1) + (size_t)first * d, d * sizeof(T), n, d * sizeof(T));
   if ((int)threadIdx.x < n) cp_async4(bias + threadIdx.x, a.b1 + first + threadIdx.x);
   cp_async_commit();
@@ -524,8 +549,8 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_feed_forward_kernel(cons
     outputs[owner * pitch_sums + c - owner * opc] = v;
   });
   __syncthreads();
-  if (warp < DB_CTAS) push(cluster, sums + rank * pitch_sums, outputs + warp * pitch_sums, pitch_sums * sizeof(Acc), warp);
-  cluster.sync();
+  if (warp < DB_CTAS) push(&mail.arrived[0], sums + rank * pitch_sums, outputs + warp * pitch_sums, pitch_sums * sizeof(Acc), warp);
+  mail.wait(0, a.status);
   Acc* out = static_cast<Acc*>(a.parts) + (size_t)(blockIdx.x / DB_CTAS) * d + rank * opc;
   if (const int c = threadIdx.x; c < opc) {
     Acc s = 0;
@@ -644,7 +669,7 @@ bool block_fits(int d, int heads, int hidden, int context) {
 template <typename T, typename Acc>
 int run_attention(hl_ctx* ctx, const DecodeBlock& b) {
   AttentionArgs a{b.x, b.ln1_gamma, b.ln1_beta, b.wqkv, b.bqkv, b.qkv, b.state, b.wo, b.attention_parts, b.d, b.d / b.heads,
-                  ceil_div(b.context, DB_CTAS), b.window};
+                  ceil_div(b.context, DB_CTAS), b.window, ctx->status_dev + ST_WAIT_EXPIRED};
   const AttentionLayout<T, Acc> at(a.d, a.hd, a.cap, a.window);
   auto kern = decode_attention_block_kernel<T, Acc>;
   HL_ALLOW_SHARED(ctx, DB_MAX_SHARED, kern);
@@ -655,7 +680,7 @@ int run_attention(hl_ctx* ctx, const DecodeBlock& b) {
 
 template <typename T, typename Acc>
 int run_feed_forward(hl_ctx* ctx, const DecodeBlock& b, const DecodeRow& x, int units, int clusters) {
-  FeedForwardArgs a{x, b.ln2_gamma, b.ln2_beta, b.w1, b.b1, b.w2, b.feed_forward_parts, b.d, b.hidden, units};
+  FeedForwardArgs a{x, b.ln2_gamma, b.ln2_beta, b.w1, b.b1, b.w2, b.feed_forward_parts, b.d, b.hidden, units, ctx->status_dev + ST_WAIT_EXPIRED};
   const FeedForwardLayout<T, Acc> at(a.d, units);
   auto kern = decode_feed_forward_kernel<T, Acc>;
   HL_ALLOW_SHARED(ctx, DB_MAX_SHARED, kern);
