@@ -16,7 +16,7 @@
 // query row) work on tile j while the tensor cores run P·V of tile j-1 and Q·Kᵀ of tile j+1.  P is formed against a reference maximum
 // that a row raises only when its maximum has grown by more than 2^8; the row then rescales its O in place (tensor-memory load,
 // multiply, store) between two P·V products.  P goes to the tensor cores out of tensor memory: through shared memory it was a third
-// of that memory's traffic, which was three quarters of what an SM can do (heads of 128: B4 H12 T4096 211.7 us with it, now 196.6).
+// of that memory's traffic, which was three quarters of what an SM can do (heads of 128: B4 H12 T4096 211.7 us with it, now 197.1).
 //
 // Work items go round persistent streams without a gap, several of them on an SM, so that one's tensor work and waits lie under
 // another's exponentials.  Heads of 128 have room for two, a CTA each (192 threads, 112 KB of shared memory, 256 tensor-memory columns);
@@ -50,7 +50,7 @@ struct FaShared {
   uint64_t q_full, q_empty;
   uint64_t k_full[FA_K_STAGES], k_empty[FA_K_STAGES];
   uint64_t v_full[FA_V_STAGES], v_empty[FA_V_STAGES];
-  uint64_t s_full[2], p_full[2], o_full;
+  uint64_t s_full[2], p_full[2], o_full[2];  // by tile
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -112,10 +112,10 @@ flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
     for (int i = 0; i < 2; ++i) {
       tc05::mbar_init(&sh->s_full[i], 1);
       tc05::mbar_init(&sh->p_full[i], FA_SOFTMAX_WARPS);
+      tc05::mbar_init(&sh->o_full[i], 1);
     }
     tc05::mbar_init(&sh->q_full, 1);
     tc05::mbar_init(&sh->q_empty, FA_SOFTMAX_WARPS);
-    tc05::mbar_init(&sh->o_full, 1);
     sh->abort_flag = layout_ok ? 0 : 1;
     tc05::fence_barrier_init();
   }
@@ -176,6 +176,8 @@ flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
         const int s = qg % FA_K_STAGES;
         if (qj == 0 && !tc05::mbar_wait(&sh->q_full, (uint32_t)qi.local & 1u, abort_flag)) return false;
         if (!tc05::mbar_wait(&sh->k_full[s], (uint32_t)(qg / FA_K_STAGES) & 1u, abort_flag)) return false;
+        // P·V of two tiles before reads the P that stands here: products of other sizes are not kept in order
+        if (qg >= 2 && !tc05::mbar_wait(&sh->o_full[qg & 1], (uint32_t)((qg - 2) >> 1) & 1u, abort_flag)) return false;
         tc05::tc_fence_after_sync();
         const uint32_t aq = tc05::smem_u32(sq), ak = tc05::smem_u32(sk + s * FA_KV_BYTES);
 #pragma unroll
@@ -206,8 +208,7 @@ flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
             ++ahead;
           }
           if (!ok) break;
-          // P(g) stands in S(g)'s columns and, in an item's first tile, the last item's O has been read.  The scores two tiles on take the
-          // same columns; they are queued behind the product that reads P.
+          // P(g) stands in S(g)'s columns and, in an item's first tile, the last item's O has been read
           if (!tc05::mbar_wait(&sh->p_full[g & 1], (uint32_t)(g >> 1) & 1u, abort_flag)) { ok = false; break; }
           tc05::tc_fence_after_sync();
           const int s = g % FA_V_STAGES;
@@ -221,7 +222,7 @@ flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
             tc05::umma_ts(tmem_o0, tmem_s0 + (uint32_t)((g & 1) * FA_BN + ks * 8), db, idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
           }
           tc05::umma_commit(&sh->v_empty[s]);
-          tc05::umma_commit(&sh->o_full);
+          tc05::umma_commit(&sh->o_full[g & 1]);
           --ahead;
           if (ahead < 1 && qi.n_tiles > 0) {  // at the end of an item
             ok = issue_qk();
@@ -276,7 +277,7 @@ flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
       } else if (__any_sync(0xffffffffu, raise)) {
         // rows of this warp rescale their O in place; P·V of tile j-1 must have landed, and P·V of tile j is not
         // issued before this warp has handed over P(j)
-        if (!tc05::mbar_wait(&sh->o_full, (uint32_t)(g - 1) & 1u, abort_flag)) { ok = false; break; }
+        if (!tc05::mbar_wait(&sh->o_full[(g - 1) & 1], (uint32_t)((g - 1) >> 1) & 1u, abort_flag)) { ok = false; break; }
         tc05::tc_fence_after_sync();
         const float a = raise ? ex2_fast(m_ref - m_new) : 1.0f;
         if (raise) m_ref = m_new;
@@ -315,7 +316,7 @@ flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
       if (lane == 0) tc05::mbar_arrive(&sh->p_full[g & 1]);
     }
     if (!ok) break;
-    ok = tc05::mbar_wait(&sh->o_full, (uint32_t)(g - 1) & 1u, abort_flag);  // the last P·V
+    ok = tc05::mbar_wait(&sh->o_full[(g - 1) & 1], (uint32_t)((g - 1) >> 1) & 1u, abort_flag);  // the last P·V
     tc05::tc_fence_after_sync();
     if (ok) {
       // O leaves through the Q tile's shared memory (every product that read Q has finished): a warp stages its 32

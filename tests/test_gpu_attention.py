@@ -40,6 +40,46 @@ def test_flash_forward_matches_oracle(B, T, H, hd):
     assert_close("lse", host(lse), reference_lse(qn, kn, H), atol=1e-4, rtol=1e-5)
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("B,T,H", [(1, 1, 1), (2, 33, 1), (1, 65, 3), (3, 97, 2), (1, 129, 2), (90, 64, 5), (40, 200, 6)])
+def test_flash_forward_of_streams_with_several_items_and_rising_scores(B, T, H, hd):
+    """Items fewer and more than the streams of the chip, tiles of which a warp's rows see none, one or both halves, and scores that grow
+    along the keys, so that rows raise the maximum that P is formed against (by far more than 2^8) in most tiles.  Bounds as above: P has
+    one bf16 rounding, whatever it is formed against."""
+    from heirloom_b200 import cuda
+    c = ctx()
+    C = hd * H
+    rng = np.random.default_rng(T + H)
+    qkv = rng.standard_normal((B, T, 3 * C)) * 1.2
+    qkv[..., C:2 * C] = 0.1 * qkv[..., C:2 * C] + np.linspace(0, 4, T)[None, :, None]
+    qkv[..., :C] = np.abs(qkv[..., :C])
+    qkv = ho.bf16_round(qkv.reshape(B * T, 3 * C))
+    fused = dev(qkv, torch.bfloat16)
+    out, lse = cuda.flash_attention_forward(c, fused[:, :C], fused[:, C:2 * C], fused[:, 2 * C:], B, T, H)
+    qn, kn, vn = (qkv[:, i * C:(i + 1) * C].reshape(B, T, C) for i in range(3))
+    want = ho.causal_attention(qn, kn, vn, H, round_probs_bf16=True)
+    assert_close("flash out", host(out).reshape(B, T, C), want, atol=1e-2, rtol=2 ** -6)
+    assert_close("lse", host(lse), reference_lse(qn, kn, H), atol=1e-4, rtol=1e-5)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("B,T,H", [(4, 4096, 12), (64, 300, 8)])
+def test_flash_forward_gives_the_same_bits_every_time(B, T, H, hd):
+    """Nothing in it depends on the order of events: P that is replaced, or O that is rescaled, before a product has read or written it
+    shows as rows that differ from call to call."""
+    from heirloom_b200 import cuda
+    c = ctx()
+    C = hd * H
+    qkv = torch.randn(B * T, 3 * C, device="cuda", generator=torch.Generator(device="cuda").manual_seed(T)).to(torch.bfloat16)
+    q, k, v = qkv.split(C, dim=1)
+    torch.cuda.synchronize()
+    first = cuda.flash_attention_forward(c, q, k, v, B, T, H)
+    for _ in range(8):
+        again = cuda.flash_attention_forward(c, q, k, v, B, T, H)
+        c.sync()
+        assert torch.equal(again[0], first[0]) and torch.equal(again[1], first[1])
+
+
 def test_flash_forward_rejects_unsupported_shapes():
     from heirloom_b200 import cuda
     from heirloom_b200._lib import HeirloomError
