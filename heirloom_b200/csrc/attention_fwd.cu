@@ -16,7 +16,7 @@
 // query row) work on tile j while the tensor cores run P·V of tile j-1 and Q·Kᵀ of tile j+1.  P is formed against a reference maximum
 // that a row raises only when its maximum has grown by more than 2^8; the row then rescales its O in place (tensor-memory load,
 // multiply, store) between two P·V products.  P goes to the tensor cores out of tensor memory: through shared memory it was a third
-// of that memory's traffic, which was three quarters of what an SM can do (heads of 128: B4 H12 T4096 211.7 us with it, now 197.1).
+// of that memory's traffic, which was three quarters of what an SM can do (heads of 128: B4 H12 T4096 211.7 us with it, now 200.5).
 //
 // Work items go round persistent streams without a gap, several of them on an SM, so that one's tensor work and waits lie under
 // another's exponentials.  Heads of 128 have room for two, a CTA each (192 threads, 112 KB of shared memory, 256 tensor-memory columns);
@@ -295,7 +295,7 @@ flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
       }
       const float neg_m = -m_ref;
       const uint32_t tp = tmem_s0 + (uint32_t)((g & 1) * FA_BN) + lane_sel;
-      float2 sums[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+      float l_tile = 0.f;  // key after key, as ever: the results are the same bits
 #pragma unroll
       for (int q = 0; q < 4; ++q) {  // sixteen keys
         uint32_t w[8];
@@ -304,12 +304,12 @@ flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
           const float2 x = fma2(make_float2(__uint_as_float(sb[q * 16 + 2 * e]), __uint_as_float(sb[q * 16 + 2 * e + 1])),
                                 both(p.scale_log2), both(neg_m));
           const float2 pr = make_float2(ex2_fast(x.x), ex2_fast(x.y));
-          sums[e & 1] = add2(sums[e & 1], pr);
+          l_tile += pr.x + pr.y;
           w[e] = pack_bf16x2(pr.x, pr.y);
         }
         tc05::tmem_st_32x32b_x8(tp + q * 8, w);
       }
-      l_run += (sums[0].x + sums[0].y) + (sums[1].x + sums[1].y);
+      l_run += l_tile;
       tc05::tmem_st_wait();
       tc05::tc_fence_before_sync();
       __syncwarp();
@@ -376,8 +376,8 @@ flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
 // What bounds these is the softmax: 64 exponentials a row and tile are 512 cycles of a scheduler's, the products 256.  A warp's chain (scores,
 // maximum, exponentials, hand-over) takes three times that, so that three warps share a scheduler: one CTA an SM walks three streams
 // of items side by side, each with its own tiles, four softmax warps and a warp whose elected thread queues both loads and products
-// (B16 H12 T1024: two CTAs of four softmax warps 62.8 us, three streams 58.3, P in tensor memory 55.2, its place waited for when half of
-// P has been formed 52.5; B4 H12 T4096 175.5, 176.5, 164.5, 153.7).
+// (B16 H12 T1024: two CTAs of four softmax warps 62.8 us, three streams 58.3, P in tensor memory and its place waited for
+// when half of P has been formed 54.9; B4 H12 T4096 175.5, 176.5, 167).
 // That thread waits for scores that have been read and P that has been written, and for nothing else: when S(g) has been read, Q·K(g)
 // is done and K(g) can be replaced; when P(g) has been written, P·V(g-1) is done and V(g-1) can.
 // A stream has S, P and O in tensor memory (160 columns), and Q, a place for the result, three K and two V in shared memory: 72 KB.
@@ -595,7 +595,8 @@ flash_attention_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __
           tc05::tmem_st_wait();
         }
         const float neg_m = -m_ref;
-        float2 sums[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        float l_tile = 0.f;  // key after key, as ever: the results are the same bits (two chains of pairs: T4096 153 us; the sums behind
+                             // the hand-over of P: 182 to 191)
         auto half = [&](auto which, uint32_t (&w)[2][8]) {  // of P, sixteen keys each
           constexpr int H = decltype(which)::value;
           if (halves <= H) {
@@ -608,7 +609,7 @@ flash_attention_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __
             const float2 x = fma2(make_float2(__uint_as_float(sb[H * 32 + 2 * e]), __uint_as_float(sb[H * 32 + 2 * e + 1])), both(p.scale_log2),
                                   both(neg_m));
             const float2 pr = make_float2(ex2_fast(x.x), ex2_fast(x.y));
-            sums[e & 1] = add2(sums[e & 1], pr);
+            l_tile += pr.x + pr.y;
             w[e / 8][e % 8] = pack_bf16x2(pr.x, pr.y);
           }
         };
@@ -621,7 +622,7 @@ flash_attention_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __
         half(std::integral_constant<int, 1>{}, w);
         tc05::tmem_st_32x32b_x8(tmem_p + lane_sel + 16, w[0]);
         tc05::tmem_st_32x32b_x8(tmem_p + lane_sel + 24, w[1]);
-        l_run += (sums[0].x + sums[0].y) + (sums[1].x + sums[1].y);
+        l_run += l_tile;
         tc05::tmem_st_wait();
         tc05::tc_fence_before_sync();
         __syncwarp();
