@@ -9,7 +9,8 @@
 // what dQ costs there: 480 KB a 128 x 128 tile.  The whole backward call, before and after: B4 H12 T4096 1046 and 632 us, B16 H6 T1024
 // 188 and 126.  What bounds it now: the path out of the SM, 70 % busy with dQ's 64 KB of f32 reductions a tile, and the chain of
 // hand-overs dS -> dK -> dQ -> read-out -> dP -> dS (the tensor core is busy half of the time).  Sixteen softmax warps of 32 queries
-// instead of eight of 64 were slower (685 us); the same kernel for 64 channels was as fast as the one there is.
+// instead of eight of 64 were slower (685 us); the same kernel for 64 channels was as fast as the one there is.  Scores worked on two an
+// instruction: 579 -> 573.5 us.
 //
 // Tensor memory (512 columns): dV and dK 128 each, S and Pᵀ over it 128, and 128 for dP, dSᵀ over it and dQ over that once dK has read
 // it.  S of tile g + 1 follows dV of tile g, beside the softmax warps' work on dS; dP of tile g + 1 follows the read-out of dQ.  The
@@ -355,12 +356,17 @@ flash_attention_bwd_t_kernel(const __grid_constant__ CUtensorMap map_q, const __
 #pragma unroll
         for (int i = 0; i < 16; i += 4) {
           const float4 l = *reinterpret_cast<const float4*>(lse + ch * 16 + i);
-          const float ll[4] = {l.x, l.y, l.z, l.w};
+          const float2 ll[2] = {make_float2(l.x, l.y), make_float2(l.z, l.w)};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            float v = ex2_fast(fmaf(__uint_as_float(raw[ch & 1][i + e]), p.scale_log2, ll[e]));
-            if constexpr (Diag) v = r > half * 64 + ch * 16 + i + e ? 0.f : v;  // keys after the query
-            pv[ch * 16 + i + e] = v;
+          for (int e = 0; e < 4; e += 2) {
+            const float2 x = fma2(make_float2(__uint_as_float(raw[ch & 1][i + e]), __uint_as_float(raw[ch & 1][i + e + 1])), both(p.scale_log2), ll[e / 2]);
+            float2 v = make_float2(ex2_fast(x.x), ex2_fast(x.y));
+            if constexpr (Diag) {  // keys after the query
+              if (r > half * 64 + ch * 16 + i + e) v.x = 0.f;
+              if (r > half * 64 + ch * 16 + i + e + 1) v.y = 0.f;
+            }
+            pv[ch * 16 + i + e] = v.x;
+            pv[ch * 16 + i + e + 1] = v.y;
           }
           w[i / 2] = pack_bf16x2(pv[ch * 16 + i], pv[ch * 16 + i + 1]);
           w[i / 2 + 1] = pack_bf16x2(pv[ch * 16 + i + 2], pv[ch * 16 + i + 3]);
@@ -386,12 +392,13 @@ flash_attention_bwd_t_kernel(const __grid_constant__ CUtensorMap map_q, const __
 #pragma unroll
         for (int i = 0; i < 16; i += 4) {
           const float4 l = *reinterpret_cast<const float4*>(delta + ch * 16 + i);
-          const float ll[4] = {l.x, l.y, l.z, l.w};
-          float ds[4];
+          const float2 ll[2] = {make_float2(l.x, l.y), make_float2(l.z, l.w)};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) ds[e] = pv[ch * 16 + i + e] * fmaf(__uint_as_float(raw[ch & 1][i + e]), p.scale, ll[e]);
-          w[i / 2] = pack_bf16x2(ds[0], ds[1]);
-          w[i / 2 + 1] = pack_bf16x2(ds[2], ds[3]);
+          for (int e = 0; e < 4; e += 2) {
+            const float2 ds = mul2(make_float2(pv[ch * 16 + i + e], pv[ch * 16 + i + e + 1]),
+                                   fma2(make_float2(__uint_as_float(raw[ch & 1][i + e]), __uint_as_float(raw[ch & 1][i + e + 1])), both(p.scale), ll[e / 2]));
+            w[(i + e) / 2] = pack_bf16x2(ds.x, ds.y);
+          }
         }
         tc05::tmem_st_32x32b_x8(tdp + ch * 8, w);
         *reinterpret_cast<uint4*>(line + (((ch * 2) ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
