@@ -156,7 +156,9 @@ struct Mail {
     if (bytes1) tc05::mbar_arrive_expect_tx(&arrived[1], bytes1);
   }
   __device__ __forceinline__ void wait(int i, int* status) {
-    if (!tc05::mbar_wait(&arrived[i], 0, &abort_flag)) *status = 1;
+    if (tc05::mbar_wait(&arrived[i], 0, &abort_flag)) return;
+    for (int k = 0; k < 2000; ++k) __nanosleep(100);  // what is on its way lands before shared memory is released
+    *status = 1;
   }
 };
 // `bytes` (whole sixteens) of this CTA's shared memory into a peer's, by one warp.  A store to a peer takes its turn whatever its width:
