@@ -1026,6 +1026,15 @@ static bool pair_form(const hl_ctx* ctx, const hl_gemm_desc* d, const GemmPlan& 
   return plan.sk_tiles == 0 && d->m > BM && sms >= 2 && ctx->gemm_skip_kblock < 0 && pairs_enabled(d, plan.splits, sms);
 }
 
+// Beside another stream's kernels (collectives in flight) whole tiles and equal splits are handed out by a counter
+// instead of round-robin: per launch it costs about a microsecond, and it keeps a CTA that starts late from holding
+// up its share of the tiles.  HEIRLOOM_GEMM_DYNAMIC=1 / 0 forces it on / off.
+static bool draws_tiles(const hl_ctx* ctx, const GemmPlan& plan, bool pair) {
+  const char* e = getenv("HEIRLOOM_GEMM_DYNAMIC");
+  const bool dynamic = e && (e[0] == '0' || e[0] == '1') ? e[0] == '1' : nccl_active(ctx);
+  return dynamic && !pair && plan.sk_tiles == 0 && ctx->gemm_skip_kblock < 0;
+}
+
 int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, void* c, const float* bias,
                   const void* aux_in, void* aux_out, float* workspace, size_t workspace_bytes, unsigned* stream_flags,
                   const GemmRowStats* row_stats) {
@@ -1072,18 +1081,9 @@ int gemm_bf16_run(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void*
     if (seq == 0) seq = ++g_stream_launch_number;  // 0 means "never written"
     p.sk_seq = seq;
   }
-  // Beside another stream's kernels (collectives in flight) whole tiles and equal splits are handed out by a counter
-  // instead of round-robin: per launch it costs about a microsecond, and it keeps a CTA that starts late from holding
-  // up its share of the tiles.  HEIRLOOM_GEMM_DYNAMIC=1 / 0 forces it on / off.  Every tile advances the counter by
-  // one, so the host knows its value at the start of the next launch without touching the device.
-  {
-    const char* e = getenv("HEIRLOOM_GEMM_DYNAMIC");
-    const bool dynamic = e && (e[0] == '0' || e[0] == '1') ? e[0] == '1' : nccl_active(ctx);
-    p.sched = (dynamic && !pair && plan.sk_tiles == 0 && ctx->gemm_skip_kblock < 0) ? ctx->gemm_sched : nullptr;
-    if (p.sched) {
-      p.sched_base = ctx->gemm_sched_base;  // advanced below, once the launch has been queued
-    }
-  }
+  // Every tile advances the counter by one, so the host knows its value at the start of the next launch without touching the device.
+  p.sched = draws_tiles(ctx, plan, pair) ? ctx->gemm_sched : nullptr;
+  p.sched_base = ctx->gemm_sched_base;  // advanced below, once the launch has been queued
   p.k_blocks_per_split = ceil_div(p.k_blocks, splits);
   p.epilogue = d->epilogue;
   p.out_dtype = d->out_dtype;
@@ -1242,7 +1242,7 @@ bool gemm_bf16_scratch(hl_ctx* ctx, const hl_gemm_desc* d, size_t* bytes) {
   const GemmPlan plan = gemm_plan(d, sms);
   const bool small = small_plan(ctx, d, plan, sms).splits > 0;
   *bytes = small ? 0 : plan.splitk_bytes;
-  return small || plan.sk_tiles == 0;
+  return small || (plan.sk_tiles == 0 && !draws_tiles(ctx, plan, pair_form(ctx, d, plan, sms)));
 }
 bool gemm_bf16_small_applies(hl_ctx* ctx, const hl_gemm_desc* d) {
   const int sms = persistent_sms(ctx);

@@ -48,7 +48,8 @@ int gemm_small_run(hl_ctx* ctx, const hl_gemm_desc* d, const GemmSmallPlan& plan
 // The GEMM with its scratch taken from (and grown in) the context.
 int gemm_bf16_ctx(hl_ctx* ctx, const hl_gemm_desc* d, const void* a, const void* b, void* c, const float* bias,
                   const void* aux_in, void* aux_out);
-// The scratch that gemm_bf16_ctx would take, or false where the product also uses the context's flags, which only one stream may.
+// The scratch that gemm_bf16_ctx would take, or false where the product also uses the context's flags or its tile counter, which only one
+// stream may: the launches' shares of the counter follow one another in the order in which they were queued.
 bool gemm_bf16_scratch(hl_ctx* ctx, const hl_gemm_desc* d, size_t* bytes);
 // A plain product with the sums of A's rows over the contraction beside it (a weight gradient and its bias gradient), where
 // that costs no launch of its own; *done tells whether it was one of those, otherwise nothing has been launched.

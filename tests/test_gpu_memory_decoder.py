@@ -329,3 +329,40 @@ def test_what_runs_beside_the_backward_pass_equals_everything_in_one_stream(prec
             scale = np.abs(want[name]).max()
             assert np.abs(g - want[name]).max() <= limit * scale + 1e-12, (name, np.abs(g - want[name]).max() / scale)
     model.close()
+
+
+@pytest.mark.parametrize("pairs,width", [("0", 256), (None, 64)])
+def test_gradients_beside_the_backward_pass_with_tiles_from_a_counter(monkeypatch, pairs, width):
+    """HEIRLOOM_GEMM_DYNAMIC=1 without a communicator: every product on single CTAs draws its tiles from one counter, whose value at a
+    launch's start the host knows, so that no two of them may run at once; the memory projections' weight gradients are such products
+    here, with pairs switched off or because they have no more than 128 rows.  Per-kernel timing keeps everything in one stream.  The
+    limit is that of the test above; the last product shows that the host still knows the counter."""
+    from heirloom_b200 import cuda, nn
+    c = ctx()
+    kw, mem = dict(KW, vocab=1024), dict(MEM, key_dim=width, value_dim=width, top_k=16)
+    model = nn.DecoderLm(c, nn.DecoderConfig(batch=32, **kw), nn.MemoryConfig(**mem))
+    model.load_state_dict(ho.init_memory_parameters(ho.DecoderConfig(**kw), ho.MemoryConfig(**mem), 3))
+    tok = torch.tensor(ho.zipf_tokens(np.random.default_rng(5), kw["vocab"], (32, 129)), device="cuda")
+    x, y = tok[:, :-1].contiguous(), tok[:, 1:].contiguous()
+    monkeypatch.setenv("HEIRLOOM_GEMM_DYNAMIC", "1")
+    if pairs:
+        monkeypatch.setenv("HEIRLOOM_GEMM_PAIRS", pairs)
+
+    def gradients():
+        model.forward_backward(x, y)
+        return {n: model.grad(n).astype(np.float64) for n in model.parameter_names() if not n.endswith("k_proj.bias")}
+    cuda.check(c.lib.hl_profile_enable(c.handle, 1))
+    try:
+        want = gradients()
+    finally:
+        cuda.check(c.lib.hl_profile_enable(c.handle, 0))
+    for _ in range(5):
+        for name, g in gradients().items():
+            scale = np.abs(want[name]).max()
+            assert np.abs(g - want[name]).max() <= 4e-3 * scale + 1e-12, (name, np.abs(g - want[name]).max() / scale)
+    model.close()
+    a, b = torch.randn(4096, 320, device="cuda").bfloat16(), torch.randn(2048, 320, device="cuda").bfloat16()
+    out = cuda.gemm_bf16(c, a, b, 4096, 2048, 320, out_dtype=torch.float32)
+    c.sync()
+    want = a.float() @ b.float().T
+    assert (out - want).norm() <= 1e-3 * want.norm()
