@@ -448,8 +448,10 @@ product_key_topk_kernel(const float* __restrict__ left, const float* __restrict_
 // tables of 512 x 256, of which the selection wants 32 in 512.  So the tensor core forms all of them first out of bf16 pieces, hi * hi +
 // lo * hi + hi * lo, and only what can be among the beam's is formed again as it has to be: with |approximate - exact| <= E, every
 // key of the beam has an approximate score of at least the beam-th largest minus 2 E.  In terms of S, the norm of the token's half
-// query times the largest norm of a half key (sum |q k| <= S): the f32 sum is off by at most 2 half * 2^-24 S, the dropped pieces by
-// 3 * 2^-18 S, and each of the 3 half / 16 tensor-core steps by 17 terms cut off at 2^-23, together less than (5.1e-7 half + 1.2e-5) S.
+// query times the largest norm of a half key (sum |q k| <= S): rounding to bf16 leaves up to 2^-8 of a value, and rounding that again up to
+// 2^-17 of the value, so that lo * lo is up to 2^-16 S and the two remainders up to 2^-17 S each, 2^-15 S in all; the f32 sum is off by at
+// most 2 half * 2^-24 S, and each of the 3 half / 16 tensor-core steps by 17 terms cut off at 2^-23: together less than (5.0e-7 half + 3.06e-5) S.
+// The band is taken with 5.4e-7 and 3.2e-5, for what the norms' own sums round.
 // Where S is not within 1e-30 and 1e37 (or a norm below 1e-18: its squares and the pieces of such values lose bits), or more than 64 keys come into
 // question, all scores of that token and side are formed exactly.  The selections are the same bit by bit.  The kernel takes 226 us of the 276,
 // two thirds of the shared memory's rate: rows are staged there for the lanes that walk them; 5 or 6 blocks an SM: 230 and 234.
@@ -580,7 +582,7 @@ product_key_lookup_kernel(const float* __restrict__ left_approx, const float* __
   for (int sd = 0; sd < 2; ++sd) {
     const float qn = sqrtf(warp_sum(squares[sd])), kn = norms[sd], s = qn * kn;
     const bool within = qn >= 1e-18f && kn >= 1e-18f && s >= 1e-30f && s <= 1e37f;  // (false for NaN)
-    const float band = 2.f * s * (5.4e-7f * (float)half + 2e-5f);
+    const float band = 2.f * s * (5.4e-7f * (float)half + 3.2e-5f);
     count[sd] = within ? find_candidates((sd ? right_approx : left_approx) + (size_t)token * side, side, beam, band, cand[sd], sc) : -1;
   }
   int more[2] = {max(0, count[0] - 32), max(0, count[1] - 32)};  // beyond a warp's lanes

@@ -511,3 +511,39 @@ def test_lookup_of_the_step_selects_what_exact_scores_do(tokens, side, key_dim, 
                                            cuda._p(approx[0]), cuda._p(approx[1]), cuda._p(got), c_int(tokens), c_int(side), c_int(key_dim),
                                            c_int(top_k), c_int(beam)))
     np.testing.assert_array_equal(host(got), host(want))
+
+
+@pytest.mark.parametrize("tokens,side,key_dim,top_k", [(64, 64, 64, 8), (130, 512, 128, 32), (257, 256, 1024, 16)])
+def test_lookup_of_values_whose_pieces_are_at_their_worst(tokens, side, key_dim, top_k):
+    """1 + 2^-8 - 2^-17 - 2^-23 and 1 + 2^-8 - 2^-16 and their like, of either sign: a bf16 piece leaves 2^-8 of them, two leave 2^-17.  The
+    approximate scores are off by what was derived, 2^-15 S from the pieces and 17 terms cut off at 2^-23 in each of the 3 half / 16
+    steps.  More than 3 * 2^-18 S is seen.  Selected rows as by exact scores."""
+    from ctypes import c_int
+
+    from heirloom_b200 import cuda
+    c = ctx()
+    rng = np.random.default_rng(side + key_dim)
+    half = key_dim // 2
+    worst = np.array([1 + 2 ** -8 - 2 ** -17 - 2 ** -23, 1 + 2 ** -8 - 2 ** -16, 1 + 2 ** -8 - 2 ** -17], np.float32)
+    draw = lambda *shape: (rng.choice(worst, shape, p=[0.8, 0.1, 0.1]) * rng.choice([1, 1, 1, -1], shape)).astype(np.float32)
+    q, keys = draw(tokens, key_dim), [draw(side, half) for _ in range(2)]
+    q[0], keys[0][0], keys[1][-1] = np.abs(q[0]), np.abs(keys[0][0]), np.abs(keys[1][-1])
+    query, left, right = dev(q), dev(keys[0]), dev(keys[1])
+    beam = min(side, max(top_k, int(np.ceil(np.sqrt(top_k)))))
+    want = cuda.product_key_topk_from_side_scores(c, *cuda.product_key_side_scores(c, query, left, right), top_k, beam)
+    got = torch.full_like(want, -1)
+    pieces = torch.empty(6 * side * key_dim + 256, dtype=torch.uint8, device="cuda")
+    query_pieces = torch.empty(tokens, 2 * key_dim, dtype=torch.bfloat16, device="cuda")
+    approx = torch.empty(2, tokens, side, device="cuda")
+    cuda.check(c.lib.hl_product_key_lookup(c.handle, cuda._p(query), cuda._p(left), cuda._p(right), cuda._p(pieces), cuda._p(query_pieces),
+                                           cuda._p(approx[0]), cuda._p(approx[1]), cuda._p(got), c_int(tokens), c_int(side), c_int(key_dim),
+                                           c_int(top_k), c_int(beam)))
+    np.testing.assert_array_equal(host(got), host(want))
+    seen = 0.0
+    for sd in range(2):
+        x, k = q[:, sd * half:][:, :half].astype(np.float64), keys[sd].astype(np.float64)
+        s = np.linalg.norm(x, axis=1)[:, None] * np.linalg.norm(k, axis=1).max()
+        off = np.abs(host(approx[sd]).astype(np.float64) - x @ k.T) / s
+        assert off.max() <= 2 ** -15 + 3 * half / 16 * 17 * 2 ** -23
+        seen = max(seen, off.max())
+    assert seen > 3 * 2 ** -18
