@@ -80,6 +80,27 @@ def test_flash_forward_gives_the_same_bits_every_time(B, T, H, hd):
         assert torch.equal(again[0], first[0]) and torch.equal(again[1], first[1])
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("B,T,H", [(4, 2048, 10), (1, 4096, 20), (64, 300, 8)])
+def test_flash_backward_gives_the_same_dk_and_dv_every_time(B, T, H, hd):
+    """dK and dV are sums in a fixed order (dQ's parts are not): P that is replaced before dV has read it, or dS before dK has, shows as rows
+    that differ from call to call."""
+    from heirloom_b200 import cuda
+    c = ctx()
+    C = hd * H
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    qkv = torch.randn(B * T, 3 * C, device="cuda", generator=gen).to(torch.bfloat16)
+    dout = torch.randn(B * T, C, device="cuda", generator=gen).to(torch.bfloat16)
+    q, k, v = qkv.split(C, dim=1)
+    torch.cuda.synchronize()
+    out, lse = cuda.flash_attention_forward(c, q, k, v, B, T, H)
+    first = cuda.flash_attention_backward(c, q, k, v, out, dout, lse, B, T, H)
+    for _ in range(8):
+        again = cuda.flash_attention_backward(c, q, k, v, out, dout, lse, B, T, H)
+        c.sync()
+        assert torch.equal(again[:, C:], first[:, C:])
+
+
 def test_flash_forward_rejects_unsupported_shapes():
     from heirloom_b200 import cuda
     from heirloom_b200._lib import HeirloomError
