@@ -664,6 +664,7 @@ bool block_fits(int d, int heads, int hidden, int context) {
   // contractions in whole steps of the matrix instruction, rows of weights and slices of them on sixteen bytes
   if (d > GV_SPAN || d % 16 || hd % (DB_CTAS * 2) || hidden % 8 || heads > DB_MAX_PARTS) return false;
   if (ceil_div(context, DB_CTAS) > DB_KEY_TURNS * DB_SLOTS) return false;
+  if (feed_forward_units<T>(hidden) > DB_THREADS) return false;  // a thread a hidden unit
   return AttentionLayout<T, Acc>(d, hd, ceil_div(context, DB_CTAS), false).total <= (int)DB_MAX_SHARED && 3 * hd <= DB_THREADS &&
          FeedForwardLayout<T, Acc>(d, feed_forward_units<T>(hidden)).total <= (int)DB_MAX_SHARED;
 }

@@ -290,6 +290,8 @@ def test_one_token_steps_equal_the_full_window(heads, memory):
     (256, 2, 776, 1024, 1000), # a thread's second key
     (128, 1, 64, 1030, 1021),  # contexts beyond that: kernels of their own
     (64, 8, 64, 19, 10),       # heads of 8 channels: kernels of their own
+    (16, 1, 65536, 9, 1),      # a hidden unit a thread
+    (16, 1, 65544, 9, 1),      # more of them: kernels of their own
 ])
 def test_one_token_steps_of_all_sizes_equal_the_full_window(d_model, heads, d_ff, context, prefix):
     """prefill + decode_next against a full-window pass, on both sides of every limit of the kernels that take a block in two
