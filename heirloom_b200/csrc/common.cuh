@@ -66,7 +66,7 @@ struct Counters {
 struct hl_ctx {
   int device = 0;
   int sm_count = 0;
-  unsigned long long wait_limit_ns = 0;  // bound of the pipeline waits in the GEMM kernel (0 = the two-second default)
+  unsigned long long wait_limit_ns = 0;  // bound of the kernels' waits where they take one (0 = the two-second default)
   bool forward_only = false;           // no backward pass follows: what only it would read need not be written
   int gemm_skip_kblock = -1;           // test hook of hl_ctx_set_test_hooks
   int reserve_sms = 0;                 // SMs the persistent kernels leave free while gradient collectives are in flight

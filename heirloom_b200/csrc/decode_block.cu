@@ -155,10 +155,15 @@ struct Mail {
     if (bytes0) tc05::mbar_arrive_expect_tx(&arrived[0], bytes0);
     if (bytes1) tc05::mbar_arrive_expect_tx(&arrived[1], bytes1);
   }
-  __device__ __forceinline__ void wait(int i, int* status) {
-    if (tc05::mbar_wait(&arrived[i], 0, &abort_flag)) return;
-    for (int k = 0; k < 2000; ++k) __nanosleep(100);  // what is on its way lands before shared memory is released
-    *status = 1;
+  __device__ __forceinline__ void wait(int i, unsigned long long limit_ns, int* status) {
+    if (!tc05::mbar_wait(&arrived[i], 0, &abort_flag, limit_ns)) *status = 1;
+  }
+  // At the end of the kernel.  A CTA whose wait ran out stays until its peers, whose waits are bounded as well, have left or are here too,
+  // and then until what they sent has landed: a peer may be late and not lost.
+  __device__ __forceinline__ void leave() {
+    if (!*static_cast<volatile int*>(&abort_flag)) return;
+    tc05::cluster_meet();
+    for (int k = 0; k < 2000; ++k) __nanosleep(100);
   }
 };
 // `bytes` (whole sixteens) of this CTA's shared memory into a peer's, by one warp.  A store to a peer takes its turn whatever its width:
@@ -292,6 +297,8 @@ struct AttentionArgs {
   int d, hd, cap;
   bool window;
   int* status;
+  unsigned long long wait_limit_ns;
+  int withheld;  // test hook: bytes that are waited for and never sent
 };
 
 template <typename T, typename Acc>
@@ -319,7 +326,7 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_attention_block_kernel(c
   const long long ld = 3 * d;
   T* qkv = static_cast<T*>(a.qkv) + h * hd;
   pdl_trigger();
-  if (threadIdx.x == 0) mail.open(a.window ? 0 : (DB_CTAS - 1) * pitch_fresh * 4, (DB_CTAS - 1) * pitch_all * (int)sizeof(Acc));
+  if (threadIdx.x == 0) mail.open(a.window ? 0 : (DB_CTAS - 1) * pitch_fresh * 4 + a.withheld, (DB_CTAS - 1) * pitch_all * (int)sizeof(Acc) + a.withheld);
   // The position was copied here before the first kernel of the sequence started.
   const int t = (int)a.state[0], keys = t + 1, chunk = (keys + DB_CTAS - 1) / DB_CTAS;
   const int k0 = min(keys, rank * chunk), k1 = min(keys, k0 + chunk);
@@ -360,7 +367,7 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_attention_block_kernel(c
     __syncthreads();
     if (warp < DB_CTAS && warp != rank) push(&mail.arrived[0], own, own, pitch_fresh * 4, warp);
     cp_async_wait_all();
-    mail.wait(0, a.status);
+    mail.wait(0, a.wait_limit_ns, a.status);
     if (const int i = threadIdx.x; i < rows) {  // (nobody waits for these)
       const int which = i < cpc ? 0 : i < 2 * cpc ? 1 : 2;
       qkv[(long long)t * ld + which * d + rank * cpc + i - which * cpc] = stored<T>(y);
@@ -441,7 +448,7 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_attention_block_kernel(c
   if (const int c = threadIdx.x; c < hd + 2) own[c] = c == hd ? mx : sum_of_warps(c < hd ? part : red_sum, c < hd ? hd : 1, c < hd ? c : 0);
   __syncthreads();
   if (warp < DB_CTAS && warp != rank) push(&mail.arrived[1], own, own, pitch_all * sizeof(Acc), warp);
-  mail.wait(1, a.status);
+  mail.wait(1, a.wait_limit_ns, a.status);
   {
     const Acc* mine = all + (lane & 7) * pitch_all + hd;
     const Acc m = mine[0];
@@ -465,6 +472,7 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_attention_block_kernel(c
   __syncthreads();
   Acc* out = static_cast<Acc*>(a.parts) + (size_t)h * d + rank * opc;
   multiply_columns(wo, hd + PAD, opc, att, hd, [&](int o, Acc v) { out[o] = v; });
+  mail.leave();
 }
 
 // Layer norm, the hidden units of a CTA and their share of every output; the shares of a cluster are added up within it.
@@ -497,6 +505,8 @@ struct FeedForwardArgs {
   void* parts;  // [clusters][d]
   int d, hidden, units;  // units: hidden units a CTA
   int* status;
+  unsigned long long wait_limit_ns;
+  int withheld;  // as above
 };
 
 template <typename T, typename Acc>
@@ -519,7 +529,7 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_feed_forward_kernel(cons
   const int warp = threadIdx.x >> 5, rank = (int)(blockIdx.x % DB_CTAS);
   const int first = min(a.hidden, (int)blockIdx.x * units), n = min(units, a.hidden - first);  // n may be 0
   pdl_trigger();
-  if (threadIdx.x == 0) mail.open(DB_CTAS * pitch_sums * (int)sizeof(Acc), 0);
+  if (threadIdx.x == 0) mail.open(DB_CTAS * pitch_sums * (int)sizeof(Acc) + a.withheld, 0);
   stage_rows(w1, (d + PAD) * sizeof(T), static_cast<const T*>(a.w1) + (size_t)first * d, d * sizeof(T), n, d * sizeof(T));
   if ((int)threadIdx.x < n) cp_async4(bias + threadIdx.x, a.b1 + first + threadIdx.x);
   cp_async_commit();
@@ -552,7 +562,7 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_feed_forward_kernel(cons
   });
   __syncthreads();
   if (warp < DB_CTAS) push(&mail.arrived[0], sums + rank * pitch_sums, outputs + warp * pitch_sums, pitch_sums * sizeof(Acc), warp);
-  mail.wait(0, a.status);
+  mail.wait(0, a.wait_limit_ns, a.status);
   Acc* out = static_cast<Acc*>(a.parts) + (size_t)(blockIdx.x / DB_CTAS) * d + rank * opc;
   if (const int c = threadIdx.x; c < opc) {
     Acc s = 0;
@@ -560,6 +570,7 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_feed_forward_kernel(cons
     for (int r = 0; r < DB_CTAS; ++r) s += sums[r * pitch_sums + c];
     out[c] = s;
   }
+  mail.leave();
 }
 
 // The row itself, for kernels that read it.
@@ -669,10 +680,13 @@ bool block_fits(int d, int heads, int hidden, int context) {
          FeedForwardLayout<T, Acc>(d, feed_forward_units<T>(hidden)).total <= (int)DB_MAX_SHARED;
 }
 
+unsigned long long wait_limit(const hl_ctx* ctx) { return ctx->wait_limit_ns ? ctx->wait_limit_ns : tc05::kWaitLimitNs; }
+int withheld(const hl_ctx* ctx) { return ctx->gemm_skip_kblock >= 0 ? 16 : 0; }
+
 template <typename T, typename Acc>
 int run_attention(hl_ctx* ctx, const DecodeBlock& b) {
   AttentionArgs a{b.x, b.ln1_gamma, b.ln1_beta, b.wqkv, b.bqkv, b.qkv, b.state, b.wo, b.attention_parts, b.d, b.d / b.heads,
-                  ceil_div(b.context, DB_CTAS), b.window, ctx->status_dev + ST_WAIT_EXPIRED};
+                  ceil_div(b.context, DB_CTAS), b.window, ctx->status_dev + ST_WAIT_EXPIRED, wait_limit(ctx), withheld(ctx)};
   const AttentionLayout<T, Acc> at(a.d, a.hd, a.cap, a.window);
   auto kern = decode_attention_block_kernel<T, Acc>;
   HL_ALLOW_SHARED(ctx, DB_MAX_SHARED, kern);
@@ -683,7 +697,8 @@ int run_attention(hl_ctx* ctx, const DecodeBlock& b) {
 
 template <typename T, typename Acc>
 int run_feed_forward(hl_ctx* ctx, const DecodeBlock& b, const DecodeRow& x, int units, int clusters) {
-  FeedForwardArgs a{x, b.ln2_gamma, b.ln2_beta, b.w1, b.b1, b.w2, b.feed_forward_parts, b.d, b.hidden, units, ctx->status_dev + ST_WAIT_EXPIRED};
+  FeedForwardArgs a{x, b.ln2_gamma, b.ln2_beta, b.w1, b.b1, b.w2, b.feed_forward_parts, b.d, b.hidden, units, ctx->status_dev + ST_WAIT_EXPIRED, wait_limit(ctx),
+                    withheld(ctx)};
   const FeedForwardLayout<T, Acc> at(a.d, units);
   auto kern = decode_feed_forward_kernel<T, Acc>;
   HL_ALLOW_SHARED(ctx, DB_MAX_SHARED, kern);

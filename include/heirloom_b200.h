@@ -45,7 +45,8 @@ int hl_ctx_sync(hl_ctx* ctx);
  * wait runs out the kernel leaves its loops, frees its tensor memory, returns, and sets a status word that the next
  * hl_ctx_sync reports as HL_ERR_DEVICE; the context stays usable.  `wait_limit_ns` shortens the bound for hl_gemm_bf16
  * (0 = default) and `gemm_skip_kblock` >= 0 makes the GEMM's TMA producer leave out that k block of its first tile (and the
- * tensor-core form of the half-key gradients that stage of tokens), so that the wait for it runs out; -1 switches the hook off.  The reference has no such path: its kernels have no
+ * tensor-core form of the half-key gradients that stage of tokens), and the kernels of one-token steps wait for sixteen bytes that no
+ * CTA of their cluster sends, so that the wait runs out; -1 switches the hook off.  The reference has no such path: its kernels have no
  * device-side waits (single-role kernels, heirloom-kernels/src/ptx/tensor_core.ptx). */
 int hl_ctx_set_test_hooks(hl_ctx* ctx, unsigned long long wait_limit_ns, int gemm_skip_kblock);
 /* The compute stream as a cudaStream_t, for callers that time with their own events. */

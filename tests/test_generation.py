@@ -434,6 +434,36 @@ def test_evaluation_and_generation_report_the_device_status(precision):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("d_model,heads", [(128, 1), (128, 8), (256, 4)])
+def test_one_token_steps_whose_peers_do_not_answer_end_in_an_error(d_model, heads):
+    """The hook makes every CTA of a cluster wait for bytes that no peer sends: the step ends with an error after the limit, leaves nothing
+    cached, and the same calls work afterwards.  f32, whose other kernels take no hook; the window's last block has the same exchange."""
+    from heirloom_b200 import nn
+    from heirloom_b200._lib import HeirloomError
+    from tests.gpu_util import ctx
+    c = ctx()
+    model = nn.DecoderLm(c, nn.DecoderConfig(vocab=64, d_model=d_model, n_layers=2, n_heads=heads, d_ff=256, context=32, batch=1,
+                                             precision=nn.PRECISION_F32))
+    rng = np.random.default_rng(3)
+    model.load_state_dict({n: rng.standard_normal(s) * 0.2 for n, s in model.parameter_shapes().items()})
+    prompt = rng.integers(0, 64, 20)
+    steps = lambda: [model.prefill(prompt)] + [model.decode_next(t) for t in (5, 6)]
+    want = steps()
+    for call in (lambda: model.decode_next(7), lambda: model.prefill(prompt)):
+        model.prefill(prompt)
+        c.set_test_hooks(wait_limit_ns=200_000, gemm_skip_kblock=0)
+        try:
+            with pytest.raises(HeirloomError, match="wait expired"):
+                call()
+        finally:
+            c.set_test_hooks(0, -1)
+        assert model.cached_positions == 0
+        for got, right in zip(steps(), want):
+            np.testing.assert_array_equal(got, right)
+    model.close()
+
+
+@pytest.mark.gpu
 def test_a_pass_that_ends_in_an_error_leaves_no_cache():
     """A training pass that runs out of memory in its first block (its fc2 product, 20 x 4 tiles over a contraction of 12288, deals out
     k blocks and wants 19 MB of scratch), after it has overwritten the block's q/k/v rows of a cached window."""
