@@ -34,8 +34,8 @@ DATASHEET_BF16_TFLOPS = 2250.0
 # dram__bytes_read.sum + dram__bytes_write.sum per GEMM launch, averaged over the GEMM launches of one training step
 # in a one-pass ncu launch list of this command (summary kept under profiles/), and the first 16 hex digits of the
 # SHA-256 of the GEMM sources the capture ran with: kernels changed since then get no traffic figure, not a stale one.
-GEMM_DRAM_BYTES_PER_LAUNCH = 220.4e6
-GEMM_SOURCE_AT_CAPTURE = "25910fe13dba10e2"
+GEMM_DRAM_BYTES_PER_LAUNCH = 212.5e6
+GEMM_SOURCE_AT_CAPTURE = "c10b8156a301e97f"
 
 
 def gemm_traffic():
