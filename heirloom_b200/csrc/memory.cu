@@ -1672,10 +1672,19 @@ int hl_product_key_side_scores_f32(hl_ctx* ctx, const float* query, long long ld
   return HL_OK;
 }
 
-// product_key_pieces and product_key_lookup for a caller that brings all buffers (the step has its own).
 int hl_product_key_lookup(hl_ctx* ctx, const float* query, const float* left_keys, const float* right_keys, void* pieces, void* query_pieces,
                           float* left_approx, float* right_approx, int64_t* out, int tokens, int side, int key_dim, int top_k, int beam) {
-  if (tokens < 1 || !product_key_lookup_takes(side, key_dim, beam)) return fail("hl_product_key_lookup: sizes of the general form");
+  HL_REQUIRE(ctx && query && left_keys && right_keys && pieces && query_pieces && left_approx && right_approx && out,
+             "hl_product_key_lookup: null argument");
+  HL_REQUIRE(tokens > 0 && side > 0 && key_dim > 0, "hl_product_key_lookup: requires non-zero sizes");
+  HL_REQUIRE(beam > 0 && beam <= 32 && beam <= side, "hl_product_key_lookup: beam must be in [1, min(32, side)]");
+  HL_REQUIRE(top_k > 0 && top_k <= beam * beam, "hl_product_key_lookup: top_k must be in [1, beam^2]");
+  HL_REQUIRE(product_key_lookup_takes(side, key_dim, beam),
+             "hl_product_key_lookup: side must be a multiple of 8 up to 512, key_dim a multiple of 64 up to 1024");
+  HL_REQUIRE(((reinterpret_cast<uintptr_t>(query) | reinterpret_cast<uintptr_t>(left_keys) | reinterpret_cast<uintptr_t>(right_keys) |
+               reinterpret_cast<uintptr_t>(pieces) | reinterpret_cast<uintptr_t>(query_pieces) | reinterpret_cast<uintptr_t>(left_approx) |
+               reinterpret_cast<uintptr_t>(right_approx)) & 15) == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0,
+             "hl_product_key_lookup: pointers must be 16-byte aligned");
   const int rc = product_key_pieces(ctx, left_keys, right_keys, side, key_dim, pieces);
   if (rc != HL_OK) return rc;
   return product_key_lookup(ctx, query, left_keys, right_keys, pieces, static_cast<__nv_bfloat16*>(query_pieces), left_approx, right_approx, out,

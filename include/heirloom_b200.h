@@ -342,6 +342,13 @@ int hl_product_key_side_scores_f32(hl_ctx* ctx, const float* query, long long ld
  * slot = left*side + right (src/memory_transformer.rs:847-924; kernels.ptx:2121).  beam <= 32. */
 int hl_product_key_topk_from_side_scores(hl_ctx* ctx, const float* left_scores, const float* right_scores,
                                          int64_t* out, int tokens, int side, int top_k, int beam);
+/* The two above in one, with the same slots bit by bit: the tensor cores form all side scores approximately, out of bf16 pieces, and
+ * what may be selected is summed exactly.  side a multiple of 8 up to 512, key_dim of 64 up to 1024; query [tokens, key_dim].  Scratch
+ * of the caller: pieces 6 * side * key_dim + 256 bytes, query_pieces 4 * tokens * key_dim bytes, left_approx and right_approx
+ * [tokens, side]; all pointers on 16 bytes. */
+int hl_product_key_lookup(hl_ctx* ctx, const float* query, const float* left_keys, const float* right_keys, void* pieces,
+                          void* query_pieces, float* left_approx, float* right_approx, int64_t* out, int tokens,
+                          int side, int key_dim, int top_k, int beam);
 /* row / side and row % side (src/tensor.rs:1654-1719; kernels.ptx:2263). */
 int hl_product_key_split_rows(hl_ctx* ctx, const int64_t* rows, int64_t* left, int64_t* right, long long n, int side);
 /* Differentiable re-scoring of the chosen slots.  side > 0: product-key tables

@@ -547,3 +547,32 @@ def test_lookup_of_values_whose_pieces_are_at_their_worst(tokens, side, key_dim,
         assert off.max() <= 2 ** -15 + 3 * half / 16 * 17 * 2 ** -23
         seen = max(seen, off.max())
     assert seen > 3 * 2 ** -18
+
+
+def test_lookup_refuses_what_its_kernels_cannot_take():
+    """On the host, before anything is launched: sizes of the general form, more slots than the beams have pairs, no pointer, and one that
+    sixteen-byte loads cannot read."""
+    from ctypes import c_int, c_void_p
+
+    from heirloom_b200 import cuda
+    c = ctx()
+    room = torch.zeros(1 << 20, dtype=torch.uint8, device="cuda")
+    at = lambda i: c_void_p(room.data_ptr() + 65536 * i)
+
+    def refused(match, tokens=4, side=16, key_dim=64, top_k=4, beam=4, **pointers):
+        p = [pointers.get(n, at(i)) for i, n in enumerate(("query", "left", "right", "pieces", "query_pieces", "left_approx", "right_approx", "out"))]
+        with pytest.raises(cuda.HeirloomError, match=match):
+            cuda.check(c.lib.hl_product_key_lookup(c.handle, *p, c_int(tokens), c_int(side), c_int(key_dim), c_int(top_k), c_int(beam)))
+    before = c.counters().launches
+    for sizes in (dict(side=12), dict(side=520), dict(key_dim=96), dict(key_dim=1088)):
+        refused("must be a multiple", **sizes)
+    refused("top_k", top_k=17)
+    refused("top_k", top_k=0)
+    refused("beam", beam=17)
+    refused("beam", side=64, beam=33)
+    refused("non-zero", tokens=0)
+    for i, name in enumerate(("query", "left", "right", "pieces", "query_pieces", "left_approx", "right_approx", "out")):
+        refused("null", **{name: c_void_p(0)})
+        refused("aligned", **{name: c_void_p(room.data_ptr() + 65536 * i + 4)})
+    assert c.counters().launches == before
+    c.sync()
