@@ -134,7 +134,7 @@ struct hl_decoder {
   cudaEvent_t zero_event = nullptr;  // the scattered gradients have been zeroed there
   cudaEvent_t sort_event = nullptr;  // the selections that the forward pass has left so far are in row order
   void* sort_scratch = nullptr;      // of those sorts, one at a time
-  bool lookup = false;               // passes over whole windows select by product_key_lookup
+  bool lookup = false;               // buffers for product_key_lookup are there (looks_up: whether a pass takes it)
   void* key_pieces = nullptr;        // of the half keys, made at the start of every pass
   __nv_bfloat16* query_pieces = nullptr;
   bool sorted = false;               // this pass sorts them there
@@ -373,6 +373,12 @@ size_t memory_side_bytes(const hl_decoder* m) {
   return most;
 }
 
+// Exact scores of all keys and the selection take 421 us a block at 16384 tokens, sides of 512 and keys of 512, the lookup 276; steps with
+// two blocks, all keys against the lookup: 1102 and 1020 us at 128 tokens of the same tables, 869 and 861 at 2048 tokens, sides of 128 and
+// keys of 64, 690 and 708 at 512 tokens of these.  It is the pass's own tokens that count: a prompt may be far shorter than the model's batch.
+constexpr size_t kLookupProducts = size_t(1) << 24;  // tokens * side * key_dim
+bool looks_up(const hl_decoder* m) { return m->lookup && (size_t)m->N * m->side * m->mem.key_dim >= kLookupProducts; }
+
 // Buffers of the memory feed-forward blocks; appended to either route's arena.
 void plan_memory_buffers(hl_decoder* m, uint8_t*& cur) {
   m->tok_flags = carve<unsigned char>(cur, (size_t)m->cfg.vocab);
@@ -413,10 +419,7 @@ void plan_memory_buffers(hl_decoder* m, uint8_t*& cur) {
   m->m_dw = carve<float>(cur, N * k);
   m->m_dscores = carve<float>(cur, N * k);
   m->m_dq = carve<float>(cur, N * kd);
-  // Exact scores of all keys and the selection take 421 us a block at 16384 tokens, sides of 512 and keys of 512, the lookup 276; steps with
-  // two blocks, all keys against the lookup: 1102 and 1020 us at 128 tokens of the same tables, 869 and 861 at 2048 tokens, sides of 128 and
-  // keys of 64, 690 and 708 at 512 tokens of these.
-  m->lookup = !m->lean && N * m->side * kd >= (1ull << 24) && product_key_lookup_takes(m->side, (int)kd, (int)k);
+  m->lookup = !m->lean && N * m->side * kd >= kLookupProducts && product_key_lookup_takes(m->side, (int)kd, (int)k);
   if (m->cfg.precision == HL_PRECISION_AMP_BF16) {
     m->p_dx_side = carve<__nv_bfloat16>(cur, N * 2 * d);
     m->p_dx_rows = carve<__nv_bfloat16>(cur, 2 * N * d);
@@ -749,7 +752,7 @@ int memory_core_forward(hl_decoder* m, int l, bool one_token = false) {
   const float* P = m->params;
   const int N = m->N, kd = m->mem.key_dim, vd = m->mem.value_dim, k = m->mem.top_k, side = m->side;
   const int beam = std::min(side, std::max(k, (int)ceil(sqrt((double)k))));  // product_key_beam, :2014-2016
-  if (!one_token && m->lookup) {
+  if (!one_token && looks_up(m)) {
     HL_TRY(product_key_lookup(ctx, a.query, P + m->off_kl, P + m->off_kr, m->key_pieces, m->query_pieces, m->m_ls, m->m_rs, idx, N, side, kd, k, beam));
   } else {
     ProfileScope prof(ctx, HL_PROF_OTHER, 2.0 * (double)N * side * 4.0);
@@ -772,7 +775,7 @@ int memory_core_forward(hl_decoder* m, int l, bool one_token = false) {
 
 // What every memory block's lookup of a pass reads of the tables, which all of them share.
 int prepare_lookups(hl_decoder* m) {
-  if (!m->lookup) return HL_OK;
+  if (!looks_up(m)) return HL_OK;
   return product_key_pieces(m->ctx, m->params + m->off_kl, m->params + m->off_kr, m->side, m->mem.key_dim, m->key_pieces);
 }
 

@@ -366,3 +366,23 @@ def test_gradients_beside_the_backward_pass_with_tiles_from_a_counter(monkeypatc
     c.sync()
     want = a.float() @ b.float().T
     assert (out - want).norm() <= 1e-3 * want.norm()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_a_short_prompt_takes_the_kernels_of_its_own_length(precision):
+    """Whether a pass selects by the lookup depends on its own tokens: a prompt of ten takes as many launches in a model made for 4 x 128
+    tokens (2^24 products of tokens, side and key_dim and more) as in one for 128, and gives the same logits."""
+    from heirloom_b200 import generation, nn
+    c = ctx()
+    mem = dict(MEM, slots=128 * 128, key_dim=256)
+    runs = []
+    for batch in (1, 4):
+        model = nn.DecoderLm(c, nn.DecoderConfig(batch=batch, precision=nn.PRECISION_AMP_BF16 if precision else nn.PRECISION_F32, **KW),
+                             nn.MemoryConfig(**mem))
+        model.load_state_dict(ho.init_memory_parameters(ho.DecoderConfig(**KW), ho.MemoryConfig(**mem), 3))
+        before = c.counters().launches
+        logits = generation.next_token_logits(model, list(range(10)))
+        runs.append((c.counters().launches - before, logits))
+        model.close()
+    assert runs[0][0] == runs[1][0]
+    np.testing.assert_array_equal(runs[0][1], runs[1][1])
