@@ -1746,15 +1746,19 @@ int hl_memory_selected_scores_backward(hl_ctx* ctx, const int64_t* indices, cons
   // the tensor-core form's scratch holds the queries' pieces as well: where the device has no room for them, the f32 form
   const bool tensor = token_blocks > 0 && try_workspace(ctx, key_gradient_bytes(keys, token_blocks));
   int* clear = tensor ? static_cast<int*>(ctx->workspace) : nullptr;
-  if (side > 0 && grad_query && rows_of_16_bytes(key_dim, ld_grad_query, grad_query, left_or_keys, right_keys))
-    pdl(selected_query_gradient_kernel, (unsigned)ceil_div_ll((long long)tokens * ceil_div(key_dim, 128), 4), 128, 0, ctx->stream)(
-        indices, left_or_keys, right_keys, grad_scores, grad_query, ld_grad_query, tokens, top_k, side, key_dim, slots, clear);
-  else
-    pdl(selected_scores_bwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream)(
-        indices, query, ld_query, left_or_keys, right_keys, grad_scores, grad_query, ld_grad_query, grad_left_or_keys,
-        grad_right_keys, tokens, top_k, side, key_dim, slots, clear);
-  HL_LAUNCH_CHECK("selected_scores_bwd_kernel");
-  count_launch(ctx);
+  if (side > 0 && !grad_query) {  // the tables' gradients alone
+    if (clear) HL_CUDA(cudaMemsetAsync(clear, 0, sizeof(int), ctx->stream));
+  } else {
+    if (side > 0 && rows_of_16_bytes(key_dim, ld_grad_query, grad_query, left_or_keys, right_keys))
+      pdl(selected_query_gradient_kernel, (unsigned)ceil_div_ll((long long)tokens * ceil_div(key_dim, 128), 4), 128, 0, ctx->stream)(
+          indices, left_or_keys, right_keys, grad_scores, grad_query, ld_grad_query, tokens, top_k, side, key_dim, slots, clear);
+    else
+      pdl(selected_scores_bwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream)(
+          indices, query, ld_query, left_or_keys, right_keys, grad_scores, grad_query, ld_grad_query, grad_left_or_keys,
+          grad_right_keys, tokens, top_k, side, key_dim, slots, clear);
+    HL_LAUNCH_CHECK("selected_scores_bwd_kernel");
+    count_launch(ctx);
+  }
   if (half_keys) {
     const int col_blocks = ceil_div(half, DK_COLS), row_blocks = ceil_div(side, DK_ROWS);
     if (!tensor) {

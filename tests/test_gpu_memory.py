@@ -576,3 +576,35 @@ def test_lookup_refuses_what_its_kernels_cannot_take():
         refused("aligned", **{name: c_void_p(room.data_ptr() + 65536 * i + 4)})
     assert c.counters().launches == before
     c.sync()
+
+
+@pytest.mark.parametrize("tokens", [65, 2048])
+def test_half_key_gradients_without_the_querys(tokens):
+    """A call for the tables' gradients alone gives the bits of one for all three, with a launch fewer; also behind a call whose
+    values are too wide for bf16 pieces, which sets a word that every call of that form clears."""
+    from ctypes import c_int, c_longlong, c_void_p
+
+    from heirloom_b200 import cuda
+    c = ctx()
+    rng = np.random.default_rng(tokens)
+    side, key_dim, top_k = 24, 64, 8
+    q, g = dev(rng.standard_normal((tokens, key_dim)).astype(np.float32)), dev(rng.standard_normal((tokens, top_k)).astype(np.float32))
+    kl, kr = (dev(rng.standard_normal((side, key_dim // 2)).astype(np.float32)) for _ in range(2))
+    idx = dev(rng.integers(0, side * side, (tokens, top_k)), I64)
+
+    def tables(query):
+        dl, dr = torch.zeros_like(kl), torch.zeros_like(kr)
+        cuda.check(c.lib.hl_memory_selected_scores_backward(
+            c.handle, cuda._p(idx), cuda._p(query), c_longlong(key_dim), cuda._p(kl), cuda._p(kr), cuda._p(g), c_void_p(0), c_longlong(key_dim),
+            cuda._p(dl), cuda._p(dr), c_int(tokens), c_int(top_k), c_int(side), c_int(key_dim), c_int(side * side)))
+        return dl, dr
+    before = c.counters().launches
+    _, dl, dr = cuda.memory_selected_scores_backward(c, idx, q, kl, kr, g)
+    whole = c.counters().launches - before
+    wide = q.clone()
+    wide[3, 5] = 2.0 ** 50
+    for query in (q, wide, q):
+        before = c.counters().launches
+        got = tables(query)
+        assert c.counters().launches - before == whole - 1
+    assert torch.equal(got[0], dl) and torch.equal(got[1], dr)
