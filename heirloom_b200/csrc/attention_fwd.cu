@@ -19,8 +19,8 @@
 // of that memory's traffic, which was three quarters of what an SM can do (heads of 128: B4 H12 T4096 211.7 us with it, now 200.5).
 //
 // Work items go round persistent streams without a gap, several of them on an SM, so that one's tensor work and waits lie under
-// another's exponentials.  Heads of 128 have room for two, a CTA each (192 threads, 112 KB of shared memory, 256 tensor-memory columns);
-// heads of 64 for three in one CTA (below).  With a CTA per item (heads of 64, B16 H12 T1024: 69 us) 29 us were starts and ends.
+// another's exponentials: two streams, a CTA each (192 threads, 56 or 112 KB of shared memory, 256 tensor-memory columns), or, for heads of
+// 64 in many items, three in one CTA (below).  With a CTA per item (heads of 64, B16 H12 T1024: 69 us) 29 us were starts and ends.
 #include <type_traits>
 
 #include "common.cuh"
@@ -35,16 +35,18 @@ constexpr int FA_SOFTMAX_WARPS = 4;
 constexpr int FA_THREADS = (FA_SOFTMAX_WARPS + 2) * 32;  // + TMA warp + MMA warp
 constexpr int FA_TMEM_COLS = 256;  // S: 2 x 64 columns, O: head_dim columns (allocations are powers of two)
 
-// Heads of 128 channels.  Operands wider than one 128-byte swizzle row are kept as blocks of 64 channels side by side: a Q block is
-// [128 rows x 128 bytes], a K or V block [64 keys x 128 bytes].
-constexpr int FA_HD = 128, FA_BLOCKS = FA_HD / 64;
+// A CTA with one stream of items.  Operands wider than one 128-byte swizzle row are kept as blocks of 64 channels side by side: a Q
+// block is [128 rows x 128 bytes], a K or V block [64 keys x 128 bytes].
 constexpr int FA_K_STAGES = 3, FA_V_STAGES = 2;
 constexpr int FA_Q_BLOCK = FA_BM * 128, FA_KV_BLOCK = FA_BN * 128;
-constexpr int FA_Q_BYTES = FA_BLOCKS * FA_Q_BLOCK, FA_KV_BYTES = FA_BLOCKS * FA_KV_BLOCK;
-constexpr int FA_DATA = FA_Q_BYTES + (FA_K_STAGES + FA_V_STAGES) * FA_KV_BYTES;  // 112 KB
-constexpr int FA_SMEM = FA_DATA + 256;                                           // barriers behind the tiles
-static_assert(2 * (FA_SMEM + 1024) <= 228 * 1024, "shared memory per SM");
-static_assert(2 * FA_BN + FA_HD <= FA_TMEM_COLS, "tensor memory columns");
+template <int HD>
+struct FaShape {
+  static constexpr int BLOCKS = HD / 64, Q_BYTES = BLOCKS * FA_Q_BLOCK, KV_BYTES = BLOCKS * FA_KV_BLOCK;
+  static constexpr int DATA = Q_BYTES + (FA_K_STAGES + FA_V_STAGES) * KV_BYTES;  // 56 or 112 KB
+  static constexpr int SMEM = DATA + 256;                                        // barriers behind the tiles
+  static_assert(2 * (SMEM + 1024) <= 228 * 1024, "shared memory per SM");
+  static_assert(2 * FA_BN + HD <= FA_TMEM_COLS, "tensor memory columns");
+};
 
 struct FaShared {
   uint64_t q_full, q_empty;
@@ -58,8 +60,6 @@ static_assert(sizeof(FaShared) <= 256, "barriers outgrow their place");
 
 struct FaParams {
   int B, T, H;
-  long long ld_out;
-  __nv_bfloat16* out;
   float* lse;
   QuickDiv by_heads, by_h;  // all heads, a batch entry's
   float scale_log2;  // softmax scale times log2(e)
@@ -86,15 +86,17 @@ __device__ __forceinline__ FaItem fa_item(int local, const FaParams& p, int cta,
 
 __device__ __forceinline__ FaItem fa_item(int local, const FaParams& p) { return fa_item(local, p, (int)blockIdx.x, (int)gridDim.x); }
 
+template <int HD>
 __global__ void __launch_bounds__(FA_THREADS, 2)
-flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+flash_attention_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                            const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
                            const FaParams p) {
+  using Z = FaShape<HD>;
   extern __shared__ __align__(1024) uint8_t fa_smem[];  // swizzled tiles want 1024 bytes; checked below
   uint8_t* sq = fa_smem;
-  uint8_t* sk = sq + FA_Q_BYTES;
-  uint8_t* sv = sk + FA_K_STAGES * FA_KV_BYTES;
-  FaShared* sh = reinterpret_cast<FaShared*>(fa_smem + FA_DATA);
+  uint8_t* sk = sq + Z::Q_BYTES;
+  uint8_t* sv = sk + FA_K_STAGES * Z::KV_BYTES;
+  FaShared* sh = reinterpret_cast<FaShared*>(fa_smem + Z::DATA);
   const bool layout_ok = (tc05::smem_u32(fa_smem) & 1023u) == 0;
   volatile int* abort_flag = &sh->abort_flag;
 
@@ -140,25 +142,25 @@ flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
       int g = 0;  // key tiles loaded so far
       for (FaItem it = fa_item(0, p); ok && it.n_tiles > 0; it = fa_item(it.local + 1, p)) {
         if (!tc05::mbar_wait(&sh->q_empty, ((uint32_t)it.local & 1u) ^ 1u, abort_flag)) break;
-        tc05::mbar_arrive_expect_tx(&sh->q_full, FA_Q_BYTES);
+        tc05::mbar_arrive_expect_tx(&sh->q_full, Z::Q_BYTES);
 #pragma unroll
-        for (int blk = 0; blk < FA_BLOCKS; ++blk)
-          tc05::tma_load_3d(sq + blk * FA_Q_BLOCK, &map_q, &sh->q_full, it.h * FA_HD + blk * 64, it.q0, it.b);
+        for (int blk = 0; blk < Z::BLOCKS; ++blk)
+          tc05::tma_load_3d(sq + blk * FA_Q_BLOCK, &map_q, &sh->q_full, it.h * HD + blk * 64, it.q0, it.b);
         for (int j = 0; j < it.n_tiles; ++j, ++g) {
           const int s = g % FA_K_STAGES, vs = g % FA_V_STAGES;
           ok = tc05::mbar_wait(&sh->k_empty[s], ((uint32_t)(g / FA_K_STAGES) & 1u) ^ 1u, abort_flag);
           if (!ok) break;
-          tc05::mbar_arrive_expect_tx(&sh->k_full[s], FA_KV_BYTES);
+          tc05::mbar_arrive_expect_tx(&sh->k_full[s], Z::KV_BYTES);
 #pragma unroll
-          for (int blk = 0; blk < FA_BLOCKS; ++blk)
-            tc05::tma_load_3d(sk + s * FA_KV_BYTES + blk * FA_KV_BLOCK, &map_k, &sh->k_full[s], it.h * FA_HD + blk * 64,
+          for (int blk = 0; blk < Z::BLOCKS; ++blk)
+            tc05::tma_load_3d(sk + s * Z::KV_BYTES + blk * FA_KV_BLOCK, &map_k, &sh->k_full[s], it.h * HD + blk * 64,
                               j * FA_BN, it.b);
           ok = tc05::mbar_wait(&sh->v_empty[vs], ((uint32_t)(g / FA_V_STAGES) & 1u) ^ 1u, abort_flag);
           if (!ok) break;
-          tc05::mbar_arrive_expect_tx(&sh->v_full[vs], FA_KV_BYTES);
+          tc05::mbar_arrive_expect_tx(&sh->v_full[vs], Z::KV_BYTES);
 #pragma unroll
-          for (int blk = 0; blk < FA_BLOCKS; ++blk)
-            tc05::tma_load_3d(sv + vs * FA_KV_BYTES + blk * FA_KV_BLOCK, &map_v, &sh->v_full[vs], it.h * FA_HD + blk * 64,
+          for (int blk = 0; blk < Z::BLOCKS; ++blk)
+            tc05::tma_load_3d(sv + vs * Z::KV_BYTES + blk * FA_KV_BLOCK, &map_v, &sh->v_full[vs], it.h * HD + blk * 64,
                               j * FA_BN, it.b);
         }
       }
@@ -167,7 +169,7 @@ flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
     // -------------------------------------------------------------------------- MMA issuer
     if (tc05::elect_one() && !*abort_flag) {
       constexpr uint32_t idesc_qk = tc05::instr_desc_bf16_f32(FA_BM, FA_BN, false, false);
-      constexpr uint32_t idesc_pv = tc05::instr_desc_bf16_f32(FA_BM, FA_HD, false, true);
+      constexpr uint32_t idesc_pv = tc05::instr_desc_bf16_f32(FA_BM, HD, false, true);
       // Q·Kᵀ runs two tiles ahead of P·V, into the next item where this one ends.
       FaItem qi = fa_item(0, p);
       int qj = 0, qg = 0;  // the next scores: tile of the item, tile of the CTA
@@ -179,9 +181,9 @@ flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
         // P·V of two tiles before reads the P that stands here: products of other sizes are not kept in order
         if (qg >= 2 && !tc05::mbar_wait(&sh->o_full[qg & 1], (uint32_t)((qg - 2) >> 1) & 1u, abort_flag)) return false;
         tc05::tc_fence_after_sync();
-        const uint32_t aq = tc05::smem_u32(sq), ak = tc05::smem_u32(sk + s * FA_KV_BYTES);
+        const uint32_t aq = tc05::smem_u32(sq), ak = tc05::smem_u32(sk + s * Z::KV_BYTES);
 #pragma unroll
-        for (int ks = 0; ks < FA_HD / 16; ++ks)  // 16 channels a step; four steps per 64-channel block
+        for (int ks = 0; ks < HD / 16; ++ks)  // 16 channels a step; four steps per 64-channel block
           tc05::umma_ss(tmem_s0 + (uint32_t)((qg & 1) * FA_BN),
                         tc05::smem_desc_sw128(aq + (ks / 4) * FA_Q_BLOCK + (ks % 4) * 32, 16, 1024),
                         tc05::smem_desc_sw128(ak + (ks / 4) * FA_KV_BLOCK + (ks % 4) * 32, 16, 1024), idesc_qk,
@@ -214,7 +216,7 @@ flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
           const int s = g % FA_V_STAGES;
           if (!tc05::mbar_wait(&sh->v_full[s], (uint32_t)(g / FA_V_STAGES) & 1u, abort_flag)) { ok = false; break; }
           tc05::tc_fence_after_sync();
-          const uint32_t av = tc05::smem_u32(sv + s * FA_KV_BYTES);
+          const uint32_t av = tc05::smem_u32(sv + s * Z::KV_BYTES);
 #pragma unroll
           for (int ks = 0; ks < FA_BN / 16; ++ks) {
             // A = P, two keys a column; B = V: rows are keys (MN-major), 16 keys per step, channel blocks FA_KV_BLOCK apart
@@ -283,7 +285,7 @@ flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
         if (raise) m_ref = m_new;
         l_run *= a;
 #pragma unroll
-        for (int hb = 0; hb < FA_HD / 32; ++hb) {
+        for (int hb = 0; hb < HD / 32; ++hb) {
           uint32_t ob[32];
           tc05::tmem_ld_32x32b_x32(tmem_o0 + lane_sel + hb * 32, ob);
           tc05::tmem_ld_wait();
@@ -325,7 +327,7 @@ flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
       // the tensor map.
       const float inv = 1.0f / l_run;
 #pragma unroll
-      for (int hb = 0; hb < FA_HD / 32; ++hb) {
+      for (int hb = 0; hb < HD / 32; ++hb) {
         uint32_t ob[32];
         tc05::tmem_ld_32x32b_x32(tmem_o0 + lane_sel + hb * 32, ob);
         tc05::tmem_ld_wait();
@@ -345,8 +347,8 @@ flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
       __syncwarp();
       if (lane == 0) {
 #pragma unroll
-        for (int blk = 0; blk < FA_BLOCKS; ++blk)
-          tc05::tma_store_3d(&map_o, sq + blk * FA_Q_BLOCK + warp * (32 * 128), it.h * FA_HD + blk * 64, it.q0 + warp * 32, it.b);
+        for (int blk = 0; blk < Z::BLOCKS; ++blk)
+          tc05::tma_store_3d(&map_o, sq + blk * FA_Q_BLOCK + warp * (32 * 128), it.h * HD + blk * 64, it.q0 + warp * 32, it.b);
         tc05::tma_store_commit();
         tc05::tma_store_wait_read();  // the next item's Q waits for it
         tc05::mbar_arrive(&sh->q_empty);
@@ -372,7 +374,7 @@ flash_attention_fwd128_kernel(const __grid_constant__ CUtensorMap map_q, const _
   }
 }
 
-// ---- heads of 64 channels ---------------------------------------------------------------------------------------------------
+// ---- heads of 64 channels, many items ---------------------------------------------------------------------------------------
 // What bounds these is the softmax: 64 exponentials a row and tile are 512 cycles of a scheduler's, the products 256.  A warp's chain (scores,
 // maximum, exponentials, hand-over) takes three times that, so that three warps share a scheduler: one CTA an SM walks three streams
 // of items side by side, each with its own tiles, four softmax warps and a warp whose elected thread queues both loads and products
@@ -679,6 +681,15 @@ flash_attention_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __
   }
 }
 
+// Three streams an SM are more work at a time, two are faster each (0.86 and 0.67 us a tile of a stream that is alone), and a call
+// lasts no less than its longest item.  So three where an SM's share of the tiles is a few times that item: share / longest of
+// 1.9 + (rows / 128) / 16, and up to 2048 rows.  Two / three streams, us: B16 T512 H8 15.8 / 13.8, B16 T1024 H12 59.6 / 51.1, B16 T1024 H5
+// 24.8 / 24.1, B8 T1024 H8 20.8 / 22.5, B4 T2048 H16 62.3 / 61.6, B4 T2048 H10 39.5 / 42.6, B5 T700 H13 14.4 / 16.9, B1 T4096 H16 55 / 75, B1 T4096
+// H24 84.6 / 84.1, B2 T4096 H20 133 / 139, B1 T8192 H32 391 / 407.
+bool three_streams(int items, int tiles, int sms) {
+  return tiles <= 16 && 8ll * items * (tiles + 1) >= (long long)sms * tiles * (30 + tiles);
+}
+
 }  // namespace
 
 int flash_attention_forward_impl(hl_ctx* ctx, const void* q, const void* k, const void* v, long long ld_qkv, void* out,
@@ -714,23 +725,23 @@ int flash_attention_forward_impl(hl_ctx* ctx, const void* q, const void* k, cons
   }
   FaParams p{};
   p.B = batch; p.T = time; p.H = n_heads;
-  p.ld_out = ld_out;
-  p.out = reinterpret_cast<__nv_bfloat16*>(out);
   p.lse = lse;
   p.by_heads = QuickDiv((uint32_t)(batch * n_heads));
   p.by_h = QuickDiv((uint32_t)n_heads);
   p.scale_log2 = (1.0f / sqrtf((float)head_dim)) * 1.4426950408889634f;
   p.status = ctx->status_dev;
-  const int grid = std::min(ceil_div(time, FA_BM) * batch * n_heads, 2 * persistent_sms(ctx));
+  const int sms = persistent_sms(ctx), tiles = ceil_div(time, FA_BM), items = tiles * batch * n_heads;
   // causal algorithmic work: QK^T and PV over the lower triangle
   ProfileScope prof(ctx, HL_PROF_ATTENTION_FWD, 2.0 * batch * n_heads * (double)time * time * head_dim);
-  if (head_dim == 64) {
+  if (head_dim == 64 && three_streams(items, tiles, sms)) {
     HL_ALLOW_SHARED(ctx, F3_SMEM, flash_attention_fwd64_kernel);
-    pdl(flash_attention_fwd64_kernel, std::min(ceil_div(time, FA_BM) * batch * n_heads, persistent_sms(ctx)), F3_THREADS, F3_SMEM, ctx->stream)(
-        mq, mk, mv, mo, p);
+    pdl(flash_attention_fwd64_kernel, std::min(items, sms), F3_THREADS, F3_SMEM, ctx->stream)(mq, mk, mv, mo, p);
+  } else if (head_dim == 64) {
+    HL_ALLOW_SHARED(ctx, FaShape<64>::SMEM, flash_attention_fwd_kernel<64>);
+    pdl(flash_attention_fwd_kernel<64>, std::min(items, 2 * sms), FA_THREADS, FaShape<64>::SMEM, ctx->stream)(mq, mk, mv, mo, p);
   } else {
-    HL_ALLOW_SHARED(ctx, FA_SMEM, flash_attention_fwd128_kernel);
-    pdl(flash_attention_fwd128_kernel, grid, FA_THREADS, FA_SMEM, ctx->stream)(mq, mk, mv, mo, p);
+    HL_ALLOW_SHARED(ctx, FaShape<128>::SMEM, flash_attention_fwd_kernel<128>);
+    pdl(flash_attention_fwd_kernel<128>, std::min(items, 2 * sms), FA_THREADS, FaShape<128>::SMEM, ctx->stream)(mq, mk, mv, mo, p);
   }
   HL_LAUNCH_CHECK("flash_attention_fwd_kernel");
   count_launch(ctx);

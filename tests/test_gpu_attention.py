@@ -101,6 +101,22 @@ def test_flash_backward_gives_the_same_dk_and_dv_every_time(B, T, H, hd):
         assert torch.equal(again[:, C:], first[:, C:])
 
 
+@pytest.mark.parametrize("T,H", [(128, 12), (300, 8), (1000, 5), (2048, 4)])
+def test_flash_forward_of_a_batch_equals_its_entries(T, H):
+    """Heads of 64 take three streams an SM where there are many items and two where there are few: the same sums in the same order."""
+    from heirloom_b200 import cuda
+    c = ctx()
+    C, B = 64 * H, 40
+    qkv = torch.randn(B * T, 3 * C, device="cuda", generator=torch.Generator(device="cuda").manual_seed(T)).to(torch.bfloat16)
+    q, k, v = qkv.split(C, dim=1)
+    out, lse = cuda.flash_attention_forward(c, q, k, v, B, T, H)
+    for b in (0, 17, 39):
+        rows = slice(b * T, (b + 1) * T)
+        alone = cuda.flash_attention_forward(c, q[rows], k[rows], v[rows], 1, T, H)
+        c.sync()
+        assert torch.equal(alone[0], out[rows]) and torch.equal(alone[1].reshape(-1), lse[b].reshape(-1))
+
+
 def test_flash_forward_rejects_unsupported_shapes():
     from heirloom_b200 import cuda
     from heirloom_b200._lib import HeirloomError
