@@ -705,26 +705,40 @@ __device__ __forceinline__ int sum8_index() { return (threadIdx.x & 31) >> 2; } 
 
 // The kernels that gather table rows (selected scores and weighted value, forward and backward) are bound by how many rows are on
 // their way: by L2 for many tokens (16384 tokens of 32 rows of 2 KB: 50 to 100 us a kernel), and for few by latency, since with a warp
-// a token, a row after the other, 2048 tokens keep a tenth of the memory busy.  So a warp takes eight rows at a time, and where
-// columns do not meet, 128 of the columns only.  Scores, their gradient and value at 2048 tokens 21, 31 and 37 -> 13, 12 and 21 us, at 16384 tokens
-// 100, 67 and 51 -> 64, 61 and 53.
+// a token, a row after the other, 2048 tokens keep a tenth of the memory busy.  So a warp asks for eight pieces of rows at a time, and where
+// columns do not meet, for a few of a row's pieces only (by_pieces).  Scores, their gradient and value of 32 slots of 512 columns at 2048
+// tokens 21, 25 and 18 -> 13, 9 and 10 us, at 16384 tokens 100, 77 and 72 -> 64, 53 and 57.
 constexpr int GATHER = 8;
 __device__ __forceinline__ float4 row_piece(const float* table, long long row, int dim, int piece, bool on) {
   return on && row >= 0 ? __ldg(reinterpret_cast<const float4*>(table + (size_t)row * dim) + piece) : make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
+__device__ __forceinline__ void add_scaled(float4& acc, float w, const float4& v) {
+  acc.x = fmaf(w, v.x, acc.x); acc.y = fmaf(w, v.y, acc.y); acc.z = fmaf(w, v.z, acc.z); acc.w = fmaf(w, v.w, acc.w);
+}
+// launch(pieces of a row a lane has): as many as leave a warp several rows on their way, and more where a token has a slot or two, so
+// that as many bytes are asked for.  Value of 16384 tokens of 512 columns, one, two, four pieces, us: 1 slot 18.8, 10.4, 8.0, 8 slots 23.4,
+// 17.9, 17.7, 32 slots 65, 57, 57; 2048 tokens of 32 slots 13.1, 10.2, 10.3; 64 tokens 5.6, 4.1, 6.1.
+template <typename F> void by_pieces(int top_k, int dim, F launch) {
+  if (dim <= 128) launch(std::integral_constant<int, 1>{});
+  else if (dim <= 256 || top_k > 2) launch(std::integral_constant<int, 2>{});
+  else launch(std::integral_constant<int, 4>{});
+}
+
 // ---- selected scores: score[t,k] = q_L . K_L[idx/side] + q_R . K_R[idx%side]  (src/tensor.rs:3593-3769).
-// Product-key form, key_dim up to 128 U, sixteen-byte rows: a CTA of four warps a token, eight of every 32 slots each; the query sits
-// in registers.  A lane's share (at most 4 U products) is summed in f32, the 32 shares in f64: f64 multiply-adds run at a
+// Product-key form, key_dim up to 128 U, sixteen-byte rows: one, two or four warps a token, eight slots each at a time (a CTA a token left
+// three of its warps idle for up to eight slots: 2048 tokens of 8 slots of 512 columns 14.4 us, 10.0 before that); the query sits in registers.  A lane's share (at most 4 U products) is summed in f32, the 32 shares in f64: f64 multiply-adds run at a
 // fraction of the f32 rate.
 template <int U>
 __global__ void __launch_bounds__(128)
 selected_scores_rows_kernel(const int64_t* __restrict__ idx, const float* __restrict__ query, long long ld_q,
-                            const float* __restrict__ left, const float* __restrict__ right, float* __restrict__ scores, int top_k,
-                            int side, int key_dim, int slots, int* __restrict__ status) {
+                            const float* __restrict__ left, const float* __restrict__ right, float* __restrict__ scores, int tokens,
+                            int top_k, int side, int key_dim, int slots, int log_warps, int* __restrict__ status) {
   pdl_begin();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const size_t token = blockIdx.x;
+  const int lane = threadIdx.x & 31, w = (int)blockIdx.x * 4 + (int)(threadIdx.x >> 5);
+  if (w >> log_warps >= tokens) return;
+  const size_t token = w >> log_warps;
+  const int first = (w & ((1 << log_warps) - 1)) * GATHER, step = GATHER << log_warps;
   const int half = key_dim / 2, groups = key_dim / 4, half_groups = half / 4;
   float4 qv[U];
 #pragma unroll
@@ -732,7 +746,7 @@ selected_scores_rows_kernel(const int64_t* __restrict__ idx, const float* __rest
     const int gi = u * 32 + lane;
     qv[u] = gi < groups ? *reinterpret_cast<const float4*>(query + token * ld_q + gi * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  for (int k0 = warp * GATHER; k0 < top_k; k0 += 32) {
+  for (int k0 = first; k0 < top_k; k0 += step) {
     int my_li = -1, my_ri = 0;
     if (lane < GATHER && k0 + lane < top_k) {
       const long long slot = idx[token * top_k + k0 + lane];
@@ -801,20 +815,21 @@ __global__ void selected_scores_fwd_kernel(const int64_t* __restrict__ idx, cons
   }
 }
 
-// dq[t,:] = sum_k g[t,k] * [K_L[li]; K_R[ri]] of the product-key form, sixteen-byte rows: a warp a token and 128 columns.
+// dq[t,:] = sum_k g[t,k] * [K_L[li]; K_R[ri]] of the product-key form, sixteen-byte rows: a warp a token and 128 U columns.
+template <int U>
 __global__ void __launch_bounds__(128)
 selected_query_gradient_kernel(const int64_t* __restrict__ idx, const float* __restrict__ left, const float* __restrict__ right,
                                const float* __restrict__ grad_scores, float* __restrict__ dq, long long ld_dq, int tokens, int top_k,
                                int side, int key_dim, int slots, int* __restrict__ clear) {
   pdl_begin();
   if (clear && blockIdx.x == 0 && threadIdx.x == 0) *clear = 0;  // a word that the kernels behind this one set and read
-  const int lane = threadIdx.x & 31, slices = (key_dim + 127) / 128, w = blockIdx.x * 4 + (threadIdx.x >> 5);
-  const int token = w / slices, gi = (w - token * slices) * 32 + lane, half = key_dim / 2;
+  constexpr int ROWS = GATHER / U;
+  const int lane = threadIdx.x & 31, slices = (key_dim + 128 * U - 1) / (128 * U), w = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int token = w / slices, g0 = (w - token * slices) * 32 * U + lane, half = key_dim / 2, groups = key_dim / 4, half_groups = half / 4;
   if (token >= tokens) return;
-  const bool on = gi < key_dim / 4, in_left = gi < half / 4;
-  const float* table = in_left ? left : right;
-  const int piece = in_left ? gi : gi - half / 4;
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 acc[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int k0 = 0; k0 < top_k; k0 += 32) {
     int my_li = -1, my_ri = -1;
     float my_g = 0.f;
@@ -826,26 +841,32 @@ selected_query_gradient_kernel(const int64_t* __restrict__ idx, const float* __r
         my_g = grad_scores[(size_t)token * top_k + k0 + lane];
       }
     }
-    for (int k = 0; k < min(32, top_k - k0); k += GATHER) {
-      float4 v[GATHER];
-      float g[GATHER];
-      bool there[GATHER];
+    for (int k = 0; k < min(32, top_k - k0); k += ROWS) {
+      float4 v[ROWS][U];
+      float g[ROWS];
+      bool there[ROWS];
 #pragma unroll
-      for (int j = 0; j < GATHER; ++j) {
+      for (int j = 0; j < ROWS; ++j) {
         const int li = __shfl_sync(0xffffffffu, my_li, k + j), ri = __shfl_sync(0xffffffffu, my_ri, k + j);
         g[j] = __shfl_sync(0xffffffffu, my_g, k + j);
         there[j] = li >= 0;
-        v[j] = row_piece(table, in_left ? li : ri, half, piece, on);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int gi = g0 + u * 32;
+          const bool in_left = gi < half_groups;
+          v[j][u] = row_piece(in_left ? left : right, in_left ? li : ri, half, in_left ? gi : gi - half_groups, gi < groups);
+        }
       }
 #pragma unroll
-      for (int j = 0; j < GATHER; ++j)
-        if (there[j]) {
-          acc.x = fmaf(g[j], v[j].x, acc.x); acc.y = fmaf(g[j], v[j].y, acc.y);
-          acc.z = fmaf(g[j], v[j].z, acc.z); acc.w = fmaf(g[j], v[j].w, acc.w);
-        }
+      for (int j = 0; j < ROWS; ++j)
+        if (there[j])
+#pragma unroll
+          for (int u = 0; u < U; ++u) add_scaled(acc[u], g[j], v[j][u]);
     }
   }
-  if (on) *reinterpret_cast<float4*>(dq + (size_t)token * ld_dq + gi * 4) = acc;
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (g0 + u * 32 < groups) *reinterpret_cast<float4*>(dq + (size_t)token * ld_dq + (g0 + u * 32) * 4) = acc[u];
 }
 
 // The same for any sizes, and in `exact` mode with dK[idx,:] += g[t,k] q[t]
@@ -1072,16 +1093,19 @@ __global__ void softmax_rows_bwd_kernel(const float* __restrict__ y, const float
 }
 
 // ---- weighted value: out[t,:] = sum_k w[t,k] V[idx[t,k],:] (* gate[t,:] when given)  (src/tensor.rs:3771-3900).
-// A warp a token and 128 columns; at most top_k products a column in f32 (f64 multiply-adds run at a fraction of the f32 rate).
+// A warp a token and 128 U columns; at most top_k products a column in f32 (f64 multiply-adds run at a fraction of the f32 rate).
+template <int U>
 __global__ void __launch_bounds__(128)
 weighted_value_rows_kernel(const int64_t* __restrict__ idx, const float* __restrict__ weights, const float* __restrict__ values,
                            float* __restrict__ out, int tokens, int top_k, int rows, int dim, int* __restrict__ status) {
   pdl_begin();
-  const int lane = threadIdx.x & 31, slices = (dim + 127) / 128, w = blockIdx.x * 4 + (threadIdx.x >> 5);
-  const int token = w / slices, gi = (w - token * slices) * 32 + lane;
+  constexpr int ROWS = GATHER / U;
+  const int lane = threadIdx.x & 31, slices = (dim + 128 * U - 1) / (128 * U), w = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int token = w / slices, g0 = (w - token * slices) * 32 * U + lane, groups = dim / 4;
   if (token >= tokens) return;
-  const bool on = gi < dim / 4;
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 acc[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int k0 = 0; k0 < top_k; k0 += 32) {
     int my_row = -1;
     float my_w = 0.f;
@@ -1091,26 +1115,28 @@ weighted_value_rows_kernel(const int64_t* __restrict__ idx, const float* __restr
       if (r < 0 || r >= rows) atomicExch(status + ST_BAD_INDEX, 1);
       else my_row = (int)r;
     }
-    for (int k = 0; k < min(32, top_k - k0); k += GATHER) {
-      float4 v[GATHER];
-      float wt[GATHER];
-      bool there[GATHER];
+    for (int k = 0; k < min(32, top_k - k0); k += ROWS) {
+      float4 v[ROWS][U];
+      float wt[ROWS];
+      bool there[ROWS];
 #pragma unroll
-      for (int j = 0; j < GATHER; ++j) {
+      for (int j = 0; j < ROWS; ++j) {
         const int r = __shfl_sync(0xffffffffu, my_row, k + j);
         wt[j] = __shfl_sync(0xffffffffu, my_w, k + j);
         there[j] = r >= 0;
-        v[j] = row_piece(values, r, dim, gi, on);
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[j][u] = row_piece(values, r, dim, g0 + u * 32, g0 + u * 32 < groups);
       }
 #pragma unroll
-      for (int j = 0; j < GATHER; ++j)
-        if (there[j]) {
-          acc.x = fmaf(wt[j], v[j].x, acc.x); acc.y = fmaf(wt[j], v[j].y, acc.y);
-          acc.z = fmaf(wt[j], v[j].z, acc.z); acc.w = fmaf(wt[j], v[j].w, acc.w);
-        }
+      for (int j = 0; j < ROWS; ++j)
+        if (there[j])
+#pragma unroll
+          for (int u = 0; u < U; ++u) add_scaled(acc[u], wt[j], v[j][u]);
     }
   }
-  if (on) reinterpret_cast<float4*>(out + (size_t)token * dim)[gi] = acc;
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (g0 + u * 32 < groups) reinterpret_cast<float4*>(out + (size_t)token * dim)[g0 + u * 32] = acc[u];
 }
 
 // The same for rows of more than 1024.
@@ -1715,8 +1741,9 @@ int hl_memory_selected_scores_forward(hl_ctx* ctx, const int64_t* indices, const
              "hl_memory_selected_scores_forward: product-key mode needs both half tables, even key_dim and square slots");
   if (side > 0 && rows_of_16_bytes(key_dim, ld_query, query, left_or_keys, right_keys)) {
     auto launch = [&](auto kern) {
-      pdl(kern, tokens, 128, 0, ctx->stream).streaming(4.0 * tokens * top_k * key_dim)(indices, query, ld_query, left_or_keys, right_keys, scores,
-                                                                                      top_k, side, key_dim, slots, ctx->status_dev);
+      const int log_warps = top_k <= GATHER ? 0 : top_k <= 2 * GATHER ? 1 : 2;  // a token's
+      pdl(kern, (unsigned)ceil_div_ll((long long)tokens << log_warps, 4), 128, 0, ctx->stream).streaming(4.0 * tokens * top_k * key_dim)(
+          indices, query, ld_query, left_or_keys, right_keys, scores, tokens, top_k, side, key_dim, slots, log_warps, ctx->status_dev);
     };
     if (key_dim <= 128) launch(selected_scores_rows_kernel<1>);
     else if (key_dim <= 256) launch(selected_scores_rows_kernel<2>);
@@ -1750,8 +1777,11 @@ int hl_memory_selected_scores_backward(hl_ctx* ctx, const int64_t* indices, cons
     if (clear) HL_CUDA(cudaMemsetAsync(clear, 0, sizeof(int), ctx->stream));
   } else {
     if (side > 0 && rows_of_16_bytes(key_dim, ld_grad_query, grad_query, left_or_keys, right_keys))
-      pdl(selected_query_gradient_kernel, (unsigned)ceil_div_ll((long long)tokens * ceil_div(key_dim, 128), 4), 128, 0, ctx->stream)(
-          indices, left_or_keys, right_keys, grad_scores, grad_query, ld_grad_query, tokens, top_k, side, key_dim, slots, clear);
+      by_pieces(top_k, key_dim, [&](auto pieces) {
+        constexpr int U = decltype(pieces)::value;
+        pdl(selected_query_gradient_kernel<U>, (unsigned)ceil_div_ll((long long)tokens * ceil_div(key_dim, 128 * U), 4), 128, 0, ctx->stream)(
+            indices, left_or_keys, right_keys, grad_scores, grad_query, ld_grad_query, tokens, top_k, side, key_dim, slots, clear);
+      });
     else
       pdl(selected_scores_bwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream)(
           indices, query, ld_query, left_or_keys, right_keys, grad_scores, grad_query, ld_grad_query, grad_left_or_keys,
@@ -1812,8 +1842,11 @@ int hl_memory_weighted_value_forward(hl_ctx* ctx, const int64_t* indices, const 
   if (rc != HL_OK) return rc;
   HL_REQUIRE(rows > 0 && dim % 4 == 0, "hl_memory_weighted_value_forward: non-zero rows/row_dim, row_dim a multiple of 4");
   if (dim <= 1024)
-    pdl(weighted_value_rows_kernel, (unsigned)ceil_div_ll((long long)tokens * ceil_div(dim, 128), 4), 128, 0, ctx->stream)(
-        indices, weights, values, out, tokens, top_k, rows, dim, ctx->status_dev);
+    by_pieces(top_k, dim, [&](auto pieces) {
+      constexpr int U = decltype(pieces)::value;
+      pdl(weighted_value_rows_kernel<U>, (unsigned)ceil_div_ll((long long)tokens * ceil_div(dim, 128 * U), 4), 128, 0, ctx->stream)(
+          indices, weights, values, out, tokens, top_k, rows, dim, ctx->status_dev);
+    });
   else
     pdl(weighted_value_fwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream)(indices, weights, values, out, tokens, top_k, rows, dim,
                                                                             ctx->status_dev);

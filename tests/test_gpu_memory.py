@@ -608,3 +608,45 @@ def test_half_key_gradients_without_the_querys(tokens):
         got = tables(query)
         assert c.counters().launches - before == whole - 1
     assert torch.equal(got[0], dl) and torch.equal(got[1], dr)
+
+
+@pytest.mark.parametrize("tokens,top_k,key_dim,dim", [(1, 1, 8, 4), (37, 1, 512, 1024), (1100, 2, 264, 516), (300, 3, 1024, 640), (65, 8, 256, 260),
+                                                      (66, 9, 512, 256), (67, 16, 128, 128), (69, 17, 384, 132), (4097, 3, 64, 388)])
+def test_gathers_of_few_slots(tokens, top_k, key_dim, dim):
+    """One, two and four warps or pieces of a row for a token, at the slots and columns where one gives way to the other, with a slot that
+    does not exist.  Bounds as in the test of the forms' edges above."""
+    from heirloom_b200 import cuda
+    c = ctx()
+    rng = np.random.default_rng(tokens + key_dim)
+    side = 16
+    q = rng.standard_normal((tokens, key_dim)).astype(np.float32)
+    kl, kr = (rng.standard_normal((side, key_dim // 2)).astype(np.float32) for _ in range(2))
+    vals = rng.standard_normal((side * side, dim)).astype(np.float32)
+    idx = rng.integers(0, side * side, (tokens, top_k))
+    w, g = (rng.standard_normal((tokens, top_k)).astype(np.float32) for _ in range(2))
+    go = rng.standard_normal((tokens, dim)).astype(np.float32)
+    for bad in (None, side * side, -1):
+        if bad is not None:
+            idx[tokens // 2, top_k - 1] = bad
+        there = (idx >= 0) & (idx < side * side)
+        at = np.where(there, idx, 0)
+        di = dev(idx, I64)
+        keys = np.concatenate([kl[at // side], kr[at % side]], axis=2).astype(np.float64) * there[..., None]
+        picked = vals[at].astype(np.float64) * there[..., None]
+        scores = cuda.memory_selected_scores_forward(c, di, dev(q), dev(kl), dev(kr))
+        dq, _, _ = cuda.memory_selected_scores_backward(c, di, dev(q), dev(kl), dev(kr), dev(g))
+        value = cuda.memory_weighted_value_forward(c, di, dev(w), dev(vals))
+        dw, dv = cuda.memory_weighted_value_backward(c, di, dev(w), dev(vals), dev(go))
+        if bad is None:
+            c.sync()
+        else:
+            with pytest.raises(cuda.HeirloomError, match="out-of-range index"):
+                c.sync()
+        assert_close("scores", host(scores), np.einsum("td,tkd->tk", q.astype(np.float64), keys), atol=4e-6 * np.sqrt(key_dim), rtol=1e-6)
+        assert_close("dq", host(dq), np.einsum("tk,tkd->td", g.astype(np.float64), keys), atol=4e-6 * np.sqrt(top_k), rtol=1e-6)
+        assert_close("value", host(value), np.einsum("tk,tkd->td", w.astype(np.float64), picked), atol=4e-6 * np.sqrt(top_k), rtol=1e-6)
+        assert_close("dw", host(dw)[there], np.einsum("td,tkd->tk", go.astype(np.float64), picked)[there], atol=4e-6 * np.sqrt(dim), rtol=1e-6)
+        want = np.zeros((side * side, dim))
+        np.add.at(want, at[there], w[there][:, None].astype(np.float64) * np.repeat(go[:, None], top_k, 1)[there])
+        run = np.bincount(at[there], minlength=1).max()
+        assert_close("dv", host(dv), want, atol=1e-6 * np.sqrt(run) * 4 + 2e-7 * run, rtol=1e-6)
