@@ -1216,7 +1216,7 @@ __global__ void weighted_value_bwd_rows_kernel(const int64_t* __restrict__ idx, 
     }
   }
 }
-// The same for longer rows, a warp a token.
+// The same for longer rows, and for tokens of few slots: a warp a token.
 __global__ void weighted_value_bwd_kernel(const int64_t* __restrict__ idx, const float* __restrict__ weights,
                                           const float* __restrict__ values, const float* __restrict__ grad_out,
                                           float* __restrict__ dweights, float* __restrict__ dvalues, int tokens, int top_k,
@@ -1410,7 +1410,9 @@ weighted_value_bwd_sorted_kernel(const int* __restrict__ keys, const int* __rest
                                  const float* __restrict__ weights, const float* __restrict__ values,
                                  const float* __restrict__ grad_out, float* __restrict__ dweights,
                                  float* __restrict__ dvalues, long long n, int top_k, int rows, int dim) {
-  pdl_begin();
+  // Short chunks are thousands of CTAs: a successor that came in beside them would sit where they ran and leave other SMs empty (the sort of
+  // a next call of 65536 events of 512 columns 95 -> 62 us a call; long chunks gain from it: 32 and 131072 events of 64 columns 87 -> 72).
+  pdl_begin(CHUNK < 32);
   const int lane = threadIdx.x & 31;
   const long long base = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * CHUNK;
   if (base >= n) return;
@@ -1901,9 +1903,10 @@ int weighted_value_backward_ordered(hl_ctx* ctx, const int* keys, const int* eve
     pdl(kern, (unsigned)ceil_div_ll(ceil_div_ll(n, chunk), 4), 128, 0, ctx->stream)(keys, events, weights, values, grad_out, grad_weights,
                                                                                     grad_values, n, top_k, rows, dim);
   };
-  // Short chunks where the warps of long ones would not fill the chip, us a call with its sort, long / short: 65536 events 210 / 200 and
-  // 155 / 145 (many and few distinct rows), 131072 260 / 265 and 180 / 180, 524288 375 / 380 and 240 / 255.
-  const bool few = n < 100000;
+  // Short chunks where the warps of long ones would not fill the chip, us a call with its sort, long / short: 65536 events of 512 columns
+  // 118 / 60 and 72 / 50 (many and few distinct rows), 131072 132 / 104 and 73 / 82, of 64 columns 72 / 98 and 61 / 75, 262144 90 / 146 and 80 / 114
+  // (256 columns); rows of 1024 columns: 32768 events 96 / 74 and 59 / 55, 65536 135 / 135 and 80 / 77 to 138 / 153 and 80 / 81.
+  const bool few = n < (dim > 512 ? 50000 : 100000);
   if (dim <= 512) few ? launch(weighted_value_bwd_sorted_kernel<4, 8>, 8) : launch(weighted_value_bwd_sorted_kernel<4, 32>, 32);
   else few ? launch(weighted_value_bwd_sorted_kernel<8, 8>, 8) : launch(weighted_value_bwd_sorted_kernel<8, 32>, 32);
   HL_LAUNCH_CHECK("weighted_value_bwd_sorted_kernel");
@@ -1931,7 +1934,10 @@ int hl_memory_weighted_value_backward(hl_ctx* ctx, const int64_t* indices, const
     if (rc != HL_OK) return rc;
     return weighted_value_backward_ordered(ctx, keys, events, weights, values, grad_out, grad_weights, grad_values, n, top_k, rows, dim);
   }
-  if (dim <= 1024)
+  // A CTA a token pays from a few slots on; us, a warp a token / a CTA a token: 16384 tokens of 1 slot of 512 columns 11.4 / 36, 8192 of 3
+  // 14.9 / 20.7, 2048 of 2 5.8 / 6.3, of 3 7.7 / 6.8, 1024 of 2 4.0 / 4.0, 512 of 3 4.7 / 3.4, 64 of 2 3.5 / 2.6.
+  const bool by_warp = dim > 1024 || top_k == 1 || (top_k <= 3 && tokens >= 64 << (2 * top_k));
+  if (!by_warp)
     pdl(weighted_value_bwd_rows_kernel, tokens, 32 * ceil_div(dim, 128), 0, ctx->stream)(indices, weights, values, grad_out, grad_weights,
                                                                                         grad_values, top_k, rows, dim);
   else
