@@ -373,11 +373,23 @@ size_t memory_side_bytes(const hl_decoder* m) {
   return most;
 }
 
-// Exact scores of all keys and the selection take 421 us a block at 16384 tokens, sides of 512 and keys of 512, the lookup 276; steps with
-// two blocks, all keys against the lookup: 1102 and 1020 us at 128 tokens of the same tables, 869 and 861 at 2048 tokens, sides of 128 and
-// keys of 64, 690 and 708 at 512 tokens of these.  It is the pass's own tokens that count: a prompt may be far shorter than the model's batch.
+// Whether a pass selects by the lookup.  Exact scores of all keys cost tokens * side * key_dim products, sides in tiles of 128, and no less than one
+// tile's walk along the keys, which few tokens feel; the lookup costs three products of the pieces, a pass over all approximate scores and
+// top_k exact products a side.  us a block and pass, lookup less all keys (two blocks of a two-layer model, top_k 4 / 32):
+//     tokens            1024        2048        4096        8192       16384
+//     side 512, 512    -56 / -50   -61 / -50   -65 / -43   -99 / -60  -222 / -149
+//     side 256, 256    -29 / -31   -25 / -25   -18 / -9    -19 / +6    -14 / +29
+//     side 128, 512    -22 / -27   -55 / -43   -43 / -18   -20 / +19    -7 / +67
+//     side 128, 128     -7 / -3    -11 / -8     -6 / +2     +2 / +18   +12 / +40
+//     side 32, 64                                +5 / +1     +7 / +12   +18 / +20
+// Below 2^24 products it is the launches that count (256 tokens, sides of 128 and keys of 256: -1 / +5).  It is the pass's own tokens that count: a prompt
+// may be far shorter than the model's batch.
 constexpr size_t kLookupProducts = size_t(1) << 24;  // tokens * side * key_dim
-bool looks_up(const hl_decoder* m) { return m->lookup && (size_t)m->N * m->side * m->mem.key_dim >= kLookupProducts; }
+bool looks_up(const hl_decoder* m) {
+  const double n = m->N, side = m->side, kd = m->mem.key_dim, k = m->mem.top_k;
+  return m->lookup && n * side * kd >= (double)kLookupProducts &&
+         (1.0 + 1.6 * (4096.0 / n) * (4096.0 / n)) * std::max(side, 128.0) * kd > 16000.0 + (100.0 + 4.0 * k) * kd + 60.0 * side;
+}
 
 // Buffers of the memory feed-forward blocks; appended to either route's arena.
 void plan_memory_buffers(hl_decoder* m, uint8_t*& cur) {
