@@ -155,17 +155,18 @@ struct Mail {
     if (bytes0) tc05::mbar_arrive_expect_tx(&arrived[0], bytes0);
     if (bytes1) tc05::mbar_arrive_expect_tx(&arrived[1], bytes1);
   }
-  __device__ __forceinline__ void wait(int i, unsigned long long limit_ns, int* status) {
-    if (!tc05::mbar_wait(&arrived[i], 0, &abort_flag, limit_ns)) *status = 1;
-  }
-  // At the end of the kernel.  A CTA whose wait ran out stays until its peers, whose waits are bounded as well, have left or are here too,
-  // and then until what they sent has landed: a peer may be late and not lost.
-  __device__ __forceinline__ void leave() {
-    if (!*static_cast<volatile int*>(&abort_flag)) return;
-    tc05::cluster_meet();
-    for (int k = 0; k < 2000; ++k) __nanosleep(100);
+  __device__ __forceinline__ bool wait(int i, unsigned long long limit_ns, int* status) {
+    const bool all = tc05::mbar_wait(&arrived[i], 0, &abort_flag, limit_ns);
+    if (!all) *status = 1;
+    return all;
   }
 };
+// At the end of a kernel whose wait ran out.  The thread, and with it its CTA, stays until the peers, whose waits are bounded as well, have left
+// or are here too, and then until what they sent has landed: a peer may be late and not lost.
+__device__ __noinline__ void outstay_peers() {
+  tc05::cluster_meet();
+  for (int k = 0; k < 2000; ++k) __nanosleep(100);
+}
 // `bytes` (whole sixteens) of this CTA's shared memory into a peer's, by one warp.  A store to a peer takes its turn whatever its width:
 // 96 of 32 bytes held a kernel up for 3300 cycles.
 __device__ __forceinline__ void push(uint64_t* arrived, void* to, const void* from, int bytes, int peer) {
@@ -349,6 +350,7 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_attention_block_kernel(c
   const Row<T, Acc> in(a.x, a.gamma, a.beta, a.window ? 0 : d);
   const Acc scale = (Acc)1 / sqrt((Acc)hd);
   const int fresh_at = (int)threadIdx.x / cpc * pitch_fresh + (int)threadIdx.x % cpc;
+  bool answered = true;
   tc05::cluster_meet();  // the peers have started: their shared memory may be written
   pdl_wait();
   if (a.window) {
@@ -367,7 +369,7 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_attention_block_kernel(c
     __syncthreads();
     if (warp < DB_CTAS && warp != rank) push(&mail.arrived[0], own, own, pitch_fresh * 4, warp);
     cp_async_wait_all();
-    mail.wait(0, a.wait_limit_ns, a.status);
+    answered = mail.wait(0, a.wait_limit_ns, a.status);
     if (const int i = threadIdx.x; i < rows) {  // (nobody waits for these)
       const int which = i < cpc ? 0 : i < 2 * cpc ? 1 : 2;
       qkv[(long long)t * ld + which * d + rank * cpc + i - which * cpc] = stored<T>(y);
@@ -448,7 +450,7 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_attention_block_kernel(c
   if (const int c = threadIdx.x; c < hd + 2) own[c] = c == hd ? mx : sum_of_warps(c < hd ? part : red_sum, c < hd ? hd : 1, c < hd ? c : 0);
   __syncthreads();
   if (warp < DB_CTAS && warp != rank) push(&mail.arrived[1], own, own, pitch_all * sizeof(Acc), warp);
-  mail.wait(1, a.wait_limit_ns, a.status);
+  answered &= mail.wait(1, a.wait_limit_ns, a.status);
   {
     const Acc* mine = all + (lane & 7) * pitch_all + hd;
     const Acc m = mine[0];
@@ -472,7 +474,7 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_attention_block_kernel(c
   __syncthreads();
   Acc* out = static_cast<Acc*>(a.parts) + (size_t)h * d + rank * opc;
   multiply_columns(wo, hd + PAD, opc, att, hd, [&](int o, Acc v) { out[o] = v; });
-  mail.leave();
+  if (!answered) outstay_peers();
 }
 
 // Layer norm, the hidden units of a CTA and their share of every output; the shares of a cluster are added up within it.
@@ -562,7 +564,7 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_feed_forward_kernel(cons
   });
   __syncthreads();
   if (warp < DB_CTAS) push(&mail.arrived[0], sums + rank * pitch_sums, outputs + warp * pitch_sums, pitch_sums * sizeof(Acc), warp);
-  mail.wait(0, a.wait_limit_ns, a.status);
+  const bool answered = mail.wait(0, a.wait_limit_ns, a.status);
   Acc* out = static_cast<Acc*>(a.parts) + (size_t)(blockIdx.x / DB_CTAS) * d + rank * opc;
   if (const int c = threadIdx.x; c < opc) {
     Acc s = 0;
@@ -570,7 +572,7 @@ __global__ void __launch_bounds__(DB_THREADS, 2) decode_feed_forward_kernel(cons
     for (int r = 0; r < DB_CTAS; ++r) s += sums[r * pitch_sums + c];
     out[c] = s;
   }
-  mail.leave();
+  if (!answered) outstay_peers();
 }
 
 // The row itself, for kernels that read it.
