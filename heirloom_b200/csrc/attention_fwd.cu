@@ -683,11 +683,11 @@ flash_attention_fwd64_kernel(const __grid_constant__ CUtensorMap map_q, const __
 
 // Three streams an SM are more work at a time, two are faster each (0.86 and 0.67 us a tile of a stream that is alone), and a call
 // lasts no less than its longest item.  So three where an SM's share of the tiles is a few times that item: share / longest of
-// 1.9 + (rows / 128) / 16, and up to 2048 rows.  Two / three streams, us: B16 T512 H8 15.8 / 13.8, B16 T1024 H12 59.6 / 51.1, B16 T1024 H5
+// 1.75 + (rows / 128) / 16, and up to 2048 rows.  Two / three streams, us: B16 T512 H8 15.8 / 13.8, B16 T1024 H12 59.6 / 51.1, B16 T1024 H5
 // 24.8 / 24.1, B8 T1024 H8 20.8 / 22.5, B4 T2048 H16 62.3 / 61.6, B4 T2048 H10 39.5 / 42.6, B5 T700 H13 14.4 / 16.9, B1 T4096 H16 55 / 75, B1 T4096
 // H24 84.6 / 84.1, B2 T4096 H20 133 / 139, B1 T8192 H32 391 / 407.
 bool three_streams(int items, int tiles, int sms) {
-  return tiles <= 16 && 8ll * items * (tiles + 1) >= (long long)sms * tiles * (30 + tiles);
+  return tiles <= 16 && 8ll * items * (tiles + 1) >= (long long)sms * tiles * (28 + tiles);
 }
 
 }  // namespace
