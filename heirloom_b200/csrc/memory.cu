@@ -1780,19 +1780,20 @@ int hl_memory_selected_scores_backward(hl_ctx* ctx, const int64_t* indices, cons
   // the tensor-core form's scratch holds the queries' pieces as well: where the device has no room for them, the f32 form
   const bool tensor = token_blocks > 0 && try_workspace(ctx, key_gradient_bytes(keys, token_blocks));
   int* clear = tensor ? static_cast<int*>(ctx->workspace) : nullptr;
-  if (side > 0 && !grad_query) {  // the tables' gradients alone
-    if (clear) HL_CUDA(cudaMemsetAsync(clear, 0, sizeof(int), ctx->stream));
-  } else {
-    if (side > 0 && rows_of_16_bytes(key_dim, ld_grad_query, grad_query, left_or_keys, right_keys))
-      by_pieces(top_k, key_dim, [&](auto pieces) {
-        constexpr int U = decltype(pieces)::value;
-        pdl(selected_query_gradient_kernel<U>, (unsigned)ceil_div_ll((long long)tokens * ceil_div(key_dim, 128 * U), 4), 128, 0, ctx->stream)(
-            indices, left_or_keys, right_keys, grad_scores, grad_query, ld_grad_query, tokens, top_k, side, key_dim, slots, clear);
-      });
-    else
-      pdl(selected_scores_bwd_kernel, ceil_div(tokens, 4), 128, 0, ctx->stream)(
-          indices, query, ld_query, left_or_keys, right_keys, grad_scores, grad_query, ld_grad_query, grad_left_or_keys,
-          grad_right_keys, tokens, top_k, side, key_dim, slots, clear);
+  const bool alone = side > 0 && !grad_query;  // the tables' gradients, whose kernels come below
+  if (alone && !clear) {
+  } else if (side > 0 && !alone && rows_of_16_bytes(key_dim, ld_grad_query, grad_query, left_or_keys, right_keys)) {
+    by_pieces(top_k, key_dim, [&](auto pieces) {
+      constexpr int U = decltype(pieces)::value;
+      pdl(selected_query_gradient_kernel<U>, (unsigned)ceil_div_ll((long long)tokens * ceil_div(key_dim, 128 * U), 4), 128, 0, ctx->stream)(
+          indices, left_or_keys, right_keys, grad_scores, grad_query, ld_grad_query, tokens, top_k, side, key_dim, slots, clear);
+    });
+    HL_LAUNCH_CHECK("selected_query_gradient_kernel");
+    count_launch(ctx);
+  } else {  // `alone`: a block that clears the word (a memset in front of dependent launches: 2320 us a step of sparse fine-tuning, 2275)
+    pdl(selected_scores_bwd_kernel, alone ? 1 : ceil_div(tokens, 4), 128, 0, ctx->stream)(
+        indices, query, ld_query, left_or_keys, right_keys, grad_scores, grad_query, ld_grad_query, grad_left_or_keys,
+        grad_right_keys, tokens, top_k, side, key_dim, slots, clear);
     HL_LAUNCH_CHECK("selected_scores_bwd_kernel");
     count_launch(ctx);
   }
