@@ -13,8 +13,9 @@
 // again for every row of weights (24 rows of 768: 2700 cycles); on the matrix instruction the row is the second operand, the same in
 // all of its columns, and the warps share the contraction (1100).
 //
-// A one-token step of the GPT-sized model at 500 positions: 271 -> 225 us (attention kernel 10, feed-forward 6.6, head 20); generation
-// of 8 tokens behind a prefix of 500 2690 -> 2377 us, of 32 with four f32 blocks of 128 channels (24 one-token steps) 3550 -> 3080.
+// A one-token step of the GPT-sized model at 500 positions: 271 -> 211 us (attention kernel 9.8, feed-forward 5.6, head 19, the choice
+// 7.6); generation of 8 tokens behind a prefix of 500 2690 -> 2215 us, of 32 with four f32 blocks of 128 channels (24 one-token steps)
+// 3550 -> 3010.
 #include "decode.cuh"
 #include "tc05.cuh"
 
@@ -69,7 +70,15 @@ struct RowMma {
   }
 };
 
-// Rows of weights times x, both in shared memory.  bf16: the warps share the contraction, red[warp][row] is left for sum_of_warps
+template <typename Acc>
+__device__ __forceinline__ Acc sum_of_warps(const Acc* red, int rows, int r) {
+  Acc s = 0;
+#pragma unroll
+  for (int w = 0; w < DB_WARPS; ++w) s += red[w * rows + r];
+  return s;
+}
+
+// Rows of weights times x, both in shared memory.  bf16: the warps share the contraction, red[warp][row] is left for product_of_row
 // behind a barrier; k a multiple of 16.  f64 sums: a warp a row (the f64 matrix instruction, four values a step, took longer).
 __device__ __forceinline__ void multiply_rows(const __nv_bfloat16* w, int pitch, int rows, const __nv_bfloat16* x, int k, float* red) {
   const int warp = threadIdx.x >> 5;
@@ -81,12 +90,7 @@ __device__ __forceinline__ void multiply_rows(const __nv_bfloat16* w, int pitch,
     t.rows(rows - 1 - m, [&](int r, float v) { red[warp * rows + m + r] = v; });
   }
 }
-__device__ __forceinline__ float product_of_row(const float* red, int rows, int r) {
-  float s = 0;
-#pragma unroll
-  for (int w = 0; w < DB_WARPS; ++w) s += red[w * rows + r];
-  return s;
-}
+__device__ __forceinline__ float product_of_row(const float* red, int rows, int r) { return sum_of_warps(red, rows, r); }
 __device__ __forceinline__ void multiply_rows(const float* w, int pitch, int rows, const float* x, int k, double* red) {
 #pragma unroll 1
   for (int r = threadIdx.x >> 5; r < rows; r += DB_WARPS) {
@@ -132,14 +136,6 @@ __device__ __forceinline__ void multiply_columns(const float* w, int pitch, int 
     }
     put(r, acc);
   }
-}
-
-template <typename Acc>
-__device__ __forceinline__ Acc sum_of_warps(const Acc* red, int rows, int r) {
-  Acc s = 0;
-#pragma unroll
-  for (int w = 0; w < DB_WARPS; ++w) s += red[w * rows + r];
-  return s;
 }
 
 // What the peers of a cluster send arrives on barriers that count its bytes: a barrier of the cluster behind the stores cost a release,
