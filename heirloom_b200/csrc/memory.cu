@@ -1781,8 +1781,7 @@ int hl_memory_selected_scores_backward(hl_ctx* ctx, const int64_t* indices, cons
   const bool tensor = token_blocks > 0 && try_workspace(ctx, key_gradient_bytes(keys, token_blocks));
   int* clear = tensor ? static_cast<int*>(ctx->workspace) : nullptr;
   const bool alone = side > 0 && !grad_query;  // the tables' gradients, whose kernels come below
-  if (alone && !clear) {
-  } else if (side > 0 && !alone && rows_of_16_bytes(key_dim, ld_grad_query, grad_query, left_or_keys, right_keys)) {
+  if (side > 0 && !alone && rows_of_16_bytes(key_dim, ld_grad_query, grad_query, left_or_keys, right_keys)) {
     by_pieces(top_k, key_dim, [&](auto pieces) {
       constexpr int U = decltype(pieces)::value;
       pdl(selected_query_gradient_kernel<U>, (unsigned)ceil_div_ll((long long)tokens * ceil_div(key_dim, 128 * U), 4), 128, 0, ctx->stream)(
@@ -1790,7 +1789,7 @@ int hl_memory_selected_scores_backward(hl_ctx* ctx, const int64_t* indices, cons
     });
     HL_LAUNCH_CHECK("selected_query_gradient_kernel");
     count_launch(ctx);
-  } else {  // `alone`: a block that clears the word (a memset in front of dependent launches: 2320 us a step of sparse fine-tuning, 2275)
+  } else if (!alone || clear) {  // `alone`: a block that clears the word (a memset in front of dependent launches: 2320 us a step of sparse fine-tuning, 2275)
     pdl(selected_scores_bwd_kernel, alone ? 1 : ceil_div(tokens, 4), 128, 0, ctx->stream)(
         indices, query, ld_query, left_or_keys, right_keys, grad_scores, grad_query, ld_grad_query, grad_left_or_keys,
         grad_right_keys, tokens, top_k, side, key_dim, slots, clear);
